@@ -11,6 +11,7 @@
 #include "moe_common.cuh"
 #include "prof.cuh"
 #include "ptx.cuh"
+#include "split_gemm.cuh"
 
 namespace kb2 {
 
@@ -219,8 +220,11 @@ cudaError_t launch_dense_gemm(const void* x, const void* w, void* out, const flo
 cudaError_t launch_dense_gemm_scatter(const void* x, const void* w, void* out, const float* bias, int M, int N, int K,
                                       long long ldo, bool out_f32, int num_sms, cudaStream_t s, const CombineScatter& sc) {
   if (sc.n_ranks > 0 && (out_f32 || M % sc.n_ranks || sc.rows_per_rank * sc.n_ranks != M)) return cudaErrorInvalidValue;
-  KernelSpan ks(K_DENSE_BF16, s);
   if (K % kBlockK || N % 16 || M <= 0) return cudaErrorInvalidValue;
+  SplitPlan plan;
+  if (sc.n_ranks == 0 && split_gemm_plan(M, N, K, out_f32, num_sms, &plan))
+    return launch_split_gemm(x, w, out, bias, M, N, K, ldo, out_f32, plan, nullptr, nullptr, 1, s);
+  KernelSpan ks(K_DENSE_BF16, s);
   alignas(64) CUtensorMap tx, tw;
   cudaError_t e = make_tmap_bf16_rows(&tx, x, M, K, 128);
   if (e != cudaSuccess) return e;

@@ -49,6 +49,8 @@ import torch
 from . import seqops as ops
 
 
+# rows up to which kb2_seq_gemm runs its GEMV kernels
+GEMV_ROWS = 8
 _core = None
 
 
@@ -67,13 +69,13 @@ def _core_lib():
     return _core
 
 
-def lin(a: torch.Tensor, w: torch.Tensor, out_dtype=torch.float32, min_n: int = 256) -> torch.Tensor:
-    """a [M, K] @ w [N, K]^T with fp32 accumulation.  min_n: the narrowest output that still goes to the tcgen05 kernel (its tiles are
-    256 columns wide; a router's few columns are worth it all the same when the step is long)."""
+def lin(a: torch.Tensor, w: torch.Tensor, out_dtype=torch.float32) -> torch.Tensor:
+    """a [M, K] @ w [N, K]^T with fp32 accumulation.  Bfloat16 products of more rows than a GEMV takes run on the tensor cores (the core
+    library picks the kernel by the sizes); at 8 rows and fewer the weights are streamed by `gemv_nt_vec`."""
     M, K = a.shape
     N = w.shape[0]
-    if (a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and M >= 256 and K % 64 == 0 and N % 16 == 0 and N >= min_n
-            and a.is_contiguous() and w.is_contiguous()):
+    if (a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and M > GEMV_ROWS and K % 64 == 0 and N % 16 == 0 and a.is_contiguous()
+            and w.is_contiguous() and w.shape[1] == K and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
         core = _core_lib()
         if core:
             from . import capi
@@ -348,7 +350,7 @@ class SelectiveScan:
         proj = lin(h, self.w_in, torch.float32)                                               # [T, x: C | z: C]
         xc = ops.conv(proj, self.C, self.taps, None, True, tail, tb, bias_out=self.conv_b)    # [T, C] fp32
         big = self.dtype == torch.bfloat16 and T >= 256 and bool(_core_lib())
-        xp = lin(xc.to(torch.bfloat16) if big else xc, self.w_x, torch.float32, min_n=16)     # [T, dt: R | B: N | C: N]
+        xp = lin(xc.to(torch.bfloat16) if big else xc, self.w_x, torch.float32)     # [T, dt: R | B: N | C: N]
         dt_in = lin_cols(xp, 0, self.R, self.w_dt, self.dtype)                                # [T, C]
         y = torch.empty((T, self.C), dtype=self.dtype, device=h.device)
         ops.check(lib.kb2_seq_selective_scan(xc.data_ptr(), xc.stride(0), dt_in.data_ptr(), dt_in.stride(0), self.dt_b.data_ptr(),
@@ -940,7 +942,7 @@ class RoutedExperts:
 
     def route(self, h: torch.Tensor):
         """(ids, weights, router product [T, >= E + identity] whose column sg_col is the shared expert's gate input)."""
-        z = lin(h, self.w_router, torch.float32, min_n=16)
+        z = lin(h, self.w_router, torch.float32)
         return ops.route(z, self.correction, self.top, self.groups, self.keep, self.score, self.renorm, self.out_scale, self.group_score,
                          experts=self.E + self.ident, bias=self.router_bias) + (z,)
 
