@@ -226,6 +226,12 @@ KB2_API int kb2_linear_bf16_grouped(const void* x_dev, const void* w_dev, void* 
                                     const int32_t* tile_group_dev, const int32_t* num_row_tiles_dev, int32_t groups, int32_t device,
                                     void* stream);
 
+/* The same for runs padded to tiles of tile_rows rows (a multiple of 16, at most 128), for groups that bring few rows each: the time is that
+ * of the weights, and small tiles leave little padding. */
+KB2_API int kb2_linear_bf16_binned(const void* x_dev, const void* w_dev, void* out_dev, int32_t M, int32_t N, int32_t K, int32_t out_f32,
+                                   int32_t tile_rows, const int32_t* tile_group_dev, const int32_t* num_row_tiles_dev, int32_t groups,
+                                   int32_t device, void* stream);
+
 /* flashinfer.norm.rmsnorm (residual_dev == NULL) / fused_add_rmsnorm (residual_dev != NULL: residual += x, in place)
  * as used at python/krasis/layer.py:163-183,283-308.  x, residual, out: [M][H] bf16 (out may alias x); weight [H] f32. */
 KB2_API int kb2_rmsnorm(void* x_dev, void* residual_dev, const float* weight_dev, void* out_dev, int32_t M, int32_t H,

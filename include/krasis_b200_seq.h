@@ -190,6 +190,12 @@ KB2SEQ_API int kb2_seq_route(const float* z, long long ldz, int T, int E, const 
 KB2SEQ_API int kb2_seq_moe_tile_rows(void);
 KB2SEQ_API int kb2_seq_moe_bin(const int* ids, long long slots, int E, int tile_rows, int* counts, int* offs, int* cursor, int* tile_expert,
                                int* n_tiles, int* slot_row, long long max_rows, int* pos_of_slot, void* stream);
+/* The same tables with tiles of any multiple of 16 rows, and bf16 rows copied into that order: xs [max_rows][W], row p = h[slot_row[p] / top]
+ * (padding rows stay unwritten); W and ldh multiples of 8, both pointers 16-byte aligned. */
+KB2SEQ_API int kb2_seq_moe_bin16(const int* ids, long long slots, int E, int tile_rows, int* counts, int* offs, int* cursor, int* tile_expert,
+                                 int* n_tiles, int* slot_row, long long max_rows, int* pos_of_slot, void* stream);
+KB2SEQ_API int kb2_seq_moe_gather(const void* h, long long ldh, const int* slot_row, int top, const int* n_tiles, int tile_rows, long long max_rows,
+                                  void* xs, int W, void* stream);
 /* C[p, :] = A[src(p), :] * B[tile_expert[p / tile]]^T (B: [experts][N][ldb], expert stride sB) for the rows of the first n_tiles[0] tiles;
  * src(p) = p, or row_map[p] / div when row_map is given (negative: zeros). */
 KB2SEQ_API int kb2_seq_moe_gemm(const void* A, int dtA, long long lda, const int* row_map, int div, const void* B, int dtB, long long ldb,

@@ -7,6 +7,7 @@
 
 #include "../../include/krasis_b200.h"
 #include "moe_common.cuh"
+#include "split_gemm.cuh"
 
 namespace kb2 {
 struct GdnDims {
@@ -152,6 +153,18 @@ KB2_API int kb2_linear_bf16_grouped(const void* x_dev, const void* w_dev, void* 
   CUDA_TRY(cudaSetDevice(device));
   CUDA_TRY(launch_dense_gemm_grouped(x_dev, w_dev, out_dev, M, N, K, N, out_f32 != 0, tile_group_dev, num_row_tiles_dev, groups,
                                      device_sms(device), (cudaStream_t)stream));
+  return KB2_OK;
+}
+
+KB2_API int kb2_linear_bf16_binned(const void* x_dev, const void* w_dev, void* out_dev, int32_t M, int32_t N, int32_t K, int32_t out_f32,
+                                   int32_t tile_rows, const int32_t* tile_group_dev, const int32_t* num_row_tiles_dev, int32_t groups,
+                                   int32_t device, void* stream) {
+  if (!x_dev || !w_dev || !out_dev || !tile_group_dev || !num_row_tiles_dev) return failf(KB2_ERR_VALUE, "null argument");
+  if (M <= 0 || N <= 0 || K <= 0 || K % 64 || N % 16 || groups <= 0 || tile_rows < 16 || tile_rows > 128 || tile_rows % 16 || M % tile_rows)
+    return failf(KB2_ERR_VALUE, "binned linear: need M>0, K %% 64 == 0, N %% 16 == 0, groups > 0, tiles of 16..128 rows that divide M (M=%d N=%d K=%d)", M, N, K);
+  CUDA_TRY(cudaSetDevice(device));
+  CUDA_TRY(launch_split_gemm(x_dev, w_dev, out_dev, nullptr, M, N, K, N, out_f32 != 0, split_gemm_binned_plan(N, K, out_f32 != 0, tile_rows),
+                             tile_group_dev, num_row_tiles_dev, groups, (cudaStream_t)stream));
   return KB2_OK;
 }
 

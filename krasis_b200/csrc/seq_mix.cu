@@ -672,6 +672,79 @@ __global__ void moe_scatter_kernel(const int* __restrict__ ids, long long slots,
   }
 }
 
+// All of the above in one block for short steps, where five launches cost more than the work (768 slots, 64 experts: 11 us as two fills and
+// three kernels): counters and cursors in shared memory, a warp's scan over the experts.  The tables are the same.
+constexpr int kBinThreads = 1024, kBinMaxExperts = 1024;
+constexpr long long kBinMaxSlots = 8192;
+__global__ void __launch_bounds__(kBinThreads) moe_bin_block_kernel(const int* __restrict__ ids, int slots, int E, int tile_rows,
+                                                                    int* __restrict__ counts, int* __restrict__ offs, int* __restrict__ tile_expert,
+                                                                    int* __restrict__ n_tiles, int* __restrict__ slot_row, int max_rows,
+                                                                    int* __restrict__ pos_of_slot) {
+  __shared__ int cnt[kBinMaxExperts], first[kBinMaxExperts + 1];
+  for (int e = threadIdx.x; e < E; e += kBinThreads) cnt[e] = 0;
+  for (int r = threadIdx.x; r < max_rows; r += kBinThreads) slot_row[r] = -1;
+  __syncthreads();
+  for (int i = threadIdx.x; i < slots; i += kBinThreads) {
+    const int e = ids[i];
+    if (e >= 0 && e < E) atomicAdd(&cnt[e], 1);
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    int before = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + threadIdx.x;
+      const int tiles = e < E ? (cnt[e] + tile_rows - 1) / tile_rows : 0;
+      int upto = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (threadIdx.x >= o) upto += v;
+      }
+      if (e < E) first[e] = before + upto - tiles;
+      before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (threadIdx.x == 0) {
+      first[E] = before;
+      n_tiles[0] = before;
+      offs[E] = before * tile_rows;
+    }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += kBinThreads) {
+    counts[e] = cnt[e];
+    offs[e] = first[e] * tile_rows;
+    for (int t = first[e]; t < first[e + 1]; ++t) tile_expert[t] = e;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += kBinThreads) cnt[e] = first[e] * tile_rows;       // from here on: the next free row of the run
+  __syncthreads();
+  for (int i = threadIdx.x; i < slots; i += kBinThreads) {
+    const int e = ids[i];
+    int p = -1;
+    if (e >= 0 && e < E) {
+      p = atomicAdd(&cnt[e], 1);
+      slot_row[p] = i;
+    }
+    pos_of_slot[i] = p;
+  }
+}
+
+// xs[p, :] = h[slot_row[p] / top, :] for the rows of the first n_tiles[0] tiles, a warp per row, 16 bytes per lane; padding rows are left as
+// they are (a product's row depends on its own input row only, and nothing reads theirs).  Bound by traffic: 2 x 4 KB per row of 2048.
+__global__ void __launch_bounds__(256) moe_gather_kernel(const bf16* __restrict__ h, long long ldh, const int* __restrict__ slot_row, int top,
+                                                         const int* __restrict__ n_tiles, int tile_rows, bf16* __restrict__ xs, int W) {
+  const int lane = threadIdx.x & 31;
+  const long long rows = (long long)n_tiles[0] * tile_rows;
+  for (long long p = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); p < rows; p += (long long)gridDim.x * 8) {
+    const int slot = slot_row[p];
+    if (slot < 0) continue;
+    const uint4* src = reinterpret_cast<const uint4*>(h + (long long)(slot / top) * ldh);
+    uint4* dst = reinterpret_cast<uint4*>(xs + p * W);
+#pragma unroll 4
+    for (int d = lane; d < W / 8; d += 32) dst[d] = src[d];
+  }
+}
+
 // C[p, :] = A[src(p), :] * B[expert of p's tile]^T for the rows p of tile blockIdx.y.  src(p) = p, or row_map[p] / div through a map
 // (negative: a padding row, computed as zeros).  64 x 64 tile, fp32 FMA, every output sums its K products in one fixed order.
 template <typename TA, typename TB, typename TC>
@@ -960,12 +1033,17 @@ KB2SEQ_API int kb2_seq_route(const float* z, long long ldz, int T, int E, const 
 
 KB2SEQ_API int kb2_seq_moe_tile_rows(void) { return kMoeBM; }
 
-KB2SEQ_API int kb2_seq_moe_bin(const int* ids, long long slots, int E, int tile_rows, int* counts, int* offs, int* cursor, int* tile_expert,
-                               int* n_tiles, int* slot_row, long long max_rows, int* pos_of_slot, void* stream) {
+static int moe_bin(const int* ids, long long slots, int E, int tile_rows, int* counts, int* offs, int* cursor, int* tile_expert, int* n_tiles,
+                   int* slot_row, long long max_rows, int* pos_of_slot, cudaStream_t s) {
   if (!ids || !counts || !offs || !cursor || !tile_expert || !n_tiles || !slot_row || !pos_of_slot || slots <= 0 || E <= 0 ||
-      tile_rows <= 0 || tile_rows % kMoeBM || max_rows < slots + (long long)E * (tile_rows - 1))
+      max_rows < slots + (long long)E * (tile_rows - 1))
     return failf(KB2SEQ_ERR_VALUE, "moe_bin: bad argument");
-  cudaStream_t s = (cudaStream_t)stream;
+  if (slots <= kBinMaxSlots && E <= kBinMaxExperts && max_rows <= 1 << 18) {
+    moe_bin_block_kernel<<<1, kBinThreads, 0, s>>>(ids, (int)slots, E, tile_rows, counts, offs, tile_expert, n_tiles, slot_row, (int)max_rows,
+                                                   pos_of_slot);
+    SEQ_LAUNCHED();
+    return KB2SEQ_OK;
+  }
   SEQ_CUDA(cudaMemsetAsync(counts, 0, (size_t)E * 4, s));
   SEQ_CUDA(cudaMemsetAsync(slot_row, 0xFF, (size_t)max_rows * 4, s));
   const unsigned blocks = (unsigned)((slots + 255) / 256 > 1024 ? 1024 : (slots + 255) / 256);
@@ -974,6 +1052,29 @@ KB2SEQ_API int kb2_seq_moe_bin(const int* ids, long long slots, int E, int tile_
   moe_plan_kernel<<<1, 256, 0, s>>>(counts, E, tile_rows, offs, cursor, tile_expert, n_tiles);
   SEQ_LAUNCHED();
   moe_scatter_kernel<<<blocks, 256, 0, s>>>(ids, slots, E, offs, cursor, slot_row, pos_of_slot);
+  SEQ_LAUNCHED();
+  return KB2SEQ_OK;
+}
+
+KB2SEQ_API int kb2_seq_moe_bin(const int* ids, long long slots, int E, int tile_rows, int* counts, int* offs, int* cursor, int* tile_expert,
+                               int* n_tiles, int* slot_row, long long max_rows, int* pos_of_slot, void* stream) {
+  if (tile_rows <= 0 || tile_rows % kMoeBM) return failf(KB2SEQ_ERR_VALUE, "moe_bin: tiles are multiples of %d rows", kMoeBM);
+  return moe_bin(ids, slots, E, tile_rows, counts, offs, cursor, tile_expert, n_tiles, slot_row, max_rows, pos_of_slot, (cudaStream_t)stream);
+}
+
+KB2SEQ_API int kb2_seq_moe_bin16(const int* ids, long long slots, int E, int tile_rows, int* counts, int* offs, int* cursor, int* tile_expert,
+                                 int* n_tiles, int* slot_row, long long max_rows, int* pos_of_slot, void* stream) {
+  if (tile_rows <= 0 || tile_rows % 16) return failf(KB2SEQ_ERR_VALUE, "moe_bin16: tiles are multiples of 16 rows");
+  return moe_bin(ids, slots, E, tile_rows, counts, offs, cursor, tile_expert, n_tiles, slot_row, max_rows, pos_of_slot, (cudaStream_t)stream);
+}
+
+KB2SEQ_API int kb2_seq_moe_gather(const void* h, long long ldh, const int* slot_row, int top, const int* n_tiles, int tile_rows, long long max_rows,
+                                  void* xs, int W, void* stream) {
+  if (!h || !slot_row || !n_tiles || !xs || top <= 0 || tile_rows <= 0 || max_rows <= 0 || W <= 0 || W % 8 || ldh % 8 || ((uintptr_t)h & 15) ||
+      ((uintptr_t)xs & 15))
+    return failf(KB2SEQ_ERR_VALUE, "moe_gather: bad argument");
+  const unsigned blocks = (unsigned)((max_rows + 7) / 8 > 2368 ? 2368 : (max_rows + 7) / 8);
+  moe_gather_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>((const bf16*)h, ldh, slot_row, top, n_tiles, tile_rows, (bf16*)xs, W);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
 }

@@ -251,6 +251,16 @@ bool split_gemm_plan(int M, int N, int K, bool out_f32, int num_sms, SplitPlan* 
   return found;
 }
 
+SplitPlan split_gemm_binned_plan(int N, int K, bool out_f32, int tile_rows) {
+  SplitPlan p;
+  p.nt = tile_rows;
+  int n_acc = out_f32 ? ceil_div(K / kBlockK, kSplitChunk) : 1;
+  while (n_acc > 1 && n_acc * tile_rows > 256) n_acc = ceil_div(n_acc, 2);         // half of the tensor memory, so that two CTAs share an SM
+  p.chunk = ceil_div(K / kBlockK, n_acc);
+  p.stages = ring_stages(tile_rows, K / kBlockK, true);
+  return p;
+}
+
 cudaError_t launch_split_gemm(const void* x, const void* w, void* out, const float* bias, int M, int N, int K, long long ldo, bool out_f32,
                               const SplitPlan& plan, const int* tile_group, const int* n_tiles_dev, int groups, cudaStream_t s) {
   KernelSpan span(K_DENSE_BF16, s);

@@ -19,6 +19,9 @@ struct SplitPlan {
 // false: the 128 x 256 tiles of dense_gemm.cu are the better cut of this product
 bool split_gemm_plan(int M, int N, int K, bool out_f32, int num_sms, SplitPlan* out);
 
+// binned rows (one weight matrix per row tile): a CTA per tile and 128 columns, K uncut
+SplitPlan split_gemm_binned_plan(int N, int K, bool out_f32, int tile_rows);
+
 cudaError_t launch_split_gemm(const void* x, const void* w, void* out, const float* bias, int M, int N, int K, long long ldo, bool out_f32,
                               const SplitPlan& plan, const int* tile_group, const int* n_tiles_dev, int groups, cudaStream_t s);
 

@@ -896,8 +896,8 @@ class RoutedExperts:
                                alpha=alpha) if "shared_up" in weights else None
         self.tile = ops.load().kb2_seq_moe_tile_rows()
         self.gemv_max_tokens = 8
-        # bfloat16 steps that bring at least this many rows per expert on average run on the grouped tcgen05 GEMM (128-row tiles)
-        self.tc_min_rows_per_expert = 16
+        # bfloat16 steps longer than the GEMV's that bring at least this many rows per expert run on the tensor cores
+        self.tc_min_rows_per_expert = 0
 
     def _bin(self, ids, slots, tile):
         """Device tables of the binned order with runs padded to `tile` rows (see kb2_seq_moe_bin)."""
@@ -908,37 +908,52 @@ class RoutedExperts:
         t = {"counts": ints[:E], "offs": ints[E:2 * E + 1], "cursor": ints[2 * E + 1:3 * E + 1], "n_tiles": ints[3 * E + 1:3 * E + 2],
              "tile_expert": ints[3 * E + 2:3 * E + 2 + max_tiles], "slot_row": ints[3 * E + 2 + max_tiles:3 * E + 2 + max_tiles + max_rows],
              "pos": ints[3 * E + 2 + max_tiles + max_rows:], "max_rows": max_rows, "max_tiles": max_tiles}
-        ops.check(ops.load().kb2_seq_moe_bin(ids.data_ptr(), slots, E, tile, t["counts"].data_ptr(), t["offs"].data_ptr(), t["cursor"].data_ptr(),
-                                             t["tile_expert"].data_ptr(), t["n_tiles"].data_ptr(), t["slot_row"].data_ptr(), max_rows,
-                                             t["pos"].data_ptr(), torch.cuda.current_stream(dev).cuda_stream))
+        fn = ops.load().kb2_seq_moe_bin if tile % self.tile == 0 else ops.load().kb2_seq_moe_bin16
+        ops.check(fn(ids.data_ptr(), slots, E, tile, t["counts"].data_ptr(), t["offs"].data_ptr(), t["cursor"].data_ptr(), t["tile_expert"].data_ptr(),
+                     t["n_tiles"].data_ptr(), t["slot_row"].data_ptr(), max_rows, t["pos"].data_ptr(), torch.cuda.current_stream(dev).cuda_stream))
         return t
 
     def _tensor_core_ok(self, h, slots):
         W = h.shape[1]
-        return (self.dtype == torch.bfloat16 and h.dtype == torch.bfloat16 and h.is_contiguous() and W % 64 == 0 and self.F % 64 == 0
-                and slots >= self.tc_min_rows_per_expert * self.E and bool(_core_lib()))
+        return (self.dtype == torch.bfloat16 and h.dtype == torch.bfloat16 and h.is_contiguous() and h.data_ptr() % 16 == 0 and W % 64 == 0
+                and self.F % 64 == 0 and slots >= self.tc_min_rows_per_expert * self.E and bool(_core_lib()))
+
+    def _tile_rows(self, slots):
+        """Rows of a tile of the binned order, by the rows an expert has on average: the smallest tile that most runs fit in.  64 experts,
+        width 2048, ff 1024, us per block: 12 rows 185 (tiles of 16) / 195 (32); 24 rows 213 / 196; 36 rows 222 (32) / 209 (48); 48 rows
+        232 (48) / 225 (64); 72 rows 291 (64) / 263 (128)."""
+        mean = slots / self.E
+        for tile, most in ((16, 14), (32, 28), (48, 42), (64, 56)):
+            if mean <= most:
+                return tile
+        return 128
 
     def _forward_tensor_core(self, h, ids, slots, in_w):
-        """Long bfloat16 steps: rows gathered into the binned order (runs padded to the 128-row tiles of the tcgen05 GEMM), then ONE
-        grouped GEMM per projection: every row tile multiplies its expert's matrix, picked from the device-side tile table, and only
-        the tiles that exist are computed — no host round trip."""
+        """bfloat16 steps: rows gathered into the binned order (runs padded to whole tiles), then ONE grouped GEMM per projection: every
+        row tile multiplies its expert's matrix, picked from the device-side tile table, and only the tiles that exist are computed — no
+        host round trip.  Few rows per expert: tiles of 32 or 64 rows, a CTA per tile and 128 columns, so that the time is that of the
+        weights; many: the 128 x 256 tiles of the dense GEMM."""
         from . import capi
         core, E, top, W, F, dev = _core_lib(), self.E, self.top, h.shape[1], self.F, h.device
         s = torch.cuda.current_stream(dev).cuda_stream
-        t = self._bin(ids, slots, 128)
+        tile = self._tile_rows(slots)
+        t = self._bin(ids, slots, tile)
         rows, di = t["max_rows"], dev.index or 0
-        src = torch.div(t["slot_row"].clamp_min(0), top, rounding_mode="floor").to(torch.int64)     # padding rows read token 0; never used
-        xs = h.index_select(0, src)
-        F1 = self.w_gu.shape[1]
-        gu = torch.empty((rows, F1), dtype=torch.bfloat16, device=dev)
-        capi.check(core.kb2_linear_bf16_grouped(xs.data_ptr(), self.w_gu.data_ptr(), gu.data_ptr(), rows, F1, W, 0, t["tile_expert"].data_ptr(),
-                                                t["n_tiles"].data_ptr(), E, di, s))
-        act = ops.glu(gu, torch.bfloat16, self.act_kind, self.limit, self.alpha, n_tiles=t["n_tiles"], tile_rows=128, row_w=in_w,
+        xs = torch.empty((rows, W), dtype=torch.bfloat16, device=dev)
+        ops.check(ops.load().kb2_seq_moe_gather(h.data_ptr(), h.stride(0), t["slot_row"].data_ptr(), top, t["n_tiles"].data_ptr(), tile, rows,
+                                                xs.data_ptr(), W, s))
+
+        def product(x, w, out, f32):
+            table = (t["tile_expert"].data_ptr(), t["n_tiles"].data_ptr(), E, di, s)
+            if tile == 128:
+                capi.check(core.kb2_linear_bf16_grouped(x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, w.shape[1], w.shape[2], f32, *table))
+            else:
+                capi.check(core.kb2_linear_bf16_binned(x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, w.shape[1], w.shape[2], f32, tile, *table))
+            return out
+        gu = product(xs, self.w_gu, torch.empty((rows, self.w_gu.shape[1]), dtype=torch.bfloat16, device=dev), 0)
+        act = ops.glu(gu, torch.bfloat16, self.act_kind, self.limit, self.alpha, n_tiles=t["n_tiles"], tile_rows=tile, row_w=in_w,
                       row_map=t["slot_row"])
-        y = torch.empty((rows, W), dtype=torch.float32, device=dev)
-        capi.check(core.kb2_linear_bf16_grouped(act.data_ptr(), self.w_down.data_ptr(), y.data_ptr(), rows, W, F, 1, t["tile_expert"].data_ptr(),
-                                                t["n_tiles"].data_ptr(), E, di, s))
-        return y, t["pos"]
+        return product(act, self.w_down, torch.empty((rows, W), dtype=torch.float32, device=dev), 1), t["pos"]
 
     def route(self, h: torch.Tensor):
         """(ids, weights, router product [T, >= E + identity] whose column sg_col is the shared expert's gate input)."""

@@ -49,3 +49,57 @@ def test_misaligned_rows_take_the_general_kernel():
     x, w = flat[1:].view(40, 128), torch.randn(48, 128, device="cuda").bfloat16()
     want = x.double() @ w.double().T
     assert ((lin(x, w, torch.float32).double() - want).abs() <= _bound(x, w) + 1e-6).all()
+
+
+# mean rows per expert on both sides of every tile size (16, 32, 48, 64, 128), with experts that get no row and one that gets most
+@pytest.mark.parametrize("T,E,top", [(9, 64, 2), (13, 2, 2), (30, 2, 1), (84, 2, 1), (85, 2, 1), (112, 2, 1), (113, 2, 1), (300, 3, 2), (1500, 5, 3)])
+@pytest.mark.parametrize("skew", [0.0, 3.0])
+def test_binned_experts_of_any_run_length(T, E, top, skew):
+    from krasis_b200.mixers import RoutedExperts
+    W, F = 192, 128
+    g = torch.Generator().manual_seed(T + E)
+    r = lambda *s, sd: (torch.randn(*s, generator=g) * sd).bfloat16()  # noqa: E731
+    w = {"router": r(E, W, sd=W ** -0.5)}
+    for e in range(E):
+        w.update({f"e{e}_gate": r(F, W, sd=W ** -0.5), f"e{e}_up": r(F, W, sd=W ** -0.5), f"e{e}_down": r(W, F, sd=F ** -0.5)})
+    bias = torch.zeros(E)
+    bias[0] = skew                                            # most rows choose expert 0; with many experts some get none
+    w["router_b"] = bias
+    h = r(T, W, sd=1.0).cuda()
+    mod = RoutedExperts(w, E, 0, top, torch.bfloat16, "cuda", score="softmax")
+    assert mod._tensor_core_ok(h, T * top)
+    ids, wts, _ = mod.route(h)
+    got = mod.forward(h).double().cpu()
+    x, want = h.double().cpu(), torch.zeros(T, W, dtype=torch.float64)
+    for e in range(E):
+        tok, j = torch.nonzero(ids.cpu() == e, as_tuple=True)
+        if tok.numel():
+            gu = [(x[tok] @ w[f"e{e}_{n}"].double().T).bfloat16().double() for n in ("gate", "up")]
+            a = (torch.nn.functional.silu(gu[0]) * gu[1]).bfloat16().double()
+            want.index_add_(0, tok, (a @ w[f"e{e}_down"].double().T) * wts.cpu()[tok, j].double()[:, None])
+    # the oracle rounds to bf16 where the kernels do; a gate, up or activation next to a rounding edge may fall on the other side: one
+    # bf16 step (2^-8) of a few of the F terms, well inside 2^-8 of the row's norm
+    assert ((got - want).norm(dim=1) <= 2.0 ** -8 * want.norm(dim=1) + 1e-6).all()
+
+
+def test_long_and_short_binning_agree():
+    """Steps of up to 8192 slots bin in one block, longer ones in three launches: the same tables but for the order inside a run."""
+    from krasis_b200.mixers import RoutedExperts
+    E = 37
+    mod = RoutedExperts({"router": torch.zeros(E, 64), **{f"e{e}_{n}": torch.zeros(64, 64) for e in range(E) for n in ("gate", "up", "down")}}, E, 0, 1,
+                        torch.bfloat16, "cuda")
+    g = torch.Generator(device="cuda").manual_seed(1)
+    for slots in (1, 8192, 8193, 20000):
+        ids = torch.randint(-1, E + 2, (slots,), device="cuda", generator=g, dtype=torch.int32)     # some slots name no expert
+        for tile in (16, 64, 128):
+            t = mod._bin(ids, slots, tile)
+            counts = torch.bincount(ids[(ids >= 0) & (ids < E)].long(), minlength=E)
+            tiles = (counts + tile - 1) // tile
+            n = int(tiles.sum())
+            assert int(t["n_tiles"][0]) == n and torch.equal(t["offs"].long(), torch.cat([tiles.new_zeros(1), tiles.cumsum(0)]) * tile)
+            assert torch.equal(t["tile_expert"][:n].long(), torch.arange(E, device="cuda").repeat_interleave(tiles))
+            rows = t["slot_row"][:n * tile].long()
+            real = rows >= 0
+            assert torch.equal(torch.sort(rows[real])[0], torch.nonzero((ids >= 0) & (ids < E)).flatten())
+            assert torch.equal(ids[rows[real]].long(), t["tile_expert"][:n].long().repeat_interleave(tile)[real])
+            assert torch.equal(t["pos"].long()[rows[real]], torch.nonzero(real).flatten()) and int((t["pos"] < 0).sum()) == slots - int(real.sum())
