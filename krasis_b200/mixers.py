@@ -95,6 +95,22 @@ def layer_runs(n: int, start: int = 0, stop: int = 0, times: int = 1):
             + [(i, False) for i in range(stop, n)])
 
 
+def portion_runs(tb, min_long):
+    """The step's rows as runs of neighbouring sequences of one kind: [(long, sequences, first row, rows)], long where every portion of the
+    run has at least min_long tokens (None: no portion counts as long)."""
+    runs, i = [], 0
+    kind = [min_long is not None and n >= min_long for _, n, _, _ in tb.layout]
+    while i < tb.S:
+        j = i
+        while j < tb.S and kind[j] == kind[i]:
+            j += 1
+        r0, rows = tb.layout[i][0], tb.layout[j - 1][0] + tb.layout[j - 1][1] - tb.layout[i][0]
+        if rows:
+            runs.append((kind[i], range(i, j), r0, rows))
+        i = j
+    return runs
+
+
 def yarn_table(dims: int, base: float, scaling):
     """Angular frequency of each rotated pair (fp64) and the amplitude both sin and cos carry.
     scaling = {factor, original, fast, slow} or None: pairs that turn more than `fast` times over `original` positions keep their
@@ -187,37 +203,38 @@ class WindowLatentAttention:
         ldg = proj_in.stride(0)
         o = torch.empty((T, H, self.dv), dtype=torch.float32 if gated else self.dtype, device=h.device)
         core = _core_lib() if self.tc_shape else False
-        fast = [i for i, (_, n, _, _) in enumerate(tb.layout) if n >= self.tc_min_portion] if core else []
-        if len(fast) < tb.S:
-            q_abs = torch.empty((T, H, self.r), dtype=torch.float32, device=h.device)
-            ops.gemm_heads(q[:, :, :self.dn], self.uk_t, q_abs)
-            o_lat = torch.empty((T, H, self.r), dtype=torch.float32, device=h.device)
-            # a step of few tokens (decoding) cuts each token's keys into pieces so that the whole GPU works on them
-            blocks = T * ((H + 7) // 8)
-            max_keys = max(min(self.window, start + n) for _, n, start, _ in tb.layout)
-            nsplit = max(1, min(296 // max(blocks, 1), (max_keys + 31) // 32, 64))
-            part_acc = torch.empty((T, nsplit, H, self.r), dtype=torch.float32, device=h.device) if nsplit > 1 else None
-            part_ml = torch.empty((T, nsplit, H, 2), dtype=torch.float32, device=h.device) if nsplit > 1 else None
-            ops.check(lib.kb2_seq_latent_window_attn(q_abs.data_ptr(), proj.data_ptr(), ldp, T, H, self.dn, self.dr, self.r, ckv.data_ptr(),
-                                                     kr.data_ptr(), dtc, tb.positions.data_ptr(), tb.seq_of.data_ptr(), tb.pages.data_ptr(),
-                                                     tb.max_pages, page_size, ops._ptr(self.sink), self.scale, self.window,
-                                                     o_lat.data_ptr(), tb.cu.data_ptr() if fast else None, self.tc_min_portion, nsplit,
-                                                     part_acc.data_ptr() if nsplit > 1 else None,
-                                                     part_ml.data_ptr() if nsplit > 1 else None, ops._ptr(hg), ldg, s))
-            ops.gemm_heads(o_lat, self.uv, o)
-        for i in fast:
+        for fast, seqs, r0, n in portion_runs(tb, self.tc_min_portion if core else None):
+            hgr = hg[r0:] if hg is not None else None
+            if not fast:
+                q_abs = torch.empty((n, H, self.r), dtype=torch.float32, device=h.device)
+                ops.gemm_heads(q[r0:r0 + n, :, :self.dn], self.uk_t, q_abs)
+                o_lat = torch.empty((n, H, self.r), dtype=torch.float32, device=h.device)
+                # few tokens (decoding): each token's keys are cut into pieces so that the whole GPU works on them
+                blocks = n * ((H + 7) // 8)
+                max_keys = max(min(self.window, tb.layout[i][2] + tb.layout[i][1]) for i in seqs)
+                nsplit = max(1, min(296 // max(blocks, 1), (max_keys + 31) // 32, 64))
+                part_acc = torch.empty((n, nsplit, H, self.r), dtype=torch.float32, device=h.device) if nsplit > 1 else None
+                part_ml = torch.empty((n, nsplit, H, 2), dtype=torch.float32, device=h.device) if nsplit > 1 else None
+                ops.check(lib.kb2_seq_latent_window_attn(q_abs.data_ptr(), proj[r0:].data_ptr(), ldp, n, H, self.dn, self.dr, self.r,
+                                                         ckv.data_ptr(), kr.data_ptr(), dtc, tb.positions[r0:].data_ptr(),
+                                                         tb.seq_of[r0:].data_ptr(), tb.pages.data_ptr(), tb.max_pages, page_size,
+                                                         ops._ptr(self.sink), self.scale, self.window, o_lat.data_ptr(), None,
+                                                         self.tc_min_portion, nsplit, ops._ptr(part_acc), ops._ptr(part_ml), ops._ptr(hgr), ldg, s))
+                ops.gemm_heads(o_lat, self.uv, o[r0:r0 + n])
+                continue
             from . import capi
-            row0, n, start, _ = tb.layout[i]
-            lo, rows = ops.key_rows(tb, i, self.window, page_size)
-            kv_up = lin(ckv.view(-1, self.r).index_select(0, rows), self.w_kv_up, torch.bfloat16)     # [keys, H * (128 + 128)]
-            kpe = kr.view(-1, self.dr).index_select(0, rows)
-            q_bf = proj[row0:row0 + n, :H * (self.dn + self.dr)].to(torch.bfloat16).contiguous()
-            o_rows = torch.empty((n, H, self.dv), dtype=torch.bfloat16, device=h.device) if gated else o[row0:row0 + n]
-            capi.check(core.kb2_fmha_latent_gated(q_bf.data_ptr(), kv_up.data_ptr(), kpe.data_ptr(), o_rows.data_ptr(), n, start - lo,
-                                                  start - lo + n, H, self.scale, min(self.window, 1 << 30), ops._ptr(self.sink),
-                                                  hg[row0:].data_ptr() if hg is not None else None, ldg, h.device.index or 0, s))
-            if gated:
-                o[row0:row0 + n].copy_(o_rows)
+            for i in seqs:
+                row0, n, start, _ = tb.layout[i]
+                lo, rows = ops.key_rows(tb, i, self.window, page_size)
+                kv_up = lin(ckv.view(-1, self.r).index_select(0, rows), self.w_kv_up, torch.bfloat16)     # [keys, H * (128 + 128)]
+                kpe = kr.view(-1, self.dr).index_select(0, rows)
+                q_bf = proj[row0:row0 + n, :H * (self.dn + self.dr)].to(torch.bfloat16).contiguous()
+                o_rows = torch.empty((n, H, self.dv), dtype=torch.bfloat16, device=h.device) if gated else o[row0:row0 + n]
+                capi.check(core.kb2_fmha_latent_gated(q_bf.data_ptr(), kv_up.data_ptr(), kpe.data_ptr(), o_rows.data_ptr(), n, start - lo,
+                                                      start - lo + n, H, self.scale, min(self.window, 1 << 30), ops._ptr(self.sink),
+                                                      hg[row0:].data_ptr() if hg is not None else None, ldg, h.device.index or 0, s))
+                if gated:
+                    o[row0:row0 + n].copy_(o_rows)
         if gated:
             o = ops.head_norm_gate(o.view(T, H * self.dv), H, self.dv, self.dtype, gate=proj_in[:, self.gate_off:], gate_act="sigmoid")
         return lin(o.view(T, H * self.dv), self.w_o, torch.float32)
@@ -794,47 +811,54 @@ class MultiMapAttention:
         if self.pool:                                # the tokens that complete a block write its mean key and value
             ops.check(lib.kb2_seq_kv_pool(kc.data_ptr(), vc.data_ptr(), kp.data_ptr(), vp.data_ptr(), dtc, G * M * self.d, G * self.dv, self.pool,
                                           T, tb.positions.data_ptr(), tb.seq_of.data_ptr(), tb.pages.data_ptr(), tb.max_pages, page_size, s))
-        # a step of few tokens (decoding) cuts each token's keys into pieces so that the whole GPU works on them
-        reach = min(self.window, self.chunk) if self.chunk else self.window
-        max_keys = max(min(reach, start + n) + ((start + n) // self.pool if self.pool else 0) for _, n, start, _ in tb.layout)
-        nsplit = max(1, min(296 // max(T * G, 1), (max_keys + 31) // 32, 64))
-        core = _core_lib() if self.tc_shape else False
-        fast = [i for i, (_, n, _, _) in enumerate(tb.layout) if n >= self.tc_min_portion] if core else []
-        if fast:
-            nsplit = 1
-        a = part_acc = part_ml = None
-        if nsplit > 1:
-            part_acc = torch.empty((T * H * M, nsplit, self.dv), dtype=torch.float32, device=h.device)
-            part_ml = torch.empty((T * H * M, nsplit, 2), dtype=torch.float32, device=h.device)
-            a = part_acc                                                     # unused by the kernels when the range is cut
-        else:
-            a = torch.empty((T, H, M, self.dv), dtype=torch.float32, device=h.device)
-        if len(fast) < tb.S:
-            ops.check(lib.kb2_seq_paged_attn(proj.data_ptr(), ldp, T, H, G, M, self.d, self.dv, kc.data_ptr(), vc.data_ptr(), dtc,
-                                             tb.positions.data_ptr(), tb.seq_of.data_ptr(), tb.pages.data_ptr(), tb.max_pages, page_size,
-                                             self.scale, self.chunk, min(self.window, 1 << 30), a.data_ptr(), nsplit, ops._ptr(part_acc),
-                                             ops._ptr(part_ml), tb.cu.data_ptr() if fast else None, self.tc_min_portion, self.softcap,
-                                             ops._ptr(self.sink), self.pool, ops._ptr(kp), ops._ptr(vp), 0, ops._ptr(self.slopes), s))
-        lse = torch.empty((T, H), dtype=torch.float32, device=h.device) if (fast and self.pool) else None
-        for i in fast:
-            self._tensor_core_portion(core, proj, a, tb, i, kc, vc, page_size, s, lse=lse)
-        if fast and self.pool:                       # the pooled blocks of the long portions: a second pass, joined by the log-sum-exps
-            p_acc = torch.empty((T * H, self.dv), dtype=torch.float32, device=h.device)
-            p_ml = torch.empty((T * H, 2), dtype=torch.float32, device=h.device)
-            ops.check(lib.kb2_seq_paged_attn(proj.data_ptr(), ldp, T, H, G, M, self.d, self.dv, kc.data_ptr(), vc.data_ptr(), dtc,
-                                             tb.positions.data_ptr(), tb.seq_of.data_ptr(), tb.pages.data_ptr(), tb.max_pages, page_size,
-                                             self.scale, 0, min(self.window, 1 << 30), a.data_ptr(), 1, p_acc.data_ptr(), p_ml.data_ptr(),
-                                             tb.cu.data_ptr(), self.tc_min_portion, self.softcap, None, self.pool, kp.data_ptr(),
-                                             vp.data_ptr(), 1, None, s))
-            ops.check(lib.kb2_seq_pool_merge(a.data_ptr(), lse.data_ptr(), p_acc.data_ptr(), p_ml.data_ptr(), T, H, self.dv,
-                                             tb.seq_of.data_ptr(), tb.cu.data_ptr(), self.tc_min_portion, s))
+        a = torch.empty((T, H, M, self.dv), dtype=torch.float32, device=h.device)
         o = torch.empty((T, H * self.dv), dtype=self.dtype, device=h.device)
         gate = proj_in[:, self.gate_off:] if self.gate_off >= 0 else None
-        ops.check(lib.kb2_seq_attn_finish(a.data_ptr(), ops._ptr(part_acc), ops._ptr(part_ml), nsplit, T, H, M, self.dv, ops._ptr(self.map_coef),
-                                          int(self.unit_norm), self.eps, self.post_scale, ops._ptr(gate), proj_in.stride(0), o.data_ptr(),
-                                          ops.dt_code(self.dtype), None, None, 0, int(self.gate_wide), tb.positions.data_ptr(),
-                                          ops._ptr(self.vfreq), int(self.rot_half), s))
+        core = _core_lib() if self.tc_shape else False
+        # long portions on the tensor cores, the others on the plain kernel with a key range of their own to cut (beside one portion of 512
+        # tokens, three decoded tokens at 2048 keys take 15 us instead of 230 uncut)
+        for fast, seqs, r0, rows in portion_runs(tb, self.tc_min_portion if core else None):
+            self._attend(core if fast else None, proj, a, o, gate, tb, seqs, r0, rows, kc, vc, kp, vp, page_size, s)
         return lin(o, self.w_o, torch.float32)
+
+    def _attend(self, core, proj, a, o, gate, tb, seqs, r0, T, kc, vc, kp, vp, page_size, s):
+        """Rows r0 .. r0 + T - 1 of the step (the sequences `seqs`): attention into a, the finished heads into o.  core: the library whose
+        tensor-core attention runs these portions, None for the plain kernel."""
+        lib, H, G, M, dtc, dev = ops.load(), self.H, self.G, self.M, ops.dt_code(kc.dtype), proj.device
+        positions, seq_of, window = tb.positions[r0:], tb.seq_of[r0:], min(self.window, 1 << 30)
+        nsplit, part_acc, part_ml = 1, None, None
+
+        def plain(out, acc, ml, pool_only):
+            ops.check(lib.kb2_seq_paged_attn(proj[r0:].data_ptr(), proj.stride(0), T, H, G, M, self.d, self.dv, kc.data_ptr(), vc.data_ptr(), dtc,
+                                             positions.data_ptr(), seq_of.data_ptr(), tb.pages.data_ptr(), tb.max_pages, page_size, self.scale,
+                                             0 if pool_only else self.chunk, window, out.data_ptr(), nsplit, ops._ptr(acc), ops._ptr(ml),
+                                             tb.cu.data_ptr() if pool_only else None,
+                                             self.tc_min_portion, self.softcap, None if pool_only else ops._ptr(self.sink), self.pool, ops._ptr(kp),
+                                             ops._ptr(vp), int(pool_only), None if pool_only else ops._ptr(self.slopes), s))
+        if core is None:
+            # few tokens (decoding): each token's keys are cut into pieces so that the whole GPU works on them
+            reach = min(self.window, self.chunk) if self.chunk else self.window
+            ends = [start + n for _, n, start, _ in (tb.layout[q] for q in seqs)]
+            max_keys = max(min(reach, e) + (e // self.pool if self.pool else 0) for e in ends)
+            nsplit = max(1, min(296 // max(T * G, 1), (max_keys + 31) // 32, 64))
+            if nsplit > 1:
+                part_acc = torch.empty((T * H * M, nsplit, self.dv), dtype=torch.float32, device=dev)
+                part_ml = torch.empty((T * H * M, nsplit, 2), dtype=torch.float32, device=dev)
+            plain(a[r0:], part_acc, part_ml, False)
+        else:
+            lse = torch.empty((proj.shape[0], H), dtype=torch.float32, device=dev) if self.pool else None
+            for q in seqs:
+                self._tensor_core_portion(core, proj, a, tb, q, kc, vc, page_size, s, lse=lse)
+            if self.pool:                            # the pooled blocks of the long portions: a second pass, joined by the log-sum-exps
+                p_acc = torch.empty((T * H, self.dv), dtype=torch.float32, device=dev)
+                p_ml = torch.empty((T * H, 2), dtype=torch.float32, device=dev)
+                plain(a[r0:], p_acc, p_ml, True)
+                ops.check(lib.kb2_seq_pool_merge(a[r0:].data_ptr(), lse[r0:].data_ptr(), p_acc.data_ptr(), p_ml.data_ptr(), T, H, self.dv,
+                                                 seq_of.data_ptr(), tb.cu.data_ptr(), self.tc_min_portion, s))
+        ops.check(lib.kb2_seq_attn_finish(a[r0:].data_ptr(), ops._ptr(part_acc), ops._ptr(part_ml), nsplit, T, H, M, self.dv, ops._ptr(self.map_coef),
+                                          int(self.unit_norm), self.eps, self.post_scale, ops._ptr(gate[r0:] if gate is not None else None),
+                                          gate.stride(0) if gate is not None else proj.stride(0), o[r0:].data_ptr(), ops.dt_code(self.dtype), None,
+                                          None, 0, int(self.gate_wide), positions.data_ptr(), ops._ptr(self.vfreq), int(self.rot_half), s))
 
 
 class RoutedExperts:
