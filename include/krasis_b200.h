@@ -232,6 +232,15 @@ KB2_API int kb2_linear_bf16_binned(const void* x_dev, const void* w_dev, void* o
                                    int32_t tile_rows, const int32_t* tile_group_dev, const int32_t* num_row_tiles_dev, int32_t groups,
                                    int32_t device, void* stream);
 
+/* Products of fp32 rows on the tensor cores with the accuracy of fp32 sums: out[g][m] = x[g][m] . w[g]^T for M rows in each of `groups` groups,
+ * x fp32 (row stride x_ld, group stride x_group), w [groups][N][K] fp32 (w_f32) or bf16, out fp32 or bf16 (row stride out_ld, group stride
+ * out_group, multiples of 4).  K % 64 == 0, N % 16 == 0.  The operands are cut into exact bf16 parts in workspace_dev
+ * (kb2_linear_f32_workspace bytes, 16-byte aligned; 0: sizes not taken). */
+KB2_API size_t kb2_linear_f32_workspace(int32_t M, int32_t N, int32_t K, int32_t w_f32, int32_t groups, int32_t device);
+KB2_API int kb2_linear_f32(const float* x_dev, int64_t x_ld, int64_t x_group, const void* w_dev, int32_t w_f32, void* out_dev, int32_t out_f32,
+                           int64_t out_ld, int64_t out_group, int32_t M, int32_t N, int32_t K, int32_t groups, void* workspace_dev,
+                           size_t workspace_bytes, int32_t device, void* stream);
+
 /* flashinfer.norm.rmsnorm (residual_dev == NULL) / fused_add_rmsnorm (residual_dev != NULL: residual += x, in place)
  * as used at python/krasis/layer.py:163-183,283-308.  x, residual, out: [M][H] bf16 (out may alias x); weight [H] f32. */
 KB2_API int kb2_rmsnorm(void* x_dev, void* residual_dev, const float* weight_dev, void* out_dev, int32_t M, int32_t H,

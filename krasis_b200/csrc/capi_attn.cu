@@ -1,5 +1,6 @@
 // C-ABI for the attention blocks that feed the MoE path (include/krasis_b200.h, "attention" section).
 // Host state mirrors python/krasis/linear_attention.py:GatedDeltaNetAttention (weights + conv/recurrent state).
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <string>
@@ -163,8 +164,66 @@ KB2_API int kb2_linear_bf16_binned(const void* x_dev, const void* w_dev, void* o
   if (M <= 0 || N <= 0 || K <= 0 || K % 64 || N % 16 || groups <= 0 || tile_rows < 16 || tile_rows > 128 || tile_rows % 16 || M % tile_rows)
     return failf(KB2_ERR_VALUE, "binned linear: need M>0, K %% 64 == 0, N %% 16 == 0, groups > 0, tiles of 16..128 rows that divide M (M=%d N=%d K=%d)", M, N, K);
   CUDA_TRY(cudaSetDevice(device));
-  CUDA_TRY(launch_split_gemm(x_dev, w_dev, out_dev, nullptr, M, N, K, N, out_f32 != 0, split_gemm_binned_plan(N, K, out_f32 != 0, tile_rows),
-                             tile_group_dev, num_row_tiles_dev, groups, (cudaStream_t)stream));
+  SplitGemm g;
+  g.x = x_dev; g.w = w_dev; g.out = out_dev;
+  g.M = M; g.N = N; g.K = K; g.ldo = N; g.out_f32 = out_f32 != 0;
+  g.groups = groups; g.tile_group = tile_group_dev; g.n_tiles_dev = num_row_tiles_dev;
+  CUDA_TRY(launch_split_gemm(g, split_gemm_binned_plan(N, K, out_f32 != 0, tile_rows), (cudaStream_t)stream));
+  return KB2_OK;
+}
+
+// The parts of fp32 weights are made and used a slice of columns at a time: the workspace stays bounded, and the parts stay in L2.
+constexpr size_t kWPartsBytes = 96u << 20;
+static int32_t linear_f32_columns(int32_t N, int32_t K, int32_t w_f32, int32_t groups) {
+  if (!w_f32 || groups > 1) return N;
+  const size_t most = kWPartsBytes / ((size_t)K * 6) / 128 * 128;
+  const int32_t slices = most >= 128 ? (int32_t)((N + most - 1) / most) : (N + 127) / 128;
+  return std::min(N, ((N + slices - 1) / slices + 127) / 128 * 128);
+}
+static bool linear_f32_plan(int32_t M, int32_t N, int32_t K, int32_t w_f32, int32_t groups, int32_t device, SplitPlan* plan) {
+  return M > 0 && N > 0 && K > 0 && K % 64 == 0 && N % 16 == 0 && groups > 0 &&
+         split_gemm_plan(M, N, K, true, device_sms(device), 3, w_f32 ? 3 : 1, groups, plan);
+}
+static size_t x_parts_bytes(const SplitPlan& plan, int32_t M, int32_t K, int32_t groups) {
+  return (size_t)groups * ((M + plan.mt - 1) / plan.mt) * plan.mt * 3 * K * 2;
+}
+
+KB2_API size_t kb2_linear_f32_workspace(int32_t M, int32_t N, int32_t K, int32_t w_f32, int32_t groups, int32_t device) {
+  SplitPlan plan;
+  if (M <= 0 || N <= 0 || K <= 0 || groups <= 0) return 0;
+  const int32_t cols = linear_f32_columns(N, K, w_f32, groups);
+  if (N % 16 || !linear_f32_plan(M, cols, K, w_f32, groups, device, &plan)) return 0;
+  return x_parts_bytes(plan, M, K, groups) + (w_f32 ? (size_t)groups * cols * 3 * K * 2 : 0);
+}
+
+KB2_API int kb2_linear_f32(const float* x_dev, int64_t x_ld, int64_t x_group, const void* w_dev, int32_t w_f32, void* out_dev, int32_t out_f32,
+                           int64_t out_ld, int64_t out_group, int32_t M, int32_t N, int32_t K, int32_t groups, void* workspace_dev,
+                           size_t workspace_bytes, int32_t device, void* stream) {
+  if (!x_dev || !w_dev || !out_dev || !workspace_dev) return failf(KB2_ERR_VALUE, "null argument");
+  const size_t need = kb2_linear_f32_workspace(M, N, K, w_f32, groups, device);
+  if (!need) return failf(KB2_ERR_VALUE, "fp32 linear: need M>0, K %% 64 == 0, N %% 16 == 0, groups > 0 (M=%d N=%d K=%d)", M, N, K);
+  if (workspace_bytes < need || ((uintptr_t)workspace_dev & 15) || ((uintptr_t)out_dev & 15) || (!w_f32 && ((uintptr_t)w_dev & 15)) ||
+      out_ld % 4 || out_group % 4)
+    return failf(KB2_ERR_VALUE, "fp32 linear: workspace of %zu bytes, 16-byte aligned pointers and output strides that are multiples of 4", need);
+  CUDA_TRY(cudaSetDevice(device));
+  cudaStream_t s = (cudaStream_t)stream;
+  const int32_t cols = linear_f32_columns(N, K, w_f32, groups);
+  SplitPlan plan;                       // one plan for all slices: the row tiles of the parts follow it
+  linear_f32_plan(M, cols, K, w_f32, groups, device, &plan);
+  char* wparts = (char*)workspace_dev + x_parts_bytes(plan, M, K, groups);
+  CUDA_TRY(launch_split_parts(x_dev, x_ld, x_group, M, K, plan.mt, groups, workspace_dev, s));
+  for (int32_t n0 = 0; n0 < N; n0 += cols) {
+    SplitGemm g;
+    g.N = std::min(cols, N - n0);
+    if (w_f32) CUDA_TRY(launch_split_parts((const float*)w_dev + (size_t)n0 * K, K, 0, groups * g.N, K, groups * g.N, 1, wparts, s));
+    g.x = workspace_dev; g.w = w_f32 ? wparts : w_dev;
+    g.out = (char*)out_dev + (size_t)n0 * (out_f32 ? 4 : 2);
+    g.M = M; g.K = K; g.ldo = out_ld; g.out_f32 = out_f32 != 0;
+    g.xparts = 3; g.wparts = w_f32 ? 3 : 1; g.groups = groups; g.batched = true; g.out_group = out_group;
+    g.x_raw = x_dev; g.x_ld = x_ld; g.x_group = x_group;
+    g.w_raw = w_f32 ? (const void*)((const float*)w_dev + (size_t)n0 * K) : w_dev;
+    CUDA_TRY(launch_split_gemm(g, plan, s));
+  }
   return KB2_OK;
 }
 

@@ -222,8 +222,12 @@ cudaError_t launch_dense_gemm_scatter(const void* x, const void* w, void* out, c
   if (sc.n_ranks > 0 && (out_f32 || M % sc.n_ranks || sc.rows_per_rank * sc.n_ranks != M)) return cudaErrorInvalidValue;
   if (K % kBlockK || N % 16 || M <= 0) return cudaErrorInvalidValue;
   SplitPlan plan;
-  if (sc.n_ranks == 0 && split_gemm_plan(M, N, K, out_f32, num_sms, &plan))
-    return launch_split_gemm(x, w, out, bias, M, N, K, ldo, out_f32, plan, nullptr, nullptr, 1, s);
+  if (sc.n_ranks == 0 && split_gemm_plan(M, N, K, out_f32, num_sms, 1, 1, 1, &plan)) {
+    SplitGemm g;
+    g.x = x; g.w = w; g.out = out; g.bias = bias;
+    g.M = M; g.N = N; g.K = K; g.ldo = ldo; g.out_f32 = out_f32;
+    return launch_split_gemm(g, plan, s);
+  }
   KernelSpan ks(K_DENSE_BF16, s);
   alignas(64) CUtensorMap tx, tw;
   cudaError_t e = make_tmap_bf16_rows(&tx, x, M, K, 128);

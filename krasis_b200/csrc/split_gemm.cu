@@ -1,14 +1,21 @@
-// Dense BF16 product for few rows:  Y[M,N] = X[M,K] (bf16) x W[N,K]^T (bf16), fp32 accumulation in TMEM, BF16 or FP32 output.
+// Dense product for few rows:  Y[M,N] = X[M,K] x W[N,K]^T with bf16 operands, fp32 accumulation in TMEM, BF16 or FP32 output; and the same for
+// fp32 operands, as exact bf16 parts.
 //
 // Bound: the weights.  Up to a few hundred rows the time is N * K * 2 bytes from HBM, and dense_gemm.cu's 128 x 256 tiles leave most SMs
 // without a tile (N = 2048: 8 tiles per 128 rows).  So the roles of the operands are swapped — 128 weight rows are the UMMA's M side, the
 // rows of X (any multiple of 16 up to 256) its N side, which costs no padding to 128 rows — and K is cut over the CTAs of a cluster
 // (1, 2, 4 or 8).  A CTA has one tile: its TMA ring streams the weights while two CTAs share an SM, so that one fills its ring while the
 // other drains.  The partial tiles of a cluster meet in shared memory (one [row][128] fp32 image per CTA, read through distributed shared
-// memory); every output is summed in rank order, so a result does not depend on timing.
+// memory); every output is summed in rank order, so a result does not depend on timing.  From HBM, 77 rows: N 16384, K 2048 15.0 us (11.1 us
+// of traffic), N 2048, K 8192 12.6 us (5.4 us), where fp32-FMA tiles took 697 and 449 us.
 //
 // Grouped form: row tile i of X multiplies matrix tile_group[i] (routed experts on binned rows); only the first n_tiles_dev[0] row tiles
-// exist, the CTAs of the others return at once.
+// exist, the CTAs of the others return at once.  Batched form: group g has M rows and a matrix of its own (per-head products).
+//
+// fp32 operands: x = x1 + x2 + x3 with bf16 parts of 8 bits each, exactly.  The parts of a tile's rows lie side by side on the N side, so one
+// weight tile serves all of them: w x1 goes to the main accumulators, w x2 and w x3 to two small ones.  With fp32 weights in three parts
+// too, w1 [x1 x2 x3], w2 [x1 x2] and w3 [x1] are added in: six of the nine products, the other three are below 2^-26 of the result.  512 rows,
+// N 16384, K 2048: 231 us, 2-norm error 4.7e-7; fp32-FMA tiles 1494 us, 8.1e-7.
 #include <cuda.h>
 
 #include <algorithm>
@@ -28,10 +35,13 @@ constexpr int kSMaxStages = 12;
 struct SplitArgs {
   void* out;
   const float* bias;
-  long long ldo;
-  int M, N, n_kblocks, nt, stages, chunk, tmem_cols;
+  long long ldo, out_group, w_part_rows;
+  int M, N, n_kblocks, mt, xparts, wparts, stages, chunk, tmem_cols, tiles_per_group;
   const int* tile_group;
   const int* n_tiles_dev;
+  const float* x_raw;
+  long long x_ld, x_group;
+  const void* w_raw;
 };
 
 __device__ __forceinline__ void cluster_sync_all() {
@@ -46,6 +56,14 @@ __device__ __forceinline__ float4 ld_dsmem_f4(uint32_t local_addr, uint32_t rank
   return v;
 }
 
+// One output from the fp32 operands themselves (see SplitGemm::x_raw).
+__device__ __noinline__ float product_again(const float* x, const void* w, long long w0, bool w_f32, int K) {
+  float acc = 0.f;
+  for (int k = 0; k < K; ++k)
+    acc = fmaf(x[k], w_f32 ? reinterpret_cast<const float*>(w)[w0 + k] : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(w)[w0 + k]), acc);
+  return acc;
+}
+
 // KS CTAs of a cluster share one output tile along K.
 template <bool kOutF32, int KS>
 __global__ void __launch_bounds__(kSThreads)
@@ -53,14 +71,16 @@ __global__ void __launch_bounds__(kSThreads)
   extern __shared__ __align__(1024) uint8_t smem[];
   const int row_tile = blockIdx.x / KS, rank = blockIdx.x % KS;
   if (p.n_tiles_dev != nullptr && row_tile >= p.n_tiles_dev[0]) return;      // the same decision in every CTA of the cluster
-  const int stage_bytes = kSWBytes + p.nt * 128;
+  const int nt = p.xparts * p.mt, w_bytes = p.wparts * kSWBytes, stage_bytes = w_bytes + nt * 128;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + p.stages * stage_bytes);
   uint64_t* empty = full + kSMaxStages;
   uint64_t* done = empty + kSMaxStages;
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(done + 1);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int m0 = row_tile * p.nt, n0 = blockIdx.y * kSRows;
-  const int w0 = n0 + (p.tile_group != nullptr ? p.tile_group[row_tile] * p.N : 0);        // row of W
+  const int n0 = blockIdx.y * kSRows;
+  const int group = p.tile_group != nullptr ? p.tile_group[row_tile] : p.tiles_per_group > 0 ? row_tile / p.tiles_per_group : 0;
+  const int m0 = (p.tiles_per_group > 0 ? row_tile % p.tiles_per_group : row_tile) * p.mt;     // row of the output (of its group)
+  const int w0 = n0 + group * p.N;                                                             // row of W
   const int kb0 = (int)((long long)p.n_kblocks * rank / KS), kb1 = (int)((long long)p.n_kblocks * (rank + 1) / KS);
 
   if (threadIdx.x == 32) {
@@ -90,8 +110,8 @@ __global__ void __launch_bounds__(kSThreads)
       uint8_t* a = smem + stage * stage_bytes;
       if (elect_one()) {
         mbar_arrive_expect_tx(&full[stage], stage_bytes);
-        tma_load_2d(a, &tmap_w, kb * kBlockK, w0, &full[stage]);
-        tma_load_2d(a + kSWBytes, &tmap_x, kb * kBlockK, m0, &full[stage]);
+        for (int q = 0; q < p.wparts; ++q) tma_load_2d(a + q * kSWBytes, &tmap_w, kb * kBlockK, w0 + (int)(q * p.w_part_rows), &full[stage]);
+        tma_load_2d(a + w_bytes, &tmap_x, kb * kBlockK, row_tile * nt, &full[stage]);
       }
       __syncwarp();
       if (++stage == p.stages) { stage = 0; phase ^= 1; }
@@ -99,22 +119,35 @@ __global__ void __launch_bounds__(kSThreads)
   } else if (warp == 1) {
     int stage = 0;
     uint32_t phase = 0;
-    const uint32_t idesc = umma_idesc_bf16_m128(p.nt);
-    uint32_t acc = tmem_base;
+    const uint32_t idesc1 = umma_idesc_bf16_m128(p.mt), idesc2 = umma_idesc_bf16_m128(2 * p.mt);
+    const uint32_t small = tmem_base;                                        // w x2, w x3 and what the further parts of w bring
+    uint32_t acc = tmem_base + (p.xparts > 1 ? 2 * p.mt : 0);                // w x1, a set of columns per chunk
     int in_chunk = 0;
     for (int kb = kb0; kb < kb1; ++kb) {
       mbar_wait(&full[stage], phase);
       tc_fence_after_sync();
       const uint32_t a_addr = smem_u32(smem + stage * stage_bytes);
       const uint64_t ad = umma_desc_k_sw128(a_addr);
-      const uint64_t bd = umma_desc_k_sw128(a_addr + kSWBytes);
+      const uint64_t bd = umma_desc_k_sw128(a_addr + w_bytes);               // x1; x2 and x3 follow mt rows apart
       if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) umma_bf16(acc, ad + 2 * k, bd + 2 * k, idesc, (in_chunk > 0 || k > 0) ? 1u : 0u);
+        for (int k = 0; k < 4; ++k) umma_bf16(acc, ad + 2 * k, bd + 2 * k, idesc1, (in_chunk > 0 || k > 0) ? 1u : 0u);
+        if (p.xparts > 1) {
+          const uint64_t bd2 = umma_desc_k_sw128(a_addr + w_bytes + p.mt * 128);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_bf16(small, ad + 2 * k, bd2 + 2 * k, idesc2, (kb > kb0 || k > 0) ? 1u : 0u);
+          if (p.wparts > 1) {
+            const uint64_t ad2 = umma_desc_k_sw128(a_addr + kSWBytes), ad3 = umma_desc_k_sw128(a_addr + 2 * kSWBytes);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) umma_bf16(small, ad2 + 2 * k, bd + 2 * k, idesc2, 1u);             // w2 [x1 x2]
+#pragma unroll
+            for (int k = 0; k < 4; ++k) umma_bf16(small + p.mt, ad3 + 2 * k, bd + 2 * k, idesc1, 1u);      // w3 x1
+          }
+        }
         umma_commit(&empty[stage]);
       }
       __syncwarp();
-      if (++in_chunk == p.chunk) { in_chunk = 0; acc += p.nt; }
+      if (++in_chunk == p.chunk) { in_chunk = 0; acc += p.mt; }
       if (++stage == p.stages) { stage = 0; phase ^= 1; }
     }
     if (elect_one()) umma_commit(done);
@@ -123,18 +156,18 @@ __global__ void __launch_bounds__(kSThreads)
   __syncwarp();
   mbar_wait(done, 0);                              // every load has been consumed: the ring's memory is free
   tc_fence_after_sync();
-  float* part = reinterpret_cast<float*>(smem);    // [nt][128]
+  float* part = reinterpret_cast<float*>(smem);    // [mt][128]
   const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16);
-  const int n_acc = (kb1 - kb0 + p.chunk - 1) / p.chunk;
-  for (int c0 = 0; c0 < p.nt; c0 += 16) {
+  const int n_sets = (kb1 - kb0 + p.chunk - 1) / p.chunk + (p.xparts > 1 ? 2 : 0);      // the small ones come first
+  for (int c0 = 0; c0 < p.mt; c0 += 16) {
     float v[16];
     uint32_t r[16];
     tmem_ld16(taddr + c0, r);
     tmem_ld_wait();
 #pragma unroll
     for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
-    for (int a = 1; a < n_acc; ++a) {
-      tmem_ld16(taddr + a * p.nt + c0, r);
+    for (int a = 1; a < n_sets; ++a) {
+      tmem_ld16(taddr + a * p.mt + c0, r);
       tmem_ld_wait();
 #pragma unroll
       for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(r[j]);
@@ -149,7 +182,8 @@ __global__ void __launch_bounds__(kSThreads)
   if (n < p.N) {                                   // N % 16 == 0 is required by the launcher
     float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
     if (p.bias != nullptr) b = make_float4(p.bias[n], p.bias[n + 1], p.bias[n + 2], p.bias[n + 3]);
-    const int rows = min(p.nt, p.M - m0);
+    const int rows = min(p.mt, p.M - m0);
+    const long long out0 = group * p.out_group + (long long)m0 * p.ldo + n;
 #pragma unroll 2
     for (int c = rank + KS * warp; c < rows; c += KS * 4) {
       const uint32_t at = smem_u32(part + c * kSRows + lane * 4);
@@ -162,14 +196,23 @@ __global__ void __launch_bounds__(kSThreads)
       float4 s = v[0];
 #pragma unroll
       for (int i = 1; i < KS; ++i) { s.x += v[i].x; s.y += v[i].y; s.z += v[i].z; s.w += v[i].w; }
+      if (p.x_raw != nullptr && (isnan(s.x) || isnan(s.y) || isnan(s.z) || isnan(s.w))) {
+        const float* xr = p.x_raw + group * p.x_group + (long long)(m0 + c) * p.x_ld;
+        const int K = p.n_kblocks * kBlockK;
+        const long long wr = ((long long)group * p.N + n) * K;
+        s.x = product_again(xr, p.w_raw, wr, p.wparts > 1, K);
+        s.y = product_again(xr, p.w_raw, wr + K, p.wparts > 1, K);
+        s.z = product_again(xr, p.w_raw, wr + 2 * K, p.wparts > 1, K);
+        s.w = product_again(xr, p.w_raw, wr + 3 * K, p.wparts > 1, K);
+      }
       s.x += b.x; s.y += b.y; s.z += b.z; s.w += b.w;
       if constexpr (kOutF32) {
-        *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + (long long)(m0 + c) * p.ldo + n) = s;
+        *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + out0 + c * p.ldo) = s;
       } else {
         uint2 o;
         o.x = bf16x2_bits_rn(s.y, s.x);
         o.y = bf16x2_bits_rn(s.w, s.z);
-        *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + (long long)(m0 + c) * p.ldo + n) = o;
+        *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + out0 + c * p.ldo) = o;
       }
     }
   }
@@ -205,12 +248,12 @@ static cudaError_t launch_one_split(const CUtensorMap& tx, const CUtensorMap& tw
 
 static int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
-// Depth of the ring: two CTAs share an SM where there are more tiles than SMs and the tile is narrow enough for four stages in half the
-// shared memory (nt <= 64); wider tiles run faster alone with a deep ring (N 16384, K 2048, 256 rows in tiles of 128: 25 us with seven
-// stages, 32 us with two CTAs of three).
-static int ring_stages(int nt, int kb, bool share) {
-  const int stage = kSWBytes + nt * 128, room = (share && nt <= 64 ? 113 : 226) * 1024 - 256;
-  return std::max(std::min({kSMaxStages, room / stage, kb}), ceil_div((long long)nt * kSRows * 4, stage));
+// Depth of the ring: two CTAs share an SM where there are more tiles than SMs and a stage is small enough for four of them in half the
+// shared memory; larger tiles run faster alone with a deep ring (N 16384, K 2048, 256 rows in tiles of 128: 25 us with seven stages,
+// 32 us with two CTAs of three).
+static int ring_stages(int stage, int mt, int kb, bool share) {
+  const int room = (share && 4 * stage <= 112 * 1024 ? 113 : 226) * 1024 - 256;
+  return std::max(std::min({kSMaxStages, room / stage, kb}), ceil_div((long long)mt * kSRows * 4, stage));
 }
 
 // The plan with the least estimated time (us), and whether that beats the 128 x 256 tiles of dense_gemm.cu.  Constants fitted to 700
@@ -218,34 +261,39 @@ static int ring_stages(int nt, int kb, bool share) {
 // 190 KB/us, HBM 5.76 MB/us, a 64-wide K block costs 0.135 us of latency at least, reading out a row 0.05 us + 1.2 ns per accumulator, a
 // launch 1.9 us.  The 128 x 256 tiles take 0.355 us per K block and 5 us around it.  Measured on both sides of the line: M 1000, N 2048, K 2048
 // 12.1 against 18.3 us; M 2048 at the same shape 23.2 against 18.7; M 256, N 12352 21.7 against 23.0; M 515 39.5 against 39.0.
-bool split_gemm_plan(int M, int N, int K, bool out_f32, int num_sms, SplitPlan* out) {
-  if (M > 2048 || K % kBlockK || N % 16) return false;
-  const int nkb = K / kBlockK, nb = ceil_div(N, kSRows);
+bool split_gemm_plan(int M, int N, int K, bool out_f32, int num_sms, int xparts, int wparts, int groups, SplitPlan* out) {
+  const bool plain = xparts == 1 && wparts == 1 && groups == 1;
+  if (K % kBlockK || N % 16 || (plain && M > 2048)) return false;
+  const int nkb = K / kBlockK, nb = ceil_div(N, kSRows), most = 256 / xparts / 16 * 16;
   static const float kShare[4] = {0.f, 0.45f, 0.55f, 1.0f};
-  float best = 0.355f * nkb * ceil_div((long long)ceil_div(M, 128) * ceil_div(N, 256), num_sms) + 5.f;
+  float best = plain ? 0.355f * nkb * ceil_div((long long)ceil_div(M, 128) * ceil_div(N, 256), num_sms) + 5.f : 1e30f;
   bool found = false;
-  int last_nt = 0;
-  for (int t = ceil_div(M, 256), tries = 0; tries < 8; ++t, ++tries) {
-    const int nt = ceil_div(ceil_div(M, t), 16) * 16;
-    if (nt == last_nt || (nt < 32 && M > 32)) continue;
-    last_nt = nt;
+  int last = 0;
+  for (int t = ceil_div(M, most), tries = 0; tries < 8; ++t, ++tries) {
+    const int mt = ceil_div(ceil_div(M, t), 16) * 16;
+    if (mt == last || (mt < 32 && M > 32 && xparts == 1)) continue;
+    last = mt;
     for (int i = 0; i < 4; ++i) {
       const int ks = 1 << i;
       if (ks > 1 && nkb < 2 * ks) break;
-      const int kb = ceil_div(nkb, ks), n_acc = out_f32 ? ceil_div(kb, kSplitChunk) : 1;
-      if (n_acc * nt > 512) continue;
-      const long long ctas = (long long)ceil_div(M, nt) * nb * ks;
-      const int per_sm = ceil_div(ctas, num_sms);
-      const float load = (float)per_sm * kb * (kSWBytes + 128 * nt) / 190e3f, hbm = (float)N * K * 2.f / 5.76e6f;
-      const float time = std::max({load, hbm, 0.135f * kb}) + nt * (0.05f + 0.0012f * n_acc) * ceil_div(per_sm, 2) +
+      const int kb = ceil_div(nkb, ks);
+      const int chunk = !out_f32 && xparts == 1 ? kb : nkb <= kSplitChunk ? kSplitChunkShort : kSplitChunk;
+      const int sets = ceil_div(kb, chunk) + (xparts > 1 ? 2 : 0);
+      const int stage = wparts * kSWBytes + xparts * mt * 128;
+      if (sets * mt > 512 || ceil_div((long long)mt * kSRows * 4, stage) * stage > 226 * 1024 - 256) continue;
+      const long long ctas = (long long)ceil_div(M, mt) * groups * nb * ks;
+      const int per_sm = ceil_div(ctas, num_sms), cols = mt * (xparts == 1 ? 1 : wparts == 1 ? 3 : 6);
+      const float load = (float)per_sm * kb * stage / 190e3f, math = (float)per_sm * kb * cols * (2.f / 1700.f);
+      const float hbm = (float)N * K * 2.f * wparts * groups / 5.76e6f;
+      const float time = std::max({load, math, hbm, 0.135f * kb}) + mt * (0.05f + 0.0012f * sets) * ceil_div(per_sm, 2) +
                          kShare[i] * ceil_div(per_sm, 2) + 1.9f;
       if (time >= best) continue;
       best = time;
       found = true;
-      out->nt = nt;
+      out->mt = mt;
       out->ks = ks;
-      out->stages = ring_stages(nt, kb, ctas > num_sms);
-      out->chunk = out_f32 ? kSplitChunk : kb;
+      out->chunk = chunk;
+      out->stages = ring_stages(stage, mt, kb, ctas > num_sms);
     }
   }
   return found;
@@ -253,49 +301,61 @@ bool split_gemm_plan(int M, int N, int K, bool out_f32, int num_sms, SplitPlan* 
 
 SplitPlan split_gemm_binned_plan(int N, int K, bool out_f32, int tile_rows) {
   SplitPlan p;
-  p.nt = tile_rows;
+  p.mt = tile_rows;
   int n_acc = out_f32 ? ceil_div(K / kBlockK, kSplitChunk) : 1;
   while (n_acc > 1 && n_acc * tile_rows > 256) n_acc = ceil_div(n_acc, 2);         // half of the tensor memory, so that two CTAs share an SM
   p.chunk = ceil_div(K / kBlockK, n_acc);
-  p.stages = ring_stages(tile_rows, K / kBlockK, true);
+  p.stages = ring_stages(kSWBytes + tile_rows * 128, tile_rows, K / kBlockK, true);
   return p;
 }
 
-cudaError_t launch_split_gemm(const void* x, const void* w, void* out, const float* bias, int M, int N, int K, long long ldo, bool out_f32,
-                              const SplitPlan& plan, const int* tile_group, const int* n_tiles_dev, int groups, cudaStream_t s) {
+cudaError_t launch_split_gemm(const SplitGemm& g, const SplitPlan& plan, cudaStream_t s) {
   KernelSpan span(K_DENSE_BF16, s);
-  if (K % kBlockK || N % 16 || M <= 0 || plan.nt < 16 || plan.nt > 256 || plan.nt % 16 || K / kBlockK < plan.ks) return cudaErrorInvalidValue;
+  const int nkb = g.K / kBlockK, nt = g.xparts * plan.mt;
+  if (g.K % kBlockK || g.N % 16 || g.M <= 0 || g.groups <= 0 || plan.mt < 16 || nt > 256 || plan.mt % 16 || plan.ks < 1 || nkb < plan.ks ||
+      plan.chunk < 1 || (g.xparts != 1 && g.xparts != 3) || (g.wparts != 1 && g.wparts != g.xparts))
+    return cudaErrorInvalidValue;
+  const int tiles = ceil_div(g.M, plan.mt), row_tiles = g.batched ? tiles * g.groups : tiles;
   alignas(64) CUtensorMap tx, tw;
-  cudaError_t e = make_tmap_bf16_rows(&tx, x, M, K, plan.nt);
+  // three parts: whole tiles of zero-padded rows; else the caller's M rows (rows beyond them read as zeros)
+  cudaError_t e = make_tmap_bf16_rows(&tx, g.x, g.xparts > 1 ? (long long)row_tiles * nt : (long long)g.M, g.K, nt);
   if (e != cudaSuccess) return e;
-  e = make_tmap_bf16_rows(&tw, w, (long long)groups * N, K, kSRows);
+  e = make_tmap_bf16_rows(&tw, g.w, (long long)g.wparts * g.groups * g.N, g.K, kSRows);
   if (e != cudaSuccess) return e;
   SplitArgs p{};
-  p.out = out;
-  p.bias = bias;
-  p.ldo = ldo;
-  p.M = M;
-  p.N = N;
-  p.n_kblocks = K / kBlockK;
-  p.nt = plan.nt;
+  p.out = g.out;
+  p.bias = g.bias;
+  p.ldo = g.ldo;
+  p.out_group = g.batched ? g.out_group : 0;
+  p.w_part_rows = (long long)g.groups * g.N;
+  p.M = g.M;
+  p.N = g.N;
+  p.n_kblocks = nkb;
+  p.mt = plan.mt;
+  p.xparts = g.xparts;
+  p.wparts = g.wparts;
   p.stages = plan.stages;
   p.chunk = plan.chunk;
-  const int n_acc = plan.chunk > 0 ? ((p.n_kblocks + plan.ks - 1) / plan.ks + plan.chunk - 1) / plan.chunk : 0;
+  const int sets = ceil_div(ceil_div(nkb, plan.ks), plan.chunk) + (g.xparts > 1 ? 2 : 0);
   p.tmem_cols = 32;
-  while (p.tmem_cols < n_acc * plan.nt) p.tmem_cols *= 2;
-  if (n_acc < 1 || p.tmem_cols > 512) return cudaErrorInvalidValue;
-  p.tile_group = tile_group;
-  p.n_tiles_dev = n_tiles_dev;
-  const int ring = plan.stages * (kSWBytes + plan.nt * 128);
+  while (p.tmem_cols < sets * plan.mt) p.tmem_cols *= 2;
+  if (p.tmem_cols > 512) return cudaErrorInvalidValue;
+  p.tiles_per_group = g.batched ? tiles : 0;
+  p.tile_group = g.tile_group;
+  p.n_tiles_dev = g.n_tiles_dev;
+  p.x_raw = g.xparts > 1 ? g.x_raw : nullptr;
+  p.x_ld = g.x_ld;
+  p.x_group = g.x_group;
+  p.w_raw = g.w_raw;
+  const int ring = plan.stages * (g.wparts * kSWBytes + nt * 128);
   // a CTA that waits for tensor memory may have cluster peers that others wait for in turn, so co-resident CTAs must never ask for more
   // than the 512 columns together: each takes at least 430 bytes of shared memory per column (1 KB of it is the system's); of 228 KB that
   // leaves fewer than 544 columns, and columns come in multiples of 32
   const int smem = std::max(ring + 2 * kSMaxStages * 8 + 16, p.tmem_cols * 430 - 1024);
-  if (plan.stages < 1 || plan.stages > kSMaxStages || ring < plan.nt * kSRows * 4 || smem > 227 * 1024) return cudaErrorInvalidValue;
-  const int row_tiles = (M + plan.nt - 1) / plan.nt;
-  const dim3 grid(row_tiles * plan.ks, (N + kSRows - 1) / kSRows);
+  if (plan.stages < 1 || plan.stages > kSMaxStages || ring < plan.mt * kSRows * 4 || smem > 227 * 1024) return cudaErrorInvalidValue;
+  const dim3 grid(row_tiles * plan.ks, (g.N + kSRows - 1) / kSRows);
 #define KB2_SPLIT(KSV)                                                                  \
-  (out_f32 ? launch_one_split<true, KSV>(tx, tw, p, grid, smem, s) : launch_one_split<false, KSV>(tx, tw, p, grid, smem, s))
+  (g.out_f32 ? launch_one_split<true, KSV>(tx, tw, p, grid, smem, s) : launch_one_split<false, KSV>(tx, tw, p, grid, smem, s))
   switch (plan.ks) {
     case 1: return KB2_SPLIT(1);
     case 2: return KB2_SPLIT(2);
@@ -304,6 +364,68 @@ cudaError_t launch_split_gemm(const void* x, const void* w, void* out, const flo
     default: return cudaErrorInvalidValue;
   }
 #undef KB2_SPLIT
+}
+
+// ------------------------------------------------------------------------------------------------ fp32 -> three bf16 parts
+// hi = bf16(v), mid = bf16(v - hi), lo = v - hi - mid: nearest rounding leaves 9 + 9 bits behind, so 24 bits are carried exactly (a value next
+// to the largest fp32 number is truncated instead of rounded to infinity; what is not finite goes into hi alone).  bf16 numbers end at 2^-133: below 1e-33 the low parts miss up to 2^-134.
+__device__ __forceinline__ void split3(float v, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  const uint32_t bits = __float_as_uint(v), e = bits & 0x7F800000u;
+  hi = bf16_bits_rn(v);
+  if (e != 0x7F800000u && (hi & 0x7F80u) == 0x7F80u) hi = bits >> 16;
+  float r = v - __uint_as_float(hi << 16);
+  if (e == 0x7F800000u) r = 0.f;
+  mid = bf16_bits_rn(r);
+  lo = bf16_bits_rn(r - __uint_as_float(mid << 16));
+}
+
+// Bound by traffic (4 bytes in, 6 out); a thread takes eight neighbouring columns.
+template <bool kVec>
+__global__ void __launch_bounds__(256) split_parts_kernel(const float* __restrict__ x, long long ld, long long group_stride, int rows, int K, int mt,
+                                                          int tiles, long long total, __nv_bfloat16* __restrict__ parts) {
+  const int k8 = K >> 3;
+  for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
+    const long long r = i / k8;                      // row of the padded [groups][tiles][mt] order
+    const int c = (int)(i - r * k8) * 8;
+    const long long tile = r / mt;
+    const int in = (int)(r - tile * mt), group = (int)(tile / tiles), row = (int)(tile - (long long)group * tiles) * mt + in;
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = 0.f;
+    if (row < rows) {
+      const float* src = x + group * group_stride + (long long)row * ld + c;
+      if constexpr (kVec) {
+        const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = src[j];
+      }
+    }
+    uint32_t o[3][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      uint32_t a[3], b[3];
+      split3(v[2 * j], a[0], a[1], a[2]);
+      split3(v[2 * j + 1], b[0], b[1], b[2]);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) o[q][j] = a[q] | (b[q] << 16);
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      *reinterpret_cast<uint4*>(parts + ((tile * 3 + q) * mt + in) * K + c) = make_uint4(o[q][0], o[q][1], o[q][2], o[q][3]);
+  }
+}
+
+cudaError_t launch_split_parts(const float* x, long long ld, long long group_stride, int rows, int K, int mt, int groups, void* parts, cudaStream_t s) {
+  KernelSpan span(K_DENSE_BF16, s);
+  const int tiles = ceil_div(rows, mt);
+  const long long total = (long long)groups * tiles * mt * (K / 8);
+  const unsigned blocks = (unsigned)std::min<long long>((total + 255) / 256, 148 * 16);
+  const bool vec = !((uintptr_t)x & 15) && ld % 4 == 0 && group_stride % 4 == 0;
+  if (vec) split_parts_kernel<true><<<blocks, 256, 0, s>>>(x, ld, group_stride, rows, K, mt, tiles, total, (__nv_bfloat16*)parts);
+  else split_parts_kernel<false><<<blocks, 256, 0, s>>>(x, ld, group_stride, rows, K, mt, tiles, total, (__nv_bfloat16*)parts);
+  return cudaGetLastError();
 }
 
 }  // namespace kb2

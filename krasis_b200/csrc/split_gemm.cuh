@@ -1,28 +1,53 @@
-// Host side of split_gemm.cu: how a product with few rows is cut.
+// Host side of split_gemm.cu: how a product with few rows, or with fp32 operands, is cut.
 #pragma once
 #include <cuda_runtime.h>
 
 namespace kb2 {
 
 // 64-wide K blocks per accumulator of an fp32 result.  The tensor core truncates when it adds to an accumulator: the error of a sum grows by
-// 1.0e-9 per K (2.1e-6 at K = 2048, 4.4e-6 at 4096, in the 2-norm).  Sums of 512 products meet in fp32 round-to-nearest instead: 4.8e-7 at
-// any K measured, what sequential fp32 FMAs have.
-constexpr int kSplitChunk = 8;
+// 9.3e-10 per K (2.1e-6 at K = 2048, 4.4e-6 at 4096, in the 2-norm).  Sums of 512 products meet in fp32 round-to-nearest instead: 4.8e-7 at
+// any K measured, where sequential fp32 FMAs are 8.1e-7 off at K = 2048 and 1.6e-6 at 8192.  Up to K = 512, where those are 2.0e-7 (K 128)
+// to 4.1e-7 (K 512) off, sums of 256: 2.4e-7.
+constexpr int kSplitChunk = 8, kSplitChunkShort = 4;
 
 struct SplitPlan {
-  int nt = 0;       // rows of X per tile (a multiple of 16, at most 256)
+  int mt = 0;       // rows of X per tile (a multiple of 16)
   int ks = 1;       // CTAs of a cluster that share a tile along K
   int stages = 0;   // depth of the TMA ring
-  int chunk = kSplitChunk;   // K blocks per accumulator
+  int chunk = 0;    // K blocks per accumulator
 };
 
-// false: the 128 x 256 tiles of dense_gemm.cu are the better cut of this product
-bool split_gemm_plan(int M, int N, int K, bool out_f32, int num_sms, SplitPlan* out);
+// x [M][K] and w [groups][N][K] as bf16 arrays, or as three bf16 parts of fp32 arrays laid out by launch_split_parts.
+struct SplitGemm {
+  const void* x = nullptr;
+  const void* w = nullptr;
+  void* out = nullptr;
+  const float* bias = nullptr;
+  int M = 0, N = 0, K = 0;
+  long long ldo = 0;
+  bool out_f32 = false;
+  int xparts = 1, wparts = 1;               // 1 or 3; three parts of w only with three of x
+  int groups = 1;
+  const int* tile_group = nullptr;          // binned rows: matrix of each row tile, and the number of row tiles (device)
+  const int* n_tiles_dev = nullptr;
+  bool batched = false;                     // every group has M rows of its own: out row m of group g at g * out_group + m * ldo
+  long long out_group = 0;
+  // the operands the parts were made of (three parts only): an output that is not a number is computed again from them, since parts of an
+  // infinity times a zero part are not what the product is
+  const float* x_raw = nullptr;
+  long long x_ld = 0, x_group = 0;
+  const void* w_raw = nullptr;              // fp32 when wparts is 3, else bf16; rows of K
+};
 
+// false: the 128 x 256 tiles of dense_gemm.cu are the better cut of this product (one part, one group only)
+bool split_gemm_plan(int M, int N, int K, bool out_f32, int num_sms, int xparts, int wparts, int groups, SplitPlan* out);
 // binned rows (one weight matrix per row tile): a CTA per tile and 128 columns, K uncut
 SplitPlan split_gemm_binned_plan(int N, int K, bool out_f32, int tile_rows);
 
-cudaError_t launch_split_gemm(const void* x, const void* w, void* out, const float* bias, int M, int N, int K, long long ldo, bool out_f32,
-                              const SplitPlan& plan, const int* tile_group, const int* n_tiles_dev, int groups, cudaStream_t s);
+cudaError_t launch_split_gemm(const SplitGemm& g, const SplitPlan& plan, cudaStream_t s);
+
+// fp32 [groups][rows][K] (row stride ld, group stride group_stride) -> bf16 parts hi, mid, lo with hi + mid + lo = value (24 bits), laid out
+// [groups][tiles][3][mt][K] with zero rows behind the last one
+cudaError_t launch_split_parts(const float* x, long long ld, long long group_stride, int rows, int K, int mt, int groups, void* parts, cudaStream_t s);
 
 }  // namespace kb2

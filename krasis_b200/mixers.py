@@ -70,8 +70,8 @@ def _core_lib():
 
 
 def lin(a: torch.Tensor, w: torch.Tensor, out_dtype=torch.float32) -> torch.Tensor:
-    """a [M, K] @ w [N, K]^T with fp32 accumulation.  Bfloat16 products of more rows than a GEMV takes run on the tensor cores (the core
-    library picks the kernel by the sizes); at 8 rows and fewer the weights are streamed by `gemv_nt_vec`."""
+    """a [M, K] (row stride free) @ w [N, K]^T with fp32 accumulation.  Products of more rows than a GEMV takes run on the tensor cores (the
+    core library picks the kernel by the sizes), fp32 operands as exact bf16 parts; at 8 rows and fewer the weights are streamed once."""
     M, K = a.shape
     N = w.shape[0]
     if (a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and M > GEMV_ROWS and K % 64 == 0 and N % 16 == 0 and a.is_contiguous()
@@ -83,7 +83,42 @@ def lin(a: torch.Tensor, w: torch.Tensor, out_dtype=torch.float32) -> torch.Tens
             capi.check(core.kb2_linear_bf16(a.data_ptr(), w.data_ptr(), None, out.data_ptr(), M, N, K, int(out_dtype == torch.float32),
                                             a.device.index or 0, torch.cuda.current_stream(a.device).cuda_stream))
             return out
+    if a.dtype == torch.float32 and M > GEMV_ROWS and out_dtype in (torch.float32, torch.bfloat16):
+        out = torch.empty((M, N), dtype=out_dtype, device=a.device)
+        return out if _lin_f32(a.unsqueeze(1), w.unsqueeze(0), out.unsqueeze(1)) else ops.gemm(a, w, out_dtype, out=out)
     return ops.gemm(a, w, out_dtype)
+
+
+def _lin_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
+    """out[:, g] = a[:, g] @ w[g]^T for fp32 a [M, G, K] and fp32 or bfloat16 w [G, N, K] on the tensor cores, the operands as exact bf16
+    parts: the accuracy of fp32 sums (kb2_linear_f32).  False: sizes, strides or alignment it does not take (K below 128 too, where the
+    FMA kernel's few steps cost less than the pass that makes the parts: 10 us against 6 at K = 128, 5 against 6 at K = 64)."""
+    M, G, K = a.shape
+    N = w.shape[1]
+    if (K < 128 or K % 64 or N % 16 or w.shape[0] != G or w.shape[2] != K or a.stride(2) != 1 or not w.is_contiguous() or out.stride(2) != 1
+            or out.stride(0) % 4 or out.stride(1) % 4 or out.data_ptr() % 16 or w.dtype not in (torch.float32, torch.bfloat16)
+            or (w.dtype == torch.bfloat16 and w.data_ptr() % 16) or not (a.is_cuda and w.is_cuda)):
+        return False
+    core = _core_lib()
+    if not core:
+        return False
+    from . import capi
+    dev, wide = a.device.index or 0, int(w.dtype == torch.float32)
+    size = core.kb2_linear_f32_workspace(M, N, K, wide, G, dev)
+    if not size:
+        return False
+    work = torch.empty(size, dtype=torch.uint8, device=a.device)
+    capi.check(core.kb2_linear_f32(a.data_ptr(), a.stride(0), a.stride(1), w.data_ptr(), wide, out.data_ptr(), int(out.dtype == torch.float32),
+                                   out.stride(0), out.stride(1), M, N, K, G, work.data_ptr(), size, dev,
+                                   torch.cuda.current_stream(a.device).cuda_stream))
+    return True
+
+
+def lin_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+    """Per-head products: a [M, H, K] fp32 (unit last stride), w [H, N, K] -> out [M, H, N]."""
+    if a.dtype == torch.float32 and a.shape[0] > GEMV_ROWS and _lin_f32(a, w, out):
+        return out
+    return ops.gemm_heads(a, w, out)
 
 
 def layer_runs(n: int, start: int = 0, stop: int = 0, times: int = 1):
@@ -207,7 +242,7 @@ class WindowLatentAttention:
             hgr = hg[r0:] if hg is not None else None
             if not fast:
                 q_abs = torch.empty((n, H, self.r), dtype=torch.float32, device=h.device)
-                ops.gemm_heads(q[r0:r0 + n, :, :self.dn], self.uk_t, q_abs)
+                lin_heads(q[r0:r0 + n, :, :self.dn], self.uk_t, q_abs)
                 o_lat = torch.empty((n, H, self.r), dtype=torch.float32, device=h.device)
                 # few tokens (decoding): each token's keys are cut into pieces so that the whole GPU works on them
                 blocks = n * ((H + 7) // 8)
@@ -220,7 +255,7 @@ class WindowLatentAttention:
                                                          tb.seq_of[r0:].data_ptr(), tb.pages.data_ptr(), tb.max_pages, page_size,
                                                          ops._ptr(self.sink), self.scale, self.window, o_lat.data_ptr(), None,
                                                          self.tc_min_portion, nsplit, ops._ptr(part_acc), ops._ptr(part_ml), ops._ptr(hgr), ldg, s))
-                ops.gemm_heads(o_lat, self.uv, o[r0:r0 + n])
+                lin_heads(o_lat, self.uv, o[r0:r0 + n])
                 continue
             from . import capi
             for i in seqs:
@@ -288,7 +323,7 @@ def lin_cols(proj: torch.Tensor, off: int, r: int, w: torch.Tensor, dtype) -> to
     a = proj[:, off:off + r]
     if dtype == torch.bfloat16 and proj.shape[0] >= 256 and r % 64 == 0 and _core_lib():
         return lin(a.to(torch.bfloat16).contiguous(), w, torch.float32)
-    return ops.gemm(a, w, torch.float32)
+    return lin(a, w, torch.float32)
 
 
 class GatedLinearAttention:
@@ -468,7 +503,7 @@ class GatedRecurrentUnit:
         core = _core_lib() if self.w_gates_twice is not None and T >= self.tc_min_tokens else False
         if not core:
             z = torch.empty((T, self.B, 2 * self.bs), dtype=torch.float32, device=dev)
-            ops.gemm_heads(u.view(T, self.B, self.bs), self.w_gates, z)
+            lin_heads(u.view(T, self.B, self.bs), self.w_gates, z)
             return z, 2 * self.C, 2 * self.bs
         from . import capi
         tp = (T + 127) // 128 * 128
@@ -555,7 +590,7 @@ class ChannelDeltaMixer:
         a = proj[:, off:off + r]
         if self.dtype == torch.bfloat16 and proj.shape[0] >= 256 and r % 64 == 0 and _core_lib():
             return lin(a.to(torch.bfloat16).contiguous(), w, torch.float32)
-        return ops.gemm(a, w, torch.float32)
+        return lin(a, w, torch.float32)
 
     def forward(self, h: torch.Tensor, tb: ops.StepTables, tail: torch.Tensor, state: torch.Tensor) -> torch.Tensor:
         lib, T, H = ops.load(), h.shape[0], self.H

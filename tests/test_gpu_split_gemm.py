@@ -103,3 +103,53 @@ def test_long_and_short_binning_agree():
             assert torch.equal(torch.sort(rows[real])[0], torch.nonzero((ids >= 0) & (ids < E)).flatten())
             assert torch.equal(ids[rows[real]].long(), t["tile_expert"][:n].long().repeat_interleave(tile)[real])
             assert torch.equal(t["pos"].long()[rows[real]], torch.nonzero(real).flatten()) and int((t["pos"] < 0).sum()) == slots - int(real.sum())
+
+
+def _f32(x, w, out):
+    from krasis_b200.mixers import _lin_f32
+    assert _lin_f32(x, w, out)
+    return out
+
+
+# rows around a tile (16, 80 per tile of parts), uneven K cuts, heads side by side, a slice border of the weight parts (N 8192, K 4096)
+@pytest.mark.parametrize("M,N,K,G", [(9, 16, 128, 1), (17, 144, 192, 3), (80, 272, 512, 1), (81, 128, 576, 2), (255, 512, 128, 16), (300, 2048, 2048, 1),
+                                     (33, 8192, 4096, 1)])
+@pytest.mark.parametrize("wide", [True, False])
+def test_fp32_rows_are_as_exact_as_fp32_sums(M, N, K, G, wide):
+    from krasis_b200 import seqops as ops
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn(M, G, K, device="cuda", generator=g) * torch.exp(torch.randn(M, G, 1, device="cuda", generator=g) * 8)      # rows of any size
+    w = torch.randn(G, N, K, device="cuda", generator=g) * K ** -0.5
+    w = w if wide else w.bfloat16()
+    want = torch.einsum("mgk,gnk->mgn", x.double(), w.double())
+    err = lambda y: ((y.double() - want).norm(dim=2) / want.norm(dim=2)).square().mean().sqrt().item()  # noqa: E731
+    got = _f32(x, w, torch.full((M, G, N), float("nan"), device="cuda"))
+    fma = ops.gemm_heads(x, w, torch.empty(M, G, N, device="cuda"))
+    assert err(got) <= err(fma) < 4e-6
+    half = _f32(x, w, torch.empty(M, G, N, device="cuda", dtype=torch.bfloat16))
+    assert ((half.double() - want).abs() <= 2.0 ** -8 * want.abs() + 4e-6 * want.norm(dim=2, keepdim=True)).all()
+
+
+@pytest.mark.parametrize("wide", [True, False])
+def test_fp32_rows_with_extreme_values(wide):
+    """Infinities, NaN, the largest and the smallest numbers come out as a plain fp32 product gives them."""
+    M, N, K = 24, 128, 128
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x, w = torch.randn(M, 1, K, device="cuda", generator=g), torch.randn(1, N, K, device="cuda", generator=g)
+    x[0, 0, 3], x[1, 0, 5], x[2, 0, 7] = float("inf"), float("-inf"), float("nan")
+    x[3], x[4] = 0.0, 0.0
+    x[3, 0, 9] = 3.4028e38                       # rounds to infinity in bf16
+    x[4, 0, 9] = 1e-38
+    x[5, 0, 0], x[5, 0, 1] = float("inf"), float("-inf")
+    w = w.bfloat16().float()
+    w[0, 7, 3], w[0, 9, :] = 0.0, 0.0            # infinity times zero
+    w[0, :, 9] = w[0, :, 9].clamp(-0.875, 0.875)
+    if wide:
+        w[0, 11, 0] = float("inf")
+    want = (x[:, 0].unsqueeze(1).double() * w[0].unsqueeze(0).double()).float().sum(-1)
+    got = _f32(x, w if wide else w.bfloat16(), torch.empty(M, 1, N, device="cuda"))[:, 0]
+    same = (got == want) | (got.isnan() & want.isnan())
+    # beside the rounding of sums: bf16 numbers end at 2^-133, so what a part of x misses is at most 2^-134 in absolute terms, times |w| (it
+    # shows for x below 1e-33 only, here in row 4)
+    room = 1e-6 * (x[:, 0].abs().unsqueeze(1) * w[0].abs().unsqueeze(0)).sum(-1) + 2.0 ** -133 * w[0].abs().amax(-1)
+    assert (same | (want.isfinite() & got.isfinite() & ((got - want).abs() <= room))).all()
