@@ -36,6 +36,18 @@ __global__ void embed_scale_kernel(const T* __restrict__ table, const int* __res
   const long long row = tokens[t];
   for (int d = threadIdx.x; d < W; d += blockDim.x) x[t * W + d] = ldf(table, row * W + d) * scale;
 }
+// bf16 tables whose rows start on 16 bytes: eight columns per thread, so that a row's cold loads are all in flight at once
+__global__ void __launch_bounds__(256) embed_scale_vec_kernel(const bf16* __restrict__ table, const int* __restrict__ tokens, float* __restrict__ x, int W,
+                                                              float scale) {
+  const long long t = blockIdx.x, row = tokens[t];
+  for (int d = threadIdx.x * 8; d < W; d += 256 * 8) {
+    float f[8];
+    unpack8(*reinterpret_cast<const uint4*>(table + row * W + d), f);
+    float4* o = reinterpret_cast<float4*>(x + t * W + d);
+    o[0] = make_float4(f[0] * scale, f[1] * scale, f[2] * scale, f[3] * scale);
+    o[1] = make_float4(f[4] * scale, f[5] * scale, f[6] * scale, f[7] * scale);
+  }
+}
 
 // ------------------------------------------------------------------------------------------------ GEMM
 // C[M,N] = A[M,K] * B[N,K]^T.  64x64 tile, 16-wide K steps, 4x4 outputs per thread, fp32 FMA.  Each output sums its K products
@@ -223,11 +235,123 @@ static bool launch_gemv_vec(const void* A, long long lda, const void* B, long lo
   return true;
 }
 
+// ---- few bfloat16 rows against bfloat16 weights, on the warp-level tensor instructions
+// Bound: the weights' way from HBM; the arithmetic has to stay out of the way (fp32 FMAs on unpacked values took 200 instructions per KB of
+// weights at 4 rows).  A warp owns 16 weight rows (the 16-row side of mma.m16n8k16) and up to 8 rows of A (its 8-column side).  A product
+// does not care about the order along K, so a lane takes 16 neighbouring bytes of its weight row and the same 16 of its row of A, and word
+// pairs of the two go into two instructions as they are: no shuffles, no shared memory, 64-byte runs per quad and load.  KS warps of a block
+// share the rows and take pieces of 128 numbers in turn; the loads of the next piece are in flight under the current one.  Each instruction
+// pair starts from zero, its 32 products are added to one of four running sums in round-to-nearest, and the sums meet pairwise: the error is
+// that of the FMA form (8e-8).  From HBM at 4 rows, us before (gemv_nt_vec) and now: N 16384, K 2048 32.3 -> 14.1 (floor 10.3);
+// N 2048, K 8192 19.8 -> 8.9 (5.1); N 32768, K 2048 44.3 -> 24.1 (20.5); N 2048, K 2048 7.1 -> 4.0.
+__device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <typename TC, int KS>
+__global__ void __launch_bounds__(KS > 8 ? 512 : 256) gemv_mma_kernel(const bf16* __restrict__ A, long long lda, const bf16* __restrict__ B, long long ldb,
+                                                                      TC* __restrict__ C, long long ldc, int M, int N, int K, long long sA, long long sB,
+                                                                      long long sC) {
+  constexpr int kStep = 128, kWarps = KS > 8 ? 16 : 8, kGroups = kWarps / KS;
+  __shared__ float red[kWarps][8][17];                   // [warp][row of A][weight row], odd pitch
+  A += (long long)blockIdx.z * sA;
+  B += (long long)blockIdx.z * sB;
+  C += (long long)blockIdx.z * sC;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quad = lane >> 2, t8 = (lane & 3) * 8;
+  const int n0 = (blockIdx.x * kGroups + warp / KS) * 16;
+  // rows beyond the last one are read as the last one and not written
+  const bf16* w0 = B + (long long)min(n0 + quad, N - 1) * ldb + t8;
+  const bf16* w1 = B + (long long)min(n0 + quad + 8, N - 1) * ldb + t8;
+  const bf16* x = A + (long long)min(quad, M - 1) * lda + t8;
+  const bool row = quad < M;
+  uint4 cur[2][4], nxt[2][4];
+  auto fetch = [&](uint4 (&to)[2][4], int k) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int kj = k + j * 32;
+      const bool in = kj + t8 < K;
+      to[0][j] = in ? ld_stream16(w0 + kj) : make_uint4(0, 0, 0, 0);
+      to[1][j] = in ? ld_stream16(w1 + kj) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  float sum[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sum[j][i] = 0.f;
+  int k = (warp % KS) * kStep;
+  if (n0 < N) fetch(cur, k);
+  for (; n0 < N && k < K; k += KS * kStep) {
+    if (k + KS * kStep < K) fetch(nxt, k + KS * kStep);
+    uint4 xv[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      xv[j] = row && k + j * 32 + t8 < K ? *reinterpret_cast<const uint4*>(x + k + j * 32) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint4 a = cur[0][j], c = cur[1][j];
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
+      mma16816(d, a.x, c.x, a.y, c.y, xv[j].x, xv[j].y);
+      mma16816(d, a.z, c.z, a.w, c.w, xv[j].z, xv[j].w);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sum[j][i] += d[i];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      cur[0][j] = nxt[0][j];
+      cur[1][j] = nxt[1][j];
+    }
+  }
+  // sum[.][0], [1]: weight row quad, rows 2 (lane & 3) and + 1 of A; [2], [3]: weight row quad + 8
+  const int m = (lane & 3) * 2;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) red[warp][m + (i & 1)][quad + (i >> 1) * 8] = (sum[0][i] + sum[1][i]) + (sum[2][i] + sum[3][i]);
+  __syncthreads();
+  for (int i = threadIdx.x; i < kGroups * 128; i += kWarps * 32) {
+    const int g = i >> 7, mm = (i >> 4) & 7, r = i & 15, n = (blockIdx.x * kGroups + g) * 16 + r;
+    if (mm >= M || n >= N) continue;
+    float v[KS];
+#pragma unroll
+    for (int p = 0; p < KS; ++p) v[p] = red[g * KS + p][mm][r];
+#pragma unroll
+    for (int o = KS / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int p = 0; p < o; ++p) v[p] += v[p + o];
+    stf(C, (long long)mm * ldc + n, v[0]);
+  }
+}
+
+template <typename TC>
+static bool launch_gemv_mma(const void* A, long long lda, const void* B, long long ldb, void* C, long long ldc, int M, int N, int K,
+                            int batch, long long sA, long long sB, long long sC, cudaStream_t s) {
+  if (K % 8 || ldb % 8 || sB % 8 || ((uintptr_t)B & 15) || ((uintptr_t)A & 15) || lda % 8 || sA % 8) return false;
+  // a small matrix and one or two rows: a launch's latency, and gemv_nt_vec's is shorter (N 256, K 2048, 1 row 2.2 us against 2.9; at
+  // N 4096, K 512 3.1 against 3.0)
+  if (M <= 2 && (long long)N * K * batch < (1 << 20)) return false;
+  const int groups = (N + 15) / 16;
+  int ks = 1;                                  // about 2048 warps, in one wave of two blocks per SM, as long as each has a piece of K
+  while (ks < 16 && (long long)groups * batch * 2 * ks <= 2368 && K > 128 * ks) ks *= 2;
+  const int per = (ks > 8 ? 16 : 8) / ks;
+  const dim3 grid((groups + per - 1) / per, 1, batch);
+#define KB2_GEMV(KSV)                                                                                                                        \
+  case KSV:                                                                                                                                  \
+    gemv_mma_kernel<TC, KSV><<<grid, KSV > 8 ? 512 : 256, 0, s>>>((const bf16*)A, lda, (const bf16*)B, ldb, (TC*)C, ldc, M, N, K, sA, sB, sC); \
+    break;
+  switch (ks) { KB2_GEMV(1) KB2_GEMV(2) KB2_GEMV(4) KB2_GEMV(8) KB2_GEMV(16) }
+#undef KB2_GEMV
+  return true;
+}
+
 template <typename TA, typename TB, typename TC>
 static void launch_gemm(const void* A, long long lda, const void* B, long long ldb, void* C, long long ldc, int M, int N, int K,
                         int batch, long long sA, long long sB, long long sC, cudaStream_t s) {
   if (M <= 8) {
     if constexpr (sizeof(TB) == 2) {
+      if constexpr (sizeof(TA) == 2) {
+        if (launch_gemv_mma<TC>(A, lda, B, ldb, C, ldc, M, N, K, batch, sA, sB, sC, s)) return;
+      }
       if (launch_gemv_vec<TA, TC>(A, lda, B, ldb, C, ldc, M, N, K, batch, sA, sB, sC, s)) return;
     }
     dim3 grid((N + 7) / 8, 1, batch);
@@ -315,6 +439,130 @@ __global__ void __launch_bounds__(256) residual_norm_kernel(float* __restrict__ 
   q = block_sum(q, red);
   const float rstd = 1.f / sqrtf(q * inv_w + eps);
   for (int d = threadIdx.x; d < W; d += blockDim.x) st_dt(h, dt_h, row * W + d, (rowbuf[d] - mean) * rstd * wb[d] + (bb != nullptr ? bb[d] : 0.f));
+}
+
+// The same for widths that are multiples of 4 up to 1024 NV: a thread keeps its 4 NV columns in registers and asks for everything the row
+// needs before the first sum, and a sum over the block costs one barrier.  Bound by traffic on long steps, by the chain of (up to) four sums
+// on short ones.
+template <int NV>
+__global__ void __launch_bounds__(256) residual_norm_vec_kernel(float* __restrict__ x, const float* __restrict__ y, int y_mode,
+                                                                const float* __restrict__ wa, const float* __restrict__ ba,
+                                                                const float* __restrict__ x0, const float* __restrict__ wb,
+                                                                const float* __restrict__ bb, void* __restrict__ h, int dt_h, int W, float eps,
+                                                                const float* __restrict__ y2) {
+  __shared__ float red[4][8];
+  const long long base = (long long)blockIdx.x * W;
+  const int tid = threadIdx.x;
+  const float inv_w = 1.f / (float)W;
+  int turn = 0;
+  auto row_sum = [&](float v) {                // four sums at most, each in a row of `red` of its own
+    v = warp_sum(v);
+    float* r = red[turn++ & 3];
+    if ((tid & 31) == 0) r[tid >> 5] = v;
+    __syncthreads();
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t += r[i];
+    return t;
+  };
+  auto at = [&](int i) { return (i * 256 + tid) * 4; };
+  auto load = [&](const float* p, int i) {
+    return p != nullptr && at(i) < W ? *reinterpret_cast<const float4*>(p + at(i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  auto row = [&](const float* p) { return p != nullptr ? p + base : nullptr; };
+  float4 v[NV], yv[NV], av[NV], cv[NV], gv[NV], bv[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    v[i] = load(row(x), i);
+    yv[i] = load(row(y), i);
+    av[i] = load(row(x0), i);
+    cv[i] = load(row(y2), i);
+  }
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    gv[i] = load(y != nullptr && y_mode != 3 ? wa : nullptr, i);
+    bv[i] = load(y != nullptr && y_mode == 1 ? ba : nullptr, i);
+  }
+  auto sum4 = [](const float4& q) { return (q.x + q.y) + (q.z + q.w); };
+  auto sq4 = [](const float4& q, float m) {
+    const float a = q.x - m, b = q.y - m, c = q.z - m, d = q.w - m;
+    return (a * a + b * b) + (c * c + d * d);
+  };
+  auto squares = [&](const float4 (&q)[NV], float m) {      // columns beyond the row do not count
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) t += at(i) < W ? sq4(q[i], m) : 0.f;
+    return t;
+  };
+  if (y != nullptr && y_mode != 3) {
+    float mean = 0.f;
+    if (y_mode == 1) {
+      float t = 0.f;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) t += sum4(yv[i]);
+      mean = row_sum(t) * inv_w;
+    }
+    const float rstd = 1.f / sqrtf(row_sum(squares(yv, mean)) * inv_w + eps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      v[i].x += fmaf((yv[i].x - mean) * rstd, gv[i].x, bv[i].x);
+      v[i].y += fmaf((yv[i].y - mean) * rstd, gv[i].y, bv[i].y);
+      v[i].z += fmaf((yv[i].z - mean) * rstd, gv[i].z, bv[i].z);
+      v[i].w += fmaf((yv[i].w - mean) * rstd, gv[i].w, bv[i].w);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      v[i].x += yv[i].x + cv[i].x;
+      v[i].y += yv[i].y + cv[i].y;
+      v[i].z += yv[i].z + cv[i].z;
+      v[i].w += yv[i].w + cv[i].w;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    v[i].x += av[i].x;
+    v[i].y += av[i].y;
+    v[i].z += av[i].z;
+    v[i].w += av[i].w;
+    if ((y != nullptr || x0 != nullptr) && at(i) < W) *reinterpret_cast<float4*>(x + base + at(i)) = v[i];
+    gv[i] = load(h != nullptr ? wb : nullptr, i);
+    bv[i] = load(h != nullptr ? bb : nullptr, i);
+  }
+  if (h == nullptr) return;
+  float t = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) t += sum4(v[i]);
+  const float mean = row_sum(t) * inv_w;
+  const float rstd = 1.f / sqrtf(row_sum(squares(v, mean)) * inv_w + eps);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    if (at(i) >= W) continue;
+    const float4 o = make_float4(fmaf((v[i].x - mean) * rstd, gv[i].x, bv[i].x), fmaf((v[i].y - mean) * rstd, gv[i].y, bv[i].y),
+                                 fmaf((v[i].z - mean) * rstd, gv[i].z, bv[i].z), fmaf((v[i].w - mean) * rstd, gv[i].w, bv[i].w));
+    if (dt_h == 0) {
+      *reinterpret_cast<float4*>((float*)h + base + at(i)) = o;
+    } else {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(o.x, o.y), hi = __floats2bfloat162_rn(o.z, o.w);
+      *reinterpret_cast<uint2*>((bf16*)h + base + at(i)) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+  }
+}
+
+static int launch_residual_norm(float* x, const float* y, int y_mode, const float* wa, const float* ba, const float* x0, const float* wb,
+                                const float* bb, void* h, int dt_h, int T, int W, float eps, const float* y2, cudaStream_t s) {
+  const uintptr_t all = (uintptr_t)x | (uintptr_t)y | (uintptr_t)wa | (uintptr_t)ba | (uintptr_t)x0 | (uintptr_t)wb | (uintptr_t)bb | (uintptr_t)h | (uintptr_t)y2;
+  if (W % 4 == 0 && W <= 8192 && !(all & 15)) {
+#define KB2_RN(NVV) residual_norm_vec_kernel<NVV><<<T, 256, 0, s>>>(x, y, y_mode, wa, ba, x0, wb, bb, h, dt_h, W, eps, y2)
+    if (W <= 1024) KB2_RN(1); else if (W <= 2048) KB2_RN(2); else if (W <= 4096) KB2_RN(4); else KB2_RN(8);
+#undef KB2_RN
+  } else {
+    const size_t smem = (size_t)W * 4;
+    if (smem > 48 * 1024) SEQ_CUDA(cudaFuncSetAttribute(residual_norm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    residual_norm_kernel<<<T, 256, smem, s>>>(x, y, y_mode, wa, ba, x0, wb, bb, h, dt_h, W, eps, y2);
+  }
+  SEQ_LAUNCHED();
+  return KB2SEQ_OK;
 }
 
 // One block per token row.  x (fp32) += y_mult * y (y may be null); then h = x / sqrt(mean(x^2) + eps) * (w_shift + w) if h is given
@@ -1142,7 +1390,9 @@ KB2SEQ_API long long kb2_seq_total_launches(void) { return g_launches; }
 
 KB2SEQ_API int kb2_seq_embed(const void* table, int dt, const int* tokens, float* x, int T, int W, float scale, void* stream) {
   if (!table || !tokens || !x || T <= 0 || W <= 0 || bad_dt(dt)) return failf(KB2SEQ_ERR_VALUE, "embed: bad argument");
-  if (dt) embed_scale_kernel<bf16><<<T, 128, 0, (cudaStream_t)stream>>>((const bf16*)table, tokens, x, W, scale);
+  if (dt && W % 8 == 0 && !((uintptr_t)table & 15) && !((uintptr_t)x & 15))
+    embed_scale_vec_kernel<<<T, 256, 0, (cudaStream_t)stream>>>((const bf16*)table, tokens, x, W, scale);
+  else if (dt) embed_scale_kernel<bf16><<<T, 128, 0, (cudaStream_t)stream>>>((const bf16*)table, tokens, x, W, scale);
   else embed_scale_kernel<float><<<T, 128, 0, (cudaStream_t)stream>>>((const float*)table, tokens, x, W, scale);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
@@ -1177,10 +1427,7 @@ KB2SEQ_API int kb2_seq_residual_norm(float* x, const float* y, int y_mode, const
   if (h && (!wb || !bb)) return failf(KB2SEQ_ERR_VALUE, "residual_norm: output norm needs weight and bias");
   const size_t smem = (size_t)W * 4;
   if (smem > 200 * 1024) return failf(KB2SEQ_ERR_VALUE, "residual_norm: width %d too large", W);
-  if (smem > 48 * 1024) SEQ_CUDA(cudaFuncSetAttribute(residual_norm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  residual_norm_kernel<<<T, 256, smem, (cudaStream_t)stream>>>(x, y, y_mode, wa, ba, x0, wb, bb, h, dt_h, W, eps, nullptr);
-  SEQ_LAUNCHED();
-  return KB2SEQ_OK;
+  return launch_residual_norm(x, y, y_mode, wa, ba, x0, wb, bb, h, dt_h, T, W, eps, nullptr, (cudaStream_t)stream);
 }
 
 KB2SEQ_API int kb2_seq_residual_add_norm(float* x, const float* y, const float* y2, const float* wb, const float* bb, void* h, int dt_h,
@@ -1189,10 +1436,7 @@ KB2SEQ_API int kb2_seq_residual_add_norm(float* x, const float* y, const float* 
   if (h && !wb) return failf(KB2SEQ_ERR_VALUE, "residual_add_norm: output norm needs its weight");
   const size_t smem = (size_t)W * 4;
   if (smem > 200 * 1024) return failf(KB2SEQ_ERR_VALUE, "residual_add_norm: width %d too large", W);
-  if (smem > 48 * 1024) SEQ_CUDA(cudaFuncSetAttribute(residual_norm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  residual_norm_kernel<<<T, 256, smem, (cudaStream_t)stream>>>(x, y, 3, nullptr, nullptr, nullptr, wb, bb, h, dt_h, W, eps, y2);
-  SEQ_LAUNCHED();
-  return KB2SEQ_OK;
+  return launch_residual_norm(x, y, 3, nullptr, nullptr, nullptr, wb, bb, h, dt_h, T, W, eps, y2, (cudaStream_t)stream);
 }
 
 KB2SEQ_API int kb2_seq_act_mul(const void* in, int dt_in, void* out, int dt_out, int T, int F, void* stream) {

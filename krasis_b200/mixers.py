@@ -71,7 +71,7 @@ def _core_lib():
 
 def lin(a: torch.Tensor, w: torch.Tensor, out_dtype=torch.float32) -> torch.Tensor:
     """a [M, K] (row stride free) @ w [N, K]^T with fp32 accumulation.  Products of more rows than a GEMV takes run on the tensor cores (the
-    core library picks the kernel by the sizes), fp32 operands as exact bf16 parts; at 8 rows and fewer the weights are streamed once."""
+    core library picks the kernel by the sizes), fp32 operands as exact bf16 parts; at 8 rows and fewer the weights are streamed by a GEMV."""
     M, K = a.shape
     N = w.shape[0]
     if (a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and M > GEMV_ROWS and K % 64 == 0 and N % 16 == 0 and a.is_contiguous()
@@ -83,7 +83,10 @@ def lin(a: torch.Tensor, w: torch.Tensor, out_dtype=torch.float32) -> torch.Tens
             capi.check(core.kb2_linear_bf16(a.data_ptr(), w.data_ptr(), None, out.data_ptr(), M, N, K, int(out_dtype == torch.float32),
                                             a.device.index or 0, torch.cuda.current_stream(a.device).cuda_stream))
             return out
-    if a.dtype == torch.float32 and M > GEMV_ROWS and out_dtype in (torch.float32, torch.bfloat16):
+    # fp32 rows: a handful of them against a large bfloat16 matrix too (an output head of 32768 x 2048: 4 rows 41 us as a GEMV, 32 in parts;
+    # 8 rows 80 against 32; one row 28 against 31)
+    few = 3 <= M <= GEMV_ROWS and w.dtype == torch.bfloat16 and N * K >= 1 << 24
+    if a.dtype == torch.float32 and (M > GEMV_ROWS or few) and out_dtype in (torch.float32, torch.bfloat16):
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
         return out if _lin_f32(a.unsqueeze(1), w.unsqueeze(0), out.unsqueeze(1)) else ops.gemm(a, w, out_dtype, out=out)
     return ops.gemm(a, w, out_dtype)
