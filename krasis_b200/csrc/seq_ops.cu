@@ -37,6 +37,7 @@ __global__ void embed_scale_kernel(const T* __restrict__ table, const int* __res
   for (int d = threadIdx.x; d < W; d += blockDim.x) x[t * W + d] = ldf(table, row * W + d) * scale;
 }
 // bf16 tables whose rows start on 16 bytes: eight columns per thread, so that a row's cold loads are all in flight at once
+// (4 tokens of 2048 columns took 9.5 us with eight rounds of loads)
 __global__ void __launch_bounds__(256) embed_scale_vec_kernel(const bf16* __restrict__ table, const int* __restrict__ tokens, float* __restrict__ x, int W,
                                                               float scale) {
   const long long t = blockIdx.x, row = tokens[t];
@@ -241,9 +242,9 @@ static bool launch_gemv_vec(const void* A, long long lda, const void* B, long lo
 // does not care about the order along K, so a lane takes 16 neighbouring bytes of its weight row and the same 16 of its row of A, and word
 // pairs of the two go into two instructions as they are: no shuffles, no shared memory, 64-byte runs per quad and load.  KS warps of a block
 // share the rows and take pieces of 128 numbers in turn; the loads of the next piece are in flight under the current one.  Each instruction
-// pair starts from zero, its 32 products are added to one of four running sums in round-to-nearest, and the sums meet pairwise: the error is
-// that of the FMA form (8e-8).  From HBM at 4 rows, us before (gemv_nt_vec) and now: N 16384, K 2048 32.3 -> 14.1 (floor 10.3);
-// N 2048, K 8192 19.8 -> 8.9 (5.1); N 32768, K 2048 44.3 -> 24.1 (20.5); N 2048, K 2048 7.1 -> 4.0.
+// pair starts from zero, its 32 products join a compensated running sum, and the warps' sums meet pairwise: the error is that of the FMA form
+// (8e-8) or less.  From HBM at 4 rows, us before (gemv_nt_vec) and now: N 16384, K 2048 32.3 -> 13.7 (floor 10.3);
+// N 2048, K 8192 19.8 -> 9.2 (5.1); N 32768, K 2048 44.4 -> 25.3 (20.5); N 2048, K 2048 7.3 -> 3.8.
 __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -276,38 +277,45 @@ __global__ void __launch_bounds__(KS > 8 ? 512 : 256) gemv_mma_kernel(const bf16
       to[1][j] = in ? ld_stream16(w1 + kj) : make_uint4(0, 0, 0, 0);
     }
   };
-  float sum[4][4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) sum[j][i] = 0.f;
-  int k = (warp % KS) * kStep;
-  if (n0 < N) fetch(cur, k);
-  for (; n0 < N && k < K; k += KS * kStep) {
-    if (k + KS * kStep < K) fetch(nxt, k + KS * kStep);
+  float sum[4] = {0.f, 0.f, 0.f, 0.f}, lost[4] = {0.f, 0.f, 0.f, 0.f};
+  auto piece = [&](const uint4 (&w)[2][4], int k) {
     uint4 xv[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       xv[j] = row && k + j * 32 + t8 < K ? *reinterpret_cast<const uint4*>(x + k + j * 32) : make_uint4(0, 0, 0, 0);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const uint4 a = cur[0][j], c = cur[1][j];
+      const uint4 a = w[0][j], c = w[1][j];
       float d[4] = {0.f, 0.f, 0.f, 0.f};
       mma16816(d, a.x, c.x, a.y, c.y, xv[j].x, xv[j].y);
       mma16816(d, a.z, c.z, a.w, c.w, xv[j].z, xv[j].w);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) sum[j][i] += d[i];
+      for (int i = 0; i < 4; ++i) {                // compensated: what the addition rounds off goes into the next one
+        const float add = d[i] - lost[i], t = sum[i] + add;
+        lost[i] = (t - sum[i]) - add;
+        sum[i] = t;
+      }
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      cur[0][j] = nxt[0][j];
-      cur[1][j] = nxt[1][j];
+  };
+  // two pieces per round, so that no copy between the buffers waits for the loads in flight
+  int k = (warp % KS) * kStep;
+  const int step = KS * kStep;
+  if (n0 < N) {
+    fetch(cur, k);
+    while (k < K) {
+      if (k + step < K) fetch(nxt, k + step);
+      piece(cur, k);
+      k += step;
+      if (k >= K) break;
+      if (k + step < K) fetch(cur, k + step);
+      piece(nxt, k);
+      k += step;
     }
   }
-  // sum[.][0], [1]: weight row quad, rows 2 (lane & 3) and + 1 of A; [2], [3]: weight row quad + 8
+  // sum[0], [1]: weight row quad, rows 2 (lane & 3) and + 1 of A; [2], [3]: weight row quad + 8
   const int m = (lane & 3) * 2;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) red[warp][m + (i & 1)][quad + (i >> 1) * 8] = (sum[0][i] + sum[1][i]) + (sum[2][i] + sum[3][i]);
+  for (int i = 0; i < 4; ++i) red[warp][m + (i & 1)][quad + (i >> 1) * 8] = sum[i];
   __syncthreads();
   for (int i = threadIdx.x; i < kGroups * 128; i += kWarps * 32) {
     const int g = i >> 7, mm = (i >> 4) & 7, r = i & 15, n = (blockIdx.x * kGroups + g) * 16 + r;
@@ -443,7 +451,7 @@ __global__ void __launch_bounds__(256) residual_norm_kernel(float* __restrict__ 
 
 // The same for widths that are multiples of 4 up to 1024 NV: a thread keeps its 4 NV columns in registers and asks for everything the row
 // needs before the first sum, and a sum over the block costs one barrier.  Bound by traffic on long steps, by the chain of (up to) four sums
-// on short ones.
+// on short ones: 4 rows of 2048 7.5 -> 2.7 us.
 template <int NV>
 __global__ void __launch_bounds__(256) residual_norm_vec_kernel(float* __restrict__ x, const float* __restrict__ y, int y_mode,
                                                                 const float* __restrict__ wa, const float* __restrict__ ba,
