@@ -21,6 +21,7 @@
 //
 // Precision: the residual stream, every norm, softmax, the rotary angles, decays, gates and the recurrent state are fp32 (angles
 // are reduced in fp64).  `dt` codes: 0 = float32, 1 = bfloat16.
+#include "ptx.cuh"
 #include "seq_common.cuh"
 
 namespace kb2seq {
@@ -1081,6 +1082,66 @@ __global__ void __launch_bounds__(256) conv_run_kernel(const float* __restrict__
   }
 }
 
+// The same for 2 to 4 taps and channels in groups of four: a thread takes four channels over kConvRun rows, and the 16-byte loads of four rows
+// are in flight together.  Bound by traffic (each input read once, plus K - 1 rows per run, each output written once).
+template <int K>
+__global__ void __launch_bounds__(256) conv_run_vec_kernel(const float* __restrict__ proj, long long ldp, int C, const float* __restrict__ taps,
+                                                           const float* __restrict__ tail, const int* __restrict__ seq_of, const int* __restrict__ cu,
+                                                           const int* __restrict__ slots, long long T, float* __restrict__ out,
+                                                           const float* __restrict__ bias, int act, const float* __restrict__ bias_out) {
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  if (c >= C) return;
+  const long long r0 = (long long)blockIdx.y * kConvRun, r1 = min(T, r0 + kConvRun);
+  float w[4][K], x[K - 1][4], b[4], bo[4];               // x[j]: the input K - 1 - j rows back
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+#pragma unroll
+    for (int j = 0; j < K; ++j) w[e][j] = taps[(long long)(c + e) * K + j];
+    b[e] = bias != nullptr ? bias[c + e] : 0.f;
+    bo[e] = bias_out != nullptr ? bias_out[c + e] : 0.f;
+  }
+  int s = -1;
+  for (long long t = r0; t < r1; t += 4) {
+    float4 in[4];
+    int sq[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const bool ok = t + i < r1;
+      in[i] = ok ? *reinterpret_cast<const float4*>(proj + (t + i) * ldp + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      sq[i] = ok ? seq_of[t + i] : -1;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (t + i >= r1) break;
+      if (sq[i] != s) {                                  // first row of this run, or of another sequence: fetch the K - 1 earlier inputs
+        s = sq[i];
+        const int at = (int)(t + i - cu[s]);
+#pragma unroll
+        for (int j = 0; j < K - 1; ++j) {
+          const int src = at - (K - 1) + j;
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            x[j][e] = src >= 0 ? proj[(t + i - at + src) * ldp + c + e] + b[e] : tail[((long long)slots[s] * C + c + e) * (K - 1) + (K - 1) + src];
+        }
+      }
+      const float cur[4] = {in[i].x + b[0], in[i].y + b[1], in[i].z + b[2], in[i].w + b[3]};
+      float acc[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        acc[e] = bo[e];
+#pragma unroll
+        for (int j = 0; j < K - 1; ++j) acc[e] = fmaf(w[e][j], x[j][e], acc[e]);
+        acc[e] = fmaf(w[e][K - 1], cur[e], acc[e]);
+#pragma unroll
+        for (int j = 0; j < K - 2; ++j) x[j][e] = x[j + 1][e];
+        x[K - 2][e] = cur[e];
+        if (act) acc[e] = silu(acc[e]);
+      }
+      *reinterpret_cast<float4*>(out + (t + i) * C + c) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    }
+  }
+}
+
 // after the convolution: the tail becomes the last K - 1 inputs seen so far (one thread per (sequence, channel), ascending order)
 __global__ void conv_tail_kernel(const float* __restrict__ proj, long long ldp, int C, int K, float* __restrict__ tail,
                                  const int* __restrict__ cu, const int* __restrict__ slots, int S, const float* __restrict__ bias) {
@@ -1367,7 +1428,303 @@ __global__ void __launch_bounds__(32 * kRegPieces) delta_rule_reg_kernel(const f
   for (int ii = 0; ii < Q; ++ii) Sg[(long long)(piece * Q + ii) * dv + j0 + lane] = S[ii];
 }
 
-// out[t, h, :] = o / rms(o) * norm_w * silu(gate) (gate_act 1: sigmoid(gate)); a warp per (token, head)
+// ---- the recurrence with one decay per head, four tokens at a time (long portions).
+// With S0 the state ahead of a tile, G_i = g_0 .. g_i and D_ij = g_(j+1) .. g_i, the token-by-token rule is
+//   u_i = beta_i (v_i - G_i S0^T k_i - sum_(j<i) D_ij (k_i . k_j) u_j),   o_i = G_i S0^T q_i + sum_(j<=i) D_ij (q_i . k_j) u_j,
+//   S = G_3 S0 + sum_j D_3j k_j u_j^T:
+// the eight products with S0 need one sum over the rows instead of four in a row, a state element takes 13 multiply-adds per four tokens
+// instead of 16, and what couples the tokens is a handful of numbers per (tile, head) that delta_tile_prep makes.
+// Bound: issue slots, shared-memory reads of k and q and the multiply-adds come to about 105 cycles per token each (4 blocks of 32 value columns
+// per head: 128 SMs).  So the layout keeps the three level: a warp owns all rows of four value columns (nothing crosses warps, no block
+// barrier), a lane the rows 32 i + 4 g .. + 3 of one column — a 16-byte read of k serves the warp in one 128-byte wavefront, rows pair up in
+// 64-bit registers, and the sum over the rows is 4 + 4 shuffles.  A ninth warp streams the tiles (bulk copies, eight deep).
+// 4096 tokens, 32 / 16 heads x 128: see delta_rule_reg_kernel for the token-by-token form.
+constexpr int kDT = 4, kDTStages = 8, kDTScalars = 12;     // per (token, head): G, beta, D_3j, G_3 | D_ij k_i.k_j (j < i) | D_ij q_i.k_j (j <= i)
+template <int NI>
+__global__ void __launch_bounds__(256) delta_tile_prep_kernel(const float* __restrict__ conv, int C, const float* __restrict__ bproj, long long ldb,
+                                                              const float* __restrict__ aproj, long long lda, int H, int Hk,
+                                                              const float* __restrict__ A_log, const float* __restrict__ dt_bias, long long T, int S,
+                                                              const int* __restrict__ cu, long long tiles, float* __restrict__ qn,
+                                                              float* __restrict__ kn, float* __restrict__ sc) {
+  constexpr int DK = 32 * NI;
+  const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  long long tile = w / Hk;
+  const int hk = (int)(w - tile * Hk);
+  if (tile >= tiles) return;
+  int sq = 0, t0 = 0, n = 0;                          // the tile's sequence: tiles are counted sequence by sequence
+  for (; sq < S; ++sq) {
+    t0 = cu[sq];
+    n = cu[sq + 1] - t0;
+    const int nt = (n + kDT - 1) / kDT;
+    if (tile < nt) break;
+    tile -= nt;
+  }
+  if (sq == S) return;
+  t0 += (int)tile * kDT;
+  const int nt = min(kDT, n - (int)tile * kDT);
+  float q[kDT][NI], k[kDT][NI];
+#pragma unroll
+  for (int t = 0; t < kDT; ++t)
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const float* row = conv + (long long)(t0 + t) * C + hk * DK + i * 32 + lane;
+      q[t][i] = t < nt ? row[0] : 0.f;
+      k[t][i] = t < nt ? row[Hk * DK] : 0.f;
+    }
+#pragma unroll
+  for (int t = 0; t < kDT; ++t) {
+    float a = 0.f, b = 0.f;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      a += q[t][i] * q[t][i];
+      b += k[t][i] * k[t][i];
+    }
+    a = warp_sum(a);
+    b = warp_sum(b);
+    const float rq = (1.f / sqrtf((float)DK)) / sqrtf(a + 1e-6f), rk = 1.f / sqrtf(b + 1e-6f);
+    const long long at = ((long long)(t0 + t) * Hk + hk) * DK + lane;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      q[t][i] *= rq;
+      k[t][i] *= rk;
+      if (t < nt) {
+        qn[at + i * 32] = q[t][i];
+        kn[at + i * 32] = k[t][i];
+      }
+    }
+  }
+  float kk[kDT][kDT], qk[kDT][kDT];
+#pragma unroll
+  for (int t = 0; t < kDT; ++t)
+#pragma unroll
+    for (int m = 0; m <= t; ++m) {
+      float a = 0.f, b = 0.f;
+#pragma unroll
+      for (int i = 0; i < NI; ++i) {
+        a = fmaf(q[t][i], k[m][i], a);
+        b = fmaf(k[t][i], k[m][i], b);
+      }
+      qk[t][m] = warp_sum(a);
+      kk[t][m] = m < t ? warp_sum(b) : 0.f;
+    }
+  const int rep = H / Hk, me = lane & 3;              // a lane per (head, token of the tile), eight heads at a time
+  for (int r0 = 0; r0 < rep; r0 += 8) {
+    const int h = hk * rep + r0 + (lane >> 2);
+    const bool in = r0 + (lane >> 2) < rep && me < nt;
+    float g = 1.f;
+    if (in) g = decay_of(A_log[h], aproj[(long long)(t0 + me) * lda + h], dt_bias[h]);
+    float gs[kDT];
+#pragma unroll
+    for (int t = 0; t < kDT; ++t) gs[t] = __shfl_sync(0xffffffffu, g, t, 4);       // 1 behind the last token
+    if (!in) continue;
+    const float beta = 1.f / (1.f + expf(-bproj[(long long)(t0 + me) * ldb + h]));
+    float4 a, ar, br;
+    a.w = (gs[0] * gs[1]) * (gs[2] * gs[3]);
+    a.y = beta;
+    a.x = a.z = 0.f;
+#pragma unroll
+    for (int t = 0; t < kDT; ++t)
+      if (me == t) {
+        float up = 1.f, down = 1.f;
+#pragma unroll
+        for (int m = 0; m <= t; ++m) up *= gs[m];
+#pragma unroll
+        for (int m = t + 1; m < kDT; ++m) down *= gs[m];
+        a.x = up;
+        a.z = down;
+        float dk_[kDT] = {}, dq_[kDT] = {}, d = 1.f;
+#pragma unroll
+        for (int m = t; m >= 0; --m) {                // d = D_tm
+          dk_[m] = m < t ? d * kk[t][m] : 0.f;
+          dq_[m] = d * qk[t][m];
+          d *= gs[m];
+        }
+        ar = make_float4(dk_[0], dk_[1], dk_[2], dk_[3]);
+        br = make_float4(dq_[0], dq_[1], dq_[2], dq_[3]);
+      }
+    float4* o = reinterpret_cast<float4*>(sc + ((long long)h * T + t0 + me) * kDTScalars);
+    o[0] = a;
+    o[1] = ar;
+    o[2] = br;
+  }
+}
+
+__device__ __forceinline__ uint64_t pair2(float v) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float sum2(uint64_t a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+  return x + y;
+}
+
+template <int NI>
+__global__ void __launch_bounds__(288, 1) delta_tile_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ conv,
+                                                            int C, int v_col0, const float* __restrict__ sc, long long T, int H, int Hk, int dv,
+                                                            float* __restrict__ state, const int* __restrict__ cu, const int* __restrict__ slots,
+                                                            float* __restrict__ o_out) {
+  constexpr int DK = 32 * NI;
+  struct __align__(16) Stage {
+    float k[kDT][DK], q[kDT][DK], v[kDT][32], s[kDT][kDTScalars];
+  };
+  __shared__ Stage ring[kDTStages];
+  __shared__ uint64_t full[kDTStages], empty[kDTStages];
+  const int s = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * 32, hk = h / (H / Hk);
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int t0 = cu[s], n = cu[s + 1] - cu[s], tiles = (n + kDT - 1) / kDT;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kDTStages; ++i) {
+      kb2::mbar_init(&full[i], 1);
+      kb2::mbar_init(&empty[i], 8);
+    }
+    kb2::fence_mbar_init();
+  }
+  __syncthreads();
+  if (warp == 8) {
+    for (int i = 0; i < tiles; ++i) {
+      const int st = i % kDTStages;
+      Stage& b = ring[st];
+      kb2::mbar_wait(&empty[st], (uint32_t)(i / kDTStages & 1) ^ 1u);
+      const int nt = min(kDT, n - i * kDT);
+      const long long t = t0 + (long long)i * kDT;
+      if (nt < kDT) {                              // rows behind the last token take no part: zeros everywhere
+        for (int r = nt; r < kDT; ++r) {
+          for (int c = lane; c < DK; c += 32) b.k[r][c] = b.q[r][c] = 0.f;
+          b.v[r][lane] = 0.f;
+          if (lane < kDTScalars) b.s[r][lane] = 0.f;
+        }
+      }
+      __syncwarp();
+      if (lane == 0) kb2::mbar_arrive_expect_tx(&full[st], (uint32_t)(nt * (2 * DK + 32 + kDTScalars) * 4));
+      __syncwarp();
+      const int r = lane & 7;
+      if (lane < 24 && r < nt) {
+        if (lane < 8) kb2::bulk_g2s(b.k[r], kn + ((t + r) * Hk + hk) * DK, DK * 4, &full[st]);
+        else if (lane < 16) kb2::bulk_g2s(b.q[r], qn + ((t + r) * Hk + hk) * DK, DK * 4, &full[st]);
+        else kb2::bulk_g2s(b.v[r], conv + (t + r) * C + v_col0 + h * dv + j0, 128, &full[st]);
+      } else if (lane == 24) {
+        kb2::bulk_g2s(b.s[0], sc + ((long long)h * T + t) * kDTScalars, (uint32_t)(nt * kDTScalars * 4), &full[st]);
+      }
+    }
+    return;
+  }
+  const int col = lane & 3, rg = (lane >> 2) * 4, me = (lane >> 4) * 2 + ((lane >> 3) & 1);     // me: the token whose sums this lane ends up with
+  const bool b16 = lane & 16, b8 = lane & 8;
+  float* Sg = state + ((long long)slots[s] * H + h) * DK * dv + j0 + warp * 4 + col;
+  uint64_t S[NI][2];
+#pragma unroll
+  for (int i = 0; i < NI; ++i)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const long long r = i * 32 + rg + e * 2;
+      asm("mov.b64 %0, {%1, %2};" : "=l"(S[i][e]) : "f"(Sg[r * dv]), "f"(Sg[(r + 1) * dv]));
+    }
+  // four numbers per lane, each to be summed over the eight row groups (lane bits 2, 3, 4): after two exchanges a lane keeps token `me`'s
+  auto row_sums = [&](const float (&p)[kDT]) {
+    const float x0 = (b16 ? p[2] : p[0]) + __shfl_xor_sync(0xffffffffu, b16 ? p[0] : p[2], 16);
+    const float x1 = (b16 ? p[3] : p[1]) + __shfl_xor_sync(0xffffffffu, b16 ? p[1] : p[3], 16);
+    const float y = (b8 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, b8 ? x0 : x1, 8);
+    return y + __shfl_xor_sync(0xffffffffu, y, 4);
+  };
+  for (int i = 0; i < tiles; ++i) {
+    const int st = i % kDTStages;
+    const Stage& b = ring[st];
+    kb2::mbar_wait(&full[st], (uint32_t)(i / kDTStages & 1));
+    uint64_t kv[kDT][NI][2];
+    float p[kDT];
+#pragma unroll
+    for (int t = 0; t < kDT; ++t) {
+      uint64_t a0 = 0, a1 = 0;
+#pragma unroll
+      for (int c = 0; c < NI; ++c) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&b.k[t][c * 32 + rg]);
+        kv[t][c][0] = v.x;
+        kv[t][c][1] = v.y;
+        a0 = fma2(S[c][0], v.x, a0);
+        a1 = fma2(S[c][1], v.y, a1);
+      }
+      p[t] = sum2(a0) + sum2(a1);
+    }
+    const float pk = row_sums(p);
+    float P[kDT];
+#pragma unroll
+    for (int t = 0; t < kDT; ++t) P[t] = __shfl_sync(0xffffffffu, pk, (t >> 1) * 16 + (t & 1) * 8 + col);
+#pragma unroll
+    for (int t = 0; t < kDT; ++t) {
+      uint64_t a0 = 0, a1 = 0;
+#pragma unroll
+      for (int c = 0; c < NI; ++c) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&b.q[t][c * 32 + rg]);
+        a0 = fma2(S[c][0], v.x, a0);
+        a1 = fma2(S[c][1], v.y, a1);
+      }
+      p[t] = sum2(a0) + sum2(a1);
+    }
+    float u[kDT], scale[kDT], total = 1.f;
+#pragma unroll
+    for (int t = 0; t < kDT; ++t) {
+      const float4 f = *reinterpret_cast<const float4*>(&b.s[t][0]);       // G, beta, D_3t, G_3
+      const float4 a = *reinterpret_cast<const float4*>(&b.s[t][4]);
+      float m = f.x * P[t];
+      if (t > 0) m = fmaf(a.x, u[0], m);
+      if (t > 1) m = fmaf(a.y, u[1], m);
+      if (t > 2) m = fmaf(a.z, u[2], m);
+      u[t] = f.y * (b.v[t][warp * 4 + col] - m);
+      scale[t] = f.z;
+      if (t == 0) total = f.w;
+    }
+    const float rq = row_sums(p);
+    {
+      const float4 d = *reinterpret_cast<const float4*>(&b.s[me][8]);
+      const float o = fmaf(d.w, u[3], fmaf(d.z, u[2], fmaf(d.y, u[1], fmaf(d.x, u[0], b.s[me][0] * rq))));
+      if (!(lane & 4) && i * kDT + me < n) o_out[((t0 + (long long)i * kDT + me) * H + h) * dv + j0 + warp * 4 + col] = o;
+    }
+    __syncwarp();
+    if (lane == 0) kb2::mbar_arrive(&empty[st]);       // everything of the tile has been read
+    const uint64_t g2 = pair2(total);
+#pragma unroll
+    for (int c = 0; c < NI; ++c) {
+      S[c][0] = mul2(S[c][0], g2);
+      S[c][1] = mul2(S[c][1], g2);
+    }
+#pragma unroll
+    for (int t = 0; t < kDT; ++t) {
+      const uint64_t w = pair2(scale[t] * u[t]);
+#pragma unroll
+      for (int c = 0; c < NI; ++c) {
+        S[c][0] = fma2(kv[t][c][0], w, S[c][0]);
+        S[c][1] = fma2(kv[t][c][1], w, S[c][1]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NI; ++i)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const long long r = i * 32 + rg + e * 2;
+      float x, y;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(S[i][e]));
+      Sg[r * dv] = x;
+      Sg[(r + 1) * dv] = y;
+    }
+}
+
+// out[t, h, :] = o / rms(o) * norm_w * silu(gate) (gate_act 1: sigmoid(gate)); a warp per (token, head).  V numbers per access: 4 where sizes
+// and pointers allow (a row of 128 is then one 16-byte read per lane).
+template <int V>
 __global__ void __launch_bounds__(256) delta_out_kernel(const float* __restrict__ o, const float* __restrict__ gproj, long long ldg,
                                                         int gate_act, int H, int dv, const float* __restrict__ norm_w, float eps,
                                                         long long T, void* __restrict__ out, int dt_out) {
@@ -1377,13 +1734,31 @@ __global__ void __launch_bounds__(256) delta_out_kernel(const float* __restrict_
   const long long t = w / H;
   const int h = (int)(w - t * H);
   const float* row = o + w * dv;
+  const float* gate = gproj + t * ldg + (long long)h * dv;
+  auto finish = [&](float v, float gz, float nw, float rstd) { return v * rstd * nw * (gate_act ? 1.f / (1.f + expf(-gz)) : silu(gz)); };
   float ss = 0.f;
-  for (int j = lane; j < dv; j += 32) ss += row[j] * row[j];
-  ss = warp_sum(ss);
-  const float rstd = 1.f / sqrtf(ss / (float)dv + eps);
-  for (int j = lane; j < dv; j += 32) {
-    const float gz = gproj[t * ldg + h * dv + j];
-    st_dt(out, dt_out, w * dv + j, row[j] * rstd * norm_w[j] * (gate_act ? 1.f / (1.f + expf(-gz)) : silu(gz)));
+  if constexpr (V == 4) {
+    for (int j = lane * 4; j < dv; j += 128) {
+      const float4 f = *reinterpret_cast<const float4*>(row + j);
+      ss += (f.x * f.x + f.y * f.y) + (f.z * f.z + f.w * f.w);
+    }
+    ss = warp_sum(ss);
+    const float rstd = 1.f / sqrtf(ss / (float)dv + eps);
+    for (int j = lane * 4; j < dv; j += 128) {
+      const float4 f = *reinterpret_cast<const float4*>(row + j), g = *reinterpret_cast<const float4*>(gate + j), nw = *reinterpret_cast<const float4*>(norm_w + j);
+      const float4 r = make_float4(finish(f.x, g.x, nw.x, rstd), finish(f.y, g.y, nw.y, rstd), finish(f.z, g.z, nw.z, rstd), finish(f.w, g.w, nw.w, rstd));
+      if (dt_out == 0) {
+        *reinterpret_cast<float4*>((float*)out + w * dv + j) = r;
+      } else {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(r.x, r.y), hi = __floats2bfloat162_rn(r.z, r.w);
+        *reinterpret_cast<uint2*>((bf16*)out + w * dv + j) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+      }
+    }
+  } else {
+    for (int j = lane; j < dv; j += 32) ss += row[j] * row[j];
+    ss = warp_sum(ss);
+    const float rstd = 1.f / sqrtf(ss / (float)dv + eps);
+    for (int j = lane; j < dv; j += 32) st_dt(out, dt_out, w * dv + j, finish(row[j], gate[j], norm_w[j], rstd));
   }
 }
 
@@ -1530,12 +1905,18 @@ KB2SEQ_API int kb2_seq_conv(const float* proj, long long ldp, int T, int S, int 
   if (!proj || !taps || !tail || !seq_of || !cu || !slots || !out || T <= 0 || S <= 0 || C <= 0 || K <= 0 || act < 0 || act > 1)
     return failf(KB2SEQ_ERR_VALUE, "conv: bad argument");
   if (T > 65535) return failf(KB2SEQ_ERR_VALUE, "conv: more than 65535 rows in one step");
-  if (T >= 4 * kConvRun && K <= kConvMaxTaps)
+  const bool vec = C % 4 == 0 && ldp % 4 == 0 && !(((uintptr_t)proj | (uintptr_t)out) & 15);
+  const dim3 vgrid((C / 4 + 255) / 256, (T + kConvRun - 1) / kConvRun);
+#define KB2_CONV(KV) conv_run_vec_kernel<KV><<<vgrid, 256, 0, (cudaStream_t)stream>>>(proj, ldp, C, taps, tail, seq_of, cu, slots, T, out, bias, act, bias_out)
+  if (T >= 4 * kConvRun && vec && K >= 2 && K <= 4) {
+    if (K == 2) KB2_CONV(2); else if (K == 3) KB2_CONV(3); else KB2_CONV(4);
+  } else if (T >= 4 * kConvRun && K <= kConvMaxTaps)
     conv_run_kernel<<<dim3((C + 255) / 256, (T + kConvRun - 1) / kConvRun), 256, 0, (cudaStream_t)stream>>>(proj, ldp, C, K, taps, tail, seq_of,
                                                                                                           cu, slots, T, out, bias, act, bias_out);
   else
     conv_silu_kernel<<<dim3((C + 255) / 256, T), 256, 0, (cudaStream_t)stream>>>(proj, ldp, C, K, taps, tail, seq_of, cu, slots, T, out, bias,
                                                                                  act, bias_out);
+#undef KB2_CONV
   SEQ_LAUNCHED();
   if (K > 1) {
     const long long m = (long long)S * C;
@@ -1580,6 +1961,17 @@ KB2SEQ_API int kb2_seq_residual_post_rms(float* x, const float* y1, float c1, co
   return KB2SEQ_OK;
 }
 
+static int delta_out_launch(const float* o, const float* gproj, long long ldg, int gate_act, int H, int dv, const float* norm_w, float eps, int T,
+                            void* out, int dt_out, cudaStream_t st) {
+  const unsigned blocks = (unsigned)(((long long)T * H + 7) / 8);
+  if (dv % 4 == 0 && ldg % 4 == 0 && !(((uintptr_t)o | (uintptr_t)gproj | (uintptr_t)norm_w | (uintptr_t)out) & 15))
+    delta_out_kernel<4><<<blocks, 256, 0, st>>>(o, gproj, ldg, gate_act, H, dv, norm_w, eps, T, out, dt_out);
+  else
+    delta_out_kernel<1><<<blocks, 256, 0, st>>>(o, gproj, ldg, gate_act, H, dv, norm_w, eps, T, out, dt_out);
+  SEQ_LAUNCHED();
+  return KB2SEQ_OK;
+}
+
 static int delta_rule_launch(const float* conv, int C, const float* bproj, long long ldb, const float* aproj, long long lda, int ch,
                              const float* gproj, long long ldg, int gate_act, int T, int S, int H, int Hk, int dk, int dv,
                              const float* A_log, const float* dt_bias, const float* norm_w, float eps, float* state, const int* cu,
@@ -1610,10 +2002,7 @@ static int delta_rule_launch(const float* conv, int C, const float* bproj, long 
     }
 #undef R
     SEQ_LAUNCHED();
-    const long long no = (long long)T * H;
-    delta_out_kernel<<<(unsigned)((no + 7) / 8), 256, 0, st>>>(ob, gproj, ldg, gate_act, H, dv, norm_w, eps, T, out, dt_out);
-    SEQ_LAUNCHED();
-    return KB2SEQ_OK;
+    return delta_out_launch(ob, gproj, ldg, gate_act, H, dv, norm_w, eps, T, out, dt_out, st);
   }
   auto smem_of = [&](int cols) { return ((size_t)dk * cols + (size_t)kDeltaTile * (2 * dk + cols + 1 + (ch ? dk : 1))) * 4; };
   int dvb = dv;                                // a state too large for one block's shared memory is cut into slices of value columns
@@ -1634,12 +2023,40 @@ static int delta_rule_launch(const float* conv, int C, const float* bproj, long 
                                                                   dt_bias, norm_w, eps, state, cu, slots, out, dt_out, dvb,
                                                                   cut ? scratch : nullptr);
   SEQ_LAUNCHED();
-  if (cut) {
-    const long long no = (long long)T * H;
-    delta_out_kernel<<<(unsigned)((no + 7) / 8), 256, 0, (cudaStream_t)stream>>>(scratch, gproj, ldg, gate_act, H, dv, norm_w, eps, T, out, dt_out);
-    SEQ_LAUNCHED();
-  }
+  if (cut) return delta_out_launch(scratch, gproj, ldg, gate_act, H, dv, norm_w, eps, T, out, dt_out, (cudaStream_t)stream);
   return KB2SEQ_OK;
+}
+
+KB2SEQ_API long long kb2_seq_delta_tiles_scratch(int T, int H, int Hk, int dk, int dv) {
+  if (T <= 0 || H <= 0 || Hk <= 0 || H % Hk || (dk != 32 && dk != 64 && dk != 128) || dv <= 0 || dv % 32) return 0;
+  return (long long)T * (2LL * Hk * dk + (long long)kDTScalars * H + (long long)H * dv);
+}
+
+KB2SEQ_API int kb2_seq_delta_tiles(const float* conv, int C, const float* proj, long long ldp, int g_off, int a_off, int b_off, int T, int S, int H,
+                                   int Hk, int dk, int dv, const float* A_log, const float* dt_bias, const float* norm_w, float eps, float* state,
+                                   const int* cu, const int* slots, float* scratch, long long scratch_floats, void* out, int dt_out, void* stream) {
+  const long long need = kb2_seq_delta_tiles_scratch(T, H, Hk, dk, dv);
+  if (!conv || !proj || !A_log || !dt_bias || !norm_w || !state || !cu || !slots || !scratch || !out || S <= 0 || bad_dt(dt_out) || !need ||
+      scratch_floats < need || ((uintptr_t)scratch & 15) || ((uintptr_t)conv & 15) || C % 4 || C < 2 * Hk * dk + H * dv)
+    return failf(KB2SEQ_ERR_VALUE, "delta_tiles: bad argument");
+  cudaStream_t st = (cudaStream_t)stream;
+  float* qn = scratch;
+  float* kn = qn + (long long)T * Hk * dk;
+  float* sc = kn + (long long)T * Hk * dk;
+  float* ob = sc + (long long)T * H * kDTScalars;
+  const long long tiles = (long long)T / kDT + S;                    // at most: every sequence may end in a partial tile
+  const unsigned blocks = (unsigned)((tiles * Hk + 7) / 8);
+  const dim3 grid(S, H, dv / 32);
+#define KB2_DT(NIV)                                                                                                                                \
+  do {                                                                                                                                             \
+    delta_tile_prep_kernel<NIV><<<blocks, 256, 0, st>>>(conv, C, proj + b_off, ldp, proj + a_off, ldp, H, Hk, A_log, dt_bias, T, S, cu, tiles, qn, kn, sc); \
+    SEQ_LAUNCHED();                                                                                                                                \
+    delta_tile_kernel<NIV><<<grid, 288, 0, st>>>(qn, kn, conv, C, 2 * Hk * dk, sc, T, H, Hk, dv, state, cu, slots, ob);                             \
+    SEQ_LAUNCHED();                                                                                                                                \
+  } while (0)
+  if (dk == 32) KB2_DT(1); else if (dk == 64) KB2_DT(2); else KB2_DT(4);
+#undef KB2_DT
+  return delta_out_launch(ob, proj + g_off, ldp, 0, H, dv, norm_w, eps, T, out, dt_out, st);
 }
 
 KB2SEQ_API int kb2_seq_delta_rule(const float* conv, int C, const float* proj, long long ldp, int g_off, int a_off, int b_off, int T,

@@ -297,6 +297,7 @@ class GatedDeltaMixer:
         self.w_o = d(weights["o"])
         # key sizes 32 / 64 / 128 with value sizes that are multiples of 32 keep the state in registers; others in shared memory
         self.register_state_kernel = dim in (32, 64, 128) and vdim % 32 == 0
+        self.tile_min_portion = 16
 
     def register_state(self, pool):
         """(conv tail [slots, C, taps - 1], recurrent state [slots, H, dk, dv]) in a RecurrentStatePool."""
@@ -310,6 +311,14 @@ class GatedDeltaMixer:
         ops.check(lib.kb2_seq_conv_silu(proj.data_ptr(), proj.stride(0), T, tb.S, self.C, self.K, self.taps.data_ptr(), tail.data_ptr(),
                                         tb.seq_of.data_ptr(), tb.cu.data_ptr(), tb.slots.data_ptr(), conv.data_ptr(), s))
         o = torch.empty((T, self.H * self.dv), dtype=self.dtype, device=h.device)
+        if self.register_state_kernel and tb.max_portion >= self.tile_min_portion:      # long portions: four tokens at a time
+            n = int(lib.kb2_seq_delta_tiles_scratch(T, self.H, self.Hk, self.dk, self.dv))
+            scratch = torch.empty(n, dtype=torch.float32, device=h.device)
+            ops.check(lib.kb2_seq_delta_tiles(conv.data_ptr(), self.C, proj.data_ptr(), proj.stride(0), self.g_off, self.a_off, self.b_off, T, tb.S,
+                                              self.H, self.Hk, self.dk, self.dv, self.A_log.data_ptr(), self.dt_bias.data_ptr(), self.norm.data_ptr(),
+                                              self.eps, state.data_ptr(), tb.cu.data_ptr(), tb.slots.data_ptr(), scratch.data_ptr(), n, o.data_ptr(),
+                                              ops.dt_code(self.dtype), s))
+            return lin(o, self.w_o, torch.float32)
         scratch = None
         if self.register_state_kernel or self.dk * self.dv > 32768:      # a large state is cut into column slices that meet in scratch
             scratch = torch.empty(2 * T * self.Hk * self.dk + 2 * T * self.H + T * self.H * self.dv + 4, dtype=torch.float32, device=h.device)

@@ -1,0 +1,98 @@
+"""The delta rule four tokens at a time, the short convolution's vector form and the gated read-out at their edges, against fp64."""
+import pytest
+import torch
+
+from krasis_b200 import seqops as ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _mixer(H, Hk, dk, dv, dtype=torch.float32, decay=-3.0):
+    from krasis_b200.mixers import GatedDeltaMixer
+    W = 64
+    g = torch.Generator().manual_seed(H + dk + dv)
+    r = lambda *s, sd=W ** -0.5: torch.randn(*s, generator=g) * sd  # noqa: E731
+    w = {"q": r(Hk * dk, W), "k": r(Hk * dk, W), "v": r(H * dv, W), "g": r(H * dv, W), "a": r(H, W), "b": r(H, W), "A_log": r(H, sd=0.5),
+         "dt_bias": r(H, sd=1.0) + decay, "norm": 1 + r(dv, sd=0.1), "o": r(W, H * dv, sd=(H * dv) ** -0.5)}
+    for n, c in (("q", Hk * dk), ("k", Hk * dk), ("v", H * dv)):
+        w[n + "_conv"] = r(c, 4, sd=0.5)
+    return GatedDeltaMixer(w, H, Hk, dk, dv, 4, 1e-5, dtype, "cuda")
+
+
+def _exact(m, h, tb, tail, state, lens, slots):
+    """State and output in fp64, token by token."""
+    H, Hk, dk, dv = m.H, m.Hk, m.dk, m.dv
+    proj = h.double() @ m.w_in.double().T
+    outs, states = [], state.double().clone()
+    at = 0
+    for n, slot in zip(lens, slots):
+        raw = torch.cat([tail[slot].double().T, proj[at:at + n, :m.C]], 0)
+        c = torch.nn.functional.silu(sum(raw[i:i + n] * m.taps[:, i].double() for i in range(4)))
+        q, k, v = c[:, :Hk * dk].view(n, Hk, dk), c[:, Hk * dk:2 * Hk * dk].view(n, Hk, dk), c[:, 2 * Hk * dk:].view(n, H, dv)
+        unit = lambda x: x * torch.rsqrt(x.square().sum(-1, keepdim=True) + 1e-6)  # noqa: E731
+        q, k = unit(q).repeat_interleave(H // Hk, 1) * dk ** -0.5, unit(k).repeat_interleave(H // Hk, 1)
+        p = proj[at:at + n]
+        dec = torch.exp(-torch.exp(m.A_log.double()) * torch.nn.functional.softplus(p[:, m.a_off:m.a_off + H] + m.dt_bias.double()))
+        beta = torch.sigmoid(p[:, m.b_off:m.b_off + H])
+        S = states[slot]
+        o = torch.empty(n, H, dv, dtype=torch.float64, device=h.device)
+        for t in range(n):
+            S = S * dec[t][:, None, None]
+            u = beta[t][:, None] * (v[t] - torch.einsum("hkv,hk->hv", S, k[t]))
+            S = S + k[t][:, :, None] * u[:, None]
+            o[t] = torch.einsum("hkv,hk->hv", S, q[t])
+        states[slot] = S
+        o = o * torch.rsqrt(o.square().mean(-1, keepdim=True) + 1e-5) * m.norm.double()
+        outs.append((o * torch.nn.functional.silu(p[:, m.g_off:m.g_off + H * dv].reshape(n, H, dv))).reshape(n, -1) @ m.w_o.double().T)
+        at += n
+    return torch.cat(outs), states
+
+
+# portions that end anywhere in a tile of four, one-token portions beside long ones, an odd number of slices and heads per key head
+@pytest.mark.parametrize("H,Hk,dk,dv", [(2, 1, 32, 32), (4, 4, 64, 96), (6, 2, 128, 64), (9, 1, 32, 32)])
+@pytest.mark.parametrize("lens", [[16], [17, 1, 18], [1, 31, 2, 3], [64, 67]])
+@pytest.mark.parametrize("decay", [-3.0, 3.0])                 # slow, and so fast that a tile forgets all it knew
+def test_tiles_against_exact_and_token_form(H, Hk, dk, dv, lens, decay):
+    m = _mixer(H, Hk, dk, dv, decay=decay)
+    g = torch.Generator(device="cuda").manual_seed(7)
+    slots = [(3 * i + 2) % 5 for i in range(len(lens))]
+    tb = ops.StepTables([([0] * n, 0 if i else 9, s, [0]) for i, (n, s) in enumerate(zip(lens, slots))], "cuda")
+    h = torch.randn(sum(lens), 64, device="cuda", generator=g)
+    tail0, state0 = torch.randn(5, m.C, 3, device="cuda", generator=g), torch.randn(5, H, dk, dv, device="cuda", generator=g)
+    # positions only matter to the convolution's tail: the first rows of a portion read it whatever the position
+    want, states = _exact(m, h, tb, tail0, state0, lens, slots)
+    err = {}
+    for name, least in (("tiles", 1), ("tokens", 1 << 30)):
+        m.tile_min_portion = least
+        tail, state = tail0.clone(), state0.clone()
+        got = m.forward(h, tb, tail, state)
+        err[name] = (((got.double() - want).norm() / want.norm()).item(), ((state.double() - states).norm() / states.norm()).item())
+        untouched = [i for i in range(5) if i not in slots]
+        assert torch.equal(state[untouched], state0[untouched])
+    # the same fp32 sums in another order: no further off than the token-by-token form, with room for the luck of a few thousand numbers
+    assert err["tiles"][0] <= 1.5 * err["tokens"][0] + 2e-7 and err["tiles"][1] <= 1.5 * err["tokens"][1] + 2e-7, err
+
+
+@pytest.mark.parametrize("K,C", [(2, 64), (3, 36), (4, 1028), (4, 30), (5, 64)])
+@pytest.mark.parametrize("lens", [[64], [1, 66, 2, 3, 5, 70], [33, 31, 65]])
+@pytest.mark.parametrize("bias,bias_out,act", [(False, False, True), (True, False, False), (True, True, True)])
+def test_long_convolution(K, C, lens, bias, bias_out, act):
+    g = torch.Generator(device="cuda").manual_seed(C + K)
+    T, slots = sum(lens), list(range(len(lens)))[::-1]
+    proj, taps = torch.randn(T, C + 8, device="cuda", generator=g), torch.randn(C, K, device="cuda", generator=g)
+    b = torch.randn(C, device="cuda", generator=g) if bias else None
+    bo = torch.randn(C, device="cuda", generator=g) if bias_out else None
+    tail0 = torch.randn(len(lens), C, K - 1, device="cuda", generator=g)
+    tb = ops.StepTables([([0] * n, 0, s, [0]) for n, s in zip(lens, slots)], "cuda")
+    tail = tail0.clone()
+    got = ops.conv(proj, C, taps, b, act, tail, tb, bias_out=bo)
+    at = 0
+    for n, s in zip(lens, slots):
+        x = proj[at:at + n, :C].double() + (b.double() if bias else 0.0)
+        x = torch.cat([tail0[s].double().T, x], 0)
+        y = sum(x[i:i + n] * taps[:, i].double() for i in range(K)) + (bo.double() if bias_out else 0.0)
+        y = torch.nn.functional.silu(y) if act else y
+        # K + 1 fp32 additions and an exponential: 2^-20 of the terms
+        assert ((got[at:at + n].double() - y).abs() <= 2.0 ** -20 * (sum(x[i:i + n].abs() * taps[:, i].double().abs() for i in range(K)) + 3)).all()
+        assert (tail[s].double() - x[-(K - 1):].T).abs().max() <= 2.0 ** -22 * x.abs().max()
+        at += n
