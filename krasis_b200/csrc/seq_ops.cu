@@ -1428,30 +1428,55 @@ __global__ void __launch_bounds__(32 * kRegPieces) delta_rule_reg_kernel(const f
   for (int ii = 0; ii < Q; ++ii) Sg[(long long)(piece * Q + ii) * dv + j0 + lane] = S[ii];
 }
 
-// ---- the recurrence with one decay per head, four tokens at a time (long portions).
+// ---- the recurrence with one decay per head, eight tokens at a time on the warp-level tensor instructions (long portions).
 // With S0 the state ahead of a tile, G_i = g_0 .. g_i and D_ij = g_(j+1) .. g_i, the token-by-token rule is
 //   u_i = beta_i (v_i - G_i S0^T k_i - sum_(j<i) D_ij (k_i . k_j) u_j),   o_i = G_i S0^T q_i + sum_(j<=i) D_ij (q_i . k_j) u_j,
-//   S = G_3 S0 + sum_j D_3j k_j u_j^T:
-// the eight products with S0 need one sum over the rows instead of four in a row, a state element takes 13 multiply-adds per four tokens
-// instead of 16, and what couples the tokens is a handful of numbers per (tile, head) that delta_tile_prep makes.
-// Bound: issue slots, shared-memory reads of k and q and the multiply-adds come to about 105 cycles per token each (4 blocks of 32 value columns
-// per head: 128 SMs).  So the layout keeps the three level: a warp owns all rows of four value columns (nothing crosses warps, no block
-// barrier), a lane the rows 32 i + 4 g .. + 3 of one column — a 16-byte read of k serves the warp in one 128-byte wavefront, rows pair up in
-// 64-bit registers, and the sum over the rows is 4 + 4 shuffles.  A ninth warp streams the tiles (bulk copies, eight deep).
-// 4096 tokens, 32 / 16 heads x 128: see delta_rule_reg_kernel for the token-by-token form.
-constexpr int kDT = 4, kDTStages = 8, kDTScalars = 12;     // per (token, head): G, beta, D_3j, G_3 | D_ij k_i.k_j (j < i) | D_ij q_i.k_j (j <= i)
+//   S = G_7 S0 + sum_j D_7j k_j u_j^T:
+// two small products with the state per tile, one sum over its rows instead of eight in a row, and 64 numbers per (tile, head) that couple the
+// tokens, made ahead for all tiles at once (delta_tile_prep).  Everything stays at fp32 grade: the operands of the products go in as three
+// bf16 parts each (24 bits; six of nine products, the rest is below 2^-26), tensor sums run over 32 rows or 8 tokens and start from zero, and
+// the state itself is updated by fp32 multiply-adds.
+// Bound: the chain of a tile.  The token-by-token form (delta_rule_reg) spends 510 cycles per token on shared-memory broadcasts and a block
+// barrier; a form with four tokens per tile on packed FMAs 394, because a 16-byte shared-memory read takes four passes however many lanes
+// share an address.  Here a warp keeps 16 value columns x 32 rows as accumulator fragments, which are the operand fragments of the next
+// tile's product as they stand; k and q arrive as ready images (one bulk copy per tile, ahead of time) and enter through ldmatrix, plain for
+// S0^T k and transposed for k u^T.  The DK / 32 warps of a column group meet once per tile and then each solve the eight steps by themselves.
+constexpr int kDT = 8, kDTStages = 4, kDTScalars = 20;     // per (token, head): G, beta, D_7j, G_7 | D_ij k_i.k_j (j < i) | D_ij q_i.k_j (j <= i)
+template <int NI> struct DeltaTile {
+  static constexpr int DK = 32 * NI, kPitch = DK + 8;      // bf16 row pitch: 16 bytes more, so that the eight rows of an ldmatrix do not collide
+  static constexpr int kPart = 2 * kDT * kPitch;           // bf16 of one part: k rows, then q rows
+  static constexpr int kImage = 3 * kPart;                 // bf16 of a (tile, key head): hi, mid, lo
+  static constexpr int kImageBytes = kImage * 2, kScalarBytes = kDT * kDTScalars * 4, kVBytes = kDT * 32 * 4;
+  static constexpr int kStageBytes = kImageBytes + kVBytes + kScalarBytes;
+  static constexpr int kRedFloats = 2 * 2 * NI * 16 * 20;  // [buffer][column group][row piece][column][16 products + pad]
+  static constexpr int kUFloats = 2 * NI * 16 * 12;        // [warp][column][8 tokens + pad]
+  static constexpr int kSmem = kDTStages * kStageBytes + (kRedFloats + kUFloats) * 4 + 2 * kDTStages * 8;
+  static_assert(kImageBytes % 16 == 0 && kStageBytes % 16 == 0, "bulk copies");
+};
+
+// fp32 pair -> three words of bf16 pairs whose sums they are, exact to 24 bits (3.39e38 and more becomes NaN; in the recurrence an infinity
+// does one token later)
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t (&p)[3]) {
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p[0]) : "f"(y), "f"(x));
+  const float rx = x - __uint_as_float(p[0] << 16), ry = y - __uint_as_float(p[0] & 0xFFFF0000u);
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p[1]) : "f"(ry), "f"(rx));
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p[2]) : "f"(ry - __uint_as_float(p[1] & 0xFFFF0000u)), "f"(rx - __uint_as_float(p[1] << 16)));
+}
+
 template <int NI>
 __global__ void __launch_bounds__(256) delta_tile_prep_kernel(const float* __restrict__ conv, int C, const float* __restrict__ bproj, long long ldb,
                                                               const float* __restrict__ aproj, long long lda, int H, int Hk,
-                                                              const float* __restrict__ A_log, const float* __restrict__ dt_bias, long long T, int S,
-                                                              const int* __restrict__ cu, long long tiles, float* __restrict__ qn,
-                                                              float* __restrict__ kn, float* __restrict__ sc) {
-  constexpr int DK = 32 * NI;
+                                                              const float* __restrict__ A_log, const float* __restrict__ dt_bias, int S,
+                                                              const int* __restrict__ cu, long long tiles, bf16* __restrict__ image,
+                                                              float* __restrict__ sc) {
+  using D = DeltaTile<NI>;
+  constexpr int DK = D::DK;
   const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  long long tile = w / Hk;
-  const int hk = (int)(w - tile * Hk);
-  if (tile >= tiles) return;
+  const long long flat = w / Hk;
+  const int hk = (int)(w - flat * Hk);
+  if (flat >= tiles) return;
+  long long tile = flat;
   int sq = 0, t0 = 0, n = 0;                          // the tile's sequence: tiles are counted sequence by sequence
   for (; sq < S; ++sq) {
     t0 = cu[sq];
@@ -1463,15 +1488,34 @@ __global__ void __launch_bounds__(256) delta_tile_prep_kernel(const float* __res
   if (sq == S) return;
   t0 += (int)tile * kDT;
   const int nt = min(kDT, n - (int)tile * kDT);
-  float q[kDT][NI], k[kDT][NI];
+  float q[kDT][NI], k[kDT][NI];                       // a lane's NI neighbouring numbers of every row
 #pragma unroll
   for (int t = 0; t < kDT; ++t)
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
-      const float* row = conv + (long long)(t0 + t) * C + hk * DK + i * 32 + lane;
+      const float* row = conv + (long long)(t0 + t) * C + hk * DK + lane * NI + i;
       q[t][i] = t < nt ? row[0] : 0.f;
       k[t][i] = t < nt ? row[Hk * DK] : 0.f;
     }
+  bf16* img = image + (flat * Hk + hk) * D::kImage;
+  auto store = [&](bf16* at, const float (&v)[NI]) {  // the three parts of a row, behind the last token zeros
+    if constexpr (NI == 1) {
+      const float other = __shfl_down_sync(0xffffffffu, v[0], 1);
+      uint32_t p[3];
+      split_pair(v[0], other, p);
+      if (!(lane & 1))
+#pragma unroll
+        for (int c = 0; c < 3; ++c) *reinterpret_cast<uint32_t*>(at + c * D::kPart + lane) = p[c];
+    } else {
+#pragma unroll
+      for (int i = 0; i < NI; i += 2) {
+        uint32_t p[3];
+        split_pair(v[i], v[i + 1], p);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) *reinterpret_cast<uint32_t*>(at + c * D::kPart + lane * NI + i) = p[c];
+      }
+    }
+  };
 #pragma unroll
   for (int t = 0; t < kDT; ++t) {
     float a = 0.f, b = 0.f;
@@ -1483,243 +1527,249 @@ __global__ void __launch_bounds__(256) delta_tile_prep_kernel(const float* __res
     a = warp_sum(a);
     b = warp_sum(b);
     const float rq = (1.f / sqrtf((float)DK)) / sqrtf(a + 1e-6f), rk = 1.f / sqrtf(b + 1e-6f);
-    const long long at = ((long long)(t0 + t) * Hk + hk) * DK + lane;
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
       q[t][i] *= rq;
       k[t][i] *= rk;
-      if (t < nt) {
-        qn[at + i * 32] = q[t][i];
-        kn[at + i * 32] = k[t][i];
-      }
     }
+    store(img + t * D::kPitch, k[t]);
+    store(img + (kDT + t) * D::kPitch, q[t]);
   }
-  float kk[kDT][kDT], qk[kDT][kDT];
-#pragma unroll
-  for (int t = 0; t < kDT; ++t)
-#pragma unroll
-    for (int m = 0; m <= t; ++m) {
-      float a = 0.f, b = 0.f;
-#pragma unroll
-      for (int i = 0; i < NI; ++i) {
-        a = fmaf(q[t][i], k[m][i], a);
-        b = fmaf(k[t][i], k[m][i], b);
-      }
-      qk[t][m] = warp_sum(a);
-      kk[t][m] = m < t ? warp_sum(b) : 0.f;
+  const int rep = H / Hk, me = lane & 7;              // a lane per (head, token of the tile), four heads at a time
+  for (int r0 = 0; r0 < rep; r0 += 4) {
+    const int h = hk * rep + r0 + (lane >> 3);
+    const bool head = r0 + (lane >> 3) < rep;
+    float g = 1.f, beta = 0.f;
+    if (head && me < nt) {
+      g = decay_of(A_log[h], aproj[(long long)(t0 + me) * lda + h], dt_bias[h]);
+      beta = 1.f / (1.f + expf(-bproj[(long long)(t0 + me) * ldb + h]));
     }
-  const int rep = H / Hk, me = lane & 3;              // a lane per (head, token of the tile), eight heads at a time
-  for (int r0 = 0; r0 < rep; r0 += 8) {
-    const int h = hk * rep + r0 + (lane >> 2);
-    const bool in = r0 + (lane >> 2) < rep && me < nt;
-    float g = 1.f;
-    if (in) g = decay_of(A_log[h], aproj[(long long)(t0 + me) * lda + h], dt_bias[h]);
     float gs[kDT];
 #pragma unroll
-    for (int t = 0; t < kDT; ++t) gs[t] = __shfl_sync(0xffffffffu, g, t, 4);       // 1 behind the last token
-    if (!in) continue;
-    const float beta = 1.f / (1.f + expf(-bproj[(long long)(t0 + me) * ldb + h]));
-    float4 a, ar, br;
-    a.w = (gs[0] * gs[1]) * (gs[2] * gs[3]);
-    a.y = beta;
-    a.x = a.z = 0.f;
+    for (int t = 0; t < kDT; ++t) gs[t] = __shfl_sync(0xffffffffu, g, t, 8);       // 1 behind the last token
+    float up = 1.f, down = 1.f, all = 1.f, d = 1.f, row[2][kDT];                   // d: D_me,j for the j at hand, from j = 7 down
 #pragma unroll
-    for (int t = 0; t < kDT; ++t)
-      if (me == t) {
-        float up = 1.f, down = 1.f;
+    for (int t = 0; t < kDT; ++t) {
+      all *= gs[t];
+      if (t <= me) up *= gs[t];
+      if (t > me) down *= gs[t];
+    }
 #pragma unroll
-        for (int m = 0; m <= t; ++m) up *= gs[m];
+    for (int j = kDT - 1; j >= 0; --j) {
+      float kk = 0.f, qk = 0.f;                       // k_me . k_j and q_me . k_j: all pairs of the tile, of which a lane keeps its own row
 #pragma unroll
-        for (int m = t + 1; m < kDT; ++m) down *= gs[m];
-        a.x = up;
-        a.z = down;
-        float dk_[kDT] = {}, dq_[kDT] = {}, d = 1.f;
+      for (int t = 0; t < kDT; ++t) {
+        if (t < j) continue;
+        float a = 0.f, b = 0.f;
 #pragma unroll
-        for (int m = t; m >= 0; --m) {                // d = D_tm
-          dk_[m] = m < t ? d * kk[t][m] : 0.f;
-          dq_[m] = d * qk[t][m];
-          d *= gs[m];
+        for (int i = 0; i < NI; ++i) {
+          a = fmaf(k[t][i], k[j][i], a);
+          b = fmaf(q[t][i], k[j][i], b);
         }
-        ar = make_float4(dk_[0], dk_[1], dk_[2], dk_[3]);
-        br = make_float4(dq_[0], dq_[1], dq_[2], dq_[3]);
+        b = warp_sum(b);
+        if (t > j) a = warp_sum(a);
+        if (me == t) {
+          kk = t > j ? a : 0.f;
+          qk = b;
+        }
       }
-    float4* o = reinterpret_cast<float4*>(sc + ((long long)h * T + t0 + me) * kDTScalars);
-    o[0] = a;
-    o[1] = ar;
-    o[2] = br;
+      row[0][j] = j < me ? d * kk : 0.f;
+      row[1][j] = j <= me ? d * qk : 0.f;
+      if (j <= me) d *= gs[j];
+    }
+    if (!head) continue;
+    float4* o = reinterpret_cast<float4*>(sc + ((flat * H + h) * kDT + me) * kDTScalars);
+    const bool in = me < nt;                          // tokens behind the last one take no part
+    o[0] = make_float4(in ? up : 0.f, beta, in ? down : 0.f, all);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      o[1 + 2 * c] = in ? make_float4(row[c][0], row[c][1], row[c][2], row[c][3]) : make_float4(0.f, 0.f, 0.f, 0.f);
+      o[2 + 2 * c] = in ? make_float4(row[c][4], row[c][5], row[c][6], row[c][7]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
   }
 }
 
-__device__ __forceinline__ uint64_t pair2(float v) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
-  return r;
+__device__ __forceinline__ void mma1688(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a0), "r"(a1), "r"(b0));
 }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ float sum2(uint64_t a) {
-  float x, y;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
-  return x + y;
+template <bool kTrans> __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const void* row) {
+  const uint32_t at = (uint32_t)__cvta_generic_to_shared(row);
+  if constexpr (kTrans)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
 }
 
+// A block: 32 value columns of a (sequence, head) as two groups of 16, NI warps per group (32 rows each), and a warp that streams the tiles.
 template <int NI>
-__global__ void __launch_bounds__(288, 1) delta_tile_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ conv,
-                                                            int C, int v_col0, const float* __restrict__ sc, long long T, int H, int Hk, int dv,
-                                                            float* __restrict__ state, const int* __restrict__ cu, const int* __restrict__ slots,
-                                                            float* __restrict__ o_out) {
-  constexpr int DK = 32 * NI;
-  struct __align__(16) Stage {
-    float k[kDT][DK], q[kDT][DK], v[kDT][32], s[kDT][kDTScalars];
-  };
-  __shared__ Stage ring[kDTStages];
-  __shared__ uint64_t full[kDTStages], empty[kDTStages];
+__global__ void __launch_bounds__(64 * NI + 32, 1) delta_tile_kernel(const bf16* __restrict__ image, const float* __restrict__ conv, int C, int v_col0,
+                                                                     const float* __restrict__ sc, int H, int Hk, int dv, float* __restrict__ state,
+                                                                     const int* __restrict__ cu, const int* __restrict__ slots, float* __restrict__ o_out) {
+  using D = DeltaTile<NI>;
+  extern __shared__ __align__(128) uint8_t tsm[];
+  float* red = reinterpret_cast<float*>(tsm + kDTStages * D::kStageBytes);
+  float* ubuf = red + D::kRedFloats;
+  uint64_t* full = reinterpret_cast<uint64_t*>(ubuf + D::kUFloats);
+  uint64_t* empty = full + kDTStages;
   const int s = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * 32, hk = h / (H / Hk);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int t0 = cu[s], n = cu[s + 1] - cu[s], tiles = (n + kDT - 1) / kDT;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kDTStages; ++i) {
       kb2::mbar_init(&full[i], 1);
-      kb2::mbar_init(&empty[i], 8);
+      kb2::mbar_init(&empty[i], 2 * NI);
     }
     kb2::fence_mbar_init();
   }
   __syncthreads();
-  if (warp == 8) {
+  if (warp == 2 * NI) {
+    long long first = 0;                           // the sequence's tiles come after those of the sequences before it
+    for (int i = 0; i < s; ++i) first += (cu[i + 1] - cu[i] + kDT - 1) / kDT;
     for (int i = 0; i < tiles; ++i) {
       const int st = i % kDTStages;
-      Stage& b = ring[st];
+      uint8_t* b = tsm + st * D::kStageBytes;
       kb2::mbar_wait(&empty[st], (uint32_t)(i / kDTStages & 1) ^ 1u);
       const int nt = min(kDT, n - i * kDT);
       const long long t = t0 + (long long)i * kDT;
-      if (nt < kDT) {                              // rows behind the last token take no part: zeros everywhere
-        for (int r = nt; r < kDT; ++r) {
-          for (int c = lane; c < DK; c += 32) b.k[r][c] = b.q[r][c] = 0.f;
-          b.v[r][lane] = 0.f;
-          if (lane < kDTScalars) b.s[r][lane] = 0.f;
-        }
-      }
+      for (int r = nt; r < kDT; ++r) reinterpret_cast<float*>(b + D::kImageBytes)[r * 32 + lane] = 0.f;      // values behind the last token
       __syncwarp();
-      if (lane == 0) kb2::mbar_arrive_expect_tx(&full[st], (uint32_t)(nt * (2 * DK + 32 + kDTScalars) * 4));
+      if (lane == 0) kb2::mbar_arrive_expect_tx(&full[st], (uint32_t)(D::kImageBytes + D::kScalarBytes + nt * 128));
       __syncwarp();
-      const int r = lane & 7;
-      if (lane < 24 && r < nt) {
-        if (lane < 8) kb2::bulk_g2s(b.k[r], kn + ((t + r) * Hk + hk) * DK, DK * 4, &full[st]);
-        else if (lane < 16) kb2::bulk_g2s(b.q[r], qn + ((t + r) * Hk + hk) * DK, DK * 4, &full[st]);
-        else kb2::bulk_g2s(b.v[r], conv + (t + r) * C + v_col0 + h * dv + j0, 128, &full[st]);
-      } else if (lane == 24) {
-        kb2::bulk_g2s(b.s[0], sc + ((long long)h * T + t) * kDTScalars, (uint32_t)(nt * kDTScalars * 4), &full[st]);
-      }
+      if (lane < nt) kb2::bulk_g2s(b + D::kImageBytes + lane * 128, conv + (t + lane) * C + v_col0 + h * dv + j0, 128, &full[st]);
+      else if (lane == 8) kb2::bulk_g2s(b, image + ((first + i) * Hk + hk) * D::kImage, D::kImageBytes, &full[st]);
+      else if (lane == 9) kb2::bulk_g2s(b + D::kImageBytes + D::kVBytes, sc + ((first + i) * H + h) * kDT * kDTScalars, D::kScalarBytes, &full[st]);
     }
     return;
   }
-  const int col = lane & 3, rg = (lane >> 2) * 4, me = (lane >> 4) * 2 + ((lane >> 3) & 1);     // me: the token whose sums this lane ends up with
-  const bool b16 = lane & 16, b8 = lane & 8;
-  float* Sg = state + ((long long)slots[s] * H + h) * DK * dv + j0 + warp * 4 + col;
-  uint64_t S[NI][2];
+  const int cg = warp / NI, piece = warp % NI, quad = lane >> 2, pair = (lane & 3) * 2;      // fragment: columns quad, quad + 8; rows pair, pair + 1
+  float* Sg = state + ((long long)slots[s] * H + h) * D::DK * dv + (long long)piece * 32 * dv + j0 + cg * 16;
+  float S[4][4];                                   // [eight rows][column quad: 2 rows, column quad + 8: 2 rows]
 #pragma unroll
-  for (int i = 0; i < NI; ++i)
+  for (int r = 0; r < 4; ++r)
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const long long r = i * 32 + rg + e * 2;
-      asm("mov.b64 %0, {%1, %2};" : "=l"(S[i][e]) : "f"(Sg[r * dv]), "f"(Sg[(r + 1) * dv]));
-    }
-  // four numbers per lane, each to be summed over the eight row groups (lane bits 2, 3, 4): after two exchanges a lane keeps token `me`'s
-  auto row_sums = [&](const float (&p)[kDT]) {
-    const float x0 = (b16 ? p[2] : p[0]) + __shfl_xor_sync(0xffffffffu, b16 ? p[0] : p[2], 16);
-    const float x1 = (b16 ? p[3] : p[1]) + __shfl_xor_sync(0xffffffffu, b16 ? p[1] : p[3], 16);
-    const float y = (b8 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, b8 ? x0 : x1, 8);
-    return y + __shfl_xor_sync(0xffffffffu, y, 4);
-  };
+    for (int e = 0; e < 4; ++e) S[r][e] = Sg[(long long)(r * 8 + pair + (e & 1)) * dv + quad + (e >> 1) * 8];
+  const int col = lane & 15, half = lane >> 4;
+  float* myu = ubuf + warp * 16 * 12;
   for (int i = 0; i < tiles; ++i) {
     const int st = i % kDTStages;
-    const Stage& b = ring[st];
+    const uint8_t* b = tsm + st * D::kStageBytes;
+    const bf16* img = reinterpret_cast<const bf16*>(b);
+    const float* vs = reinterpret_cast<const float*>(b + D::kImageBytes);
+    const float* ss = vs + kDT * 32;
+    float* buf = red + (i & 1) * (2 * NI * 16 * 20) + cg * (NI * 16 * 20);
+    // S0^T [k | q] over the warp's 32 rows
+    uint32_t sp[2][3][4];                          // [16 rows][part][operand words]
+#pragma unroll
+    for (int kb = 0; kb < 2; ++kb)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        uint32_t p[3];
+        split_pair(S[2 * kb + (e >> 1)][(e & 1) * 2], S[2 * kb + (e >> 1)][(e & 1) * 2 + 1], p);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) sp[kb][c][e] = p[c];
+      }
     kb2::mbar_wait(&full[st], (uint32_t)(i / kDTStages & 1));
-    uint64_t kv[kDT][NI][2];
+    float dk[2][4] = {}, dq[2][4] = {};            // [big terms, small terms]
+#pragma unroll
+    for (int kb = 0; kb < 2; ++kb) {
+      uint32_t x[3][4];                            // k rows 0..7, k rows 8..15 of the block; q the same
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        ldmatrix4<false>(x[c], img + c * D::kPart + ((lane >> 4) * kDT + (lane & 7)) * D::kPitch + piece * 32 + kb * 16 + ((lane >> 3) & 1) * 8);
+      auto six = [&](float (&big)[4], float (&small)[4], int o) {
+        mma16816(small, sp[kb][2][0], sp[kb][2][1], sp[kb][2][2], sp[kb][2][3], x[0][o], x[0][o + 1]);
+        mma16816(big, sp[kb][0][0], sp[kb][0][1], sp[kb][0][2], sp[kb][0][3], x[0][o], x[0][o + 1]);
+        mma16816(small, sp[kb][0][0], sp[kb][0][1], sp[kb][0][2], sp[kb][0][3], x[2][o], x[2][o + 1]);
+        mma16816(small, sp[kb][1][0], sp[kb][1][1], sp[kb][1][2], sp[kb][1][3], x[1][o], x[1][o + 1]);
+        mma16816(small, sp[kb][0][0], sp[kb][0][1], sp[kb][0][2], sp[kb][0][3], x[1][o], x[1][o + 1]);
+        mma16816(small, sp[kb][1][0], sp[kb][1][1], sp[kb][1][2], sp[kb][1][3], x[0][o], x[0][o + 1]);
+      };
+      six(dk[0], dk[1], 0);
+      six(dq[0], dq[1], 2);
+    }
+    float* mine = buf + piece * 16 * 20;
+    *reinterpret_cast<float2*>(mine + quad * 20 + pair) = make_float2(dk[0][0] + dk[1][0], dk[0][1] + dk[1][1]);
+    *reinterpret_cast<float2*>(mine + (quad + 8) * 20 + pair) = make_float2(dk[0][2] + dk[1][2], dk[0][3] + dk[1][3]);
+    *reinterpret_cast<float2*>(mine + quad * 20 + 8 + pair) = make_float2(dq[0][0] + dq[1][0], dq[0][1] + dq[1][1]);
+    *reinterpret_cast<float2*>(mine + (quad + 8) * 20 + 8 + pair) = make_float2(dq[0][2] + dq[1][2], dq[0][3] + dq[1][3]);
+    // the k parts of the update do not wait for anything: transposed, tokens along the summed side
+    uint32_t kt[3][4];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) ldmatrix4<true>(kt[c], img + c * D::kPart + (lane & 7) * D::kPitch + piece * 32 + (lane >> 3) * 8);
+    float u[kDT];                                  // first v_i, in the end u_i
+#pragma unroll
+    for (int t = 0; t < kDT; ++t) u[t] = vs[t * 32 + cg * 16 + col];
+    kb2::named_bar_sync(1 + cg, NI * 32);
+    // every warp of the group solves for the group's 16 columns: a lane per column, the two halves share the row pieces
     float p[kDT];
 #pragma unroll
-    for (int t = 0; t < kDT; ++t) {
-      uint64_t a0 = 0, a1 = 0;
+    for (int t = 0; t < kDT; ++t) p[t] = 0.f;
 #pragma unroll
-      for (int c = 0; c < NI; ++c) {
-        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&b.k[t][c * 32 + rg]);
-        kv[t][c][0] = v.x;
-        kv[t][c][1] = v.y;
-        a0 = fma2(S[c][0], v.x, a0);
-        a1 = fma2(S[c][1], v.y, a1);
+    for (int r = 0; r < (NI + 1) / 2; ++r) {
+      const int pc = NI == 1 ? 0 : half * (NI / 2) + r;
+      const float* from = buf + (pc * 16 + col) * 20;
+      const float4 x = *reinterpret_cast<const float4*>(from), y = *reinterpret_cast<const float4*>(from + 4);
+      if (NI > 1 || half == 0) {
+        p[0] += x.x; p[1] += x.y; p[2] += x.z; p[3] += x.w;
+        p[4] += y.x; p[5] += y.y; p[6] += y.z; p[7] += y.w;
       }
-      p[t] = sum2(a0) + sum2(a1);
     }
-    const float pk = row_sums(p);
-    float P[kDT];
 #pragma unroll
-    for (int t = 0; t < kDT; ++t) P[t] = __shfl_sync(0xffffffffu, pk, (t >> 1) * 16 + (t & 1) * 8 + col);
+    for (int t = 0; t < kDT; ++t) p[t] += __shfl_xor_sync(0xffffffffu, p[t], 16);
+#pragma unroll
+    for (int t = 0; t < kDT; ++t) u[t] = fmaf(-ss[t * kDTScalars], p[t], u[t]);
 #pragma unroll
     for (int t = 0; t < kDT; ++t) {
-      uint64_t a0 = 0, a1 = 0;
+      u[t] *= ss[t * kDTScalars + 1];
 #pragma unroll
-      for (int c = 0; c < NI; ++c) {
-        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&b.q[t][c * 32 + rg]);
-        a0 = fma2(S[c][0], v.x, a0);
-        a1 = fma2(S[c][1], v.y, a1);
-      }
-      p[t] = sum2(a0) + sum2(a1);
+      for (int m = t + 1; m < kDT; ++m) u[m] = fmaf(-ss[m * kDTScalars + 4 + t], u[t], u[m]);
     }
-    float u[kDT], scale[kDT], total = 1.f;
-#pragma unroll
-    for (int t = 0; t < kDT; ++t) {
-      const float4 f = *reinterpret_cast<const float4*>(&b.s[t][0]);       // G, beta, D_3t, G_3
-      const float4 a = *reinterpret_cast<const float4*>(&b.s[t][4]);
-      float m = f.x * P[t];
-      if (t > 0) m = fmaf(a.x, u[0], m);
-      if (t > 1) m = fmaf(a.y, u[1], m);
-      if (t > 2) m = fmaf(a.z, u[2], m);
-      u[t] = f.y * (b.v[t][warp * 4 + col] - m);
-      scale[t] = f.z;
-      if (t == 0) total = f.w;
-    }
-    const float rq = row_sums(p);
-    {
-      const float4 d = *reinterpret_cast<const float4*>(&b.s[me][8]);
-      const float o = fmaf(d.w, u[3], fmaf(d.z, u[2], fmaf(d.y, u[1], fmaf(d.x, u[0], b.s[me][0] * rq))));
-      if (!(lane & 4) && i * kDT + me < n) o_out[((t0 + (long long)i * kDT + me) * H + h) * dv + j0 + warp * 4 + col] = o;
+    if (half == 0) {                               // D_7j u_j, for the update
+      *reinterpret_cast<float4*>(myu + col * 12) = make_float4(u[0] * ss[2], u[1] * ss[kDTScalars + 2], u[2] * ss[2 * kDTScalars + 2], u[3] * ss[3 * kDTScalars + 2]);
+      *reinterpret_cast<float4*>(myu + col * 12 + 4) =
+          make_float4(u[4] * ss[4 * kDTScalars + 2], u[5] * ss[5 * kDTScalars + 2], u[6] * ss[6 * kDTScalars + 2], u[7] * ss[7 * kDTScalars + 2]);
     }
     __syncwarp();
-    if (lane == 0) kb2::mbar_arrive(&empty[st]);       // everything of the tile has been read
-    const uint64_t g2 = pair2(total);
+    const float2 ua = *reinterpret_cast<const float2*>(myu + quad * 12 + pair), ub = *reinterpret_cast<const float2*>(myu + (quad + 8) * 12 + pair);
+    uint32_t up[2][3];
+    split_pair(ua.x, ua.y, up[0]);
+    split_pair(ub.x, ub.y, up[1]);
+    const float total = ss[3];
 #pragma unroll
-    for (int c = 0; c < NI; ++c) {
-      S[c][0] = mul2(S[c][0], g2);
-      S[c][1] = mul2(S[c][1], g2);
+    for (int r = 0; r < 4; ++r) {
+      float big[4] = {}, small[4] = {};
+      mma1688(small, up[0][2], up[1][2], kt[0][r]);
+      mma1688(big, up[0][0], up[1][0], kt[0][r]);
+      mma1688(small, up[0][0], up[1][0], kt[2][r]);
+      mma1688(small, up[0][1], up[1][1], kt[1][r]);
+      mma1688(small, up[0][0], up[1][0], kt[1][r]);
+      mma1688(small, up[0][1], up[1][1], kt[0][r]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) S[r][e] = fmaf(S[r][e], total, big[e] + small[e]);
     }
+    // the read-outs are shared out: 8 / (2 NI) tokens per half warp
+    constexpr int kMine = kDT / (2 * NI);
 #pragma unroll
-    for (int t = 0; t < kDT; ++t) {
-      const uint64_t w = pair2(scale[t] * u[t]);
+    for (int m = 0; m < kMine; ++m) {
+      const int t = (piece * 2 + half) * kMine + m;
+      float r = 0.f;
 #pragma unroll
-      for (int c = 0; c < NI; ++c) {
-        S[c][0] = fma2(kv[t][c][0], w, S[c][0]);
-        S[c][1] = fma2(kv[t][c][1], w, S[c][1]);
-      }
+      for (int pc = 0; pc < NI; ++pc) r += buf[(pc * 16 + col) * 20 + 8 + t];
+      const float4 x = *reinterpret_cast<const float4*>(ss + t * kDTScalars + 12), y = *reinterpret_cast<const float4*>(ss + t * kDTScalars + 16);
+      float o = ss[t * kDTScalars] * r;
+      o = fmaf(x.x, u[0], o); o = fmaf(x.y, u[1], o); o = fmaf(x.z, u[2], o); o = fmaf(x.w, u[3], o);
+      o = fmaf(y.x, u[4], o); o = fmaf(y.y, u[5], o); o = fmaf(y.z, u[6], o); o = fmaf(y.w, u[7], o);
+      if (i * kDT + t < n) o_out[((t0 + (long long)i * kDT + t) * H + h) * dv + j0 + cg * 16 + col] = o;
     }
+    __syncwarp();
+    if (lane == 0) kb2::mbar_arrive(&empty[st]);   // everything of the tile has been read
   }
 #pragma unroll
-  for (int i = 0; i < NI; ++i)
+  for (int r = 0; r < 4; ++r)
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const long long r = i * 32 + rg + e * 2;
-      float x, y;
-      asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(S[i][e]));
-      Sg[r * dv] = x;
-      Sg[(r + 1) * dv] = y;
-    }
+    for (int e = 0; e < 4; ++e) Sg[(long long)(r * 8 + pair + (e & 1)) * dv + quad + (e >> 1) * 8] = S[r][e];
 }
 
 // out[t, h, :] = o / rms(o) * norm_w * silu(gate) (gate_act 1: sigmoid(gate)); a warp per (token, head).  V numbers per access: 4 where sizes
@@ -2027,32 +2077,34 @@ static int delta_rule_launch(const float* conv, int C, const float* bproj, long 
   return KB2SEQ_OK;
 }
 
-KB2SEQ_API long long kb2_seq_delta_tiles_scratch(int T, int H, int Hk, int dk, int dv) {
-  if (T <= 0 || H <= 0 || Hk <= 0 || H % Hk || (dk != 32 && dk != 64 && dk != 128) || dv <= 0 || dv % 32) return 0;
-  return (long long)T * (2LL * Hk * dk + (long long)kDTScalars * H + (long long)H * dv);
+// scratch: images of k and q [tiles][Hk] | scalars [tiles][H][8][20] | o [T, H, dv]; at most T / 8 + S tiles, a partial one per sequence
+static long long delta_image_floats(int dk) { return dk == 32 ? DeltaTile<1>::kImage / 2 : dk == 64 ? DeltaTile<2>::kImage / 2 : DeltaTile<4>::kImage / 2; }
+KB2SEQ_API long long kb2_seq_delta_tiles_scratch(int T, int S, int H, int Hk, int dk, int dv) {
+  if (T <= 0 || S <= 0 || H <= 0 || Hk <= 0 || H % Hk || (dk != 32 && dk != 64 && dk != 128) || dv <= 0 || dv % 32) return 0;
+  return ((long long)T / kDT + S) * (Hk * delta_image_floats(dk) + (long long)H * kDT * kDTScalars) + (long long)T * H * dv;
 }
 
 KB2SEQ_API int kb2_seq_delta_tiles(const float* conv, int C, const float* proj, long long ldp, int g_off, int a_off, int b_off, int T, int S, int H,
                                    int Hk, int dk, int dv, const float* A_log, const float* dt_bias, const float* norm_w, float eps, float* state,
                                    const int* cu, const int* slots, float* scratch, long long scratch_floats, void* out, int dt_out, void* stream) {
-  const long long need = kb2_seq_delta_tiles_scratch(T, H, Hk, dk, dv);
-  if (!conv || !proj || !A_log || !dt_bias || !norm_w || !state || !cu || !slots || !scratch || !out || S <= 0 || bad_dt(dt_out) || !need ||
+  const long long need = kb2_seq_delta_tiles_scratch(T, S, H, Hk, dk, dv);
+  if (!conv || !proj || !A_log || !dt_bias || !norm_w || !state || !cu || !slots || !scratch || !out || bad_dt(dt_out) || !need ||
       scratch_floats < need || ((uintptr_t)scratch & 15) || ((uintptr_t)conv & 15) || C % 4 || C < 2 * Hk * dk + H * dv)
     return failf(KB2SEQ_ERR_VALUE, "delta_tiles: bad argument");
   cudaStream_t st = (cudaStream_t)stream;
-  float* qn = scratch;
-  float* kn = qn + (long long)T * Hk * dk;
-  float* sc = kn + (long long)T * Hk * dk;
-  float* ob = sc + (long long)T * H * kDTScalars;
-  const long long tiles = (long long)T / kDT + S;                    // at most: every sequence may end in a partial tile
+  const long long tiles = (long long)T / kDT + S;
+  bf16* image = (bf16*)scratch;
+  float* sc = scratch + tiles * Hk * delta_image_floats(dk);
+  float* ob = sc + tiles * H * kDT * kDTScalars;
   const unsigned blocks = (unsigned)((tiles * Hk + 7) / 8);
   const dim3 grid(S, H, dv / 32);
-#define KB2_DT(NIV)                                                                                                                                \
-  do {                                                                                                                                             \
-    delta_tile_prep_kernel<NIV><<<blocks, 256, 0, st>>>(conv, C, proj + b_off, ldp, proj + a_off, ldp, H, Hk, A_log, dt_bias, T, S, cu, tiles, qn, kn, sc); \
-    SEQ_LAUNCHED();                                                                                                                                \
-    delta_tile_kernel<NIV><<<grid, 288, 0, st>>>(qn, kn, conv, C, 2 * Hk * dk, sc, T, H, Hk, dv, state, cu, slots, ob);                             \
-    SEQ_LAUNCHED();                                                                                                                                \
+#define KB2_DT(NIV)                                                                                                                                   \
+  do {                                                                                                                                                \
+    SEQ_CUDA(cudaFuncSetAttribute(delta_tile_kernel<NIV>, cudaFuncAttributeMaxDynamicSharedMemorySize, DeltaTile<NIV>::kSmem));                        \
+    delta_tile_prep_kernel<NIV><<<blocks, 256, 0, st>>>(conv, C, proj + b_off, ldp, proj + a_off, ldp, H, Hk, A_log, dt_bias, S, cu, tiles, image, sc); \
+    SEQ_LAUNCHED();                                                                                                                                   \
+    delta_tile_kernel<NIV><<<grid, 64 * NIV + 32, DeltaTile<NIV>::kSmem, st>>>(image, conv, C, 2 * Hk * dk, sc, H, Hk, dv, state, cu, slots, ob);        \
+    SEQ_LAUNCHED();                                                                                                                                   \
   } while (0)
   if (dk == 32) KB2_DT(1); else if (dk == 64) KB2_DT(2); else KB2_DT(4);
 #undef KB2_DT

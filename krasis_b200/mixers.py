@@ -311,8 +311,8 @@ class GatedDeltaMixer:
         ops.check(lib.kb2_seq_conv_silu(proj.data_ptr(), proj.stride(0), T, tb.S, self.C, self.K, self.taps.data_ptr(), tail.data_ptr(),
                                         tb.seq_of.data_ptr(), tb.cu.data_ptr(), tb.slots.data_ptr(), conv.data_ptr(), s))
         o = torch.empty((T, self.H * self.dv), dtype=self.dtype, device=h.device)
-        if self.register_state_kernel and tb.max_portion >= self.tile_min_portion:      # long portions: four tokens at a time
-            n = int(lib.kb2_seq_delta_tiles_scratch(T, self.H, self.Hk, self.dk, self.dv))
+        if self.register_state_kernel and tb.max_portion >= self.tile_min_portion:      # long portions: eight tokens at a time
+            n = int(lib.kb2_seq_delta_tiles_scratch(T, tb.S, self.H, self.Hk, self.dk, self.dv))
             scratch = torch.empty(n, dtype=torch.float32, device=h.device)
             ops.check(lib.kb2_seq_delta_tiles(conv.data_ptr(), self.C, proj.data_ptr(), proj.stride(0), self.g_off, self.a_off, self.b_off, T, tb.S,
                                               self.H, self.Hk, self.dk, self.dv, self.A_log.data_ptr(), self.dt_bias.data_ptr(), self.norm.data_ptr(),

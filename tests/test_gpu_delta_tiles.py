@@ -1,4 +1,4 @@
-"""The delta rule four tokens at a time, the short convolution's vector form and the gated read-out at their edges, against fp64."""
+"""The delta rule eight tokens at a time, the short convolution's vector form and the gated read-out at their edges, against fp64."""
 import pytest
 import torch
 
@@ -48,9 +48,9 @@ def _exact(m, h, tb, tail, state, lens, slots):
     return torch.cat(outs), states
 
 
-# portions that end anywhere in a tile of four, one-token portions beside long ones, an odd number of slices and heads per key head
+# portions that end anywhere in a tile of eight, one-token portions beside long ones, an odd number of slices and heads per key head
 @pytest.mark.parametrize("H,Hk,dk,dv", [(2, 1, 32, 32), (4, 4, 64, 96), (6, 2, 128, 64), (9, 1, 32, 32)])
-@pytest.mark.parametrize("lens", [[16], [17, 1, 18], [1, 31, 2, 3], [64, 67]])
+@pytest.mark.parametrize("lens", [[16], [17, 1, 18], [1, 31, 2, 3], [64, 67], [71, 70, 69, 68]])
 @pytest.mark.parametrize("decay", [-3.0, 3.0])                 # slow, and so fast that a tile forgets all it knew
 def test_tiles_against_exact_and_token_form(H, Hk, dk, dv, lens, decay):
     m = _mixer(H, Hk, dk, dv, decay=decay)
