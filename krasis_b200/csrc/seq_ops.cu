@@ -247,7 +247,7 @@ static bool launch_gemv_vec(const void* A, long long lda, const void* B, long lo
 // (8e-8) or less.  From HBM at 4 rows, us before (gemv_nt_vec) and now: N 16384, K 2048 32.3 -> 13.7 (floor 10.3);
 // N 2048, K 8192 19.8 -> 9.2 (5.1); N 32768, K 2048 44.4 -> 25.3 (20.5); N 2048, K 2048 7.3 -> 3.8.
 __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
@@ -1441,12 +1441,17 @@ __global__ void __launch_bounds__(32 * kRegPieces) delta_rule_reg_kernel(const f
 // share an address.  Here a warp keeps 16 value columns x 32 rows as accumulator fragments, which are the operand fragments of the next
 // tile's product as they stand; k and q arrive as ready images (one bulk copy per tile, ahead of time) and enter through ldmatrix, plain for
 // S0^T k and transposed for k u^T.  The DK / 32 warps of a column group meet once per tile and then each solve the eight steps by themselves.
-constexpr int kDT = 8, kDTStages = 4, kDTScalars = 20;     // per (token, head): G, beta, D_7j, G_7 | D_ij k_i.k_j (j < i) | D_ij q_i.k_j (j <= i)
+// 4096 tokens, 32 / 16 heads x 128: 1048 -> 648 us (prep 48 -> 56); left: two warps per scheduler and 2400 cycles per tile of dependent short
+// phases, the tensor pipe 37 % and shared memory 46 % busy.
+constexpr int kDT = 8, kDTStages = 4;
+// what couples the tokens of a (tile, head), as the kernel reads it: G[8] | beta[8] | D_7j [8] | G_7 and padding | D_ij k_i.k_j as [j][i > j] |
+// D_ij q_i.k_j as [i][j <= i]
+constexpr int kDTG = 0, kDTBeta = 8, kDTEnd = 16, kDTAll = 24, kDTKK = 32, kDTQK = 96, kDTScalars = 160;
 template <int NI> struct DeltaTile {
   static constexpr int DK = 32 * NI, kPitch = DK + 8;      // bf16 row pitch: 16 bytes more, so that the eight rows of an ldmatrix do not collide
   static constexpr int kPart = 2 * kDT * kPitch;           // bf16 of one part: k rows, then q rows
   static constexpr int kImage = 3 * kPart;                 // bf16 of a (tile, key head): hi, mid, lo
-  static constexpr int kImageBytes = kImage * 2, kScalarBytes = kDT * kDTScalars * 4, kVBytes = kDT * 32 * 4;
+  static constexpr int kImageBytes = kImage * 2, kScalarBytes = kDTScalars * 4, kVBytes = kDT * 32 * 4;
   static constexpr int kStageBytes = kImageBytes + kVBytes + kScalarBytes;
   static constexpr int kRedFloats = 2 * 2 * NI * 16 * 20;  // [buffer][column group][row piece][column][16 products + pad]
   static constexpr int kUFloats = 2 * NI * 16 * 12;        // [warp][column][8 tokens + pad]
@@ -1578,19 +1583,22 @@ __global__ void __launch_bounds__(256) delta_tile_prep_kernel(const float* __res
       if (j <= me) d *= gs[j];
     }
     if (!head) continue;
-    float4* o = reinterpret_cast<float4*>(sc + ((flat * H + h) * kDT + me) * kDTScalars);
+    float* o = sc + (flat * H + h) * kDTScalars;
     const bool in = me < nt;                          // tokens behind the last one take no part
-    o[0] = make_float4(in ? up : 0.f, beta, in ? down : 0.f, all);
+    o[kDTG + me] = in ? up : 0.f;
+    o[kDTBeta + me] = beta;
+    o[kDTEnd + me] = in ? down : 0.f;
+    if (me == 0) o[kDTAll] = all;
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      o[1 + 2 * c] = in ? make_float4(row[c][0], row[c][1], row[c][2], row[c][3]) : make_float4(0.f, 0.f, 0.f, 0.f);
-      o[2 + 2 * c] = in ? make_float4(row[c][4], row[c][5], row[c][6], row[c][7]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < kDT; ++j) {
+      o[kDTKK + j * kDT + me] = in ? row[0][j] : 0.f;
+      o[kDTQK + me * kDT + j] = in ? row[1][j] : 0.f;
     }
   }
 }
 
 __device__ __forceinline__ void mma1688(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a0), "r"(a1), "r"(b0));
 }
@@ -1639,7 +1647,7 @@ __global__ void __launch_bounds__(64 * NI + 32, 1) delta_tile_kernel(const bf16*
       __syncwarp();
       if (lane < nt) kb2::bulk_g2s(b + D::kImageBytes + lane * 128, conv + (t + lane) * C + v_col0 + h * dv + j0, 128, &full[st]);
       else if (lane == 8) kb2::bulk_g2s(b, image + ((first + i) * Hk + hk) * D::kImage, D::kImageBytes, &full[st]);
-      else if (lane == 9) kb2::bulk_g2s(b + D::kImageBytes + D::kVBytes, sc + ((first + i) * H + h) * kDT * kDTScalars, D::kScalarBytes, &full[st]);
+      else if (lane == 9) kb2::bulk_g2s(b + D::kImageBytes + D::kVBytes, sc + ((first + i) * H + h) * kDTScalars, D::kScalarBytes, &full[st]);
     }
     return;
   }
@@ -1671,33 +1679,42 @@ __global__ void __launch_bounds__(64 * NI + 32, 1) delta_tile_kernel(const bf16*
         for (int c = 0; c < 3; ++c) sp[kb][c][e] = p[c];
       }
     kb2::mbar_wait(&full[st], (uint32_t)(i / kDTStages & 1));
-    float dk[2][4] = {}, dq[2][4] = {};            // [big terms, small terms]
+    float dk[4][4] = {}, dq[4][4] = {};            // four sums each (the products by size), so that no instruction waits for the one before it
 #pragma unroll
     for (int kb = 0; kb < 2; ++kb) {
       uint32_t x[3][4];                            // k rows 0..7, k rows 8..15 of the block; q the same
 #pragma unroll
       for (int c = 0; c < 3; ++c)
         ldmatrix4<false>(x[c], img + c * D::kPart + ((lane >> 4) * kDT + (lane & 7)) * D::kPitch + piece * 32 + kb * 16 + ((lane >> 3) & 1) * 8);
-      auto six = [&](float (&big)[4], float (&small)[4], int o) {
-        mma16816(small, sp[kb][2][0], sp[kb][2][1], sp[kb][2][2], sp[kb][2][3], x[0][o], x[0][o + 1]);
-        mma16816(big, sp[kb][0][0], sp[kb][0][1], sp[kb][0][2], sp[kb][0][3], x[0][o], x[0][o + 1]);
-        mma16816(small, sp[kb][0][0], sp[kb][0][1], sp[kb][0][2], sp[kb][0][3], x[2][o], x[2][o + 1]);
-        mma16816(small, sp[kb][1][0], sp[kb][1][1], sp[kb][1][2], sp[kb][1][3], x[1][o], x[1][o + 1]);
-        mma16816(small, sp[kb][0][0], sp[kb][0][1], sp[kb][0][2], sp[kb][0][3], x[1][o], x[1][o + 1]);
-        mma16816(small, sp[kb][1][0], sp[kb][1][1], sp[kb][1][2], sp[kb][1][3], x[0][o], x[0][o + 1]);
+      auto product = [&](int sum, int sc_, int xc) {
+        mma16816(dk[sum], sp[kb][sc_][0], sp[kb][sc_][1], sp[kb][sc_][2], sp[kb][sc_][3], x[xc][0], x[xc][1]);
+        mma16816(dq[sum], sp[kb][sc_][0], sp[kb][sc_][1], sp[kb][sc_][2], sp[kb][sc_][3], x[xc][2], x[xc][3]);
       };
-      six(dk[0], dk[1], 0);
-      six(dq[0], dq[1], 2);
+      product(0, 0, 0);
+      product(1, 0, 1);
+      product(2, 1, 0);
+      product(3, 2, 0);
+      product(3, 0, 2);
+      product(3, 1, 1);
     }
+    auto whole = [](const float (&d)[4][4], int e) { return d[0][e] + (d[1][e] + (d[2][e] + d[3][e])); };
     float* mine = buf + piece * 16 * 20;
-    *reinterpret_cast<float2*>(mine + quad * 20 + pair) = make_float2(dk[0][0] + dk[1][0], dk[0][1] + dk[1][1]);
-    *reinterpret_cast<float2*>(mine + (quad + 8) * 20 + pair) = make_float2(dk[0][2] + dk[1][2], dk[0][3] + dk[1][3]);
-    *reinterpret_cast<float2*>(mine + quad * 20 + 8 + pair) = make_float2(dq[0][0] + dq[1][0], dq[0][1] + dq[1][1]);
-    *reinterpret_cast<float2*>(mine + (quad + 8) * 20 + 8 + pair) = make_float2(dq[0][2] + dq[1][2], dq[0][3] + dq[1][3]);
+    *reinterpret_cast<float2*>(mine + quad * 20 + pair) = make_float2(whole(dk, 0), whole(dk, 1));
+    *reinterpret_cast<float2*>(mine + (quad + 8) * 20 + pair) = make_float2(whole(dk, 2), whole(dk, 3));
+    *reinterpret_cast<float2*>(mine + quad * 20 + 8 + pair) = make_float2(whole(dq, 0), whole(dq, 1));
+    *reinterpret_cast<float2*>(mine + (quad + 8) * 20 + 8 + pair) = make_float2(whole(dq, 2), whole(dq, 3));
     // the k parts of the update do not wait for anything: transposed, tokens along the summed side
     uint32_t kt[3][4];
 #pragma unroll
     for (int c = 0; c < 3; ++c) ldmatrix4<true>(kt[c], img + c * D::kPart + (lane & 7) * D::kPitch + piece * 32 + (lane >> 3) * 8);
+    auto eight = [&](int at, float (&to)[kDT]) {
+      const float4 x = *reinterpret_cast<const float4*>(ss + at), y = *reinterpret_cast<const float4*>(ss + at + 4);
+      to[0] = x.x; to[1] = x.y; to[2] = x.z; to[3] = x.w; to[4] = y.x; to[5] = y.y; to[6] = y.z; to[7] = y.w;
+    };
+    float g[kDT], beta[kDT], end[kDT];
+    eight(kDTG, g);
+    eight(kDTBeta, beta);
+    eight(kDTEnd, end);
     float u[kDT];                                  // first v_i, in the end u_i
 #pragma unroll
     for (int t = 0; t < kDT; ++t) u[t] = vs[t * 32 + cg * 16 + col];
@@ -1719,35 +1736,38 @@ __global__ void __launch_bounds__(64 * NI + 32, 1) delta_tile_kernel(const bf16*
 #pragma unroll
     for (int t = 0; t < kDT; ++t) p[t] += __shfl_xor_sync(0xffffffffu, p[t], 16);
 #pragma unroll
-    for (int t = 0; t < kDT; ++t) u[t] = fmaf(-ss[t * kDTScalars], p[t], u[t]);
+    for (int t = 0; t < kDT; ++t) u[t] = fmaf(-g[t], p[t], u[t]);
 #pragma unroll
     for (int t = 0; t < kDT; ++t) {
-      u[t] *= ss[t * kDTScalars + 1];
+      u[t] *= beta[t];
+      if (t + 1 < kDT) {
+        float a[kDT];
+        eight(kDTKK + t * kDT, a);
 #pragma unroll
-      for (int m = t + 1; m < kDT; ++m) u[m] = fmaf(-ss[m * kDTScalars + 4 + t], u[t], u[m]);
+        for (int m = t + 1; m < kDT; ++m) u[m] = fmaf(-a[m], u[t], u[m]);
+      }
     }
     if (half == 0) {                               // D_7j u_j, for the update
-      *reinterpret_cast<float4*>(myu + col * 12) = make_float4(u[0] * ss[2], u[1] * ss[kDTScalars + 2], u[2] * ss[2 * kDTScalars + 2], u[3] * ss[3 * kDTScalars + 2]);
-      *reinterpret_cast<float4*>(myu + col * 12 + 4) =
-          make_float4(u[4] * ss[4 * kDTScalars + 2], u[5] * ss[5 * kDTScalars + 2], u[6] * ss[6 * kDTScalars + 2], u[7] * ss[7 * kDTScalars + 2]);
+      *reinterpret_cast<float4*>(myu + col * 12) = make_float4(u[0] * end[0], u[1] * end[1], u[2] * end[2], u[3] * end[3]);
+      *reinterpret_cast<float4*>(myu + col * 12 + 4) = make_float4(u[4] * end[4], u[5] * end[5], u[6] * end[6], u[7] * end[7]);
     }
     __syncwarp();
     const float2 ua = *reinterpret_cast<const float2*>(myu + quad * 12 + pair), ub = *reinterpret_cast<const float2*>(myu + (quad + 8) * 12 + pair);
     uint32_t up[2][3];
     split_pair(ua.x, ua.y, up[0]);
     split_pair(ub.x, ub.y, up[1]);
-    const float total = ss[3];
+    const float total = ss[kDTAll];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      float big[4] = {}, small[4] = {};
-      mma1688(small, up[0][2], up[1][2], kt[0][r]);
+      float big[4] = {}, small[2][4] = {};
       mma1688(big, up[0][0], up[1][0], kt[0][r]);
-      mma1688(small, up[0][0], up[1][0], kt[2][r]);
-      mma1688(small, up[0][1], up[1][1], kt[1][r]);
-      mma1688(small, up[0][0], up[1][0], kt[1][r]);
-      mma1688(small, up[0][1], up[1][1], kt[0][r]);
+      mma1688(small[0], up[0][0], up[1][0], kt[1][r]);
+      mma1688(small[1], up[0][1], up[1][1], kt[0][r]);
+      mma1688(small[0], up[0][2], up[1][2], kt[0][r]);
+      mma1688(small[1], up[0][0], up[1][0], kt[2][r]);
+      mma1688(small[0], up[0][1], up[1][1], kt[1][r]);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) S[r][e] = fmaf(S[r][e], total, big[e] + small[e]);
+      for (int e = 0; e < 4; ++e) S[r][e] = fmaf(S[r][e], total, big[e] + (small[0][e] + small[1][e]));
     }
     // the read-outs are shared out: 8 / (2 NI) tokens per half warp
     constexpr int kMine = kDT / (2 * NI);
@@ -1757,10 +1777,10 @@ __global__ void __launch_bounds__(64 * NI + 32, 1) delta_tile_kernel(const bf16*
       float r = 0.f;
 #pragma unroll
       for (int pc = 0; pc < NI; ++pc) r += buf[(pc * 16 + col) * 20 + 8 + t];
-      const float4 x = *reinterpret_cast<const float4*>(ss + t * kDTScalars + 12), y = *reinterpret_cast<const float4*>(ss + t * kDTScalars + 16);
-      float o = ss[t * kDTScalars] * r;
-      o = fmaf(x.x, u[0], o); o = fmaf(x.y, u[1], o); o = fmaf(x.z, u[2], o); o = fmaf(x.w, u[3], o);
-      o = fmaf(y.x, u[4], o); o = fmaf(y.y, u[5], o); o = fmaf(y.z, u[6], o); o = fmaf(y.w, u[7], o);
+      float a[kDT], o = ss[kDTG + t] * r;
+      eight(kDTQK + t * kDT, a);
+#pragma unroll
+      for (int j = 0; j < kDT; ++j) o = fmaf(a[j], u[j], o);
       if (i * kDT + t < n) o_out[((t0 + (long long)i * kDT + t) * H + h) * dv + j0 + cg * 16 + col] = o;
     }
     __syncwarp();
@@ -2077,11 +2097,11 @@ static int delta_rule_launch(const float* conv, int C, const float* bproj, long 
   return KB2SEQ_OK;
 }
 
-// scratch: images of k and q [tiles][Hk] | scalars [tiles][H][8][20] | o [T, H, dv]; at most T / 8 + S tiles, a partial one per sequence
+// scratch: images of k and q [tiles][Hk] | scalars [tiles][H][160] | o [T, H, dv]; at most T / 8 + S tiles, a partial one per sequence
 static long long delta_image_floats(int dk) { return dk == 32 ? DeltaTile<1>::kImage / 2 : dk == 64 ? DeltaTile<2>::kImage / 2 : DeltaTile<4>::kImage / 2; }
 KB2SEQ_API long long kb2_seq_delta_tiles_scratch(int T, int S, int H, int Hk, int dk, int dv) {
   if (T <= 0 || S <= 0 || H <= 0 || Hk <= 0 || H % Hk || (dk != 32 && dk != 64 && dk != 128) || dv <= 0 || dv % 32) return 0;
-  return ((long long)T / kDT + S) * (Hk * delta_image_floats(dk) + (long long)H * kDT * kDTScalars) + (long long)T * H * dv;
+  return ((long long)T / kDT + S) * (Hk * delta_image_floats(dk) + (long long)H * kDTScalars) + (long long)T * H * dv;
 }
 
 KB2SEQ_API int kb2_seq_delta_tiles(const float* conv, int C, const float* proj, long long ldp, int g_off, int a_off, int b_off, int T, int S, int H,
@@ -2095,7 +2115,7 @@ KB2SEQ_API int kb2_seq_delta_tiles(const float* conv, int C, const float* proj, 
   const long long tiles = (long long)T / kDT + S;
   bf16* image = (bf16*)scratch;
   float* sc = scratch + tiles * Hk * delta_image_floats(dk);
-  float* ob = sc + tiles * H * kDT * kDTScalars;
+  float* ob = sc + tiles * H * kDTScalars;
   const unsigned blocks = (unsigned)((tiles * Hk + 7) / 8);
   const dim3 grid(S, H, dv / 32);
 #define KB2_DT(NIV)                                                                                                                                   \
