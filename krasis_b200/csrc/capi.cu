@@ -16,7 +16,7 @@
 #include <mutex>
 
 namespace kb2 {
-cudaError_t launch_grouped_gemm(int fmt, bool gemm1, const GemmParams& p, const void* tmap_b, int num_sms,
+cudaError_t launch_grouped_gemm(int fmt, bool gemm1, int chunk_tokens, const GemmParams& p, const void* tmap_b, int num_sms,
                                 cudaStream_t stream);
 cudaError_t make_tmap_bf16_rows(void* out_tmap, const void* base, long long rows, long long cols, int box_rows);
 int gemm_b_box_rows();
@@ -27,12 +27,10 @@ cudaError_t launch_router_gemm(const void* x, const void* tmap_g, const float* b
                                int H, cudaStream_t s);
 cudaError_t launch_router_topk(const float* logits, const float* corr_bias, int M, int E, int top_k, int scoring,
                                int renorm, int* ids, float* wts, cudaStream_t s);
-cudaError_t launch_binning(const int* ids, const float* wts, int M, int top_k, int e_start, int e_end, int* counts,
+cudaError_t launch_binning(const int* ids, const float* wts, int M, int top_k, int e_start, int e_end, int chunk_tokens, int* counts,
                            int* offsets, int* cursor, ChunkDesc* chunks, int* n_chunks, float* sorted_w, int* slot_of,
-                           int* sorted_ids, const void* x, void* x_sorted, int H, cudaStream_t s);
-cudaError_t launch_binning_index(const int* ids, const float* wts, int M, int top_k, int e_start, int e_end, int* counts,
-                                 int* offsets, int* cursor, ChunkDesc* chunks, int* n_chunks, float* sorted_w, int* slot_of,
-                                 int* sorted_tok, cudaStream_t s);
+                           int* sorted_ids, int* sorted_tok, const void* x, void* x_sorted, int H, cudaStream_t s);
+int binning_launches(long long n);
 cudaError_t make_tmap_bf16_gather(void* out_tmap, const void* base, long long rows, long long cols);
 cudaError_t launch_combine_scatter(const void* c3, const int* slot_of, int M, int H, int top_k, float rsf, int apply_rsf,
                                    const void* shared, void* out, const CombineScatter& sc, cudaStream_t s);
@@ -256,7 +254,7 @@ KB2_API int kb2_create(const kb2_config* c, kb2_engine** out) {
   e->num_sms = prop.multiProcessorCount;
   e->layers.resize(c->num_moe_layers);
   const size_t MK = (size_t)c->max_tokens * c->num_experts_per_tok;
-  const size_t max_chunks = c->n_routed_experts + MK / kMaxChunkTokens + 1;
+  const size_t max_chunks = c->n_routed_experts + MK / kShortChunkTokens + 1;
   // a failed allocation must not leak the engine or the buffers made so far: kb2_destroy frees whatever exists
 #define ALLOC(ptr, bytes)                                                                               \
   do {                                                                                                  \
@@ -539,16 +537,17 @@ static int moe_forward_impl(kb2_engine* e, int layer, const void* x, const int32
   const char* gev = getenv("KB2_MOE_GATHER");
   const bool gather = gev ? gev[0] == '1' : kDefaultMoeGather;
   alignas(64) unsigned char tmap_gather[128];
+  // Short chunks where experts get few rows on average (or can get few only): the weights' way from memory and through the dequantisers bounds
+  // the GEMMs, not their MMAs.  A whole pass, short / wide: 64 experts of 1408 columns, 4 bits, 36 rows per expert 136 / 142 us, 48 rows 142 / 148,
+  // 56 rows 161 / 151; 512 experts of 512 columns, 49 rows 382 / 386, 59 rows 445 / 407.  With the 8 KB and larger tiles, of which the wide form
+  // keeps two in flight: 36 rows 155 / 206, 56 rows 177 / 214, 66 rows 218 / 224.
+  const int short_mean = f13 == kFmtInt4G128 || f13 == kFmtQ4_K ? 48 : 64;
+  const int chunk_tokens = M <= kShortChunkTokens || (long long)M * K <= (long long)short_mean * e->e_local ? kShortChunkTokens : kMaxChunkTokens;
   { ProfSpan ps(e, KB2_PROF_BINNING, s);
-    if (gather) {
-      CUDA_TRY(launch_binning_index(ids, wts, M, K, e->e_start, e->e_end, e->counts, e->offsets, e->cursor, e->chunks,
-                                    e->n_chunks, e->sorted_w, e->slot_of, e->sorted_tok, s));
-      CUDA_TRY(make_tmap_bf16_gather(tmap_gather, x, M, H));
-    } else {
-      CUDA_TRY(launch_binning(ids, wts, M, K, e->e_start, e->e_end, e->counts, e->offsets, e->cursor, e->chunks,
-                              e->n_chunks, e->sorted_w, e->slot_of, nullptr, x, e->x_sorted, H, s));
-    } }
-  e->launches += 3;
+    CUDA_TRY(launch_binning(ids, wts, M, K, e->e_start, e->e_end, chunk_tokens, e->counts, e->offsets, e->cursor, e->chunks, e->n_chunks,
+                            e->sorted_w, e->slot_of, nullptr, gather ? e->sorted_tok : nullptr, x, gather ? nullptr : e->x_sorted, H, s));
+    if (gather) CUDA_TRY(make_tmap_bf16_gather(tmap_gather, x, M, H)); }
+  e->launches += binning_launches((long long)M * K);
 
   GemmParams g1{};
   g1.wq = L.w13_q; g1.ws = L.w13_s;
@@ -560,7 +559,7 @@ static int moe_forward_impl(kb2_engine* e, int layer, const void* x, const int32
   g1.out = (__nv_bfloat16*)e->act; g1.out_ld = I; g1.slot_weight = nullptr;
   g1.gather_rows = gather ? e->sorted_tok : nullptr;
   { ProfSpan ps(e, KB2_PROF_GEMM1, s);
-    CUDA_TRY(launch_grouped_gemm(f13, true, g1, gather ? tmap_gather : e->tmap_x, e->num_sms, s)); }
+    CUDA_TRY(launch_grouped_gemm(f13, true, chunk_tokens, g1, gather ? tmap_gather : e->tmap_x, e->num_sms, s)); }
 
   GemmParams g2{};
   g2.wq = L.w2_q; g2.ws = L.w2_s;
@@ -571,7 +570,7 @@ static int moe_forward_impl(kb2_engine* e, int layer, const void* x, const int32
   g2.chunks = e->chunks; g2.n_chunks = e->n_chunks;
   g2.out = (__nv_bfloat16*)e->c3; g2.out_ld = H; g2.slot_weight = e->sorted_w;
   { ProfSpan ps(e, KB2_PROF_GEMM2, s);
-    CUDA_TRY(launch_grouped_gemm(f2, false, g2, e->tmap_act, e->num_sms, s)); }
+    CUDA_TRY(launch_grouped_gemm(f2, false, chunk_tokens, g2, e->tmap_act, e->num_sms, s)); }
 
   { ProfSpan ps(e, KB2_PROF_COMBINE, s);
     if (scatter) CUDA_TRY(launch_combine_scatter(e->c3, e->slot_of, M, H, K, e->cfg.routed_scaling_factor, 0, nullptr, nullptr, *scatter, s));
@@ -643,10 +642,10 @@ KB2_API int kb2_ep_bin_rows(kb2_engine* e, const void* x, const int32_t* ids, co
   CUDA_TRY(cudaSetDevice(e->cfg.device));
   cudaStream_t s = (cudaStream_t)stream;
   ProfSpan ps(e, KB2_PROF_BINNING, s);
-  CUDA_TRY(launch_binning(ids, wts, M, e->cfg.num_experts_per_tok, 0, e->cfg.n_routed_experts, counts, e->offsets,
-                          e->cursor, e->chunks, e->n_chunks, w_sorted, slot_of, ids_sorted, x, x_sorted,
+  CUDA_TRY(launch_binning(ids, wts, M, e->cfg.num_experts_per_tok, 0, e->cfg.n_routed_experts, kMaxChunkTokens, counts, e->offsets,
+                          e->cursor, e->chunks, e->n_chunks, w_sorted, slot_of, ids_sorted, nullptr, x, x_sorted,
                           e->cfg.hidden_size, s));
-  e->launches += 3;
+  e->launches += binning_launches((long long)M * e->cfg.num_experts_per_tok);
   return KB2_OK;
 }
 

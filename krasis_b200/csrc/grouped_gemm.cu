@@ -19,14 +19,22 @@
 // exceeded the 128 B/clk smem port in the first version of this kernel (profiles/r01a_*).
 //   GEMM1: the pair is (gate tile t, up tile t) -> SiLU(gate)*up fused in the epilogue, BF16 act out
 //   GEMM2: the pair is two consecutive down-proj tiles -> x routing weight, BF16 c3 out
-// Warp roles (512 threads):
+// Warp roles (896 threads):
 //   warp 0      : bulk-TMA producer of packed weight tiles + scale tiles (one elected lane)
 //   warp 1      : tcgen05.mma issuer (one elected lane)
 //   warp 2      : 2-D TMA producer of the token (B) operand (one elected lane)
-//   warps 4-7   : dequantisers of weight tile 0 (thread t owns weight row t = TMEM lane t)
-//   warps 8-11  : epilogue
-//   warps 12-15 : dequantisers of weight tile 1
+//   warps 4-7   : dequantisers of weight tile 0, even k-blocks (thread t owns weight row t = TMEM lane t); warps 16-19: odd k-blocks
+//   warps 12-15 : dequantisers of weight tile 1, even k-blocks; warps 20-23: odd k-blocks
+//   warps 8-11  : epilogue of tile 0; warps 24-27: of tile 1
+// A k-block costs a dequantiser 870 cycles (two waits of 70, shared-memory and TMEM round trips, 680 of arithmetic at two warps per scheduler),
+// whatever the format and the token count, where its MMAs take 200 (N = 16) to 640 (N = 160): with one group the K loop ran at that pace for
+// every shape, and the accumulators stood still for 3000 cycles per item while four warps drained them.  Two groups, pauses between polls (half of
+// all instructions were polls), and waits under the MMAs: gate/up of 8192 x 10 tokens over 512 experts (H 2048, I 512, INT4) 316 -> 273 us, down
+// 197 -> 182; 389 x 6 over 64 experts (I 1408, INT8, with short chunks) 106 -> 75 and 60 -> 43.  Left: the wide K loop takes 830 cycles per block
+// for 640 of MMAs, with 29 KB of tiles per block through the SM's copy engine; the short one is bound by issue slots (60 % busy).
 // TMEM columns: [0,192) acc0 | [192,384) acc1 | [384,512) two A stages x (tile0 32 cols | tile1 32 cols)
+// Short chunks (at most 64 tokens, launched where experts get few rows): the kernel above waited for weights, with 34-35 KB of them in flight per
+// SM, and its B and staging tiles lay idle.  The short form's rings: see SmemLayout.
 // Numerics (oracle/moe.py, GPU-path): W = bf16((nib-8)*scale) exactly as Marlin's BF16 dequant,
 // fp32 accumulation in TMEM, BF16 rounding at C1, A and C3.
 #include <cuda.h>
@@ -39,62 +47,50 @@
 
 namespace kb2 {
 
-constexpr int kNumThreads = 512;
-constexpr int kStagesA = 2;                                     // A operand stages in TMEM
-constexpr int kBStageBytes = kMaxChunkTokens * kBlockK * 2;     // 24 KB
+constexpr int kNumThreads = 896;
 constexpr int kBBoxRows = 32;                                   // TMA box = 32 token rows x 64 K
 constexpr int kBBoxBytes = kBBoxRows * kBlockK * 2;             // 4 KB
 constexpr int kTmemCols = 512;
-constexpr int kAcc1Col = kMaxChunkTokens;                       // 192
-constexpr int kATmemCol = 2 * kMaxChunkTokens;                  // 384
 constexpr int kATileCols = kBlockK / 2;                         // 32 columns = 128 rows x 64 bf16
-constexpr int kNumDequantThreads = 256;
-constexpr int kNumEpiThreads = 128;
+constexpr int kNumDequantThreads = 256;                         // of one k-block
+constexpr int kNumEpiThreads = 256;
 
 template <int FMT>
 struct Fmt;
-template <>
-struct Fmt<kFmtInt4G128> {
-  static constexpr int kTileBytes = kInt4TileBytes;
-  static constexpr int kStagesW = 4;   // packed-weight ring depth
-};
-template <>
-struct Fmt<kFmtInt8G128> {
-  static constexpr int kTileBytes = kInt8TileBytes;
-  static constexpr int kStagesW = 2;
-};
-template <>
-struct Fmt<kFmtQ8_0> {
-  static constexpr int kTileBytes = kQ8_0TileBytes;
-  static constexpr int kStagesW = 2;
-};
-template <>
-struct Fmt<kFmtQ4_K> {
-  static constexpr int kTileBytes = kQ4KTileBytes;
-  static constexpr int kStagesW = 3;
-};
-template <>
-struct Fmt<kFmtAffine8> {
-  static constexpr int kTileBytes = kAffine8TileBytes;
-  static constexpr int kStagesW = 2;
-};
+// kStagesW: packed-weight ring depth of the wide form
+template <> struct Fmt<kFmtInt4G128> { static constexpr int kTileBytes = kInt4TileBytes, kStagesW = 4; };
+template <> struct Fmt<kFmtInt8G128> { static constexpr int kTileBytes = kInt8TileBytes, kStagesW = 2; };
+template <> struct Fmt<kFmtQ8_0> { static constexpr int kTileBytes = kQ8_0TileBytes, kStagesW = 2; };
+template <> struct Fmt<kFmtQ4_K> { static constexpr int kTileBytes = kQ4KTileBytes, kStagesW = 3; };
+template <> struct Fmt<kFmtAffine8> { static constexpr int kTileBytes = kAffine8TileBytes, kStagesW = 2; };
 template <int FMT>
 constexpr bool kHasScaleTiles = (FMT == kFmtInt4G128 || FMT == kFmtInt8G128);
 
-template <int FMT, bool kGemm1>
+// NT = tokens per chunk: kMaxChunkTokens (wide), or kShortChunkTokens (short), which trades the token tiles' shared memory and TMEM for a
+// weight ring of 135-140 KB, four A stages and a second pair of accumulators (the epilogue of one item runs under the next item's MMAs).
+template <int FMT, bool kGemm1, int NT>
 struct SmemLayout {
-  static constexpr int kStagesW = Fmt<FMT>::kStagesW;
+  static constexpr bool kShort = NT != kMaxChunkTokens;
+  static constexpr int kStagesA = kShort ? 4 : 2;                               // A operand stages in TMEM
+  static constexpr int kAccBufs = kShort ? 2 : 1;
+  static constexpr int kAcc1Col = NT;                                           // second tile's accumulator within a buffer
+  static constexpr int kATmemCol = 2 * NT * kAccBufs;
+  static_assert(kBlockK == 64, "four MMA steps per k-block");
+  static_assert(kATmemCol + kStagesA * 2 * kATileCols <= kTmemCols, "TMEM columns");
+  static constexpr int kBStageBytes = NT * kBlockK * 2;
   // token (B operand) ring: 4 stages wherever they fit the 227 KB (everything but the 12 KB Affine8 tiles).  With tcgen05.mma issued
   // at full rate the K loop waited ~200 cycles per k-block on token rows with 3 stages (profiles/r02i_gemm_item_timeline_*).
-  static constexpr int kStagesB = (FMT == kFmtAffine8) ? 3 : 4;
+  static constexpr int kStagesB = kShort ? 6 : (FMT == kFmtAffine8) ? 3 : 4;
   static constexpr int kWStageBytes = 2 * Fmt<FMT>::kTileBytes + (kHasScaleTiles<FMT> ? 2 * kScaleTileBytes : 0);
   static constexpr int kStageRowBytes = 2 * kTileRows * 2;   // epilogue staging: 512 B per token (gate|up or two down tiles)
   static constexpr int kOffB = 0;                                               // 1024-aligned (swizzle atoms)
   static constexpr int kOffStage = kOffB + kStagesB * kBStageBytes;
-  static constexpr int kOffW = kOffStage + kMaxChunkTokens * kStageRowBytes;
+  static constexpr int kOffW = kOffStage + NT * kStageRowBytes;
+  static constexpr int kFitW = (227 * 1024 - 1024 - kOffW) / kWStageBytes;      // 1 KB left for weights of slots and barriers
+  static constexpr int kStagesW = !kShort ? Fmt<FMT>::kStagesW : kFitW < 16 ? kFitW : 16;
   static constexpr int kOffSlotW = kOffW + kStagesW * kWStageBytes;             // GEMM2: routing weight of the chunk's token slots (f32)
-  static constexpr int kOffBar = kOffSlotW + kMaxChunkTokens * 4;
-  static constexpr int kNumBars = 2 * kStagesW + 2 * kStagesA + 2 * kStagesB + 2;
+  static constexpr int kOffBar = kOffSlotW + NT * 4;
+  static constexpr int kNumBars = 2 * kStagesW + 2 * kStagesA + 2 * kStagesB + 2 * kAccBufs;
   static constexpr int kOffTmemPtr = kOffBar + kNumBars * 8;
   static constexpr int kTotal = kOffTmemPtr + 16;
   static_assert(kTotal <= 227 * 1024, "CTA shared memory exceeds the 227 KB sm_100 limit");
@@ -110,6 +106,12 @@ struct Ring {
       phase ^= 1;
     }
   }
+  __device__ __forceinline__ void advance2(int n) {      // n >= 2
+    if ((stage += 2) >= n) {
+      stage -= n;
+      phase ^= 1;
+    }
+  }
 };
 
 __device__ __forceinline__ float silu_f(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
@@ -117,8 +119,9 @@ __device__ __forceinline__ float silu_f(float x) { return __fdividef(x, 1.0f + _
 // (w & 0x000F000F) | 0x43004300 == bf16x2 {128 + nib_lo, 128 + nib_hi}; subtracting 136 gives the
 // signed value exactly, the multiply by the BF16 group scale then rounds once (RNE) — identical to
 // bf16((nib - 8) * scale) of the oracle.
-__device__ __forceinline__ uint32_t deq_pair_int4(uint32_t w_shifted, __nv_bfloat162 scale2) {
-  uint32_t t = (w_shifted & 0x000F000Fu) | 0x43004300u;
+// `magic` is 0x43004300 from the kernel's parameters: with two literals the compiler makes two instructions of the and and the or.
+__device__ __forceinline__ uint32_t deq_pair_int4(uint32_t w_shifted, uint32_t magic, __nv_bfloat162 scale2) {
+  uint32_t t = (w_shifted & 0x000F000Fu) | magic;
   __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&t);
   const uint32_t k136 = 0x43084308u;  // bf16 136.0 x2
   v = __hsub2(v, *reinterpret_cast<const __nv_bfloat162*>(&k136));
@@ -126,10 +129,31 @@ __device__ __forceinline__ uint32_t deq_pair_int4(uint32_t w_shifted, __nv_bfloa
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-template <int FMT, bool kGemm1>
+// Two signed bytes (the low or the high pair of a word) as bf16 x scale.  0x43b as bf16 is 128 + (b & 127) with the sign bit moved out, and
+// 0x4300 | (b & 128) is 128 or 256: their difference is the signed value, exactly, and the multiply rounds once, like bf16(float(b) * scale)
+// (|b| <= 128 and the scale have 8 significant bits each).  Integer to float conversions run at a quarter of this rate: with them the dequantisers
+// took 1000 cycles per 64 columns of K, more than the bytes need from memory.
+__device__ __forceinline__ uint32_t deq_pair_int8(uint32_t word, int hi, __nv_bfloat162 scale2) {
+  const uint32_t w = __byte_perm(word, 0x43434343u, hi ? 0x4342 : 0x4140);
+  const uint32_t t = w & 0xFF7FFF7Fu, c = w & 0xFF80FF80u;
+  __nv_bfloat162 v = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&t), *reinterpret_cast<const __nv_bfloat162*>(&c));
+  v = __hmul2(v, scale2);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+
+// Two signed bytes as floats, exactly: the byte + 128 becomes the low mantissa byte of 2^23.
+__device__ __forceinline__ float2 s8_pair(uint32_t word, int hi) {
+  const uint32_t u = word ^ 0x80808080u;
+  return make_float2(__uint_as_float(__byte_perm(u, 0x4B000000u, hi ? 0x7442 : 0x7440)) - 8388736.0f,
+                     __uint_as_float(__byte_perm(u, 0x4B000000u, hi ? 0x7443 : 0x7441)) - 8388736.0f);
+}
+
+template <int FMT, bool kGemm1, int NT, bool TRACE>
 __global__ void __launch_bounds__(kNumThreads, 1)
     grouped_gemm_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap_b) {
-  using L = SmemLayout<FMT, kGemm1>;
+  using L = SmemLayout<FMT, kGemm1, NT>;
+  constexpr int kStagesA = L::kStagesA, kAccBufs = L::kAccBufs, kAcc1Col = L::kAcc1Col, kATmemCol = L::kATmemCol;
+  constexpr int kBStageBytes = L::kBStageBytes;
   constexpr int kStagesW = L::kStagesW;
   constexpr int TB = Fmt<FMT>::kTileBytes;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -142,7 +166,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
   constexpr int kStagesB = L::kStagesB;
   uint64_t* b_empty = b_full + kStagesB;
   uint64_t* tmem_full = b_empty + kStagesB;
-  uint64_t* tmem_empty = tmem_full + 1;
+  uint64_t* tmem_empty = tmem_full + kAccBufs;
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem + L::kOffTmemPtr);
 
   // warp index through a shuffle: the compiler then KNOWS the role branches below are warp-uniform and keeps the operands of the
@@ -166,8 +190,10 @@ __global__ void __launch_bounds__(kNumThreads, 1)
       mbar_init(&b_full[i], 1);
       mbar_init(&b_empty[i], 1);
     }
-    mbar_init(tmem_full, 1);
-    mbar_init(tmem_empty, kNumEpiThreads);
+    for (int i = 0; i < kAccBufs; ++i) {
+      mbar_init(&tmem_full[i], 1);
+      mbar_init(&tmem_empty[i], kNumEpiThreads);
+    }
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(tmem_ptr_smem, kTmemCols);
@@ -181,7 +207,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
   const int n_items = n_chunks * p.items_per_chunk;
   const int nkb = p.n_kblocks;
   // tuning aid: per work item of CTA 0, slot = clock64 stamp or accumulated wait cycles (see scripts/gemm_trace.py)
-  const bool tracing = p.trace != nullptr && blockIdx.x == 0;
+  const bool tracing = TRACE && blockIdx.x == 0;
   auto stamp = [&](int it, int slot, long long v) {
     if (tracing && it < 16 && (lane == 0 || threadIdx.x == 256)) p.trace[it * 16 + slot] = v;
   };
@@ -200,7 +226,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
         long long wacc = 0;
         for (int kb = 0; kb < nkb; ++kb) {
           const long long c0 = tracing ? clock64() : 0;
-          mbar_wait(&w_empty[rw.stage], rw.phase ^ 1);
+          mbar_wait_paused<64>(&w_empty[rw.stage], rw.phase ^ 1);
           if (tracing) wacc += clock64() - c0;
           uint8_t* dst = smem + L::kOffW + rw.stage * L::kWStageBytes;
           if (elect_one()) {
@@ -223,48 +249,72 @@ __global__ void __launch_bounds__(kNumThreads, 1)
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (whole warp runs the loop, one elected lane issues)
     {
-      Ring ra, rb;
-      uint32_t tphase = 0;
+      Ring ra, rb, racc;
       for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
         const ChunkDesc cd = p.chunks[item / p.items_per_chunk];
         const uint32_t n_pad = (uint32_t)((cd.n_tok + 15) & ~15);
         const uint32_t idesc = umma_idesc_bf16_m128(n_pad);
         const int ti = item / (int)gridDim.x;
         stamp(ti, 0, tracing ? clock64() : 0);
-        mbar_wait(tmem_empty, tphase ^ 1);
+        mbar_wait(&tmem_empty[racc.stage], racc.phase ^ 1);
+        const uint32_t acc_t = tmem_base + racc.stage * 2 * NT;
         tc_fence_after_sync();
         stamp(ti, 1, tracing ? clock64() : 0);
         long long wa = 0, wb = 0;
-        for (int kb = 0; kb < nkb; ++kb) {
+        auto wait_a = [&]() {
           const long long c0 = tracing ? clock64() : 0;
           mbar_wait(&a_full[ra.stage], ra.phase);
-          const long long c1 = tracing ? clock64() : 0;
+          if (tracing) wa += clock64() - c0;
+        };
+        auto wait_b = [&]() {
+          const long long c0 = tracing ? clock64() : 0;
           mbar_wait(&b_full[rb.stage], rb.phase);
-          if (tracing) { wa += c1 - c0; wb += clock64() - c1; }
-          tc_fence_after_sync();
+          if (tracing) wb += clock64() - c0;
+        };
+        wait_b();
+        wait_a();
+        tc_fence_after_sync();
+        for (int kb = 0; kb < nkb; ++kb) {
           const uint32_t a_t = tmem_base + kATmemCol + ra.stage * 2 * kATileCols;
           const uint64_t b0 = umma_desc_k_sw128(smem_u32(smem + L::kOffB + rb.stage * kBStageBytes));
+          uint64_t* const a_done = &a_empty[ra.stage];
+          uint64_t* const b_done = &b_empty[rb.stage];
+          auto issue = [&](int k) {
+            const uint32_t acc = (kb > 0 || k > 0) ? 1u : 0u;
+            umma_bf16_ts(acc_t, a_t + 8 * k, b0 + 2 * k, idesc, acc);
+            umma_bf16_ts(acc_t + kAcc1Col, a_t + kATileCols + 8 * k, b0 + 2 * k, idesc, acc);
+          };
           if (elect_one()) {
-#pragma unroll
-            for (int k = 0; k < kBlockK / 16; ++k) {
-              const uint32_t acc = (kb > 0 || k > 0) ? 1u : 0u;
-              umma_bf16_ts(tmem_base, a_t + 8 * k, b0 + 2 * k, idesc, acc);
-              umma_bf16_ts(tmem_base + kAcc1Col, a_t + kATileCols + 8 * k, b0 + 2 * k, idesc, acc);
-            }
-            umma_commit(&a_empty[ra.stage]);
-            umma_commit(&b_empty[rb.stage]);
+            issue(0);
+            issue(1);
           }
           __syncwarp();
           ra.advance(kStagesA);
           rb.advance(kStagesB);
+          // The next block's operands are waited for under this block's MMAs: the tensor pipe queues only a few of them, and two waits between
+          // blocks (90 cycles each, even on a barrier that has flipped) left it idle for 200 of 840 cycles per block.  The token tile first: it is
+          // there long before the weights, whose TMEM stage the block before this one has only just left.
+          if (kb + 1 < nkb) wait_b();
+          if (elect_one()) issue(2);
+          __syncwarp();
+          if (kb + 1 < nkb) {
+            wait_a();
+            tc_fence_after_sync();
+          }
+          if (elect_one()) {
+            issue(3);
+            umma_commit(a_done);
+            umma_commit(b_done);
+          }
+          __syncwarp();
         }
-        if (elect_one()) umma_commit(tmem_full);
+        if (elect_one()) umma_commit(&tmem_full[racc.stage]);
         __syncwarp();
         stamp(ti, 2, tracing ? clock64() : 0);
         stamp(ti, 3, wa);
         stamp(ti, 4, wb);
         stamp(ti, 14, (long long)cd.n_tok);
-        tphase ^= 1;
+        racc.advance(kAccBufs);
       }
     }
   } else if (warp == 2) {
@@ -277,18 +327,18 @@ __global__ void __launch_bounds__(kNumThreads, 1)
       for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
         const ChunkDesc cd = p.chunks[item / p.items_per_chunk];
         const int n_pad = (cd.n_tok + 15) & ~15;
-        int idx[kMaxChunkTokens / 32];
+        int idx[NT / 32];
 #pragma unroll
-        for (int q = 0; q < kMaxChunkTokens / 32; ++q) idx[q] = (q * 32 + lane < n_pad) ? p.gather_rows[cd.slot_begin + q * 32 + lane] : 0;
+        for (int q = 0; q < NT / 32; ++q) idx[q] = (q * 32 + lane < n_pad) ? p.gather_rows[cd.slot_begin + q * 32 + lane] : 0;
         for (int kb = 0; kb < nkb; ++kb) {
           if (lane == 0) {
-            mbar_wait(&b_empty[rb.stage], rb.phase ^ 1);
+            mbar_wait_paused<64>(&b_empty[rb.stage], rb.phase ^ 1);
             mbar_arrive_expect_tx(&b_full[rb.stage], n_pad * kBlockK * 2);
           }
           __syncwarp();
           uint8_t* dst = smem + L::kOffB + rb.stage * kBStageBytes;
 #pragma unroll
-          for (int q = 0; q < kMaxChunkTokens / 32; ++q) {
+          for (int q = 0; q < NT / 32; ++q) {
             if (q * 32 < n_pad) {
 #pragma unroll
               for (int g = 0; g < 8; ++g) {
@@ -311,7 +361,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
         long long bacc = 0;
         for (int kb = 0; kb < nkb; ++kb) {
           const long long c0 = tracing ? clock64() : 0;
-          mbar_wait(&b_empty[rb.stage], rb.phase ^ 1);
+          mbar_wait_paused<64>(&b_empty[rb.stage], rb.phase ^ 1);
           if (tracing) bacc += clock64() - c0;
           uint8_t* dst = smem + L::kOffB + rb.stage * kBStageBytes;
           if (elect_one()) {
@@ -328,18 +378,24 @@ __global__ void __launch_bounds__(kNumThreads, 1)
     __syncwarp();
   } else if (warp == 3) {
     // idle
-  } else if (warp < 8 || warp >= 12) {
+  } else if (warp < 8 || (warp >= 12 && warp < 24)) {
     // ------------------------------------------------------------ dequantisers -> A operand in TMEM
-    const int tile = warp >= 12 ? 1 : 0;                 // warps 4-7: weight tile 0, warps 12-15: tile 1
+    const int tile = (warp >= 12 && warp < 16) || warp >= 20 ? 1 : 0;
+    const int odd = warp >= 16;                          // the k-blocks of this group, counted over all items
     const int t = (warp & 3) * 32 + lane;                // weight row within the tile == TMEM lane
     Ring rw, ra;
+    int first = odd;
+    if (odd) {
+      rw.advance(kStagesW);
+      ra.advance(kStagesA);
+    }
     const uint32_t lane_base = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kATmemCol + tile * kATileCols;
     const bool dtr = tracing && threadIdx.x == 128;
     for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
       long long ww_ = 0, wae = 0, wst = 0;
-      for (int kb = 0; kb < nkb; ++kb) {
+      for (int kb = first; kb < nkb; kb += 2) {
         const long long c0 = dtr ? clock64() : 0;
-        mbar_wait(&w_full[rw.stage], rw.phase);
+        mbar_wait_paused<32>(&w_full[rw.stage], rw.phase);
         if (dtr) ww_ += clock64() - c0;
         const uint8_t* wsrc = smem + L::kOffW + rw.stage * L::kWStageBytes;
         __nv_bfloat16 s = __float2bfloat16_rn(0.f);
@@ -357,10 +413,8 @@ __global__ void __launch_bounds__(kNumThreads, 1)
             const float sf = q < 2 ? d0 : d1;
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-              const uint32_t word = ww[e >> 1];
-              const int b0 = (int)(int8_t)((word >> ((e & 1) * 16)) & 0xFF);
-              const int b1 = (int)(int8_t)((word >> ((e & 1) * 16 + 8)) & 0xFF);
-              __nv_bfloat162 v = __floats2bfloat162_rn((float)b0 * sf, (float)b1 * sf);
+              const float2 c = s8_pair(ww[e >> 1], e & 1);
+              __nv_bfloat162 v = __floats2bfloat162_rn(c.x * sf, c.y * sf);
               o[q * 8 + e] = *reinterpret_cast<uint32_t*>(&v);
             }
           }
@@ -376,10 +430,8 @@ __global__ void __launch_bounds__(kNumThreads, 1)
             const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-              const uint32_t word = ww[e >> 1];
-              const int b0 = (int)(int8_t)((word >> ((e & 1) * 16)) & 0xFF);
-              const int b1 = (int)(int8_t)((word >> ((e & 1) * 16 + 8)) & 0xFF);
-              __nv_bfloat162 v = __floats2bfloat162_rn(fmaf(av[q], (float)b0, -bv[q]), fmaf(av[q], (float)b1, -bv[q]));
+              const float2 c = s8_pair(ww[e >> 1], e & 1);
+              __nv_bfloat162 v = __floats2bfloat162_rn(fmaf(av[q], c.x, -bv[q]), fmaf(av[q], c.y, -bv[q]));
               o[q * 8 + e] = *reinterpret_cast<uint32_t*>(&v);
             }
           }
@@ -420,32 +472,26 @@ __global__ void __launch_bounds__(kNumThreads, 1)
             const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              o[h * 16 + j * 4 + 0] = deq_pair_int4(ww[j], s2);
-              o[h * 16 + j * 4 + 1] = deq_pair_int4(ww[j] >> 4, s2);
-              o[h * 16 + j * 4 + 2] = deq_pair_int4(ww[j] >> 8, s2);
-              o[h * 16 + j * 4 + 3] = deq_pair_int4(ww[j] >> 12, s2);
+              o[h * 16 + j * 4 + 0] = deq_pair_int4(ww[j], p.magic, s2);
+              o[h * 16 + j * 4 + 1] = deq_pair_int4(ww[j] >> 4, p.magic, s2);
+              o[h * 16 + j * 4 + 2] = deq_pair_int4(ww[j] >> 8, p.magic, s2);
+              o[h * 16 + j * 4 + 3] = deq_pair_int4(ww[j] >> 12, p.magic, s2);
             }
           }
         } else {
           // INT8 tile: [quarter q in 0..3][row][16 B], 16 consecutive K columns per 16 B
-          const float sf = __bfloat162float(s);
+          const __nv_bfloat162 s2 = __halves2bfloat162(s, s);
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const uint4 w = *reinterpret_cast<const uint4*>(wsrc + tile * TB + q * 2048 + t * 16);
             const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const uint32_t word = ww[e >> 1];
-              const int b0 = (int)(int8_t)((word >> ((e & 1) * 16)) & 0xFF);
-              const int b1 = (int)(int8_t)((word >> ((e & 1) * 16 + 8)) & 0xFF);
-              __nv_bfloat162 v = __floats2bfloat162_rn((float)b0 * sf, (float)b1 * sf);
-              o[q * 8 + e] = *reinterpret_cast<uint32_t*>(&v);
-            }
+            for (int e = 0; e < 8; ++e) o[q * 8 + e] = deq_pair_int8(ww[e >> 1], e & 1, s2);
           }
         }
         mbar_arrive(&w_empty[rw.stage]);     // packed words are now in registers
         const long long c1 = dtr ? clock64() : 0;
-        mbar_wait(&a_empty[ra.stage], ra.phase ^ 1);
+        mbar_wait_paused<32>(&a_empty[ra.stage], ra.phase ^ 1);
         const long long c2 = dtr ? clock64() : 0;
         tc_fence_after_sync();
         tmem_st32(lane_base + ra.stage * 2 * kATileCols, o);
@@ -453,9 +499,10 @@ __global__ void __launch_bounds__(kNumThreads, 1)
         tc_fence_before_sync();
         mbar_arrive(&a_full[ra.stage]);
         if (dtr) { wae += c2 - c1; wst += clock64() - c2; }
-        rw.advance(kStagesW);
-        ra.advance(kStagesA);
+        rw.advance2(kStagesW);
+        ra.advance2(kStagesA);
       }
+      first ^= nkb & 1;
       if (dtr) {
         const int ti = item / (int)gridDim.x;
         stamp(ti, 8, ww_); stamp(ti, 9, wae); stamp(ti, 10, wst); stamp(ti, 11, clock64());
@@ -468,10 +515,11 @@ __global__ void __launch_bounds__(kNumThreads, 1)
     // Phase 2: staging -> (GEMM1: SiLU(gate)*up) -> 16 B coalesced global stores.
     const int q = warp & 3;                    // TMEM lane quadrant this warp may access
     const int row = q * 32 + lane;             // weight row within the 128-row tile
-    const int et = threadIdx.x - 256;          // 0..127
+    const int tile = warp >= 24;
+    const int et = (threadIdx.x & 127) + tile * 128;
     uint8_t* stage = smem + L::kOffStage;
     constexpr int kRowB = L::kStageRowBytes;   // 512
-    uint32_t tphase = 0;
+    Ring racc;
     for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
       const ChunkDesc cd = p.chunks[item / p.items_per_chunk];
       const int rt = item % p.items_per_chunk;
@@ -481,20 +529,17 @@ __global__ void __launch_bounds__(kNumThreads, 1)
         // drain loop made phase 1 of the down projection 3x longer than the gate/up one: profiles/r02h_gemm_item_timeline.txt)
         float* sw = reinterpret_cast<float*>(smem + L::kOffSlotW);
         for (int i = et; i < n_pad; i += kNumEpiThreads) sw[i] = (i < cd.n_tok) ? p.slot_weight[cd.slot_begin + i] : 0.f;
-        named_bar_sync(1, kNumEpiThreads);
       }
-      mbar_wait(tmem_full, tphase);
+      if (et < 32) mbar_wait_paused<32>(&tmem_full[racc.stage], racc.phase);      // one warp polls, seven sleep at the barrier
+      named_bar_sync(1, kNumEpiThreads);
       tc_fence_after_sync();
       const bool etr = tracing && et == 0;
       const int ti = item / (int)gridDim.x;
       if (etr) stamp(ti, 5, clock64());
-      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
+      const uint32_t taddr = tmem_base + racc.stage * 2 * NT + ((uint32_t)(q * 32) << 16);
       // 16 accumulator columns (tokens) per step, software-pipelined over two register sets: the tcgen05.ld of the next step is in
       // flight while this step is rounded to BF16 and staged (the exposed TMEM load latency was ~1/3 of this phase, which holds TMEM)
-      auto load_cols = [&](int c0, uint32_t (&a)[16], uint32_t (&b)[16]) {
-        tmem_ld16(taddr + c0, a);
-        tmem_ld16(taddr + kAcc1Col + c0, b);
-      };
+      const uint32_t tcol = taddr + tile * kAcc1Col;
       auto load_weights = [&](int c0, float (&wv)[16]) {
         if constexpr (!kGemm1) {
           // routing weights of the column group, loaded BEFORE the staging stores of the step (a shared-memory load cannot be moved
@@ -507,42 +552,36 @@ __global__ void __launch_bounds__(kNumThreads, 1)
           }
         }
       };
-      auto stage_cols = [&](int c0, const uint32_t (&a)[16], const uint32_t (&b)[16], const float (&wv)[16]) {
+      auto stage_cols = [&](int c0, const uint32_t (&a)[16], const float (&wv)[16]) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          float v0 = __uint_as_float(a[j]);
-          float v1 = __uint_as_float(b[j]);
-          if constexpr (!kGemm1) {
-            v0 *= wv[j];
-            v1 *= wv[j];
-          }
-          __nv_bfloat16* srow = reinterpret_cast<__nv_bfloat16*>(stage + (c0 + j) * kRowB);
-          srow[row] = __float2bfloat16_rn(v0);
-          srow[kTileRows + row] = __float2bfloat16_rn(v1);
+          float v = __uint_as_float(a[j]);
+          if constexpr (!kGemm1) v *= wv[j];
+          reinterpret_cast<__nv_bfloat16*>(stage + (c0 + j) * kRowB)[tile * kTileRows + row] = __float2bfloat16_rn(v);
         }
       };
       {
-        uint32_t a0[16], b0[16], a1[16], b1[16];
-        float w0[16], w1[16];
-        load_cols(0, a0, b0);
+        uint32_t a0[16], a1[16];
+        float wv[16];
+        tmem_ld16(tcol, a0);
         for (int c0 = 0; c0 < n_pad; c0 += 32) {
           const bool second = c0 + 16 < n_pad;
-          load_weights(c0, w0);
-          if (second) load_weights(c0 + 16, w1);
+          load_weights(c0, wv);
           tmem_ld_wait();                                      // set 0 is in registers
-          if (second) load_cols(c0 + 16, a1, b1);
-          stage_cols(c0, a0, b0, w0);
+          if (second) tmem_ld16(tcol + c0 + 16, a1);
+          stage_cols(c0, a0, wv);
           if (second) {
+            load_weights(c0 + 16, wv);
             tmem_ld_wait();                                    // set 1 is in registers
-            if (c0 + 32 < n_pad) load_cols(c0 + 32, a0, b0);
-            stage_cols(c0 + 16, a1, b1, w1);
+            if (c0 + 32 < n_pad) tmem_ld16(tcol + c0 + 32, a0);
+            stage_cols(c0 + 16, a1, wv);
           }
         }
       }
       tc_fence_before_sync();
-      mbar_arrive(tmem_empty);                 // accumulators drained: the next tile's MMAs may start
+      mbar_arrive(&tmem_empty[racc.stage]);    // accumulators drained: the next tile's MMAs may start
       if (etr) stamp(ti, 6, clock64());
-      tphase ^= 1;
+      racc.advance(kAccBufs);
       named_bar_sync(1, kNumEpiThreads);       // staging tile complete
       if constexpr (kGemm1) {
         // 16 outputs per step: gate chunk v and up chunk v of one token -> 8 activations (16 B store)
@@ -636,10 +675,10 @@ cudaError_t make_tmap_bf16_gather(void* out_tmap, const void* base, long long ro
   return make_tmap_bf16_rows(out_tmap, base, rows, cols, 1);
 }
 
-template <int FMT, bool kGemm1>
-static cudaError_t launch_one(const GemmParams& p, const CUtensorMap& tmap, int num_sms, cudaStream_t stream) {
-  auto kern = grouped_gemm_kernel<FMT, kGemm1>;
-  constexpr int smem = SmemLayout<FMT, kGemm1>::kTotal;
+template <int FMT, bool kGemm1, int NT, bool TRACE>
+static cudaError_t launch_kernel(const GemmParams& p, const CUtensorMap& tmap, int num_sms, cudaStream_t stream, long long* trace) {
+  auto kern = grouped_gemm_kernel<FMT, kGemm1, NT, TRACE>;
+  constexpr int smem = SmemLayout<FMT, kGemm1, NT>::kTotal;
   static PerDeviceOnce once;
   if (const int dev = once.pending(); dev >= 0) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -648,32 +687,35 @@ static cudaError_t launch_one(const GemmParams& p, const CUtensorMap& tmap, int 
   }
   KernelSpan ks(kGemm1 ? K_GEMM1_GATE_UP : K_GEMM2_DOWN, stream);
   GemmParams pp = p;
-  const char* tv = getenv(kGemm1 ? "KB2_GEMM1_TRACE" : "KB2_GEMM2_TRACE");      // tuning only: device pointer to [16][16] int64
-  pp.trace = tv ? reinterpret_cast<long long*>(strtoull(tv, nullptr, 0)) : nullptr;
+  pp.trace = trace;
+  pp.magic = 0x43004300u;
   kern<<<num_sms, kNumThreads, smem, stream>>>(pp, tmap);
   return cudaGetLastError();
 }
 
-cudaError_t launch_grouped_gemm(int fmt, bool gemm1, const GemmParams& p, const void* tmap_b, int num_sms,
+template <int FMT, bool kGemm1, int NT>
+static cudaError_t launch_one(const GemmParams& p, const CUtensorMap& tmap, int num_sms, cudaStream_t stream) {
+  const char* tv = getenv(kGemm1 ? "KB2_GEMM1_TRACE" : "KB2_GEMM2_TRACE");      // tuning only: device pointer to [16][16] int64
+  if (tv) return launch_kernel<FMT, kGemm1, NT, true>(p, tmap, num_sms, stream, reinterpret_cast<long long*>(strtoull(tv, nullptr, 0)));
+  return launch_kernel<FMT, kGemm1, NT, false>(p, tmap, num_sms, stream, nullptr);
+}
+template <int FMT>
+static cudaError_t launch_format(bool gemm1, int chunk_tokens, const GemmParams& p, const CUtensorMap& tm, int num_sms, cudaStream_t s) {
+  if (chunk_tokens == kShortChunkTokens)
+    return gemm1 ? launch_one<FMT, true, kShortChunkTokens>(p, tm, num_sms, s) : launch_one<FMT, false, kShortChunkTokens>(p, tm, num_sms, s);
+  return gemm1 ? launch_one<FMT, true, kMaxChunkTokens>(p, tm, num_sms, s) : launch_one<FMT, false, kMaxChunkTokens>(p, tm, num_sms, s);
+}
+
+// chunk_tokens: kMaxChunkTokens or kShortChunkTokens, the limit that the chunks in p were cut with
+cudaError_t launch_grouped_gemm(int fmt, bool gemm1, int chunk_tokens, const GemmParams& p, const void* tmap_b, int num_sms,
                                 cudaStream_t stream) {
   const CUtensorMap& tm = *reinterpret_cast<const CUtensorMap*>(tmap_b);
-  if (fmt == kFmtInt4G128) {
-    return gemm1 ? launch_one<kFmtInt4G128, true>(p, tm, num_sms, stream)
-                 : launch_one<kFmtInt4G128, false>(p, tm, num_sms, stream);
-  }
-  if (fmt == kFmtInt8G128) {
-    return gemm1 ? launch_one<kFmtInt8G128, true>(p, tm, num_sms, stream)
-                 : launch_one<kFmtInt8G128, false>(p, tm, num_sms, stream);
-  }
-  if (fmt == kFmtQ8_0) {
-    return gemm1 ? launch_one<kFmtQ8_0, true>(p, tm, num_sms, stream) : launch_one<kFmtQ8_0, false>(p, tm, num_sms, stream);
-  }
-  if (fmt == kFmtQ4_K) {
-    return gemm1 ? launch_one<kFmtQ4_K, true>(p, tm, num_sms, stream) : launch_one<kFmtQ4_K, false>(p, tm, num_sms, stream);
-  }
-  if (fmt >= kFmtAffine8 && fmt <= kFmtQ4_0) {      // Q6_K / Q5_K / Q5_0 / Q4_0 share the decoded-affine tile kernel
-    return gemm1 ? launch_one<kFmtAffine8, true>(p, tm, num_sms, stream) : launch_one<kFmtAffine8, false>(p, tm, num_sms, stream);
-  }
+  if (fmt == kFmtInt4G128) return launch_format<kFmtInt4G128>(gemm1, chunk_tokens, p, tm, num_sms, stream);
+  if (fmt == kFmtInt8G128) return launch_format<kFmtInt8G128>(gemm1, chunk_tokens, p, tm, num_sms, stream);
+  if (fmt == kFmtQ8_0) return launch_format<kFmtQ8_0>(gemm1, chunk_tokens, p, tm, num_sms, stream);
+  if (fmt == kFmtQ4_K) return launch_format<kFmtQ4_K>(gemm1, chunk_tokens, p, tm, num_sms, stream);
+  if (fmt >= kFmtAffine8 && fmt <= kFmtQ4_0)        // Q6_K / Q5_K / Q5_0 / Q4_0 share the decoded-affine tile kernel
+    return launch_format<kFmtAffine8>(gemm1, chunk_tokens, p, tm, num_sms, stream);
   return cudaErrorInvalidValue;
 }
 

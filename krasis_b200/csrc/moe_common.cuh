@@ -69,15 +69,16 @@ constexpr int kQ4KTileBytes = kTileRows * kBlockK / 2 + kTileRows * 8; // 5120
 //   Affine8 (128 rows x 64 K): [quarter 0..3][row][16 B] int8 codes (8192 B) | [row][4 x (a f32, b f32)] one pair per 16 elements (4096 B)
 constexpr int kAffine8TileBytes = kTileRows * kBlockK + kTileRows * 32;  // 12288
 
-// One unit of grouped-GEMM work along the token axis: a run of <= kMaxChunkTokens sorted slots of one expert.
+// One unit of grouped-GEMM work along the token axis: a run of <= kMaxChunkTokens (kShortChunkTokens) sorted slots of one expert.
 struct ChunkDesc {
   int expert;      // local expert index
   int slot_begin;  // first sorted slot
-  int n_tok;       // real token slots in this chunk (1..kMaxChunkTokens)
+  int n_tok;       // real token slots in this chunk (1..the limit they were cut with)
   int pad_;
 };
 
 constexpr int kMaxChunkTokens = 192;   // UMMA N per chunk; 2 accumulators x 192 + 2 A stages x 64 = 512 TMEM columns
+constexpr int kShortChunkTokens = 64;  // short chunks: 4 accumulators x 64 + 4 A stages x 64
 
 struct GemmParams {
   const uint8_t* wq;          // packed tiles, all local experts
@@ -95,6 +96,7 @@ struct GemmParams {
   const float* slot_weight;   // GEMM2: routing weight per sorted slot
   const int* gather_rows;     // GEMM1, gather mode: token row of every sorted slot (the B operand is fetched from the caller's
                               // activation matrix with TMA gather4 instead of a pre-sorted copy); nullptr = B rows are contiguous
+  uint32_t magic;             // set by the launcher
   long long* trace;           // optional (tuning only, KB2_GEMM_TRACE=<device pointer>): clock64 stamps of CTA 0, [item < 16][16]
 };
 

@@ -123,36 +123,65 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const float* __restric
     const int e = i * 32 + lane;
     key[i] = e < E ? score[i] + ((corr_bias && scoring != 2) ? corr_bias[e] : 0.f) : -INFINITY;
   }
+  // Best key of each group of PG of the lane's keys: a round takes one key, so only that key's group and the comparison of the groups are done
+  // again, and the warp agrees by two integer reductions (largest key, then smallest index among equals).  8192 x 512, ten choices: 31 -> 22 us
+  // (all keys and a shuffle tree per round before); the choices, exponentials and divisions are bound by issue.
+  constexpr int PG = PER_LANE < 4 ? PER_LANE : 4, NG = PER_LANE / PG;
+  float gv[NG];
+  int gi[NG];
+#pragma unroll
+  for (int g = 0; g < NG; ++g) {
+    gv[g] = -INFINITY;
+    gi[g] = 0x7fffffff;
+#pragma unroll
+    for (int i = g * PG; i < g * PG + PG; ++i)   // ascending expert index within the lane: strict '>' keeps the lower index
+      if (key[i] > gv[g]) {
+        gv[g] = key[i];
+        gi[g] = i * 32 + lane;
+      }
+  }
+  unsigned taken = 0;                            // of this lane's keys
   float wsum = 0.f, my_w = 0.f;
   int my_id = 0;
   float first_val = 0.f;
   for (int j = 0; j < top_k; ++j) {
-    float bv = -INFINITY;
-    int bi = 0x7fffffff;
+    float bv = gv[0];
+    int bi = gi[0];
+#pragma unroll
+    for (int g = 1; g < NG; ++g)
+      if (gv[g] > bv) {
+        bv = gv[g];
+        bi = gi[g];
+      }
+    const unsigned bits = __float_as_uint(bv + 0.f);                     // -0 counts as +0
+    const unsigned ord = bits & 0x80000000u ? ~bits : bits | 0x80000000u;
+    const unsigned top = __reduce_max_sync(0xffffffffu, ord);
+    bi = (int)__reduce_min_sync(0xffffffffu, ord == top ? (unsigned)bi : 0x7fffffffu);
+    const int wi = bi >> 5, G = wi / PG;                                 // uniform; past every group where no key is left
+    if ((bi & 31) == lane) taken |= 1u << (wi & 31);
+    float q[PG], v = -INFINITY;                                          // the group again, without what was taken
+    int vi = 0x7fffffff;
+#pragma unroll
+    for (int i = 0; i < PG; ++i) {
+      q[i] = key[i];
+#pragma unroll
+      for (int g = 1; g < NG; ++g) q[i] = G == g ? key[g * PG + i] : q[i];
+      const bool better = q[i] > v && !(taken >> ((G * PG + i) & 31) & 1u);
+      v = better ? q[i] : v;
+      vi = better ? (G * PG + i) * 32 + lane : vi;
+    }
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+      gv[g] = G == g ? v : gv[g];
+      gi[g] = G == g ? vi : gi[g];
+    }
     float bs = 0.f;
+    if (corr_bias && scoring != 2) {                                     // the key is not the score
 #pragma unroll
-    for (int i = 0; i < PER_LANE; ++i) {       // ascending expert index within the lane: strict '>' keeps the lower index
-      if (key[i] > bv) {
-        bv = key[i];
-        bi = i * 32 + lane;
-        bs = score[i];
-      }
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      const float os = __shfl_xor_sync(0xffffffffu, bs, o);
-      if (ov > bv || (ov == bv && oi < bi)) {
-        bv = ov;
-        bi = oi;
-        bs = os;
-      }
-    }
-    if ((bi & 31) == lane) {
-#pragma unroll
-      for (int i = 0; i < PER_LANE; ++i)
-        if (i == (bi >> 5)) key[i] = -INFINITY;
+      for (int i = 0; i < PER_LANE; ++i) bs = wi == i ? score[i] : bs;
+      bs = __shfl_sync(0xffffffffu, bs, bi & 31);
+    } else if (bi != 0x7fffffff) {
+      bs = __uint_as_float(top & 0x80000000u ? top & 0x7fffffffu : ~top);
     }
     float wj = bs;
     if (scoring == 2) {
@@ -175,21 +204,45 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const float* __restric
 // ------------------------------------------------------------------------------------------------
 // Binning: count -> scan (+ chunk descriptors) -> scatter
 // ------------------------------------------------------------------------------------------------
-__global__ void count_kernel(const int* __restrict__ ids, int n, int e_start, int e_end, int* __restrict__ counts) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int e = ids[i];
-  if (e >= e_start && e < e_end) atomicAdd(&counts[e - e_start], 1);
+// 4096 entries per block are counted in shared memory first: one global atomic per entry met 160 others on its counter (12 us for 81920 entries).
+constexpr int kCountPerBlock = 4096;
+__global__ void __launch_bounds__(1024) count_kernel(const int* __restrict__ ids, int n, int e_start, int e_end, int* __restrict__ counts) {
+  __shared__ int s_cnt[1024];
+  s_cnt[threadIdx.x] = 0;
+  __syncthreads();
+  const int E = e_end - e_start;
+#pragma unroll
+  for (int r = 0; r < kCountPerBlock / 1024; ++r) {
+    const int i = blockIdx.x * kCountPerBlock + r * 1024 + threadIdx.x;
+    const int e = i < n ? ids[i] : -1;
+    if (i < n && e >= e_start && e < e_end) atomicAdd(&s_cnt[e - e_start], 1);
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < E && s_cnt[threadIdx.x]) atomicAdd(&counts[threadIdx.x], s_cnt[threadIdx.x]);
+}
+
+// The c slots of expert e from `off` as nch chunks of about the same size, a multiple of 16.
+__device__ __forceinline__ void write_chunks(ChunkDesc* chunks, int e, int off, int c, int nch) {
+  if (nch == 0) return;
+  const int per = ((c + nch - 1) / nch + 15) & ~15;
+  for (int i = 0; i < nch; ++i) {
+    ChunkDesc d;
+    d.expert = e;
+    d.slot_begin = off + i * per;
+    d.n_tok = min(per, c - i * per);
+    d.pad_ = 0;
+    chunks[i] = d;
+  }
 }
 
 // single block of 1024 threads; E_local <= 1024
-__global__ void __launch_bounds__(1024) scan_kernel(const int* __restrict__ counts, int E, int* __restrict__ offsets,
+__global__ void __launch_bounds__(1024) scan_kernel(const int* __restrict__ counts, int E, int chunk_tokens, int* __restrict__ offsets,
                                                     int* __restrict__ cursor, ChunkDesc* __restrict__ chunks,
                                                     int* __restrict__ n_chunks) {
   __shared__ int s_cnt[1024], s_chk[1024];
   const int t = threadIdx.x;
   const int c = t < E ? counts[t] : 0;
-  const int nch = (c + kMaxChunkTokens - 1) / kMaxChunkTokens;
+  const int nch = (c + chunk_tokens - 1) / chunk_tokens;
   s_cnt[t] = c;
   s_chk[t] = nch;
   __syncthreads();
@@ -208,23 +261,103 @@ __global__ void __launch_bounds__(1024) scan_kernel(const int* __restrict__ coun
   if (t < E) {
     offsets[t] = off;
     cursor[t] = 0;
-    if (nch > 0) {
-      int per = (c + nch - 1) / nch;
-      per = (per + 15) & ~15;
-      for (int i = 0; i < nch; ++i) {
-        ChunkDesc d;
-        d.expert = t;
-        d.slot_begin = off + i * per;
-        d.n_tok = min(per, c - i * per);
-        d.pad_ = 0;
-        chunks[choff + i] = d;
-      }
-    }
+    write_chunks(chunks + choff, t, off, c, nch);
   }
   if (t == 1023) {
     offsets[E] = s_cnt[1023];
     *n_chunks = s_chk[1023];
   }
+}
+
+// Up to kBinRowsMax entries: the whole binning and the row copies in one launch.  Every block counts all entries in shared memory and scans the
+// counters by itself, so blocks need nothing from one another; a warp finds its entry's place in the expert's run by counting the equal ids before
+// it (a stable order), and copies the row.  Block 0 also writes the tables.  Past kBinRowsMax the counting, n^2 / 32 reads in all, is worth more
+// than the three launches that it saves.
+constexpr int kBinRowsMax = 4096;
+__global__ void __launch_bounds__(256) bin_rows_kernel(const int* __restrict__ ids, const float* __restrict__ wts, int n, int top_k, int e_start,
+                                                       int E, int chunk_tokens, int* __restrict__ counts, int* __restrict__ offsets,
+                                                       ChunkDesc* __restrict__ chunks, int* __restrict__ n_chunks, float* __restrict__ sorted_w,
+                                                       int* __restrict__ slot_of, int* __restrict__ sorted_ids, int* __restrict__ sorted_tok,
+                                                       const uint4* __restrict__ x, uint4* __restrict__ x_sorted, int vec_per_row) {
+  __shared__ short s_id[kBinRowsMax];
+  __shared__ int s_cnt[1024], s_off[1024], s_warp[2][8];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) s_cnt[i * 256 + t] = 0;
+  __syncthreads();
+  for (int i = t; i < n; i += 256) {
+    const int e = ids[i] - e_start;
+    const bool mine = ids[i] >= e_start && e < E;
+    s_id[i] = mine ? (short)e : (short)-1;
+    if (mine) atomicAdd(&s_cnt[e], 1);
+  }
+  __syncthreads();
+  // exclusive scans over the experts, four per thread: slots, and (high half) chunks
+  int c[4], nch[4], sum_c = 0, sum_n = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    c[i] = s_cnt[t * 4 + i];
+    nch[i] = (c[i] + chunk_tokens - 1) / chunk_tokens;
+    sum_c += c[i];
+    sum_n += nch[i];
+  }
+  int in_c = sum_c, in_n = sum_n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, in_c, o), b = __shfl_up_sync(0xffffffffu, in_n, o);
+    if (lane >= o) {
+      in_c += a;
+      in_n += b;
+    }
+  }
+  if (lane == 31) {
+    s_warp[0][warp] = in_c;
+    s_warp[1][warp] = in_n;
+  }
+  __syncthreads();
+  int off = in_c - sum_c, choff = in_n - sum_n;
+  for (int w = 0; w < warp; ++w) {
+    off += s_warp[0][w];
+    choff += s_warp[1][w];
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int e = t * 4 + i;
+    s_off[e] = off;
+    if (blockIdx.x == 0 && e < E) {
+      counts[e] = c[i];
+      offsets[e] = off;
+      write_chunks(chunks + choff, e, off, c[i], nch[i]);
+    }
+    off += c[i];
+    choff += nch[i];
+  }
+  if (blockIdx.x == 0 && t == 255) {
+    offsets[E] = off;
+    *n_chunks = choff;
+  }
+  __syncthreads();
+  const int i = blockIdx.x * 8 + warp;
+  if (i >= n) return;
+  const int e = s_id[i];
+  if (e < 0) {
+    if (lane == 0) slot_of[i] = -1;
+    return;
+  }
+  int before = 0;
+  for (int j = lane; j < i; j += 32) before += s_id[j] == e;
+  const int slot = s_off[e] + __reduce_add_sync(0xffffffffu, before);
+  if (lane == 0) {
+    slot_of[i] = slot;
+    sorted_w[slot] = wts[i];
+    if (sorted_ids) sorted_ids[slot] = e + e_start;
+    if (sorted_tok) sorted_tok[slot] = i / top_k;
+  }
+  if (!x_sorted) return;
+  const uint4* src = x + (long long)(i / top_k) * vec_per_row;
+  uint4* dst = x_sorted + (long long)slot * vec_per_row;
+#pragma unroll 4
+  for (int v = lane; v < vec_per_row; v += 32) dst[v] = src[v];
 }
 
 // Token scatter: one warp per (token, k) routing entry.  Lane 0 claims a slot in the expert's contiguous run,
@@ -278,25 +411,35 @@ __global__ void __launch_bounds__(256) scatter_index_kernel(const int* __restric
 
 // ------------------------------------------------------------------------------------------------
 // Combine: out[m] = bf16( sum_j f32(c3[slot_of[m][j]]) ) in j order; then bf16(rsf*out) (+ shared)
-// one thread = 8 consecutive h (16 B)
+// one thread = 8 consecutive h (16 B); four rows in flight per thread (8192 x 10 rows of 4 KB: 67 us, 5.5 TB/s; one
+// after the other 82 us)
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) combine_kernel(const __nv_bfloat16* __restrict__ c3,
+constexpr int kCombineThreads = 128;
+__global__ void __launch_bounds__(kCombineThreads) combine_kernel(const __nv_bfloat16* __restrict__ c3,
                                                       const int* __restrict__ slot_of, int M, int H, int top_k,
                                                       float rsf, int apply_rsf,
                                                       const __nv_bfloat16* __restrict__ shared,
                                                       __nv_bfloat16* __restrict__ out, CombineScatter sc) {
   const int vec_per_row = H >> 3;
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)M * vec_per_row) return;
-  const int m = (int)(idx / vec_per_row), v = (int)(idx % vec_per_row);
+  const int m = blockIdx.x, v = blockIdx.y * kCombineThreads + threadIdx.x;
+  if (v >= vec_per_row) return;
   float acc[8] = {};
-  for (int j = 0; j < top_k; ++j) {
-    const int slot = slot_of ? slot_of[(long long)m * top_k + j] : m * top_k + j;     // no table: rows already in token order
-    if (slot < 0) continue;
-    const uint4 x = *reinterpret_cast<const uint4*>(c3 + (long long)slot * H + v * 8);
-    const __nv_bfloat16* px = reinterpret_cast<const __nv_bfloat16*>(&x);
+  for (int j0 = 0; j0 < top_k; j0 += 4) {
+    int slot[4];
+    uint4 x[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] += __bfloat162float(px[i]);
+    for (int j = 0; j < 4; ++j)
+      slot[j] = j0 + j >= top_k ? -1 : slot_of ? slot_of[(long long)m * top_k + j0 + j] : m * top_k + j0 + j;   // no table: rows already in token order
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (slot[j] >= 0) x[j] = *reinterpret_cast<const uint4*>(c3 + (long long)slot[j] * H + v * 8);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (slot[j] < 0) continue;
+      const __nv_bfloat16* px = reinterpret_cast<const __nv_bfloat16*>(&x[j]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] += __bfloat162float(px[i]);
+    }
   }
   uint4 sh = make_uint4(0, 0, 0, 0);
   if (shared) sh = *reinterpret_cast<const uint4*>(shared + (long long)m * H + v * 8);
@@ -588,33 +731,29 @@ cudaError_t launch_router_topk(const float* logits, const float* corr_bias, int 
   return cudaGetLastError();
 }
 
-cudaError_t launch_binning(const int* ids, const float* wts, int M, int top_k, int e_start, int e_end, int* counts,
+// kernels that a binning of n entries launches
+int binning_launches(long long n) { return n > 0 && n <= kBinRowsMax ? 1 : 3; }
+
+// chunk_tokens: the most slots of one chunk.  Either x_sorted (rows copied into their slots) or sorted_tok (their indices recorded) is given.
+cudaError_t launch_binning(const int* ids, const float* wts, int M, int top_k, int e_start, int e_end, int chunk_tokens, int* counts,
                            int* offsets, int* cursor, ChunkDesc* chunks, int* n_chunks, float* sorted_w, int* slot_of,
-                           int* sorted_ids, const void* x, void* x_sorted, int H, cudaStream_t s) {
-  KernelSpan ks(K_BINNING, s, 3);
+                           int* sorted_ids, int* sorted_tok, const void* x, void* x_sorted, int H, cudaStream_t s) {
   const int n = M * top_k, E = e_end - e_start;
+  KernelSpan ks(K_BINNING, s, binning_launches(n));
   if (E > 1024) return cudaErrorInvalidValue;
+  if (n > 0 && n <= kBinRowsMax) {      // measured with 2048 columns: 24 entries 9.3 -> 4.1 us (memset, count, scan, scatter before), 2334 entries 13 -> 6.6 us
+    bin_rows_kernel<<<(n + 7) / 8, 256, 0, s>>>(ids, wts, n, top_k, e_start, E, chunk_tokens, counts, offsets, chunks, n_chunks, sorted_w, slot_of,
+                                                sorted_ids, sorted_tok, (const uint4*)x, (uint4*)x_sorted, H / 8);
+    return cudaGetLastError();
+  }
   cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(int) * E, s);
   if (e != cudaSuccess) return e;
-  if (n > 0) count_kernel<<<(n + 255) / 256, 256, 0, s>>>(ids, n, e_start, e_end, counts);
-  scan_kernel<<<1, 1024, 0, s>>>(counts, E, offsets, cursor, chunks, n_chunks);
-  if (n > 0)
+  if (n > 0) count_kernel<<<(n + kCountPerBlock - 1) / kCountPerBlock, 1024, 0, s>>>(ids, n, e_start, e_end, counts);
+  scan_kernel<<<1, 1024, 0, s>>>(counts, E, chunk_tokens, offsets, cursor, chunks, n_chunks);
+  if (n > 0 && x_sorted)
     scatter_kernel<<<(n + 7) / 8, 256, 0, s>>>(ids, wts, n, top_k, e_start, e_end, offsets, cursor, sorted_w, slot_of,
                                                sorted_ids, (const uint4*)x, (uint4*)x_sorted, H / 8);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_binning_index(const int* ids, const float* wts, int M, int top_k, int e_start, int e_end, int* counts,
-                                 int* offsets, int* cursor, ChunkDesc* chunks, int* n_chunks, float* sorted_w, int* slot_of,
-                                 int* sorted_tok, cudaStream_t s) {
-  KernelSpan ks(K_BINNING, s, 3);
-  const int n = M * top_k, E = e_end - e_start;
-  if (E > 1024) return cudaErrorInvalidValue;
-  cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(int) * E, s);
-  if (e != cudaSuccess) return e;
-  if (n > 0) count_kernel<<<(n + 255) / 256, 256, 0, s>>>(ids, n, e_start, e_end, counts);
-  scan_kernel<<<1, 1024, 0, s>>>(counts, E, offsets, cursor, chunks, n_chunks);
-  if (n > 0)
+  else if (n > 0)
     scatter_index_kernel<<<(n + 255) / 256, 256, 0, s>>>(ids, wts, n, top_k, e_start, e_end, offsets, cursor, sorted_w, slot_of,
                                                          sorted_tok);
   return cudaGetLastError();
@@ -623,9 +762,8 @@ cudaError_t launch_binning_index(const int* ids, const float* wts, int M, int to
 cudaError_t launch_combine_scatter(const void* c3, const int* slot_of, int M, int H, int top_k, float rsf, int apply_rsf,
                                    const void* shared, void* out, const CombineScatter& sc, cudaStream_t s) {
   KernelSpan ks(K_COMBINE, s);
-  const long long total = (long long)M * (H / 8);
-  if (total == 0) return cudaSuccess;
-  combine_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>((const __nv_bfloat16*)c3, slot_of, M, H, top_k, rsf,
+  if (M <= 0 || H < 8) return cudaSuccess;
+  combine_kernel<<<dim3(M, (H / 8 + kCombineThreads - 1) / kCombineThreads), kCombineThreads, 0, s>>>((const __nv_bfloat16*)c3, slot_of, M, H, top_k, rsf,
                                                                 apply_rsf, (const __nv_bfloat16*)shared,
                                                                 (__nv_bfloat16*)out, sc);
   return cudaGetLastError();

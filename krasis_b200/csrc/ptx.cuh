@@ -55,6 +55,18 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
     }
   }
 }
+// The same with a pause of up to 2 * NS ns between tries, for warps that wait long and often: a poll costs about ten issue slots.
+template <int NS>
+__device__ __forceinline__ void mbar_wait_paused(uint64_t* bar, uint32_t parity) {
+  if (mbar_try_wait(bar, parity)) return;
+  for (uint32_t spins = 0; !mbar_try_wait(bar, parity);) {
+    __nanosleep(NS);
+    if ((++spins & 0xFFFu) == 0) {
+      mbar_wait(bar, parity);                       // after 4096 pauses the bounded wait above takes over
+      return;
+    }
+  }
+}
 
 // ------------------------------------------------------------------ proxies / fences
 // generic-proxy smem writes (st.shared, cp.async) -> visible to the async proxy (tcgen05.mma, TMA)

@@ -5,7 +5,7 @@
 // from cuBLAS sgemm only in summation order / rounding of partial sums — the same class of difference as
 // between any two fp32 GEMMs (see oracle/router.py).  Id parity is asserted by tests away from near-ties.
 //
-// One CTA per (128-token tile, 256-expert column block): UMMA M = 128, N <= 256.  With E = 512 that is 2 x 64 = 128 CTAs at 8192
+// One CTA per (128-token tile, 256-expert column block; 64 for few tokens, see the launcher): UMMA M = 128, N <= 256.  With E = 512 that is 2 x 64 = 128 CTAs at 8192
 // tokens (one CTA per token tile and all 512 columns left 84 of the 148 SMs idle and ran at 0.27 of the tensor peak).  Both operands
 // arrive by 2-D TMA with 128 B swizzle, 64-wide K blocks, 4-stage ring; one warp produces, one elected lane issues tcgen05.mma (SS),
 // four warps drain TMEM and write fp32 logits rows (64 B contiguous per thread per tcgen05.ld).
@@ -18,18 +18,23 @@
 namespace kb2 {
 
 constexpr int kRThreads = 256;
-constexpr int kRStages = 4;
 constexpr int kRATile = 128 * kBlockK * 2;        // 16 KB
-constexpr int kRBMax = 256 * kBlockK * 2;         // 32 KB
-constexpr int kRStage = kRATile + kRBMax;         // 48 KB
-constexpr int kROffBar = kRStages * kRStage;
-constexpr int kRSmem = kROffBar + 64;
+// NB = expert columns per CTA
+template <int NB> struct RouterTile {
+  static constexpr int kStage = kRATile + NB * kBlockK * 2;
+  static constexpr int kStages = NB == 256 ? 4 : 9;
+  static constexpr int kOffBar = kStages * kStage;
+  static constexpr int kSmem = kOffBar + (2 * kStages + 1) * 8 + 8;
+};
 
+template <int NB>
 __global__ void __launch_bounds__(kRThreads, 1)
     router_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_g,
                        const float* __restrict__ gate_bias, float* __restrict__ logits, int M, int E, int H) {
+  using R = RouterTile<NB>;
+  constexpr int kRStages = R::kStages, kRStage = R::kStage;
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kROffBar);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + R::kOffBar);
   uint64_t* empty = full + kRStages;
   uint64_t* done = empty + kRStages;
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(done + 1);
@@ -37,8 +42,8 @@ __global__ void __launch_bounds__(kRThreads, 1)
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * 128;
   const int nkb = H / kBlockK;
-  const int col0 = blockIdx.y * 256;         // first expert column of this CTA
-  const int n0 = E - col0 > 256 ? 256 : E - col0;
+  const int col0 = blockIdx.y * NB;         // first expert column of this CTA
+  const int n0 = E - col0 > NB ? NB : E - col0;
 
   if (threadIdx.x == 32) {
     if (smem_u32(smem) & 1023u) __trap();
@@ -49,7 +54,7 @@ __global__ void __launch_bounds__(kRThreads, 1)
     mbar_init(done, 1);
     fence_mbar_init();
   }
-  if (warp == 0) tmem_alloc(tmem_ptr_smem, 256);
+  if (warp == 0) tmem_alloc(tmem_ptr_smem, NB);
   if (threadIdx.x == 64) {
     prefetch_tmap(&tmap_x);
     prefetch_tmap(&tmap_g);
@@ -131,12 +136,24 @@ __global__ void __launch_bounds__(kRThreads, 1)
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem_base, 256);
+  if (warp == 0) tmem_dealloc(tmem_base, NB);
 }
 
 cudaError_t make_tmap_bf16_rows(void* out_tmap, const void* base, long long rows, long long cols, int box_rows);
 
 bool router_gemm_supported(int E, int H) { return E >= 16 && E <= 512 && E % 64 == 0 && H % kBlockK == 0; }
+
+template <int NB>
+static cudaError_t launch_router_tile(const CUtensorMap& tx, const CUtensorMap& tg, const float* bias, float* logits, int M, int E, int H, cudaStream_t s) {
+  static PerDeviceOnce once;
+  if (const int dev = once.pending(); dev >= 0) {
+    cudaError_t e = cudaFuncSetAttribute(router_gemm_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, RouterTile<NB>::kSmem);
+    if (e != cudaSuccess) return e;
+    once.mark(dev);
+  }
+  router_gemm_kernel<NB><<<dim3((M + 127) / 128, (E + NB - 1) / NB), kRThreads, RouterTile<NB>::kSmem, s>>>(tx, tg, bias, logits, M, E, H);
+  return cudaGetLastError();
+}
 
 // tmap_g: tensor map over gate [E][H] with box rows 64 (built once per layer); x: [M][H] bf16
 cudaError_t launch_router_gemm(const void* x, const void* tmap_g, const float* bias, float* logits, int M, int E,
@@ -145,15 +162,11 @@ cudaError_t launch_router_gemm(const void* x, const void* tmap_g, const float* b
   alignas(64) CUtensorMap tx;
   cudaError_t e = make_tmap_bf16_rows(&tx, x, M, H, 128);
   if (e != cudaSuccess) return e;
-  static PerDeviceOnce once;
-  if (const int dev = once.pending(); dev >= 0) {
-    e = cudaFuncSetAttribute(router_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRSmem);
-    if (e != cudaSuccess) return e;
-    once.mark(dev);
-  }
-  router_gemm_kernel<<<dim3((M + 127) / 128, (E + 255) / 256), kRThreads, kRSmem, s>>>(tx, *reinterpret_cast<const CUtensorMap*>(tmap_g), bias,
-                                                               logits, M, E, H);
-  return cudaGetLastError();
+  const CUtensorMap& tg = *reinterpret_cast<const CUtensorMap*>(tmap_g);
+  // Few tokens: the K loop waits for its tiles, so more and narrower CTAs with nine stages in flight (3 x 256 experts 12.4 -> 7.4 us, 389 x 64 11.8 -> 8.9), as long as one wave of
+  // them holds the problem: past that the token tile is read E / 64 times where wide CTAs read it E / 256 times.
+  if ((long long)((M + 127) / 128) * ((E + 63) / 64) <= 148) return launch_router_tile<64>(tx, tg, bias, logits, M, E, H, s);
+  return launch_router_tile<256>(tx, tg, bias, logits, M, E, H, s);
 }
 
 }  // namespace kb2
