@@ -42,6 +42,7 @@ cudaError_t launch_add_bf16(const void* a, const void* b, void* out, long long n
 struct GqaDims {
   int H, nh, nkv, d, rotary_dim, gated;
   float theta, eps;
+  long long q_ld = 0, kv_ld = 0;
 };
 cudaError_t launch_gqa_core(const GqaDims& g, const void* q_raw, const void* k_raw, const void* v_raw, const float* q_norm,
                             const float* k_norm, const int* positions, const int* kv_indices, void* q_rot, void* k_cache,
@@ -55,6 +56,7 @@ cudaError_t launch_fmha_maps(const void* q, const void* k, const void* v, float*
 struct MlaDims {
   int H, nh, nope, rope, dv, lora;
   float eps;
+  long long q_ld = 0, kva_ld = 0;
 };
 cudaError_t launch_mla_core(const MlaDims& m, void* q_full, const void* kv_a, const float* kv_norm_w, const float* inv_freq,
                             const void* w_kv, const int* positions, const int* kv_indices, void* ckv_cache, void* kpe_cache,
@@ -475,7 +477,7 @@ KB2_API int kb2_gdn_forward(kb2_gdn* h, int layer, const void* hidden_dev, void*
 
 // ------------------------------------------------------------------------------------------------ GQA
 struct GqaLayer {
-  void *wq = nullptr, *wk = nullptr, *wv = nullptr, *wo = nullptr;
+  void *wqkv = nullptr, *wo = nullptr;       // [q_proj ; k_proj ; v_proj] as one projection
   float *q_norm = nullptr, *k_norm = nullptr;
   bool loaded = false;
 };
@@ -483,7 +485,7 @@ struct kb2_gqa {
   kb2_gqa_config cfg{};
   GqaDims g{};
   std::vector<GqaLayer> layers;
-  void *q_raw = nullptr, *k_raw = nullptr, *v_raw = nullptr, *q_rot = nullptr, *attn = nullptr;
+  void *qkv_raw = nullptr, *q_rot = nullptr, *attn = nullptr;
   void *k_bf = nullptr, *v_bf = nullptr;     // dense BF16 upcast of the sequence's FP8 pages, [kv_cap][nkv*d] each
   long long kv_cap = 0;
   CombineScatter out_scatter{};
@@ -505,11 +507,10 @@ KB2_API int kb2_gqa_create(const kb2_gqa_config* c, kb2_gqa** out) {
   kb2_gqa* h = new kb2_gqa();
   h->cfg = *c;
   h->g = GqaDims{c->hidden_size, c->num_heads, c->num_kv_heads, c->head_dim, c->rotary_dim, c->gated ? 1 : 0, c->rope_theta, c->rms_norm_eps};
+  h->g.q_ld = h->g.kv_ld = ((long long)c->num_heads * (c->gated ? 2 : 1) + 2 * c->num_kv_heads) * c->head_dim;
   h->layers.resize(c->num_layers);
   const size_t M = c->max_tokens, qd = (size_t)c->num_heads * c->head_dim, kvd = (size_t)c->num_kv_heads * c->head_dim;
-  CUDA_TRY(cudaMalloc(&h->q_raw, M * qd * (c->gated ? 2 : 1) * 2));
-  CUDA_TRY(cudaMalloc(&h->k_raw, M * kvd * 2));
-  CUDA_TRY(cudaMalloc(&h->v_raw, M * kvd * 2));
+  CUDA_TRY(cudaMalloc(&h->qkv_raw, M * (qd * (c->gated ? 2 : 1) + 2 * kvd) * 2));
   CUDA_TRY(cudaMalloc(&h->q_rot, M * qd * 2));
   CUDA_TRY(cudaMalloc(&h->attn, M * qd * 2));
   *out = h;
@@ -524,8 +525,8 @@ KB2_API int kb2_gqa_set_output_scatter(kb2_gqa* h, void* const* peer_recv_host, 
 KB2_API void kb2_gqa_destroy(kb2_gqa* h) {
   if (!h) return;
   cudaSetDevice(h->cfg.device);
-  for (auto& L : h->layers) { cudaFree(L.wq); cudaFree(L.wk); cudaFree(L.wv); cudaFree(L.wo); cudaFree(L.q_norm); cudaFree(L.k_norm); }
-  cudaFree(h->q_raw); cudaFree(h->k_raw); cudaFree(h->v_raw); cudaFree(h->q_rot); cudaFree(h->attn);
+  for (auto& L : h->layers) { cudaFree(L.wqkv); cudaFree(L.wo); cudaFree(L.q_norm); cudaFree(L.k_norm); }
+  cudaFree(h->qkv_raw); cudaFree(h->q_rot); cudaFree(h->attn);
   cudaFree(h->k_bf); cudaFree(h->v_bf);
   delete h;
 }
@@ -543,9 +544,11 @@ KB2_API int kb2_gqa_set_weights_host(kb2_gqa* h, int layer, const void* q_proj, 
     if (!*dst) { cudaError_t e = cudaMalloc(dst, bytes); if (e != cudaSuccess) return e; }
     return cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
   };
-  CUDA_TRY(up(&L.wq, q_proj, qd * (c.gated ? 2 : 1) * H * 2));
-  CUDA_TRY(up(&L.wk, k_proj, kvd * H * 2));
-  CUDA_TRY(up(&L.wv, v_proj, kvd * H * 2));
+  const size_t qw = qd * (c.gated ? 2 : 1);
+  if (!L.wqkv) CUDA_TRY(cudaMalloc(&L.wqkv, (qw + 2 * kvd) * H * 2));
+  CUDA_TRY(cudaMemcpy(L.wqkv, q_proj, qw * H * 2, cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaMemcpy((char*)L.wqkv + qw * H * 2, k_proj, kvd * H * 2, cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaMemcpy((char*)L.wqkv + (qw + kvd) * H * 2, v_proj, kvd * H * 2, cudaMemcpyHostToDevice));
   CUDA_TRY(up(&L.wo, o_proj, H * qd * 2));
   if (q_norm) { auto v = bf16_to_f32_host(q_norm, c.head_dim); CUDA_TRY(up((void**)&L.q_norm, v.data(), v.size() * 4)); }
   if (k_norm) { auto v = bf16_to_f32_host(k_norm, c.head_dim); CUDA_TRY(up((void**)&L.k_norm, v.data(), v.size() * 4)); }
@@ -569,9 +572,9 @@ KB2_API int kb2_gqa_forward(kb2_gqa* h, int layer, const void* hidden_dev, const
   const auto& c = h->cfg;
   const int qd = c.num_heads * c.head_dim, kvd = c.num_kv_heads * c.head_dim, H = c.hidden_size, sms = device_sms(c.device);
   const int qw = qd * (c.gated ? 2 : 1);
-  CUDA_TRY(launch_dense_gemm(hidden_dev, L.wq, h->q_raw, nullptr, M, qw, H, qw, false, sms, s));
-  CUDA_TRY(launch_dense_gemm(hidden_dev, L.wk, h->k_raw, nullptr, M, kvd, H, kvd, false, sms, s));
-  CUDA_TRY(launch_dense_gemm(hidden_dev, L.wv, h->v_raw, nullptr, M, kvd, H, kvd, false, sms, s));
+  // one GEMM: the k and v projections alone, 13 us each at 2048 x 512 x 2048, leave most SMs waiting for a short K loop
+  CUDA_TRY(launch_dense_gemm(hidden_dev, L.wqkv, h->qkv_raw, nullptr, M, qw + 2 * kvd, H, qw + 2 * kvd, false, sms, s));
+  const char* raw = (const char*)h->qkv_raw;
   if (kv_len_after > h->kv_cap) {              // grow the upcast scratch (cudaFree synchronises: no kernel still reads it)
     const long long cap = kv_len_after > 2 * h->kv_cap ? kv_len_after : 2 * h->kv_cap;
     cudaFree(h->k_bf); cudaFree(h->v_bf);
@@ -581,7 +584,7 @@ KB2_API int kb2_gqa_forward(kb2_gqa* h, int layer, const void* hidden_dev, const
     CUDA_TRY(cudaMalloc(&h->v_bf, (size_t)cap * kvd * 2));
     h->kv_cap = cap;
   }
-  CUDA_TRY(launch_gqa_core(h->g, h->q_raw, h->k_raw, h->v_raw, L.q_norm, L.k_norm, positions_dev, kv_indices_dev, h->q_rot,
+  CUDA_TRY(launch_gqa_core(h->g, raw, raw + (size_t)qw * 2, raw + (size_t)(qw + kvd) * 2, L.q_norm, L.k_norm, positions_dev, kv_indices_dev, h->q_rot,
                            k_cache_layer_dev, v_cache_layer_dev, h->k_bf, h->v_bf, h->attn, M, first_position, kv_len_after, s));
   CUDA_TRY(launch_dense_gemm_scatter(h->attn, L.wo, out_dev, nullptr, M, H, qd, H, false, sms, s, scatter_for(h->out_scatter, M)));
   return KB2_OK;
@@ -590,7 +593,8 @@ KB2_API int kb2_gqa_forward(kb2_gqa* h, int layer, const void* hidden_dev, const
 
 // ---------------------------------------------------------------------------------------------- MLA
 struct MlaLayer {
-  void *wq = nullptr, *wqa = nullptr, *wkva = nullptr, *wkv = nullptr, *wo = nullptr;
+  void *wq = nullptr, *wqa = nullptr, *wkva = nullptr;   // without q_lora_rank wq is [q_proj ; kv_a_proj_with_mqa] and wkva stays null
+  void *wkv = nullptr, *wo = nullptr;
   float *qa_norm = nullptr, *kv_norm = nullptr, *inv_freq = nullptr;
   bool loaded = false;
 };
@@ -622,9 +626,12 @@ KB2_API int kb2_mla_create(const kb2_mla_config* c, kb2_mla** out) {
   h->m = MlaDims{c->hidden_size, c->num_heads, c->qk_nope_head_dim, c->qk_rope_head_dim, c->v_head_dim, c->kv_lora_rank, c->rms_norm_eps};
   h->layers.resize(c->num_layers);
   const size_t M = c->max_tokens, T = c->max_kv_len, nh = c->num_heads;
-  CUDA_TRY(cudaMalloc(&h->q_full, M * nh * 192 * 2));
+  const bool stacked = c->q_lora_rank == 0;
+  h->m.q_ld = nh * 192 + (stacked ? c->kv_lora_rank + 64 : 0);
+  h->m.kva_ld = stacked ? h->m.q_ld : c->kv_lora_rank + 64;
+  CUDA_TRY(cudaMalloc(&h->q_full, M * h->m.q_ld * 2));
   if (c->q_lora_rank) CUDA_TRY(cudaMalloc(&h->q_a, M * c->q_lora_rank * 2 * 2));     // raw + normed
-  CUDA_TRY(cudaMalloc(&h->kv_a, M * (c->kv_lora_rank + 64) * 2));
+  if (!stacked) CUDA_TRY(cudaMalloc(&h->kv_a, M * (c->kv_lora_rank + 64) * 2));
   CUDA_TRY(cudaMalloc(&h->ckv_bf16, T * c->kv_lora_rank * 2));
   CUDA_TRY(cudaMalloc(&h->kpe_bf16, T * 64 * 2));
   CUDA_TRY(cudaMalloc(&h->kv_up, T * nh * 256 * 2));
@@ -666,13 +673,16 @@ KB2_API int kb2_mla_set_weights_host(kb2_mla* h, int layer, const void* q_proj_o
     return cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
   };
   const size_t H = c.hidden_size, nh = c.num_heads, lora = c.kv_lora_rank, qin = c.q_lora_rank ? c.q_lora_rank : H;
-  CUDA_TRY(up(&L.wq, q_proj_or_q_b_proj, nh * 192 * qin * 2));
+  const size_t q_bytes = nh * 192 * qin * 2, kva_bytes = (lora + 64) * H * 2;
+  if (!L.wq) CUDA_TRY(cudaMalloc(&L.wq, q_bytes + (c.q_lora_rank ? 0 : kva_bytes)));
+  CUDA_TRY(cudaMemcpy(L.wq, q_proj_or_q_b_proj, q_bytes, cudaMemcpyHostToDevice));
   if (c.q_lora_rank) {
     CUDA_TRY(up(&L.wqa, q_a_proj, (size_t)c.q_lora_rank * H * 2));
     auto v = bf16_to_f32_host(q_a_layernorm, c.q_lora_rank);
     CUDA_TRY(up((void**)&L.qa_norm, v.data(), v.size() * 4));
   }
-  CUDA_TRY(up(&L.wkva, kv_a_proj_with_mqa, (lora + 64) * H * 2));
+  if (c.q_lora_rank) CUDA_TRY(up(&L.wkva, kv_a_proj_with_mqa, kva_bytes));
+  else CUDA_TRY(cudaMemcpy((char*)L.wq + q_bytes, kv_a_proj_with_mqa, kva_bytes, cudaMemcpyHostToDevice));
   {
     auto v = bf16_to_f32_host(kv_a_layernorm, (int)lora);
     CUDA_TRY(up((void**)&L.kv_norm, v.data(), v.size() * 4));
@@ -703,16 +713,19 @@ KB2_API int kb2_mla_forward(kb2_mla* h, int layer, const void* hidden_dev, const
   CUDA_TRY(cudaSetDevice(c.device));
   cudaStream_t s = (cudaStream_t)stream;
   const int H = c.hidden_size, nh = c.num_heads, lora = c.kv_lora_rank, sms = device_sms(c.device);
-  CUDA_TRY(launch_dense_gemm(hidden_dev, L.wkva, h->kv_a, nullptr, M, lora + 64, H, lora + 64, false, sms, s));
+  const void* kv_a = h->kv_a;
   if (c.q_lora_rank) {
+    CUDA_TRY(launch_dense_gemm(hidden_dev, L.wkva, h->kv_a, nullptr, M, lora + 64, H, lora + 64, false, sms, s));
     void* q_a_normed = (char*)h->q_a + (size_t)c.max_tokens * c.q_lora_rank * 2;
     CUDA_TRY(launch_dense_gemm(hidden_dev, L.wqa, h->q_a, nullptr, M, c.q_lora_rank, H, c.q_lora_rank, false, sms, s));
     CUDA_TRY(launch_rmsnorm(h->q_a, nullptr, L.qa_norm, q_a_normed, M, c.q_lora_rank, c.rms_norm_eps, s));
     CUDA_TRY(launch_dense_gemm(q_a_normed, L.wq, h->q_full, nullptr, M, nh * 192, c.q_lora_rank, nh * 192, false, sms, s));
   } else {
-    CUDA_TRY(launch_dense_gemm(hidden_dev, L.wq, h->q_full, nullptr, M, nh * 192, H, nh * 192, false, sms, s));
+    // one GEMM: kv_a alone has 5 column tiles of 128 (1000 x 576 x 2048: 11 us of its own)
+    CUDA_TRY(launch_dense_gemm(hidden_dev, L.wq, h->q_full, nullptr, M, (int)h->m.q_ld, H, h->m.q_ld, false, sms, s));
+    kv_a = (const char*)h->q_full + (size_t)nh * 192 * 2;
   }
-  CUDA_TRY(launch_mla_core(h->m, h->q_full, h->kv_a, L.kv_norm, L.inv_freq, L.wkv, positions_dev, kv_indices_dev,
+  CUDA_TRY(launch_mla_core(h->m, h->q_full, kv_a, L.kv_norm, L.inv_freq, L.wkv, positions_dev, kv_indices_dev,
                            ckv_cache_layer_dev, kpe_cache_layer_dev, h->ckv_bf16, h->kpe_bf16, h->kv_up, h->attn, M,
                            first_position, kv_len_after, c.sm_scale, sms, s));
   CUDA_TRY(launch_dense_gemm_scatter(h->attn, L.wo, out_dev, nullptr, M, H, nh * 128, H, false, sms, s, scatter_for(h->out_scatter, M)));

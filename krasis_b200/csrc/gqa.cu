@@ -27,6 +27,7 @@ namespace kb2 {
 struct GqaDims {
   int H, nh, nkv, d, rotary_dim, gated;
   float theta, eps;
+  long long q_ld = 0, kv_ld = 0;   // row strides of q_raw and of k_raw / v_raw (elements)
 };
 
 __device__ __forceinline__ float bf16r_(float x) { return bf16_round_rn(x); }
@@ -36,8 +37,8 @@ __device__ __forceinline__ float bf16r_(float x) { return bf16_round_rn(x); }
 // computed once per CTA (powf + cosf + sinf per (head, pair) was most of this kernel: 20 heads recomputed the same 32 angles at QCN
 // geometry, 72 heads the same 64 at Qwen3-235B); rows move as BF16 pairs / FP8 pairs.
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) gqa_prep_kernel(GqaDims g, const __nv_bfloat16* __restrict__ q_raw,   // [M][nh*d*(1+gated)]
-                                                       const __nv_bfloat16* __restrict__ k_raw,             // [M][nkv*d]
+__global__ void __launch_bounds__(256) gqa_prep_kernel(GqaDims g, const __nv_bfloat16* __restrict__ q_raw,   // [M][q_ld], nh*d*(1+gated) of them used
+                                                       const __nv_bfloat16* __restrict__ k_raw,             // [M][kv_ld]
                                                        const __nv_bfloat16* __restrict__ v_raw,
                                                        const float* __restrict__ q_norm, const float* __restrict__ k_norm,
                                                        const int* __restrict__ positions, const int* __restrict__ kv_indices,
@@ -62,8 +63,8 @@ __global__ void __launch_bounds__(256) gqa_prep_kernel(GqaDims g, const __nv_bfl
   for (int hh = warp; hh < g.nh + 2 * g.nkv; hh += nw) {
     const bool is_q = hh < g.nh, is_k = !is_q && hh < g.nh + g.nkv;
     const int h = is_q ? hh : (is_k ? hh - g.nh : hh - g.nh - g.nkv);
-    const __nv_bfloat16* src = is_q ? q_raw + (long long)t * g.nh * d * (1 + g.gated) + (long long)h * d * (1 + g.gated)
-                                    : (is_k ? k_raw : v_raw) + (long long)t * g.nkv * d + (long long)h * d;
+    const __nv_bfloat16* src = is_q ? q_raw + t * g.q_ld + (long long)h * d * (1 + g.gated)
+                                    : (is_k ? k_raw : v_raw) + t * g.kv_ld + (long long)h * d;
     float ss = 0.f;
     for (int i = 2 * lane; i < d; i += 64) {                        // d is even, rows are 4-byte aligned (d % 8 == 0)
       const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(src + i));
@@ -210,8 +211,11 @@ __global__ void __launch_bounds__(kFThreads, 1)
   // shuffle-broadcast warp index: role branches provably warp-uniform -> TMA / tcgen05 operands stay in uniform registers (issued
   // from a divergent `lane == 0` branch each tcgen05.mma pays an ELECT + R2UR.BROADCAST loop of ~50 cycles, more than an N=64 MMA runs)
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int qt = gridDim.x - 1 - blockIdx.x;       // heavy (late) query tiles first
-  const int head = blockIdx.y, kvh = (head / maps) / ((g.nh / maps) / g.nkv), kkh = kvh * maps + head % maps;
+  // heavy (late) query tiles first, over all heads: with them first within each head only, the last head's heaviest tile began with the last
+  // wave (16 heads x 16 tiles of 128 queries after 2500 cached keys, one CTA per SM: 159 -> 142 us)
+  const int lin = blockIdx.y * gridDim.x + blockIdx.x;
+  const int qt = gridDim.x - 1 - lin / (int)gridDim.y;
+  const int head = lin % (int)gridDim.y, kvh = (head / maps) / ((g.nh / maps) / g.nkv), kkh = kvh * maps + head % maps;
   const int q0 = qt * kFQ;
   // keys visible to this tile: positions <= q_start + min(q0 + 127, M - 1)
   const int last_q = min(q0 + kFQ - 1, M - 1);
@@ -474,7 +478,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
       float inv_l = l_sum > 0.f ? 1.0f / l_sum : 0.f;
       if (head_gate != nullptr && live) inv_l *= 1.0f / (1.0f + expf(-head_gate[(long long)qi * ldg + head]));
       const long long obase = (long long)qi * g.nh * DV + (long long)head * DV;
-      const long long gbase = (long long)qi * g.nh * D * 2 + (long long)head * 2 * D + D;   // gate half of q_raw
+      const long long gbase = qi * g.q_ld + (long long)head * 2 * D + D;   // gate half of q_raw
       const bool gated = g.gated != 0;
 #pragma unroll 2
       for (int c0 = hf * OH; c0 < (hf + 1) * OH; c0 += 16) {
@@ -612,10 +616,11 @@ cudaError_t launch_gqa_core(const GqaDims& g, const void* q_raw, const void* k_r
 struct MlaDims {
   int H, nh, nope, rope, dv, lora;
   float eps;
+  long long q_ld = 0, kva_ld = 0;   // row strides of q_full and kv_a (elements)
 };
 
-__global__ void __launch_bounds__(256) mla_prep_kernel(MlaDims m, const __nv_bfloat16* __restrict__ kv_a,   // [M][lora+rope]
-                                                       __nv_bfloat16* __restrict__ q_full,                 // [M][nh*(nope+rope)]
+__global__ void __launch_bounds__(256) mla_prep_kernel(MlaDims m, const __nv_bfloat16* __restrict__ kv_a,   // [M][kva_ld], lora+rope used
+                                                       __nv_bfloat16* __restrict__ q_full,                 // [M][q_ld], nh*(nope+rope) used
                                                        const float* __restrict__ kv_norm_w,
                                                        const float* __restrict__ inv_freq,                 // [rope/2]
                                                        const int* __restrict__ positions,
@@ -626,7 +631,7 @@ __global__ void __launch_bounds__(256) mla_prep_kernel(MlaDims m, const __nv_bfl
   const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int pos = positions[t];
   const long long slot = (long long)kv_indices[pos >> 4] * 16 + (pos & 15);
-  const __nv_bfloat16* row = kv_a + (long long)t * (m.lora + m.rope);
+  const __nv_bfloat16* row = kv_a + t * m.kva_ld;
   // KV LayerNorm (flashinfer.norm.rmsnorm: fp32, output BF16) then the cache cast
   float ss = 0.f;
   for (int i = tid; i < m.lora; i += 256) {
@@ -648,7 +653,7 @@ __global__ void __launch_bounds__(256) mla_prep_kernel(MlaDims m, const __nv_bfl
   // RoPE: interleaved (re, im) pairs -> half-split, BF16 tables, every product / sum rounded to BF16 (:190-211)
   const int half = m.rope / 2, hd = m.nope + m.rope;
   for (int u = warp; u < m.nh + 1; u += 8) {         // unit nh = the shared key
-    __nv_bfloat16* src = u < m.nh ? q_full + (long long)t * m.nh * hd + (long long)u * hd + m.nope : nullptr;
+    __nv_bfloat16* src = u < m.nh ? q_full + t * m.q_ld + (long long)u * hd + m.nope : nullptr;
     for (int i0 = 0; i0 < half; i0 += 32) {
       const int i = i0 + lane;
       float x1 = 0.f, x2 = 0.f;
@@ -698,7 +703,7 @@ __global__ void __launch_bounds__(256) mla_gather_kernel(const uint8_t* __restri
 cudaError_t launch_dense_gemm(const void* x, const void* w, void* out, const float* bias, int M, int N, int K,
                               long long ldo, bool out_f32, int num_sms, cudaStream_t s);
 
-// q_full [M][nh*192] (q_proj output; rotated in place), kv_a [M][lora+rope]; w_kv [nh*(nope+dv)][lora] = [w_kc ; w_vc];
+// q_full [M][m.q_ld] (q_proj output, nh*192 columns; rotated in place), kv_a [M][m.kva_ld] (lora+rope columns); w_kv [nh*(nope+dv)][lora] = [w_kc ; w_vc];
 // scratch: ckv_bf16 [T][lora], kpe_bf16 [T][rope], kv_up [T][nh*(nope+dv)]; attn_out [M][nh*dv]
 cudaError_t launch_mla_core(const MlaDims& m, void* q_full, const void* kv_a, const float* kv_norm_w, const float* inv_freq,
                             const void* w_kv, const int* positions, const int* kv_indices, void* ckv_cache, void* kpe_cache,
@@ -721,7 +726,7 @@ cudaError_t launch_mla_core(const MlaDims& m, void* q_full, const void* kv_a, co
   cudaError_t e = launch_dense_gemm(ckv_bf16, w_kv, kv_up, nullptr, kv_len, up, m.lora, up, false, num_sms, s);
   if (e != cudaSuccess) return e;
   alignas(64) CUtensorMap tq, tk, tpe;
-  e = make_tmap_bf16_rows(&tq, q_full, M, (long long)m.nh * (m.nope + m.rope), kFQ);
+  e = make_tmap_bf16_rows(&tq, q_full, M, m.q_ld, kFQ);
   if (e != cudaSuccess) return e;
   e = make_tmap_bf16_rows(&tk, kv_up, kv_len, up, kFK);
   if (e != cudaSuccess) return e;
