@@ -513,6 +513,9 @@ KB2_API int kb2_gqa_create(const kb2_gqa_config* c, kb2_gqa** out) {
   CUDA_TRY(cudaMalloc(&h->qkv_raw, M * (qd * (c->gated ? 2 : 1) + 2 * kvd) * 2));
   CUDA_TRY(cudaMalloc(&h->q_rot, M * qd * 2));
   CUDA_TRY(cudaMalloc(&h->attn, M * qd * 2));
+  CUDA_TRY(cudaMalloc(&h->k_bf, M * kvd * 2));       // grown by the forward pass when a sequence gets longer than this
+  CUDA_TRY(cudaMalloc(&h->v_bf, M * kvd * 2));
+  h->kv_cap = (long long)M;
   *out = h;
   return KB2_OK;
 }

@@ -627,10 +627,15 @@ __global__ void __launch_bounds__(256) mla_prep_kernel(MlaDims m, const __nv_bfl
                                                        const int* __restrict__ kv_indices,
                                                        uint8_t* __restrict__ ckv_cache, uint8_t* __restrict__ kpe_cache,
                                                        int M) {
-  __shared__ float red[8];
+  __shared__ float red[8], s_cos[32], s_sin[32];      // the launcher requires rope == 64
   const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int pos = positions[t];
   const long long slot = (long long)kv_indices[pos >> 4] * 16 + (pos & 15);
+  if (tid >= 224 && lane < m.rope / 2) {              // once per token, not per head (16 heads, 1000 tokens: 9.4 -> 7.2 us)
+    const float ang = (float)pos * inv_freq[lane];
+    s_cos[lane] = bf16r_(cosf(ang));
+    s_sin[lane] = bf16r_(sinf(ang));
+  }
   const __nv_bfloat16* row = kv_a + t * m.kva_ld;
   // KV LayerNorm (flashinfer.norm.rmsnorm: fp32, output BF16) then the cache cast
   float ss = 0.f;
@@ -663,8 +668,7 @@ __global__ void __launch_bounds__(256) mla_prep_kernel(MlaDims m, const __nv_bfl
       }
       __syncwarp();                                  // all lanes have read before anyone overwrites (in place for q)
       if (i < half) {
-        const float ang = (float)pos * inv_freq[i];
-        const float c = bf16r_(cosf(ang)), sn = bf16r_(sinf(ang));
+        const float c = s_cos[i], sn = s_sin[i];
         const float r1 = bf16r_(bf16r_(x1 * c) - bf16r_(x2 * sn));
         const float r2 = bf16r_(bf16r_(x2 * c) + bf16r_(x1 * sn));
         if (u < m.nh) {
