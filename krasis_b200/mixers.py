@@ -133,9 +133,17 @@ def layer_runs(n: int, start: int = 0, stop: int = 0, times: int = 1):
             + [(i, False) for i in range(stop, n)])
 
 
+def _row(t, r: int):
+    """Address of row r (a slice of the tensor made for its address alone costs a microsecond); None for no tensor."""
+    return t.data_ptr() + r * t.stride(0) * t.element_size() if t is not None else None
+
+
 def portion_runs(tb, min_long):
     """The step's rows as runs of neighbouring sequences of one kind: [(long, sequences, first row, rows)], long where every portion of the
     run has at least min_long tokens (None: no portion counts as long)."""
+    if tb.S == 1:
+        n = tb.layout[0][1]
+        return [(min_long is not None and n >= min_long, range(1), 0, n)] if n else []
     runs, i = [], 0
     kind = [min_long is not None and n >= min_long for _, n, _, _ in tb.layout]
     while i < tb.S:
@@ -242,7 +250,6 @@ class WindowLatentAttention:
         o = torch.empty((T, H, self.dv), dtype=torch.float32 if gated else self.dtype, device=h.device)
         core = _core_lib() if self.tc_shape else False
         for fast, seqs, r0, n in portion_runs(tb, self.tc_min_portion if core else None):
-            hgr = hg[r0:] if hg is not None else None
             if not fast:
                 q_abs = torch.empty((n, H, self.r), dtype=torch.float32, device=h.device)
                 lin_heads(q[r0:r0 + n, :, :self.dn], self.uk_t, q_abs)
@@ -253,11 +260,11 @@ class WindowLatentAttention:
                 nsplit = max(1, min(296 // max(blocks, 1), (max_keys + 31) // 32, 64))
                 part_acc = torch.empty((n, nsplit, H, self.r), dtype=torch.float32, device=h.device) if nsplit > 1 else None
                 part_ml = torch.empty((n, nsplit, H, 2), dtype=torch.float32, device=h.device) if nsplit > 1 else None
-                ops.check(lib.kb2_seq_latent_window_attn(q_abs.data_ptr(), proj[r0:].data_ptr(), ldp, n, H, self.dn, self.dr, self.r,
-                                                         ckv.data_ptr(), kr.data_ptr(), dtc, tb.positions[r0:].data_ptr(),
-                                                         tb.seq_of[r0:].data_ptr(), tb.pages.data_ptr(), tb.max_pages, page_size,
+                ops.check(lib.kb2_seq_latent_window_attn(q_abs.data_ptr(), _row(proj, r0), ldp, n, H, self.dn, self.dr, self.r,
+                                                         ckv.data_ptr(), kr.data_ptr(), dtc, _row(tb.positions, r0),
+                                                         _row(tb.seq_of, r0), tb.pages.data_ptr(), tb.max_pages, page_size,
                                                          ops._ptr(self.sink), self.scale, self.window, o_lat.data_ptr(), None,
-                                                         self.tc_min_portion, nsplit, ops._ptr(part_acc), ops._ptr(part_ml), ops._ptr(hgr), ldg, s))
+                                                         self.tc_min_portion, nsplit, ops._ptr(part_acc), ops._ptr(part_ml), _row(hg, r0), ldg, s))
                 lin_heads(o_lat, self.uv, o[r0:r0 + n])
                 continue
             from . import capi
@@ -872,13 +879,13 @@ class MultiMapAttention:
         """Rows r0 .. r0 + T - 1 of the step (the sequences `seqs`): attention into a, the finished heads into o.  core: the library whose
         tensor-core attention runs these portions, None for the plain kernel."""
         lib, H, G, M, dtc, dev = ops.load(), self.H, self.G, self.M, ops.dt_code(kc.dtype), proj.device
-        positions, seq_of, window = tb.positions[r0:], tb.seq_of[r0:], min(self.window, 1 << 30)
+        positions, seq_of, window = _row(tb.positions, r0), _row(tb.seq_of, r0), min(self.window, 1 << 30)
         nsplit, part_acc, part_ml = 1, None, None
 
         def plain(out, acc, ml, pool_only):
-            ops.check(lib.kb2_seq_paged_attn(proj[r0:].data_ptr(), proj.stride(0), T, H, G, M, self.d, self.dv, kc.data_ptr(), vc.data_ptr(), dtc,
-                                             positions.data_ptr(), seq_of.data_ptr(), tb.pages.data_ptr(), tb.max_pages, page_size, self.scale,
-                                             0 if pool_only else self.chunk, window, out.data_ptr(), nsplit, ops._ptr(acc), ops._ptr(ml),
+            ops.check(lib.kb2_seq_paged_attn(_row(proj, r0), proj.stride(0), T, H, G, M, self.d, self.dv, kc.data_ptr(), vc.data_ptr(), dtc,
+                                             positions, seq_of, tb.pages.data_ptr(), tb.max_pages, page_size, self.scale,
+                                             0 if pool_only else self.chunk, window, out, nsplit, ops._ptr(acc), ops._ptr(ml),
                                              tb.cu.data_ptr() if pool_only else None,
                                              self.tc_min_portion, self.softcap, None if pool_only else ops._ptr(self.sink), self.pool, ops._ptr(kp),
                                              ops._ptr(vp), int(pool_only), None if pool_only else ops._ptr(self.slopes), s))
@@ -891,7 +898,7 @@ class MultiMapAttention:
             if nsplit > 1:
                 part_acc = torch.empty((T * H * M, nsplit, self.dv), dtype=torch.float32, device=dev)
                 part_ml = torch.empty((T * H * M, nsplit, 2), dtype=torch.float32, device=dev)
-            plain(a[r0:], part_acc, part_ml, False)
+            plain(_row(a, r0), part_acc, part_ml, False)
         else:
             lse = torch.empty((proj.shape[0], H), dtype=torch.float32, device=dev) if self.pool else None
             for q in seqs:
@@ -899,13 +906,13 @@ class MultiMapAttention:
             if self.pool:                            # the pooled blocks of the long portions: a second pass, joined by the log-sum-exps
                 p_acc = torch.empty((T * H, self.dv), dtype=torch.float32, device=dev)
                 p_ml = torch.empty((T * H, 2), dtype=torch.float32, device=dev)
-                plain(a[r0:], p_acc, p_ml, True)
-                ops.check(lib.kb2_seq_pool_merge(a[r0:].data_ptr(), lse[r0:].data_ptr(), p_acc.data_ptr(), p_ml.data_ptr(), T, H, self.dv,
-                                                 seq_of.data_ptr(), tb.cu.data_ptr(), self.tc_min_portion, s))
-        ops.check(lib.kb2_seq_attn_finish(a[r0:].data_ptr(), ops._ptr(part_acc), ops._ptr(part_ml), nsplit, T, H, M, self.dv, ops._ptr(self.map_coef),
-                                          int(self.unit_norm), self.eps, self.post_scale, ops._ptr(gate[r0:] if gate is not None else None),
-                                          gate.stride(0) if gate is not None else proj.stride(0), o[r0:].data_ptr(), ops.dt_code(self.dtype), None,
-                                          None, 0, int(self.gate_wide), positions.data_ptr(), ops._ptr(self.vfreq), int(self.rot_half), s))
+                plain(_row(a, r0), p_acc, p_ml, True)
+                ops.check(lib.kb2_seq_pool_merge(_row(a, r0), _row(lse, r0), p_acc.data_ptr(), p_ml.data_ptr(), T, H, self.dv,
+                                                 seq_of, tb.cu.data_ptr(), self.tc_min_portion, s))
+        ops.check(lib.kb2_seq_attn_finish(_row(a, r0), ops._ptr(part_acc), ops._ptr(part_ml), nsplit, T, H, M, self.dv, ops._ptr(self.map_coef),
+                                          int(self.unit_norm), self.eps, self.post_scale, _row(gate, r0),
+                                          gate.stride(0) if gate is not None else proj.stride(0), _row(o, r0), ops.dt_code(self.dtype), None,
+                                          None, 0, int(self.gate_wide), positions, ops._ptr(self.vfreq), int(self.rot_half), s))
 
 
 class RoutedExperts:
