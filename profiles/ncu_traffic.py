@@ -10,8 +10,8 @@ import os
 import sys
 
 CLASSES = [("dense_gemm_kernel<0", "dense_gemm<bf16>"), ("dense_gemm_kernel<1", "dense_gemm<bf16>"), ("dense_gemm_kernel<2", "dense_gemm<int8>"),
-           ("grouped_gemm_kernel<0, 1>", "grouped_gemm<gate_up+silu_mul>"), ("grouped_gemm_kernel<0, 0>", "grouped_gemm<down>"),
-           ("grouped_gemm_kernel<1, 1>", "grouped_gemm<gate_up+silu_mul>"), ("grouped_gemm_kernel<1, 0>", "grouped_gemm<down>"),
+           ("grouped_gemm_kernel<0, 1", "grouped_gemm<gate_up+silu_mul>"), ("grouped_gemm_kernel<0, 0", "grouped_gemm<down>"),
+           ("grouped_gemm_kernel<1, 1", "grouped_gemm<gate_up+silu_mul>"), ("grouped_gemm_kernel<1, 0", "grouped_gemm<down>"),
            ("gdn_scan_tc", "gdn_chunk_scan"), ("gdn_chunk_scan", "gdn_chunk_scan"), ("gdn_prepare_tc", "gdn_chunk_prepare"),
            ("gdn_chunk_prepare", "gdn_chunk_prepare"), ("gqa_fmha_kernel", "fmha"), ("combine_kernel", "combine"), ("gdn_prep_vec", "gdn_prep(conv+l2norm+gates)")]
 
