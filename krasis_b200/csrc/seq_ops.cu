@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(KS > 8 ? 512 : 256) gemv_mma_kernel(const bf16
 #pragma unroll
       for (int i = 0; i < 4; ++i) {                // compensated: what the addition rounds off goes into the next one
         const float add = d[i] - lost[i], t = sum[i] + add;
-        lost[i] = (t - sum[i]) - add;
+        lost[i] = isfinite(t) ? (t - sum[i]) - add : 0.f;      // an infinity stays one: inf - inf must not reach the next addition
         sum[i] = t;
       }
     }

@@ -27,6 +27,35 @@ def test_gemv(N, K, H, M, dtype):
         assert ((one[0].double() - want[0]).abs() <= room[0]).all()
 
 
+# at the first number, within and at the end of a piece, in the middle and in the last one; K past one piece of every cut
+@pytest.mark.parametrize("M", [1, 4, 8])
+@pytest.mark.parametrize("N,K", [(512, 2048), (70000, 264), (64, 16392)])
+def test_gemv_keeps_infinities(N, K, M):
+    """An infinite or overflowing sum is what plain fp32 sums give, infinity and not NaN; the other outputs are as without it."""
+    g = torch.Generator(device="cuda").manual_seed(N)
+    inf, nan = float("inf"), float("nan")
+    a = (torch.randn(M, K, device="cuda", generator=g).abs() + 0.1).bfloat16()          # one sign: no infinities that cancel
+    w0 = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    want0 = ops.gemm(a, w0)
+    at = sorted({0, 31, 127, 128, K // 2, K - 1})
+    for i, values in enumerate([[inf], [-inf], [nan], [inf, -inf], [3e38, 3e38], [-3e38, -3e38]]):
+        w = w0.clone()
+        rows = torch.arange(len(at), device="cuda") * 9 + i                              # a weight row per place
+        for r, k in zip(rows.tolist(), at):
+            for j, v in enumerate(values):
+                w[r, (k + 200 * j) % K] = v
+        big = a.clone()
+        if abs(values[0]) < inf:
+            big[:] = 1.0                                                                 # two terms of 3e38 overflow
+        want = (big.double() @ w[rows].double().T).float()                               # beyond fp32: infinite
+        got = ops.gemm(big, w)
+        torch.testing.assert_close(got[:, rows], want, rtol=0, atol=0, equal_nan=True)
+        if abs(values[0]) == inf:
+            keep = torch.ones(N, dtype=torch.bool, device="cuda")
+            keep[rows] = False
+            assert torch.equal(got[:, keep], want0[:, keep])
+
+
 @pytest.mark.parametrize("W", [1, 6, 512, 1024, 1028, 2048, 2052, 4096, 4100, 8192, 8196])
 @pytest.mark.parametrize("mode", ["layer", "rms", "plain", "none"])
 @pytest.mark.parametrize("x0", [False, True])
