@@ -1780,7 +1780,8 @@ __global__ void __launch_bounds__(64 * NI + 32, 1) delta_tile_kernel(const bf16*
       float a[kDT], o = ss[kDTG + t] * r;
       eight(kDTQK + t * kDT, a);
 #pragma unroll
-      for (int j = 0; j < kDT; ++j) o = fmaf(a[j], u[j], o);
+      for (int j = 0; j < kDT; ++j)
+        if (j <= t) o = fmaf(a[j], u[j], o);           // not by the zeros of later tokens: theirs may be infinite
       if (i * kDT + t < n) o_out[((t0 + (long long)i * kDT + t) * H + h) * dv + j0 + cg * 16 + col] = o;
     }
     __syncwarp();

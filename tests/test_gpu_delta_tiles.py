@@ -73,6 +73,49 @@ def test_tiles_against_exact_and_token_form(H, Hk, dk, dv, lens, decay):
     assert err["tiles"][0] <= 1.5 * err["tokens"][0] + 2e-7 and err["tiles"][1] <= 1.5 * err["tokens"][1] + 2e-7, err
 
 
+def _rule(conv, proj, H, Hk, dk, dv, lens, state, tiles=True):
+    """The rule alone on given rows of the convolution [T, q | k | v] and the projection [T, gate | decay | write strength]."""
+    lib, S, dev = ops.load(), len(lens), conv.device
+    T, C = conv.shape
+    cu = torch.tensor([sum(lens[:i]) for i in range(S + 1)], dtype=torch.int32, device=dev)
+    slots = torch.arange(S, dtype=torch.int32, device=dev)
+    g = torch.Generator(device="cuda").manual_seed(11)
+    A_log, dt_bias = torch.randn(H, device=dev, generator=g) * 0.5, torch.randn(H, device=dev, generator=g) - 3.0
+    norm = torch.ones(dv, device=dev)
+    state, out = state.clone(), torch.full((T, H * dv), float("nan"), device=dev)
+    n = lib.kb2_seq_delta_tiles_scratch(T, S, H, Hk, dk, dv) if tiles else 2 * T * Hk * dk + 2 * T * H + T * H * dv + 4
+    scratch = torch.empty(int(n), device=dev)
+    a = (conv.data_ptr(), C, proj.data_ptr(), proj.stride(0), 0, H * dv, H * dv + H, T, S, H, Hk, dk, dv, A_log.data_ptr(), dt_bias.data_ptr(),
+         norm.data_ptr(), 1e-5, state.data_ptr(), cu.data_ptr(), slots.data_ptr(), scratch.data_ptr())
+    s = torch.cuda.current_stream().cuda_stream
+    ops.check(lib.kb2_seq_delta_tiles(*a, int(n), out.data_ptr(), 0, s) if tiles else lib.kb2_seq_delta_rule(*a, out.data_ptr(), 0, s))
+    return out.view(T, H, dv), state
+
+
+@pytest.mark.parametrize("what", ["value", "key", "query", "decay", "strength"])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("H,Hk,dk,dv", [(2, 1, 32, 32), (4, 2, 64, 64), (2, 2, 128, 64)])
+def test_numbers_of_a_token_reach_no_earlier_one(H, Hk, dk, dv, bad, what):
+    """An infinity or a NaN in any place of a tile leaves the tokens before it, the other sequences and (in a value) the other heads alone."""
+    lens, first = [19, 13], 19
+    g = torch.Generator(device="cuda").manual_seed(H + dk)
+    T = sum(lens)
+    conv, proj = torch.randn(T, 2 * Hk * dk + H * dv, device="cuda", generator=g), torch.randn(T, H * dv + 2 * H, device="cuda", generator=g)
+    state = torch.randn(2, H, dk, dv, device="cuda", generator=g)
+    want, _ = _rule(conv, proj, H, Hk, dk, dv, lens, state)
+    assert torch.isfinite(want).all()
+    for t in (0, 3, 6, 7, 8, 15, 17, 18):
+        c, p = conv.clone(), proj.clone()
+        if what in ("decay", "strength"):
+            p[t, H * dv + (H if what == "strength" else 0)] = bad
+        else:
+            c[t, {"value": 2 * Hk * dk, "key": Hk * dk + 1, "query": 1}[what]] = bad
+        got, _ = _rule(c, p, H, Hk, dk, dv, lens, state)
+        assert torch.equal(got[:t], want[:t]) and torch.equal(got[first:], want[first:]), t
+        if what in ("value", "decay", "strength"):
+            assert torch.equal(got[:, 1:], want[:, 1:]), t                        # all of head 0
+
+
 @pytest.mark.parametrize("K,C", [(2, 64), (3, 36), (4, 1028), (4, 30), (5, 64)])
 @pytest.mark.parametrize("lens", [[64], [1, 66, 2, 3, 5, 70], [33, 31, 65]])
 @pytest.mark.parametrize("bias,bias_out,act", [(False, False, True), (True, False, False), (True, True, True)])
