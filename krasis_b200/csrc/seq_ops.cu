@@ -1459,10 +1459,10 @@ template <int NI> struct DeltaTile {
   static_assert(kImageBytes % 16 == 0 && kStageBytes % 16 == 0, "bulk copies");
 };
 
-// fp32 pair -> three words of bf16 pairs whose sums they are, exact to 24 bits (3.39e38 and more becomes NaN; in the recurrence an infinity
-// does one token later)
+// fp32 pair -> three words of bf16 pairs whose sums they are, exact to 24 bits (the largest finite numbers too: their first part stops at the
+// largest bf16 number instead of rounding to infinity; an infinity becomes NaN, as in the recurrence it does one token later)
 __device__ __forceinline__ void split_pair(float x, float y, uint32_t (&p)[3]) {
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p[0]) : "f"(y), "f"(x));
+  asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(p[0]) : "f"(y), "f"(x));
   const float rx = x - __uint_as_float(p[0] << 16), ry = y - __uint_as_float(p[0] & 0xFFFF0000u);
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p[1]) : "f"(ry), "f"(rx));
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p[2]) : "f"(ry - __uint_as_float(p[1] & 0xFFFF0000u)), "f"(rx - __uint_as_float(p[1] << 16)));

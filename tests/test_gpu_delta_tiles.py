@@ -116,6 +116,24 @@ def test_numbers_of_a_token_reach_no_earlier_one(H, Hk, dk, dv, bad, what):
             assert torch.equal(got[:, 1:], want[:, 1:]), t                        # all of head 0
 
 
+@pytest.mark.parametrize("big", [3.3895e38, 3.4e38, -3.4e38])
+@pytest.mark.parametrize("H,Hk,dk,dv", [(2, 1, 32, 32), (2, 2, 128, 64)])
+def test_largest_finite_numbers_stay_finite(H, Hk, dk, dv, big):
+    """A state next to the end of fp32 is decayed and updated as the token-by-token form does it."""
+    lens = [11]
+    g = torch.Generator(device="cuda").manual_seed(dv)
+    conv, proj = torch.randn(11, 2 * Hk * dk + H * dv, device="cuda", generator=g), torch.randn(11, H * dv + 2 * H, device="cuda", generator=g)
+    proj[:, H * dv + H:] = -40.0                                                  # hardly any writing: the state only decays
+    state = torch.randn(1, H, dk, dv, device="cuda", generator=g)
+    state[0, :, dk // 2, ::3] = big
+    want, want_state = _rule(conv, proj, H, Hk, dk, dv, lens, state, tiles=False)
+    got, got_state = _rule(conv, proj, H, Hk, dk, dv, lens, state)
+    assert torch.isfinite(want_state).all() and torch.isfinite(got_state).all()
+    # decays of 11 tokens multiplied one by one or first together, and writes of e^-40 of the products: 32 roundings at most
+    assert ((got_state.double() - want_state.double()).abs() <= 2.0 ** -19 * want_state.double().abs() + 1e-6 * want_state.abs().max().double()).all()
+    assert torch.equal(got.isfinite(), want.isfinite())
+
+
 @pytest.mark.parametrize("K,C", [(2, 64), (3, 36), (4, 1028), (4, 30), (5, 64)])
 @pytest.mark.parametrize("lens", [[64], [1, 66, 2, 3, 5, 70], [33, 31, 65]])
 @pytest.mark.parametrize("bias,bias_out,act", [(False, False, True), (True, False, False), (True, True, True)])
