@@ -215,7 +215,9 @@ KB2_API int64_t kb2_launch_count(const kb2_engine* e);
 
 /* torch.nn.functional.linear for BF16 weights (the reference keeps attention projections in BF16,
  * python/krasis/attention.py:526-529, config.py:209): out[M][N] = x[M][K] . w[N][K]^T (+ bias[N] f32),
- * fp32 accumulate, BF16 (out_f32=0) or FP32 output.  K % 64 == 0, N % 16 == 0. */
+ * fp32 accumulate, BF16 (out_f32=0) or FP32 output.  K % 64 == 0, N % 16 == 0.
+ * A row's sums depend on N and K, not on the rows beside it: one accumulator over K for BF16 output at any M and for FP32 output from 256 rows
+ * on; FP32 output of fewer rows is summed as kb2_linear_bf16_chunked does. */
 KB2_API int kb2_linear_bf16(const void* x_dev, const void* w_dev, const float* bias_dev, void* out_dev, int32_t M,
                             int32_t N, int32_t K, int32_t out_f32, int32_t device, void* stream);
 
@@ -232,9 +234,15 @@ KB2_API int kb2_linear_bf16_binned(const void* x_dev, const void* w_dev, void* o
                                    int32_t tile_rows, const int32_t* tile_group_dev, const int32_t* num_row_tiles_dev, int32_t groups,
                                    int32_t device, void* stream);
 
+/* kb2_linear_bf16 with the accuracy of fp32 sums: 512 products (256 up to K = 512) at a time on the tensor cores, joined in round-to-nearest fp32.
+ * A row's sums depend on N and K, not on the rows beside it.  Meant for a few hundred rows at most: the weights are read once per 128 to 256. */
+KB2_API int kb2_linear_bf16_chunked(const void* x_dev, const void* w_dev, const float* bias_dev, void* out_dev, int32_t M, int32_t N, int32_t K,
+                                    int32_t out_f32, int32_t device, void* stream);
+
 /* Products of fp32 rows on the tensor cores with the accuracy of fp32 sums: out[g][m] = x[g][m] . w[g]^T for M rows in each of `groups` groups,
  * x fp32 (row stride x_ld, group stride x_group), w [groups][N][K] fp32 (w_f32) or bf16, out fp32 or bf16 (row stride out_ld, group stride
- * out_group, multiples of 4).  K % 64 == 0, N % 16 == 0.  The operands are cut into exact bf16 parts in workspace_dev
+ * out_group, multiples of 4).  K % 64 == 0, N % 16 == 0.  A row's sums depend on N, K and groups, not on M.  The operands are cut into exact bf16
+ * parts in workspace_dev
  * (kb2_linear_f32_workspace bytes, 16-byte aligned; 0: sizes not taken). */
 KB2_API size_t kb2_linear_f32_workspace(int32_t M, int32_t N, int32_t K, int32_t w_f32, int32_t groups, int32_t device);
 KB2_API int kb2_linear_f32(const float* x_dev, int64_t x_ld, int64_t x_group, const void* w_dev, int32_t w_f32, void* out_dev, int32_t out_f32,

@@ -143,7 +143,22 @@ KB2_API int kb2_linear_bf16(const void* x_dev, const void* w_dev, const float* b
   if (!x_dev || !w_dev || !out_dev) return failf(KB2_ERR_VALUE, "null argument");
   if (M <= 0 || N <= 0 || K <= 0 || K % 64 || N % 16) return failf(KB2_ERR_VALUE, "linear: need M>0, K %% 64 == 0, N %% 16 == 0 (M=%d N=%d K=%d)", M, N, K);
   CUDA_TRY(cudaSetDevice(device));
+  if (out_f32 && M < kWholeSumRows) return kb2_linear_bf16_chunked(x_dev, w_dev, bias_dev, out_dev, M, N, K, out_f32, device, stream);
   CUDA_TRY(launch_dense_gemm(x_dev, w_dev, out_dev, bias_dev, M, N, K, N, out_f32 != 0, device_sms(device), (cudaStream_t)stream));
+  return KB2_OK;
+}
+
+KB2_API int kb2_linear_bf16_chunked(const void* x_dev, const void* w_dev, const float* bias_dev, void* out_dev, int32_t M, int32_t N, int32_t K,
+                                    int32_t out_f32, int32_t device, void* stream) {
+  if (!x_dev || !w_dev || !out_dev) return failf(KB2_ERR_VALUE, "null argument");
+  SplitPlan plan;
+  if (N <= 0 || !split_gemm_plan(M, N, K, device_sms(device), 1, 1, 1, &plan))
+    return failf(KB2_ERR_VALUE, "linear: need M>0, K %% 64 == 0, N %% 16 == 0 (M=%d N=%d K=%d)", M, N, K);
+  CUDA_TRY(cudaSetDevice(device));
+  SplitGemm g;
+  g.x = x_dev; g.w = w_dev; g.out = out_dev; g.bias = bias_dev;
+  g.M = M; g.N = N; g.K = K; g.ldo = N; g.out_f32 = out_f32 != 0;
+  CUDA_TRY(launch_split_gemm(g, plan, (cudaStream_t)stream));
   return KB2_OK;
 }
 
@@ -184,7 +199,7 @@ static int32_t linear_f32_columns(int32_t N, int32_t K, int32_t w_f32, int32_t g
 }
 static bool linear_f32_plan(int32_t M, int32_t N, int32_t K, int32_t w_f32, int32_t groups, int32_t device, SplitPlan* plan) {
   return M > 0 && N > 0 && K > 0 && K % 64 == 0 && N % 16 == 0 && groups > 0 &&
-         split_gemm_plan(M, N, K, true, device_sms(device), 3, w_f32 ? 3 : 1, groups, plan);
+         split_gemm_plan(M, N, K, device_sms(device), 3, w_f32 ? 3 : 1, groups, plan);
 }
 static size_t x_parts_bytes(const SplitPlan& plan, int32_t M, int32_t K, int32_t groups) {
   return (size_t)groups * ((M + plan.mt - 1) / plan.mt) * plan.mt * 3 * K * 2;

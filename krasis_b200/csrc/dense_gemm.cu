@@ -222,7 +222,7 @@ cudaError_t launch_dense_gemm_scatter(const void* x, const void* w, void* out, c
   if (sc.n_ranks > 0 && (out_f32 || M % sc.n_ranks || sc.rows_per_rank * sc.n_ranks != M)) return cudaErrorInvalidValue;
   if (K % kBlockK || N % 16 || M <= 0) return cudaErrorInvalidValue;
   SplitPlan plan;
-  if (sc.n_ranks == 0 && split_gemm_plan(M, N, K, out_f32, num_sms, 1, 1, 1, &plan)) {
+  if (sc.n_ranks == 0 && split_gemm_plan_whole(M, N, K, num_sms, &plan)) {      // the same sums
     SplitGemm g;
     g.x = x; g.w = w; g.out = out; g.bias = bias;
     g.M = M; g.N = N; g.K = K; g.ldo = ldo; g.out_f32 = out_f32;

@@ -256,39 +256,36 @@ static int ring_stages(int stage, int mt, int kb, bool share) {
   return std::max(std::min({kSMaxStages, room / stage, kb}), ceil_div((long long)mt * kSRows * 4, stage));
 }
 
-// The plan with the least estimated time (us), and whether that beats the 128 x 256 tiles of dense_gemm.cu.  Constants fitted to 700
+// The plan with the least estimated time (us) among those that cut K over ks CTAs (0: over 1, 2, 4 or 8); false: none fits.  Constants fitted to 700
 // timings of M 4..2048 x 14 weight shapes from HBM (the chosen plan is 5 % slower than the best one on average, 20 % at most): an SM takes in
 // 190 KB/us, HBM 5.76 MB/us, a 64-wide K block costs 0.135 us of latency at least, reading out a row 0.05 us + 1.2 ns per accumulator, a
-// launch 1.9 us.  The 128 x 256 tiles take 0.355 us per K block and 5 us around it.  Measured on both sides of the line: M 1000, N 2048, K 2048
-// 12.1 against 18.3 us; M 2048 at the same shape 23.2 against 18.7; M 256, N 12352 21.7 against 23.0; M 515 39.5 against 39.0.
-bool split_gemm_plan(int M, int N, int K, bool out_f32, int num_sms, int xparts, int wparts, int groups, SplitPlan* out) {
-  const bool plain = xparts == 1 && wparts == 1 && groups == 1;
-  if (K % kBlockK || N % 16 || (plain && M > 2048)) return false;
-  const int nkb = K / kBlockK, nb = ceil_div(N, kSRows), most = 256 / xparts / 16 * 16;
+// launch 1.9 us.
+static bool cheapest(int M, int N, int K, bool whole, int num_sms, int xparts, int wparts, int groups, int ks_only, float* best, SplitPlan* out) {
+  const int nkb = K / kBlockK, nb = ceil_div(N, kSRows);
   static const float kShare[4] = {0.f, 0.45f, 0.55f, 1.0f};
-  float best = plain ? 0.355f * nkb * ceil_div((long long)ceil_div(M, 128) * ceil_div(N, 256), num_sms) + 5.f : 1e30f;
   bool found = false;
-  int last = 0;
-  for (int t = ceil_div(M, most), tries = 0; tries < 8; ++t, ++tries) {
-    const int mt = ceil_div(ceil_div(M, t), 16) * 16;
-    if (mt == last || (mt < 32 && M > 32 && xparts == 1)) continue;
-    last = mt;
-    for (int i = 0; i < 4; ++i) {
-      const int ks = 1 << i;
-      if (ks > 1 && nkb < 2 * ks) break;
-      const int kb = ceil_div(nkb, ks);
-      const int chunk = !out_f32 && xparts == 1 ? kb : nkb <= kSplitChunk ? kSplitChunkShort : kSplitChunk;
-      const int sets = ceil_div(kb, chunk) + (xparts > 1 ? 2 : 0);
+  for (int i = 0; i < 4; ++i) {
+    const int ks = 1 << i;
+    if (ks_only ? ks != ks_only : ks > 1 && (whole || nkb < 2 * ks)) continue;
+    const int kb = ceil_div(nkb, ks);
+    const int chunk = whole ? kb : std::max(nkb <= kSplitChunk ? kSplitChunkShort : kSplitChunk, ceil_div(kb, 30));      // tensor memory holds 32 of 16 rows
+    const int sets = ceil_div(kb, chunk) + (xparts > 1 ? 2 : 0);
+    const int most = std::min(256 / xparts, 512 / sets) / 16 * 16;
+    int last = 0;
+    for (int t = ceil_div(M, most), tries = 0; tries < 8; ++t, ++tries) {
+      const int mt = ceil_div(ceil_div(M, t), 16) * 16;
+      if (mt == last || (mt < 32 && most >= 32 && M > 32 && xparts == 1)) continue;
+      last = mt;
       const int stage = wparts * kSWBytes + xparts * mt * 128;
-      if (sets * mt > 512 || ceil_div((long long)mt * kSRows * 4, stage) * stage > 226 * 1024 - 256) continue;
+      if (ceil_div((long long)mt * kSRows * 4, stage) * stage > 226 * 1024 - 256) continue;
       const long long ctas = (long long)ceil_div(M, mt) * groups * nb * ks;
       const int per_sm = ceil_div(ctas, num_sms), cols = mt * (xparts == 1 ? 1 : wparts == 1 ? 3 : 6);
       const float load = (float)per_sm * kb * stage / 190e3f, math = (float)per_sm * kb * cols * (2.f / 1700.f);
       const float hbm = (float)N * K * 2.f * wparts * groups / 5.76e6f;
       const float time = std::max({load, math, hbm, 0.135f * kb}) + mt * (0.05f + 0.0012f * sets) * ceil_div(per_sm, 2) +
                          kShare[i] * ceil_div(per_sm, 2) + 1.9f;
-      if (time >= best) continue;
-      best = time;
+      if (time >= *best) continue;
+      *best = time;
       found = true;
       out->mt = mt;
       out->ks = ks;
@@ -297,6 +294,27 @@ bool split_gemm_plan(int M, int N, int K, bool out_f32, int num_sms, int xparts,
     }
   }
   return found;
+}
+
+// The 128 x 256 tiles of dense_gemm.cu take 0.355 us per K block and 5 us around it; taken here only where that is more.  Measured on both sides
+// of the line: M 1000, N 2048, K 2048 12.1 against 18.3 us; M 2048 at the same shape 23.2 against 18.7; M 256, N 12352 21.7 against 23.0;
+// M 515 39.5 against 39.0.
+bool split_gemm_plan_whole(int M, int N, int K, int num_sms, SplitPlan* out) {
+  if (M <= 0 || M > 2048 || K % kBlockK || N % 16) return false;
+  float best = 0.355f * (K / kBlockK) * ceil_div((long long)ceil_div(M, 128) * ceil_div(N, 256), num_sms) + 5.f;
+  return cheapest(M, N, K, true, num_sms, 1, 1, 1, 1, &best, out);
+}
+
+// K is cut as for a step of 64 rows (128 with operands in parts), whatever M is, so that a row's sums do not depend on the rows beside it.  By the
+// estimate above that costs nothing at 9..255 rows of 14 weight shapes (at most 4 % but for two of 112 cases), and 3 % on average with parts
+// at 9..2048 rows (50 % in the worst case, N 1024, K 2048 at 2048 rows).
+bool split_gemm_plan(int M, int N, int K, int num_sms, int xparts, int wparts, int groups, SplitPlan* out) {
+  if (M <= 0 || K <= 0 || K % kBlockK || N % 16) return false;
+  float best = 1e30f;
+  if (!cheapest(xparts > 1 ? 128 : 64, N, K, false, num_sms, xparts, wparts, groups, 0, &best, out)) return false;
+  const int ks = out->ks;
+  best = 1e30f;
+  return cheapest(M, N, K, false, num_sms, xparts, wparts, groups, ks, &best, out);
 }
 
 SplitPlan split_gemm_binned_plan(int N, int K, bool out_f32, int tile_rows) {

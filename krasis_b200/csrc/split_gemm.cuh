@@ -4,17 +4,19 @@
 
 namespace kb2 {
 
-// 64-wide K blocks per accumulator of an fp32 result.  The tensor core truncates when it adds to an accumulator: the error of a sum grows by
+// 64-wide K blocks per accumulator of sums in chunks.  The tensor core truncates when it adds to an accumulator: the error of a sum grows by
 // 9.3e-10 per K (2.1e-6 at K = 2048, 4.4e-6 at 4096, in the 2-norm).  Sums of 512 products meet in fp32 round-to-nearest instead: 4.8e-7 at
 // any K measured, where sequential fp32 FMAs are 8.1e-7 off at K = 2048 and 1.6e-6 at 8192.  Up to K = 512, where those are 2.0e-7 (K 128)
 // to 4.1e-7 (K 512) off, sums of 256: 2.4e-7.
 constexpr int kSplitChunk = 8, kSplitChunkShort = 4;
+// Products of fewer rows sum in chunks where an fp32 result is asked for (kb2_linear_bf16).
+constexpr int kWholeSumRows = 256;
 
 struct SplitPlan {
   int mt = 0;       // rows of X per tile (a multiple of 16)
   int ks = 1;       // CTAs of a cluster that share a tile along K
   int stages = 0;   // depth of the TMA ring
-  int chunk = 0;    // K blocks per accumulator
+  int chunk = 0;    // K blocks per accumulator (all of a CTA's: one sum)
 };
 
 // x [M][K] and w [groups][N][K] as bf16 arrays, or as three bf16 parts of fp32 arrays laid out by launch_split_parts.
@@ -39,8 +41,10 @@ struct SplitGemm {
   const void* w_raw = nullptr;              // fp32 when wparts is 3, else bf16; rows of K
 };
 
-// false: the 128 x 256 tiles of dense_gemm.cu are the better cut of this product (one part, one group only)
-bool split_gemm_plan(int M, int N, int K, bool out_f32, int num_sms, int xparts, int wparts, int groups, SplitPlan* out);
+// One accumulator over all of K, K block by K block: the sums of dense_gemm.cu, bit for bit.  false: its 128 x 256 tiles are the better cut.
+bool split_gemm_plan_whole(int M, int N, int K, int num_sms, SplitPlan* out);
+// Sums in chunks, in an order that depends on N, K, the parts and the groups, not on M.  false: sizes not taken.
+bool split_gemm_plan(int M, int N, int K, int num_sms, int xparts, int wparts, int groups, SplitPlan* out);
 // binned rows (one weight matrix per row tile): a CTA per tile and 128 columns, K uncut
 SplitPlan split_gemm_binned_plan(int N, int K, bool out_f32, int tile_rows);
 

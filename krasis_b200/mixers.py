@@ -69,9 +69,11 @@ def _core_lib():
     return _core
 
 
-def lin(a: torch.Tensor, w: torch.Tensor, out_dtype=torch.float32) -> torch.Tensor:
-    """a [M, K] (row stride free) @ w [N, K]^T with fp32 accumulation.  Products of more rows than a GEMV takes run on the tensor cores (the
-    core library picks the kernel by the sizes), fp32 operands as exact bf16 parts; at 8 rows and fewer the weights are streamed by a GEMV."""
+def lin(a: torch.Tensor, w: torch.Tensor, out_dtype=torch.float32, min_n: int = 256) -> torch.Tensor:
+    """a [M, K] (row stride free) @ w [N, K]^T with fp32 accumulation.  bfloat16 products run as a GEMV (at most 8 rows, the weights are
+    streamed), on the tensor cores with chunked sums (fewer than 256 rows, or fewer than min_n columns: the accuracy of fp32 sums) or with one
+    accumulator; fp32 products as a GEMV or as exact bf16 parts on the tensor cores.  In each of these a row's sums depend on the sizes of w, not
+    on the rows beside it."""
     M, K = a.shape
     N = w.shape[0]
     if (a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and M > GEMV_ROWS and K % 64 == 0 and N % 16 == 0 and a.is_contiguous()
@@ -80,8 +82,9 @@ def lin(a: torch.Tensor, w: torch.Tensor, out_dtype=torch.float32) -> torch.Tens
         if core:
             from . import capi
             out = torch.empty((M, N), dtype=out_dtype, device=a.device)
-            capi.check(core.kb2_linear_bf16(a.data_ptr(), w.data_ptr(), None, out.data_ptr(), M, N, K, int(out_dtype == torch.float32),
-                                            a.device.index or 0, torch.cuda.current_stream(a.device).cuda_stream))
+            fn = core.kb2_linear_bf16 if M >= 256 and N >= min_n else core.kb2_linear_bf16_chunked
+            capi.check(fn(a.data_ptr(), w.data_ptr(), None, out.data_ptr(), M, N, K, int(out_dtype == torch.float32), a.device.index or 0,
+                          torch.cuda.current_stream(a.device).cuda_stream))
             return out
     # fp32 rows: a handful of them against a large bfloat16 matrix too (an output head of 32768 x 2048: 4 rows 41 us as a GEMV, 32 in parts;
     # 8 rows 80 against 32; one row 28 against 31)
@@ -421,7 +424,7 @@ class SelectiveScan:
         proj = lin(h, self.w_in, torch.float32)                                               # [T, x: C | z: C]
         xc = ops.conv(proj, self.C, self.taps, None, True, tail, tb, bias_out=self.conv_b)    # [T, C] fp32
         big = self.dtype == torch.bfloat16 and T >= 256 and bool(_core_lib())
-        xp = lin(xc.to(torch.bfloat16) if big else xc, self.w_x, torch.float32)     # [T, dt: R | B: N | C: N]
+        xp = lin(xc.to(torch.bfloat16) if big else xc, self.w_x, torch.float32, min_n=16)     # [T, dt: R | B: N | C: N]
         dt_in = lin_cols(xp, 0, self.R, self.w_dt, self.dtype)                                # [T, C]
         y = torch.empty((T, self.C), dtype=self.dtype, device=h.device)
         ops.check(lib.kb2_seq_selective_scan(xc.data_ptr(), xc.stride(0), dt_in.data_ptr(), dt_in.stride(0), self.dt_b.data_ptr(),
@@ -1035,7 +1038,7 @@ class RoutedExperts:
 
     def route(self, h: torch.Tensor):
         """(ids, weights, router product [T, >= E + identity] whose column sg_col is the shared expert's gate input)."""
-        z = lin(h, self.w_router, torch.float32)
+        z = lin(h, self.w_router, torch.float32, min_n=16)
         return ops.route(z, self.correction, self.top, self.groups, self.keep, self.score, self.renorm, self.out_scale, self.group_score,
                          experts=self.E + self.ident, bias=self.router_bias) + (z,)
 
