@@ -229,7 +229,8 @@ KB2_API int kb2_linear_bf16_grouped(const void* x_dev, const void* w_dev, void* 
                                     void* stream);
 
 /* The same for runs padded to tiles of tile_rows rows (a multiple of 16, at most 128), for groups that bring few rows each: the time is that
- * of the weights, and small tiles leave little padding. */
+ * of the weights, and small tiles leave little padding.  Tiles of 16 rows are summed as kb2_linear_bf16_chunked does, larger ones in one
+ * accumulator as above. */
 KB2_API int kb2_linear_bf16_binned(const void* x_dev, const void* w_dev, void* out_dev, int32_t M, int32_t N, int32_t K, int32_t out_f32,
                                    int32_t tile_rows, const int32_t* tile_group_dev, const int32_t* num_row_tiles_dev, int32_t groups,
                                    int32_t device, void* stream);

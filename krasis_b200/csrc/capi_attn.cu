@@ -185,7 +185,7 @@ KB2_API int kb2_linear_bf16_binned(const void* x_dev, const void* w_dev, void* o
   g.x = x_dev; g.w = w_dev; g.out = out_dev;
   g.M = M; g.N = N; g.K = K; g.ldo = N; g.out_f32 = out_f32 != 0;
   g.groups = groups; g.tile_group = tile_group_dev; g.n_tiles_dev = num_row_tiles_dev;
-  CUDA_TRY(launch_split_gemm(g, split_gemm_binned_plan(N, K, out_f32 != 0, tile_rows), (cudaStream_t)stream));
+  CUDA_TRY(launch_split_gemm(g, split_gemm_binned_plan(K, tile_rows), (cudaStream_t)stream));
   return KB2_OK;
 }
 

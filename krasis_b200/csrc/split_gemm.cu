@@ -317,13 +317,14 @@ bool split_gemm_plan(int M, int N, int K, int num_sms, int xparts, int wparts, i
   return cheapest(M, N, K, false, num_sms, xparts, wparts, groups, ks, &best, out);
 }
 
-SplitPlan split_gemm_binned_plan(int N, int K, bool out_f32, int tile_rows) {
+// Tiles of 16 rows sum in chunks, as the products of 9 to 255 rows do; larger ones in one accumulator, as the tiles of 128 rows do: which tile
+// of these a run gets changes nothing in its rows.
+SplitPlan split_gemm_binned_plan(int K, int tile_rows) {
+  const int nkb = K / kBlockK;
   SplitPlan p;
   p.mt = tile_rows;
-  int n_acc = out_f32 ? ceil_div(K / kBlockK, kSplitChunk) : 1;
-  while (n_acc > 1 && n_acc * tile_rows > 256) n_acc = ceil_div(n_acc, 2);         // half of the tensor memory, so that two CTAs share an SM
-  p.chunk = ceil_div(K / kBlockK, n_acc);
-  p.stages = ring_stages(kSWBytes + tile_rows * 128, tile_rows, K / kBlockK, true);
+  p.chunk = tile_rows > 16 ? nkb : std::max(nkb <= kSplitChunk ? kSplitChunkShort : kSplitChunk, ceil_div(nkb, 512 / 16));
+  p.stages = ring_stages(kSWBytes + tile_rows * 128, tile_rows, nkb, true);
   return p;
 }
 

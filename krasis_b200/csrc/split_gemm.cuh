@@ -46,7 +46,7 @@ bool split_gemm_plan_whole(int M, int N, int K, int num_sms, SplitPlan* out);
 // Sums in chunks, in an order that depends on N, K, the parts and the groups, not on M.  false: sizes not taken.
 bool split_gemm_plan(int M, int N, int K, int num_sms, int xparts, int wparts, int groups, SplitPlan* out);
 // binned rows (one weight matrix per row tile): a CTA per tile and 128 columns, K uncut
-SplitPlan split_gemm_binned_plan(int N, int K, bool out_f32, int tile_rows);
+SplitPlan split_gemm_binned_plan(int K, int tile_rows);
 
 cudaError_t launch_split_gemm(const SplitGemm& g, const SplitPlan& plan, cudaStream_t s);
 

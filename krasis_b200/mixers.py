@@ -977,7 +977,7 @@ class RoutedExperts:
                                alpha=alpha) if "shared_up" in weights else None
         self.tile = ops.load().kb2_seq_moe_tile_rows()
         self.gemv_max_tokens = 8
-        # bfloat16 steps longer than the GEMV's that bring at least this many rows per expert run on the tensor cores
+        # bfloat16 steps longer than the GEMV's that bring at least this many rows per expert run on the tensor cores (0: all of them)
         self.tc_min_rows_per_expert = 0
 
     def _bin(self, ids, slots, tile):
@@ -1002,9 +1002,12 @@ class RoutedExperts:
     def _tile_rows(self, slots):
         """Rows of a tile of the binned order, by the rows an expert has on average: the smallest tile that most runs fit in.  64 experts,
         width 2048, ff 1024, us per block: 12 rows 185 (tiles of 16) / 195 (32); 24 rows 213 / 196; 36 rows 222 (32) / 209 (48); 48 rows
-        232 (48) / 225 (64); 72 rows 291 (64) / 263 (128)."""
+        232 (48) / 225 (64); 72 rows 291 (64) / 263 (128).  Tiles of 16 rows sum in chunks and all others in one accumulator, so the line
+        between these two, at a mean of 16 rows, is the only one that a row's sums notice."""
+        if slots < 16 * self.E:
+            return 16
         mean = slots / self.E
-        for tile, most in ((16, 14), (32, 28), (48, 42), (64, 56)):
+        for tile, most in ((32, 28), (48, 42), (64, 56)):
             if mean <= most:
                 return tile
         return 128
@@ -1012,7 +1015,7 @@ class RoutedExperts:
     def _forward_tensor_core(self, h, ids, slots, in_w):
         """bfloat16 steps: rows gathered into the binned order (runs padded to whole tiles), then ONE grouped GEMM per projection: every
         row tile multiplies its expert's matrix, picked from the device-side tile table, and only the tiles that exist are computed — no
-        host round trip.  Few rows per expert: tiles of 32 or 64 rows, a CTA per tile and 128 columns, so that the time is that of the
+        host round trip.  Few rows per expert: tiles of 16 to 64 rows, a CTA per tile and 128 columns, so that the time is that of the
         weights; many: the 128 x 256 tiles of the dense GEMM."""
         from . import capi
         core, E, top, W, F, dev = _core_lib(), self.E, self.top, h.shape[1], self.F, h.device

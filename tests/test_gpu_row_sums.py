@@ -76,3 +76,55 @@ def test_fp32_outputs_are_as_exact_as_fp32_sums(N, K, M):
     # a bf16 result: the nearest bf16 numbers of sums that good; 2e-5 of a rounding error is what sums 7e-7 off can add to it
     got, best = lin(x, w, torch.bfloat16).double(), want.float().bfloat16().double()
     assert (got - want).norm() <= (1 + 2e-5) * (best - want).norm()
+
+
+@pytest.mark.parametrize("W,F", [(2048, 1024), (512, 2560), (256, 8192)])
+def test_expert_rows_do_not_depend_on_the_step(W, F):
+    """Below a mean of 16 rows per expert and from there on, at the depth of a served model (the ring of a tile wraps, several accumulators per tile)."""
+    from krasis_b200.mixers import RoutedExperts
+    E, top = 8, 2
+    g = torch.Generator().manual_seed(F)
+    r = lambda *s, sd: (torch.randn(*s, generator=g) * sd).bfloat16()  # noqa: E731
+    w = {"router": r(E, W, sd=W ** -0.5)}
+    for e in range(E):
+        w.update({f"e{e}_gate": r(F, W, sd=W ** -0.5), f"e{e}_up": r(F, W, sd=W ** -0.5), f"e{e}_down": r(W, F, sd=F ** -0.5)})
+    mod = RoutedExperts(w, E, 0, top, torch.bfloat16, "cuda", score="softmax", renorm=True)
+    h = r(700, W, sd=1.0).cuda()
+    ids, wts, _ = mod.route(h)
+    for lens in ((9, 20, 40, 63), (64, 100, 112, 150, 168, 200, 224, 230, 256, 700)):      # tiles of 16; 32, 48, 64 and 128
+        outs = {}
+        for n in lens:
+            hn = h[:n].contiguous()
+            y, pos = mod._forward_tensor_core(hn, ids[:n].contiguous(), n * top, None)
+            outs[n] = y[pos.long()].view(n, top, W)
+        for n in lens:
+            assert torch.equal(outs[n], outs[lens[-1]][:n]), n
+        x, want = h[:lens[-1]].double(), outs[lens[-1]].double()
+        for e in range(E):
+            tok, j = torch.nonzero(ids[:lens[-1]] == e, as_tuple=True)
+            gu = [(x[tok] @ w[f"e{e}_{n}"].cuda().double().T).bfloat16().double() for n in ("gate", "up")]
+            a = (torch.nn.functional.silu(gu[0]) * gu[1]).bfloat16().double()
+            ref = a @ w[f"e{e}_down"].cuda().double().T
+            # as in the other expert tests: a number next to a rounding edge may fall on the other side, one bf16 step of a few of the F terms
+            assert ((want[tok, j] - ref).norm(dim=1) <= 2.0 ** -8 * ref.norm(dim=1)).all()
+
+
+# a direct call with fp32 output: tiles of 16 rows are as exact as fp32 sums at any depth, the others have one accumulator (1.1e-9 of the sum per K)
+@pytest.mark.parametrize("tile", [16, 32, 48, 64])
+@pytest.mark.parametrize("N,K", [(272, 2048), (144, 8192)])
+def test_binned_product(tile, N, K):
+    from krasis_b200 import capi
+    core = capi.load()
+    E, tiles = 3, 7
+    x, _ = _data(tile * tiles, 16, K)
+    w = (torch.randn(E, N, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(tile)) * K ** -0.5).bfloat16()
+    of = torch.tensor([0, 2, 2, 1, 0, 1, 2], dtype=torch.int32, device="cuda")
+    n = torch.tensor([tiles - 1], dtype=torch.int32, device="cuda")                        # the last tile does not exist
+    out = torch.full((tile * tiles, N), -7.0, device="cuda")
+    capi.check(core.kb2_linear_bf16_binned(x.data_ptr(), w.data_ptr(), out.data_ptr(), tile * tiles, N, K, 1, tile, of.data_ptr(), n.data_ptr(), E, 0,
+                                           torch.cuda.current_stream().cuda_stream))
+    want = torch.einsum("tmk,tnk->tmn", x.view(tiles, tile, K).double(), w[of.long()].double()).view(-1, N)
+    last = tile * (tiles - 1)
+    assert (out[last:] == -7.0).all()
+    err = ((out[:last].double() - want[:last]).norm() / want[:last].norm()).item()
+    assert err < (7e-7 if tile == 16 else 1.2e-9 * K), err
