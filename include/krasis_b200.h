@@ -471,6 +471,10 @@ KB2_API int kb2_comm_reduce_bf16(kb2_comm* c, const void* send_dev, void* recv_d
 KB2_API int kb2_profile_enable(kb2_engine* e, int on);
 KB2_API int kb2_profile_collect(kb2_engine* e, double* total_ms, int64_t* n_spans);
 
+/* The kernels' waits on their own pipelines are bounded (about two seconds); one that runs out lets its kernel finish with wrong data and raises a
+ * flag.  Waits for the device, counts the flags that are up and sets all of them to `put` (0 clears them). */
+KB2_API int kb2_wait_timeouts(int32_t device, int32_t put, int32_t* up);
+
 /* Process-wide kernel accounting: every kernel this library launches is counted (kb2_total_launches) and, while
  * kb2_kernel_profile_enable(1) is in effect, timed with CUDA events on its launching stream.  kb2_kernel_profile_collect
  * synchronises the device and fills total_ms[k] / n_spans[k] for k < kb2_kernel_profile_num(), then clears the record. */

@@ -32,6 +32,9 @@ extern "C" {
 
 KB2SEQ_API const char* kb2_seq_last_error(void);
 KB2SEQ_API long long kb2_seq_total_launches(void);
+/* Waits for the device, counts the bounded waits of this library's kernels that ran out since the flags were last cleared (such a kernel ended with
+ * wrong data) by kernel file, and sets all flags to `put` (0 clears them). */
+KB2SEQ_API int kb2_seq_wait_timeouts(int device, int put, int* up);
 
 /* x[t, :] = table[tokens[t], :] * scale, fp32 out */
 KB2SEQ_API int kb2_seq_embed(const void* table, int dt, const int* tokens, float* x, int T, int W, float scale, void* stream);

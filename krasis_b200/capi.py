@@ -140,6 +140,7 @@ SIGNATURES = {
                                           C.c_int32, C.c_void_p]),
     "kb2_finish_routed_slots": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p]),
     "kb2_comm_reduce_bf16": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_int32, C.c_void_p]),
+    "kb2_wait_timeouts": (C.c_int, [C.c_int32, C.c_int32, C.POINTER(C.c_int32)]),
     "kb2_total_launches": (C.c_int64, []),
     "kb2_kernel_profile_num": (C.c_int, []),
     "kb2_kernel_profile_name": (C.c_char_p, [C.c_int]),
@@ -180,6 +181,14 @@ def kernel_profile_collect():
     ms, cnt = (C.c_double * n)(), (C.c_int64 * n)()
     check(lib.kb2_kernel_profile_collect(ms, cnt))
     return {lib.kb2_kernel_profile_name(i).decode(): (ms[i], cnt[i]) for i in range(n) if cnt[i]}
+
+
+def check_waits(device: int = 0):
+    """Raises if a kernel of this library gave up a wait since the last call: its results are wrong.  Waits for the device."""
+    up = C.c_int32()
+    check(load().kb2_wait_timeouts(device, 0, C.byref(up)))
+    if up.value:
+        raise Kb2Error(f"a kernel gave up waiting for its own pipeline on device {device}: results since the last check are not valid")
 
 
 def total_launches() -> int:

@@ -11,6 +11,7 @@
 
 #include "../../include/krasis_b200.h"
 #include "moe_common.cuh"
+#include "ptx.cuh"
 #include "prof.cuh"
 #include <atomic>
 #include <mutex>
@@ -741,6 +742,12 @@ KB2_API int kb2_last_expert_counts(kb2_engine* e, int32_t* counts_host, void* st
   return KB2_OK;
 }
 
+KB2_API int kb2_wait_timeouts(int32_t device, int32_t put, int32_t* up) {
+  if (!up) return fail(KB2_ERR_VALUE, "null argument");
+  CUDA_TRY(cudaSetDevice(device));
+  CUDA_TRY(exchange_wait_flags(put, up));
+  return KB2_OK;
+}
 KB2_API int64_t kb2_total_launches(void) { return (int64_t)g_launches.load(); }
 KB2_API int kb2_kernel_profile_num(void) { return K_NUM; }
 KB2_API const char* kb2_kernel_profile_name(int id) { return id >= 0 && id < K_NUM ? kKernelNames[id] : ""; }

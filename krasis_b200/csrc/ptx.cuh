@@ -3,6 +3,7 @@
 // Everything here is architecture-specific on purpose: this library targets B200 only.
 #pragma once
 #include <cstdint>
+#include <vector>
 #include <cuda_runtime.h>
 
 namespace kb2 {
@@ -36,9 +37,36 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait: a barrier that does not complete within ~2 s of SM clocks raises a sticky per-module flag and returns, so that a
-// mis-counted pipeline runs to its end (with wrong data) and releases its tensor memory instead of spinning for ever.
+// Bounded wait: a barrier that does not complete within ~2 s of SM clocks raises a sticky flag of its translation unit and returns, so that a
+// mis-counted pipeline runs to its end (with wrong data) and releases its tensor memory instead of spinning for ever.  While the flag is up later
+// waits give up early too: the host reads and clears the flags of a library through wait_flags() where it synchronises anyway.
 static __device__ int g_mbar_timed_out = 0;
+using WaitFlag = cudaError_t (*)(int put, int* was);
+inline std::vector<WaitFlag>& wait_flags() {
+  static std::vector<WaitFlag> all;
+  return all;
+}
+namespace {
+struct ListWaitFlag {
+  ListWaitFlag() {
+    wait_flags().push_back([](int put, int* was) {
+      cudaError_t e = cudaMemcpyFromSymbol(was, g_mbar_timed_out, sizeof(int));
+      return e != cudaSuccess || *was == put ? e : cudaMemcpyToSymbol(g_mbar_timed_out, &put, sizeof(int));
+    });
+  }
+} list_wait_flag;
+}  // namespace
+// Sets every flag of this library on the current device to `put` and counts those that were up; waits for the device.
+inline cudaError_t exchange_wait_flags(int put, int* up) {
+  *up = 0;
+  cudaError_t e = cudaDeviceSynchronize();
+  for (size_t i = 0; i < wait_flags().size() && e == cudaSuccess; ++i) {
+    int was = 0;
+    e = wait_flags()[i](put, &was);
+    *up += was != 0;
+  }
+  return e;
+}
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
   if (mbar_try_wait(bar, parity)) return;
   uint32_t spins = 0;

@@ -867,6 +867,10 @@ class KrasisModel:
     def timing_start(self):
         self.timing, self._spans = True, []
 
+    def check(self):
+        """Waits for the device and raises if a kernel gave up a wait since the last call (see capi.check_waits)."""
+        capi.check_waits(torch.device(self.device).index or 0)
+
     def timing_collect(self):
         torch.cuda.synchronize()
         out = {}

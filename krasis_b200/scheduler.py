@@ -181,4 +181,6 @@ class Scheduler:
                         results[req.index] = req.output
                         running.remove(req)
                         self.finish(req.id)
+        if torch.cuda.is_available() and prompts:
+            ops.check_waits(torch.device(self.model.device).index or 0)
         return results

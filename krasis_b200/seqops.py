@@ -16,6 +16,7 @@ _P, _I, _L, _F = C.c_void_p, C.c_int, C.c_longlong, C.c_float
 SIGNATURES = {
     "kb2_seq_last_error": (C.c_char_p, []),
     "kb2_seq_total_launches": (C.c_longlong, []),
+    "kb2_seq_wait_timeouts": (_I, [_I, _I, C.POINTER(C.c_int)]),
     "kb2_seq_embed": (_I, [_P, _I, _P, _P, _I, _I, _F, _P]),
     "kb2_seq_gemm": (_I, [_P, _I, _L, _P, _I, _L, _P, _I, _L, _I, _I, _I, _I, _L, _L, _L, _P]),
     "kb2_seq_residual_norm": (_I, [_P, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _F, _P]),
@@ -87,6 +88,18 @@ def check(rc: int):
     if rc == 2:
         raise ValueError(msg)
     raise SeqOpsError(msg)
+
+
+def check_waits(device: int = 0):
+    """Raises if a kernel of the sequence library, or of the core library if the process uses it, gave up a wait since the last call: its results
+    are wrong.  Waits for the device."""
+    from . import capi
+    up = C.c_int()
+    check(load().kb2_seq_wait_timeouts(device, 0, C.byref(up)))
+    if capi._lib is not None:
+        capi.check_waits(device)
+    if up.value:
+        raise SeqOpsError(f"a kernel gave up waiting for its own pipeline on device {device}: results since the last check are not valid")
 
 
 def total_launches() -> int:

@@ -24,6 +24,7 @@ def main(argv=None) -> int:
     a = ap.parse_args(argv)
 
     import torch
+    from . import seqops as ops
     from .registry import load_model
     from .scheduler import Scheduler
 
@@ -40,14 +41,13 @@ def main(argv=None) -> int:
             continue
         msg = json.loads(line)
         logits = sched.step([(e["id"], e["tokens"], e.get("want", [])) for e in msg.get("entries", [])])
+        ops.check_waits(a.device)                   # waits for the step
         if logits is not None:
             data = logits.to(torch.float32).contiguous().cpu().numpy().astype("<f4")
             tmp = os.path.join(a.out, f".{msg['step']}.part")
             with open(tmp, "wb") as f:
                 f.write(data.tobytes())
             os.replace(tmp, os.path.join(a.out, f"{msg['step']}.f32"))
-        else:
-            torch.cuda.synchronize()
         for rid in msg.get("end", []):
             if rid in sched.live:
                 sched.finish(rid)
