@@ -37,6 +37,7 @@ from . import capi
 from .attention import (GatedDeltaNetAttention, GQAAttention, MLAAttention, MLAPagedKVCache, PagedKVCache,
                         SequenceKVState)
 from .engine import KrasisEngine
+from .graphs import capture
 from . import layers as L
 
 
@@ -829,10 +830,7 @@ class KrasisModel:
                 for _ in range(2):
                     fresh_step()
             torch.cuda.current_stream(self.device).wait_stream(side)
-            torch.cuda.synchronize(self.device)
-            graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(graph):
-                out = fresh_step()
+            graph, out = capture(fresh_step, self.device)
             return (graph, st_tok, st_pos, out, seq)
         except Exception as exc:                 # noqa: BLE001 — any capture problem means "use the eager path", never a wrong result
             import warnings

@@ -15,6 +15,7 @@ import torch
 
 from . import seqops as ops
 from .attention import SequenceKVState
+from .graphs import capture
 from .sampling import Sampler, SamplingParams
 
 
@@ -111,10 +112,7 @@ class Scheduler:
                 with torch.cuda.stream(side):
                     self.model.forward_step(tb, all_rows)
                 torch.cuda.current_stream(dev).wait_stream(side)
-                torch.cuda.synchronize(dev)
-                graph = torch.cuda.CUDAGraph()
-                with torch.cuda.graph(graph):
-                    out = self.model.forward_step(tb, all_rows)
+                graph, out = capture(lambda: self.model.forward_step(tb, all_rows), dev)
                 for t, sv in zip(self.state_pool.tensors, saved):
                     t.copy_(sv)
                 ent = (graph, buf, out, all_rows)          # everything the captured launches read stays alive with the graph
