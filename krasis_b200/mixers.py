@@ -321,21 +321,24 @@ class GatedDeltaMixer:
         ops.check(lib.kb2_seq_conv_silu(proj.data_ptr(), proj.stride(0), T, tb.S, self.C, self.K, self.taps.data_ptr(), tail.data_ptr(),
                                         tb.seq_of.data_ptr(), tb.cu.data_ptr(), tb.slots.data_ptr(), conv.data_ptr(), s))
         o = torch.empty((T, self.H * self.dv), dtype=self.dtype, device=h.device)
-        if self.register_state_kernel and tb.max_portion >= self.tile_min_portion:      # long portions: eight tokens at a time
-            n = int(lib.kb2_seq_delta_tiles_scratch(T, tb.S, self.H, self.Hk, self.dk, self.dv))
-            scratch = torch.empty(n, dtype=torch.float32, device=h.device)
-            ops.check(lib.kb2_seq_delta_tiles(conv.data_ptr(), self.C, proj.data_ptr(), proj.stride(0), self.g_off, self.a_off, self.b_off, T, tb.S,
-                                              self.H, self.Hk, self.dk, self.dv, self.A_log.data_ptr(), self.dt_bias.data_ptr(), self.norm.data_ptr(),
-                                              self.eps, state.data_ptr(), tb.cu.data_ptr(), tb.slots.data_ptr(), scratch.data_ptr(), n, o.data_ptr(),
-                                              ops.dt_code(self.dtype), s))
-            return lin(o, self.w_o, torch.float32)
-        scratch = None
-        if self.register_state_kernel or self.dk * self.dv > 32768:      # a large state is cut into column slices that meet in scratch
-            scratch = torch.empty(2 * T * self.Hk * self.dk + 2 * T * self.H + T * self.H * self.dv + 4, dtype=torch.float32, device=h.device)
-        ops.check(lib.kb2_seq_delta_rule(conv.data_ptr(), self.C, proj.data_ptr(), proj.stride(0), self.g_off, self.a_off, self.b_off, T,
-                                         tb.S, self.H, self.Hk, self.dk, self.dv, self.A_log.data_ptr(), self.dt_bias.data_ptr(),
-                                         self.norm.data_ptr(), self.eps, state.data_ptr(), tb.cu.data_ptr(), tb.slots.data_ptr(),
-                                         scratch.data_ptr() if scratch is not None else None, o.data_ptr(), ops.dt_code(self.dtype), s))
+        # the form follows from a sequence's own portion, so that its sums do not depend on the other sequences of the step
+        runs = portion_runs(tb, self.tile_min_portion if self.register_state_kernel else None)
+        for tiles, seqs, r0, n in runs:
+            cu, slots = tb.cu, tb.slots
+            if len(runs) > 1:
+                cu, slots = cu[seqs[0]:seqs[-1] + 2] - r0, slots[seqs[0]:seqs[-1] + 1]
+            S = len(seqs)
+            args = (_row(conv, r0), self.C, _row(proj, r0), proj.stride(0), self.g_off, self.a_off, self.b_off, n, S, self.H, self.Hk, self.dk, self.dv,
+                    self.A_log.data_ptr(), self.dt_bias.data_ptr(), self.norm.data_ptr(), self.eps, state.data_ptr(), cu.data_ptr(), slots.data_ptr())
+            if tiles:                    # long portions: eight tokens at a time
+                size = int(lib.kb2_seq_delta_tiles_scratch(n, S, self.H, self.Hk, self.dk, self.dv))
+                scratch = torch.empty(size, dtype=torch.float32, device=h.device)
+                ops.check(lib.kb2_seq_delta_tiles(*args, scratch.data_ptr(), size, _row(o, r0), ops.dt_code(self.dtype), s))
+                continue
+            scratch = None
+            if self.register_state_kernel or self.dk * self.dv > 32768:      # a large state is cut into column slices that meet in scratch
+                scratch = torch.empty(2 * n * self.Hk * self.dk + 2 * n * self.H + n * self.H * self.dv + 4, dtype=torch.float32, device=h.device)
+            ops.check(lib.kb2_seq_delta_rule(*args, ops._ptr(scratch), _row(o, r0), ops.dt_code(self.dtype), s))
         return lin(o, self.w_o, torch.float32)
 
 

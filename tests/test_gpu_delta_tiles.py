@@ -69,8 +69,31 @@ def test_tiles_against_exact_and_token_form(H, Hk, dk, dv, lens, decay):
         err[name] = (((got.double() - want).norm() / want.norm()).item(), ((state.double() - states).norm() / states.norm()).item())
         untouched = [i for i in range(5) if i not in slots]
         assert torch.equal(state[untouched], state0[untouched])
-    # the same fp32 sums in another order: no further off than the token-by-token form, with room for the luck of a few thousand numbers
-    assert err["tiles"][0] <= 1.5 * err["tokens"][0] + 2e-7 and err["tiles"][1] <= 1.5 * err["tokens"][1] + 2e-7, err
+    # the same fp32 sums in another order: no further off than the token-by-token form, with room for the luck of a few thousand numbers (measured
+    # over these and longer portions: outputs 0.81 to 1.02 times its error, states 0.57 to 1.13 times)
+    assert err["tiles"][0] <= 1.05 * err["tokens"][0] and err["tiles"][1] <= 1.2 * err["tokens"][1], err
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lens", [[70, 20, 12, 65], [12, 300, 20], [64, 63, 64], [9, 128]])
+def test_a_sequence_does_not_depend_on_the_step(lens, dtype):
+    """Portions on both sides of the tile form's first length, beside one another and alone: the same numbers bit for bit."""
+    m = _mixer(8, 4, 128, 64, dtype)
+    g = torch.Generator(device="cuda").manual_seed(9)
+    h = torch.randn(sum(lens), 64, device="cuda", generator=g).to(dtype)
+    tail0, state0 = torch.randn(5, m.C, 3, device="cuda", generator=g), torch.randn(5, 8, 128, 64, device="cuda", generator=g)
+
+    def run(rows, entries):
+        tail, state = tail0.clone(), state0.clone()
+        o = m.forward(rows, ops.StepTables(entries, "cuda"), tail, state)
+        return o, tail, state
+    whole, tail, state = run(h, [([0] * n, 9, s, [0]) for s, n in enumerate(lens)])
+    at = 0
+    for s, n in enumerate(lens):
+        if dtype == torch.float32 or (n >= 256) == (sum(lens) >= 256):              # bf16 projections take another kernel from 256 rows on
+            alone, t1, s1 = run(h[at:at + n].contiguous(), [([0] * n, 9, s, [0])])
+            assert torch.equal(state[s], s1[s]) and torch.equal(tail[s], t1[s]) and torch.equal(whole[at:at + n], alone)
+        at += n
 
 
 def _rule(conv, proj, H, Hk, dk, dv, lens, state, tiles=True):
