@@ -42,8 +42,8 @@ __global__ void __launch_bounds__(kDThreads, 1)
   uint64_t* acc_full = empty + kDStages;     // [2]
   uint64_t* acc_empty = acc_full + 2;        // [2]
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(acc_empty + 2);
-  // warp index through a shuffle so that the role branches are provably warp-uniform: the single-thread instructions (TMA, tcgen05.mma,
-  // commit) then take their operands from uniform registers instead of an ELECT + R2UR.BROADCAST loop per instruction
+  // warp index through a shuffle so that the role branches are provably warp-uniform: tcgen05.mma issued from a divergent single-thread branch
+  // cost about 50 cycles more each (profiles/r02h_mma_uniform_ubench.txt)
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int n_tiles = (N + kDTileN - 1) / kDTileN, m_tiles_max = (M + kDTileM - 1) / kDTileM;
   const int m_tiles = m_tiles_dev != nullptr ? min(m_tiles_max, m_tiles_dev[0]) : m_tiles_max;

@@ -91,9 +91,8 @@ __device__ __forceinline__ uint32_t sw128_off(int row, int k, int chunk_stride) 
   return (uint32_t)((k >> 6) * chunk_stride + row * 128 + ((((kk >> 3) ^ (row & 7)) << 4) | ((kk & 7) << 1)));
 }
 
-// x = hi + lo with hi = bf16_rne(x), lo = bf16_rne(x - hi): |x - hi - lo| <= 2^-17 |x|.  Both conversions go through the packed
-// converter (bf16_bits_rn, ptx.cuh): the F2F.BF16.F32 nvcc emitted for the hi half issues at quarter rate and was the bound of the
-// tile-writing phases.  (An integer-arithmetic variant with a truncated lo was measured slower, 340 vs 318 us per scan.)
+// x = hi + lo with hi = bf16_rne(x), lo = bf16_rne(x - hi): |x - hi - lo| <= 2^-17 |x|.  Both are packed conversions (bf16_bits_rn, ptx.cuh):
+// single ones were the bound of the tile-writing phases.  (An integer-arithmetic variant with a truncated lo was measured slower, 340 vs 318 us per scan.)
 __device__ __forceinline__ void split_bf16(float x, unsigned short& hi, unsigned short& lo) {
   const uint32_t h = bf16_bits_rn(x);
   const uint32_t l = bf16_bits_rn(x - __uint_as_float(h << 16));
@@ -147,8 +146,8 @@ __global__ void __launch_bounds__(kT3Threads, 1)
   uint64_t* g2_done = bars + 7;
   uint64_t* g3_done = bars + 8;
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 10);
-  // warp index through a shuffle: the role branches are then provably warp-uniform and the operands of tcgen05.mma / commit / TMA
-  // stay in uniform registers (from a divergent `tid == 288` branch every MMA paid an ELECT + R2UR.BROADCAST loop, ~50 cycles)
+  // warp index through a shuffle: the role branches are then provably warp-uniform (from a divergent `tid == 288` branch every MMA cost about 50
+  // cycles of issue)
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int h = blockIdx.x, sl = blockIdx.y;
   const int kh = h / (p.nv / p.nk);

@@ -208,8 +208,8 @@ __global__ void __launch_bounds__(kFThreads, 1)
   uint64_t* p_full = bars + 7;
   uint64_t* pv_done = bars + 8;      // [2]: PV(it) commits to pv_done[it & 1] (P is double-buffered)
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 14);
-  // shuffle-broadcast warp index: role branches provably warp-uniform -> TMA / tcgen05 operands stay in uniform registers (issued
-  // from a divergent `lane == 0` branch each tcgen05.mma pays an ELECT + R2UR.BROADCAST loop of ~50 cycles, more than an N=64 MMA runs)
+  // shuffle-broadcast warp index: role branches provably warp-uniform (issued from a divergent `lane == 0` branch each tcgen05.mma costs about
+  // 50 cycles, more than an N=64 MMA runs)
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   // heavy (late) query tiles first, over all heads: with them first within each head only, the last head's heaviest tile began with the last
   // wave (16 heads x 16 tiles of 128 queries after 2500 cached keys, one CTA per SM: 159 -> 142 us)

@@ -119,7 +119,7 @@ __device__ __forceinline__ float silu_f(float x) { return __fdividef(x, 1.0f + _
 // (w & 0x000F000F) | 0x43004300 == bf16x2 {128 + nib_lo, 128 + nib_hi}; subtracting 136 gives the
 // signed value exactly, the multiply by the BF16 group scale then rounds once (RNE) — identical to
 // bf16((nib - 8) * scale) of the oracle.
-// `magic` is 0x43004300 from the kernel's parameters: with two literals the compiler makes two instructions of the and and the or.
+// `magic` is 0x43004300, a kernel parameter and not a literal: part of the figures at the head of this file.
 __device__ __forceinline__ uint32_t deq_pair_int4(uint32_t w_shifted, uint32_t magic, __nv_bfloat162 scale2) {
   uint32_t t = (w_shifted & 0x000F000Fu) | magic;
   __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&t);
@@ -169,10 +169,9 @@ __global__ void __launch_bounds__(kNumThreads, 1)
   uint64_t* tmem_empty = tmem_full + kAccBufs;
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(smem + L::kOffTmemPtr);
 
-  // warp index through a shuffle: the compiler then KNOWS the role branches below are warp-uniform and keeps the operands of the
-  // single-thread instructions (tcgen05.mma / commit, TMA) in uniform registers.  Issued from a divergent `lane == 0` branch every
-  // tcgen05.mma was wrapped in an ELECT + 5 x R2UR.BROADCAST loop: ~50 cycles of issue per MMA, which made the K loop issue-bound
-  // (135 cycles per N=160 MMA in situ against 80 of execution: profiles/r02h_gemm_item_timeline.txt, r02h_mma_uniform_ubench.txt).
+  // warp index through a shuffle: the role branches below are then provably warp-uniform.  Issued from a divergent `lane == 0` branch every
+  // tcgen05.mma took about 50 cycles of issue, which made the K loop issue-bound (135
+  // cycles per N=160 MMA in situ against 80 of execution: profiles/r02h_gemm_item_timeline.txt, r02h_mma_uniform_ubench.txt).
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
 

@@ -187,25 +187,23 @@ __device__ __forceinline__ uint64_t umma_desc_k_sw128(uint32_t smem_addr) {
 }
 // Instruction descriptor for kind::f16, A=B=BF16, D=F32, both K-major, M=128, N=n
 // (cute::UMMA::InstrDescriptor: c_format [4,6)=1 | a_format [7,10)=1 | b_format [10,13)=1 | n>>3 [17,23) | m>>4 [24,29)).
-// e^x through one MUFU.EX2, executed unconditionally: written as `cond ? acc * __expf(x) : 0.f` nvcc branches around the exponential,
-// and one divergent basic block per element (with the MUFU latency exposed in each) made the masked decay matrices of the GDN
-// chunk-prepare latency-bound.  Compute first, select afterwards.
+// e^x by one ex2.approx, executed unconditionally: written as `cond ? acc * __expf(x) : 0.f` the masked decay matrices of the GDN
+// chunk-prepare were latency-bound.  Compute first, select afterwards.
 __device__ __forceinline__ float exp_fast_nobranch(float x) {
   float y;
   asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
   return y;
 }
 
-// bf16 RNE of one float, result in the LOW 16 bits (high bits zero), through the PACKED converter (F2FP.BF16.F32.PACK_AB, full
-// rate).  When the converted value is reused as an integer nvcc picks the single-value F2F.BF16.F32 for __float2bfloat16_rn, which
-// issues on the quarter-rate conversion pipe: 8 issue cycles per warp instruction bounded the CUDA-core phases of the tcgen05
-// Gated-DeltaNet kernels (profiles/r02g_*).
+// bf16 RNE of one float, result in the LOW 16 bits (high bits zero), by the packed conversion: with __float2bfloat16_rn on single values that are
+// reused as integers, conversions bounded the CUDA-core phases of the tcgen05 Gated-DeltaNet kernels (gdn_prep 155 -> 129 us, prepare 347 -> 325 us,
+// profiles/r02g_*).
 __device__ __forceinline__ uint32_t bf16_bits_rn(float x) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(0.f), "f"(x));
   return r;
 }
-// round to bf16 and back (the "bf16r" of the numerics contracts) without the quarter-rate F2F
+// round to bf16 and back (the "bf16r" of the numerics contracts)
 __device__ __forceinline__ float bf16_round_rn(float x) { return __uint_as_float(bf16_bits_rn(x) << 16); }
 // two floats -> packed bf16x2 {low half = bf16(lo), high half = bf16(hi)}
 __device__ __forceinline__ uint32_t bf16x2_bits_rn(float hi, float lo) {

@@ -1,7 +1,7 @@
 // Micro-benchmark (tuning aid, not product): cost of issuing small tcgen05.mma instructions from one thread.
 //   for N in {32, 64, 128, 256}: 64 back-to-back MMAs (M=128, K=16, BF16) with (a) descriptors recomputed per MMA, (b) one
 //   descriptor pair reused; clock64 from first issue to last issue ("issue") and to the commit's mbarrier completion ("done").
-// Build: nvcc -gencode arch=compute_100a,code=sm_100a -O3 -I krasis_b200/csrc scripts/ubench/mma_issue.cu -o gpurun_out/mma_issue
+// Build: nvcc -gencode arch=compute_100a,code=sm_100a -O3 -I krasis_b200/csrc scripts/ubench/mma_issue.cu -o krasis_b200/_lib/mma_issue
 #include <cstdio>
 #include <cuda_runtime.h>
 #include "ptx.cuh"

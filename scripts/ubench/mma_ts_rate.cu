@@ -1,7 +1,7 @@
 // Micro-benchmark (tuning aid, not product): sustained rate of the grouped GEMM's MMA pattern.
 //   per "K step": 4 x (acc0 += A0[k] B[k]; acc1 += A1[k] B[k]) with M=128, K=16, N tokens; A from TMEM (TS) or from shared memory (SS)
 //   256 K steps back to back from one thread, one commit at the end.  Reports cycles per MMA and MAC/clk.
-// Build: nvcc -gencode arch=compute_100a,code=sm_100a -O3 -I krasis_b200/csrc scripts/ubench/mma_ts_rate.cu -o gpurun_out/mma_ts_rate
+// Build: nvcc -gencode arch=compute_100a,code=sm_100a -O3 -I krasis_b200/csrc scripts/ubench/mma_ts_rate.cu -o krasis_b200/_lib/mma_ts_rate
 #include <cstdio>
 #include <cuda_runtime.h>
 #include "ptx.cuh"

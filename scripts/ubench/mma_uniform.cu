@@ -1,6 +1,6 @@
 // Micro-benchmark (tuning aid, not product): cost of issuing tcgen05.mma from (a) a divergent single-thread branch
-// (`if (threadIdx.x == 32)`: nvcc wraps every MMA in an ELECT / R2UR.BROADCAST uniformisation loop) versus (b) a branch the compiler
-// knows to be warp-uniform (warp index taken through __shfl_sync) with the MMA under elect.sync: operands live in uniform registers.
+// (`if (threadIdx.x == 32)`) versus (b) a branch the compiler knows to be warp-uniform (warp index taken through __shfl_sync) with the MMA under
+// elect.sync.
 // Build: nvcc -gencode arch=compute_100a,code=sm_100a -O3 -I krasis_b200/csrc scripts/ubench/mma_uniform.cu -o krasis_b200/_lib/mma_uniform
 #include <cstdio>
 #include <cuda_runtime.h>

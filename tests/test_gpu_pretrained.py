@@ -1,4 +1,4 @@
-"""Real-format checkpoints through KrasisModel.from_pretrained (VERDICT r01 item 6): the test WRITES a tiny HF-layout model
+"""Real-format checkpoints through KrasisModel.from_pretrained: the test WRITES a tiny HF-layout model
 directory (config.json + model.safetensors with the tensor names, dtypes and storage conventions of the real checkpoints:
 Qwen3-Next norm weights stored as w - 1, A_log / dt_bias in F32, per-expert or stacked expert tensors, kv_b_proj, tied or
 separate lm_head), loads it like the reference's KrasisModel.load() (python/krasis/model.py:505-611) and compares

@@ -1,4 +1,4 @@
-"""Parity at the sizes the benchmark runs (VERDICT r01 "next round" item 1).
+"""Parity at the sizes the benchmark runs.
 
 (i)   GQA flash attention (`gqa_fmha_kernel<256,256>`) at M = 8192, 16 query / 2 KV heads, gated, partial rotary, FP8
       paged cache: one 8192-token call and a 4096 + 4096 two-chunk call, against the fp32 oracle on sampled query rows of
