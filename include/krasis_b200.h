@@ -242,8 +242,8 @@ KB2_API int kb2_linear_bf16_chunked(const void* x_dev, const void* w_dev, const 
 
 /* Products of fp32 rows on the tensor cores with the accuracy of fp32 sums: out[g][m] = x[g][m] . w[g]^T for M rows in each of `groups` groups,
  * x fp32 (row stride x_ld, group stride x_group), w [groups][N][K] fp32 (w_f32) or bf16, out fp32 or bf16 (row stride out_ld, group stride
- * out_group, multiples of 4).  K % 64 == 0, N % 16 == 0.  A row's sums depend on N, K and groups, not on M.  The operands are cut into exact bf16
- * parts in workspace_dev
+ * out_group, multiples of 4).  K % 64 == 0, N % 16 == 0.  A row's sums depend on N, K and groups, not on M.  The operands are cut into bf16
+ * parts in workspace_dev, exact but for what lies below 2^-134 (numbers below 1e-33 keep fewer than 24 bits)
  * (kb2_linear_f32_workspace bytes, 16-byte aligned; 0: sizes not taken). */
 KB2_API size_t kb2_linear_f32_workspace(int32_t M, int32_t N, int32_t K, int32_t w_f32, int32_t groups, int32_t device);
 KB2_API int kb2_linear_f32(const float* x_dev, int64_t x_ld, int64_t x_group, const void* w_dev, int32_t w_f32, void* out_dev, int32_t out_f32,

@@ -25,7 +25,7 @@ cudaError_t launch_router_logits(const void* h, const void* gate, const float* b
                                  int H, cudaStream_t s);
 bool router_gemm_supported(int E, int H);
 cudaError_t launch_router_gemm(const void* x, const void* tmap_g, const float* bias, float* logits, int M, int E,
-                               int H, cudaStream_t s);
+                               int H, int num_sms, cudaStream_t s);
 cudaError_t launch_router_topk(const float* logits, const float* corr_bias, int M, int E, int top_k, int scoring,
                                int renorm, int* ids, float* wts, cudaStream_t s);
 cudaError_t launch_binning(const int* ids, const float* wts, int M, int top_k, int e_start, int e_end, int chunk_tokens, int* counts,
@@ -517,7 +517,7 @@ KB2_API int kb2_route(kb2_engine* e, int layer, const void* hidden, int32_t M, i
   cudaStream_t s = (cudaStream_t)stream;
   { ProfSpan ps(e, KB2_PROF_ROUTER_LOGITS, s);
     if (L.has_tmap_gate)   // tcgen05 path (E <= 512); the fp32-FMA kernel remains for larger / odd expert counts
-      CUDA_TRY(launch_router_gemm(hidden, L.tmap_gate, L.gate_bias, e->logits, M, e->cfg.n_routed_experts, e->cfg.hidden_size, s));
+      CUDA_TRY(launch_router_gemm(hidden, L.tmap_gate, L.gate_bias, e->logits, M, e->cfg.n_routed_experts, e->cfg.hidden_size, e->num_sms, s));
     else
       CUDA_TRY(launch_router_logits(hidden, L.gate, L.gate_bias, e->logits, M, e->cfg.n_routed_experts, e->cfg.hidden_size, s)); }
   ProfSpan ps2(e, KB2_PROF_ROUTER_TOPK, s);

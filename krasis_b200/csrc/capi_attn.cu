@@ -228,11 +228,11 @@ KB2_API int kb2_linear_f32(const float* x_dev, int64_t x_ld, int64_t x_group, co
   SplitPlan plan;                       // one plan for all slices: the row tiles of the parts follow it
   linear_f32_plan(M, cols, K, w_f32, groups, device, &plan);
   char* wparts = (char*)workspace_dev + x_parts_bytes(plan, M, K, groups);
-  CUDA_TRY(launch_split_parts(x_dev, x_ld, x_group, M, K, plan.mt, groups, workspace_dev, s));
+  CUDA_TRY(launch_split_parts(x_dev, x_ld, x_group, M, K, plan.mt, groups, workspace_dev, device_sms(device), s));
   for (int32_t n0 = 0; n0 < N; n0 += cols) {
     SplitGemm g;
     g.N = std::min(cols, N - n0);
-    if (w_f32) CUDA_TRY(launch_split_parts((const float*)w_dev + (size_t)n0 * K, K, 0, groups * g.N, K, groups * g.N, 1, wparts, s));
+    if (w_f32) CUDA_TRY(launch_split_parts((const float*)w_dev + (size_t)n0 * K, K, 0, groups * g.N, K, groups * g.N, 1, wparts, device_sms(device), s));
     g.x = workspace_dev; g.w = w_f32 ? wparts : w_dev;
     g.out = (char*)out_dev + (size_t)n0 * (out_f32 ? 4 : 2);
     g.M = M; g.K = K; g.ldo = out_ld; g.out_f32 = out_f32 != 0;

@@ -157,7 +157,7 @@ static cudaError_t launch_router_tile(const CUtensorMap& tx, const CUtensorMap& 
 
 // tmap_g: tensor map over gate [E][H] with box rows 64 (built once per layer); x: [M][H] bf16
 cudaError_t launch_router_gemm(const void* x, const void* tmap_g, const float* bias, float* logits, int M, int E,
-                               int H, cudaStream_t s) {
+                               int H, int num_sms, cudaStream_t s) {
   KernelSpan ks(K_ROUTER_GEMM, s);
   alignas(64) CUtensorMap tx;
   cudaError_t e = make_tmap_bf16_rows(&tx, x, M, H, 128);
@@ -165,7 +165,7 @@ cudaError_t launch_router_gemm(const void* x, const void* tmap_g, const float* b
   const CUtensorMap& tg = *reinterpret_cast<const CUtensorMap*>(tmap_g);
   // Few tokens: the K loop waits for its tiles, so more and narrower CTAs with nine stages in flight (3 x 256 experts 12.4 -> 7.4 us, 389 x 64 11.8 -> 8.9), as long as one wave of
   // them holds the problem: past that the token tile is read E / 64 times where wide CTAs read it E / 256 times.
-  if ((long long)((M + 127) / 128) * ((E + 63) / 64) <= 148) return launch_router_tile<64>(tx, tg, bias, logits, M, E, H, s);
+  if ((long long)((M + 127) / 128) * ((E + 63) / 64) <= num_sms) return launch_router_tile<64>(tx, tg, bias, logits, M, E, H, s);
   return launch_router_tile<256>(tx, tg, bias, logits, M, E, H, s);
 }
 

@@ -12,7 +12,8 @@
 // Grouped form: row tile i of X multiplies matrix tile_group[i] (routed experts on binned rows); only the first n_tiles_dev[0] row tiles
 // exist, the CTAs of the others return at once.  Batched form: group g has M rows and a matrix of its own (per-head products).
 //
-// fp32 operands: x = x1 + x2 + x3 with bf16 parts of 8 bits each, exactly.  The parts of a tile's rows lie side by side on the N side, so one
+// fp32 operands: x = x1 + x2 + x3 with bf16 parts of 8 bits each, exactly (Henry, Tang and Heinecke, "Leveraging the bfloat16 Artificial
+// Intelligence Datatype For Higher-Precision Computations", ARITH 2019).  The parts of a tile's rows lie side by side on the N side, so one
 // weight tile serves all of them: w x1 goes to the main accumulators, w x2 and w x3 to two small ones.  With fp32 weights in three parts
 // too, w1 [x1 x2 x3], w2 [x1 x2] and w3 [x1] are added in: six of the nine products, the other three are below 2^-26 of the result.  512 rows,
 // N 16384, K 2048: 231 us, 2-norm error 4.7e-7; fp32-FMA tiles 1494 us, 8.1e-7.
@@ -436,11 +437,12 @@ __global__ void __launch_bounds__(256) split_parts_kernel(const float* __restric
   }
 }
 
-cudaError_t launch_split_parts(const float* x, long long ld, long long group_stride, int rows, int K, int mt, int groups, void* parts, cudaStream_t s) {
+cudaError_t launch_split_parts(const float* x, long long ld, long long group_stride, int rows, int K, int mt, int groups, void* parts,
+                               int num_sms, cudaStream_t s) {
   KernelSpan span(K_DENSE_BF16, s);
   const int tiles = ceil_div(rows, mt);
   const long long total = (long long)groups * tiles * mt * (K / 8);
-  const unsigned blocks = (unsigned)std::min<long long>((total + 255) / 256, 148 * 16);
+  const unsigned blocks = (unsigned)std::min<long long>((total + 255) / 256, num_sms * 16);
   const bool vec = !((uintptr_t)x & 15) && ld % 4 == 0 && group_stride % 4 == 0;
   if (vec) split_parts_kernel<true><<<blocks, 256, 0, s>>>(x, ld, group_stride, rows, K, mt, tiles, total, (__nv_bfloat16*)parts);
   else split_parts_kernel<false><<<blocks, 256, 0, s>>>(x, ld, group_stride, rows, K, mt, tiles, total, (__nv_bfloat16*)parts);

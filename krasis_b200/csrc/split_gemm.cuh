@@ -52,6 +52,7 @@ cudaError_t launch_split_gemm(const SplitGemm& g, const SplitPlan& plan, cudaStr
 
 // fp32 [groups][rows][K] (row stride ld, group stride group_stride) -> bf16 parts hi, mid, lo with hi + mid + lo = value (24 bits), laid out
 // [groups][tiles][3][mt][K] with zero rows behind the last one
-cudaError_t launch_split_parts(const float* x, long long ld, long long group_stride, int rows, int K, int mt, int groups, void* parts, cudaStream_t s);
+cudaError_t launch_split_parts(const float* x, long long ld, long long group_stride, int rows, int K, int mt, int groups, void* parts, int num_sms,
+                               cudaStream_t s);
 
 }  // namespace kb2
