@@ -51,6 +51,9 @@ from . import seqops as ops
 
 # rows up to which kb2_seq_gemm runs its GEMV kernels
 GEMV_ROWS = 8
+# tokens from which a portion runs the delta rule in tiles (prep, rule and read-out at 64 tokens 25 us either way, at 256 59 (tiles) against 80 us,
+# at 16 17 against 13), and tokens from which its attention runs on the tensor cores
+TILE_PORTION, TC_PORTION = 64, 128
 _core = None
 
 
@@ -225,7 +228,7 @@ class WindowLatentAttention:
         self.w_o = d(weights["o"])
         # long prompt portions in bfloat16 with 128 + 64 query / key dims and 128 value dims run the tcgen05 attention core of the MoE
         # prefill models (non-absorbed form: keys and values of the window are up-projected from the cached latents by one GEMM)
-        self.tc_min_portion = 128
+        self.tc_min_portion = TC_PORTION
         self.tc_shape = dtype == torch.bfloat16 and dim == 128 and rot_dim == 64 and vdim == 128 and kv_rank % 64 == 0
         self.w_kv_up = d(torch.cat([weights["uk"], weights["uv"]], 0)) if self.tc_shape else None
 
@@ -307,7 +310,7 @@ class GatedDeltaMixer:
         self.w_o = d(weights["o"])
         # key sizes 32 / 64 / 128 with value sizes that are multiples of 32 keep the state in registers; others in shared memory
         self.register_state_kernel = dim in (32, 64, 128) and vdim % 32 == 0
-        self.tile_min_portion = 64          # prep, rule and read-out at 64 tokens 25 us either way, at 256 59 (tiles) against 80 us, at 16 17 against 13
+        self.tile_min_portion = TILE_PORTION
 
     def register_state(self, pool):
         """(conv tail [slots, C, taps - 1], recurrent state [slots, H, dk, dv]) in a RecurrentStatePool."""
@@ -799,7 +802,7 @@ class MultiMapAttention:
                 raise ValueError(f"{nm}_norm has {w.numel()} weights")
         # long prompt portions in bfloat16 with 128 query / key dims per map and 128 or 256 value dims run the tcgen05 attention core of
         # the MoE prefill models, one call per chunk the portion touches, on keys and values gathered from the pages
-        self.tc_min_portion = 128
+        self.tc_min_portion = TC_PORTION
         # (a sink goes into the core's softmax; pooled blocks are a second pass on the plain kernel, merged by the two log-sum-exps)
         self.tc_shape = dtype == torch.bfloat16 and dim == 128 and vdim in (128, 256) and (self.M == 1 or (self.sink is None and not self.pool))
 

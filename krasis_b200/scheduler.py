@@ -8,6 +8,7 @@ is the generation entry point that plans the steps itself: requests are admitted
 are cut into portions under a per-step token budget, and every running request adds one decoded token to each step.
 Pages (`SequenceKVState` over the model's paged cache) and state slots (`RecurrentStatePool`) go back at `finish` and are reused.
 """
+from bisect import bisect_right
 from collections import deque
 from typing import Dict, List, Optional, Sequence, Tuple
 
@@ -16,7 +17,10 @@ import torch
 from . import seqops as ops
 from .attention import SequenceKVState
 from .graphs import capture
+from .mixers import TC_PORTION, TILE_PORTION
 from .sampling import Sampler, SamplingParams
+
+_KINDS = (TILE_PORTION, TC_PORTION)
 
 
 class Request:
@@ -65,9 +69,9 @@ class Scheduler:
         self.state_pool.free(req.slot)
 
     def step(self, entries: Sequence[Tuple[object, Sequence[int], Sequence[int]]]) -> Optional[torch.Tensor]:
-        """entries: (request id, next tokens, indices among these tokens whose logits are wanted).  All entries run as one batch, the
-        shortest first: portions that run on the same kernels are neighbours whatever order they come in (eight prompt portions and eight
-        decoded tokens in turn 784 us per attention layer, sorted 498).  Returns the wanted logits in entry order (None if nothing is wanted)."""
+        """entries: (request id, next tokens, indices among these tokens whose logits are wanted).  All entries run as one batch.
+        Short portions come first, so that those that run on the same kernels are neighbours (eight prompt portions and eight decoded tokens
+        in turn 784 us per attention layer, sorted 498).  Returns the wanted logits in entry order (None if nothing is wanted)."""
         if not entries:
             return None
         reqs = []
@@ -78,7 +82,7 @@ class Scheduler:
             req.kv.ensure_capacity(len(tokens))
             reqs.append(req)
         packed, first, cu = [], [0] * len(entries), 0
-        for i in sorted(range(len(entries)), key=lambda i: len(entries[i][1])):
+        for i in sorted(range(len(entries)), key=lambda i: bisect_right(_KINDS, len(entries[i][1]))):
             packed.append((entries[i][1], reqs[i].kv.seq_len, reqs[i].slot, reqs[i].kv.pages))
             first[i] = cu
             cu += len(entries[i][1])

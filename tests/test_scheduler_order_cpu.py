@@ -1,4 +1,4 @@
-"""Entries of a step run shortest first, and the logits come back in the order of the entries.  A stand-in for the model, no GPU."""
+"""Short portions of a step run first, and the logits come back in the order of the entries.  A stand-in for the model, no GPU."""
 import torch
 
 from krasis_b200 import scheduler
@@ -38,12 +38,12 @@ def test_mixed_entries(monkeypatch):
     monkeypatch.setattr(scheduler, "SequenceKVState", _Kv)
     m = _Model()
     s = scheduler.Scheduler(m, 1000, 8)
-    m.slot_of = {100: 0, 200: 1, 300: 2, 400: 3, 150: 0, 250: 1, 350: 2, 450: 3, 151: 0}
+    m.slot_of = {1000: 0, 2000: 1, 3000: 2, 4000: 3, 5000: 4, 1500: 0, 2500: 1, 3500: 2, 4500: 3, 1600: 0}
     tok = lambda base, n: list(range(base, base + n))  # noqa: E731
-    out = s.step([("a", tok(100, 9), [8, 0]), ("b", tok(200, 1), [0]), ("c", tok(300, 30), []), ("d", tok(400, 1), [0])])
-    assert m.layouts[-1] == [(1, 0), (1, 0), (9, 0), (30, 0)]
-    assert out.tolist() == [[108, 8], [100, 0], [200, 0], [400, 0]]
-    out = s.step([("c", tok(350, 2), [1]), ("b", tok(250, 1), [0]), ("a", tok(150, 1), [0]), ("d", tok(450, 40), [0, 39])])
-    assert m.layouts[-1] == [(1, 1), (1, 9), (2, 30), (40, 1)]                       # equal lengths keep their order
-    assert out.tolist() == [[351, 31], [250, 1], [150, 9], [450, 1], [489, 40]]
-    assert s.step([("a", [151], [])]) is None
+    out = s.step([("a", tok(1000, 130), [129, 0]), ("b", tok(2000, 1), [0]), ("c", tok(3000, 300), []), ("d", tok(4000, 3), [0]), ("e", tok(5000, 64), [])])
+    assert m.layouts[-1] == [(1, 0), (3, 0), (64, 0), (130, 0), (300, 0)]
+    assert out.tolist() == [[1129, 129], [1000, 0], [2000, 0], [4000, 0]]
+    out = s.step([("c", tok(3500, 127), [1]), ("b", tok(2500, 63), [0]), ("a", tok(1500, 1), [0]), ("d", tok(4500, 128), [0, 39])])
+    assert m.layouts[-1] == [(63, 1), (1, 130), (127, 300), (128, 3)]                 # portions of one kind keep their order
+    assert out.tolist() == [[3501, 301], [2500, 1], [1500, 130], [4500, 3], [4539, 42]]
+    assert s.step([("a", [1600], [])]) is None
