@@ -336,9 +336,8 @@ template <typename TC>
 static bool launch_gemv_mma(const void* A, long long lda, const void* B, long long ldb, void* C, long long ldc, int M, int N, int K,
                             int batch, long long sA, long long sB, long long sC, cudaStream_t s) {
   if (K % 8 || ldb % 8 || sB % 8 || ((uintptr_t)B & 15) || ((uintptr_t)A & 15) || lda % 8 || sA % 8) return false;
-  // a small matrix and one or two rows: a launch's latency, and gemv_nt_vec's is shorter (N 256, K 2048, 1 row 2.2 us against 2.9; at
-  // N 4096, K 512 3.1 against 3.0)
-  if (M <= 2 && (long long)N * K * batch < (1 << 20)) return false;
+  // at any number of rows, so that a row's sums do not depend on the rows beside it; gemv_nt_vec, us at 1 / 2 / 4 / 8 rows and here at any: N 512, K 1024
+  // 2.7 / 3.5 / 5.3 / 9.7, 2.1; N 4096, K 224 2.3 / 2.7 / 3.4 / 5.2, 2.2; N 256, K 2048 2.2 / 2.6 / 3.5 / 5.6, 2.7; N 128, K 8184 3.9 / 5.6 / 9.2 / 17, 6.2
   const int groups = (N + 15) / 16;
   int ks = 1;                                  // about 2048 warps, in one wave of two blocks per SM, as long as each has a piece of K
   while (ks < 16 && (long long)groups * batch * 2 * ks <= 2368 && K > 128 * ks) ks *= 2;
