@@ -6,7 +6,8 @@
 // rows of X (any multiple of 16 up to 256) its N side, which costs no padding to 128 rows — and K is cut over the CTAs of a cluster
 // (1, 2, 4 or 8).  A CTA has one tile: its TMA ring streams the weights while two CTAs share an SM, so that one fills its ring while the
 // other drains.  The partial tiles of a cluster meet in shared memory (one [row][128] fp32 image per CTA, read through distributed shared
-// memory); every output is summed in rank order, so a result does not depend on timing.  From HBM, 77 rows: N 16384, K 2048 15.0 us (11.1 us
+// memory); every output is summed in rank order, so a result does not depend on timing, and the plans (below) keep it from depending on the number
+// of rows.  From HBM, 77 rows: N 16384, K 2048 15.0 us (11.1 us
 // of traffic), N 2048, K 8192 12.6 us (5.4 us), where fp32-FMA tiles took 697 and 449 us.
 //
 // Grouped form: row tile i of X multiplies matrix tile_group[i] (routed experts on binned rows); only the first n_tiles_dev[0] row tiles

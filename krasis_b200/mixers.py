@@ -38,8 +38,8 @@ libkrasis_b200_seq (`krasis_b200.seqops`): a model composes them (krasis_b200/vo
                           experts of any of those forms (binned tile GEMMs; a GEMV form for steps of few tokens) plus an optional shared
                           expert with an optional per-token sigmoid gate; the weight multiplies an expert's output or its input
   TokenSideInput          per-layer token table slice, gated by a projection of the residual stream, RMS-normed
-`lin(a, w, out_dtype)` picks the GEMM: the tcgen05 kernel of the core library for large aligned bf16 products, the generic
-kernel of the sequence library otherwise (any shape, fp32 or bf16).
+`lin(a, w, out_dtype)` picks the product: a GEMV of the sequence library at 8 rows and fewer, the tcgen05 kernels of the core library for aligned
+bf16 operands and for fp32 ones as bf16 parts, the generic kernel of the sequence library otherwise (any shape, fp32 or bf16).
 """
 import math
 import os

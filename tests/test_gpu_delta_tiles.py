@@ -87,7 +87,12 @@ def test_a_sequence_does_not_depend_on_the_step(lens, dtype):
         tail, state = tail0.clone(), state0.clone()
         o = m.forward(rows, ops.StepTables(entries, "cuda"), tail, state)
         return o, tail, state
-    whole, tail, state = run(h, [([0] * n, 9, s, [0]) for s, n in enumerate(lens)])
+    entries = [([0] * n, 9, s, [0]) for s, n in enumerate(lens)]
+    whole, tail, state = run(h, entries)
+    want, states = _exact(m, h, ops.StepTables(entries, "cuda"), tail0, state0, lens, list(range(len(lens))))
+    # fp32: as above; bfloat16: one rounding (2^-9 at most, 2^-9 / sqrt 3 on average) of every head's output ahead of the last product
+    assert (whole.double() - want).norm() <= (1e-6 if dtype == torch.float32 else 2.0 ** -9) * want.norm()
+    assert (state.double() - states).norm() <= 1e-6 * states.norm()
     at = 0
     for s, n in enumerate(lens):
         if dtype == torch.float32 or (n >= 256) == (sum(lens) >= 256):              # bf16 projections take another kernel from 256 rows on
