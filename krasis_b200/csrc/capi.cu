@@ -744,8 +744,7 @@ KB2_API int kb2_last_expert_counts(kb2_engine* e, int32_t* counts_host, void* st
 
 KB2_API int kb2_wait_timeouts(int32_t device, int32_t put, int32_t* up) {
   if (!up) return fail(KB2_ERR_VALUE, "null argument");
-  CUDA_TRY(cudaSetDevice(device));
-  CUDA_TRY(exchange_wait_flags(put, up));
+  CUDA_TRY(exchange_wait_flags(device, put, up));
   return KB2_OK;
 }
 KB2_API int64_t kb2_total_launches(void) { return (int64_t)g_launches.load(); }

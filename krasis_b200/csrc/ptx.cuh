@@ -56,16 +56,21 @@ struct ListWaitFlag {
   }
 } list_wait_flag;
 }  // namespace
-// Sets every flag of this library on the current device to `put` and counts those that were up; waits for the device.
-inline cudaError_t exchange_wait_flags(int put, int* up) {
+// Sets every flag of this library on `device` to `put` and counts those that were up; waits for the device and leaves the current one as it is.
+inline cudaError_t exchange_wait_flags(int device, int put, int* up) {
   *up = 0;
-  cudaError_t e = cudaDeviceSynchronize();
+  int current = 0;
+  cudaError_t e = cudaGetDevice(&current);
+  if (e == cudaSuccess) e = cudaSetDevice(device);
+  if (e != cudaSuccess) return e;
+  e = cudaDeviceSynchronize();
   for (size_t i = 0; i < wait_flags().size() && e == cudaSuccess; ++i) {
     int was = 0;
     e = wait_flags()[i](put, &was);
     *up += was != 0;
   }
-  return e;
+  const cudaError_t back = cudaSetDevice(current);
+  return e != cudaSuccess ? e : back;
 }
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
   if (mbar_try_wait(bar, parity)) return;

@@ -1841,8 +1841,7 @@ extern "C" {
 KB2SEQ_API const char* kb2_seq_last_error(void) { return g_err; }
 KB2SEQ_API int kb2_seq_wait_timeouts(int device, int put, int* up) {
   if (!up) return failf(KB2SEQ_ERR_VALUE, "wait_timeouts: bad argument");
-  SEQ_CUDA(cudaSetDevice(device));
-  SEQ_CUDA(kb2::exchange_wait_flags(put, up));
+  SEQ_CUDA(kb2::exchange_wait_flags(device, put, up));
   return KB2SEQ_OK;
 }
 KB2SEQ_API long long kb2_seq_total_launches(void) { return g_launches; }
