@@ -878,11 +878,13 @@ class MultiMapAttention:
         core = _core_lib() if self.tc_shape else False
         # long portions on the tensor cores, the others on the plain kernel with a key range of their own to cut (beside one portion of 512
         # tokens, three decoded tokens at 2048 keys take 15 us instead of 230 uncut)
-        for fast, seqs, r0, rows in portion_runs(tb, self.tc_min_portion if core else None):
-            self._attend(core if fast else None, proj, a, o, gate, tb, seqs, r0, rows, kc, vc, kp, vp, page_size, s)
+        runs = portion_runs(tb, self.tc_min_portion if core else None)
+        lse = torch.empty((T, H), dtype=torch.float32, device=h.device) if self.pool and any(run[0] for run in runs) else None
+        for fast, seqs, r0, rows in runs:
+            self._attend(core if fast else None, proj, a, o, gate, tb, seqs, r0, rows, kc, vc, kp, vp, page_size, s, lse)
         return lin(o, self.w_o, torch.float32)
 
-    def _attend(self, core, proj, a, o, gate, tb, seqs, r0, T, kc, vc, kp, vp, page_size, s):
+    def _attend(self, core, proj, a, o, gate, tb, seqs, r0, T, kc, vc, kp, vp, page_size, s, lse):
         """Rows r0 .. r0 + T - 1 of the step (the sequences `seqs`): attention into a, the finished heads into o.  core: the library whose
         tensor-core attention runs these portions, None for the plain kernel."""
         lib, H, G, M, dtc, dev = ops.load(), self.H, self.G, self.M, ops.dt_code(kc.dtype), proj.device
@@ -907,7 +909,6 @@ class MultiMapAttention:
                 part_ml = torch.empty((T * H * M, nsplit, 2), dtype=torch.float32, device=dev)
             plain(_row(a, r0), part_acc, part_ml, False)
         else:
-            lse = torch.empty((proj.shape[0], H), dtype=torch.float32, device=dev) if self.pool else None
             for q in seqs:
                 self._tensor_core_portion(core, proj, a, tb, q, kc, vc, page_size, s, lse=lse)
             if self.pool:                            # the pooled blocks of the long portions: a second pass, joined by the log-sum-exps
