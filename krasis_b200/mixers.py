@@ -144,7 +144,8 @@ def _row(t, r: int):
 
 def portion_runs(tb, min_long):
     """The step's rows as runs of neighbouring sequences of one kind: [(long, sequences, first row, rows)], long where every portion of the
-    run has at least min_long tokens (None: no portion counts as long)."""
+    run has at least min_long tokens (None: no portion counts as long).  Every run has launches of its own, so whoever builds a step keeps
+    portions of one kind together, as Scheduler.step does."""
     if tb.S == 1:
         n = tb.layout[0][1]
         return [(min_long is not None and n >= min_long, range(1), 0, n)] if n else []
