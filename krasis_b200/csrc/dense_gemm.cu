@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(kDThreads, 1)
                       const float* __restrict__ row_scale, const __nv_bfloat16* __restrict__ col_scale, CombineScatter sc,
                       // grouped form (routed experts on binned rows): W holds `groups` matrices of N rows one after the other, row tile i
                       // (128 rows of X) multiplies matrix tile_group[i], and only the first m_tiles_dev[0] row tiles exist
-                      const int* __restrict__ tile_group = nullptr, const int* __restrict__ m_tiles_dev = nullptr) {
+                      const int* __restrict__ tile_group, const int* __restrict__ m_tiles_dev) {
   constexpr bool kOutF32 = MODE == 1;
   constexpr int kElemsPerBlock = MODE == 2 ? 128 : 64;     // 128 B of K per smem row
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -45,10 +45,6 @@ __global__ void __launch_bounds__(kDThreads, 1)
   // warp index through a shuffle so that the role branches are provably warp-uniform: tcgen05.mma issued from a divergent single-thread branch
   // cost about 50 cycles more each (profiles/r02h_mma_uniform_ubench.txt)
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int n_tiles = (N + kDTileN - 1) / kDTileN, m_tiles_max = (M + kDTileM - 1) / kDTileM;
-  const int m_tiles = m_tiles_dev != nullptr ? min(m_tiles_max, m_tiles_dev[0]) : m_tiles_max;
-  const int total = n_tiles * m_tiles;
-  const int nkb = K / kElemsPerBlock;
 
   if (threadIdx.x == 32) {
     if (smem_u32(smem) & 1023u) __trap();
@@ -71,6 +67,11 @@ __global__ void __launch_bounds__(kDThreads, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_enter(out, bias, row_scale, col_scale, tile_group, m_tiles_dev);
+  const int n_tiles = (N + kDTileN - 1) / kDTileN, m_tiles_max = (M + kDTileM - 1) / kDTileM;
+  const int m_tiles = m_tiles_dev != nullptr ? min(m_tiles_max, m_tiles_dev[0]) : m_tiles_max;
+  const int total = n_tiles * m_tiles;
+  const int nkb = K / kElemsPerBlock;
 
   if (warp == 0) {
     {
@@ -239,9 +240,9 @@ cudaError_t launch_dense_gemm_scatter(const void* x, const void* w, void* out, c
   const int total = ((M + kDTileM - 1) / kDTileM) * ((N + kDTileN - 1) / kDTileN);
   const int grid = total < num_sms ? total : num_sms;
   if (out_f32)
-    dense_gemm_kernel<1><<<grid, kDThreads, kDSmem, s>>>(tx, tw, out, bias, M, N, K, ldo, nullptr, nullptr, CombineScatter{});
+    launch_pdl(dense_gemm_kernel<1>, grid, kDThreads, kDSmem, s, tx, tw, out, bias, M, N, K, ldo, nullptr, nullptr, CombineScatter{}, nullptr, nullptr);
   else
-    dense_gemm_kernel<0><<<grid, kDThreads, kDSmem, s>>>(tx, tw, out, bias, M, N, K, ldo, nullptr, nullptr, sc);
+    launch_pdl(dense_gemm_kernel<0>, grid, kDThreads, kDSmem, s, tx, tw, out, bias, M, N, K, ldo, nullptr, nullptr, sc, nullptr, nullptr);
   return cudaGetLastError();
 }
 
@@ -260,10 +261,10 @@ cudaError_t launch_dense_gemm_grouped(const void* x, const void* w, void* out, i
   const int total = ((M + kDTileM - 1) / kDTileM) * ((N + kDTileN - 1) / kDTileN);
   const int grid = total < num_sms ? total : num_sms;
   if (out_f32)
-    dense_gemm_kernel<1><<<grid, kDThreads, kDSmem, s>>>(tx, tw, out, nullptr, M, N, K, ldo, nullptr, nullptr, CombineScatter{}, tile_group,
+    launch_pdl(dense_gemm_kernel<1>, grid, kDThreads, kDSmem, s, tx, tw, out, nullptr, M, N, K, ldo, nullptr, nullptr, CombineScatter{}, tile_group,
                                                         m_tiles_dev);
   else
-    dense_gemm_kernel<0><<<grid, kDThreads, kDSmem, s>>>(tx, tw, out, nullptr, M, N, K, ldo, nullptr, nullptr, CombineScatter{}, tile_group,
+    launch_pdl(dense_gemm_kernel<0>, grid, kDThreads, kDSmem, s, tx, tw, out, nullptr, M, N, K, ldo, nullptr, nullptr, CombineScatter{}, tile_group,
                                                         m_tiles_dev);
   return cudaGetLastError();
 }
@@ -282,8 +283,8 @@ cudaError_t launch_dense_gemm_i8(const void* xq, const float* x_scale, const voi
   if (e != cudaSuccess) return e;
   const int total = ((M + kDTileM - 1) / kDTileM) * ((N + kDTileN - 1) / kDTileN);
   const int grid = total < num_sms ? total : num_sms;
-  dense_gemm_kernel<2><<<grid, kDThreads, kDSmem, s>>>(tx, tw, out, nullptr, M, N, K, ldo, x_scale,
-                                                      (const __nv_bfloat16*)w_scale, CombineScatter{});
+  launch_pdl(dense_gemm_kernel<2>, grid, kDThreads, kDSmem, s, tx, tw, out, nullptr, M, N, K, ldo, x_scale,
+                                                      (const __nv_bfloat16*)w_scale, CombineScatter{}, nullptr, nullptr);
   return cudaGetLastError();
 }
 

@@ -52,8 +52,9 @@ __device__ __forceinline__ int quant_code_rhe(float x, float scale, float rscale
 template <bool kAdd, int VPL, bool kQuant = false>
 __global__ void __launch_bounds__(256) rmsnorm_warp_kernel(__nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ residual,
                                                            const float* __restrict__ w, __nv_bfloat16* __restrict__ out,
-                                                           int M, float eps, int8_t* __restrict__ q_out = nullptr,
-                                                           float* __restrict__ q_scale = nullptr) {
+                                                           int M, float eps, int8_t* __restrict__ q_out,
+                                                           float* __restrict__ q_scale) {
+  pdl_enter(x, residual, w, out, q_out, q_scale);
   constexpr int H = 256 * VPL;
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -128,6 +129,7 @@ template <bool kAdd>
 __global__ void __launch_bounds__(256) rmsnorm_kernel(__nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ residual,
                                                       const float* __restrict__ w, __nv_bfloat16* __restrict__ out,
                                                       int H, float eps) {
+  pdl_enter(x, residual, w, out);
   __shared__ float red[8];
   extern __shared__ float xs[];    // [H] fp32 copy of the (summed) row
   const long long row = blockIdx.x;
@@ -171,6 +173,7 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(__nv_bfloat16* __restrict_
 __global__ void __launch_bounds__(256) quant_rows_int8_kernel(const __nv_bfloat16* __restrict__ x, int8_t* __restrict__ q,
                                                               float* __restrict__ scale_f32,
                                                               __nv_bfloat16* __restrict__ scale_bf16, int rows, int K) {
+  pdl_enter(x, q, scale_f32, scale_bf16);
   // one warp per row, 16-byte loads, 8-byte stores (K % 8 == 0); same arithmetic as the scalar form: max is order-free,
   // x / scale is an IEEE division, rintf = round half to even
   const int lane = threadIdx.x & 31;
@@ -206,6 +209,7 @@ __global__ void __launch_bounds__(256) quant_rows_int8_kernel(const __nv_bfloat1
 
 __global__ void __launch_bounds__(256) silu_and_mul_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ out,
                                                            long long rows, int N) {
+  pdl_enter(x, out);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= rows * (N / 8)) return;
   const long long r = idx / (N / 8);
@@ -229,6 +233,7 @@ __global__ void __launch_bounds__(256) silu_and_mul_kernel(const __nv_bfloat16* 
 template <int VPL>
 __global__ void __launch_bounds__(256) silu_mul_quant_kernel(const __nv_bfloat16* __restrict__ x, int8_t* __restrict__ q,
                                                              float* __restrict__ scale_f32, int rows) {
+  pdl_enter(x, q, scale_f32);
   constexpr int N = 256 * VPL;
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -270,6 +275,7 @@ __global__ void __launch_bounds__(256) silu_mul_quant_kernel(const __nv_bfloat16
 __global__ void __launch_bounds__(256) sigmoid_gate_mul_kernel(const __nv_bfloat16* __restrict__ h,
                                                                const __nv_bfloat16* __restrict__ w,
                                                                __nv_bfloat16* __restrict__ y, int M, int H, int N) {
+  pdl_enter(h, w, y);
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (row >= M) return;
@@ -296,6 +302,7 @@ __global__ void __launch_bounds__(256) sigmoid_gate_mul_kernel(const __nv_bfloat
 
 __global__ void add_bf16_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
                                 __nv_bfloat16* __restrict__ out, long long n8) {
+  pdl_enter(a, b, out);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n8) return;
   const uint4 x = reinterpret_cast<const uint4*>(a)[i], y = reinterpret_cast<const uint4*>(b)[i];
@@ -310,7 +317,7 @@ __global__ void add_bf16_kernel(const __nv_bfloat16* __restrict__ a, const __nv_
 cudaError_t launch_add_bf16(const void* a, const void* b, void* out, long long n, cudaStream_t s) {
   KernelSpan ks(K_ADD, s);
   if (n % 8 || n <= 0) return cudaErrorInvalidValue;
-  add_bf16_kernel<<<(unsigned)((n / 8 + 255) / 256), 256, 0, s>>>((const __nv_bfloat16*)a, (const __nv_bfloat16*)b,
+  launch_pdl(add_bf16_kernel, (unsigned)((n / 8 + 255) / 256), 256, 0, s, (const __nv_bfloat16*)a, (const __nv_bfloat16*)b,
                                                                  (__nv_bfloat16*)out, n / 8);
   return cudaGetLastError();
 }
@@ -320,15 +327,17 @@ cudaError_t launch_rmsnorm(void* x, void* residual, const float* w, void* out, i
   if (H % 8 || M <= 0) return cudaErrorInvalidValue;
   if (H == 2048) {
     if (residual)
-      rmsnorm_warp_kernel<true, 8><<<(M + 7) / 8, 256, 0, s>>>((__nv_bfloat16*)x, (__nv_bfloat16*)residual, w, (__nv_bfloat16*)out, M, eps);
+      launch_pdl(rmsnorm_warp_kernel<true, 8>, (M + 7) / 8, 256, 0, s, (__nv_bfloat16*)x, (__nv_bfloat16*)residual, w, (__nv_bfloat16*)out, M, eps,
+                 nullptr, nullptr);
     else
-      rmsnorm_warp_kernel<false, 8><<<(M + 7) / 8, 256, 0, s>>>((__nv_bfloat16*)x, nullptr, w, (__nv_bfloat16*)out, M, eps);
+      launch_pdl(rmsnorm_warp_kernel<false, 8>, (M + 7) / 8, 256, 0, s, (__nv_bfloat16*)x, nullptr, w, (__nv_bfloat16*)out, M, eps, nullptr,
+                 nullptr);
     return cudaGetLastError();
   }
   if (residual)
-    rmsnorm_kernel<true><<<M, 256, H * sizeof(float), s>>>((__nv_bfloat16*)x, (__nv_bfloat16*)residual, w, (__nv_bfloat16*)out, H, eps);
+    launch_pdl(rmsnorm_kernel<true>, M, 256, H * sizeof(float), s, (__nv_bfloat16*)x, (__nv_bfloat16*)residual, w, (__nv_bfloat16*)out, H, eps);
   else
-    rmsnorm_kernel<false><<<M, 256, H * sizeof(float), s>>>((__nv_bfloat16*)x, nullptr, w, (__nv_bfloat16*)out, H, eps);
+    launch_pdl(rmsnorm_kernel<false>, M, 256, H * sizeof(float), s, (__nv_bfloat16*)x, nullptr, w, (__nv_bfloat16*)out, H, eps);
   return cudaGetLastError();
 }
 // rmsnorm (+ residual add) that also emits the INT8 row quantisation of its output; false = geometry not covered by the fused kernel
@@ -338,10 +347,10 @@ cudaError_t launch_rmsnorm_q8(void* x, void* residual, const float* w, void* out
   KernelSpan ks(K_RMSNORM, s);
   if (!rmsnorm_q8_supported(H) || M <= 0) return cudaErrorInvalidValue;
   if (residual)
-    rmsnorm_warp_kernel<true, 8, true><<<(M + 7) / 8, 256, 0, s>>>((__nv_bfloat16*)x, (__nv_bfloat16*)residual, w, (__nv_bfloat16*)out, M,
+    launch_pdl(rmsnorm_warp_kernel<true, 8, true>, (M + 7) / 8, 256, 0, s, (__nv_bfloat16*)x, (__nv_bfloat16*)residual, w, (__nv_bfloat16*)out, M,
                                                                    eps, (int8_t*)q, q_scale);
   else
-    rmsnorm_warp_kernel<false, 8, true><<<(M + 7) / 8, 256, 0, s>>>((__nv_bfloat16*)x, nullptr, w, (__nv_bfloat16*)out, M, eps, (int8_t*)q,
+    launch_pdl(rmsnorm_warp_kernel<false, 8, true>, (M + 7) / 8, 256, 0, s, (__nv_bfloat16*)x, nullptr, w, (__nv_bfloat16*)out, M, eps, (int8_t*)q,
                                                                     q_scale);
   return cudaGetLastError();
 }
@@ -351,17 +360,17 @@ cudaError_t launch_silu_mul_quant(const void* x, void* q, float* scale_f32, int 
   if (rows <= 0) return cudaErrorInvalidValue;
   const unsigned grid = (unsigned)((rows + 7) / 8);
   const __nv_bfloat16* xb = (const __nv_bfloat16*)x;
-  if (N == 256) silu_mul_quant_kernel<1><<<grid, 256, 0, s>>>(xb, (int8_t*)q, scale_f32, rows);
-  else if (N == 512) silu_mul_quant_kernel<2><<<grid, 256, 0, s>>>(xb, (int8_t*)q, scale_f32, rows);
-  else if (N == 1024) silu_mul_quant_kernel<4><<<grid, 256, 0, s>>>(xb, (int8_t*)q, scale_f32, rows);
-  else if (N == 2048) silu_mul_quant_kernel<8><<<grid, 256, 0, s>>>(xb, (int8_t*)q, scale_f32, rows);
+  if (N == 256) launch_pdl(silu_mul_quant_kernel<1>, grid, 256, 0, s, xb, (int8_t*)q, scale_f32, rows);
+  else if (N == 512) launch_pdl(silu_mul_quant_kernel<2>, grid, 256, 0, s, xb, (int8_t*)q, scale_f32, rows);
+  else if (N == 1024) launch_pdl(silu_mul_quant_kernel<4>, grid, 256, 0, s, xb, (int8_t*)q, scale_f32, rows);
+  else if (N == 2048) launch_pdl(silu_mul_quant_kernel<8>, grid, 256, 0, s, xb, (int8_t*)q, scale_f32, rows);
   else return cudaErrorInvalidValue;
   return cudaGetLastError();
 }
 cudaError_t launch_quant_rows_int8(const void* x, void* q, float* scale_f32, void* scale_bf16, int rows, int K, cudaStream_t s) {
   KernelSpan ks(K_QUANT_ROWS, s);
   if (rows <= 0 || K % 8) return cudaErrorInvalidValue;
-  quant_rows_int8_kernel<<<(rows + 7) / 8, 256, 0, s>>>((const __nv_bfloat16*)x, (int8_t*)q, scale_f32, (__nv_bfloat16*)scale_bf16,
+  launch_pdl(quant_rows_int8_kernel, (rows + 7) / 8, 256, 0, s, (const __nv_bfloat16*)x, (int8_t*)q, scale_f32, (__nv_bfloat16*)scale_bf16,
                                                         rows, K);
   return cudaGetLastError();
 }
@@ -369,13 +378,13 @@ cudaError_t launch_silu_and_mul(const void* x, void* out, int rows, int N, cudaS
   KernelSpan ks(K_SILU_MUL, s);
   if (N % 8 || rows <= 0) return cudaErrorInvalidValue;
   const long long total = (long long)rows * (N / 8);
-  silu_and_mul_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)out, rows, N);
+  launch_pdl(silu_and_mul_kernel, (unsigned)((total + 255) / 256), 256, 0, s, (const __nv_bfloat16*)x, (__nv_bfloat16*)out, rows, N);
   return cudaGetLastError();
 }
 cudaError_t launch_sigmoid_gate_mul(const void* h, const void* w, void* y, int M, int H, int N, cudaStream_t s) {
   KernelSpan ks(K_SIGMOID_GATE, s);
   if (M <= 0 || H % 8 || N % 8) return cudaErrorInvalidValue;
-  sigmoid_gate_mul_kernel<<<(M + 7) / 8, 256, 0, s>>>((const __nv_bfloat16*)h, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, M, H, N);
+  launch_pdl(sigmoid_gate_mul_kernel, (M + 7) / 8, 256, 0, s, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, M, H, N);
   return cudaGetLastError();
 }
 

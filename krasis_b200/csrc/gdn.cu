@@ -52,6 +52,7 @@ __global__ void __launch_bounds__(256) gdn_prep_kernel(GdnDims d, const __nv_bfl
                                                        __nv_bfloat16* __restrict__ qn, __nv_bfloat16* __restrict__ kn,
                                                        __nv_bfloat16* __restrict__ vc, float* __restrict__ beta,
                                                        float* __restrict__ g, int M) {
+  pdl_enter(qkvz, ba, conv_w, conv_state, A_log, dt_bias, qn, kn, vc, beta, g);
   extern __shared__ float s_conv[];   // [C]
   const int t = blockIdx.x;
   const int kd = d.nk * d.dk, vd = d.nv * d.dv, C = 2 * kd + vd;
@@ -115,6 +116,7 @@ __global__ void __launch_bounds__(256) gdn_prep_tiled_kernel(GdnDims d, const __
                                                              __nv_bfloat16* __restrict__ qn, __nv_bfloat16* __restrict__ kn,
                                                              __nv_bfloat16* __restrict__ vc, float* __restrict__ beta,
                                                              float* __restrict__ g, int M, int n_tiles) {
+  pdl_enter(qkvz, ba, conv_w, conv_state, A_log, dt_bias, qn, kn, vc, beta, g);
   constexpr int TT = 32;
   const int lane = threadIdx.x & 31;
   const long long wg = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -206,6 +208,7 @@ __global__ void __launch_bounds__(256) gdn_prep_vec_kernel(GdnDims d, const __nv
                                                            __nv_bfloat16* __restrict__ qn, __nv_bfloat16* __restrict__ kn,
                                                            __nv_bfloat16* __restrict__ vc, float* __restrict__ beta,
                                                            float* __restrict__ g, int M, int n_tiles) {
+  pdl_enter(qkvz, ba, conv_w, conv_state, A_log, dt_bias, qn, kn, vc, beta, g);
   constexpr int KW = 4;
   const int lane = threadIdx.x & 31;
   const long long wg = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -316,6 +319,7 @@ __global__ void __launch_bounds__(256) gdn_prep_vec_kernel(GdnDims d, const __nv
 // new conv state = last K pre-conv inputs (older entries come from the previous state when M < K)
 __global__ void gdn_conv_state_kernel(GdnDims d, const __nv_bfloat16* __restrict__ qkvz,
                                       __nv_bfloat16* __restrict__ conv_state, int M) {
+  pdl_enter(qkvz, conv_state);
   const int kd = d.nk * d.dk, vd = d.nv * d.dv, C = 2 * kd + vd, ld = 2 * kd + 2 * vd;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
@@ -366,6 +370,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prepare_kernel(GdnDims d, co
                                                                    float* __restrict__ vcorr, float* __restrict__ kcd,
                                                                    float* __restrict__ intra,
                                                                    float* __restrict__ gcum_out) {
+  pdl_enter(qn, kn, vc, beta, g, vcorr, kcd, intra, gcum_out);
   extern __shared__ __align__(16) unsigned char smraw[];
   const int ch = blockIdx.x, h = blockIdx.y, r = d.nv / d.nk, kh = h / r;
   const int dk = d.dk, dv = d.dv, kd = d.nk * dk, vd = d.nv * dv;
@@ -581,6 +586,7 @@ __global__ void __launch_bounds__(256, 1) gdn_chunk_scan_kernel(GdnDims d, const
                                                                 const float* __restrict__ gcum, int M, int n_chunks,
                                                                 float* __restrict__ state,       // [nv][dk][dv] in/out
                                                                 __nv_bfloat16* __restrict__ core_out) {  // [M][nv][dv] (core_attn_out.to(bf16))
+  pdl_enter(qn, kn, vcorr, kcd, intra, gcum, state, core_out);
   extern __shared__ __align__(16) unsigned char smraw[];
   const int h = blockIdx.x, sl = blockIdx.y, r = d.nv / d.nk, kh = h / r;
   const int dk = d.dk, dv = d.dv, kd = d.nk * dk, vd = d.nv * dv;
@@ -750,6 +756,7 @@ __global__ void __launch_bounds__(256) gdn_post128_kernel(GdnDims d, const __nv_
                                                           const __nv_bfloat16* __restrict__ qkvz,
                                                           const float* __restrict__ norm_w, int M,
                                                           __nv_bfloat16* __restrict__ out) {   // [M][nv*128]
+  pdl_enter(core, qkvz, norm_w, out);
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31, groups = d.nv / HP;
   if (wid >= (long long)M * groups) return;
@@ -792,6 +799,7 @@ __global__ void __launch_bounds__(256) gdn_post_kernel(GdnDims d, const __nv_bfl
                                                        const __nv_bfloat16* __restrict__ qkvz,
                                                        const float* __restrict__ norm_w, int M,
                                                        __nv_bfloat16* __restrict__ out) {   // [M][nv*dv]
+  pdl_enter(core, qkvz, norm_w, out);
   const int wid = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (wid >= M * d.nv) return;
   const int t = wid / d.nv, h = wid % d.nv, r = d.nv / d.nk;
@@ -831,12 +839,12 @@ static void launch_gdn_post(const GdnDims& d, const void* core, const void* qkvz
                             cudaStream_t s) {
   if (d.dv == 128 && d.nv % 4 == 0) {
     const long long nw = (long long)M * (d.nv / 4);
-    gdn_post128_kernel<4><<<(unsigned)((nw * 32 + 255) / 256), 256, 0, s>>>(d, (const __nv_bfloat16*)core, (const __nv_bfloat16*)qkvz,
+    launch_pdl(gdn_post128_kernel<4>, (unsigned)((nw * 32 + 255) / 256), 256, 0, s, d, (const __nv_bfloat16*)core, (const __nv_bfloat16*)qkvz,
                                                                            norm_w, M, (__nv_bfloat16*)out);
     return;
   }
   const long long nw = (long long)M * d.nv;
-  gdn_post_kernel<<<(unsigned)((nw * 32 + 255) / 256), 256, 0, s>>>(d, (const __nv_bfloat16*)core, (const __nv_bfloat16*)qkvz, norm_w, M,
+  launch_pdl(gdn_post_kernel, (unsigned)((nw * 32 + 255) / 256), 256, 0, s, d, (const __nv_bfloat16*)core, (const __nv_bfloat16*)qkvz, norm_w, M,
                                                                   (__nv_bfloat16*)out);
 }
 
@@ -887,7 +895,7 @@ cudaError_t launch_gdn_core(const GdnDims& d, const void* qkvz, const void* ba, 
       constexpr int TT = decltype(tt)::value;
       const int n_tiles = (M + TT - 1) / TT;
       const long long warps = (long long)n_tiles * (2 * d.nk + d.nv + TT / kGdnGateRows);
-      gdn_prep_vec_kernel<TT><<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(
+      launch_pdl(gdn_prep_vec_kernel<TT>, (unsigned)((warps + 7) / 8), 256, 0, s,
           d, (const __nv_bfloat16*)qkvz, (const __nv_bfloat16*)ba, (const __nv_bfloat16*)conv_w,
           (const __nv_bfloat16*)conv_state, A_log, dt_bias, (__nv_bfloat16*)qn, (__nv_bfloat16*)kn, (__nv_bfloat16*)vc, beta, g,
           M, n_tiles);
@@ -900,23 +908,23 @@ cudaError_t launch_gdn_core(const GdnDims& d, const void* qkvz, const void* ba, 
   } else if (d.dk == 128 && d.dv == 128 && d.K == 4) {
     const int n_tiles = (M + 31) / 32;
     const long long warps = (long long)n_tiles * (2 * d.nk + d.nv + 1);
-    gdn_prep_tiled_kernel<4, 4><<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(
+    launch_pdl(gdn_prep_tiled_kernel<4, 4>, (unsigned)((warps + 7) / 8), 256, 0, s,
         d, (const __nv_bfloat16*)qkvz, (const __nv_bfloat16*)ba, (const __nv_bfloat16*)conv_w,
         (const __nv_bfloat16*)conv_state, A_log, dt_bias, (__nv_bfloat16*)qn, (__nv_bfloat16*)kn, (__nv_bfloat16*)vc, beta, g,
         M, n_tiles);
   } else {
-    gdn_prep_kernel<<<M, 256, sizeof(float) * C, s>>>(d, (const __nv_bfloat16*)qkvz, (const __nv_bfloat16*)ba,
+    launch_pdl(gdn_prep_kernel, M, 256, sizeof(float) * C, s, d, (const __nv_bfloat16*)qkvz, (const __nv_bfloat16*)ba,
                                                       (const __nv_bfloat16*)conv_w, (const __nv_bfloat16*)conv_state, A_log,
                                                       dt_bias, (__nv_bfloat16*)qn, (__nv_bfloat16*)kn, (__nv_bfloat16*)vc,
                                                       beta, g, M);
   } }
   { KernelSpan ks(K_GDN_CONV_STATE, s);
-  gdn_conv_state_kernel<<<(C + 255) / 256, 256, 0, s>>>(d, (const __nv_bfloat16*)qkvz, (__nv_bfloat16*)conv_state, M); }
+  launch_pdl(gdn_conv_state_kernel, (C + 255) / 256, 256, 0, s, d, (const __nv_bfloat16*)qkvz, (__nv_bfloat16*)conv_state, M); }
   const long long nw = (long long)M * d.nv;
   if (gdn_use_tc(d)) {
     { KernelSpan ks(K_GDN_PREPARE, s);
     if (gdn_prepare_mma_sync_env()) {
-      gdn_chunk_prepare_kernel<true><<<dim3(n_chunks, d.nv), 256, gdn_prepare_smem(d), s>>>(
+      launch_pdl(gdn_chunk_prepare_kernel<true>, dim3(n_chunks, d.nv), 256, gdn_prepare_smem(d), s,
           d, (const __nv_bfloat16*)qn, (const __nv_bfloat16*)kn, (const __nv_bfloat16*)vc, beta, g, M, n_chunks, vcorr, kcd,
           intra, gcum);
     } else {
@@ -932,13 +940,13 @@ cudaError_t launch_gdn_core(const GdnDims& d, const void* qkvz, const void* ba, 
     return cudaGetLastError();
   }
   { KernelSpan ks(K_GDN_PREPARE, s);
-  gdn_chunk_prepare_kernel<false><<<dim3(n_chunks, d.nv), 256, gdn_prepare_smem(d), s>>>(
+  launch_pdl(gdn_chunk_prepare_kernel<false>, dim3(n_chunks, d.nv), 256, gdn_prepare_smem(d), s,
       d, (const __nv_bfloat16*)qn, (const __nv_bfloat16*)kn, (const __nv_bfloat16*)vc, beta, g, M, n_chunks, vcorr, kcd,
       intra, gcum); }
   // slice width: keep >= ~128 CTAs in flight (one per SM) when a rank holds only a few heads
   const int sv = d.nv * (d.dv / 32) >= 96 ? 32 : (d.nv * (d.dv / 16) >= 96 ? 16 : 8);
 #define KB2_SCAN(SV)                                                                                                  \
-  gdn_chunk_scan_kernel<SV><<<dim3(d.nv, d.dv / SV), 256, gdn_scan_smem(d), s>>>(                                      \
+  launch_pdl(gdn_chunk_scan_kernel<SV>, dim3(d.nv, d.dv / SV), 256, gdn_scan_smem(d), s,                                       \
       d, (const __nv_bfloat16*)qn, (const __nv_bfloat16*)kn, vcorr, kcd, intra, gcum, M, n_chunks, rec_state,       \
       (__nv_bfloat16*)core)
   { KernelSpan ks(K_GDN_SCAN, s);

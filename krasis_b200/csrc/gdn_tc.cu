@@ -171,6 +171,7 @@ __global__ void __launch_bounds__(kT3Threads, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_wait();
   constexpr uint32_t kColD1 = 0, kColD1b = 64, kColD2 = 96, kColD3 = 160;     // D1, D2, D3: 64 columns (hi-part | lo-part)
   const bool tracing = p.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0;
   auto stamp = [&](int c, int slot) {
@@ -527,6 +528,7 @@ __global__ void __launch_bounds__(kT3Threads, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_wait();
   constexpr uint32_t kColA = 0, kColB = 128, kColC = 256;
   const bool tracing = p.trace != nullptr && blockIdx.x == 0;
   auto stamp = [&](int it, int slot) {
@@ -884,7 +886,7 @@ cudaError_t launch_gdn_prepare_tc(const void* qn, const void* kn, const void* vc
   long long* trace = trv ? reinterpret_cast<long long*>(strtoull(trv, nullptr, 0)) : nullptr;
   GdnPrepParams p{trace, beta, g, (uint8_t*)kcd_img, (uint8_t*)intra_img, vcorr, gcum, M, n_chunks, nv, nk};
   const int n_units = nv * n_chunks;
-  gdn_prepare_tc_kernel<<<n_units < num_sms ? n_units : num_sms, kT3Threads, kP2Smem, s>>>(tq, tk, tv, p);
+  launch_pdl(gdn_prepare_tc_kernel, n_units < num_sms ? n_units : num_sms, kT3Threads, kP2Smem, s, tq, tk, tv, p);
   return cudaGetLastError();
 }
 
@@ -907,7 +909,7 @@ cudaError_t launch_gdn_scan_tc(const void* qn, const void* kn, const void* kcd_i
   e = make_tmap_bf16_rows(&tk, kn, M, (long long)nk * kTD, kTC);
   if (e != cudaSuccess) return e;
   GdnTcParams p{(const uint8_t*)kcd_img, (const uint8_t*)intra_img, vcorr, gcum, state, (__nv_bfloat16*)core_out, M, n_chunks, nv, nk, trace};
-  gdn_scan_tc_kernel<<<dim3(nv, kTD / kTSV), kT3Threads, kTcSmem, s>>>(tq, tk, p);
+  launch_pdl(gdn_scan_tc_kernel, dim3(nv, kTD / kTSV), kT3Threads, kTcSmem, s, tq, tk, p);
   return cudaGetLastError();
 }
 

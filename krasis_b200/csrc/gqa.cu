@@ -45,6 +45,7 @@ __global__ void __launch_bounds__(256) gqa_prep_kernel(GqaDims g, const __nv_bfl
                                                        __nv_bfloat16* __restrict__ q_out,                    // [M][nh*d]
                                                        uint8_t* __restrict__ k_cache, uint8_t* __restrict__ v_cache,  // [P][16][nkv][d] fp8
                                                        int M) {
+  pdl_enter(q_raw, k_raw, v_raw, q_norm, k_norm, positions, kv_indices, q_out, k_cache, v_cache);
   const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int d = g.d, d2 = g.rotary_dim / 2;
   const int pos = positions[t];
@@ -180,17 +181,17 @@ __global__ void __launch_bounds__(kFThreads, 1)
                     const __nv_bfloat16* __restrict__ q_raw,     // for the output gate (g.gated)
                     __nv_bfloat16* __restrict__ out,             // [M][nh*DV]
                     int M, int q_start, int kv_len, float sm_scale_log2, int k_col0, int v_col0,
-                    int window = 1 << 30,                        // a query sees the keys with 0 <= q_pos - key < window
-                    const float* __restrict__ sinks = nullptr,   // per head: exp(sink) joins the softmax denominator (no value)
-                    int maps = 1,                                // query heads come in groups of `maps` attention maps: map m of a head reads
+                    int window,                        // a query sees the keys with 0 <= q_pos - key < window
+                    const float* __restrict__ sinks,   // per head: exp(sink) joins the softmax denominator (no value)
+                    int maps,                                // query heads come in groups of `maps` attention maps: map m of a head reads
                                                                  // key head kvh * maps + m, every map reads value head kvh
-                    float* __restrict__ out_f32 = nullptr,       // if given, the output rows are written here in fp32 (no gate), not to `out`
-                    float cap_in = 0.f, float cap_out = 0.f,     // soft cap: a raw score s becomes cap_out * tanh(s * cap_in) with
+                    float* __restrict__ out_f32,       // if given, the output rows are written here in fp32 (no gate), not to `out`
+                    float cap_in, float cap_out,     // soft cap: a raw score s becomes cap_out * tanh(s * cap_in) with
                                                                  // cap_in = sm_scale / cap, cap_out = cap / sm_scale (0: no cap)
-                    float* __restrict__ lse_out = nullptr,       // if given, [M][nh]: log(sum of exp(scaled scores)) of every row (the sink
+                    float* __restrict__ lse_out,       // if given, [M][nh]: log(sum of exp(scaled scores)) of every row (the sink
                                                                  // included), so that a caller can merge further keys into the softmax
-                    const float* __restrict__ slopes = nullptr,  // if given, [nh]: slopes[head] * (q_pos - key) is taken off the scaled score
-                    const float* __restrict__ head_gate = nullptr, long long ldg = 0) {   // if given, [M][ldg]: head h's output rows are
+                    const float* __restrict__ slopes,  // if given, [nh]: slopes[head] * (q_pos - key) is taken off the scaled score
+                    const float* __restrict__ head_gate, long long ldg) {   // if given, [M][ldg]: head h's output rows are
                                                                  // multiplied by sigmoid(head_gate[row][h])
   using L = FmhaSmem<DQ, DV>;
   constexpr int D = DQ;
@@ -246,6 +247,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_enter(q_raw, out, sinks, out_f32, lse_out, slopes, head_gate);
   constexpr uint32_t kColS = 0, kColP = 64, kColO = 128;      // P: two buffers of 32 columns at 64 and 96
 
   if (warp < 4) {
@@ -542,6 +544,7 @@ __device__ __forceinline__ void fp8x16_to_bf16(const uint4& q, uint4& lo, uint4&
 __global__ void __launch_bounds__(256) gqa_gather_kernel(const uint8_t* __restrict__ k_cache, const uint8_t* __restrict__ v_cache,
                                                          const int* __restrict__ kv_indices, int row_bytes, int T,
                                                          __nv_bfloat16* __restrict__ k_out, __nv_bfloat16* __restrict__ v_out) {
+  pdl_enter(k_cache, v_cache, kv_indices, k_out, v_out);
   const int pieces = row_bytes / 16;                       // 16 fp8 per piece
   const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
   if (idx >= (long long)T * pieces * 2) return;
@@ -574,14 +577,14 @@ cudaError_t launch_gqa_core(const GqaDims& g, const void* q_raw, const void* k_r
     once.mark(dev);
   }
   { KernelSpan ks(K_GQA_PREP, s);
-  gqa_prep_kernel<<<M, 256, (8 * g.d + g.rotary_dim) * sizeof(float), s>>>(g, (const __nv_bfloat16*)q_raw, (const __nv_bfloat16*)k_raw,
+  launch_pdl(gqa_prep_kernel, M, 256, (8 * g.d + g.rotary_dim) * sizeof(float), s, g, (const __nv_bfloat16*)q_raw, (const __nv_bfloat16*)k_raw,
                                                           (const __nv_bfloat16*)v_raw, q_norm, k_norm, positions,
                                                           kv_indices, (__nv_bfloat16*)q_rot, (uint8_t*)k_cache,
                                                           (uint8_t*)v_cache, M); }
   const int row = g.nkv * g.d;
   const long long n_thr = (long long)kv_len * (row / 16) * 2;
   { KernelSpan ks(K_KV_GATHER, s);
-  gqa_gather_kernel<<<(unsigned)((n_thr + 255) / 256), 256, 0, s>>>((const uint8_t*)k_cache, (const uint8_t*)v_cache, kv_indices,
+  launch_pdl(gqa_gather_kernel, (unsigned)((n_thr + 255) / 256), 256, 0, s, (const uint8_t*)k_cache, (const uint8_t*)v_cache, kv_indices,
                                                                     row, kv_len, (__nv_bfloat16*)k_bf, (__nv_bfloat16*)v_bf); }
   alignas(64) CUtensorMap tq, tk, tv;
   cudaError_t e = make_tmap_bf16_rows(&tq, q_rot, M, (long long)g.nh * g.d, kFQ);
@@ -594,11 +597,13 @@ cudaError_t launch_gqa_core(const GqaDims& g, const void* q_raw, const void* k_r
   dim3 grid((M + kFQ - 1) / kFQ, g.nh);
   KernelSpan ks(K_FMHA, s);
   if (g.d == 256)
-    gqa_fmha_kernel<256, 256, false><<<grid, kFThreads, FmhaSmem<256, 256>::kTotal, s>>>(
-        tq, tk, tk, tv, g, (const __nv_bfloat16*)q_raw, (__nv_bfloat16*)attn_out, M, q_start, kv_len, sl2, 0, 0);
+    launch_pdl(gqa_fmha_kernel<256, 256, false>, grid, kFThreads, FmhaSmem<256, 256>::kTotal, s,
+        tq, tk, tk, tv, g, (const __nv_bfloat16*)q_raw, (__nv_bfloat16*)attn_out, M, q_start, kv_len, sl2, 0, 0, 1 << 30, nullptr, 1, nullptr, 0.f,
+        0.f, nullptr, nullptr, nullptr, 0);
   else
-    gqa_fmha_kernel<128, 128, false><<<grid, kFThreads, FmhaSmem<128, 128>::kTotal, s>>>(
-        tq, tk, tk, tv, g, (const __nv_bfloat16*)q_raw, (__nv_bfloat16*)attn_out, M, q_start, kv_len, sl2, 0, 0);
+    launch_pdl(gqa_fmha_kernel<128, 128, false>, grid, kFThreads, FmhaSmem<128, 128>::kTotal, s,
+        tq, tk, tk, tv, g, (const __nv_bfloat16*)q_raw, (__nv_bfloat16*)attn_out, M, q_start, kv_len, sl2, 0, 0, 1 << 30, nullptr, 1, nullptr, 0.f,
+        0.f, nullptr, nullptr, nullptr, 0);
   return cudaGetLastError();
 }
 
@@ -627,6 +632,7 @@ __global__ void __launch_bounds__(256) mla_prep_kernel(MlaDims m, const __nv_bfl
                                                        const int* __restrict__ kv_indices,
                                                        uint8_t* __restrict__ ckv_cache, uint8_t* __restrict__ kpe_cache,
                                                        int M) {
+  pdl_enter(kv_a, q_full, kv_norm_w, inv_freq, positions, kv_indices, ckv_cache, kpe_cache);
   __shared__ float red[8], s_cos[32], s_sin[32];      // the launcher requires rope == 64
   const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int pos = positions[t];
@@ -689,6 +695,7 @@ __global__ void __launch_bounds__(256) mla_gather_kernel(const uint8_t* __restri
                                                          const int* __restrict__ kv_indices, int lora, int rope, int T,
                                                          __nv_bfloat16* __restrict__ ckv_out,
                                                          __nv_bfloat16* __restrict__ kpe_out) {
+  pdl_enter(ckv_cache, kpe_cache, kv_indices, ckv_out, kpe_out);
   const int key = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (key >= T) return;
   const long long slot = (long long)kv_indices[key >> 4] * 16 + (key & 15);
@@ -721,10 +728,10 @@ cudaError_t launch_mla_core(const MlaDims& m, void* q_full, const void* kv_a, co
     once.mark(dev);
   }
   { KernelSpan ks(K_MLA_PREP, s);
-  mla_prep_kernel<<<M, 256, 0, s>>>(m, (const __nv_bfloat16*)kv_a, (__nv_bfloat16*)q_full, kv_norm_w, inv_freq, positions,
+  launch_pdl(mla_prep_kernel, M, 256, 0, s, m, (const __nv_bfloat16*)kv_a, (__nv_bfloat16*)q_full, kv_norm_w, inv_freq, positions,
                                     kv_indices, (uint8_t*)ckv_cache, (uint8_t*)kpe_cache, M); }
   { KernelSpan ks(K_KV_GATHER, s);
-  mla_gather_kernel<<<(kv_len + 7) / 8, 256, 0, s>>>((const uint8_t*)ckv_cache, (const uint8_t*)kpe_cache, kv_indices, m.lora,
+  launch_pdl(mla_gather_kernel, (kv_len + 7) / 8, 256, 0, s, (const uint8_t*)ckv_cache, (const uint8_t*)kpe_cache, kv_indices, m.lora,
                                                      m.rope, kv_len, (__nv_bfloat16*)ckv_bf16, (__nv_bfloat16*)kpe_bf16); }
   const int up = m.nh * (m.nope + m.dv);
   cudaError_t e = launch_dense_gemm(ckv_bf16, w_kv, kv_up, nullptr, kv_len, up, m.lora, up, false, num_sms, s);
@@ -740,8 +747,9 @@ cudaError_t launch_mla_core(const MlaDims& m, void* q_full, const void* kv_a, co
   const float sl2 = sm_scale * 1.4426950408889634f;
   dim3 grid((M + kFQ - 1) / kFQ, m.nh);
   KernelSpan ks(K_FMHA, s);
-  gqa_fmha_kernel<192, 128, true><<<grid, kFThreads, FmhaSmem<192, 128>::kTotal, s>>>(
-      tq, tk, tpe, tk, g, nullptr, (__nv_bfloat16*)attn_out, M, q_start, kv_len, sl2, 0, m.nh * m.nope);
+  launch_pdl(gqa_fmha_kernel<192, 128, true>, grid, kFThreads, FmhaSmem<192, 128>::kTotal, s,
+      tq, tk, tpe, tk, g, nullptr, (__nv_bfloat16*)attn_out, M, q_start, kv_len, sl2, 0, m.nh * m.nope, 1 << 30, nullptr, 1, nullptr, 0.f,
+      0.f, nullptr, nullptr, nullptr, 0);
   return cudaGetLastError();
 }
 
@@ -770,7 +778,7 @@ cudaError_t launch_fmha_latent(const void* q, const void* kv_up, const void* kpe
   GqaDims g{0, nh, nh, 192, 0, 0, 0.f, 0.f};
   dim3 grid((M + kFQ - 1) / kFQ, nh);
   KernelSpan ks(K_FMHA, s);
-  gqa_fmha_kernel<192, 128, true><<<grid, kFThreads, FmhaSmem<192, 128>::kTotal, s>>>(
+  launch_pdl(gqa_fmha_kernel<192, 128, true>, grid, kFThreads, FmhaSmem<192, 128>::kTotal, s,
       tq, tk, tpe, tk, g, nullptr, (__nv_bfloat16*)out, M, q_start, kv_len, sm_scale * 1.4426950408889634f, 0, nh * 128, window, sinks, 1,
       nullptr, 0.f, 0.f, nullptr, nullptr, head_gate, ldg);
   return cudaGetLastError();
@@ -810,11 +818,11 @@ cudaError_t launch_fmha_maps(const void* q, const void* k, const void* v, float*
   KernelSpan ks(K_FMHA, s);
   const float sl2 = sm_scale * 1.4426950408889634f;
   if (dv == 256)
-    gqa_fmha_kernel<128, 256, false><<<grid, kFThreads, FmhaSmem<128, 256>::kTotal, s>>>(tq, tk, tk, tv, g, nullptr, nullptr, M, q_start, kv_len,
-                                                                                          sl2, 0, 0, window, sinks, maps, out_f32, cap_in, cap_out, lse_out, slopes);
+    launch_pdl(gqa_fmha_kernel<128, 256, false>, grid, kFThreads, FmhaSmem<128, 256>::kTotal, s, tq, tk, tk, tv, g, nullptr, nullptr, M, q_start, kv_len,
+                                                                                          sl2, 0, 0, window, sinks, maps, out_f32, cap_in, cap_out, lse_out, slopes, nullptr, 0);
   else
-    gqa_fmha_kernel<128, 128, false><<<grid, kFThreads, FmhaSmem<128, 128>::kTotal, s>>>(tq, tk, tk, tv, g, nullptr, nullptr, M, q_start, kv_len,
-                                                                                          sl2, 0, 0, window, sinks, maps, out_f32, cap_in, cap_out, lse_out, slopes);
+    launch_pdl(gqa_fmha_kernel<128, 128, false>, grid, kFThreads, FmhaSmem<128, 128>::kTotal, s, tq, tk, tk, tv, g, nullptr, nullptr, M, q_start, kv_len,
+                                                                                          sl2, 0, 0, window, sinks, maps, out_f32, cap_in, cap_out, lse_out, slopes, nullptr, 0);
   return cudaGetLastError();
 }
 

@@ -201,6 +201,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_wait();
 
   const int n_chunks = *p.n_chunks;
   const int n_items = n_chunks * p.items_per_chunk;
@@ -688,7 +689,7 @@ static cudaError_t launch_kernel(const GemmParams& p, const CUtensorMap& tmap, i
   GemmParams pp = p;
   pp.trace = trace;
   pp.magic = 0x43004300u;
-  kern<<<num_sms, kNumThreads, smem, stream>>>(pp, tmap);
+  launch_pdl(kern, num_sms, kNumThreads, smem, stream, pp, tmap);
   return cudaGetLastError();
 }
 

@@ -6,6 +6,8 @@
 
 #include <atomic>
 
+#include "pdl.cuh"
+
 namespace kb2 {
 
 // cudaFuncAttributeMaxDynamicSharedMemorySize is a PER-DEVICE attribute: one process may drive several GPUs (the

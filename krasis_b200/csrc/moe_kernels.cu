@@ -24,6 +24,7 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const __nv_bfloat16*
                                                             const __nv_bfloat16* __restrict__ gate,
                                                             const float* __restrict__ gate_bias,
                                                             float* __restrict__ logits, int M, int E, int H) {
+  pdl_enter(h, gate, gate_bias, logits);
   __shared__ float hs[RK][RT + 4];
   __shared__ float gs[RK][RT + 4];
   const int m0 = blockIdx.y * RT, e0 = blockIdx.x * RT;
@@ -90,6 +91,7 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const float* __restric
                                                           const float* __restrict__ corr_bias, int M, int E,
                                                           int top_k, int scoring, int renorm,
                                                           int* __restrict__ ids, float* __restrict__ wts) {
+  pdl_enter(logits, corr_bias, ids, wts);
   const int lane = threadIdx.x & 31;
   const int m = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (m >= M) return;
@@ -207,6 +209,7 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const float* __restric
 // 4096 entries per block are counted in shared memory first: one global atomic per entry met 160 others on its counter (12 us for 81920 entries).
 constexpr int kCountPerBlock = 4096;
 __global__ void __launch_bounds__(1024) count_kernel(const int* __restrict__ ids, int n, int e_start, int e_end, int* __restrict__ counts) {
+  pdl_enter(ids, counts);
   __shared__ int s_cnt[1024];
   s_cnt[threadIdx.x] = 0;
   __syncthreads();
@@ -239,6 +242,7 @@ __device__ __forceinline__ void write_chunks(ChunkDesc* chunks, int e, int off, 
 __global__ void __launch_bounds__(1024) scan_kernel(const int* __restrict__ counts, int E, int chunk_tokens, int* __restrict__ offsets,
                                                     int* __restrict__ cursor, ChunkDesc* __restrict__ chunks,
                                                     int* __restrict__ n_chunks) {
+  pdl_enter(counts, offsets, cursor, chunks, n_chunks);
   __shared__ int s_cnt[1024], s_chk[1024];
   const int t = threadIdx.x;
   const int c = t < E ? counts[t] : 0;
@@ -279,6 +283,7 @@ __global__ void __launch_bounds__(256) bin_rows_kernel(const int* __restrict__ i
                                                        ChunkDesc* __restrict__ chunks, int* __restrict__ n_chunks, float* __restrict__ sorted_w,
                                                        int* __restrict__ slot_of, int* __restrict__ sorted_ids, int* __restrict__ sorted_tok,
                                                        const uint4* __restrict__ x, uint4* __restrict__ x_sorted, int vec_per_row) {
+  pdl_enter(ids, wts, counts, offsets, chunks, n_chunks, sorted_w, slot_of, sorted_ids, sorted_tok, x, x_sorted);
   __shared__ short s_id[kBinRowsMax];
   __shared__ int s_cnt[1024], s_off[1024], s_warp[2][8];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -370,6 +375,7 @@ __global__ void __launch_bounds__(256) scatter_kernel(const int* __restrict__ id
                                                       int* __restrict__ sorted_ids,
                                                       const uint4* __restrict__ x, uint4* __restrict__ x_sorted,
                                                       int vec_per_row) {
+  pdl_enter(ids, wts, offsets, cursor, sorted_w, slot_of, sorted_ids, x, x_sorted);
   const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (i >= n) return;
@@ -396,6 +402,7 @@ __global__ void __launch_bounds__(256) scatter_index_kernel(const int* __restric
                                                             int top_k, int e_start, int e_end, const int* __restrict__ offsets,
                                                             int* __restrict__ cursor, float* __restrict__ sorted_w,
                                                             int* __restrict__ slot_of, int* __restrict__ sorted_tok) {
+  pdl_enter(ids, wts, offsets, cursor, sorted_w, slot_of, sorted_tok);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int e = ids[i];
@@ -420,6 +427,7 @@ __global__ void __launch_bounds__(kCombineThreads) combine_kernel(const __nv_bfl
                                                       float rsf, int apply_rsf,
                                                       const __nv_bfloat16* __restrict__ shared,
                                                       __nv_bfloat16* __restrict__ out, CombineScatter sc) {
+  pdl_enter(c3, slot_of, shared, out);
   const int vec_per_row = H >> 3;
   const int m = blockIdx.x, v = blockIdx.y * kCombineThreads + threadIdx.x;
   if (v >= vec_per_row) return;
@@ -708,7 +716,7 @@ cudaError_t launch_router_logits(const void* h, const void* gate, const float* b
                                  int H, cudaStream_t s) {
   KernelSpan ks(K_ROUTER_GEMM, s);
   dim3 grid((E + RT - 1) / RT, (M + RT - 1) / RT);
-  router_logits_kernel<<<grid, 256, 0, s>>>((const __nv_bfloat16*)h, (const __nv_bfloat16*)gate, bias, logits, M, E, H);
+  launch_pdl(router_logits_kernel, grid, 256, 0, s, (const __nv_bfloat16*)h, (const __nv_bfloat16*)gate, bias, logits, M, E, H);
   return cudaGetLastError();
 }
 
@@ -719,15 +727,15 @@ cudaError_t launch_router_topk(const float* logits, const float* corr_bias, int 
   dim3 grid((M + warps - 1) / warps);
   if (top_k > 32 || E > 1024) return cudaErrorInvalidValue;
   if (E <= 64)
-    router_topk_kernel<2><<<grid, warps * 32, 0, s>>>(logits, corr_bias, M, E, top_k, scoring, renorm, ids, wts);
+    launch_pdl(router_topk_kernel<2>, grid, warps * 32, 0, s, logits, corr_bias, M, E, top_k, scoring, renorm, ids, wts);
   else if (E <= 128)
-    router_topk_kernel<4><<<grid, warps * 32, 0, s>>>(logits, corr_bias, M, E, top_k, scoring, renorm, ids, wts);
+    launch_pdl(router_topk_kernel<4>, grid, warps * 32, 0, s, logits, corr_bias, M, E, top_k, scoring, renorm, ids, wts);
   else if (E <= 256)
-    router_topk_kernel<8><<<grid, warps * 32, 0, s>>>(logits, corr_bias, M, E, top_k, scoring, renorm, ids, wts);
+    launch_pdl(router_topk_kernel<8>, grid, warps * 32, 0, s, logits, corr_bias, M, E, top_k, scoring, renorm, ids, wts);
   else if (E <= 512)
-    router_topk_kernel<16><<<grid, warps * 32, 0, s>>>(logits, corr_bias, M, E, top_k, scoring, renorm, ids, wts);
+    launch_pdl(router_topk_kernel<16>, grid, warps * 32, 0, s, logits, corr_bias, M, E, top_k, scoring, renorm, ids, wts);
   else
-    router_topk_kernel<32><<<grid, warps * 32, 0, s>>>(logits, corr_bias, M, E, top_k, scoring, renorm, ids, wts);
+    launch_pdl(router_topk_kernel<32>, grid, warps * 32, 0, s, logits, corr_bias, M, E, top_k, scoring, renorm, ids, wts);
   return cudaGetLastError();
 }
 
@@ -742,19 +750,19 @@ cudaError_t launch_binning(const int* ids, const float* wts, int M, int top_k, i
   KernelSpan ks(K_BINNING, s, binning_launches(n));
   if (E > 1024) return cudaErrorInvalidValue;
   if (n > 0 && n <= kBinRowsMax) {      // measured with 2048 columns: 24 entries 9.3 -> 4.1 us (memset, count, scan, scatter before), 2334 entries 13 -> 6.6 us
-    bin_rows_kernel<<<(n + 7) / 8, 256, 0, s>>>(ids, wts, n, top_k, e_start, E, chunk_tokens, counts, offsets, chunks, n_chunks, sorted_w, slot_of,
+    launch_pdl(bin_rows_kernel, (n + 7) / 8, 256, 0, s, ids, wts, n, top_k, e_start, E, chunk_tokens, counts, offsets, chunks, n_chunks, sorted_w, slot_of,
                                                 sorted_ids, sorted_tok, (const uint4*)x, (uint4*)x_sorted, H / 8);
     return cudaGetLastError();
   }
   cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(int) * E, s);
   if (e != cudaSuccess) return e;
-  if (n > 0) count_kernel<<<(n + kCountPerBlock - 1) / kCountPerBlock, 1024, 0, s>>>(ids, n, e_start, e_end, counts);
-  scan_kernel<<<1, 1024, 0, s>>>(counts, E, chunk_tokens, offsets, cursor, chunks, n_chunks);
+  if (n > 0) launch_pdl(count_kernel, (n + kCountPerBlock - 1) / kCountPerBlock, 1024, 0, s, ids, n, e_start, e_end, counts);
+  launch_pdl(scan_kernel, 1, 1024, 0, s, counts, E, chunk_tokens, offsets, cursor, chunks, n_chunks);
   if (n > 0 && x_sorted)
-    scatter_kernel<<<(n + 7) / 8, 256, 0, s>>>(ids, wts, n, top_k, e_start, e_end, offsets, cursor, sorted_w, slot_of,
+    launch_pdl(scatter_kernel, (n + 7) / 8, 256, 0, s, ids, wts, n, top_k, e_start, e_end, offsets, cursor, sorted_w, slot_of,
                                                sorted_ids, (const uint4*)x, (uint4*)x_sorted, H / 8);
   else if (n > 0)
-    scatter_index_kernel<<<(n + 255) / 256, 256, 0, s>>>(ids, wts, n, top_k, e_start, e_end, offsets, cursor, sorted_w, slot_of,
+    launch_pdl(scatter_index_kernel, (n + 255) / 256, 256, 0, s, ids, wts, n, top_k, e_start, e_end, offsets, cursor, sorted_w, slot_of,
                                                          sorted_tok);
   return cudaGetLastError();
 }
@@ -763,7 +771,7 @@ cudaError_t launch_combine_scatter(const void* c3, const int* slot_of, int M, in
                                    const void* shared, void* out, const CombineScatter& sc, cudaStream_t s) {
   KernelSpan ks(K_COMBINE, s);
   if (M <= 0 || H < 8) return cudaSuccess;
-  combine_kernel<<<dim3(M, (H / 8 + kCombineThreads - 1) / kCombineThreads), kCombineThreads, 0, s>>>((const __nv_bfloat16*)c3, slot_of, M, H, top_k, rsf,
+  launch_pdl(combine_kernel, dim3(M, (H / 8 + kCombineThreads - 1) / kCombineThreads), kCombineThreads, 0, s, (const __nv_bfloat16*)c3, slot_of, M, H, top_k, rsf,
                                                                 apply_rsf, (const __nv_bfloat16*)shared,
                                                                 (__nv_bfloat16*)out, sc);
   return cudaGetLastError();

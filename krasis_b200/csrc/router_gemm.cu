@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(kRThreads, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_enter(gate_bias, logits);
 
   if (warp == 0) {
     {
@@ -151,7 +152,7 @@ static cudaError_t launch_router_tile(const CUtensorMap& tx, const CUtensorMap& 
     if (e != cudaSuccess) return e;
     once.mark(dev);
   }
-  router_gemm_kernel<NB><<<dim3((M + 127) / 128, (E + NB - 1) / NB), kRThreads, RouterTile<NB>::kSmem, s>>>(tx, tg, bias, logits, M, E, H);
+  launch_pdl(router_gemm_kernel<NB>, dim3((M + 127) / 128, (E + NB - 1) / NB), kRThreads, RouterTile<NB>::kSmem, s, tx, tg, bias, logits, M, E, H);
   return cudaGetLastError();
 }
 

@@ -9,6 +9,7 @@
 #include <stdio.h>
 
 #include "../../include/krasis_b200_seq.h"
+#include "pdl.cuh"
 
 namespace kb2seq {
 

@@ -45,6 +45,7 @@ __global__ void __launch_bounds__(256) head_kv_prep_kernel(float* __restrict__ p
                                                            int page_size, void* __restrict__ kc, void* __restrict__ vc, int dt_cache,
                                                            int norm_whole, int rot_half, const double* __restrict__ vfreq, float amp,
                                                            int v_is_k) {
+  kb2::pdl_enter(proj, bias, qw, kw, freq, positions, seq_of, pages, kc, vc, vfreq);
   extern __shared__ float rot_tab[];          // [rot_dims / 2][2]: cos, sin of the token's position, shared by all its vectors
   __shared__ float red[32];
   const long long t = blockIdx.x;
@@ -147,6 +148,7 @@ __global__ void __launch_bounds__(256) kv_pool_kernel(const void* __restrict__ k
                                                       void* __restrict__ vp, int dt_cache, int kw, int vw, int pool, int rows_per_page,
                                                       const int* __restrict__ positions, const int* __restrict__ seq_of,
                                                       const int* __restrict__ pages, int max_pages, int page_size) {
+  kb2::pdl_enter(kc, vc, kp, vp, positions, seq_of, pages);
   const long long t = blockIdx.x;
   const int pos = positions[t];
   if (pos % pool != pool - 1) return;
@@ -177,6 +179,7 @@ __global__ void __launch_bounds__(kPAThreads) paged_attn_kernel(
     float* __restrict__ part_acc, float* __restrict__ part_ml, const int* __restrict__ cu, int skip_from, float softcap,
     const float* __restrict__ sinks, int pool, int rows_per_page, const void* __restrict__ kp, const void* __restrict__ vp, int pool_only,
     const float* __restrict__ slopes) {
+  kb2::pdl_enter(proj, kc, vc, positions, seq_of, pages, out, part_acc, part_ml, cu, sinks, kp, vp, slopes);
   extern __shared__ __align__(16) float sm[];
   constexpr int KT = kPAKT;
   const long long t = blockIdx.x;
@@ -333,6 +336,7 @@ __global__ void __launch_bounds__(256) attn_finish_kernel(const float* __restric
                                                           int dt_out, const int* __restrict__ seq_of, const int* __restrict__ cu,
                                                           int skip_from, int gate_wide, const int* __restrict__ positions,
                                                           const double* __restrict__ vfreq, int rot_half) {
+  kb2::pdl_enter(a, part_acc, part_ml, coef, gate, out, seq_of, cu, positions, vfreq);
   __shared__ float turn_buf[8][32 * NA];
   const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -433,6 +437,7 @@ __global__ void __launch_bounds__(256) attn_finish_kernel(const float* __restric
 __global__ void __launch_bounds__(256) pool_merge_kernel(float* __restrict__ a, const float* __restrict__ lse, const float* __restrict__ part_acc,
                                                          const float* __restrict__ part_ml, long long rows, int H, int dv,
                                                          const int* __restrict__ seq_of, const int* __restrict__ cu, int min_portion) {
+  kb2::pdl_enter(a, lse, part_acc, part_ml, seq_of, cu);
   const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (w >= rows) return;
@@ -468,6 +473,7 @@ __device__ __forceinline__ float glu_row_weight(const float* __restrict__ row_w,
 __global__ void glu_kernel(const void* __restrict__ in, int dt_in, long long ld_in, void* __restrict__ out, int dt_out, long long rows, int F,
                            int kind, float limit, float alpha, const int* __restrict__ n_tiles, int tile_rows, const float* __restrict__ bias,
                            const float* __restrict__ row_w, const int* __restrict__ row_map) {
+  kb2::pdl_enter(in, out, n_tiles, bias, row_w, row_map);
   if (n_tiles != nullptr) rows = min(rows, (long long)n_tiles[0] * tile_rows);
   const long long n = rows * F;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -487,6 +493,7 @@ __global__ void glu_kernel(const void* __restrict__ in, int dt_in, long long ld_
 __global__ void glu_bf16x8_kernel(const bf16* __restrict__ in, long long ld_in, bf16* __restrict__ out, long long rows, int F, int kind, float limit,
                                   float alpha, const int* __restrict__ n_tiles, int tile_rows, const float* __restrict__ bias,
                                   const float* __restrict__ row_w, const int* __restrict__ row_map) {
+  kb2::pdl_enter(in, out, n_tiles, bias, row_w, row_map);
   if (n_tiles != nullptr) rows = min(rows, (long long)n_tiles[0] * tile_rows);
   const int F8 = F >> 3;
   const long long n = rows * F8;
@@ -537,6 +544,7 @@ __global__ void __launch_bounds__(128) route_topk_kernel(const float* __restrict
                                                          const float* __restrict__ correction, int score_kind, int groups, int keep,
                                                          int top, int renorm, float out_scale, int* __restrict__ ids,
                                                          float* __restrict__ weights, int group_kind, const float* __restrict__ bias) {
+  kb2::pdl_enter(z, correction, ids, weights, bias);
   extern __shared__ float rsm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const long long t = (long long)blockIdx.x * nw + warp;
@@ -635,6 +643,7 @@ __global__ void __launch_bounds__(128) route_topk_kernel(const float* __restrict
 constexpr int kMoeBM = 64;
 // counts[e] = number of (token, k) slots routed to expert e < E (identity / absent experts have id >= E or < 0)
 __global__ void moe_count_kernel(const int* __restrict__ ids, long long slots, int E, int* __restrict__ counts) {
+  kb2::pdl_enter(ids, counts);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += (long long)gridDim.x * blockDim.x) {
     const int e = ids[i];
     if (e >= 0 && e < E) atomicAdd(&counts[e], 1);
@@ -643,6 +652,7 @@ __global__ void moe_count_kernel(const int* __restrict__ ids, long long slots, i
 // One block: offs[e] = first row of expert e's run, runs padded to whole tiles of tile_rows; tile_expert[tile]; n_tiles[0]; cursor[e] = 0.
 __global__ void moe_plan_kernel(const int* __restrict__ counts, int E, int tile_rows, int* __restrict__ offs, int* __restrict__ cursor,
                                 int* __restrict__ tile_expert, int* __restrict__ n_tiles) {
+  kb2::pdl_enter(counts, offs, cursor, tile_expert, n_tiles);
   if (threadIdx.x == 0) {
     int tiles = 0;
     for (int e = 0; e < E; ++e) {
@@ -661,6 +671,7 @@ __global__ void moe_plan_kernel(const int* __restrict__ counts, int E, int tile_
 // slot_row[p] = slot (t * top + k) that sits at row p of the binned order (-1: padding); pos_of_slot[slot] = p (-1: not routed here)
 __global__ void moe_scatter_kernel(const int* __restrict__ ids, long long slots, int E, const int* __restrict__ offs,
                                    int* __restrict__ cursor, int* __restrict__ slot_row, int* __restrict__ pos_of_slot) {
+  kb2::pdl_enter(ids, offs, cursor, slot_row, pos_of_slot);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += (long long)gridDim.x * blockDim.x) {
     const int e = ids[i];
     int p = -1;
@@ -680,6 +691,7 @@ __global__ void __launch_bounds__(kBinThreads) moe_bin_block_kernel(const int* _
                                                                     int* __restrict__ counts, int* __restrict__ offs, int* __restrict__ tile_expert,
                                                                     int* __restrict__ n_tiles, int* __restrict__ slot_row, int max_rows,
                                                                     int* __restrict__ pos_of_slot) {
+  kb2::pdl_enter(ids, counts, offs, tile_expert, n_tiles, slot_row, pos_of_slot);
   __shared__ int cnt[kBinMaxExperts], first[kBinMaxExperts + 1];
   for (int e = threadIdx.x; e < E; e += kBinThreads) cnt[e] = 0;
   for (int r = threadIdx.x; r < max_rows; r += kBinThreads) slot_row[r] = -1;
@@ -733,6 +745,7 @@ __global__ void __launch_bounds__(kBinThreads) moe_bin_block_kernel(const int* _
 // they are (a product's row depends on its own input row only, and nothing reads theirs).  Bound by traffic: 2 x 4 KB per row of 2048.
 __global__ void __launch_bounds__(256) moe_gather_kernel(const bf16* __restrict__ h, long long ldh, const int* __restrict__ slot_row, int top,
                                                          const int* __restrict__ n_tiles, int tile_rows, bf16* __restrict__ xs, int W) {
+  kb2::pdl_enter(h, slot_row, n_tiles, xs);
   const int lane = threadIdx.x & 31;
   const long long rows = (long long)n_tiles[0] * tile_rows;
   for (long long p = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); p < rows; p += (long long)gridDim.x * 8) {
@@ -752,6 +765,7 @@ __global__ void __launch_bounds__(256) moe_gemm_kernel(const TA* __restrict__ A,
                                                        const TB* __restrict__ B, long long ldb, long long sB, TC* __restrict__ C,
                                                        long long ldc, int N, int K, const int* __restrict__ tile_expert,
                                                        const int* __restrict__ n_tiles, int tile_rows) {
+  kb2::pdl_enter(A, row_map, B, C, tile_expert, n_tiles);
   constexpr int BM = kMoeBM, BN = 64, BK = 16;           // tile_rows is a multiple of BM: a block never straddles two experts
   if ((long long)blockIdx.y * BM >= (long long)n_tiles[0] * tile_rows) return;
   __shared__ float As[BK][BM + 4], Bs[BK][BN + 4];
@@ -814,6 +828,7 @@ template <typename TA, typename TB, typename TC>
 __global__ void __launch_bounds__(256) moe_gemv_kernel(const TA* __restrict__ A, long long lda, int div, const int* __restrict__ ids, int E,
                                                        const TB* __restrict__ B, long long ldb, long long sB, TC* __restrict__ C,
                                                        long long ldc, int N, int K) {
+  kb2::pdl_enter(A, ids, B, C);
   const int slot = blockIdx.y;
   const int e = ids[slot];
   if (e < 0 || e >= E) return;
@@ -853,6 +868,7 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __res
                                    const float* __restrict__ weights, int top, int E, int ident, const void* __restrict__ h, int dt_h,
                                    const float* __restrict__ shared, float* __restrict__ out, int W,
                                    const float* __restrict__ shared_gate, long long ldsg) {
+  kb2::pdl_enter(y, pos_of_slot, ids, weights, h, shared, out, shared_gate);
   const long long t = blockIdx.x;
   const float sgate = shared_gate != nullptr ? 1.f / (1.f + expf(-shared_gate[t * ldsg])) : 1.f;   // the shared expert's weight for this token
   if ((W & 3) == 0 && dt_h == 1) {           // four columns per thread, 16-byte loads of the expert rows; same order of the sum over k
@@ -914,7 +930,7 @@ KB2SEQ_API int kb2_seq_head_kv_prep(float* proj, long long ldp, int T, int H, in
       rot_dims > d || (rot_dims & 1) || (rot_dims && !freq) || page_size <= 0 || max_pages <= 0 || bad_dt(dt_cache) ||
       (G > 0 && (!kc || !vc)))
     return failf(KB2SEQ_ERR_VALUE, "head_kv_prep: bad argument");
-  head_kv_prep_kernel<<<T, 256, (size_t)rot_dims * 4, (cudaStream_t)stream>>>(proj, ldp, H, G, M, d, dv, bias, qw, kw, eps, freq, rot_dims, positions, seq_of,
+  kb2::launch_pdl(head_kv_prep_kernel, T, 256, (size_t)rot_dims * 4, (cudaStream_t)stream, proj, ldp, H, G, M, d, dv, bias, qw, kw, eps, freq, rot_dims, positions, seq_of,
                                                            pages, max_pages, page_size, kc, vc, dt_cache, norm_whole, rot_half, vfreq, amp, v_is_k);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
@@ -925,7 +941,7 @@ KB2SEQ_API int kb2_seq_kv_pool(const void* kc, const void* vc, void* kp, void* v
   if (!kc || !vc || !kp || !vp || bad_dt(dt_cache) || kw <= 0 || vw <= 0 || pool <= 0 || T <= 0 || !positions || !seq_of || !pages ||
       max_pages <= 0 || page_size <= 0)
     return failf(KB2SEQ_ERR_VALUE, "kv_pool: bad argument");
-  kv_pool_kernel<<<T, 256, 0, (cudaStream_t)stream>>>(kc, vc, kp, vp, dt_cache, kw, vw, pool, (page_size + pool - 1) / pool, positions, seq_of,
+  kb2::launch_pdl(kv_pool_kernel, T, 256, 0, (cudaStream_t)stream, kc, vc, kp, vp, dt_cache, kw, vw, pool, (page_size + pool - 1) / pool, positions, seq_of,
                                                       pages, max_pages, page_size);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
@@ -956,7 +972,7 @@ KB2SEQ_API int kb2_seq_paged_attn(const float* proj, long long ldp, int T, int H
   if (smem > 48 * 1024) SEQ_CUDA(cudaFuncSetAttribute(paged_attn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int nrb = (R + RB - 1) / RB;
   if ((long long)G * nrb > 65535) return failf(KB2SEQ_ERR_VALUE, "paged_attn: too many heads");
-  paged_attn_kernel<<<dim3(T, G * nrb, nsplit), kPAThreads, smem, (cudaStream_t)stream>>>(
+  kb2::launch_pdl(paged_attn_kernel, dim3(T, G * nrb, nsplit), kPAThreads, smem, (cudaStream_t)stream, 
       proj, ldp, H, G, M, d, dv, RB, kc, vc, dt_cache, positions, seq_of, pages, max_pages, page_size, scale, chunk, window, out, nsplit,
       part_acc, part_ml, cu, skip_from, softcap, sinks, pool, pool > 0 ? (page_size + pool - 1) / pool : 0, kp, vp, pool_only, slopes);
   SEQ_LAUNCHED();
@@ -967,7 +983,7 @@ KB2SEQ_API int kb2_seq_pool_merge(float* a, const float* lse, const float* part_
                                   const int* seq_of, const int* cu, int min_portion, void* stream) {
   if (!a || !lse || !part_acc || !part_ml || !seq_of || !cu || T <= 0 || H <= 0 || dv <= 0) return failf(KB2SEQ_ERR_VALUE, "pool_merge: bad argument");
   const long long rows = (long long)T * H;
-  pool_merge_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, (cudaStream_t)stream>>>(a, lse, part_acc, part_ml, rows, H, dv, seq_of, cu, min_portion);
+  kb2::launch_pdl(pool_merge_kernel, (unsigned)((rows + 7) / 8), 256, 0, (cudaStream_t)stream, a, lse, part_acc, part_ml, rows, H, dv, seq_of, cu, min_portion);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
 }
@@ -983,7 +999,7 @@ KB2SEQ_API int kb2_seq_attn_finish(const float* a, const float* part_acc, const 
   if (dv > 32 * kFinAcc) return failf(KB2SEQ_ERR_VALUE, "attn_finish: value size %d > %d", dv, 32 * kFinAcc);
   const long long nwarps = (long long)T * H;
 #define KB2_FIN(NAV)                                                                                                                        \
-  attn_finish_kernel<NAV><<<(unsigned)((nwarps + 7) / 8), 256, 0, (cudaStream_t)stream>>>(a, part_acc, part_ml, nsplit, T, H, M, dv, coef, unit_norm, \
+  kb2::launch_pdl(attn_finish_kernel<NAV>, (unsigned)((nwarps + 7) / 8), 256, 0, (cudaStream_t)stream, a, part_acc, part_ml, nsplit, T, H, M, dv, coef, unit_norm, \
                                                                                          eps, post_scale, gate, ldg, out, dt_out, seq_of, cu, skip_from, \
                                                                                          gate_wide, positions, vfreq, rot_half)
   if (dv <= 128) KB2_FIN(4);
@@ -1002,14 +1018,14 @@ KB2SEQ_API int kb2_seq_glu(const void* in, int dt_in, long long ld_in, void* out
   if (dt_in == 1 && dt_out == 1 && F % 8 == 0 && ld_in % 8 == 0 && !((uintptr_t)in & 15) && !((uintptr_t)out & 15) && !((uintptr_t)bias & 15)) {
     const long long n8 = rows * (F / 8);
     const unsigned blocks8 = (unsigned)((n8 + 255) / 256 > 148 * 16 ? 148 * 16 : (n8 + 255) / 256);
-    glu_bf16x8_kernel<<<blocks8, 256, 0, (cudaStream_t)stream>>>((const bf16*)in, ld_in, (bf16*)out, rows, F, kind, limit, alpha, n_tiles, tile_rows, bias, row_w,
+    kb2::launch_pdl(glu_bf16x8_kernel, blocks8, 256, 0, (cudaStream_t)stream, (const bf16*)in, ld_in, (bf16*)out, rows, F, kind, limit, alpha, n_tiles, tile_rows, bias, row_w,
                                                               row_map);
     SEQ_LAUNCHED();
     return KB2SEQ_OK;
   }
   const long long n = rows * F;
   const unsigned blocks = (unsigned)((n + 255) / 256 > 148 * 16 ? 148 * 16 : (n + 255) / 256);
-  glu_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(in, dt_in, ld_in, out, dt_out, rows, F, kind, limit, alpha, n_tiles, tile_rows, bias, row_w,
+  kb2::launch_pdl(glu_kernel, blocks, 256, 0, (cudaStream_t)stream, in, dt_in, ld_in, out, dt_out, rows, F, kind, limit, alpha, n_tiles, tile_rows, bias, row_w,
                                                               row_map);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
@@ -1025,7 +1041,7 @@ KB2SEQ_API int kb2_seq_route(const float* z, long long ldz, int T, int E, const 
   const size_t smem = (size_t)4 * (2 * E + groups) * 4;
   if (smem > 200 * 1024) return failf(KB2SEQ_ERR_VALUE, "route: %d router outputs too many", E);
   if (smem > 48 * 1024) SEQ_CUDA(cudaFuncSetAttribute(route_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  route_topk_kernel<<<(T + 3) / 4, 128, smem, (cudaStream_t)stream>>>(z, ldz, T, E, correction, score_kind, groups, keep, top, renorm,
+  kb2::launch_pdl(route_topk_kernel, (T + 3) / 4, 128, smem, (cudaStream_t)stream, z, ldz, T, E, correction, score_kind, groups, keep, top, renorm,
                                                                       out_scale, ids, weights, group_kind, bias);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
@@ -1039,7 +1055,7 @@ static int moe_bin(const int* ids, long long slots, int E, int tile_rows, int* c
       max_rows < slots + (long long)E * (tile_rows - 1))
     return failf(KB2SEQ_ERR_VALUE, "moe_bin: bad argument");
   if (slots <= kBinMaxSlots && E <= kBinMaxExperts && max_rows <= 1 << 18) {
-    moe_bin_block_kernel<<<1, kBinThreads, 0, s>>>(ids, (int)slots, E, tile_rows, counts, offs, tile_expert, n_tiles, slot_row, (int)max_rows,
+    kb2::launch_pdl(moe_bin_block_kernel, 1, kBinThreads, 0, s, ids, (int)slots, E, tile_rows, counts, offs, tile_expert, n_tiles, slot_row, (int)max_rows,
                                                    pos_of_slot);
     SEQ_LAUNCHED();
     return KB2SEQ_OK;
@@ -1047,11 +1063,11 @@ static int moe_bin(const int* ids, long long slots, int E, int tile_rows, int* c
   SEQ_CUDA(cudaMemsetAsync(counts, 0, (size_t)E * 4, s));
   SEQ_CUDA(cudaMemsetAsync(slot_row, 0xFF, (size_t)max_rows * 4, s));
   const unsigned blocks = (unsigned)((slots + 255) / 256 > 1024 ? 1024 : (slots + 255) / 256);
-  moe_count_kernel<<<blocks, 256, 0, s>>>(ids, slots, E, counts);
+  kb2::launch_pdl(moe_count_kernel, blocks, 256, 0, s, ids, slots, E, counts);
   SEQ_LAUNCHED();
-  moe_plan_kernel<<<1, 256, 0, s>>>(counts, E, tile_rows, offs, cursor, tile_expert, n_tiles);
+  kb2::launch_pdl(moe_plan_kernel, 1, 256, 0, s, counts, E, tile_rows, offs, cursor, tile_expert, n_tiles);
   SEQ_LAUNCHED();
-  moe_scatter_kernel<<<blocks, 256, 0, s>>>(ids, slots, E, offs, cursor, slot_row, pos_of_slot);
+  kb2::launch_pdl(moe_scatter_kernel, blocks, 256, 0, s, ids, slots, E, offs, cursor, slot_row, pos_of_slot);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
 }
@@ -1074,7 +1090,7 @@ KB2SEQ_API int kb2_seq_moe_gather(const void* h, long long ldh, const int* slot_
       ((uintptr_t)xs & 15))
     return failf(KB2SEQ_ERR_VALUE, "moe_gather: bad argument");
   const unsigned blocks = (unsigned)((max_rows + 7) / 8 > 2368 ? 2368 : (max_rows + 7) / 8);
-  moe_gather_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>((const bf16*)h, ldh, slot_row, top, n_tiles, tile_rows, (bf16*)xs, W);
+  kb2::launch_pdl(moe_gather_kernel, blocks, 256, 0, (cudaStream_t)stream, (const bf16*)h, ldh, slot_row, top, n_tiles, tile_rows, (bf16*)xs, W);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
 }
@@ -1088,7 +1104,7 @@ KB2SEQ_API int kb2_seq_moe_gemm(const void* A, int dtA, long long lda, const int
   cudaStream_t s = (cudaStream_t)stream;
   dim3 grid((N + 63) / 64, max_tiles * (tile_rows / kMoeBM));
 #define G(TA, TB, TC)                                                                                                          \
-  moe_gemm_kernel<TA, TB, TC><<<grid, 256, 0, s>>>((const TA*)A, lda, row_map, div, (const TB*)B, ldb, sB, (TC*)C, ldc, N, K, tile_expert, \
+  kb2::launch_pdl(moe_gemm_kernel<TA, TB, TC>, grid, 256, 0, s, (const TA*)A, lda, row_map, div, (const TB*)B, ldb, sB, (TC*)C, ldc, N, K, tile_expert, \
                                                    n_tiles, tile_rows)
   switch (dtA * 4 + dtB * 2 + dtC) {
     case 0: G(float, float, float); break;
@@ -1112,7 +1128,7 @@ KB2SEQ_API int kb2_seq_moe_gemv(const void* A, int dtA, long long lda, int div, 
     return failf(KB2SEQ_ERR_VALUE, "moe_gemv: bad argument");
   cudaStream_t s = (cudaStream_t)stream;
   dim3 grid((N + 7) / 8, slots);
-#define G(TA, TB, TC) moe_gemv_kernel<TA, TB, TC><<<grid, 256, 0, s>>>((const TA*)A, lda, div, ids, E, (const TB*)B, ldb, sB, (TC*)C, ldc, N, K)
+#define G(TA, TB, TC) kb2::launch_pdl(moe_gemv_kernel<TA, TB, TC>, grid, 256, 0, s, (const TA*)A, lda, div, ids, E, (const TB*)B, ldb, sB, (TC*)C, ldc, N, K)
   switch (dtA * 4 + dtB * 2 + dtC) {
     case 0: G(float, float, float); break;
     case 1: G(float, float, bf16); break;
@@ -1133,7 +1149,7 @@ KB2SEQ_API int kb2_seq_moe_combine(const float* y, const int* pos_of_slot, const
                                    long long ldsg, void* stream) {
   if (!ids || (!weights && ident > 0) || !out || T <= 0 || top <= 0 || E < 0 || ident < 0 || W <= 0 || (E > 0 && !y) || (ident > 0 && (!h || bad_dt(dt_h))))
     return failf(KB2SEQ_ERR_VALUE, "moe_combine: bad argument");
-  moe_combine_kernel<<<T, 256, 0, (cudaStream_t)stream>>>(y, pos_of_slot, ids, weights, top, E, ident, h, dt_h, shared, out, W, shared_gate, ldsg);
+  kb2::launch_pdl(moe_combine_kernel, T, 256, 0, (cudaStream_t)stream, y, pos_of_slot, ids, weights, top, E, ident, h, dt_h, shared, out, W, shared_gate, ldsg);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
 }

@@ -33,6 +33,7 @@ long long g_launches = 0;
 template <typename T>
 __global__ void embed_scale_kernel(const T* __restrict__ table, const int* __restrict__ tokens, float* __restrict__ x, int W,
                                    float scale) {
+  kb2::pdl_enter(table, tokens, x);
   const long long t = blockIdx.x;
   const long long row = tokens[t];
   for (int d = threadIdx.x; d < W; d += blockDim.x) x[t * W + d] = ldf(table, row * W + d) * scale;
@@ -41,6 +42,7 @@ __global__ void embed_scale_kernel(const T* __restrict__ table, const int* __res
 // (4 tokens of 2048 columns took 9.5 us with eight rounds of loads)
 __global__ void __launch_bounds__(256) embed_scale_vec_kernel(const bf16* __restrict__ table, const int* __restrict__ tokens, float* __restrict__ x, int W,
                                                               float scale) {
+  kb2::pdl_enter(table, tokens, x);
   const long long t = blockIdx.x, row = tokens[t];
   for (int d = threadIdx.x * 8; d < W; d += 256 * 8) {
     float f[8];
@@ -58,6 +60,7 @@ template <typename TA, typename TB, typename TC>
 __global__ void __launch_bounds__(256) gemm_nt_kernel(const TA* __restrict__ A, long long lda, const TB* __restrict__ B, long long ldb,
                                                       TC* __restrict__ C, long long ldc, int M, int N, int K, long long sA,
                                                       long long sB, long long sC) {
+  kb2::pdl_enter(A, B, C);
   constexpr int BM = 64, BN = 64, BK = 16;
   __shared__ float As[BK][BM + 4], Bs[BK][BN + 4];
   A += (long long)blockIdx.z * sA;
@@ -110,6 +113,7 @@ template <typename TA, typename TB, typename TC, int MR>
 __global__ void __launch_bounds__(256) gemv_nt_kernel(const TA* __restrict__ A, long long lda, const TB* __restrict__ B, long long ldb,
                                                       TC* __restrict__ C, long long ldc, int M, int N, int K, long long sA,
                                                       long long sB, long long sC) {
+  kb2::pdl_enter(A, B, C);
   A += (long long)blockIdx.z * sA;
   B += (long long)blockIdx.z * sB;
   C += (long long)blockIdx.z * sC;
@@ -146,6 +150,7 @@ template <typename TA, typename TC, int MR, int CPW, int KS>
 __global__ void __launch_bounds__(256) gemv_nt_vec_kernel(const TA* __restrict__ A, long long lda, const bf16* __restrict__ B, long long ldb,
                                                           TC* __restrict__ C, long long ldc, int M, int N, int K, long long sA,
                                                           long long sB, long long sC) {
+  kb2::pdl_enter(A, B, C);
   A += (long long)blockIdx.z * sA;
   B += (long long)blockIdx.z * sB;
   C += (long long)blockIdx.z * sC;
@@ -222,7 +227,7 @@ static bool launch_gemv_vec(const void* A, long long lda, const void* B, long lo
   // Up to 4 rows run the 4-row instantiation (half the accumulators: more blocks per SM, more weight bytes in flight).
   const long long warps = (long long)N * batch;
 #define KB2_GEMV(MRV, CPWV, KSV, GX)                                                                                        \
-  gemv_nt_vec_kernel<TA, TC, MRV, CPWV, KSV><<<dim3(GX, 1, batch), 256, 0, s>>>((const TA*)A, lda, (const bf16*)B, ldb, (TC*)C, ldc, M, N, K, \
+  kb2::launch_pdl(gemv_nt_vec_kernel<TA, TC, MRV, CPWV, KSV>, dim3(GX, 1, batch), 256, 0, s, (const TA*)A, lda, (const bf16*)B, ldb, (TC*)C, ldc, M, N, K, \
                                                                                 sA, sB, sC)
   if (warps >= 4 * 8 * 296) {
     if (M <= 4) KB2_GEMV(4, 4, 1, (N + 31) / 32); else KB2_GEMV(8, 4, 1, (N + 31) / 32);
@@ -256,6 +261,7 @@ template <typename TC, int KS>
 __global__ void __launch_bounds__(KS > 8 ? 512 : 256) gemv_mma_kernel(const bf16* __restrict__ A, long long lda, const bf16* __restrict__ B, long long ldb,
                                                                       TC* __restrict__ C, long long ldc, int M, int N, int K, long long sA, long long sB,
                                                                       long long sC) {
+  kb2::pdl_enter(A, B, C);
   constexpr int kStep = 128, kWarps = KS > 8 ? 16 : 8, kGroups = kWarps / KS;
   __shared__ float red[kWarps][8][17];                   // [warp][row of A][weight row], odd pitch
   A += (long long)blockIdx.z * sA;
@@ -345,7 +351,7 @@ static bool launch_gemv_mma(const void* A, long long lda, const void* B, long lo
   const dim3 grid((groups + per - 1) / per, 1, batch);
 #define KB2_GEMV(KSV)                                                                                                                        \
   case KSV:                                                                                                                                  \
-    gemv_mma_kernel<TC, KSV><<<grid, KSV > 8 ? 512 : 256, 0, s>>>((const bf16*)A, lda, (const bf16*)B, ldb, (TC*)C, ldc, M, N, K, sA, sB, sC); \
+    kb2::launch_pdl(gemv_mma_kernel<TC, KSV>, grid, KSV > 8 ? 512 : 256, 0, s, (const bf16*)A, lda, (const bf16*)B, ldb, (TC*)C, ldc, M, N, K, sA, sB, sC); \
     break;
   switch (ks) { KB2_GEMV(1) KB2_GEMV(2) KB2_GEMV(4) KB2_GEMV(8) KB2_GEMV(16) }
 #undef KB2_GEMV
@@ -363,10 +369,10 @@ static void launch_gemm(const void* A, long long lda, const void* B, long long l
       if (launch_gemv_vec<TA, TC>(A, lda, B, ldb, C, ldc, M, N, K, batch, sA, sB, sC, s)) return;
     }
     dim3 grid((N + 7) / 8, 1, batch);
-    gemv_nt_kernel<TA, TB, TC, 8><<<grid, 256, 0, s>>>((const TA*)A, lda, (const TB*)B, ldb, (TC*)C, ldc, M, N, K, sA, sB, sC);
+    kb2::launch_pdl(gemv_nt_kernel<TA, TB, TC, 8>, grid, 256, 0, s, (const TA*)A, lda, (const TB*)B, ldb, (TC*)C, ldc, M, N, K, sA, sB, sC);
   } else {
     dim3 grid((N + 63) / 64, (M + 63) / 64, batch);
-    gemm_nt_kernel<TA, TB, TC><<<grid, 256, 0, s>>>((const TA*)A, lda, (const TB*)B, ldb, (TC*)C, ldc, M, N, K, sA, sB, sC);
+    kb2::launch_pdl(gemm_nt_kernel<TA, TB, TC>, grid, 256, 0, s, (const TA*)A, lda, (const TB*)B, ldb, (TC*)C, ldc, M, N, K, sA, sB, sC);
   }
 }
 
@@ -380,6 +386,7 @@ __global__ void __launch_bounds__(256) residual_norm_kernel(float* __restrict__ 
                                                             const float* __restrict__ x0, const float* __restrict__ wb,
                                                             const float* __restrict__ bb, void* __restrict__ h, int dt_h, int W,
                                                             float eps, const float* __restrict__ y2) {
+  kb2::pdl_enter(x, y, wa, ba, x0, wb, bb, h, y2);
   extern __shared__ float rowbuf[];
   __shared__ float red[32];
   const long long row = blockIdx.x;
@@ -458,6 +465,7 @@ __global__ void __launch_bounds__(256) residual_norm_vec_kernel(float* __restric
                                                                 const float* __restrict__ x0, const float* __restrict__ wb,
                                                                 const float* __restrict__ bb, void* __restrict__ h, int dt_h, int W, float eps,
                                                                 const float* __restrict__ y2) {
+  kb2::pdl_enter(x, y, wa, ba, x0, wb, bb, h, y2);
   __shared__ float red[4][8];
   const long long base = (long long)blockIdx.x * W;
   const int tid = threadIdx.x;
@@ -561,13 +569,13 @@ static int launch_residual_norm(float* x, const float* y, int y_mode, const floa
                                 const float* bb, void* h, int dt_h, int T, int W, float eps, const float* y2, cudaStream_t s) {
   const uintptr_t all = (uintptr_t)x | (uintptr_t)y | (uintptr_t)wa | (uintptr_t)ba | (uintptr_t)x0 | (uintptr_t)wb | (uintptr_t)bb | (uintptr_t)h | (uintptr_t)y2;
   if (W % 4 == 0 && W <= 8192 && !(all & 15)) {
-#define KB2_RN(NVV) residual_norm_vec_kernel<NVV><<<T, 256, 0, s>>>(x, y, y_mode, wa, ba, x0, wb, bb, h, dt_h, W, eps, y2)
+#define KB2_RN(NVV) kb2::launch_pdl(residual_norm_vec_kernel<NVV>, T, 256, 0, s, x, y, y_mode, wa, ba, x0, wb, bb, h, dt_h, W, eps, y2)
     if (W <= 1024) KB2_RN(1); else if (W <= 2048) KB2_RN(2); else if (W <= 4096) KB2_RN(4); else KB2_RN(8);
 #undef KB2_RN
   } else {
     const size_t smem = (size_t)W * 4;
     if (smem > 48 * 1024) SEQ_CUDA(cudaFuncSetAttribute(residual_norm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    residual_norm_kernel<<<T, 256, smem, s>>>(x, y, y_mode, wa, ba, x0, wb, bb, h, dt_h, W, eps, y2);
+    kb2::launch_pdl(residual_norm_kernel, T, 256, smem, s, x, y, y_mode, wa, ba, x0, wb, bb, h, dt_h, W, eps, y2);
   }
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
@@ -578,6 +586,7 @@ static int launch_residual_norm(float* x, const float* y, int y_mode, const floa
 __global__ void __launch_bounds__(256) residual_scale_rms_kernel(float* x, const float* __restrict__ y, float y_mult,
                                                                  const float* __restrict__ w, float w_shift, void* h, int dt_h, int W,
                                                                  float eps) {
+  kb2::pdl_enter(x, y, w, h);
   extern __shared__ float rowbuf[];
   __shared__ float red[32];
   const long long row = blockIdx.x;
@@ -606,6 +615,7 @@ __global__ void __launch_bounds__(256) residual_post_rms_kernel(float* __restric
                                                                 const float* __restrict__ y2, float c2, const float* __restrict__ bias,
                                                                 float mult, const float* __restrict__ w, const float* __restrict__ wh,
                                                                 void* __restrict__ h, int dt_h, int W, float eps) {
+  kb2::pdl_enter(x, y1, y2, bias, w, wh, h);
   extern __shared__ __align__(16) float rowbuf[];
   __shared__ float red[32];
   const long long base = (long long)blockIdx.x * W;
@@ -693,6 +703,7 @@ __global__ void __launch_bounds__(256) residual_post_rms_kernel(float* __restric
 
 // ------------------------------------------------------------------------------------------------ elementwise
 __global__ void act_mul_kernel(const void* __restrict__ in, int dt_in, void* __restrict__ out, int dt_out, long long T, int F) {
+  kb2::pdl_enter(in, out);
   const long long t = blockIdx.y;
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= F) return;
@@ -701,6 +712,7 @@ __global__ void act_mul_kernel(const void* __restrict__ in, int dt_in, void* __r
 }
 // bf16 in and out, F a multiple of 8: 16-byte accesses
 __global__ void act_mul_bf16x8_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, int F) {
+  kb2::pdl_enter(in, out);
   const long long t = blockIdx.y;
   const int f = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (f >= F) return;
@@ -716,6 +728,7 @@ __global__ void act_mul_bf16x8_kernel(const bf16* __restrict__ in, bf16* __restr
 
 __global__ void side_gate_kernel(const float* __restrict__ g, const void* __restrict__ table, int dt_table, long long table_ld,
                                  const int* __restrict__ tokens, int col0, int dim, long long T, void* __restrict__ out, int dt_out) {
+  kb2::pdl_enter(g, table, tokens, out);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= T * dim) return;
   const long long t = i / dim;
@@ -733,6 +746,7 @@ __global__ void __launch_bounds__(128) latent_prep_kernel(float* __restrict__ pr
                                                           const int* __restrict__ seq_of, const int* __restrict__ pages, int max_pages,
                                                           int page_size, void* __restrict__ ckv, void* __restrict__ kr, int dt_cache,
                                                           const float* __restrict__ lat_rows, long long ldl) {
+  kb2::pdl_enter(proj, cw, freq, positions, seq_of, pages, ckv, kr, lat_rows);
   __shared__ float red[32];
   const long long t = blockIdx.x;
   const int pos = positions[t];
@@ -790,6 +804,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) latent_window_attn_kernel(
     const int* __restrict__ seq_of, const int* __restrict__ pages, int max_pages, int page_size, const float* __restrict__ sinks,
     float scale, int window, float* __restrict__ out, const int* __restrict__ cu, int skip_from, int nsplit,
     float* __restrict__ part_acc, float* __restrict__ part_ml, const float* __restrict__ gate, long long ldg) {
+  kb2::pdl_enter(q_abs, proj, ckv, kr, positions, seq_of, pages, sinks, out, cu, part_acc, part_ml, gate);
   static_assert(HG <= kAttnWarps, "a warp per head runs the softmax");
   constexpr int KT = kAttnKT;
   extern __shared__ __align__(16) float sm[];
@@ -976,6 +991,7 @@ __global__ void __launch_bounds__(512) latent_attn_combine_kernel(const float* _
                                                                   int H, int r, int nsplit, float* __restrict__ out,
                                                                   const int* __restrict__ seq_of, const int* __restrict__ cu, int skip_from,
                                                                   const float* __restrict__ gate, long long ldg) {
+  kb2::pdl_enter(part_acc, part_ml, out, seq_of, cu, gate);
   extern __shared__ float wz[];           // [nsplit]
   __shared__ float red[32];
   const long long t = blockIdx.x;
@@ -1021,6 +1037,7 @@ __global__ void conv_silu_kernel(const float* __restrict__ proj, long long ldp, 
                                  const float* __restrict__ tail, const int* __restrict__ seq_of, const int* __restrict__ cu,
                                  const int* __restrict__ slots, long long T, float* __restrict__ out, const float* __restrict__ bias,
                                  int act, const float* __restrict__ bias_out) {
+  kb2::pdl_enter(proj, taps, tail, seq_of, cu, slots, out, bias, bias_out);
   const long long t = blockIdx.y;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
@@ -1046,6 +1063,7 @@ __global__ void __launch_bounds__(256) conv_run_kernel(const float* __restrict__
                                                        const int* __restrict__ seq_of, const int* __restrict__ cu,
                                                        const int* __restrict__ slots, long long T, float* __restrict__ out,
                                                        const float* __restrict__ bias, int act, const float* __restrict__ bias_out) {
+  kb2::pdl_enter(proj, taps, tail, seq_of, cu, slots, out, bias, bias_out);
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   const long long r0 = (long long)blockIdx.y * kConvRun, r1 = min(T, r0 + kConvRun);
@@ -1088,6 +1106,7 @@ __global__ void __launch_bounds__(256) conv_run_vec_kernel(const float* __restri
                                                            const float* __restrict__ tail, const int* __restrict__ seq_of, const int* __restrict__ cu,
                                                            const int* __restrict__ slots, long long T, float* __restrict__ out,
                                                            const float* __restrict__ bias, int act, const float* __restrict__ bias_out) {
+  kb2::pdl_enter(proj, taps, tail, seq_of, cu, slots, out, bias, bias_out);
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (c >= C) return;
   const long long r0 = (long long)blockIdx.y * kConvRun, r1 = min(T, r0 + kConvRun);
@@ -1144,6 +1163,7 @@ __global__ void __launch_bounds__(256) conv_run_vec_kernel(const float* __restri
 // after the convolution: the tail becomes the last K - 1 inputs seen so far (one thread per (sequence, channel), ascending order)
 __global__ void conv_tail_kernel(const float* __restrict__ proj, long long ldp, int C, int K, float* __restrict__ tail,
                                  const int* __restrict__ cu, const int* __restrict__ slots, int S, const float* __restrict__ bias) {
+  kb2::pdl_enter(proj, tail, cu, slots, bias);
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)S * C) return;
   const int s = (int)(idx / C), c = (int)(idx - (long long)s * C);
@@ -1169,6 +1189,7 @@ __global__ void __launch_bounds__(1024) delta_rule_kernel(const float* __restric
                                                           float* __restrict__ state, const int* __restrict__ cu,
                                                           const int* __restrict__ slots, void* __restrict__ out, int dt_out, int dvb,
                                                           float* __restrict__ o_raw) {
+  kb2::pdl_enter(conv, bproj, aproj, gproj, A_log, dt_bias, norm_w, state, cu, slots, out, o_raw);
   // dvb = value columns of this block (the columns of the state do not meet in the recurrence).  dvb < dv: blockIdx.z picks the slice,
   // the raw read-out goes to o_raw [T, H, dv] and the norm and gate are left to delta_out_kernel.
   extern __shared__ float sm[];
@@ -1262,6 +1283,7 @@ __global__ void __launch_bounds__(256) delta_prep_kernel(const float* __restrict
                                                          int Hk, int dk, const float* __restrict__ A_log,
                                                          const float* __restrict__ dt_bias, long long T, float* __restrict__ qn,
                                                          float* __restrict__ kn, float* __restrict__ beta, float* __restrict__ dec) {
+  kb2::pdl_enter(conv, bproj, aproj, A_log, dt_bias, qn, kn, beta, dec);
   const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (w >= T * Hk) return;
@@ -1317,6 +1339,7 @@ __global__ void __launch_bounds__(32 * kRegPieces) delta_rule_reg_kernel(const f
                                                                          int H, int Hk, int dv, float* __restrict__ state,
                                                                          const int* __restrict__ cu, const int* __restrict__ slots,
                                                                          float* __restrict__ o_out) {
+  kb2::pdl_enter(qn, kn, conv, beta, dec, state, cu, slots, o_out);
   constexpr int P = kRegPieces, NT = 32 * P;
   constexpr int Q = DK / P;                 // state rows per thread
   __shared__ __align__(16) float ks[2][kRegTile][DK];
@@ -1473,6 +1496,7 @@ __global__ void __launch_bounds__(256) delta_tile_prep_kernel(const float* __res
                                                               const float* __restrict__ A_log, const float* __restrict__ dt_bias, int S,
                                                               const int* __restrict__ cu, long long tiles, bf16* __restrict__ image,
                                                               float* __restrict__ sc) {
+  kb2::pdl_enter(conv, bproj, aproj, A_log, dt_bias, cu, image, sc);
   using D = DeltaTile<NI>;
   constexpr int DK = D::DK;
   const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -1614,6 +1638,7 @@ template <int NI>
 __global__ void __launch_bounds__(64 * NI + 32, 1) delta_tile_kernel(const bf16* __restrict__ image, const float* __restrict__ conv, int C, int v_col0,
                                                                      const float* __restrict__ sc, int H, int Hk, int dv, float* __restrict__ state,
                                                                      const int* __restrict__ cu, const int* __restrict__ slots, float* __restrict__ o_out) {
+  kb2::pdl_enter(image, conv, sc, state, cu, slots, o_out);
   using D = DeltaTile<NI>;
   extern __shared__ __align__(128) uint8_t tsm[];
   float* red = reinterpret_cast<float*>(tsm + kDTStages * D::kStageBytes);
@@ -1798,6 +1823,7 @@ template <int V>
 __global__ void __launch_bounds__(256) delta_out_kernel(const float* __restrict__ o, const float* __restrict__ gproj, long long ldg,
                                                         int gate_act, int H, int dv, const float* __restrict__ norm_w, float eps,
                                                         long long T, void* __restrict__ out, int dt_out) {
+  kb2::pdl_enter(o, gproj, norm_w, out);
   const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (w >= T * H) return;
@@ -1849,9 +1875,9 @@ KB2SEQ_API long long kb2_seq_total_launches(void) { return g_launches; }
 KB2SEQ_API int kb2_seq_embed(const void* table, int dt, const int* tokens, float* x, int T, int W, float scale, void* stream) {
   if (!table || !tokens || !x || T <= 0 || W <= 0 || bad_dt(dt)) return failf(KB2SEQ_ERR_VALUE, "embed: bad argument");
   if (dt && W % 8 == 0 && !((uintptr_t)table & 15) && !((uintptr_t)x & 15))
-    embed_scale_vec_kernel<<<T, 256, 0, (cudaStream_t)stream>>>((const bf16*)table, tokens, x, W, scale);
-  else if (dt) embed_scale_kernel<bf16><<<T, 128, 0, (cudaStream_t)stream>>>((const bf16*)table, tokens, x, W, scale);
-  else embed_scale_kernel<float><<<T, 128, 0, (cudaStream_t)stream>>>((const float*)table, tokens, x, W, scale);
+    kb2::launch_pdl(embed_scale_vec_kernel, T, 256, 0, (cudaStream_t)stream, (const bf16*)table, tokens, x, W, scale);
+  else if (dt) kb2::launch_pdl(embed_scale_kernel<bf16>, T, 128, 0, (cudaStream_t)stream, (const bf16*)table, tokens, x, W, scale);
+  else kb2::launch_pdl(embed_scale_kernel<float>, T, 128, 0, (cudaStream_t)stream, (const float*)table, tokens, x, W, scale);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
 }
@@ -1901,9 +1927,9 @@ KB2SEQ_API int kb2_seq_act_mul(const void* in, int dt_in, void* out, int dt_out,
   if (!in || !out || T <= 0 || F <= 0 || bad_dt(dt_in) || bad_dt(dt_out)) return failf(KB2SEQ_ERR_VALUE, "act_mul: bad argument");
   if (T > 65535) return failf(KB2SEQ_ERR_VALUE, "act_mul: more than 65535 rows in one step");
   if (dt_in == 1 && dt_out == 1 && F % 8 == 0 && !((uintptr_t)in & 15) && !((uintptr_t)out & 15))
-    act_mul_bf16x8_kernel<<<dim3((F / 8 + 127) / 128, T), 128, 0, (cudaStream_t)stream>>>((const bf16*)in, (bf16*)out, F);
+    kb2::launch_pdl(act_mul_bf16x8_kernel, dim3((F / 8 + 127) / 128, T), 128, 0, (cudaStream_t)stream, (const bf16*)in, (bf16*)out, F);
   else
-    act_mul_kernel<<<dim3((F + 255) / 256, T), 256, 0, (cudaStream_t)stream>>>(in, dt_in, out, dt_out, T, F);
+    kb2::launch_pdl(act_mul_kernel, dim3((F + 255) / 256, T), 256, 0, (cudaStream_t)stream, in, dt_in, out, dt_out, T, F);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
 }
@@ -1913,7 +1939,7 @@ KB2SEQ_API int kb2_seq_side_gate(const float* g, const void* table, int dt_table
   if (!g || !table || !tokens || !out || T <= 0 || dim <= 0 || col0 < 0 || bad_dt(dt_table) || bad_dt(dt_out))
     return failf(KB2SEQ_ERR_VALUE, "side_gate: bad argument");
   const long long n = (long long)T * dim;
-  side_gate_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(g, table, dt_table, table_ld, tokens, col0, dim, T, out,
+  kb2::launch_pdl(side_gate_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, g, table, dt_table, table_ld, tokens, col0, dim, T, out,
                                                                                   dt_out);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
@@ -1926,7 +1952,7 @@ KB2SEQ_API int kb2_seq_latent_prep(float* proj, long long ldp, int T, int H, int
   if (!proj || !cw || !freq || !positions || !seq_of || !pages || !ckv || !kr || T <= 0 || H <= 0 || dn < 0 || dr < 0 || r <= 0 ||
       rot_dims < 0 || rot_dims > dr || (rot_dims & 1) || page_size <= 0 || max_pages <= 0 || bad_dt(dt_cache))
     return failf(KB2SEQ_ERR_VALUE, "latent_prep: bad argument");
-  latent_prep_kernel<<<T, 128, 0, (cudaStream_t)stream>>>(proj, ldp, H, dn, dr, r, cw, eps, freq, rot_dims, amp, positions, seq_of, pages,
+  kb2::launch_pdl(latent_prep_kernel, T, 128, 0, (cudaStream_t)stream, proj, ldp, H, dn, dr, r, cw, eps, freq, rot_dims, amp, positions, seq_of, pages,
                                                           max_pages, page_size, ckv, kr, dt_cache, lat, ldl);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
@@ -1954,7 +1980,7 @@ KB2SEQ_API int kb2_seq_latent_window_attn(const float* q_abs, const float* proj,
   case HGV * 32 + NCV: {                                                                                                                      \
     if (smem > 48 * 1024)                                                                                                                     \
       SEQ_CUDA(cudaFuncSetAttribute(latent_window_attn_kernel<HGV, NCV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));            \
-    latent_window_attn_kernel<HGV, NCV><<<grid, kAttnThreads, smem, (cudaStream_t)stream>>>(                                                   \
+    kb2::launch_pdl(latent_window_attn_kernel<HGV, NCV>, grid, kAttnThreads, smem, (cudaStream_t)stream,                                                    \
         q_abs, proj, ldp, H, dn, dr, r, ckv, kr, dt_cache, positions, seq_of, pages, max_pages, page_size, sinks, scale, window, out, cu,     \
         skip_from, nsplit, part_acc, part_ml, gate, ldg);                                                                                     \
     break;                                                                                                                                    \
@@ -1967,7 +1993,7 @@ KB2SEQ_API int kb2_seq_latent_window_attn(const float* q_abs, const float* proj,
 #undef KB2_LA
   SEQ_LAUNCHED();
   if (nsplit > 1) {
-    latent_attn_combine_kernel<<<dim3(T, H), r >= 512 ? 512 : (r + 31) / 32 * 32, (size_t)nsplit * 4, (cudaStream_t)stream>>>(part_acc, part_ml, H, r, nsplit, out, seq_of, cu, skip_from,
+    kb2::launch_pdl(latent_attn_combine_kernel, dim3(T, H), r >= 512 ? 512 : (r + 31) / 32 * 32, (size_t)nsplit * 4, (cudaStream_t)stream, part_acc, part_ml, H, r, nsplit, out, seq_of, cu, skip_from,
                                                                                                gate, ldg);
     SEQ_LAUNCHED();
   }
@@ -1982,20 +2008,20 @@ KB2SEQ_API int kb2_seq_conv(const float* proj, long long ldp, int T, int S, int 
   if (T > 65535) return failf(KB2SEQ_ERR_VALUE, "conv: more than 65535 rows in one step");
   const bool vec = C % 4 == 0 && ldp % 4 == 0 && !(((uintptr_t)proj | (uintptr_t)out) & 15);
   const dim3 vgrid((C / 4 + 255) / 256, (T + kConvRun - 1) / kConvRun);
-#define KB2_CONV(KV) conv_run_vec_kernel<KV><<<vgrid, 256, 0, (cudaStream_t)stream>>>(proj, ldp, C, taps, tail, seq_of, cu, slots, T, out, bias, act, bias_out)
+#define KB2_CONV(KV) kb2::launch_pdl(conv_run_vec_kernel<KV>, vgrid, 256, 0, (cudaStream_t)stream, proj, ldp, C, taps, tail, seq_of, cu, slots, T, out, bias, act, bias_out)
   if (T >= 4 * kConvRun && vec && K >= 2 && K <= 4) {
     if (K == 2) KB2_CONV(2); else if (K == 3) KB2_CONV(3); else KB2_CONV(4);
   } else if (T >= 4 * kConvRun && K <= kConvMaxTaps)
-    conv_run_kernel<<<dim3((C + 255) / 256, (T + kConvRun - 1) / kConvRun), 256, 0, (cudaStream_t)stream>>>(proj, ldp, C, K, taps, tail, seq_of,
+    kb2::launch_pdl(conv_run_kernel, dim3((C + 255) / 256, (T + kConvRun - 1) / kConvRun), 256, 0, (cudaStream_t)stream, proj, ldp, C, K, taps, tail, seq_of,
                                                                                                           cu, slots, T, out, bias, act, bias_out);
   else
-    conv_silu_kernel<<<dim3((C + 255) / 256, T), 256, 0, (cudaStream_t)stream>>>(proj, ldp, C, K, taps, tail, seq_of, cu, slots, T, out, bias,
+    kb2::launch_pdl(conv_silu_kernel, dim3((C + 255) / 256, T), 256, 0, (cudaStream_t)stream, proj, ldp, C, K, taps, tail, seq_of, cu, slots, T, out, bias,
                                                                                  act, bias_out);
 #undef KB2_CONV
   SEQ_LAUNCHED();
   if (K > 1) {
     const long long m = (long long)S * C;
-    conv_tail_kernel<<<(unsigned)((m + 255) / 256), 256, 0, (cudaStream_t)stream>>>(proj, ldp, C, K, tail, cu, slots, S, bias);
+    kb2::launch_pdl(conv_tail_kernel, (unsigned)((m + 255) / 256), 256, 0, (cudaStream_t)stream, proj, ldp, C, K, tail, cu, slots, S, bias);
     SEQ_LAUNCHED();
   }
   return KB2SEQ_OK;
@@ -2013,7 +2039,7 @@ KB2SEQ_API int kb2_seq_residual_scale_rms(float* x, const float* y, float y_mult
   const size_t smem = (size_t)W * 4;
   if (smem > 200 * 1024) return failf(KB2SEQ_ERR_VALUE, "residual_scale_rms: width %d too large", W);
   if (smem > 48 * 1024) SEQ_CUDA(cudaFuncSetAttribute(residual_scale_rms_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  residual_scale_rms_kernel<<<T, 256, smem, (cudaStream_t)stream>>>(x, y, y_mult, w, w_shift, h, dt_h, W, eps);
+  kb2::launch_pdl(residual_scale_rms_kernel, T, 256, smem, (cudaStream_t)stream, x, y, y_mult, w, w_shift, h, dt_h, W, eps);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
 }
@@ -2027,10 +2053,10 @@ KB2SEQ_API int kb2_seq_residual_post_rms(float* x, const float* y1, float c1, co
   const uintptr_t all = (uintptr_t)x | (uintptr_t)y1 | (uintptr_t)y2 | (uintptr_t)bias | (uintptr_t)w | (uintptr_t)wh | (uintptr_t)h;
   if (W % 4 == 0 && !(all & 15)) {
     if (smem > 40 * 1024) SEQ_CUDA(cudaFuncSetAttribute(residual_post_rms_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    residual_post_rms_kernel<4><<<T, 256, smem, (cudaStream_t)stream>>>(x, y1, c1, y2, c2, bias, mult, w, wh, h, dt_h, W, eps);
+    kb2::launch_pdl(residual_post_rms_kernel<4>, T, 256, smem, (cudaStream_t)stream, x, y1, c1, y2, c2, bias, mult, w, wh, h, dt_h, W, eps);
   } else {
     if (smem > 40 * 1024) SEQ_CUDA(cudaFuncSetAttribute(residual_post_rms_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    residual_post_rms_kernel<1><<<T, 256, smem, (cudaStream_t)stream>>>(x, y1, c1, y2, c2, bias, mult, w, wh, h, dt_h, W, eps);
+    kb2::launch_pdl(residual_post_rms_kernel<1>, T, 256, smem, (cudaStream_t)stream, x, y1, c1, y2, c2, bias, mult, w, wh, h, dt_h, W, eps);
   }
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
@@ -2040,9 +2066,9 @@ static int delta_out_launch(const float* o, const float* gproj, long long ldg, i
                             void* out, int dt_out, cudaStream_t st) {
   const unsigned blocks = (unsigned)(((long long)T * H + 7) / 8);
   if (dv % 4 == 0 && ldg % 4 == 0 && !(((uintptr_t)o | (uintptr_t)gproj | (uintptr_t)norm_w | (uintptr_t)out) & 15))
-    delta_out_kernel<4><<<blocks, 256, 0, st>>>(o, gproj, ldg, gate_act, H, dv, norm_w, eps, T, out, dt_out);
+    kb2::launch_pdl(delta_out_kernel<4>, blocks, 256, 0, st, o, gproj, ldg, gate_act, H, dv, norm_w, eps, T, out, dt_out);
   else
-    delta_out_kernel<1><<<blocks, 256, 0, st>>>(o, gproj, ldg, gate_act, H, dv, norm_w, eps, T, out, dt_out);
+    kb2::launch_pdl(delta_out_kernel<1>, blocks, 256, 0, st, o, gproj, ldg, gate_act, H, dv, norm_w, eps, T, out, dt_out);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
 }
@@ -2065,11 +2091,11 @@ static int delta_rule_launch(const float* conv, int C, const float* bproj, long 
     float* ob = de + (long long)T * H * (ch ? dk : 1);
     ob = (float*)(((uintptr_t)ob + 15) & ~(uintptr_t)15);
     const long long nw = (long long)T * Hk;
-    delta_prep_kernel<<<(unsigned)((nw + 7) / 8), 256, 0, st>>>(conv, C, bproj, ldb, aproj, lda, ch, H, Hk, dk, A_log, dt_bias, T, qn, kn, be, de);
+    kb2::launch_pdl(delta_prep_kernel, (unsigned)((nw + 7) / 8), 256, 0, st, conv, C, bproj, ldb, aproj, lda, ch, H, Hk, dk, A_log, dt_bias, T, qn, kn, be, de);
     SEQ_LAUNCHED();
     dim3 grid(S, H, dv / 32);
     const int v_col0 = 2 * Hk * dk;
-#define R(DK, CHV) delta_rule_reg_kernel<DK, CHV><<<grid, 32 * kRegPieces, 0, st>>>(qn, kn, conv, C, v_col0, be, de, H, Hk, dv, state, cu, slots, ob)
+#define R(DK, CHV) kb2::launch_pdl(delta_rule_reg_kernel<DK, CHV>, grid, 32 * kRegPieces, 0, st, qn, kn, conv, C, v_col0, be, de, H, Hk, dv, state, cu, slots, ob)
     if (ch) {
       if (dk == 32) R(32, true); else if (dk == 64) R(64, true); else R(128, true);
     } else {
@@ -2094,7 +2120,7 @@ static int delta_rule_launch(const float* conv, int C, const float* bproj, long 
   if (threads < 128) threads = 128;
   const bool cut = dvb < dv;
   dim3 grid(S, H, (dv + dvb - 1) / dvb);
-  delta_rule_kernel<<<grid, threads, smem, (cudaStream_t)stream>>>(conv, C, bproj, ldb, aproj, lda, ch, gproj, ldg, gate_act, H, Hk, dk, dv, A_log,
+  kb2::launch_pdl(delta_rule_kernel, grid, threads, smem, (cudaStream_t)stream, conv, C, bproj, ldb, aproj, lda, ch, gproj, ldg, gate_act, H, Hk, dk, dv, A_log,
                                                                   dt_bias, norm_w, eps, state, cu, slots, out, dt_out, dvb,
                                                                   cut ? scratch : nullptr);
   SEQ_LAUNCHED();
@@ -2126,9 +2152,9 @@ KB2SEQ_API int kb2_seq_delta_tiles(const float* conv, int C, const float* proj, 
 #define KB2_DT(NIV)                                                                                                                                   \
   do {                                                                                                                                                \
     SEQ_CUDA(cudaFuncSetAttribute(delta_tile_kernel<NIV>, cudaFuncAttributeMaxDynamicSharedMemorySize, DeltaTile<NIV>::kSmem));                        \
-    delta_tile_prep_kernel<NIV><<<blocks, 256, 0, st>>>(conv, C, proj + b_off, ldp, proj + a_off, ldp, H, Hk, A_log, dt_bias, S, cu, tiles, image, sc); \
+    kb2::launch_pdl(delta_tile_prep_kernel<NIV>, blocks, 256, 0, st, conv, C, proj + b_off, ldp, proj + a_off, ldp, H, Hk, A_log, dt_bias, S, cu, tiles, image, sc); \
     SEQ_LAUNCHED();                                                                                                                                   \
-    delta_tile_kernel<NIV><<<grid, 64 * NIV + 32, DeltaTile<NIV>::kSmem, st>>>(image, conv, C, 2 * Hk * dk, sc, H, Hk, dv, state, cu, slots, ob);        \
+    kb2::launch_pdl(delta_tile_kernel<NIV>, grid, 64 * NIV + 32, DeltaTile<NIV>::kSmem, st, image, conv, C, 2 * Hk * dk, sc, H, Hk, dv, state, cu, slots, ob);        \
     SEQ_LAUNCHED();                                                                                                                                   \
   } while (0)
   if (dk == 32) KB2_DT(1); else if (dk == 64) KB2_DT(2); else KB2_DT(4);

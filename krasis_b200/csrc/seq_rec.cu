@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(kRecThreads) gla_scan_kernel(const float* __re
                                                                const float* __restrict__ decay_bias, float inv_tau, float q_scale, int H,
                                                                int dk, int dv, int P, float* __restrict__ state, const int* __restrict__ cu,
                                                                const int* __restrict__ slots, float* __restrict__ out, MemoryGates mg) {
+  kb2::pdl_enter(qkv, decay_in, decay_bias, state, cu, slots, out);
   extern __shared__ __align__(16) float sm[];
   float4* akq = reinterpret_cast<float4*>(sm);              // [kRecTok][dk]
   const int CW = 32 / P, CB = (kRecThreads / 32) * CW;
@@ -129,6 +130,7 @@ __global__ void __launch_bounds__(kRecThreads) gla_scan_kernel(const float* __re
 // from the decays that gla_decay_kernel wrote; the warps' pieces of S^T q meet in shared memory once per tile.  No barrier inside a token.
 __global__ void gla_decay_kernel(const float* __restrict__ decay_in, long long lda, const float* __restrict__ decay_bias, float inv_tau,
                                  long long T, int n, float* __restrict__ alpha) {
+  kb2::pdl_enter(decay_in, decay_bias, alpha);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= T * n) return;
   const long long t = i / n;
@@ -152,6 +154,7 @@ __global__ void __launch_bounds__(32 * kGlaWarps) gla_reg_kernel(const float* __
                                                                  const float* __restrict__ alpha, float q_scale, int H, int dv,
                                                                  float* __restrict__ state, const int* __restrict__ cu,
                                                                  const int* __restrict__ slots, float* __restrict__ out) {
+  kb2::pdl_enter(qkv, alpha, state, cu, slots, out);
   constexpr int P = kGlaWarps, NT = 32 * P, Q = DK / P;
   extern __shared__ __align__(16) float sm[];
   float* as = sm;                                   // [2][kGlaTile][DK]
@@ -238,6 +241,7 @@ __global__ void __launch_bounds__(kGateThreads) mlstm_gates_kernel(const float* 
                                                                    int H, float* __restrict__ mstate, const int* __restrict__ cu,
                                                                    const int* __restrict__ slots, float* __restrict__ keep,
                                                                    float* __restrict__ add, float* __restrict__ mx) {
+  kb2::pdl_enter(proj, i_bias, f_bias, mstate, cu, slots, keep, add, mx);
   __shared__ double wF[32], wM[32];
   __shared__ float ms[kGateThreads + 1];             // ms[1 + k]: m of the tile's token k, ms[0]: m before the tile
   const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -343,6 +347,7 @@ __global__ void __launch_bounds__(32 * (kMemWarps + 1), 1) mlstm_reg_kernel(cons
                                                                    float q_scale, int H, int dv, float* __restrict__ state,
                                                                    const int* __restrict__ cu, const int* __restrict__ slots,
                                                                    float* __restrict__ out, MemoryGates mg) {
+  kb2::pdl_enter(qkv, state, cu, slots, out);
   using M = MemShape<DK>;
   constexpr int P = kMemWarps, NT = 32 * (P + 1), Q = M::Q, R = M::R, CPL = M::CPL, RG = M::RG, NP = P * RG, KR = DK / 32;
   extern __shared__ __align__(16) float sm[];
@@ -528,6 +533,7 @@ __global__ void __launch_bounds__(32 * NW * CG, 1) rglru_scan_kernel(const float
                                                                    const float* __restrict__ y_bias, const float* __restrict__ rate_c, int C, int bs,
                                                                    float* __restrict__ state, const int* __restrict__ cu,
                                                                    const int* __restrict__ slots, void* __restrict__ out, int dt_out) {
+  kb2::pdl_enter(u, z, y, r_bias, i_bias, y_bias, rate_c, state, cu, slots, out);
   __shared__ float Aw[2][CG][NW][32], Bw[2][CG][NW][32];
   const int s = blockIdx.x, lane = threadIdx.x & 31, grp = (threadIdx.x >> 5) / NW, warp = (threadIdx.x >> 5) % NW;
   const int c = (blockIdx.y * CG + grp) * 32 + lane;
@@ -602,6 +608,7 @@ __global__ void __launch_bounds__(32 * NW * CG, 1) rglru_scan_kernel(const float
 // u [T, ldu] fp32 -> out [blocks][Tp][2 bs] bf16: row (b, t) holds the channels of block b as [high | low], high + low = u up to 2^-17 |u|
 __global__ void __launch_bounds__(256) split_blocks_kernel(const float* __restrict__ u, long long ldu, long long T, long long Tp, int blocks, int bs,
                                                            bf16* __restrict__ out) {
+  kb2::pdl_enter(u, out);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;     // a pair of channels
   const int half = bs >> 1;
   if (i >= T * blocks * half) return;
@@ -638,6 +645,7 @@ __global__ void __launch_bounds__(kRecThreads) selective_scan_kernel(const float
                                                                      const float* __restrict__ A_log, const float* __restrict__ Dw, int inner,
                                                                      int N, int P, float* __restrict__ state, const int* __restrict__ cu,
                                                                      const int* __restrict__ slots, void* __restrict__ out, int dt_out) {
+  kb2::pdl_enter(x, dt_in, dt_bias, bc, z, A_log, Dw, state, cu, slots, out);
   extern __shared__ __align__(16) float sm[];
   const int CW = 32 / P, CB = (kRecThreads / 32) * CW;
   float* bcs = sm;                                   // [2][kRecTok][2 N]: B | C of the token
@@ -740,6 +748,7 @@ __global__ void __launch_bounds__(256) head_norm_gate_kernel(const float* __rest
                                                              const float* __restrict__ gate, long long ldg, int gate_act, int H, int dv,
                                                              long long T, void* __restrict__ out, int dt_out,
                                                              const float* __restrict__ den, int w_heads) {
+  kb2::pdl_enter(o, w, gate, out, den);
   const long long wi = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (wi >= T * H) return;
@@ -775,6 +784,7 @@ __global__ void __launch_bounds__(256) head_norm_gate_vec_kernel(const float* __
                                                                  const float* __restrict__ gate, long long ldg, int gate_act, int H, int dv,
                                                                  long long T, void* __restrict__ out, int dt_out, const float* __restrict__ den,
                                                                  int w_heads) {
+  kb2::pdl_enter(o, w, gate, out, den);
   const long long wi = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (wi >= T * H) return;
@@ -832,6 +842,7 @@ __global__ void __launch_bounds__(256) head_norm_gate_vec_kernel(const float* __
 // out[t, :n] = in[t, :n] / rms * w; a block per row
 __global__ void __launch_bounds__(256) rms_rows_kernel(const float* __restrict__ in, long long ld_in, int n, const float* __restrict__ w,
                                                        float eps, void* __restrict__ out, int dt_out, long long ld_out) {
+  kb2::pdl_enter(in, w, out);
   __shared__ float red[32];
   const long long t = blockIdx.x;
   const float* r = in + t * ld_in;
@@ -845,6 +856,7 @@ __global__ void __launch_bounds__(256) rms_rows_kernel(const float* __restrict__
 // out[t] = coef (a[t] / rms(a[t]) * wa + b[t] / rms(b[t]) * wb)
 __global__ void __launch_bounds__(256) branch_merge_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ wa,
                                                            const float* __restrict__ wb, float eps, float coef, float* __restrict__ out, int W) {
+  kb2::pdl_enter(a, b, wa, wb, out);
   __shared__ float red[32];
   const long long t = blockIdx.x;
   const float* ra = a + t * W;
@@ -865,6 +877,7 @@ __global__ void __launch_bounds__(256) branch_merge_kernel(const float* __restri
 __global__ void __launch_bounds__(256) depth_mix_kernel(float* __restrict__ stack, long long stride, int n, const float* __restrict__ coef,
                                                         float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ w,
                                                         void* __restrict__ h, int dt_h, int W, float eps) {
+  kb2::pdl_enter(stack, coef, x, y, w, h);
   __shared__ float red[32];
   const long long t = blockIdx.x;
   float* xr = x + t * W;
@@ -909,6 +922,7 @@ __global__ void __launch_bounds__(256) stream_mix_kernel(float* __restrict__ xs,
                                                          const float* __restrict__ out, const float* __restrict__ read,
                                                          const float* __restrict__ w, float w_shift, void* __restrict__ h, int dt_h, int W,
                                                          float eps) {
+  kb2::pdl_enter(xs, x0, y, mix, out, read, w, h);
   constexpr int N = NS > 0 ? NS : kMaxStreams, U = NS > 0 ? NS : 1;      // the generic form keeps its loops over the copies rolled
   extern __shared__ __align__(16) float u_row[];           // [W]
   __shared__ float cm[N * N], co[N], cr[N], red[32];
@@ -1018,10 +1032,10 @@ static int launch_gla_scan(const float* qkv, long long ld, int q_off, int k_off,
     SEQ_CUDA(cudaFuncSetAttribute(gla_scan_kernel<16, SC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   }
   if (KR <= 16)
-    gla_scan_kernel<16, SC><<<grid, kRecThreads, smem, st>>>(qkv, ld, q_off, k_off, v_off, decay_in, lda, decay_bias, inv_tau, q_scale, H, dk, dv,
+    kb2::launch_pdl(gla_scan_kernel<16, SC>, grid, kRecThreads, smem, st, qkv, ld, q_off, k_off, v_off, decay_in, lda, decay_bias, inv_tau, q_scale, H, dk, dv,
                                                              P, state, cu, slots, out, mg);
   else
-    gla_scan_kernel<32, SC><<<grid, kRecThreads, smem, st>>>(qkv, ld, q_off, k_off, v_off, decay_in, lda, decay_bias, inv_tau, q_scale, H, dk, dv,
+    kb2::launch_pdl(gla_scan_kernel<32, SC>, grid, kRecThreads, smem, st, qkv, ld, q_off, k_off, v_off, decay_in, lda, decay_bias, inv_tau, q_scale, H, dk, dv,
                                                              P, state, cu, slots, out, mg);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
@@ -1032,7 +1046,7 @@ static int launch_mlstm_reg(const float* qkv, long long ld, int q_off, int k_off
                             const int* cu, const int* slots, float* out, const MemoryGates& mg, cudaStream_t st) {
   const size_t smem = (size_t)MemShape<DK>::kFloats * 4;
   if (smem > 48 * 1024) SEQ_CUDA(cudaFuncSetAttribute(mlstm_reg_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  mlstm_reg_kernel<DK><<<dim3(S, H, dv / 32), 32 * (kMemWarps + 1), smem, st>>>(qkv, ld, q_off, k_off, v_off, q_scale, H, dv, state, cu, slots, out, mg);
+  kb2::launch_pdl(mlstm_reg_kernel<DK>, dim3(S, H, dv / 32), 32 * (kMemWarps + 1), smem, st, qkv, ld, q_off, k_off, v_off, q_scale, H, dv, state, cu, slots, out, mg);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
 }
@@ -1042,7 +1056,7 @@ static int launch_gla_reg(const float* qkv, long long ld, int q_off, int k_off, 
                           int dv, float* state, const int* cu, const int* slots, float* out, cudaStream_t st) {
   const size_t smem = (size_t)(3 * 2 * kGlaTile * DK + 2 * kGlaTile * 32 + kGlaTile * kGlaWarps * 32) * 4;
   if (smem > 48 * 1024) SEQ_CUDA(cudaFuncSetAttribute(gla_reg_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  gla_reg_kernel<DK><<<dim3(S, H, dv / 32), 32 * kGlaWarps, smem, st>>>(qkv, ld, q_off, k_off, v_off, alpha, q_scale, H, dv, state, cu, slots, out);
+  kb2::launch_pdl(gla_reg_kernel<DK>, dim3(S, H, dv / 32), 32 * kGlaWarps, smem, st, qkv, ld, q_off, k_off, v_off, alpha, q_scale, H, dv, state, cu, slots, out);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
 }
@@ -1065,7 +1079,7 @@ KB2SEQ_API int kb2_seq_gla(const float* qkv, long long ld, int q_off, int k_off,
   if (aligned && (dk == 32 || dk == 64 || dk == 128 || dk == 256) && dv % 32 == 0 && dv / 32 <= 65535) {
     cudaStream_t st0 = (cudaStream_t)stream;
     const long long ne = (long long)T * H * dk;
-    gla_decay_kernel<<<(unsigned)((ne + 255) / 256), 256, 0, st0>>>(decay_in, lda, decay_bias, 1.f / tau, T, H * dk, scratch);
+    kb2::launch_pdl(gla_decay_kernel, (unsigned)((ne + 255) / 256), 256, 0, st0, decay_in, lda, decay_bias, 1.f / tau, T, H * dk, scratch);
     SEQ_LAUNCHED();
     if (dk == 32) return launch_gla_reg<32>(qkv, ld, q_off, k_off, v_off, scratch, q_scale, S, H, dv, state, cu, slots, out, st0);
     if (dk == 64) return launch_gla_reg<64>(qkv, ld, q_off, k_off, v_off, scratch, q_scale, S, H, dv, state, cu, slots, out, st0);
@@ -1089,7 +1103,7 @@ KB2SEQ_API int kb2_seq_mlstm(const float* proj, long long ld, int q_off, int k_o
   float* add = keep + (long long)T * H;
   float* mx = add + (long long)T * H;
   const int threads = T >= kGateThreads ? kGateThreads : (T + 31) / 32 * 32;
-  mlstm_gates_kernel<<<dim3(S, H), threads, 0, st>>>(proj, ld, i_off, f_off, i_bias, f_bias, cap, H, mstate, cu, slots, keep, add, mx);
+  kb2::launch_pdl(mlstm_gates_kernel, dim3(S, H), threads, 0, st, proj, ld, i_off, f_off, i_bias, f_bias, cap, H, mstate, cu, slots, keep, add, mx);
   SEQ_LAUNCHED();
   const MemoryGates mg{keep, add, mx, nstate, den};
   const bool aligned = (((uintptr_t)proj | (uintptr_t)state) & 15) == 0 && (ld & 3) == 0 && (q_off & 3) == 0 && (k_off & 3) == 0 &&
@@ -1113,10 +1127,10 @@ KB2SEQ_API int kb2_seq_rglru(const float* u, long long ldu, const float* z, long
   if ((C + 31) / 32 > 65535) return failf(KB2SEQ_ERR_VALUE, "rglru: too many channels");
   const int groups = (C + 31) / 32;
   if (T - S + 1 <= 2)                                  // no portion is longer than two tokens
-    rglru_scan_kernel<1, kRgGroups, 2><<<dim3(S, (groups + kRgGroups - 1) / kRgGroups), 32 * kRgGroups, 0, (cudaStream_t)stream>>>(
+    kb2::launch_pdl(rglru_scan_kernel<1, kRgGroups, 2>, dim3(S, (groups + kRgGroups - 1) / kRgGroups), 32 * kRgGroups, 0, (cudaStream_t)stream, 
         u, ldu, z, ldz, zb, y, ldy, r_bias, i_bias, y_bias, rate, C, bs, state, cu, slots, out, dt_out);
   else
-    rglru_scan_kernel<kRgWarps, 1, kRgTok><<<dim3(S, groups), 32 * kRgWarps, 0, (cudaStream_t)stream>>>(
+    kb2::launch_pdl(rglru_scan_kernel<kRgWarps, 1, kRgTok>, dim3(S, groups), 32 * kRgWarps, 0, (cudaStream_t)stream, 
         u, ldu, z, ldz, zb, y, ldy, r_bias, i_bias, y_bias, rate, C, bs, state, cu, slots, out, dt_out);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
@@ -1125,7 +1139,7 @@ KB2SEQ_API int kb2_seq_rglru(const float* u, long long ldu, const float* z, long
 KB2SEQ_API int kb2_seq_split_blocks(const float* u, long long ldu, int T, int T_pad, int blocks, int bs, void* out, void* stream) {
   if (!u || !out || T <= 0 || T_pad < T || blocks <= 0 || bs <= 0 || (bs & 1)) return failf(KB2SEQ_ERR_VALUE, "split_blocks: bad argument");
   const long long n = (long long)T * blocks * (bs / 2);
-  split_blocks_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(u, ldu, T, T_pad, blocks, bs, (bf16*)out);
+  kb2::launch_pdl(split_blocks_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, u, ldu, T, T_pad, blocks, bs, (bf16*)out);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
 }
@@ -1146,7 +1160,7 @@ KB2SEQ_API int kb2_seq_selective_scan(const float* x, long long ldx, const float
   cudaStream_t st = (cudaStream_t)stream;
 #define KB2_SCAN(NRV)                                                                                                                  \
   if (smem > 48 * 1024) SEQ_CUDA(cudaFuncSetAttribute(selective_scan_kernel<NRV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-  selective_scan_kernel<NRV><<<grid, kRecThreads, smem, st>>>(x, ldx, dt_in, ldd, dt_bias, bc, ldb, b_off, z, ldz, z_off, A_log, D, inner, N, \
+  kb2::launch_pdl(selective_scan_kernel<NRV>, grid, kRecThreads, smem, st, x, ldx, dt_in, ldd, dt_bias, bc, ldb, b_off, z, ldz, z_off, A_log, D, inner, N, \
                                                               P, state, cu, slots, out, dt_out)
   if (NR == 1) { KB2_SCAN(1); } else if (NR == 2) { KB2_SCAN(2); } else if (NR == 4) { KB2_SCAN(4); } else { KB2_SCAN(8); }
 #undef KB2_SCAN
@@ -1162,14 +1176,14 @@ KB2SEQ_API int kb2_seq_head_norm_gate(const float* o, long long ldo, const float
   const uintptr_t all = (uintptr_t)o | (uintptr_t)w | (uintptr_t)gate | (uintptr_t)out;
   if (dv % 4 == 0 && dv <= 512 && ldo % 4 == 0 && ldg % 4 == 0 && !(all & 15)) {
 #define KB2_HN(NV)                                                                                                                          \
-  head_norm_gate_vec_kernel<NV><<<(unsigned)((nw + 7) / 8), 256, 0, (cudaStream_t)stream>>>(o, ldo, w, eps, gate, ldg, gate_act, H, dv, T, out, dt_out, \
+  kb2::launch_pdl(head_norm_gate_vec_kernel<NV>, (unsigned)((nw + 7) / 8), 256, 0, (cudaStream_t)stream, o, ldo, w, eps, gate, ldg, gate_act, H, dv, T, out, dt_out, \
                                                                                            den, w_heads)
     if (dv <= 128) KB2_HN(1); else if (dv <= 256) KB2_HN(2); else KB2_HN(4);
 #undef KB2_HN
     SEQ_LAUNCHED();
     return KB2SEQ_OK;
   }
-  head_norm_gate_kernel<<<(unsigned)((nw + 7) / 8), 256, 0, (cudaStream_t)stream>>>(o, ldo, w, eps, gate, ldg, gate_act, H, dv, T, out, dt_out, den,
+  kb2::launch_pdl(head_norm_gate_kernel, (unsigned)((nw + 7) / 8), 256, 0, (cudaStream_t)stream, o, ldo, w, eps, gate, ldg, gate_act, H, dv, T, out, dt_out, den,
                                                                                       w_heads);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
@@ -1178,7 +1192,7 @@ KB2SEQ_API int kb2_seq_head_norm_gate(const float* o, long long ldo, const float
 KB2SEQ_API int kb2_seq_rms_rows(const float* in, long long ld_in, int n, const float* w, float eps, void* out, int dt_out, long long ld_out,
                                 int T, void* stream) {
   if (!in || !w || !out || T <= 0 || n <= 0 || bad_dt(dt_out)) return failf(KB2SEQ_ERR_VALUE, "rms_rows: bad argument");
-  rms_rows_kernel<<<T, 256, 0, (cudaStream_t)stream>>>(in, ld_in, n, w, eps, out, dt_out, ld_out);
+  kb2::launch_pdl(rms_rows_kernel, T, 256, 0, (cudaStream_t)stream, in, ld_in, n, w, eps, out, dt_out, ld_out);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
 }
@@ -1186,7 +1200,7 @@ KB2SEQ_API int kb2_seq_rms_rows(const float* in, long long ld_in, int n, const f
 KB2SEQ_API int kb2_seq_branch_merge(const float* a, const float* b, const float* wa, const float* wb, float eps, float coef, float* out, int T,
                                     int W, void* stream) {
   if (!a || !b || !wa || !wb || !out || T <= 0 || W <= 0) return failf(KB2SEQ_ERR_VALUE, "branch_merge: bad argument");
-  branch_merge_kernel<<<T, 256, 0, (cudaStream_t)stream>>>(a, b, wa, wb, eps, coef, out, W);
+  kb2::launch_pdl(branch_merge_kernel, T, 256, 0, (cudaStream_t)stream, a, b, wa, wb, eps, coef, out, W);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
 }
@@ -1194,7 +1208,7 @@ KB2SEQ_API int kb2_seq_branch_merge(const float* a, const float* b, const float*
 KB2SEQ_API int kb2_seq_depth_mix(float* stack, long long stride, int n, const float* coef, float* x, const float* y, const float* w, void* h,
                                  int dt_h, int T, int W, float eps, void* stream) {
   if (!stack || !coef || !x || n <= 0 || T <= 0 || W <= 0 || (w && (!h || bad_dt(dt_h)))) return failf(KB2SEQ_ERR_VALUE, "depth_mix: bad argument");
-  depth_mix_kernel<<<T, 256, 0, (cudaStream_t)stream>>>(stack, stride, n, coef, x, y, w, h, dt_h, W, eps);
+  kb2::launch_pdl(depth_mix_kernel, T, 256, 0, (cudaStream_t)stream, stack, stride, n, coef, x, y, w, h, dt_h, W, eps);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
 }
@@ -1211,7 +1225,7 @@ KB2SEQ_API int kb2_seq_stream_mix(float* xs, int n, const float* x0, const float
 #define KB2_SM(NSV, VV)                                                                                                              \
   do {                                                                                                                               \
     if (smem > 40 * 1024) SEQ_CUDA(cudaFuncSetAttribute(stream_mix_kernel<NSV, VV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    stream_mix_kernel<NSV, VV><<<T, 256, smem, s>>>(xs, n, x0, y, mix, out, read, w, w_shift, h, dt_h, W, eps);                      \
+    kb2::launch_pdl(stream_mix_kernel<NSV, VV>, T, 256, smem, s, xs, n, x0, y, mix, out, read, w, w_shift, h, dt_h, W, eps);                      \
   } while (0)
   if (!vec) KB2_SM(0, 1);
   else switch (n) {

@@ -72,7 +72,6 @@ __global__ void __launch_bounds__(kSThreads)
     split_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const SplitArgs p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int row_tile = blockIdx.x / KS, rank = blockIdx.x % KS;
-  if (p.n_tiles_dev != nullptr && row_tile >= p.n_tiles_dev[0]) return;      // the same decision in every CTA of the cluster
   const int nt = p.xparts * p.mt, w_bytes = p.wparts * kSWBytes, stage_bytes = w_bytes + nt * 128;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + p.stages * stage_bytes);
   uint64_t* empty = full + kSMaxStages;
@@ -80,9 +79,7 @@ __global__ void __launch_bounds__(kSThreads)
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(done + 1);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int n0 = blockIdx.y * kSRows;
-  const int group = p.tile_group != nullptr ? p.tile_group[row_tile] : p.tiles_per_group > 0 ? row_tile / p.tiles_per_group : 0;
   const int m0 = (p.tiles_per_group > 0 ? row_tile % p.tiles_per_group : row_tile) * p.mt;     // row of the output (of its group)
-  const int w0 = n0 + group * p.N;                                                             // row of W
   const int kb0 = (int)((long long)p.n_kblocks * rank / KS), kb1 = (int)((long long)p.n_kblocks * (rank + 1) / KS);
 
   if (threadIdx.x == 32) {
@@ -103,6 +100,13 @@ __global__ void __launch_bounds__(kSThreads)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_wait();
+  if (p.n_tiles_dev != nullptr && row_tile >= p.n_tiles_dev[0]) {            // the same decision in every CTA of the cluster
+    if (warp == 0) tmem_dealloc(tmem_base, p.tmem_cols);
+    return;
+  }
+  const int group = p.tile_group != nullptr ? p.tile_group[row_tile] : p.tiles_per_group > 0 ? row_tile / p.tiles_per_group : 0;
+  const int w0 = n0 + group * p.N;                                                             // row of W
 
   if (warp == 0) {
     int stage = 0;
@@ -238,13 +242,15 @@ static cudaError_t launch_one_split(const CUtensorMap& tx, const CUtensorMap& tw
   cfg.blockDim = dim3(kSThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = KS;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = KS;
+  at[1].val.clusterDim.y = 1;
+  at[1].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = KS > 1 ? 1 : 0;
+  cfg.numAttrs = KS > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, tx, tw, p);
 }
 
@@ -404,6 +410,7 @@ __device__ __forceinline__ void split3(float v, uint32_t& hi, uint32_t& mid, uin
 template <bool kVec>
 __global__ void __launch_bounds__(256) split_parts_kernel(const float* __restrict__ x, long long ld, long long group_stride, int rows, int K, int mt,
                                                           int tiles, long long total, __nv_bfloat16* __restrict__ parts) {
+  pdl_enter(x, parts);
   const int k8 = K >> 3;
   for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
     const long long r = i / k8;                      // row of the padded [groups][tiles][mt] order
@@ -445,8 +452,8 @@ cudaError_t launch_split_parts(const float* x, long long ld, long long group_str
   const long long total = (long long)groups * tiles * mt * (K / 8);
   const unsigned blocks = (unsigned)std::min<long long>((total + 255) / 256, num_sms * 16);
   const bool vec = !((uintptr_t)x & 15) && ld % 4 == 0 && group_stride % 4 == 0;
-  if (vec) split_parts_kernel<true><<<blocks, 256, 0, s>>>(x, ld, group_stride, rows, K, mt, tiles, total, (__nv_bfloat16*)parts);
-  else split_parts_kernel<false><<<blocks, 256, 0, s>>>(x, ld, group_stride, rows, K, mt, tiles, total, (__nv_bfloat16*)parts);
+  if (vec) launch_pdl(split_parts_kernel<true>, blocks, 256, 0, s, x, ld, group_stride, rows, K, mt, tiles, total, (__nv_bfloat16*)parts);
+  else launch_pdl(split_parts_kernel<false>, blocks, 256, 0, s, x, ld, group_stride, rows, K, mt, tiles, total, (__nv_bfloat16*)parts);
   return cudaGetLastError();
 }
 
