@@ -103,8 +103,8 @@ KB2SEQ_API int kb2_seq_delta_rule(const float* conv, int C, const float* proj, l
                                   float eps, float* state, const int* cu, const int* slots, float* scratch, void* out, int dt_out,
                                   void* stream);
 
-/* The same for long portions, eight tokens at a time on the tensor instructions with the accuracy of fp32 sums: dk 32, 64 or 128, dv a multiple of 32; scratch of kb2_seq_delta_tiles_scratch floats
- * (0: sizes not taken), 16-byte aligned, as is conv; C a multiple of 4. */
+/* The same for long portions, sixteen tokens at a time on the tensor instructions with the accuracy of fp32 sums: dk 32, 64 or 128, dv a
+ * multiple of 32; scratch of kb2_seq_delta_tiles_scratch floats (0: sizes not taken), 16-byte aligned, as is conv; C a multiple of 4. */
 KB2SEQ_API long long kb2_seq_delta_tiles_scratch(int T, int S, int H, int Hk, int dk, int dv);
 KB2SEQ_API int kb2_seq_delta_tiles(const float* conv, int C, const float* proj, long long ldp, int g_off, int a_off, int b_off, int T, int S, int H,
                                    int Hk, int dk, int dv, const float* A_log, const float* dt_bias, const float* norm_w, float eps, float* state,

@@ -257,6 +257,13 @@ __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// the same without an addend
+__device__ __forceinline__ void mma16816_new(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+
 template <typename TC, int KS>
 __global__ void __launch_bounds__(KS > 8 ? 512 : 256) gemv_mma_kernel(const bf16* __restrict__ A, long long lda, const bf16* __restrict__ B, long long ldb,
                                                                       TC* __restrict__ C, long long ldc, int M, int N, int K, long long sA, long long sB,
@@ -1450,35 +1457,46 @@ __global__ void __launch_bounds__(32 * kRegPieces) delta_rule_reg_kernel(const f
   for (int ii = 0; ii < Q; ++ii) Sg[(long long)(piece * Q + ii) * dv + j0 + lane] = S[ii];
 }
 
-// ---- the recurrence with one decay per head, eight tokens at a time on the warp-level tensor instructions (long portions).
+// ---- the recurrence with one decay per head, sixteen tokens at a time on the warp-level tensor instructions (long portions).
 // With S0 the state ahead of a tile, G_i = g_0 .. g_i and D_ij = g_(j+1) .. g_i, the token-by-token rule is
 //   u_i = beta_i (v_i - G_i S0^T k_i - sum_(j<i) D_ij (k_i . k_j) u_j),   o_i = G_i S0^T q_i + sum_(j<=i) D_ij (q_i . k_j) u_j,
-//   S = G_7 S0 + sum_j D_7j k_j u_j^T:
-// two small products with the state per tile, one sum over its rows instead of eight in a row, and 64 numbers per (tile, head) that couple the
-// tokens, made ahead for all tiles at once (delta_tile_prep).  Everything stays at fp32 grade: the operands of the products go in as three
-// bf16 parts each (24 bits; six of nine products, the rest is below 2^-26), tensor sums run over 32 rows or 8 tokens and start from zero, and
-// the state itself is updated by fp32 multiply-adds.
-// Bound: the chain of a tile.  The token-by-token form (delta_rule_reg) spends 510 cycles per token on shared-memory broadcasts and a block
-// barrier; a form with four tokens per tile on packed FMAs 394, because a 16-byte shared-memory read takes four passes however many lanes
-// share an address.  Here a warp keeps 16 value columns x 32 rows as accumulator fragments, which are the operand fragments of the next
-// tile's product as they stand; k and q arrive as ready images (one bulk copy per tile, ahead of time) and enter through ldmatrix, plain for
-// S0^T k and transposed for k u^T.  The DK / 32 warps of a column group meet once per tile and then each solve the eight steps by themselves.
-// 4096 tokens, 32 / 16 heads x 128: 1048 -> 648 us (prep 48 -> 56); left: two warps per scheduler and 2400 cycles per tile of dependent short
-// phases, the tensor pipe 37 % and shared memory 46 % busy.
-constexpr int kDT = 8, kDTStages = 4;
-// what couples the tokens of a (tile, head), as the kernel reads it: G[8] | beta[8] | D_7j [8] | G_7 and padding | D_ij k_i.k_j as [j][i > j] |
-// D_ij q_i.k_j as [i][j <= i]
-constexpr int kDTG = 0, kDTBeta = 8, kDTEnd = 16, kDTAll = 24, kDTKK = 32, kDTQK = 96, kDTScalars = 160;
+//   S = G_15 S0 + sum_j D_15,j k_j u_j^T.
+// The u_i solve (I + L) u = diag(beta) (V - diag(G) K S0) with L_ij = beta_i D_ij (k_i . k_j) below the diagonal, and T = (I + L)^-1 needs no
+// state: delta_tile_prep makes V' = T diag(beta) V and W = T diag(beta G) K for all tiles at once, which leaves u = V' - W S0 for the chain of
+// tiles (the WY form of a product of Householder-like factors: Bischof and Van Loan 1987; for this rule Yang et al. 2024, "Parallelizing Linear
+// Transformers with the Delta Rule over Sequence Length").  No entry of T exceeds 1, since T_ij is made of products of the contractions
+// I - beta k k^T.  Everything stays at fp32 grade: the operands of the products go in as three bf16 parts each (24 bits; six of nine products,
+// the rest is below 2^-26), tensor sums run over 32 rows or 16 tokens and start from zero, and the state is updated by fp32 multiply-adds.
+// A token's numbers never meet those of a later one, not even times zero: the sums of the prep stop at the diagonal, rows of a tensor product
+// do not mix, and the read-out takes what is not finite out of its product and adds it to the later tokens by hand.
+//
+// A block has 32 value columns of a (sequence, head) as two groups of 16 columns.  A group has DK / 32 warps with 32 rows of the state each, as
+// accumulator fragments that are the operand fragments of the next tile's product as they stand, and a warp for the read-outs, which are off the
+// chain.  k, q and W arrive as ready images (bulk copies by a warp of their own, three tiles ahead) and enter through ldmatrix, plain for S0^T w
+// and transposed for k u^T; the partial sums of a group's warps meet in shared memory in fragment order, so nothing is moved between lanes.
+// The largest of the six products of an update and of a read-out goes eight tokens at a time, each to a sum of its own: the tensor cores cut off
+// what they add, and with sixteen at a time states were 1 % further off (6.6e-7 instead of 6.5e-7).
+// Bound: 1300 cycles of the tensor pipe and 1400 of shared memory per tile, of about 2400 (4096 tokens, 32 / 16 heads x 128: 342 us, the prep 110); left
+// is the chain split - W - exchange - u - update.  With eight tokens per tile, where each warp solved for u itself, a tile took 2400 cycles of dependent
+// short phases too, and the whole 642 + 56 us.
+constexpr int kDT = 16, kDTStages = 4;
+// what couples the tokens of a (tile, head): G[16] | D_15,j [16] | G_15 and padding to 48 floats | D_ij q_i . k_j as three bf16 parts [i][24]
+constexpr int kDTG = 0, kDTEnd = 16, kDTAll = 32, kDTQK = 48, kDTQKPitch = 24, kDTQKPart = kDT * kDTQKPitch;
+constexpr int kDTScalars = kDTQK + 3 * kDTQKPart / 2;      // floats
 template <int NI> struct DeltaTile {
   static constexpr int DK = 32 * NI, kPitch = DK + 8;      // bf16 row pitch: 16 bytes more, so that the eight rows of an ldmatrix do not collide
-  static constexpr int kPart = 2 * kDT * kPitch;           // bf16 of one part: k rows, then q rows
-  static constexpr int kImage = 3 * kPart;                 // bf16 of a (tile, key head): hi, mid, lo
-  static constexpr int kImageBytes = kImage * 2, kScalarBytes = kDTScalars * 4, kVBytes = kDT * 32 * 4;
-  static constexpr int kStageBytes = kImageBytes + kVBytes + kScalarBytes;
-  static constexpr int kRedFloats = 2 * 2 * NI * 16 * 20;  // [buffer][column group][row piece][column][16 products + pad]
-  static constexpr int kUFloats = 2 * NI * 16 * 12;        // [warp][column][8 tokens + pad]
-  static constexpr int kSmem = kDTStages * kStageBytes + (kRedFloats + kUFloats) * 4 + 2 * kDTStages * 8;
-  static_assert(kImageBytes % 16 == 0 && kStageBytes % 16 == 0, "bulk copies");
+  static constexpr int kWPart = kDT * kPitch, kPart = 2 * kWPart;      // bf16 of one part: of W; of k rows, then q rows
+  static constexpr int kImage = 3 * kPart, kWImage = 3 * kWPart;       // bf16 of a (tile, key head) and of a (tile, head): hi, mid, lo
+  static constexpr int kImageBytes = kImage * 2, kWBytes = kWImage * 2, kScalarBytes = kDTScalars * 4, kVBytes = kDT * 32 * 4;
+  static constexpr int kStageBytes = kImageBytes + kWBytes + kVBytes + kScalarBytes;
+  static constexpr int kRedFloats = 2 * 2 * NI * 4 * 128;  // [buffer][column group][row piece][W tokens 0..7, 8..15, q 0..7, 8..15][lane][4]
+  static constexpr int kUFloats = 2 * 2 * 256;             // [buffer][column group][lane][8]
+  static constexpr int kSmem = kDTStages * kStageBytes + (kRedFloats + kUFloats) * 4 + (2 * kDTStages + 12) * 8;
+  static constexpr int kThreads = 64 * NI + 96;
+// image | k | q | v of two heads | k.k and q.k in two halves | per head of a pair L, T beta G, T beta | gates
+  static constexpr int prep_smem(int vb, int rep) { return kImageBytes + (2 * kDT * DK + 2 * kDT * 32 * vb + 10 * kDT * 20 + 2 * kDT * rep) * 4; }
+  static_assert(kImageBytes % 16 == 0 && kWBytes % 16 == 0 && kScalarBytes % 16 == 0 && kStageBytes % 16 == 0, "bulk copies");
+  static_assert(kSmem <= 227 * 1024, "shared memory");
 };
 
 // fp32 pair -> three words of bf16 pairs whose sums they are, exact to 24 bits (the largest finite numbers too: their first part stops at the
@@ -1489,141 +1507,11 @@ __device__ __forceinline__ void split_pair(float x, float y, uint32_t (&p)[3]) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p[1]) : "f"(ry), "f"(rx));
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p[2]) : "f"(ry - __uint_as_float(p[1] & 0xFFFF0000u)), "f"(rx - __uint_as_float(p[1] << 16)));
 }
-
-template <int NI>
-__global__ void __launch_bounds__(256) delta_tile_prep_kernel(const float* __restrict__ conv, int C, const float* __restrict__ bproj, long long ldb,
-                                                              const float* __restrict__ aproj, long long lda, int H, int Hk,
-                                                              const float* __restrict__ A_log, const float* __restrict__ dt_bias, int S,
-                                                              const int* __restrict__ cu, long long tiles, bf16* __restrict__ image,
-                                                              float* __restrict__ sc) {
-  kb2::pdl_enter(conv, bproj, aproj, A_log, dt_bias, cu, image, sc);
-  using D = DeltaTile<NI>;
-  constexpr int DK = D::DK;
-  const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  const long long flat = w / Hk;
-  const int hk = (int)(w - flat * Hk);
-  if (flat >= tiles) return;
-  long long tile = flat;
-  int sq = 0, t0 = 0, n = 0;                          // the tile's sequence: tiles are counted sequence by sequence
-  for (; sq < S; ++sq) {
-    t0 = cu[sq];
-    n = cu[sq + 1] - t0;
-    const int nt = (n + kDT - 1) / kDT;
-    if (tile < nt) break;
-    tile -= nt;
-  }
-  if (sq == S) return;
-  t0 += (int)tile * kDT;
-  const int nt = min(kDT, n - (int)tile * kDT);
-  float q[kDT][NI], k[kDT][NI];                       // a lane's NI neighbouring numbers of every row
-#pragma unroll
-  for (int t = 0; t < kDT; ++t)
-#pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      const float* row = conv + (long long)(t0 + t) * C + hk * DK + lane * NI + i;
-      q[t][i] = t < nt ? row[0] : 0.f;
-      k[t][i] = t < nt ? row[Hk * DK] : 0.f;
-    }
-  bf16* img = image + (flat * Hk + hk) * D::kImage;
-  auto store = [&](bf16* at, const float (&v)[NI]) {  // the three parts of a row, behind the last token zeros
-    if constexpr (NI == 1) {
-      const float other = __shfl_down_sync(0xffffffffu, v[0], 1);
-      uint32_t p[3];
-      split_pair(v[0], other, p);
-      if (!(lane & 1))
-#pragma unroll
-        for (int c = 0; c < 3; ++c) *reinterpret_cast<uint32_t*>(at + c * D::kPart + lane) = p[c];
-    } else {
-#pragma unroll
-      for (int i = 0; i < NI; i += 2) {
-        uint32_t p[3];
-        split_pair(v[i], v[i + 1], p);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) *reinterpret_cast<uint32_t*>(at + c * D::kPart + lane * NI + i) = p[c];
-      }
-    }
-  };
-#pragma unroll
-  for (int t = 0; t < kDT; ++t) {
-    float a = 0.f, b = 0.f;
-#pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      a += q[t][i] * q[t][i];
-      b += k[t][i] * k[t][i];
-    }
-    a = warp_sum(a);
-    b = warp_sum(b);
-    const float rq = (1.f / sqrtf((float)DK)) / sqrtf(a + 1e-6f), rk = 1.f / sqrtf(b + 1e-6f);
-#pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      q[t][i] *= rq;
-      k[t][i] *= rk;
-    }
-    store(img + t * D::kPitch, k[t]);
-    store(img + (kDT + t) * D::kPitch, q[t]);
-  }
-  const int rep = H / Hk, me = lane & 7;              // a lane per (head, token of the tile), four heads at a time
-  for (int r0 = 0; r0 < rep; r0 += 4) {
-    const int h = hk * rep + r0 + (lane >> 3);
-    const bool head = r0 + (lane >> 3) < rep;
-    float g = 1.f, beta = 0.f;
-    if (head && me < nt) {
-      g = decay_of(A_log[h], aproj[(long long)(t0 + me) * lda + h], dt_bias[h]);
-      beta = 1.f / (1.f + expf(-bproj[(long long)(t0 + me) * ldb + h]));
-    }
-    float gs[kDT];
-#pragma unroll
-    for (int t = 0; t < kDT; ++t) gs[t] = __shfl_sync(0xffffffffu, g, t, 8);       // 1 behind the last token
-    float up = 1.f, down = 1.f, all = 1.f, d = 1.f, row[2][kDT];                   // d: D_me,j for the j at hand, from j = 7 down
-#pragma unroll
-    for (int t = 0; t < kDT; ++t) {
-      all *= gs[t];
-      if (t <= me) up *= gs[t];
-      if (t > me) down *= gs[t];
-    }
-#pragma unroll
-    for (int j = kDT - 1; j >= 0; --j) {
-      float kk = 0.f, qk = 0.f;                       // k_me . k_j and q_me . k_j: all pairs of the tile, of which a lane keeps its own row
-#pragma unroll
-      for (int t = 0; t < kDT; ++t) {
-        if (t < j) continue;
-        float a = 0.f, b = 0.f;
-#pragma unroll
-        for (int i = 0; i < NI; ++i) {
-          a = fmaf(k[t][i], k[j][i], a);
-          b = fmaf(q[t][i], k[j][i], b);
-        }
-        b = warp_sum(b);
-        if (t > j) a = warp_sum(a);
-        if (me == t) {
-          kk = t > j ? a : 0.f;
-          qk = b;
-        }
-      }
-      row[0][j] = j < me ? d * kk : 0.f;
-      row[1][j] = j <= me ? d * qk : 0.f;
-      if (j <= me) d *= gs[j];
-    }
-    if (!head) continue;
-    float* o = sc + (flat * H + h) * kDTScalars;
-    const bool in = me < nt;                          // tokens behind the last one take no part
-    o[kDTG + me] = in ? up : 0.f;
-    o[kDTBeta + me] = beta;
-    o[kDTEnd + me] = in ? down : 0.f;
-    if (me == 0) o[kDTAll] = all;
-#pragma unroll
-    for (int j = 0; j < kDT; ++j) {
-      o[kDTKK + j * kDT + me] = in ? row[0][j] : 0.f;
-      o[kDTQK + me * kDT + j] = in ? row[1][j] : 0.f;
-    }
-  }
-}
-
-__device__ __forceinline__ void mma1688(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a0), "r"(a1), "r"(b0));
+// eight tokens of the sixteen
+__device__ __forceinline__ void mma1688_new(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%7, %7, %7, %7};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(b0), "f"(0.f));
 }
 template <bool kTrans> __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const void* row) {
   const uint32_t at = (uint32_t)__cvta_generic_to_shared(row);
@@ -1632,67 +1520,465 @@ template <bool kTrans> __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4
   else
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
 }
+// The six products of two numbers in three parts that are worth having: the parts that go into product m (the largest, m = 0, has a sum of its own).
+__device__ __forceinline__ constexpr int part_a(int m) { return 0x120100 >> (4 * m) & 15; }
+__device__ __forceinline__ constexpr int part_b(int m) { return 0x102010 >> (4 * m) & 15; }
 
-// A block: 32 value columns of a (sequence, head) as two groups of 16, NI warps per group (32 rows each), and a warp that streams the tiles.
+struct DeltaPrep {
+  const float* conv;               // [T][C]: q | k | v
+  long long C, ldp;
+  const float *bproj, *aproj, *A_log, *dt_bias;
+  int H, Hk, dv, S;
+  const int* cu;
+  long long tiles;
+  bf16 *image, *wimage;
+  float *vimage, *sc;
+};
+
+// The tile's rows t0 .. t0 + nt - 1 of kWidth neighbouring channels from c on, to shared memory [16][kWidth], zeros behind the last one.
+template <int kWidth>
+__device__ __forceinline__ void delta_fetch(const DeltaPrep& p, int t0, int nt, int c, float* to) {
+  for (int i = threadIdx.x; i < kDT * kWidth / 4; i += 256) {
+    const int t = i / (kWidth / 4), e = i % (kWidth / 4) * 4;
+    if (t < nt) kb2::cp_async16(to + t * kWidth + e, p.conv + (long long)(t0 + t) * p.C + c + e);
+    else *reinterpret_cast<float4*>(to + t * kWidth + e) = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+
+// A block of eight warps per (tile, key head).  Bound by traffic: 16 bytes of k, q and v in and 26 out per token and column (4096 tokens, 32 / 16
+// heads x 128).  All loops are rolled as far as registers allow: with everything unrolled and a warp for each part the block took 35 KB of
+// instructions once, and waiting for them was most of its time.
+// image [tiles][Hk] | W [tiles][H] | V' [tiles][H][dv / 16][lane][8], in the order in which a lane of delta_tile_kernel takes them | scalars [tiles][H]
+template <int NI, int VB>
+__global__ void __launch_bounds__(256, 3) delta_tile_prep_kernel(const DeltaPrep p) {
+  kb2::pdl_wait();
+  using D = DeltaTile<NI>;
+  constexpr int DK = D::DK, kCols = 32 * VB;          // value columns of a pass
+  extern __shared__ __align__(128) uint8_t tsm[];
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = tid & 31;
+  const long long flat = blockIdx.x / p.Hk;
+  const int hk = (int)(blockIdx.x - flat * p.Hk), H = p.H, rep = H / p.Hk;
+  long long tile = flat;
+  int sq = 0, t0 = 0, n = 0;                          // the tile's sequence: tiles are counted sequence by sequence
+  for (; sq < p.S; ++sq) {
+    t0 = p.cu[sq];
+    n = p.cu[sq + 1] - t0;
+    const int nt = (n + kDT - 1) / kDT;
+    if (tile < nt) break;
+    tile -= nt;
+  }
+  if (sq == p.S) return;
+  t0 += (int)tile * kDT;
+  const int nt = min(kDT, n - (int)tile * kDT);
+  bf16* img = reinterpret_cast<bf16*>(tsm);
+  float* rows = reinterpret_cast<float*>(tsm + D::kImageBytes);        // k [16][DK] | q [16][DK] | v of two heads [2][16][kCols]
+  float* vrow = rows + 2 * kDT * DK;
+  float* pairs = vrow + 2 * kDT * kCols;              // [k.k, q.k][half of the sum][16][20]
+  float* Lb = pairs + 4 * kDT * 20;                   // [head of the pair][16][20], as T beta G and T beta
+  float* Tw = Lb + 2 * kDT * 20;
+  float* Tv = Tw + 2 * kDT * 20;
+  float* gates = Tv + 2 * kDT * 20;                   // [decay, strength][head of the key head][16]
+
+  delta_fetch<DK>(p, t0, nt, p.Hk * DK + hk * DK, rows);
+  delta_fetch<DK>(p, t0, nt, hk * DK, rows + kDT * DK);
+  kb2::cp_async_commit();
+  auto fetch_values = [&](int r0, int j0) {
+    for (int hh = 0; hh < 2 && r0 + hh < rep; ++hh)
+      delta_fetch<kCols>(p, t0, nt, 2 * p.Hk * DK + (hk * rep + r0 + hh) * p.dv + j0, vrow + hh * kDT * kCols);
+    kb2::cp_async_commit();
+  };
+  fetch_values(0, 0);
+  // decays and write strengths of the block's heads, under the wait for the rows (fp64 exponentials: a few hundred dependent instructions)
+  for (int i = tid; i < 2 * rep * kDT; i += 256) {
+    const int which = i / (rep * kDT), h = hk * rep + i % (rep * kDT) / kDT, t = i % kDT;
+    const long long row = (long long)(t0 + t) * p.ldp + h;
+    gates[i] = t >= nt ? (which ? 0.f : 1.f) : which ? 1.f / (1.f + expf(-p.bproj[row])) : decay_of(p.A_log[h], p.aproj[row], p.dt_bias[h]);
+  }
+  kb2::cp_async_wait<1>();
+  __syncthreads();
+
+  auto store = [&](bf16* to, int part, const float (&v)[NI]) {       // the three parts of a row, `part` numbers apart
+    if constexpr (NI == 1) {
+      const float other = __shfl_down_sync(0xffffffffu, v[0], 1);
+      uint32_t q[3];
+      split_pair(v[0], other, q);
+      if (!(lane & 1))
+#pragma unroll
+        for (int c = 0; c < 3; ++c) *reinterpret_cast<uint32_t*>(to + c * part + lane) = q[c];
+    } else {
+      uint32_t q[NI / 2][3];
+#pragma unroll
+      for (int i = 0; i < NI; i += 2) split_pair(v[i], v[i + 1], q[i / 2]);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        if constexpr (NI == 4) *reinterpret_cast<uint2*>(to + c * part + lane * 4) = make_uint2(q[0][c], q[1][c]);
+        else *reinterpret_cast<uint32_t*>(to + c * part + lane * 2) = q[0][c];
+      }
+    }
+  };
+  auto take = [&](const float* from, auto& v) {       // a lane's neighbouring numbers of a row
+    constexpr int N = sizeof(v) / sizeof(float);
+    if constexpr (N == 4) {
+      const float4 f = *reinterpret_cast<const float4*>(from + lane * 4);
+      v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < N; ++i) v[i] = from[lane * N + i];
+    }
+  };
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {                       // unit rows: 16 of k, then 16 of q
+    const int t = warp * 4 + r;
+    float v[NI], a = 0.f;
+    take(rows + t * DK, v);
+#pragma unroll
+    for (int i = 0; i < NI; ++i) a += v[i] * v[i];
+    a = warp_sum(a);
+    const float s = warp < 4 ? 1.f / sqrtf(a + 1e-6f) : (1.f / sqrtf((float)DK)) / sqrtf(a + 1e-6f);
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      v[i] *= s;
+      rows[t * DK + lane * NI + i] = v[i];
+    }
+    store(img + t * D::kPitch, D::kPart, v);
+  }
+  kb2::fence_proxy_async_smem();
+  __syncthreads();
+  if (tid == 128) {
+    kb2::bulk_s2g(p.image + (flat * p.Hk + hk) * D::kImage, img, D::kImageBytes);
+    kb2::bulk_commit_group();
+  }
+  if (warp < 4) {                                     // k_i . k_j (warps 0, 1: halves of the sum) and q_i . k_j (2, 3)
+    float s[2][4] = {};
+    const bf16* row = img + ((lane >> 4) * 8 + (lane & 7)) * D::kPitch + ((lane >> 3) & 1) * 8;
+    const int mine = warp < 2 ? 0 : D::kWPart;
+#pragma unroll 1
+    for (int k0 = (warp & 1) * 32; k0 < DK; k0 += 64) {
+      float big[2][2][4], small[2][4];                // [16 numbers][columns 0..7, 8..15]
+#pragma unroll
+      for (int kb = 0; kb < 2; ++kb) {
+        uint32_t x[3][4], y[3][4];                    // tokens 0..7: numbers 0..7, 8..15; tokens 8..15 the same
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          ldmatrix4<false>(x[c], row + c * D::kPart + k0 + kb * 16);
+          ldmatrix4<false>(y[c], row + c * D::kPart + mine + k0 + kb * 16);
+        }
+#pragma unroll
+        for (int m = 0; m < 6; ++m)
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            float(&d)[4] = m ? small[b] : big[kb][b];
+            const uint32_t(&ya)[4] = y[part_a(m)];
+            const uint32_t(&xb)[4] = x[part_b(m)];
+            if (m == 0 || (kb == 0 && m == 1)) mma16816_new(d, ya[0], ya[2], ya[1], ya[3], xb[2 * b], xb[2 * b + 1]);
+            else mma16816(d, ya[0], ya[2], ya[1], ya[3], xb[2 * b], xb[2 * b + 1]);
+          }
+      }
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[b][e] += (big[0][b][e] + big[1][b][e]) + small[b][e];
+    }
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        *reinterpret_cast<float2*>(pairs + warp * kDT * 20 + ((lane >> 2) + e * 8) * 20 + b * 8 + (lane & 3) * 2) = make_float2(s[b][2 * e], s[b][2 * e + 1]);
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int r0 = 0; r0 < rep; r0 += 2) {
+    if (warp < 2) {                                   // a lane per (head of the pair, token): what couples the tokens
+      const int me = lane & 15, half = lane >> 4, h = hk * rep + r0 + half;
+      const bool head = r0 + half < rep, in = me < nt;
+      float gs[kDT], up = 1.f, d = 1.f, row[kDT];     // d: D_me,j for the j at hand, from j = 15 down
+#pragma unroll
+      for (int t = 0; t < kDT; ++t) gs[t] = head ? gates[(r0 + half) * kDT + t] : 1.f;      // 1 behind the last token
+#pragma unroll
+      for (int t = 0; t < kDT; ++t)
+        if (t <= me) up *= gs[t];
+      const float* mine = pairs + (warp ? 0 : 2 * kDT * 20) + me * 20;
+#pragma unroll
+      for (int j4 = kDT - 4; j4 >= 0; j4 -= 4) {
+        const float4 a = *reinterpret_cast<const float4*>(mine + j4), b = *reinterpret_cast<const float4*>(mine + kDT * 20 + j4);
+        const float av[4] = {a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w};
+#pragma unroll
+        for (int e = 3; e >= 0; --e) {
+          const int j = j4 + e;
+          row[j] = j < me + !warp ? d * av[e] : 0.f;  // below the diagonal; q . k with it
+          if (j <= me) d *= gs[j];
+        }
+      }
+      if (warp == 0) {                                // what the chain and the read-out take as numbers; tokens behind the last one take no part
+        float down = 1.f, all = 1.f;
+#pragma unroll
+        for (int t = 0; t < kDT; ++t) {
+          all *= gs[t];
+          if (t > me) down *= gs[t];
+        }
+        if (head) {
+          float* o = p.sc + (flat * H + h) * kDTScalars;
+          o[kDTG + me] = in ? up : 0.f;
+          o[kDTEnd + me] = in ? down : 0.f;
+          o[kDTAll + me] = me == 0 ? all : 0.f;
+          uint32_t q[kDT / 2][3];
+#pragma unroll
+          for (int j = 0; j < kDT; j += 2) split_pair(in ? row[j] : 0.f, in ? row[j + 1] : 0.f, q[j / 2]);
+          bf16* parts = reinterpret_cast<bf16*>(o + kDTQK) + me * kDTQKPitch;
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+              *reinterpret_cast<uint4*>(parts + c * kDTQKPart + j * 8) = make_uint4(q[4 * j][c], q[4 * j + 1][c], q[4 * j + 2][c], q[4 * j + 3][c]);
+        }
+      } else {
+        const float beta = head ? gates[(rep + r0 + half) * kDT + me] : 0.f;
+        float* L = Lb + half * kDT * 20;
+#pragma unroll
+        for (int j = 0; j < kDT; j += 4)
+          *reinterpret_cast<float4*>(L + me * 20 + j) = make_float4(beta * row[j], beta * row[j + 1], beta * row[j + 2], beta * row[j + 3]);
+        __syncwarp();
+        float x[kDT];                                 // column `me` of T
+#pragma unroll
+        for (int i = 0; i < kDT; ++i) {
+          float a = i == me ? 1.f : 0.f;
+#pragma unroll
+          for (int j4 = 0; j4 < i; j4 += 4) {
+            const float4 l = *reinterpret_cast<const float4*>(L + i * 20 + j4);
+            const float lv[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (j4 + e < i) a = fmaf(-lv[e], x[j4 + e], a);
+          }
+          x[i] = a;
+        }
+#pragma unroll
+        for (int i = 0; i < kDT; ++i) {
+          Tv[half * kDT * 20 + i * 20 + me] = x[i] * beta;
+          Tw[half * kDT * 20 + i * 20 + me] = x[i] * beta * up;
+        }
+      }
+    }
+    const int hh = (warp >> 1) & 1, hv = hk * rep + r0 + hh, b0 = warp & 1;      // two warps per product with T: rows 0..3, 8..11 and 4..7, 12..15
+    const bool there = r0 + hh < rep;
+#pragma unroll 1
+    for (int j0 = 0; j0 < p.dv; j0 += kCols) {
+      kb2::cp_async_wait<0>();
+      __syncthreads();
+      // four rows of a product with T: no column behind a row's own
+      auto four = [&](const float* T, const float* x, int width, int ib, auto& acc) {
+        constexpr int N = sizeof(acc[0]) / sizeof(float);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int m = 0; m < N; ++m) acc[i][m] = 0.f;
+        auto block = [&](int jb, bool whole) {
+          float xr[4][N];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) take(x + (jb * 4 + j) * width, xr[j]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float4 c = *reinterpret_cast<const float4*>(T + (ib * 4 + i) * 20 + jb * 4);
+            const float cv[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (whole || j <= i)
+#pragma unroll
+                for (int m = 0; m < N; ++m) acc[i][m] = fmaf(cv[j], xr[j][m], acc[i][m]);
+          }
+        };
+#pragma unroll 1
+        for (int jb = 0; jb < ib; ++jb) block(jb, true);
+        block(ib, false);
+      };
+      if (warp < 4) {
+        if (j0 == 0 && there) {
+          bf16* wi = p.wimage + (flat * H + hv) * D::kWImage;
+#pragma unroll 1
+          for (int ib = b0; ib < 4; ib += 2) {
+            float a[4][NI];
+            four(Tw + hh * kDT * 20, rows, DK, ib, a);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) store(wi + (ib * 4 + i) * D::kPitch, D::kWPart, a[i]);
+          }
+        }
+      } else if (there) {
+        float a[4][VB], c[4][VB];
+        const float* T = Tv + hh * kDT * 20;
+        const float* x = vrow + hh * kDT * kCols;
+        four(T, x, kCols, b0, a);
+        four(T, x, kCols, b0 + 2, c);
+        float* vi = p.vimage + (flat * H + hv) * kDT * p.dv;
+#pragma unroll
+        for (int m = 0; m < VB; ++m) {
+          const int col = j0 + lane * VB + m;
+#pragma unroll
+          for (int i = 0; i < 4; i += 2)
+            *reinterpret_cast<float4*>(vi + (col >> 4) * 256 + (col & 7) * 32 + (b0 * 2 + i / 2) * 8 + ((col >> 3) & 1) * 4) =
+                make_float4(a[i][m], a[i + 1][m], c[i][m], c[i + 1][m]);
+        }
+      }
+      if (j0 + kCols < p.dv || r0 + 2 < rep) {
+        __syncthreads();
+        if (j0 + kCols < p.dv) fetch_values(r0, j0 + kCols);
+        else fetch_values(r0 + 2, 0);
+      }
+    }
+  }
+  if (tid == 128) kb2::bulk_wait_group0();            // the image has left shared memory
+}
+
 template <int NI>
-__global__ void __launch_bounds__(64 * NI + 32, 1) delta_tile_kernel(const bf16* __restrict__ image, const float* __restrict__ conv, int C, int v_col0,
-                                                                     const float* __restrict__ sc, int H, int Hk, int dv, float* __restrict__ state,
-                                                                     const int* __restrict__ cu, const int* __restrict__ slots, float* __restrict__ o_out) {
-  kb2::pdl_enter(image, conv, sc, state, cu, slots, o_out);
+__global__ void __launch_bounds__(DeltaTile<NI>::kThreads, 1)
+    delta_tile_kernel(const bf16* __restrict__ image, const bf16* __restrict__ wimage, const float* __restrict__ vimage, const float* __restrict__ sc,
+                      int H, int Hk, int dv, float* __restrict__ state, const int* __restrict__ cu, const int* __restrict__ slots,
+                      float* __restrict__ o_out) {
+  kb2::pdl_enter(image, wimage, vimage, sc, state, cu, slots, o_out);
   using D = DeltaTile<NI>;
   extern __shared__ __align__(128) uint8_t tsm[];
   float* red = reinterpret_cast<float*>(tsm + kDTStages * D::kStageBytes);
   float* ubuf = red + D::kRedFloats;
   uint64_t* full = reinterpret_cast<uint64_t*>(ubuf + D::kUFloats);
   uint64_t* empty = full + kDTStages;
+  uint64_t* w_there = empty + kDTStages;           // [buffer][column group]: all pieces of W S0
+  uint64_t* o_there = w_there + 4;                 // all pieces of q S0, and u
+  uint64_t* o_free = o_there + 4;                  // the read-out has taken them
   const int s = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * 32, hk = h / (H / Hk);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int t0 = cu[s], n = cu[s + 1] - cu[s], tiles = (n + kDT - 1) / kDT;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kDTStages; ++i) {
       kb2::mbar_init(&full[i], 1);
-      kb2::mbar_init(&empty[i], 2 * NI);
+      kb2::mbar_init(&empty[i], 2 * NI + 2);
+    }
+    for (int i = 0; i < 4; ++i) {
+      kb2::mbar_init(&w_there[i], NI);
+      kb2::mbar_init(&o_there[i], NI);
+      kb2::mbar_init(&o_free[i], 1);
     }
     kb2::fence_mbar_init();
   }
   __syncthreads();
-  if (warp == 2 * NI) {
+  const int quad = lane >> 2, pair = (lane & 3) * 2;      // fragment: columns quad, quad + 8; rows or tokens pair, pair + 1
+  if (warp == 2 * NI + 2) {                        // ---- the tiles' way into shared memory
     long long first = 0;                           // the sequence's tiles come after those of the sequences before it
     for (int i = 0; i < s; ++i) first += (cu[i + 1] - cu[i] + kDT - 1) / kDT;
     for (int i = 0; i < tiles; ++i) {
       const int st = i % kDTStages;
       uint8_t* b = tsm + st * D::kStageBytes;
       kb2::mbar_wait(&empty[st], (uint32_t)(i / kDTStages & 1) ^ 1u);
-      const int nt = min(kDT, n - i * kDT);
-      const long long t = t0 + (long long)i * kDT;
-      for (int r = nt; r < kDT; ++r) reinterpret_cast<float*>(b + D::kImageBytes)[r * 32 + lane] = 0.f;      // values behind the last token
+      if (lane == 0) kb2::mbar_arrive_expect_tx(&full[st], (uint32_t)D::kStageBytes);
       __syncwarp();
-      if (lane == 0) kb2::mbar_arrive_expect_tx(&full[st], (uint32_t)(D::kImageBytes + D::kScalarBytes + nt * 128));
-      __syncwarp();
-      if (lane < nt) kb2::bulk_g2s(b + D::kImageBytes + lane * 128, conv + (t + lane) * C + v_col0 + h * dv + j0, 128, &full[st]);
-      else if (lane == 8) kb2::bulk_g2s(b, image + ((first + i) * Hk + hk) * D::kImage, D::kImageBytes, &full[st]);
-      else if (lane == 9) kb2::bulk_g2s(b + D::kImageBytes + D::kVBytes, sc + ((first + i) * H + h) * kDTScalars, D::kScalarBytes, &full[st]);
+      const long long flat = first + i;
+      if (lane == 0) kb2::bulk_g2s(b, image + (flat * Hk + hk) * D::kImage, D::kImageBytes, &full[st]);
+      else if (lane == 1) kb2::bulk_g2s(b + D::kImageBytes, wimage + (flat * H + h) * D::kWImage, D::kWBytes, &full[st]);
+      else if (lane == 2) kb2::bulk_g2s(b + D::kImageBytes + D::kWBytes, vimage + (flat * H + h) * kDT * dv + j0 * kDT, D::kVBytes, &full[st]);
+      else if (lane == 3) kb2::bulk_g2s(b + D::kImageBytes + D::kWBytes + D::kVBytes, sc + (flat * H + h) * kDTScalars, D::kScalarBytes, &full[st]);
     }
     return;
   }
-  const int cg = warp / NI, piece = warp % NI, quad = lane >> 2, pair = (lane & 3) * 2;      // fragment: columns quad, quad + 8; rows pair, pair + 1
+  auto one = [](float (&d)[4], bool first, const uint32_t (&a)[3][4], const uint32_t (&b)[3][4], int at, int m) {      // product m of the six
+    const int p = part_a(m), r = part_b(m);
+    if (first) mma16816_new(d, a[p][0], a[p][1], a[p][2], a[p][3], b[r][at], b[r][at + 1]);
+    else mma16816(d, a[p][0], a[p][1], a[p][2], a[p][3], b[r][at], b[r][at + 1]);
+  };
+  if (warp >= 2 * NI) {                            // ---- the read-outs of a column group
+    const int cg = warp - 2 * NI;
+    for (int i = 0; i < tiles; ++i) {
+      const int st = i % kDTStages, buf = (i & 1) * 2 + cg;
+      const float* ss = reinterpret_cast<const float*>(tsm + st * D::kStageBytes + D::kImageBytes + D::kWBytes + D::kVBytes);
+      const bf16* qk = reinterpret_cast<const bf16*>(ss + kDTQK);
+      kb2::mbar_wait(&full[st], (uint32_t)(i / kDTStages & 1));
+      uint32_t b[3][4];                            // tokens 0..7 by j 0..7, j 8..15; tokens 8..15 the same
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        ldmatrix4<false>(b[c], qk + c * kDTQKPart + ((lane >> 4) * 8 + (lane & 7)) * kDTQKPitch + ((lane >> 3) & 1) * 8);
+      kb2::mbar_wait(&o_there[buf], (uint32_t)(i >> 1) & 1u);
+      float u[8], qs[8] = {};
+      {
+        const float4 x = *reinterpret_cast<const float4*>(ubuf + buf * 256 + lane * 8), y = *reinterpret_cast<const float4*>(ubuf + buf * 256 + lane * 8 + 4);
+        u[0] = x.x; u[1] = x.y; u[2] = x.z; u[3] = x.w; u[4] = y.x; u[5] = y.y; u[6] = y.z; u[7] = y.w;
+      }
+#pragma unroll
+      for (int pc = 0; pc < NI; ++pc)
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb) {
+          const float4 x = *reinterpret_cast<const float4*>(red + ((buf * NI + pc) * 4 + 2 + nb) * 128 + lane * 4);
+          qs[nb * 4] += x.x; qs[nb * 4 + 1] += x.y; qs[nb * 4 + 2] += x.z; qs[nb * 4 + 3] += x.w;
+        }
+      bool odd = false;
+      uint32_t a[3][4];
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) {
+        const bool f0 = isfinite(u[e]), f1 = isfinite(u[e + 1]);
+        odd |= !f0 | !f1;
+        uint32_t p[3];
+        split_pair(f0 ? u[e] : 0.f, f1 ? u[e + 1] : 0.f, p);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) a[c][e / 2] = p[c];
+      }
+      float big[2][2][4], small[2][4];
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb) {
+        mma1688_new(big[0][nb], a[0][0], a[0][1], b[0][2 * nb]);
+        mma1688_new(big[1][nb], a[0][2], a[0][3], b[0][2 * nb + 1]);
+      }
+#pragma unroll
+      for (int m = 1; m < 6; ++m)
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb) one(small[nb], m < 2, a, b, 2 * nb, m);
+      float o[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int t = (e >> 2) * 8 + pair + (e & 1);
+        o[e] = fmaf(ss[kDTG + t], qs[e], (big[0][e >> 2][e & 3] + big[1][e >> 2][e & 3]) + small[e >> 2][e & 3]);
+      }
+      if (__any_sync(0xffffffffu, odd)) {          // what is not finite joins its own and later tokens
+#pragma unroll 1
+        for (int j = 0; j < kDT; ++j) {
+          const float* from = ubuf + buf * 256 + (quad * 4 + ((j & 7) >> 1)) * 8 + (j >> 3) * 4 + (j & 1);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const int t = (e >> 2) * 8 + pair + (e & 1);
+            const float uj = from[((e >> 1) & 1) * 2];
+            const bf16* c = qk + t * kDTQKPitch + j;
+            if (j <= t && !isfinite(uj)) o[e] += uj * (__bfloat162float(c[0]) + (__bfloat162float(c[kDTQKPart]) + __bfloat162float(c[2 * kDTQKPart])));
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) {
+        kb2::mbar_arrive(&o_free[buf]);
+        kb2::mbar_arrive(&empty[st]);
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int t = (e >> 2) * 8 + pair + (e & 1);
+        if (i * kDT + t < n) o_out[((t0 + (long long)i * kDT + t) * H + h) * dv + j0 + cg * 16 + quad + ((e >> 1) & 1) * 8] = o[e];
+      }
+    }
+    return;
+  }
+  const int cg = warp / NI, piece = warp % NI;     // ---- the chain
   float* Sg = state + ((long long)slots[s] * H + h) * D::DK * dv + (long long)piece * 32 * dv + j0 + cg * 16;
   float S[4][4];                                   // [eight rows][column quad: 2 rows, column quad + 8: 2 rows]
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
     for (int e = 0; e < 4; ++e) S[r][e] = Sg[(long long)(r * 8 + pair + (e & 1)) * dv + quad + (e >> 1) * 8];
-  const int col = lane & 15, half = lane >> 4;
-  float* myu = ubuf + warp * 16 * 12;
+  // ldmatrix rows: tokens along the lanes' eights, plain and transposed
+  const int plain = ((lane >> 4) * 8 + (lane & 7)) * D::kPitch + piece * 32 + ((lane >> 3) & 1) * 8;
+  const int turned = (((lane >> 3) & 1) * 8 + (lane & 7)) * D::kPitch + piece * 32 + (lane >> 4) * 8;
   for (int i = 0; i < tiles; ++i) {
-    const int st = i % kDTStages;
+    const int st = i % kDTStages, buf = (i & 1) * 2 + cg;
+    const uint32_t turn = (uint32_t)(i >> 1) & 1u;
     const uint8_t* b = tsm + st * D::kStageBytes;
     const bf16* img = reinterpret_cast<const bf16*>(b);
-    const float* vs = reinterpret_cast<const float*>(b + D::kImageBytes);
-    const float* ss = vs + kDT * 32;
-    float* buf = red + (i & 1) * (2 * NI * 16 * 20) + cg * (NI * 16 * 20);
-    // S0^T [k | q] over the warp's 32 rows
-    uint32_t sp[2][3][4];                          // [16 rows][part][operand words]
+    const bf16* wim = reinterpret_cast<const bf16*>(b + D::kImageBytes);
+    const float* vs = reinterpret_cast<const float*>(b + D::kImageBytes + D::kWBytes) + cg * 256 + lane * 8;
+    const float* ss = reinterpret_cast<const float*>(b + D::kImageBytes + D::kWBytes + D::kVBytes);
+    float* mine = red + (buf * NI + piece) * 512 + lane * 4;
+    uint32_t sp[2][3][4];                          // S0^T as operand: [16 rows][part]
 #pragma unroll
     for (int kb = 0; kb < 2; ++kb)
 #pragma unroll
@@ -1702,119 +1988,130 @@ __global__ void __launch_bounds__(64 * NI + 32, 1) delta_tile_kernel(const bf16*
 #pragma unroll
         for (int c = 0; c < 3; ++c) sp[kb][c][e] = p[c];
       }
-    kb2::mbar_wait(&full[st], (uint32_t)(i / kDTStages & 1));
-    float dk[4][4] = {}, dq[4][4] = {};            // four sums each (the products by size), so that no instruction waits for the one before it
+    // S0^T [16 columns x 32 rows] times 16 tokens, in three sums of up to six instructions, each of which waits for the one before
+    auto product = [&](const bf16* rows, int part, float (&sum)[3][2][4]) {
 #pragma unroll
-    for (int kb = 0; kb < 2; ++kb) {
-      uint32_t x[3][4];                            // k rows 0..7, k rows 8..15 of the block; q the same
+      for (int kb = 0; kb < 2; ++kb) {
+        uint32_t x[3][4];
 #pragma unroll
-      for (int c = 0; c < 3; ++c)
-        ldmatrix4<false>(x[c], img + c * D::kPart + ((lane >> 4) * kDT + (lane & 7)) * D::kPitch + piece * 32 + kb * 16 + ((lane >> 3) & 1) * 8);
-      auto product = [&](int sum, int sc_, int xc) {
-        mma16816(dk[sum], sp[kb][sc_][0], sp[kb][sc_][1], sp[kb][sc_][2], sp[kb][sc_][3], x[xc][0], x[xc][1]);
-        mma16816(dq[sum], sp[kb][sc_][0], sp[kb][sc_][1], sp[kb][sc_][2], sp[kb][sc_][3], x[xc][2], x[xc][3]);
-      };
-      product(0, 0, 0);
-      product(1, 0, 1);
-      product(2, 1, 0);
-      product(3, 2, 0);
-      product(3, 0, 2);
-      product(3, 1, 1);
-    }
-    auto whole = [](const float (&d)[4][4], int e) { return d[0][e] + (d[1][e] + (d[2][e] + d[3][e])); };
-    float* mine = buf + piece * 16 * 20;
-    *reinterpret_cast<float2*>(mine + quad * 20 + pair) = make_float2(whole(dk, 0), whole(dk, 1));
-    *reinterpret_cast<float2*>(mine + (quad + 8) * 20 + pair) = make_float2(whole(dk, 2), whole(dk, 3));
-    *reinterpret_cast<float2*>(mine + quad * 20 + 8 + pair) = make_float2(whole(dq, 0), whole(dq, 1));
-    *reinterpret_cast<float2*>(mine + (quad + 8) * 20 + 8 + pair) = make_float2(whole(dq, 2), whole(dq, 3));
-    // the k parts of the update do not wait for anything: transposed, tokens along the summed side
-    uint32_t kt[3][4];
+        for (int c = 0; c < 3; ++c) ldmatrix4<false>(x[c], rows + c * part + plain + kb * 16);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) ldmatrix4<true>(kt[c], img + c * D::kPart + (lane & 7) * D::kPitch + piece * 32 + (lane >> 3) * 8);
-    auto eight = [&](int at, float (&to)[kDT]) {
-      const float4 x = *reinterpret_cast<const float4*>(ss + at), y = *reinterpret_cast<const float4*>(ss + at + 4);
-      to[0] = x.x; to[1] = x.y; to[2] = x.z; to[3] = x.w; to[4] = y.x; to[5] = y.y; to[6] = y.z; to[7] = y.w;
+        for (int m = 0; m < 6; ++m)
+#pragma unroll
+          for (int nb = 0; nb < 2; ++nb) one(sum[m ? 1 + (m & 1) : 0][nb], kb == 0 && m < 3, sp[kb], x, 2 * nb, m);
+      }
     };
-    float g[kDT], beta[kDT], end[kDT];
-    eight(kDTG, g);
-    eight(kDTBeta, beta);
-    eight(kDTEnd, end);
-    float u[kDT];                                  // first v_i, in the end u_i
+    kb2::mbar_wait(&full[st], (uint32_t)(i / kDTStages & 1));
+    kb2::mbar_wait(&o_free[buf], turn ^ 1u);
+    auto keep = [&](float* to, const float (&sum)[3][2][4]) {
 #pragma unroll
-    for (int t = 0; t < kDT; ++t) u[t] = vs[t * 32 + cg * 16 + col];
-    kb2::named_bar_sync(1 + cg, NI * 32);
-    // every warp of the group solves for the group's 16 columns: a lane per column, the two halves share the row pieces
-    float p[kDT];
+      for (int nb = 0; nb < 2; ++nb) {
+        float v[4];
 #pragma unroll
-    for (int t = 0; t < kDT; ++t) p[t] = 0.f;
-#pragma unroll
-    for (int r = 0; r < (NI + 1) / 2; ++r) {
-      const int pc = NI == 1 ? 0 : half * (NI / 2) + r;
-      const float* from = buf + (pc * 16 + col) * 20;
-      const float4 x = *reinterpret_cast<const float4*>(from), y = *reinterpret_cast<const float4*>(from + 4);
-      if (NI > 1 || half == 0) {
-        p[0] += x.x; p[1] += x.y; p[2] += x.z; p[3] += x.w;
-        p[4] += y.x; p[5] += y.y; p[6] += y.z; p[7] += y.w;
+        for (int e = 0; e < 4; ++e) v[e] = sum[0][nb][e] + (sum[1][nb][e] + sum[2][nb][e]);
+        *reinterpret_cast<float4*>(to + nb * 128) = make_float4(v[0], v[1], v[2], v[3]);
       }
-    }
-#pragma unroll
-    for (int t = 0; t < kDT; ++t) p[t] += __shfl_xor_sync(0xffffffffu, p[t], 16);
-#pragma unroll
-    for (int t = 0; t < kDT; ++t) u[t] = fmaf(-g[t], p[t], u[t]);
-#pragma unroll
-    for (int t = 0; t < kDT; ++t) {
-      u[t] *= beta[t];
-      if (t + 1 < kDT) {
-        float a[kDT];
-        eight(kDTKK + t * kDT, a);
-#pragma unroll
-        for (int m = t + 1; m < kDT; ++m) u[m] = fmaf(-a[m], u[t], u[m]);
-      }
-    }
-    if (half == 0) {                               // D_7j u_j, for the update
-      *reinterpret_cast<float4*>(myu + col * 12) = make_float4(u[0] * end[0], u[1] * end[1], u[2] * end[2], u[3] * end[3]);
-      *reinterpret_cast<float4*>(myu + col * 12 + 4) = make_float4(u[4] * end[4], u[5] * end[5], u[6] * end[6], u[7] * end[7]);
+    };
+    {
+      float ws[3][2][4];
+      product(wim, D::kWPart, ws);
+      keep(mine, ws);
     }
     __syncwarp();
-    const float2 ua = *reinterpret_cast<const float2*>(myu + quad * 12 + pair), ub = *reinterpret_cast<const float2*>(myu + (quad + 8) * 12 + pair);
-    uint32_t up[2][3];
-    split_pair(ua.x, ua.y, up[0]);
-    split_pair(ub.x, ub.y, up[1]);
+    if (lane == 0) kb2::mbar_arrive(&w_there[buf]);
+    float qs[3][2][4];                             // q, under the wait for the other pieces; put away when there is time
+    product(img + D::kWPart, D::kPart, qs);
+    uint32_t kt[2][3][4];                          // k transposed: [16 rows][part]
+#pragma unroll
+    for (int rr = 0; rr < 2; ++rr)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) ldmatrix4<true>(kt[rr][c], img + c * D::kPart + turned + rr * 16);
+    float u[8];
+    {
+      const float4 x = *reinterpret_cast<const float4*>(vs), y = *reinterpret_cast<const float4*>(vs + 4);
+      u[0] = x.x; u[1] = x.y; u[4] = x.z; u[5] = x.w; u[2] = y.x; u[3] = y.y; u[6] = y.z; u[7] = y.w;
+    }
+    const float2 e0 = *reinterpret_cast<const float2*>(ss + kDTEnd + pair), e1 = *reinterpret_cast<const float2*>(ss + kDTEnd + 8 + pair);
     const float total = ss[kDTAll];
+    kb2::mbar_wait(&w_there[buf], turn);
+    float ws[8] = {};
+#pragma unroll
+    for (int pc = 0; pc < NI; ++pc)
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb) {
+        const float4 x = *reinterpret_cast<const float4*>(red + (buf * NI + pc) * 512 + nb * 128 + lane * 4);
+        ws[nb * 4] += x.x; ws[nb * 4 + 1] += x.y; ws[nb * 4 + 2] += x.z; ws[nb * 4 + 3] += x.w;
+      }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) u[e] -= ws[e];
+    if (piece == 0) {
+      *reinterpret_cast<float4*>(ubuf + buf * 256 + lane * 8) = make_float4(u[0], u[1], u[2], u[3]);
+      *reinterpret_cast<float4*>(ubuf + buf * 256 + lane * 8 + 4) = make_float4(u[4], u[5], u[6], u[7]);
+    }
+    uint32_t up[3][4];                             // D_15,j u_j
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {
+      uint32_t p[3];
+      split_pair(u[e] * (e < 4 ? e0.x : e1.x), u[e + 1] * (e < 4 ? e0.y : e1.y), p);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) up[c][e / 2] = p[c];
+    }
+    float big[2][4][4], small[4][4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      float big[4] = {}, small[2][4] = {};
-      mma1688(big, up[0][0], up[1][0], kt[0][r]);
-      mma1688(small[0], up[0][0], up[1][0], kt[1][r]);
-      mma1688(small[1], up[0][1], up[1][1], kt[0][r]);
-      mma1688(small[0], up[0][2], up[1][2], kt[0][r]);
-      mma1688(small[1], up[0][0], up[1][0], kt[2][r]);
-      mma1688(small[0], up[0][1], up[1][1], kt[1][r]);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) S[r][e] = fmaf(S[r][e], total, big[e] + (small[0][e] + small[1][e]));
+      mma1688_new(big[0][r], up[0][0], up[0][1], kt[r >> 1][0][(r & 1) * 2]);
+      mma1688_new(big[1][r], up[0][2], up[0][3], kt[r >> 1][0][(r & 1) * 2 + 1]);
     }
-    // the read-outs are shared out: 8 / (2 NI) tokens per half warp
-    constexpr int kMine = kDT / (2 * NI);
 #pragma unroll
-    for (int m = 0; m < kMine; ++m) {
-      const int t = (piece * 2 + half) * kMine + m;
-      float r = 0.f;
+    for (int m = 1; m < 6; ++m)
 #pragma unroll
-      for (int pc = 0; pc < NI; ++pc) r += buf[(pc * 16 + col) * 20 + 8 + t];
-      float a[kDT], o = ss[kDTG + t] * r;
-      eight(kDTQK + t * kDT, a);
+      for (int r = 0; r < 4; ++r) one(small[r], m < 2, up, kt[r >> 1], (r & 1) * 2, m);
+    keep(mine + 256, qs);
 #pragma unroll
-      for (int j = 0; j < kDT; ++j)
-        if (j <= t) o = fmaf(a[j], u[j], o);           // not by the zeros of later tokens: theirs may be infinite
-      if (i * kDT + t < n) o_out[((t0 + (long long)i * kDT + t) * H + h) * dv + j0 + cg * 16 + col] = o;
-    }
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) S[r][e] = fmaf(S[r][e], total, (big[0][r][e] + big[1][r][e]) + small[r][e]);
     __syncwarp();
-    if (lane == 0) kb2::mbar_arrive(&empty[st]);   // everything of the tile has been read
+    if (lane == 0) {
+      kb2::mbar_arrive(&o_there[buf]);
+      kb2::mbar_arrive(&empty[st]);                // everything of the tile is in registers
+    }
   }
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
     for (int e = 0; e < 4; ++e) Sg[(long long)(r * 8 + pair + (e & 1)) * dv + quad + (e >> 1) * 8] = S[r][e];
+}
+
+// delta_out for long steps with 128 value columns: a warp takes four (token, head) rows, whose loads are in flight together (4096 tokens x 32
+// heads: 52 -> 44 us; a row per warp leaves too few bytes under way).
+__global__ void __launch_bounds__(256) delta_out_rows_kernel(const float* __restrict__ o, const float* __restrict__ gproj, long long ldg, int gate_act, int H,
+                                                             const float* __restrict__ norm_w, float eps, long long rows, void* __restrict__ out, int dt_out) {
+  kb2::pdl_enter(o, gproj, norm_w, out);
+  const long long w = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * 4;
+  const int j = (threadIdx.x & 31) * 4;
+  float4 f[4], g[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const long long r = min(w + i, rows - 1);
+    f[i] = *reinterpret_cast<const float4*>(o + r * 128 + j);
+    g[i] = *reinterpret_cast<const float4*>(gproj + r / H * ldg + r % H * 128 + j);
+  }
+  const float4 nw = *reinterpret_cast<const float4*>(norm_w + j);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float ss = warp_sum((f[i].x * f[i].x + f[i].y * f[i].y) + (f[i].z * f[i].z + f[i].w * f[i].w));
+    const float rstd = 1.f / sqrtf(ss / 128.f + eps);
+    auto finish = [&](float v, float gz, float n) { return v * rstd * n * (gate_act ? 1.f / (1.f + expf(-gz)) : silu(gz)); };
+    const float4 r = make_float4(finish(f[i].x, g[i].x, nw.x), finish(f[i].y, g[i].y, nw.y), finish(f[i].z, g[i].z, nw.z), finish(f[i].w, g[i].w, nw.w));
+    if (w + i >= rows) return;
+    if (dt_out == 0) {
+      *reinterpret_cast<float4*>((float*)out + (w + i) * 128 + j) = r;
+    } else {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(r.x, r.y), hi = __floats2bfloat162_rn(r.z, r.w);
+      *reinterpret_cast<uint2*>((bf16*)out + (w + i) * 128 + j) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+  }
 }
 
 // out[t, h, :] = o / rms(o) * norm_w * silu(gate) (gate_act 1: sigmoid(gate)); a warp per (token, head).  V numbers per access: 4 where sizes
@@ -2065,7 +2362,10 @@ KB2SEQ_API int kb2_seq_residual_post_rms(float* x, const float* y1, float c1, co
 static int delta_out_launch(const float* o, const float* gproj, long long ldg, int gate_act, int H, int dv, const float* norm_w, float eps, int T,
                             void* out, int dt_out, cudaStream_t st) {
   const unsigned blocks = (unsigned)(((long long)T * H + 7) / 8);
-  if (dv % 4 == 0 && ldg % 4 == 0 && !(((uintptr_t)o | (uintptr_t)gproj | (uintptr_t)norm_w | (uintptr_t)out) & 15))
+  const bool vec = dv % 4 == 0 && ldg % 4 == 0 && !(((uintptr_t)o | (uintptr_t)gproj | (uintptr_t)norm_w | (uintptr_t)out) & 15);
+  if (vec && dv == 128 && blocks >= 148 * 16)         // from two full rounds of resident blocks on
+    kb2::launch_pdl(delta_out_rows_kernel, (blocks + 3) / 4, 256, 0, st, o, gproj, ldg, gate_act, H, norm_w, eps, (long long)T * H, out, dt_out);
+  else if (vec)
     kb2::launch_pdl(delta_out_kernel<4>, blocks, 256, 0, st, o, gproj, ldg, gate_act, H, dv, norm_w, eps, T, out, dt_out);
   else
     kb2::launch_pdl(delta_out_kernel<1>, blocks, 256, 0, st, o, gproj, ldg, gate_act, H, dv, norm_w, eps, T, out, dt_out);
@@ -2128,12 +2428,41 @@ static int delta_rule_launch(const float* conv, int C, const float* bproj, long 
   return KB2SEQ_OK;
 }
 
-// scratch: images of k and q [tiles][Hk] | scalars [tiles][H][160] | o [T, H, dv]; at most T / 8 + S tiles, a partial one per sequence
-static long long delta_image_floats(int dk) { return dk == 32 ? DeltaTile<1>::kImage / 2 : dk == 64 ? DeltaTile<2>::kImage / 2 : DeltaTile<4>::kImage / 2; }
+// scratch: images of k and q [tiles][Hk] | of W [tiles][H] | V' [tiles][H][16 dv] | scalars [tiles][H] | o [T, H, dv]; at most T / 16 + S tiles, a
+// partial one per sequence
+struct DeltaScratch {
+  long long tiles, image, wimage, floats;             // floats of an image, of W, of everything
+  DeltaScratch(int T, int S, int H, int Hk, int dk, int dv) : tiles((long long)T / kDT + S) {
+    image = dk == 32 ? DeltaTile<1>::kImage / 2 : dk == 64 ? DeltaTile<2>::kImage / 2 : DeltaTile<4>::kImage / 2;
+    wimage = image / 2;
+    floats = tiles * (Hk * image + H * (wimage + (long long)kDT * dv + kDTScalars)) + (long long)T * H * dv;
+  }
+};
 KB2SEQ_API long long kb2_seq_delta_tiles_scratch(int T, int S, int H, int Hk, int dk, int dv) {
   if (T <= 0 || S <= 0 || H <= 0 || Hk <= 0 || H % Hk || (dk != 32 && dk != 64 && dk != 128) || dv <= 0 || dv % 32) return 0;
-  return ((long long)T / kDT + S) * (Hk * delta_image_floats(dk) + (long long)H * kDTScalars) + (long long)T * H * dv;
+  return DeltaScratch(T, S, H, Hk, dk, dv).floats;
 }
+
+extern "C++" {
+template <int NI, int VB>
+static int launch_delta_tiles(const DeltaScratch& z, DeltaPrep p, float* state, const int* slots, float* scratch, float** o, cudaStream_t st) {
+  using D = DeltaTile<NI>;
+  p.tiles = z.tiles;
+  p.image = (bf16*)scratch;
+  p.wimage = (bf16*)(scratch + z.tiles * p.Hk * z.image);
+  p.vimage = scratch + z.tiles * (p.Hk * z.image + p.H * z.wimage);
+  p.sc = p.vimage + z.tiles * p.H * kDT * p.dv;
+  *o = p.sc + z.tiles * p.H * kDTScalars;
+  SEQ_CUDA(cudaFuncSetAttribute(delta_tile_prep_kernel<NI, VB>, cudaFuncAttributeMaxDynamicSharedMemorySize, D::prep_smem(VB, p.H / p.Hk)));
+  SEQ_CUDA(cudaFuncSetAttribute(delta_tile_kernel<NI>, cudaFuncAttributeMaxDynamicSharedMemorySize, D::kSmem));
+  kb2::launch_pdl(delta_tile_prep_kernel<NI, VB>, (unsigned)(z.tiles * p.Hk), 256, D::prep_smem(VB, p.H / p.Hk), st, p);
+  SEQ_LAUNCHED();
+  kb2::launch_pdl(delta_tile_kernel<NI>, dim3(p.S, p.H, p.dv / 32), D::kThreads, D::kSmem, st, p.image, p.wimage, p.vimage, p.sc, p.H, p.Hk, p.dv, state,
+                  p.cu, slots, *o);
+  SEQ_LAUNCHED();
+  return KB2SEQ_OK;
+}
+}  // extern "C++"
 
 KB2SEQ_API int kb2_seq_delta_tiles(const float* conv, int C, const float* proj, long long ldp, int g_off, int a_off, int b_off, int T, int S, int H,
                                    int Hk, int dk, int dv, const float* A_log, const float* dt_bias, const float* norm_w, float eps, float* state,
@@ -2143,22 +2472,15 @@ KB2SEQ_API int kb2_seq_delta_tiles(const float* conv, int C, const float* proj, 
       scratch_floats < need || ((uintptr_t)scratch & 15) || ((uintptr_t)conv & 15) || C % 4 || C < 2 * Hk * dk + H * dv)
     return failf(KB2SEQ_ERR_VALUE, "delta_tiles: bad argument");
   cudaStream_t st = (cudaStream_t)stream;
-  const long long tiles = (long long)T / kDT + S;
-  bf16* image = (bf16*)scratch;
-  float* sc = scratch + tiles * Hk * delta_image_floats(dk);
-  float* ob = sc + tiles * H * kDTScalars;
-  const unsigned blocks = (unsigned)((tiles * Hk + 7) / 8);
-  const dim3 grid(S, H, dv / 32);
-#define KB2_DT(NIV)                                                                                                                                   \
-  do {                                                                                                                                                \
-    SEQ_CUDA(cudaFuncSetAttribute(delta_tile_kernel<NIV>, cudaFuncAttributeMaxDynamicSharedMemorySize, DeltaTile<NIV>::kSmem));                        \
-    kb2::launch_pdl(delta_tile_prep_kernel<NIV>, blocks, 256, 0, st, conv, C, proj + b_off, ldp, proj + a_off, ldp, H, Hk, A_log, dt_bias, S, cu, tiles, image, sc); \
-    SEQ_LAUNCHED();                                                                                                                                   \
-    kb2::launch_pdl(delta_tile_kernel<NIV>, grid, 64 * NIV + 32, DeltaTile<NIV>::kSmem, st, image, conv, C, 2 * Hk * dk, sc, H, Hk, dv, state, cu, slots, ob);        \
-    SEQ_LAUNCHED();                                                                                                                                   \
-  } while (0)
-  if (dk == 32) KB2_DT(1); else if (dk == 64) KB2_DT(2); else KB2_DT(4);
+  const DeltaScratch z(T, S, H, Hk, dk, dv);
+  DeltaPrep p{};
+  p.conv = conv; p.C = C; p.ldp = ldp; p.bproj = proj + b_off; p.aproj = proj + a_off; p.A_log = A_log; p.dt_bias = dt_bias;
+  p.H = H; p.Hk = Hk; p.dv = dv; p.S = S; p.cu = cu;
+  float* ob = nullptr;
+#define KB2_DT(NIV) (dv % 128 == 0 ? launch_delta_tiles<NIV, 4>(z, p, state, slots, scratch, &ob, st) : launch_delta_tiles<NIV, 1>(z, p, state, slots, scratch, &ob, st))
+  const int rc = dk == 32 ? KB2_DT(1) : dk == 64 ? KB2_DT(2) : KB2_DT(4);      // values in passes of 128 columns, or of 32
 #undef KB2_DT
+  if (rc != KB2SEQ_OK) return rc;
   return delta_out_launch(ob, proj + g_off, ldp, 0, H, dv, norm_w, eps, T, out, dt_out, st);
 }
 

@@ -332,7 +332,7 @@ class GatedDeltaMixer:
             S = len(seqs)
             args = (_row(conv, r0), self.C, _row(proj, r0), proj.stride(0), self.g_off, self.a_off, self.b_off, n, S, self.H, self.Hk, self.dk, self.dv,
                     self.A_log.data_ptr(), self.dt_bias.data_ptr(), self.norm.data_ptr(), self.eps, state.data_ptr(), cu.data_ptr(), slots.data_ptr())
-            if tiles:                    # long portions: eight tokens at a time
+            if tiles:                    # long portions: sixteen tokens at a time
                 size = int(lib.kb2_seq_delta_tiles_scratch(n, S, self.H, self.Hk, self.dk, self.dv))
                 scratch = torch.empty(size, dtype=torch.float32, device=h.device)
                 ops.check(lib.kb2_seq_delta_tiles(*args, scratch.data_ptr(), size, _row(o, r0), ops.dt_code(self.dtype), s))
