@@ -415,6 +415,11 @@ KB2_API int kb2_fmha_maps_slopes(const void* q_dev, const void* k_dev, const voi
                                  int32_t kv_len, int32_t num_q, int32_t num_kv_heads, int32_t maps, int32_t v_dim, float sm_scale,
                                  float softcap, int32_t window, const float* sinks_dev, float* lse_dev, const float* slopes_dev, int32_t device,
                                  void* stream);
+/* The same with the output rows rounded to bf16: out_dev [M][num_q * v_dim]. */
+KB2_API int kb2_fmha_maps_bf16(const void* q_dev, const void* k_dev, const void* v_dev, void* out_dev, int32_t M, int32_t q_start,
+                               int32_t kv_len, int32_t num_q, int32_t num_kv_heads, int32_t maps, int32_t v_dim, float sm_scale,
+                               float softcap, int32_t window, const float* sinks_dev, float* lse_dev, const float* slopes_dev, int32_t device,
+                               void* stream);
 
 /* GEMM -> reduce-scatter fused (head-parallel attention under token sharding): after kb2_{gdn,gqa,mla}_set_output_scatter the
  * block's out_proj GEMM stores every output row straight into the receive buffer of the rank that owns the token

@@ -785,12 +785,13 @@ cudaError_t launch_fmha_latent(const void* q, const void* kv_up, const void* kpe
 }
 
 // Attention core on dense BF16 rows for heads that carry several attention maps: q [M][nq * 128] with nq = heads * maps query
-// vectors (head by head, map by map), k [kv_len][nkv * maps * 128], v [kv_len][nkv * dv], dv 128 or 256; out_f32 [M][nq * dv] fp32.
+// vectors (head by head, map by map), k [kv_len][nkv * maps * 128], v [kv_len][nkv * dv], dv 128 or 256; out_f32 [M][nq * dv] fp32, or, if
+// null, out [M][nq * dv] bf16.
 // Query i stands at position q_start + i of the kv rows and sees the keys with 0 <= position - key < window.
 // softcap > 0: a scaled score s becomes softcap * tanh(s / softcap).  sinks (fp32 [nq], may be null): exp(sink) joins each query vector's
 // softmax denominator.  lse_out (fp32 [M][nq], may be null): the logarithm of that denominator per row.  slopes (fp32 [nq], may be null):
 // slopes[query vector] * (distance to the key) is taken off the (capped) score.
-cudaError_t launch_fmha_maps(const void* q, const void* k, const void* v, float* out_f32, int M, int q_start, int kv_len, int nq, int nkv,
+cudaError_t launch_fmha_maps(const void* q, const void* k, const void* v, float* out_f32, void* out, int M, int q_start, int kv_len, int nq, int nkv,
                              int maps, int dv, float sm_scale, int window, cudaStream_t s, float softcap, const float* sinks, float* lse_out,
                              const float* slopes) {
   if (!(softcap >= 0.f) || !(sm_scale > 0.f)) return cudaErrorInvalidValue;
@@ -818,11 +819,11 @@ cudaError_t launch_fmha_maps(const void* q, const void* k, const void* v, float*
   KernelSpan ks(K_FMHA, s);
   const float sl2 = sm_scale * 1.4426950408889634f;
   if (dv == 256)
-    launch_pdl(gqa_fmha_kernel<128, 256, false>, grid, kFThreads, FmhaSmem<128, 256>::kTotal, s, tq, tk, tk, tv, g, nullptr, nullptr, M, q_start, kv_len,
-                                                                                          sl2, 0, 0, window, sinks, maps, out_f32, cap_in, cap_out, lse_out, slopes, nullptr, 0);
+    launch_pdl(gqa_fmha_kernel<128, 256, false>, grid, kFThreads, FmhaSmem<128, 256>::kTotal, s, tq, tk, tk, tv, g, nullptr, (__nv_bfloat16*)out, M,
+               q_start, kv_len, sl2, 0, 0, window, sinks, maps, out_f32, cap_in, cap_out, lse_out, slopes, nullptr, 0);
   else
-    launch_pdl(gqa_fmha_kernel<128, 128, false>, grid, kFThreads, FmhaSmem<128, 128>::kTotal, s, tq, tk, tk, tv, g, nullptr, nullptr, M, q_start, kv_len,
-                                                                                          sl2, 0, 0, window, sinks, maps, out_f32, cap_in, cap_out, lse_out, slopes, nullptr, 0);
+    launch_pdl(gqa_fmha_kernel<128, 128, false>, grid, kFThreads, FmhaSmem<128, 128>::kTotal, s, tq, tk, tk, tv, g, nullptr, (__nv_bfloat16*)out, M,
+               q_start, kv_len, sl2, 0, 0, window, sinks, maps, out_f32, cap_in, cap_out, lse_out, slopes, nullptr, 0);
   return cudaGetLastError();
 }
 

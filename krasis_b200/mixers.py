@@ -275,10 +275,9 @@ class WindowLatentAttention:
             from . import capi
             for i in seqs:
                 row0, n, start, _ = tb.layout[i]
-                lo, rows = ops.key_rows(tb, i, self.window, page_size)
-                kv_up = lin(ckv.view(-1, self.r).index_select(0, rows), self.w_kv_up, torch.bfloat16)     # [keys, H * (128 + 128)]
-                kpe = kr.view(-1, self.dr).index_select(0, rows)
-                q_bf = proj[row0:row0 + n, :H * (self.dn + self.dr)].to(torch.bfloat16).contiguous()
+                lo = max(0, start - self.window + 1)
+                lat, kpe, q_bf = ops.portion_rows(tb, i, lo, ckv, self.r, kr, self.dr, page_size, proj, row0, n, H * (self.dn + self.dr))
+                kv_up = lin(lat, self.w_kv_up, torch.bfloat16)                                            # [keys, H * (128 + 128)]
                 o_rows = torch.empty((n, H, self.dv), dtype=torch.bfloat16, device=h.device) if gated else o[row0:row0 + n]
                 capi.check(core.kb2_fmha_latent_gated(q_bf.data_ptr(), kv_up.data_ptr(), kpe.data_ptr(), o_rows.data_ptr(), n, start - lo,
                                                       start - lo + n, H, self.scale, min(self.window, 1 << 30), ops._ptr(self.sink),
@@ -813,44 +812,25 @@ class MultiMapAttention:
         """Convolution tail [slots, C, taps - 1] in a RecurrentStatePool (None without a convolution)."""
         return pool.register(self.C, max(self.K - 1, 1)) if self.K else None
 
-    def _tensor_core_portion(self, core, proj, a, tb, i, kc, vc, page_size, stream, lse=None):
-        """Sequence i of the step on the tcgen05 kernel: a[rows of the portion] = per-map attention outputs (fp32)."""
-        import numpy as np
+    def _tensor_core_portion(self, core, proj, a, o, r0, tb, i, kc, vc, page_size, stream, lse=None):
+        """Sequence i of the step on the tcgen05 kernel: a[its rows] = per-map attention outputs (fp32), or without a its rows of o (bfloat16).
+        a and lse begin at row r0 of the step."""
         from . import capi
-        row0, n, start, pages = tb.layout[i]
+        row0, n, start, _ = tb.layout[i]
         H, G, M, d, dv, chunk = self.H, self.G, self.M, self.d, self.dv, self.chunk
         first = start // chunk * chunk if chunk else 0
         first = max(first, start - self.window + 1)
-        key = ("rows_from", i, first, page_size)                  # the layers of a step share the row list of a sequence
-        if key not in tb._key_rows:
-            j = np.arange(first, start + n, dtype=np.int64)
-            host = torch.from_numpy(np.asarray(pages, dtype=np.int64)[j // page_size] * page_size + j % page_size)
-            tb._key_rows[key] = host.to(proj.device, non_blocking=True)
-        rows = tb._key_rows[key]
-        k_rows = kc.view(-1, G * M * d).index_select(0, rows)
-        v_rows = vc.view(-1, G * dv).index_select(0, rows)
-        q = proj[row0:row0 + n, :H * M * d].to(torch.bfloat16).contiguous()
-        pos = start
+        k_rows, v_rows, q = ops.portion_rows(tb, i, first, kc, G * M * d, vc, G * dv, page_size, proj, row0, n, H * M * d)
+        dev, pos = proj.device.index or 0, start
         while pos < start + n:
             cstart = pos // chunk * chunk if chunk else 0
             end = min(start + n, cstart + chunk) if chunk else start + n
             lo = max(cstart, first)
-            m = end - pos
-            if self.slopes is not None:
-                capi.check(core.kb2_fmha_maps_slopes(q[pos - start:].data_ptr(), k_rows[lo - first:].data_ptr(), v_rows[lo - first:].data_ptr(),
-                                                     a[row0 + pos - start:].data_ptr(), m, pos - lo, end - lo, H * M, G, M, dv, self.scale,
-                                                     self.softcap, min(self.window, 1 << 30), ops._ptr(self.sink), None,
-                                                     self.map_slopes.data_ptr(), proj.device.index or 0, stream))
-            elif self.sink is not None or lse is not None:
-                capi.check(core.kb2_fmha_maps_sink(q[pos - start:].data_ptr(), k_rows[lo - first:].data_ptr(), v_rows[lo - first:].data_ptr(),
-                                                   a[row0 + pos - start:].data_ptr(), m, pos - lo, end - lo, H * M, G, M, dv, self.scale,
-                                                   self.softcap, min(self.window, 1 << 30), ops._ptr(self.sink),
-                                                   lse[row0 + pos - start:].data_ptr() if lse is not None else None,
-                                                   proj.device.index or 0, stream))
-            else:
-                capi.check(core.kb2_fmha_maps_softcap(q[pos - start:].data_ptr(), k_rows[lo - first:].data_ptr(), v_rows[lo - first:].data_ptr(),
-                                                      a[row0 + pos - start:].data_ptr(), m, pos - lo, end - lo, H * M, G, M, dv, self.scale,
-                                                      self.softcap, min(self.window, 1 << 30), proj.device.index or 0, stream))
+            m, row = end - pos, row0 + pos - start
+            args = (_row(q, pos - start), _row(k_rows, lo - first), _row(v_rows, lo - first), _row(o, row) if a is None else _row(a, row - r0), m, pos - lo,
+                    end - lo, H * M, G, M, dv, self.scale, self.softcap, min(self.window, 1 << 30))
+            extra = (ops._ptr(self.sink), _row(lse, row - r0), ops._ptr(self.map_slopes))
+            capi.check((core.kb2_fmha_maps_bf16 if a is None else core.kb2_fmha_maps_slopes)(*args, *extra, dev, stream))
             pos = end
 
     def forward(self, h: torch.Tensor, tb: ops.StepTables, kc: torch.Tensor, vc: torch.Tensor, page_size: int, tail=None, pooled=None) -> torch.Tensor:
@@ -873,23 +853,27 @@ class MultiMapAttention:
         if self.pool:                                # the tokens that complete a block write its mean key and value
             ops.check(lib.kb2_seq_kv_pool(kc.data_ptr(), vc.data_ptr(), kp.data_ptr(), vp.data_ptr(), dtc, G * M * self.d, G * self.dv, self.pool,
                                           T, tb.positions.data_ptr(), tb.seq_of.data_ptr(), tb.pages.data_ptr(), tb.max_pages, page_size, s))
-        a = torch.empty((T, H, M, self.dv), dtype=torch.float32, device=h.device)
         o = torch.empty((T, H * self.dv), dtype=self.dtype, device=h.device)
         gate = proj_in[:, self.gate_off:] if self.gate_off >= 0 else None
         core = _core_lib() if self.tc_shape else False
         # long portions on the tensor cores, the others on the plain kernel with a key range of their own to cut (beside one portion of 512
         # tokens, three decoded tokens at 2048 keys take 15 us instead of 230 uncut)
         runs = portion_runs(tb, self.tc_min_portion if core else None)
-        lse = torch.empty((T, H), dtype=torch.float32, device=h.device) if self.pool and any(run[0] for run in runs) else None
         for fast, seqs, r0, rows in runs:
-            self._attend(core if fast else None, proj, a, o, gate, tb, seqs, r0, rows, kc, vc, kp, vp, page_size, s, lse)
+            self._attend(core if fast else None, proj, o, gate, tb, seqs, r0, rows, kc, vc, kp, vp, page_size, s)
         return lin(o, self.w_o, torch.float32)
 
-    def _attend(self, core, proj, a, o, gate, tb, seqs, r0, T, kc, vc, kp, vp, page_size, s, lse):
-        """Rows r0 .. r0 + T - 1 of the step (the sequences `seqs`): attention into a, the finished heads into o.  core: the library whose
+    def _attend(self, core, proj, o, gate, tb, seqs, r0, T, kc, vc, kp, vp, page_size, s):
+        """Rows r0 .. r0 + T - 1 of the step (the sequences `seqs`): attention, the finished heads into o.  core: the library whose
         tensor-core attention runs these portions, None for the plain kernel."""
         lib, H, G, M, dtc, dev = ops.load(), self.H, self.G, self.M, ops.dt_code(kc.dtype), proj.device
+        if core is not None and M == 1 and self.map_coef is None and not self.unit_norm and gate is None and self.vfreq is None and not self.pool:
+            for q in seqs:                           # heads that are finished as the attention leaves them: rounded there
+                self._tensor_core_portion(core, proj, None, o, r0, tb, q, kc, vc, page_size, s)
+            return
         positions, seq_of, window = _row(tb.positions, r0), _row(tb.seq_of, r0), min(self.window, 1 << 30)
+        a = torch.empty((T, H, M, self.dv), dtype=torch.float32, device=dev)
+        lse = torch.empty((T, H), dtype=torch.float32, device=dev) if self.pool and core is not None else None
         nsplit, part_acc, part_ml = 1, None, None
 
         def plain(out, acc, ml, pool_only):
@@ -908,17 +892,17 @@ class MultiMapAttention:
             if nsplit > 1:
                 part_acc = torch.empty((T * H * M, nsplit, self.dv), dtype=torch.float32, device=dev)
                 part_ml = torch.empty((T * H * M, nsplit, 2), dtype=torch.float32, device=dev)
-            plain(_row(a, r0), part_acc, part_ml, False)
+            plain(a.data_ptr(), part_acc, part_ml, False)
         else:
             for q in seqs:
-                self._tensor_core_portion(core, proj, a, tb, q, kc, vc, page_size, s, lse=lse)
+                self._tensor_core_portion(core, proj, a, o, r0, tb, q, kc, vc, page_size, s, lse=lse)
             if self.pool:                            # the pooled blocks of the long portions: a second pass, joined by the log-sum-exps
                 p_acc = torch.empty((T * H, self.dv), dtype=torch.float32, device=dev)
                 p_ml = torch.empty((T * H, 2), dtype=torch.float32, device=dev)
-                plain(_row(a, r0), p_acc, p_ml, True)
-                ops.check(lib.kb2_seq_pool_merge(_row(a, r0), _row(lse, r0), p_acc.data_ptr(), p_ml.data_ptr(), T, H, self.dv,
+                plain(a.data_ptr(), p_acc, p_ml, True)
+                ops.check(lib.kb2_seq_pool_merge(a.data_ptr(), lse.data_ptr(), p_acc.data_ptr(), p_ml.data_ptr(), T, H, self.dv,
                                                  seq_of, tb.cu.data_ptr(), self.tc_min_portion, s))
-        ops.check(lib.kb2_seq_attn_finish(_row(a, r0), ops._ptr(part_acc), ops._ptr(part_ml), nsplit, T, H, M, self.dv, ops._ptr(self.map_coef),
+        ops.check(lib.kb2_seq_attn_finish(a.data_ptr(), ops._ptr(part_acc), ops._ptr(part_ml), nsplit, T, H, M, self.dv, ops._ptr(self.map_coef),
                                           int(self.unit_norm), self.eps, self.post_scale, _row(gate, r0),
                                           gate.stride(0) if gate is not None else proj.stride(0), _row(o, r0), ops.dt_code(self.dtype), None,
                                           None, 0, int(self.gate_wide), positions, ops._ptr(self.vfreq), int(self.rot_half), s))

@@ -33,6 +33,7 @@ SIGNATURES = {
     "kb2_seq_delta_rule_ch": (_I, [_P, _I, _P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _F, _P, _P, _P, _P, _P, _I, _P]),
     "kb2_seq_residual_add_norm": (_I, [_P, _P, _P, _P, _P, _P, _I, _I, _I, _F, _P]),
     "kb2_seq_head_kv_prep": (_I, [_P, _L, _I, _I, _I, _I, _I, _I, _P, _P, _P, _F, _P, _I, _P, _P, _P, _I, _I, _P, _P, _I, _I, _I, _P, _F, _I, _P]),
+    "kb2_seq_portion_rows": (_I, [_P, _I, _P, _I, _P, _I, _I, _I, _P, _P, _P, _L, _I, _I, _P, _P]),
     "kb2_seq_kv_pool": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _I, _P]),
     "kb2_seq_paged_attn": (_I, [_P, _L, _I, _I, _I, _I, _I, _I, _P, _P, _I, _P, _P, _P, _I, _I, _F, _I, _I, _P, _I, _P, _P, _P, _I, _F, _P, _I,
                                 _P, _P, _I, _P, _P]),
@@ -162,7 +163,6 @@ class StepTables:
         for toks, start, _, pages in entries:
             self.layout.append((row, len(toks), int(start), list(pages)))
             row += len(toks)
-        self._key_rows = {}
         self.max_portion = max(len(e[0]) for e in entries)
         if device_buf is not None:
             if device_buf.numel() != n:
@@ -178,18 +178,18 @@ class StepTables:
         self.h2d_bytes = n * 4
 
 
-def key_rows(tb: StepTables, s: int, window: int, page_size: int):
-    """Cache rows of the keys sequence s needs in this step under a sliding window: (first key position, int64 rows on the device),
-    computed once per step and window size."""
-    key = (s, window, page_size)
-    if key not in tb._key_rows:
-        import numpy as np
-        _, n, start, pages = tb.layout[s]
-        lo = max(0, start - window + 1)
-        j = np.arange(lo, start + n, dtype=np.int64)
-        rows = np.asarray(pages, dtype=np.int64)[j // page_size] * page_size + j % page_size
-        tb._key_rows[key] = (lo, torch.from_numpy(rows).to(tb.buf.device, non_blocking=True))
-    return tb._key_rows[key]
+def portion_rows(tb: StepTables, s: int, first: int, ca: torch.Tensor, wa: int, cb: torch.Tensor, wb: int, page_size: int, proj: torch.Tensor,
+                 row0: int, n: int, nq: int):
+    """The operands of sequence s's attention on the tensor cores, made in one launch: rows `first` up to the portion's end of two bfloat16
+    caches (wa and wb numbers per row), and the first nq columns of proj's rows row0 .. row0 + n - 1 (fp32), rounded to bfloat16."""
+    _, m, start, _ = tb.layout[s]
+    keys, dev = start + m - first, proj.device
+    a = torch.empty((keys, wa), dtype=torch.bfloat16, device=dev)
+    b = torch.empty((keys, wb), dtype=torch.bfloat16, device=dev)
+    q = torch.empty((n, nq), dtype=torch.bfloat16, device=dev)
+    check(load().kb2_seq_portion_rows(ca.data_ptr(), wa, cb.data_ptr(), wb, tb.pages.data_ptr() + 4 * s * tb.max_pages, page_size, first, keys,
+                                      a.data_ptr(), b.data_ptr(), proj.data_ptr() + row0 * proj.stride(0) * 4, proj.stride(0), n, nq, q.data_ptr(), _s(proj)))
+    return a, b, q
 
 
 def embed(table: torch.Tensor, tokens: torch.Tensor, scale: float) -> torch.Tensor:
