@@ -12,10 +12,7 @@ import numpy as np
 import torch
 
 from . import capi
-
-
-def _stream(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+from .streams import stream_on as _stream
 
 
 def _bf16_host(t) -> np.ndarray:

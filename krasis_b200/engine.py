@@ -17,6 +17,7 @@ import numpy as np
 import torch
 
 from . import capi
+from .streams import stream_on as _stream_ptr
 
 _SCORING = {"softmax": capi.SCORE_SOFTMAX, "sigmoid": capi.SCORE_SIGMOID, "topk_softmax": capi.SCORE_TOPK_SOFTMAX}
 
@@ -32,11 +33,6 @@ class QuantizedExperts:
     w13_s: np.ndarray
     w2_q: np.ndarray
     w2_s: np.ndarray
-
-
-def _stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
-
 
 class KrasisEngine:
     """Weight store + routing config behind the C ABI (the B200 counterpart of `#[pyclass] KrasisEngine`).

@@ -6,10 +6,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import capi
-
-
-def _s(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+from .streams import stream_of as _s, stream_on
 
 
 def _dev(t):
@@ -54,7 +51,7 @@ def sum_slots(slots_ptr: int, world: int, rows: int, hidden: int, device: torch.
     """bf16(sum over the `world` partial rows of every token) from a peer-filled receive buffer [rows][world][hidden] bf16."""
     out = torch.empty((rows, hidden), dtype=torch.bfloat16, device=device)
     capi.check(capi.load().kb2_sum_slots_bf16(slots_ptr, world, out.data_ptr(), rows, hidden, device.index or 0,
-                                              torch.cuda.current_stream(device).cuda_stream))
+                                              stream_on(device)))
     return out
 
 

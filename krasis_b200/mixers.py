@@ -47,6 +47,7 @@ import os
 import torch
 
 from . import seqops as ops
+from .streams import stream_of, stream_on
 
 
 # rows up to which kb2_seq_gemm runs its GEMV kernels
@@ -54,19 +55,20 @@ GEMV_ROWS = 8
 # tokens from which a portion runs the delta rule in tiles (prep, rule and read-out at 64 tokens 25 us either way, at 256 59 (tiles) against 80 us,
 # at 16 17 against 13), and tokens from which its attention runs on the tensor cores
 TILE_PORTION, TC_PORTION = 64, 128
-_core = None
+_core = _core_check = None
 
 
 def _core_lib():
-    """The core library's tcgen05 GEMM, if that library has been built (it is optional for models that run on seqops alone)."""
-    global _core
+    """The core library's tcgen05 GEMM, if that library has been built (it is optional for models that run on seqops alone); _core_check then maps
+    its error codes onto exceptions."""
+    global _core, _core_check
     if _core is None:
         _core = False
         if os.environ.get("KB2_SEQ_TCGEN05", "1") != "0":
             try:
                 from . import capi
                 if os.path.exists(capi.LIB_PATH):
-                    _core = capi.load()
+                    _core, _core_check = capi.load(), capi.check
             except Exception:       # noqa: BLE001 — optional accelerator; the generic kernel computes the same product
                 _core = False
     return _core
@@ -83,11 +85,9 @@ def lin(a: torch.Tensor, w: torch.Tensor, out_dtype=torch.float32, min_n: int = 
             and w.is_contiguous() and w.shape[1] == K and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
         core = _core_lib()
         if core:
-            from . import capi
-            out = torch.empty((M, N), dtype=out_dtype, device=a.device)
+            out, dev = torch.empty((M, N), dtype=out_dtype, device=a.device), a.get_device()
             fn = core.kb2_linear_bf16 if M >= 256 and N >= min_n else core.kb2_linear_bf16_chunked
-            capi.check(fn(a.data_ptr(), w.data_ptr(), None, out.data_ptr(), M, N, K, int(out_dtype == torch.float32), a.device.index or 0,
-                          torch.cuda.current_stream(a.device).cuda_stream))
+            _core_check(fn(a.data_ptr(), w.data_ptr(), None, out.data_ptr(), M, N, K, out_dtype == torch.float32, dev, stream_on(dev)))
             return out
     # at 8 rows and fewer the GEMV, which is three times as exact as the parts (1.6e-7 against 4.7e-7 at K = 2048)
     if a.dtype == torch.float32 and M > GEMV_ROWS and out_dtype in (torch.float32, torch.bfloat16):
@@ -109,15 +109,13 @@ def _lin_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
     core = _core_lib()
     if not core:
         return False
-    from . import capi
-    dev, wide = a.device.index or 0, int(w.dtype == torch.float32)
+    dev, wide = a.get_device(), int(w.dtype == torch.float32)
     size = core.kb2_linear_f32_workspace(M, N, K, wide, G, dev)
     if not size:
         return False
     work = torch.empty(size, dtype=torch.uint8, device=a.device)
-    capi.check(core.kb2_linear_f32(a.data_ptr(), a.stride(0), a.stride(1), w.data_ptr(), wide, out.data_ptr(), int(out.dtype == torch.float32),
-                                   out.stride(0), out.stride(1), M, N, K, G, work.data_ptr(), size, dev,
-                                   torch.cuda.current_stream(a.device).cuda_stream))
+    _core_check(core.kb2_linear_f32(a.data_ptr(), a.stride(0), a.stride(1), w.data_ptr(), wide, out.data_ptr(), int(out.dtype == torch.float32),
+                                    out.stride(0), out.stride(1), M, N, K, G, work.data_ptr(), size, dev, stream_on(dev)))
     return True
 
 
@@ -242,7 +240,7 @@ class WindowLatentAttention:
             proj = lin(ops.rms_rows(proj_in[:, :self.q_cols], self.dq_norm, self.eps, self.dtype), self.w_uq, torch.float32)
             lat = proj_in[:, self.q_cols:]
         ldp = proj.stride(0)
-        s = torch.cuda.current_stream(h.device).cuda_stream
+        s = stream_of(h)
         dtc = ops.dt_code(ckv.dtype)
         ops.check(lib.kb2_seq_latent_prep(proj.data_ptr(), ldp, T, H, self.dn, self.dr, self.r, self.dkv_norm.data_ptr(), self.eps,
                                           self.freq.data_ptr(), self.rot_dims, self.amp, tb.positions.data_ptr(), tb.seq_of.data_ptr(),
@@ -317,7 +315,7 @@ class GatedDeltaMixer:
     def forward(self, h: torch.Tensor, tb: ops.StepTables, tail: torch.Tensor, state: torch.Tensor) -> torch.Tensor:
         lib, T = ops.load(), h.shape[0]
         proj = lin(h, self.w_in, torch.float32)
-        s = torch.cuda.current_stream(h.device).cuda_stream
+        s = stream_of(h)
         conv = torch.empty((T, self.C), dtype=torch.float32, device=h.device)
         ops.check(lib.kb2_seq_conv_silu(proj.data_ptr(), proj.stride(0), T, tb.S, self.C, self.K, self.taps.data_ptr(), tail.data_ptr(),
                                         tb.seq_of.data_ptr(), tb.cu.data_ptr(), tb.slots.data_ptr(), conv.data_ptr(), s))
@@ -394,7 +392,7 @@ class GatedLinearAttention:
         ops.check(lib.kb2_seq_gla(proj.data_ptr(), proj.stride(0), self.q_off, self.k_off, self.v_off, dec_in.data_ptr(), dec_in.stride(0),
                                   self.a2_b.data_ptr(), self.tau, self.q_scale, T, tb.S, H, self.dk, self.dv, state.data_ptr(),
                                   tb.cu.data_ptr(), tb.slots.data_ptr(), ops._ptr(scratch), o.data_ptr(),
-                                  torch.cuda.current_stream(h.device).cuda_stream))
+                                  stream_of(h)))
         o = ops.head_norm_gate(o, H, self.dv, self.dtype, norm=self.norm, eps=self.eps, gate=proj[:, self.g_off:], gate_act="silu")
         return lin(o, self.w_o, torch.float32)
 
@@ -435,7 +433,7 @@ class SelectiveScan:
                                              xp.data_ptr(), xp.stride(0), self.R, proj.data_ptr(), proj.stride(0), self.C,
                                              self.A_log.data_ptr(), self.D.data_ptr(), T, tb.S, self.C, self.N, state.data_ptr(),
                                              tb.cu.data_ptr(), tb.slots.data_ptr(), y.data_ptr(), ops.dt_code(self.dtype),
-                                             torch.cuda.current_stream(h.device).cuda_stream))
+                                             stream_of(h)))
         return lin(y, self.w_o, torch.float32)
 
 
@@ -480,7 +478,7 @@ class MatrixMemory:
         ops.check(lib.kb2_seq_mlstm(proj.data_ptr(), proj.stride(0), self.q_off, self.k_off, self.v_off, self.i_off, self.f_off, ops._ptr(self.i_b),
                                     ops._ptr(self.f_b), self.cap, float(self.dk) ** -0.5, T, tb.S, H, self.dk, self.dv, state.data_ptr(),
                                     nstate.data_ptr(), mstate.data_ptr(), tb.cu.data_ptr(), tb.slots.data_ptr(), small.data_ptr(), o.data_ptr(),
-                                    small[3].data_ptr(), torch.cuda.current_stream(h.device).cuda_stream))
+                                    small[3].data_ptr(), stream_of(h)))
         o = ops.head_norm_gate(o, H, self.dv, self.dtype, norm=self.norm, eps=self.eps, gate=proj[:, self.g_off:], gate_act="sigmoid", den=small[3])
         return lin(o, self.w_o, torch.float32)
 
@@ -525,7 +523,7 @@ class GatedRecurrentUnit:
     def _gate_products(self, u: torch.Tensor):
         """u [T, C] fp32 -> (products, row stride, block stride) with both gates of a channel bs columns apart."""
         T, dev = u.shape[0], u.device
-        s = torch.cuda.current_stream(dev).cuda_stream
+        s = stream_on(dev)
         core = _core_lib() if self.w_gates_twice is not None and T >= self.tc_min_tokens else False
         if not core:
             z = torch.empty((T, self.B, 2 * self.bs), dtype=torch.float32, device=dev)
@@ -553,7 +551,7 @@ class GatedRecurrentUnit:
         ops.check(ops.load().kb2_seq_rglru(u.data_ptr(), u.stride(0), z.data_ptr(), ldz, zb, proj[:, self.C:].data_ptr(), proj.stride(0),
                                            ops._ptr(self.ra_b), ops._ptr(self.ri_b), ops._ptr(self.y_b), self.rate.data_ptr(), T, tb.S, self.C,
                                            self.bs, state.data_ptr(), tb.cu.data_ptr(), tb.slots.data_ptr(), o.data_ptr(), ops.dt_code(self.dtype),
-                                           torch.cuda.current_stream(h.device).cuda_stream))
+                                           stream_of(h)))
         return lin(o, self.w_o, torch.float32)
 
 
@@ -621,7 +619,7 @@ class ChannelDeltaMixer:
     def forward(self, h: torch.Tensor, tb: ops.StepTables, tail: torch.Tensor, state: torch.Tensor) -> torch.Tensor:
         lib, T, H = ops.load(), h.shape[0], self.H
         proj = lin(h, self.w_in, torch.float32)
-        s = torch.cuda.current_stream(h.device).cuda_stream
+        s = stream_of(h)
         conv = ops.conv(proj, self.C, self.taps, None, True, tail, tb)
         dec_in = self._second(proj, self.a_off, self.ra, self.w_a2)                 # [T, H dk]
         gate_in = self._second(proj, self.g_off, self.rg, self.w_g2)                # [T, H dv]
@@ -843,7 +841,7 @@ class MultiMapAttention:
         if self.K:                                   # q | k | v through the convolution (bias first); the gate columns stay in proj_in
             proj, bias = ops.conv(proj_in, self.C, self.taps, self.bias, False, tail, tb), None
         ldp = proj.stride(0)
-        s = torch.cuda.current_stream(h.device).cuda_stream
+        s = stream_of(h)
         dtc = ops.dt_code(kc.dtype)
         ops.check(lib.kb2_seq_head_kv_prep(proj.data_ptr(), ldp, T, H, G if self.own_kv else 0, M, self.d, self.dv, ops._ptr(bias),
                                            ops._ptr(self.q_norm), ops._ptr(self.k_norm), self.eps, ops._ptr(self.freq), self.rot_dims,
@@ -981,7 +979,7 @@ class RoutedExperts:
              "pos": ints[3 * E + 2 + max_tiles + max_rows:], "max_rows": max_rows, "max_tiles": max_tiles}
         fn = ops.load().kb2_seq_moe_bin if tile % self.tile == 0 else ops.load().kb2_seq_moe_bin16
         ops.check(fn(ids.data_ptr(), slots, E, tile, t["counts"].data_ptr(), t["offs"].data_ptr(), t["cursor"].data_ptr(), t["tile_expert"].data_ptr(),
-                     t["n_tiles"].data_ptr(), t["slot_row"].data_ptr(), max_rows, t["pos"].data_ptr(), torch.cuda.current_stream(dev).cuda_stream))
+                     t["n_tiles"].data_ptr(), t["slot_row"].data_ptr(), max_rows, t["pos"].data_ptr(), stream_on(dev)))
         return t
 
     def _tensor_core_ok(self, h, slots):
@@ -1009,7 +1007,7 @@ class RoutedExperts:
         weights; many: the 128 x 256 tiles of the dense GEMM."""
         from . import capi
         core, E, top, W, F, dev = _core_lib(), self.E, self.top, h.shape[1], self.F, h.device
-        s = torch.cuda.current_stream(dev).cuda_stream
+        s = stream_on(dev)
         tile = self._tile_rows(slots)
         t = self._bin(ids, slots, tile)
         rows, di = t["max_rows"], dev.index or 0
@@ -1037,7 +1035,7 @@ class RoutedExperts:
 
     def forward(self, h: torch.Tensor) -> torch.Tensor:
         lib, T, W, E, top = ops.load(), h.shape[0], h.shape[1], self.E, self.top
-        dev, s = h.device, torch.cuda.current_stream(h.device).cuda_stream
+        dev, s = h.device, stream_of(h)
         ids, wts, z = self.route(h)
         dt, dtc = self.dtype, ops.dt_code(self.dtype)
         slots = T * top

@@ -93,12 +93,19 @@ class Scheduler:
         if not ran:
             tb = ops.StepTables(packed, self.model.device)
             self.h2d_bytes += tb.h2d_bytes
-            want_rows = torch.tensor(rows, dtype=torch.int64, device=self.model.device) if rows else None
+            want_rows = self._rows(rows) if rows else None
             logits = self.model.forward_step(tb, want_rows)
         for rid, tokens, _ in entries:
             self.live[rid].kv.advance(len(tokens))
         self.steps_run += 1
         return logits
+
+    def _rows(self, rows) -> torch.Tensor:
+        """Row numbers on the device.  From pinned memory: a copy from pageable memory waits for all work that is queued, and the GPU then stands
+        idle while the launches of this step are prepared (two prompt steps and 16 decoded ones: 6.2 -> 5.5 ms)."""
+        dev = torch.device(self.model.device)
+        host = torch.tensor(rows, dtype=torch.int64, pin_memory=dev.type == "cuda")
+        return host.to(dev, non_blocking=True)
 
     def _decode_step_graphed(self, packed, rows):
         """One decoded token per entry, replayed from a CUDA graph.  Returns (ran, logits); ran is False where the eager path has to run."""
@@ -143,7 +150,7 @@ class Scheduler:
             return True, None
         if rows == list(range(S)):
             return True, out.clone()            # the graph's own output buffer is overwritten by the next replay
-        return True, out.index_select(0, torch.tensor(rows, dtype=torch.int64, device=dev))
+        return True, out.index_select(0, self._rows(rows))
 
     # ------------------------------------------------------------------------------------------- generation
     def generate(self, prompts: Sequence[Sequence[int]], max_new_tokens: int, sampling: Optional[SamplingParams] = None,

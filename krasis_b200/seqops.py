@@ -9,6 +9,8 @@ import os
 
 import torch
 
+from .streams import stream_of as _s
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "_lib", "libkrasis_b200_seq.so")
 
@@ -113,10 +115,6 @@ def dt_code(dtype) -> int:
     if dtype == torch.bfloat16:
         return 1
     raise ValueError(f"unsupported dtype {dtype}: float32 or bfloat16")
-
-
-def _s(t) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
 
 
 def _cuda(t, name):
