@@ -17,7 +17,9 @@
 // Intelligence Datatype For Higher-Precision Computations", ARITH 2019).  The parts of a tile's rows lie side by side on the N side, so one
 // weight tile serves all of them: w x1 goes to the main accumulators, w x2 and w x3 to two small ones.  With fp32 weights in three parts
 // too, w1 [x1 x2 x3], w2 [x1 x2] and w3 [x1] are added in: six of the nine products, the other three are below 2^-26 of the result.  512 rows,
-// N 16384, K 2048: 231 us, 2-norm error 4.7e-7; fp32-FMA tiles 1494 us, 8.1e-7.
+// N 16384, K 2048: 231 us, 2-norm error 4.7e-7; fp32-FMA tiles 1494 us, 8.1e-7.  Where w2 and w3 are zeros (the fp32 form of a bf16 checkpoint),
+// the pass that makes the parts says so per 128 rows x 256 columns; they are then neither written nor loaded nor multiplied: the same sums to
+// the last bit, 180 us (weights of 134 MB among them: 4 bytes of each read, 2 written).
 #include <cuda.h>
 
 #include <algorithm>
@@ -39,6 +41,8 @@ struct SplitArgs {
   const float* bias;
   long long ldo, out_group, w_part_rows;
   int M, N, n_kblocks, mt, xparts, wparts, stages, chunk, tmem_cols, tiles_per_group;
+  const uint8_t* w_low;      // wparts 3: [group][tile of 128 rows][low_spans], whether w2 and w3 hold anything in low_span K blocks
+  int low_span, low_spans;
   const int* tile_group;
   const int* n_tiles_dev;
   const float* x_raw;
@@ -72,8 +76,8 @@ __global__ void __launch_bounds__(kSThreads)
     split_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const SplitArgs p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int row_tile = blockIdx.x / KS, rank = blockIdx.x % KS;
-  const int nt = p.xparts * p.mt, w_bytes = p.wparts * kSWBytes, stage_bytes = w_bytes + nt * 128;
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + p.stages * stage_bytes);
+  const int nt = p.xparts * p.mt, ring_bytes = p.stages * (p.wparts * kSWBytes + nt * 128);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + ring_bytes);
   uint64_t* empty = full + kSMaxStages;
   uint64_t* done = empty + kSMaxStages;
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(done + 1);
@@ -84,7 +88,7 @@ __global__ void __launch_bounds__(kSThreads)
 
   if (threadIdx.x == 32) {
     if (smem_u32(smem) & 1023u) __trap();
-    for (int i = 0; i < p.stages; ++i) {
+    for (int i = 0; i < kSMaxStages; ++i) {
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
     }
@@ -107,20 +111,37 @@ __global__ void __launch_bounds__(kSThreads)
   }
   const int group = p.tile_group != nullptr ? p.tile_group[row_tile] : p.tiles_per_group > 0 ? row_tile / p.tiles_per_group : 0;
   const int w0 = n0 + group * p.N;                                                             // row of W
+  // spans of K blocks in which w2 and w3 take part; none: stages without room for them
+  uint32_t low = 0;
+  if (p.wparts > 1) {
+    const uint8_t* said = p.w_low + (long long)(group * gridDim.y + blockIdx.y) * p.low_spans;
+    const bool mine = lane >= kb0 / p.low_span && lane <= (kb1 - 1) / p.low_span;
+    low = __ballot_sync(0xffffffffu, mine && said[lane] != 0);
+  }
+  const int w_bytes = low ? 3 * kSWBytes : kSWBytes, stage_bytes = w_bytes + nt * 128, stages = min(kSMaxStages, ring_bytes / stage_bytes);
+
+  int span = low ? kb0 / p.low_span : 0, span_left = (span + 1) * p.low_span - kb0;      // of the K block at hand
+  auto next_block = [&]() {
+    if (--span_left == 0) {
+      ++span;
+      span_left = p.low_span;
+    }
+  };
 
   if (warp == 0) {
     int stage = 0;
     uint32_t phase = 0;
-    for (int kb = kb0; kb < kb1; ++kb) {
+    for (int kb = kb0; kb < kb1; ++kb, next_block()) {
       mbar_wait(&empty[stage], phase ^ 1);
       uint8_t* a = smem + stage * stage_bytes;
       if (elect_one()) {
-        mbar_arrive_expect_tx(&full[stage], stage_bytes);
-        for (int q = 0; q < p.wparts; ++q) tma_load_2d(a + q * kSWBytes, &tmap_w, kb * kBlockK, w0 + (int)(q * p.w_part_rows), &full[stage]);
+        const int w_parts = low >> span & 1 ? 3 : 1;
+        mbar_arrive_expect_tx(&full[stage], w_parts * kSWBytes + nt * 128);
+        for (int q = 0; q < w_parts; ++q) tma_load_2d(a + q * kSWBytes, &tmap_w, kb * kBlockK, w0 + (int)(q * p.w_part_rows), &full[stage]);
         tma_load_2d(a + w_bytes, &tmap_x, kb * kBlockK, row_tile * nt, &full[stage]);
       }
       __syncwarp();
-      if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      if (++stage == stages) { stage = 0; phase ^= 1; }
     }
   } else if (warp == 1) {
     int stage = 0;
@@ -129,7 +150,7 @@ __global__ void __launch_bounds__(kSThreads)
     const uint32_t small = tmem_base;                                        // w x2, w x3 and what the further parts of w bring
     uint32_t acc = tmem_base + (p.xparts > 1 ? 2 * p.mt : 0);                // w x1, a set of columns per chunk
     int in_chunk = 0;
-    for (int kb = kb0; kb < kb1; ++kb) {
+    for (int kb = kb0; kb < kb1; ++kb, next_block()) {
       mbar_wait(&full[stage], phase);
       tc_fence_after_sync();
       const uint32_t a_addr = smem_u32(smem + stage * stage_bytes);
@@ -142,7 +163,7 @@ __global__ void __launch_bounds__(kSThreads)
           const uint64_t bd2 = umma_desc_k_sw128(a_addr + w_bytes + p.mt * 128);
 #pragma unroll
           for (int k = 0; k < 4; ++k) umma_bf16(small, ad + 2 * k, bd2 + 2 * k, idesc2, (kb > kb0 || k > 0) ? 1u : 0u);
-          if (p.wparts > 1) {
+          if (low >> span & 1) {
             const uint64_t ad2 = umma_desc_k_sw128(a_addr + kSWBytes), ad3 = umma_desc_k_sw128(a_addr + 2 * kSWBytes);
 #pragma unroll
             for (int k = 0; k < 4; ++k) umma_bf16(small, ad2 + 2 * k, bd + 2 * k, idesc2, 1u);             // w2 [x1 x2]
@@ -154,7 +175,7 @@ __global__ void __launch_bounds__(kSThreads)
       }
       __syncwarp();
       if (++in_chunk == p.chunk) { in_chunk = 0; acc += p.mt; }
-      if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      if (++stage == stages) { stage = 0; phase ^= 1; }
     }
     if (elect_one()) umma_commit(done);
     __syncwarp();
@@ -374,6 +395,10 @@ cudaError_t launch_split_gemm(const SplitGemm& g, const SplitPlan& plan, cudaStr
   p.x_ld = g.x_ld;
   p.x_group = g.x_group;
   p.w_raw = g.w_raw;
+  p.w_low = g.w_low;
+  p.low_span = split_low_span(g.K);
+  p.low_spans = ceil_div(nkb, p.low_span);
+  if (g.wparts > 1 && g.w_low == nullptr) return cudaErrorInvalidValue;
   const int ring = plan.stages * (g.wparts * kSWBytes + nt * 128);
   // a CTA that waits for tensor memory may have cluster peers that others wait for in turn, so co-resident CTAs must never ask for more
   // than the 512 columns together: each takes at least 430 bytes of shared memory per column (1 KB of it is the system's); of 228 KB that
@@ -443,6 +468,61 @@ __global__ void __launch_bounds__(256) split_parts_kernel(const float* __restric
     for (int q = 0; q < 3; ++q)
       *reinterpret_cast<uint4*>(parts + ((tile * 3 + q) * mt + in) * K + c) = make_uint4(o[q][0], o[q][1], o[q][2], o[q][3]);
   }
+}
+
+// The parts of weights, [3][groups * N][K].  A block makes those of 128 rows x `cols` columns; it writes the low ones only if one of them is not
+// zero (usually seen in its first round, or else in a second pass over what it has just read) and says so in `low`.
+template <bool kVec>
+__global__ void __launch_bounds__(512) split_weight_parts_kernel(const float* __restrict__ w, int N, int K, long long all_rows, int tiles, int cols, int spans,
+                                                                 __nv_bfloat16* __restrict__ parts, uint8_t* __restrict__ low) {
+  pdl_enter(w, parts, low);
+  const int span = blockIdx.x % spans, gt = blockIdx.x / spans, group = gt / tiles, n0 = gt % tiles * 128, c0 = span * cols;
+  const int k8 = min(cols, K - c0) >> 3, total = min(128, N - n0) * k8;
+  const long long first = (long long)group * N + n0;
+  bool any = false, write = false;
+  for (int pass = 0; pass < 2; ++pass) {
+    for (int base = 0; base < total; base += 512) {
+      const int i = base + threadIdx.x;
+      const long long at = (first + i / k8) * K + c0 + i % k8 * 8;
+      float v[8];
+      uint32_t o[3][4];
+      if (i < total) {
+        const float* src = w + at;
+        if constexpr (kVec) {
+          const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+          v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = src[j];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint32_t a[3], b[3];
+          split3(v[2 * j], a[0], a[1], a[2]);
+          split3(v[2 * j + 1], b[0], b[1], b[2]);
+#pragma unroll
+          for (int q = 0; q < 3; ++q) o[q][j] = a[q] | (b[q] << 16);
+          any |= (o[1][j] | o[2][j]) != 0;
+        }
+        if (pass == 0) *reinterpret_cast<uint4*>(parts + at) = make_uint4(o[0][0], o[0][1], o[0][2], o[0][3]);
+      }
+      if (pass == 0 && base == 0) write = __syncthreads_or(any);
+      if (write && i < total)
+#pragma unroll
+        for (int q = 1; q < 3; ++q) *reinterpret_cast<uint4*>(parts + q * all_rows * K + at) = make_uint4(o[q][0], o[q][1], o[q][2], o[q][3]);
+    }
+    if (write || !__syncthreads_or(any)) break;
+    write = true;                                    // seen later on: once more for the low parts
+  }
+  if (threadIdx.x == 0) low[blockIdx.x] = write;
+}
+
+cudaError_t launch_split_weights(const float* w, int N, int K, int groups, void* parts, uint8_t* low, cudaStream_t s) {
+  KernelSpan span(K_DENSE_BF16, s);
+  const int tiles = ceil_div(N, kSRows), cols = split_low_span(K) * kBlockK, spans = ceil_div(K, cols);
+  const unsigned blocks = (unsigned)groups * tiles * spans;
+  auto kern = (uintptr_t)w & 15 ? split_weight_parts_kernel<false> : split_weight_parts_kernel<true>;
+  return launch_pdl(kern, blocks, 512, 0, s, w, N, K, (long long)groups * N, tiles, cols, spans, (__nv_bfloat16*)parts, low);
 }
 
 cudaError_t launch_split_parts(const float* x, long long ld, long long group_stride, int rows, int K, int mt, int groups, void* parts,

@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstdint>
+
 namespace kb2 {
 
 // 64-wide K blocks per accumulator of sums in chunks.  The tensor core truncates when it adds to an accumulator: the error of a sum grows by
@@ -39,7 +41,11 @@ struct SplitGemm {
   const float* x_raw = nullptr;
   long long x_ld = 0, x_group = 0;
   const void* w_raw = nullptr;              // fp32 when wparts is 3, else bf16; rows of K
+  const uint8_t* w_low = nullptr;           // wparts 3: what launch_split_weights says about the low parts
 };
+
+// K blocks for which launch_split_weights says together whether the low parts of 128 rows hold anything: at most 32 such spans
+inline int split_low_span(int K) { return K / 64 > 128 ? (K / 64 + 31) / 32 : 4; }
 
 // One accumulator over all of K, K block by K block: the sums of dense_gemm.cu, bit for bit.  false: its 128 x 256 tiles are the better cut.
 bool split_gemm_plan_whole(int M, int N, int K, int num_sms, SplitPlan* out);
@@ -54,5 +60,9 @@ cudaError_t launch_split_gemm(const SplitGemm& g, const SplitPlan& plan, cudaStr
 // [groups][tiles][3][mt][K] with zero rows behind the last one
 cudaError_t launch_split_parts(const float* x, long long ld, long long group_stride, int rows, int K, int mt, int groups, void* parts, int num_sms,
                                cudaStream_t s);
+
+// fp32 weights [groups][N][K] -> [3][groups * N][K]; low [groups][tiles of 128 rows][spans]: whether parts two and three of those rows and K blocks
+// hold anything.  If not, they are not written.
+cudaError_t launch_split_weights(const float* w, int N, int K, int groups, void* parts, uint8_t* low, cudaStream_t s);
 
 }  // namespace kb2
