@@ -50,10 +50,6 @@ struct SplitArgs {
   const void* w_raw;
 };
 
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float4 ld_dsmem_f4(uint32_t local_addr, uint32_t rank) {
   uint32_t a;
   float4 v;
@@ -325,12 +321,11 @@ static bool cheapest(int M, int N, int K, bool whole, int num_sms, int xparts, i
   return found;
 }
 
-// The 128 x 256 tiles of dense_gemm.cu take 0.355 us per K block and 5 us around it; taken here only where that is more.  Measured on both sides
-// of the line: M 1000, N 2048, K 2048 12.1 against 18.3 us; M 2048 at the same shape 23.2 against 18.7; M 256, N 12352 21.7 against 23.0;
-// M 515 39.5 against 39.0.
-bool split_gemm_plan_whole(int M, int N, int K, int num_sms, SplitPlan* out) {
+// Taken only where the wide tiles of dense_gemm.cu are estimated to take longer (us).  Measured on both sides of the line (this / wide): M 1000, N 2048,
+// K 2048 14.0 / 14.4 us; M 2000 at the same shape 25.2 / 18.2; M 515, N 12288 26.6 / 32.1; M 700 32.2 / 32.0; M 256, N 9216 15.6 / 15.3.
+bool split_gemm_plan_whole(int M, int N, int K, int num_sms, float us, SplitPlan* out) {
   if (M <= 0 || M > 2048 || K % kBlockK || N % 16) return false;
-  float best = 0.355f * (K / kBlockK) * ceil_div((long long)ceil_div(M, 128) * ceil_div(N, 256), num_sms) + 5.f;
+  float best = us;
   return cheapest(M, N, K, true, num_sms, 1, 1, 1, 1, &best, out);
 }
 

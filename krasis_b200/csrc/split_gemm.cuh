@@ -47,8 +47,8 @@ struct SplitGemm {
 // K blocks for which launch_split_weights says together whether the low parts of 128 rows hold anything: at most 32 such spans
 inline int split_low_span(int K) { return K / 64 > 128 ? (K / 64 + 31) / 32 : 4; }
 
-// One accumulator over all of K, K block by K block: the sums of dense_gemm.cu, bit for bit.  false: its 128 x 256 tiles are the better cut.
-bool split_gemm_plan_whole(int M, int N, int K, int num_sms, SplitPlan* out);
+// One accumulator over all of K, K block by K block: the sums of dense_gemm.cu, bit for bit.  false: not estimated to take less than `us`.
+bool split_gemm_plan_whole(int M, int N, int K, int num_sms, float us, SplitPlan* out);
 // Sums in chunks, in an order that depends on N, K, the parts and the groups, not on M.  false: sizes not taken.
 bool split_gemm_plan(int M, int N, int K, int num_sms, int xparts, int wparts, int groups, SplitPlan* out);
 // binned rows (one weight matrix per row tile): a CTA per tile and 128 columns, K uncut
