@@ -31,7 +31,10 @@
 // every shape, and the accumulators stood still for 3000 cycles per item while four warps drained them.  Two groups, pauses between polls (half of
 // all instructions were polls), and waits under the MMAs: gate/up of 8192 x 10 tokens over 512 experts (H 2048, I 512, INT4) 316 -> 273 us, down
 // 197 -> 182; 389 x 6 over 64 experts (I 1408, INT8, with short chunks) 106 -> 75 and 60 -> 43.  Left: the wide K loop takes 830 cycles per block
-// for 640 of MMAs, with 29 KB of tiles per block through the SM's copy engine; the short one is bound by issue slots (60 % busy).
+// for 640 of MMAs, with 29 KB of tiles per block through the SM's copy engine.  The short one waited for its weight producer, which takes 480 cycles
+// to issue four copies: with the packed tiles of two K blocks per copy 100 tokens x 10 of 512 experts (INT4) take 139 -> 125 us (gate/up) and 80 -> 72,
+// 590 cycles per K block; left there are the MMAs of its issuer (47 cycles each at 16 tokens) and its two waits.  Two issuing warps, one per tile, made
+// the MMAs themselves slower (755 cycles per block); asking for the next operands ahead of the MMAs 522 per block, but nothing on the whole.
 // TMEM columns: [0,192) acc0 | [192,384) acc1 | [384,512) two A stages x (tile0 32 cols | tile1 32 cols)
 // Short chunks (at most 64 tokens, launched where experts get few rows): the kernel above waited for weights, with 34-35 KB of them in flight per
 // SM, and its B and staging tiles lay idle.  The short form's rings: see SmemLayout.
@@ -81,13 +84,16 @@ struct SmemLayout {
   // token (B operand) ring: 4 stages wherever they fit the 227 KB (everything but the 12 KB Affine8 tiles).  With tcgen05.mma issued
   // at full rate the K loop waited ~200 cycles per k-block on token rows with 3 stages (profiles/r02i_gemm_item_timeline_*).
   static constexpr int kStagesB = kShort ? 6 : (FMT == kFmtAffine8) ? 3 : 4;
-  static constexpr int kWStageBytes = 2 * Fmt<FMT>::kTileBytes + (kHasScaleTiles<FMT> ? 2 * kScaleTileBytes : 0);
+  // K blocks per stage of packed weights: two, whose tiles lie side by side and whose scales are the same, wherever two stages of two fit.  The
+  // producer takes 480 cycles to issue four copies; one K block each, that was the pace of the short form whatever the format.
+  static constexpr int kKbW = kShort || Fmt<FMT>::kStagesW >= 4 ? 2 : 1;
+  static constexpr int kWStageBytes = 2 * kKbW * Fmt<FMT>::kTileBytes + (kHasScaleTiles<FMT> ? 2 * kScaleTileBytes : 0);
   static constexpr int kStageRowBytes = 2 * kTileRows * 2;   // epilogue staging: 512 B per token (gate|up or two down tiles)
   static constexpr int kOffB = 0;                                               // 1024-aligned (swizzle atoms)
   static constexpr int kOffStage = kOffB + kStagesB * kBStageBytes;
   static constexpr int kOffW = kOffStage + NT * kStageRowBytes;
   static constexpr int kFitW = (227 * 1024 - 1024 - kOffW) / kWStageBytes;      // 1 KB left for weights of slots and barriers
-  static constexpr int kStagesW = !kShort ? Fmt<FMT>::kStagesW : kFitW < 16 ? kFitW : 16;
+  static constexpr int kStagesW = !kShort ? Fmt<FMT>::kStagesW / kKbW : kFitW < 16 ? kFitW : 16;
   static constexpr int kOffSlotW = kOffW + kStagesW * kWStageBytes;             // GEMM2: routing weight of the chunk's token slots (f32)
   static constexpr int kOffBar = kOffSlotW + NT * 4;
   static constexpr int kNumBars = 2 * kStagesW + 2 * kStagesA + 2 * kStagesB + 2 * kAccBufs;
@@ -155,7 +161,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
   constexpr int kStagesA = L::kStagesA, kAccBufs = L::kAccBufs, kAcc1Col = L::kAcc1Col, kATmemCol = L::kATmemCol;
   constexpr int kBStageBytes = L::kBStageBytes;
   constexpr int kStagesW = L::kStagesW;
-  constexpr int TB = Fmt<FMT>::kTileBytes;
+  constexpr int TB = Fmt<FMT>::kTileBytes, kKbW = L::kKbW;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kOffBar);
   uint64_t* w_full = bars;
@@ -179,7 +185,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
     if (smem_u32(smem) & 1023u) __trap();   // the 128B-swizzle atoms need a 1024 B aligned base
     for (int i = 0; i < kStagesW; ++i) {
       mbar_init(&w_full[i], 1);
-      mbar_init(&w_empty[i], kNumDequantThreads);
+      mbar_init(&w_empty[i], kKbW * kNumDequantThreads);
     }
     for (int i = 0; i < kStagesA; ++i) {
       mbar_init(&a_full[i], kNumDequantThreads);
@@ -224,19 +230,19 @@ __global__ void __launch_bounds__(kNumThreads, 1)
         const uint8_t* ws_e = p.ws + (long long)cd.expert * p.ws_expert_stride;
         const int ngroups = nkb / 2;
         long long wacc = 0;
-        for (int kb = 0; kb < nkb; ++kb) {
+        for (int kb = 0; kb < nkb; kb += kKbW) {     // K is a multiple of 128
           const long long c0 = tracing ? clock64() : 0;
           mbar_wait_paused<64>(&w_empty[rw.stage], rw.phase ^ 1);
           if (tracing) wacc += clock64() - c0;
           uint8_t* dst = smem + L::kOffW + rw.stage * L::kWStageBytes;
           if (elect_one()) {
             mbar_arrive_expect_tx(&w_full[rw.stage], L::kWStageBytes);
-            bulk_g2s(dst, wq_e + ((long long)t0 * nkb + kb) * TB, TB, &w_full[rw.stage]);
-            bulk_g2s(dst + TB, wq_e + ((long long)t1 * nkb + kb) * TB, TB, &w_full[rw.stage]);
+            bulk_g2s(dst, wq_e + ((long long)t0 * nkb + kb) * TB, kKbW * TB, &w_full[rw.stage]);
+            bulk_g2s(dst + kKbW * TB, wq_e + ((long long)t1 * nkb + kb) * TB, kKbW * TB, &w_full[rw.stage]);
             if constexpr (kHasScaleTiles<FMT>) {
-              bulk_g2s(dst + 2 * TB, ws_e + ((long long)t0 * ngroups + (kb >> 1)) * kScaleTileBytes, kScaleTileBytes,
+              bulk_g2s(dst + 2 * kKbW * TB, ws_e + ((long long)t0 * ngroups + (kb >> 1)) * kScaleTileBytes, kScaleTileBytes,
                        &w_full[rw.stage]);
-              bulk_g2s(dst + 2 * TB + kScaleTileBytes, ws_e + ((long long)t1 * ngroups + (kb >> 1)) * kScaleTileBytes,
+              bulk_g2s(dst + 2 * kKbW * TB + kScaleTileBytes, ws_e + ((long long)t1 * ngroups + (kb >> 1)) * kScaleTileBytes,
                        kScaleTileBytes, &w_full[rw.stage]);
             }
           }
@@ -386,7 +392,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
     Ring rw, ra;
     int first = odd;
     if (odd) {
-      rw.advance(kStagesW);
+      if (kKbW == 1) rw.advance(kStagesW);
       ra.advance(kStagesA);
     }
     const uint32_t lane_base = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kATmemCol + tile * kATileCols;
@@ -398,17 +404,18 @@ __global__ void __launch_bounds__(kNumThreads, 1)
         mbar_wait_paused<32>(&w_full[rw.stage], rw.phase);
         if (dtr) ww_ += clock64() - c0;
         const uint8_t* wsrc = smem + L::kOffW + rw.stage * L::kWStageBytes;
+        const uint8_t* wt = wsrc + (tile * kKbW + (kb & (kKbW - 1))) * TB;
         __nv_bfloat16 s = __float2bfloat16_rn(0.f);
-        if constexpr (kHasScaleTiles<FMT>) s = reinterpret_cast<const __nv_bfloat16*>(wsrc + 2 * TB)[tile * kTileRows + t];
+        if constexpr (kHasScaleTiles<FMT>) s = reinterpret_cast<const __nv_bfloat16*>(wsrc + 2 * kKbW * TB)[tile * kTileRows + t];
         uint32_t o[32];
         if constexpr (FMT == kFmtQ8_0) {
           // w = bf16(f32(d) * q): the f32 product of an fp16 and an int8 is exact, so this is one rounding (src/gguf.rs:574-593)
-          const uint32_t dd = *reinterpret_cast<const uint32_t*>(wsrc + tile * TB + kTileRows * kBlockK + t * 4);
+          const uint32_t dd = *reinterpret_cast<const uint32_t*>(wt + kTileRows * kBlockK + t * 4);
           const float d0 = __half2float(__ushort_as_half((unsigned short)(dd & 0xFFFF)));
           const float d1 = __half2float(__ushort_as_half((unsigned short)(dd >> 16)));
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const uint4 w = *reinterpret_cast<const uint4*>(wsrc + tile * TB + q * 2048 + t * 16);
+            const uint4 w = *reinterpret_cast<const uint4*>(wt + q * 2048 + t * 16);
             const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
             const float sf = q < 2 ? d0 : d1;
 #pragma unroll
@@ -421,12 +428,12 @@ __global__ void __launch_bounds__(kNumThreads, 1)
         } else if constexpr (FMT == kFmtAffine8) {
           // GGUF Q6_K / Q5_K / Q5_0 / Q4_0 decoded at load time into int8 codes + (a, b) per 16 elements:
           // w = bf16(fma(a, code, -b)) — a, b and a*code are exact in f32, so this is the reference's single f32 rounding
-          const float4 p0 = *reinterpret_cast<const float4*>(wsrc + tile * TB + kTileRows * kBlockK + t * 32);
-          const float4 p1 = *reinterpret_cast<const float4*>(wsrc + tile * TB + kTileRows * kBlockK + t * 32 + 16);
+          const float4 p0 = *reinterpret_cast<const float4*>(wt + kTileRows * kBlockK + t * 32);
+          const float4 p1 = *reinterpret_cast<const float4*>(wt + kTileRows * kBlockK + t * 32 + 16);
           const float av[4] = {p0.x, p0.z, p1.x, p1.z}, bv[4] = {p0.y, p0.w, p1.y, p1.w};
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const uint4 w = *reinterpret_cast<const uint4*>(wsrc + tile * TB + q * 2048 + t * 16);
+            const uint4 w = *reinterpret_cast<const uint4*>(wt + q * 2048 + t * 16);
             const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
@@ -438,14 +445,14 @@ __global__ void __launch_bounds__(kNumThreads, 1)
         } else if constexpr (FMT == kFmtQ4_K) {
           // w = bf16((d*sc)*q - (dmin*mn)) evaluated like src/gguf.rs:711-730: d*sc and dmin*mn exact in f32,
           // (d*sc)*q exact, one f32 rounding at the subtraction (fmaf), then BF16.
-          const uint2 hd = *reinterpret_cast<const uint2*>(wsrc + tile * TB + kTileRows * kBlockK / 2 + t * 8);
+          const uint2 hd = *reinterpret_cast<const uint2*>(wt + kTileRows * kBlockK / 2 + t * 8);
           const float d = __half2float(__ushort_as_half((unsigned short)(hd.x & 0xFFFF)));
           const float dmin = __half2float(__ushort_as_half((unsigned short)(hd.x >> 16)));
           const float dl = d * (float)(hd.y & 0xFF), ml = dmin * (float)((hd.y >> 8) & 0xFF);
           const float dh = d * (float)((hd.y >> 16) & 0xFF), mh = dmin * (float)(hd.y >> 24);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            const uint4 w = *reinterpret_cast<const uint4*>(wsrc + tile * TB + h * 2048 + t * 16);
+            const uint4 w = *reinterpret_cast<const uint4*>(wt + h * 2048 + t * 16);
             const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -468,7 +475,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
           const __nv_bfloat162 s2 = __halves2bfloat162(s, s);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            const uint4 w = *reinterpret_cast<const uint4*>(wsrc + tile * TB + h * 2048 + t * 16);
+            const uint4 w = *reinterpret_cast<const uint4*>(wt + h * 2048 + t * 16);
             const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -483,7 +490,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
           const __nv_bfloat162 s2 = __halves2bfloat162(s, s);
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const uint4 w = *reinterpret_cast<const uint4*>(wsrc + tile * TB + q * 2048 + t * 16);
+            const uint4 w = *reinterpret_cast<const uint4*>(wt + q * 2048 + t * 16);
             const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
             for (int e = 0; e < 8; ++e) o[q * 8 + e] = deq_pair_int8(ww[e >> 1], e & 1, s2);
@@ -499,7 +506,8 @@ __global__ void __launch_bounds__(kNumThreads, 1)
         tc_fence_before_sync();
         mbar_arrive(&a_full[ra.stage]);
         if (dtr) { wae += c2 - c1; wst += clock64() - c2; }
-        rw.advance2(kStagesW);
+        if constexpr (kKbW == 1) rw.advance2(kStagesW);
+        else rw.advance(kStagesW);
         ra.advance2(kStagesA);
       }
       first ^= nkb & 1;
