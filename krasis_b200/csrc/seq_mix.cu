@@ -910,31 +910,6 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __res
   kb2::pdl_enter(y, pos_of_slot, ids, weights, h, shared, out, shared_gate);
   const long long t = blockIdx.x;
   const float sgate = shared_gate != nullptr ? 1.f / (1.f + expf(-shared_gate[t * ldsg])) : 1.f;   // the shared expert's weight for this token
-  if ((W & 3) == 0 && dt_h == 1) {           // four columns per thread, 16-byte loads of the expert rows; same order of the sum over k
-    for (int d = threadIdx.x * 4; d < W; d += blockDim.x * 4) {
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int k = 0; k < top; ++k) {
-        const long long slot = t * top + k;
-        const int e = ids[slot];
-        const float w = weights ? weights[slot] : 1.f;
-        if (e >= 0 && e < E) {
-          const long long p = pos_of_slot ? pos_of_slot[slot] : slot;
-          const float4 r = *reinterpret_cast<const float4*>(y + p * W + d);
-          v.x = fmaf(w, r.x, v.x); v.y = fmaf(w, r.y, v.y); v.z = fmaf(w, r.z, v.z); v.w = fmaf(w, r.w, v.w);
-        } else if (e >= E && e < E + ident) {
-          const bf16* hp = (const bf16*)h + t * W + d;
-          v.x = fmaf(w, __bfloat162float(hp[0]), v.x); v.y = fmaf(w, __bfloat162float(hp[1]), v.y);
-          v.z = fmaf(w, __bfloat162float(hp[2]), v.z); v.w = fmaf(w, __bfloat162float(hp[3]), v.w);
-        }
-      }
-      if (shared != nullptr) {
-        const float4 r = *reinterpret_cast<const float4*>(shared + t * W + d);
-        v.x = fmaf(sgate, r.x, v.x); v.y = fmaf(sgate, r.y, v.y); v.z = fmaf(sgate, r.z, v.z); v.w = fmaf(sgate, r.w, v.w);
-      }
-      *reinterpret_cast<float4*>(out + t * W + d) = v;
-    }
-    return;
-  }
   for (int d = threadIdx.x; d < W; d += blockDim.x) {
     float v = 0.f;
     for (int k = 0; k < top; ++k) {
@@ -951,6 +926,59 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __res
     if (shared != nullptr) v = fmaf(sgate, shared[t * W + d], v);
     out[t * W + d] = v;
   }
+}
+
+// The same for widths that are multiples of 4: a block per token and 1024 columns, four per thread.  Where a token's rows lie is looked up once, by a
+// thread per choice, and eight rows are in flight together; with the look-ups and one row after the other 128 tokens x 6 x 2048 took 10.4 us instead
+// of 4.7.  Same order of the sum over the choices.
+constexpr int kCombineTop = 64;
+__global__ void __launch_bounds__(256) moe_combine_vec_kernel(const float* __restrict__ y, const int* __restrict__ pos_of_slot, const int* __restrict__ ids,
+                                                              const float* __restrict__ weights, int top, int E, int ident, const bf16* __restrict__ h,
+                                                              const float* __restrict__ shared, float* __restrict__ out, int W,
+                                                              const float* __restrict__ shared_gate, long long ldsg) {
+  kb2::pdl_enter(y, pos_of_slot, ids, weights, h, shared, out, shared_gate);
+  __shared__ long long row[kCombineTop];               // of y; -1: the token itself (identity expert), -2: nothing
+  __shared__ float wt[kCombineTop];
+  const long long t = blockIdx.x;
+  const int d = (blockIdx.y * 256 + threadIdx.x) * 4;
+  float4 own = make_float4(0.f, 0.f, 0.f, 0.f);
+  float sgate = 1.f;
+  if (shared != nullptr) {
+    if (d < W) own = *reinterpret_cast<const float4*>(shared + t * W + d);
+    if (shared_gate != nullptr) sgate = 1.f / (1.f + expf(-shared_gate[t * ldsg]));
+  }
+  if (threadIdx.x < top) {
+    const long long slot = t * top + threadIdx.x;
+    const int e = ids[slot];
+    row[threadIdx.x] = e >= 0 && e < E ? (pos_of_slot ? pos_of_slot[slot] : slot) : e >= E && e < E + ident ? -1 : -2;
+    wt[threadIdx.x] = weights ? weights[slot] : 1.f;
+  }
+  __syncthreads();
+  if (d >= W) return;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k0 = 0; k0 < top; k0 += 8) {
+    float4 r[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const long long p = k0 + i < top ? row[k0 + i] : -2;
+      if (p >= 0) {
+        r[i] = *reinterpret_cast<const float4*>(y + p * W + d);
+      } else if (p == -1) {
+        const bf16* hp = h + t * W + d;
+        r[i] = make_float4(__bfloat162float(hp[0]), __bfloat162float(hp[1]), __bfloat162float(hp[2]), __bfloat162float(hp[3]));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (k0 + i < top && row[k0 + i] != -2) {
+        const float w = wt[k0 + i];
+        v.x = fmaf(w, r[i].x, v.x); v.y = fmaf(w, r[i].y, v.y); v.z = fmaf(w, r[i].z, v.z); v.w = fmaf(w, r[i].w, v.w);
+      }
+  }
+  if (shared != nullptr) {
+    v.x = fmaf(sgate, own.x, v.x); v.y = fmaf(sgate, own.y, v.y); v.z = fmaf(sgate, own.z, v.z); v.w = fmaf(sgate, own.w, v.w);
+  }
+  *reinterpret_cast<float4*>(out + t * W + d) = v;
 }
 
 }  // namespace kb2seq
@@ -1203,7 +1231,11 @@ KB2SEQ_API int kb2_seq_moe_combine(const float* y, const int* pos_of_slot, const
                                    long long ldsg, void* stream) {
   if (!ids || (!weights && ident > 0) || !out || T <= 0 || top <= 0 || E < 0 || ident < 0 || W <= 0 || (E > 0 && !y) || (ident > 0 && (!h || bad_dt(dt_h))))
     return failf(KB2SEQ_ERR_VALUE, "moe_combine: bad argument");
-  kb2::launch_pdl(moe_combine_kernel, T, 256, 0, (cudaStream_t)stream, y, pos_of_slot, ids, weights, top, E, ident, h, dt_h, shared, out, W, shared_gate, ldsg);
+  const bool aligned = !(((uintptr_t)y | (uintptr_t)shared | (uintptr_t)out) & 15);
+  if (W % 4 == 0 && dt_h == 1 && top <= kCombineTop && aligned)
+    kb2::launch_pdl(moe_combine_vec_kernel, dim3(T, (W + 1023) / 1024), 256, 0, (cudaStream_t)stream, y, pos_of_slot, ids, weights, top, E, ident,
+                    (const bf16*)h, shared, out, W, shared_gate, ldsg);
+  else kb2::launch_pdl(moe_combine_kernel, T, 256, 0, (cudaStream_t)stream, y, pos_of_slot, ids, weights, top, E, ident, h, dt_h, shared, out, W, shared_gate, ldsg);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
 }
