@@ -240,6 +240,17 @@ KB2_API int kb2_linear_bf16_binned(const void* x_dev, const void* w_dev, void* o
 KB2_API int kb2_linear_bf16_chunked(const void* x_dev, const void* w_dev, const float* bias_dev, void* out_dev, int32_t M, int32_t N, int32_t K,
                                     int32_t out_f32, int32_t device, void* stream);
 
+/* A gated unit on a product: out[M][F] = unit(x . gate^T, x . up^T) in bf16 for w = [gate ; up] of [2 F][K], both products rounded to bf16 first:
+ * the bits of kb2_linear_bf16 (kb2_linear_bf16_chunked below 256 rows) into bf16 and an activation pass.  kind 0: gelu_tanh(g) u, 1: silu(g) u,
+ * 2: g' sigmoid(alpha g') (u' + 1) with g' = min(g, limit), u' = clamp(u, -limit, limit).  For sizes that kb2_linear_glu_bf16_takes (others run on
+ * wide tiles, without a unit).  The binned form is that of kb2_linear_bf16_binned. */
+KB2_API int32_t kb2_linear_glu_bf16_takes(int32_t M, int32_t F, int32_t K, int32_t device);
+KB2_API int kb2_linear_glu_bf16(const void* x_dev, const void* w_dev, void* out_dev, int32_t M, int32_t F, int32_t K, int32_t kind, float limit,
+                                float alpha, int32_t device, void* stream);
+KB2_API int kb2_linear_glu_bf16_binned(const void* x_dev, const void* w_dev, void* out_dev, int32_t M, int32_t F, int32_t K, int32_t kind, float limit,
+                                       float alpha, int32_t tile_rows, const int32_t* tile_group_dev, const int32_t* num_row_tiles_dev, int32_t groups,
+                                       int32_t device, void* stream);
+
 /* Products of fp32 rows on the tensor cores with the accuracy of fp32 sums: out[g][m] = x[g][m] . w[g]^T for M rows in each of `groups` groups,
  * x fp32 (row stride x_ld, group stride x_group), w [groups][N][K] fp32 (w_f32) or bf16, out fp32 or bf16 (row stride out_ld, group stride
  * out_group, multiples of 4).  K % 64 == 0, N % 16 == 0.  A row's sums depend on N, K and groups, not on M.  The operands are cut into bf16

@@ -162,6 +162,31 @@ KB2_API int kb2_linear_bf16_chunked(const void* x_dev, const void* w_dev, const 
   return KB2_OK;
 }
 
+// the plan of the product that kb2_linear_glu_bf16 ends in a gated unit; false: the product runs on wide tiles
+static bool glu_plan(int32_t M, int32_t F, int32_t K, int32_t device, SplitPlan* plan) {
+  const int sms = device_sms(device);
+  if (M <= 0 || F <= 0 || F % 16 || K <= 0 || K % 64) return false;
+  return M < kWholeSumRows ? split_gemm_plan(M, 2 * F, K, sms, 1, 1, 1, plan) : dense_gemm_is_split(M, 2 * F, K, sms, plan);
+}
+KB2_API int32_t kb2_linear_glu_bf16_takes(int32_t M, int32_t F, int32_t K, int32_t device) {
+  SplitPlan plan;
+  return glu_plan(M, F, K, device, &plan);
+}
+KB2_API int kb2_linear_glu_bf16(const void* x_dev, const void* w_dev, void* out_dev, int32_t M, int32_t F, int32_t K, int32_t kind, float limit,
+                                float alpha, int32_t device, void* stream) {
+  if (!x_dev || !w_dev || !out_dev) return failf(KB2_ERR_VALUE, "null argument");
+  SplitPlan plan;
+  if (kind < 0 || kind > 2 || !glu_plan(M, F, K, device, &plan))
+    return failf(KB2_ERR_VALUE, "gated unit: sizes that kb2_linear_glu_bf16_takes, kind 0..2 (M=%d F=%d K=%d kind=%d)", M, F, K, kind);
+  CUDA_TRY(cudaSetDevice(device));
+  SplitGemm g;
+  g.x = x_dev; g.w = w_dev; g.out = out_dev;
+  g.M = M; g.N = 2 * F; g.K = K; g.ldo = F;
+  g.glu = true; g.glu_kind = kind; g.glu_limit = limit; g.glu_alpha = alpha;
+  CUDA_TRY(launch_split_gemm(g, plan, (cudaStream_t)stream));
+  return KB2_OK;
+}
+
 KB2_API int kb2_linear_bf16_grouped(const void* x_dev, const void* w_dev, void* out_dev, int32_t M, int32_t N, int32_t K, int32_t out_f32,
                                     const int32_t* tile_group_dev, const int32_t* num_row_tiles_dev, int32_t groups, int32_t device,
                                     void* stream) {
@@ -185,6 +210,21 @@ KB2_API int kb2_linear_bf16_binned(const void* x_dev, const void* w_dev, void* o
   g.x = x_dev; g.w = w_dev; g.out = out_dev;
   g.M = M; g.N = N; g.K = K; g.ldo = N; g.out_f32 = out_f32 != 0;
   g.groups = groups; g.tile_group = tile_group_dev; g.n_tiles_dev = num_row_tiles_dev;
+  CUDA_TRY(launch_split_gemm(g, split_gemm_binned_plan(K, tile_rows), (cudaStream_t)stream));
+  return KB2_OK;
+}
+KB2_API int kb2_linear_glu_bf16_binned(const void* x_dev, const void* w_dev, void* out_dev, int32_t M, int32_t F, int32_t K, int32_t kind, float limit,
+                                       float alpha, int32_t tile_rows, const int32_t* tile_group_dev, const int32_t* num_row_tiles_dev, int32_t groups,
+                                       int32_t device, void* stream) {
+  if (!x_dev || !w_dev || !out_dev || !tile_group_dev || !num_row_tiles_dev) return failf(KB2_ERR_VALUE, "null argument");
+  if (M <= 0 || F <= 0 || K <= 0 || K % 64 || F % 16 || groups <= 0 || tile_rows < 16 || tile_rows > 128 || tile_rows % 16 || M % tile_rows || kind < 0 || kind > 2)
+    return failf(KB2_ERR_VALUE, "binned gated unit: need M>0, K %% 64 == 0, F %% 16 == 0, groups > 0, kind 0..2, tiles of 16..128 rows that divide M (M=%d F=%d K=%d)", M, F, K);
+  CUDA_TRY(cudaSetDevice(device));
+  SplitGemm g;
+  g.x = x_dev; g.w = w_dev; g.out = out_dev;
+  g.M = M; g.N = 2 * F; g.K = K; g.ldo = F;
+  g.groups = groups; g.tile_group = tile_group_dev; g.n_tiles_dev = num_row_tiles_dev;
+  g.glu = true; g.glu_kind = kind; g.glu_limit = limit; g.glu_alpha = alpha;
   CUDA_TRY(launch_split_gemm(g, split_gemm_binned_plan(K, tile_rows), (cudaStream_t)stream));
   return KB2_OK;
 }

@@ -359,6 +359,12 @@ static int dense_pair_plan(int M, int N, int K, int num_sms, float* us) {
   return best;
 }
 
+bool dense_gemm_is_split(int M, int N, int K, int num_sms, SplitPlan* out) {
+  float us;
+  dense_pair_plan(M, N, K, num_sms, &us);
+  return split_gemm_plan_whole(M, N, K, num_sms, us, out);
+}
+
 template <int MODE>
 static cudaError_t launch_dense_pair(const CUtensorMap& tx, const CUtensorMap& tw, int nt, void* out, const float* bias, int M, int N, int K, long long ldo,
                                      const CombineScatter& sc, int num_sms, cudaStream_t s) {

@@ -10,6 +10,7 @@
 
 #include "../../include/krasis_b200_seq.h"
 #include "pdl.cuh"
+#include "seq_act.cuh"
 
 namespace kb2seq {
 
@@ -68,10 +69,9 @@ __device__ __forceinline__ uint4 ld_stream16(const void* p) {
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
-__device__ __forceinline__ float gelu_tanh(float z) {
-  return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
-}
-__device__ __forceinline__ float silu(float z) { return z / (1.f + expf(-z)); }
+using kb2act::gelu_tanh;
+using kb2act::glu_value;
+using kb2act::silu;
 // Per-token decay exp(-exp(A_log) * softplus(a + dt_bias)).  A recurrent state multiplies by it at every token, so a rounding bias of
 // the fp32 exp / log1p chain (a fraction of an ulp, but of one sign) would grow linearly with the distance to a far token; evaluated in
 // fp64 and rounded once, the fp32 decay carries only its own unbiased half ulp.

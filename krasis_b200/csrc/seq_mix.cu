@@ -496,14 +496,6 @@ __global__ void __launch_bounds__(256) pool_merge_kernel(float* __restrict__ a, 
 // weight of row r is row_w[row_map[r]], 0 for a negative entry), then plus bias [2 F].  kind 0: gelu_tanh(g) u; 1: silu(g) u; 2: g' sigmoid(alpha g') (u' + 1) with g' = min(g, limit),
 // u' = clamp(u, -limit, limit); 3: relu(g)^2 of in [rows, F] alone (no up half).  With n_tiles given only the first
 // n_tiles[0] * tile_rows rows are computed.
-__device__ __forceinline__ float glu_value(float g, float u, int kind, float limit, float alpha) {
-  if (kind == 3) return g > 0.f ? g * g : 0.f;
-  if (kind == 0) return gelu_tanh(g) * u;
-  if (kind == 1) return silu(g) * u;
-  g = fminf(g, limit);
-  u = fminf(fmaxf(u, -limit), limit);
-  return g / (1.f + expf(-alpha * g)) * (u + 1.f);
-}
 __device__ __forceinline__ float glu_row_weight(const float* __restrict__ row_w, const int* __restrict__ row_map, long long r) {
   if (row_w == nullptr) return 1.f;
   const long long i = row_map != nullptr ? row_map[r] : r;

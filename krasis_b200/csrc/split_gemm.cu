@@ -13,6 +13,9 @@
 // Grouped form: row tile i of X multiplies matrix tile_group[i] (routed experts on binned rows); only the first n_tiles_dev[0] row tiles
 // exist, the CTAs of the others return at once.  Batched form: group g has M rows and a matrix of its own (per-head products).
 //
+// Gated units: W is [gate ; up], and a tile's 128 weight rows are 64 of each, so a CTA has both numbers of an output and writes the unit itself: the
+// pass over a product of 2 F columns and its launch go away (F 8192, K 2048: 9 rows 16.2 -> 14.4 us, 77 rows 17.7 -> 15.7, 255 rows 28.1 -> 26.2).
+//
 // fp32 operands: x = x1 + x2 + x3 with bf16 parts of 8 bits each, exactly (Henry, Tang and Heinecke, "Leveraging the bfloat16 Artificial
 // Intelligence Datatype For Higher-Precision Computations", ARITH 2019).  The parts of a tile's rows lie side by side on the N side, so one
 // weight tile serves all of them: w x1 goes to the main accumulators, w x2 and w x3 to two small ones.  With fp32 weights in three parts
@@ -23,15 +26,19 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "moe_common.cuh"
 #include "prof.cuh"
 #include "ptx.cuh"
+#include "seq_act.cuh"
 #include "split_gemm.cuh"
 
 namespace kb2 {
 
-constexpr int kSThreads = 128;
+// one warp issues copies, one products; all read the accumulators back and write the rows (with four of them 255 rows, N 16384, K 2048 took 24.7 us
+// instead of 23.4, and gated units 34.2 instead of 26.2)
+constexpr int kSWarps = 8, kSThreads = 32 * kSWarps;
 constexpr int kSRows = 128;                        // weight rows per tile
 constexpr int kSWBytes = kSRows * kBlockK * 2;     // 16 KB of weights per stage
 constexpr int kSMaxStages = 12;
@@ -48,6 +55,8 @@ struct SplitArgs {
   const float* x_raw;
   long long x_ld, x_group;
   const void* w_raw;
+  int glu_kind;
+  float glu_limit, glu_alpha;
 };
 
 __device__ __forceinline__ float4 ld_dsmem_f4(uint32_t local_addr, uint32_t rank) {
@@ -67,7 +76,7 @@ __device__ __noinline__ float product_again(const float* x, const void* w, long 
 }
 
 // KS CTAs of a cluster share one output tile along K.
-template <bool kOutF32, int KS>
+template <bool kOutF32, int KS, bool kGlu>
 __global__ void __launch_bounds__(kSThreads)
     split_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const SplitArgs p) {
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -78,7 +87,8 @@ __global__ void __launch_bounds__(kSThreads)
   uint64_t* done = empty + kSMaxStages;
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(done + 1);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int n0 = blockIdx.y * kSRows;
+  constexpr int kTileCols = kGlu ? kSRows / 2 : kSRows;      // output columns of a tile
+  const int n0 = blockIdx.y * kTileCols;
   const int m0 = (p.tiles_per_group > 0 ? row_tile % p.tiles_per_group : row_tile) * p.mt;     // row of the output (of its group)
   const int kb0 = (int)((long long)p.n_kblocks * rank / KS), kb1 = (int)((long long)p.n_kblocks * (rank + 1) / KS);
 
@@ -133,7 +143,12 @@ __global__ void __launch_bounds__(kSThreads)
       if (elect_one()) {
         const int w_parts = low >> span & 1 ? 3 : 1;
         mbar_arrive_expect_tx(&full[stage], w_parts * kSWBytes + nt * 128);
-        for (int q = 0; q < w_parts; ++q) tma_load_2d(a + q * kSWBytes, &tmap_w, kb * kBlockK, w0 + (int)(q * p.w_part_rows), &full[stage]);
+        if constexpr (kGlu) {
+          tma_load_2d(a, &tmap_w, kb * kBlockK, w0, &full[stage]);
+          tma_load_2d(a + kSWBytes / 2, &tmap_w, kb * kBlockK, w0 + p.N / 2, &full[stage]);
+        } else {
+          for (int q = 0; q < w_parts; ++q) tma_load_2d(a + q * kSWBytes, &tmap_w, kb * kBlockK, w0 + (int)(q * p.w_part_rows), &full[stage]);
+        }
         tma_load_2d(a + w_bytes, &tmap_x, kb * kBlockK, row_tile * nt, &full[stage]);
       }
       __syncwarp();
@@ -180,9 +195,10 @@ __global__ void __launch_bounds__(kSThreads)
   mbar_wait(done, 0);                              // every load has been consumed: the ring's memory is free
   tc_fence_after_sync();
   float* part = reinterpret_cast<float*>(smem);    // [mt][128]
-  const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16);
+  const int lanes = warp % 4 * 32;                 // of the tensor memory that this warp can read
+  const uint32_t taddr = tmem_base + ((uint32_t)lanes << 16);
   const int n_sets = (kb1 - kb0 + p.chunk - 1) / p.chunk + (p.xparts > 1 ? 2 : 0);      // the small ones come first
-  for (int c0 = 0; c0 < p.mt; c0 += 16) {
+  for (int c0 = warp / 4 * 16; c0 < p.mt; c0 += kSWarps * 4) {
     float v[16];
     uint32_t r[16];
     tmem_ld16(taddr + c0, r);
@@ -196,46 +212,65 @@ __global__ void __launch_bounds__(kSThreads)
       for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(r[j]);
     }
 #pragma unroll
-    for (int j = 0; j < 16; ++j) part[(c0 + j) * kSRows + warp * 32 + lane] = v[j];
+    for (int j = 0; j < 16; ++j) part[(c0 + j) * kSRows + lanes + lane] = v[j];
   }
   tc_fence_before_sync();
   if constexpr (KS > 1) cluster_sync_all(); else __syncthreads();
-  // the cluster's CTAs take the tile's rows in turn; a warp writes one row of 128 columns, four per lane
-  const int n = n0 + lane * 4;
-  if (n < p.N) {                                   // N % 16 == 0 is required by the launcher
-    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p.bias != nullptr) b = make_float4(p.bias[n], p.bias[n + 1], p.bias[n + 2], p.bias[n + 3]);
-    const int rows = min(p.mt, p.M - m0);
-    const long long out0 = group * p.out_group + (long long)m0 * p.ldo + n;
+  auto whole = [&](int c, int col) {               // four columns of a row, summed over the cluster's images
+    float4 v[KS];
+#pragma unroll
+    for (int i = 0; i < KS; ++i) {
+      if constexpr (KS > 1) v[i] = ld_dsmem_f4(smem_u32(part + c * kSRows + col), i);
+      else v[i] = *reinterpret_cast<const float4*>(part + c * kSRows + col);
+    }
+    float4 s = v[0];
+#pragma unroll
+    for (int i = 1; i < KS; ++i) { s.x += v[i].x; s.y += v[i].y; s.z += v[i].z; s.w += v[i].w; }
+    return s;
+  };
+  if constexpr (kGlu) {                            // half a warp per row of 64 columns
+    const int n = n0 + (lane & 15) * 4, rows = n < p.N / 2 ? min(p.mt, p.M - m0) : 0;
+    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + group * p.out_group + (long long)m0 * p.ldo + n;
+    auto write = [&](auto kind) {
+      auto unit = [&](float g, float u) { return kb2act::glu_value(bf16_round_rn(g), bf16_round_rn(u), decltype(kind)::value, p.glu_limit, p.glu_alpha); };
 #pragma unroll 2
-    for (int c = rank + KS * warp; c < rows; c += KS * 4) {
-      const uint32_t at = smem_u32(part + c * kSRows + lane * 4);
-      float4 v[KS];
-#pragma unroll
-      for (int i = 0; i < KS; ++i) {
-        if constexpr (KS > 1) v[i] = ld_dsmem_f4(at, i);
-        else v[i] = *reinterpret_cast<const float4*>(part + c * kSRows + lane * 4);
+      for (int c = (rank + KS * warp) * 2 + (lane >> 4); c < rows; c += KS * kSWarps * 2) {
+        const float4 g = whole(c, (lane & 15) * 4), u = whole(c, 64 + (lane & 15) * 4);
+        *reinterpret_cast<uint2*>(out + c * p.ldo) = make_uint2(bf16x2_bits_rn(unit(g.y, u.y), unit(g.x, u.x)), bf16x2_bits_rn(unit(g.w, u.w), unit(g.z, u.z)));
       }
-      float4 s = v[0];
-#pragma unroll
-      for (int i = 1; i < KS; ++i) { s.x += v[i].x; s.y += v[i].y; s.z += v[i].z; s.w += v[i].w; }
-      if (p.x_raw != nullptr && (isnan(s.x) || isnan(s.y) || isnan(s.z) || isnan(s.w))) {
-        const float* xr = p.x_raw + group * p.x_group + (long long)(m0 + c) * p.x_ld;
-        const int K = p.n_kblocks * kBlockK;
-        const long long wr = ((long long)group * p.N + n) * K;
-        s.x = product_again(xr, p.w_raw, wr, p.wparts > 1, K);
-        s.y = product_again(xr, p.w_raw, wr + K, p.wparts > 1, K);
-        s.z = product_again(xr, p.w_raw, wr + 2 * K, p.wparts > 1, K);
-        s.w = product_again(xr, p.w_raw, wr + 3 * K, p.wparts > 1, K);
-      }
-      s.x += b.x; s.y += b.y; s.z += b.z; s.w += b.w;
-      if constexpr (kOutF32) {
-        *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + out0 + c * p.ldo) = s;
-      } else {
-        uint2 o;
-        o.x = bf16x2_bits_rn(s.y, s.x);
-        o.y = bf16x2_bits_rn(s.w, s.z);
-        *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + out0 + c * p.ldo) = o;
+    };
+    if (p.glu_kind == 0) write(std::integral_constant<int, 0>{});
+    else if (p.glu_kind == 1) write(std::integral_constant<int, 1>{});
+    else write(std::integral_constant<int, 2>{});
+  } else {
+    // the cluster's CTAs take the tile's rows in turn; a warp writes one row of 128 columns, four per lane
+    const int n = n0 + lane * 4;
+    if (n < p.N) {                                   // N % 16 == 0 is required by the launcher
+      float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (p.bias != nullptr) b = make_float4(p.bias[n], p.bias[n + 1], p.bias[n + 2], p.bias[n + 3]);
+      const int rows = min(p.mt, p.M - m0);
+      const long long out0 = group * p.out_group + (long long)m0 * p.ldo + n;
+#pragma unroll 2
+      for (int c = rank + KS * warp; c < rows; c += KS * kSWarps) {
+        float4 s = whole(c, lane * 4);
+        if (p.x_raw != nullptr && (isnan(s.x) || isnan(s.y) || isnan(s.z) || isnan(s.w))) {
+          const float* xr = p.x_raw + group * p.x_group + (long long)(m0 + c) * p.x_ld;
+          const int K = p.n_kblocks * kBlockK;
+          const long long wr = ((long long)group * p.N + n) * K;
+          s.x = product_again(xr, p.w_raw, wr, p.wparts > 1, K);
+          s.y = product_again(xr, p.w_raw, wr + K, p.wparts > 1, K);
+          s.z = product_again(xr, p.w_raw, wr + 2 * K, p.wparts > 1, K);
+          s.w = product_again(xr, p.w_raw, wr + 3 * K, p.wparts > 1, K);
+        }
+        s.x += b.x; s.y += b.y; s.z += b.z; s.w += b.w;
+        if constexpr (kOutF32) {
+          *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + out0 + c * p.ldo) = s;
+        } else {
+          uint2 o;
+          o.x = bf16x2_bits_rn(s.y, s.x);
+          o.y = bf16x2_bits_rn(s.w, s.z);
+          *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + out0 + c * p.ldo) = o;
+        }
       }
     }
   }
@@ -245,9 +280,9 @@ __global__ void __launch_bounds__(kSThreads)
 
 cudaError_t make_tmap_bf16_rows(void* out_tmap, const void* base, long long rows, long long cols, int box_rows);
 
-template <bool F32, int KS>
+template <bool F32, int KS, bool kGlu>
 static cudaError_t launch_one_split(const CUtensorMap& tx, const CUtensorMap& tw, const SplitArgs& p, dim3 grid, int smem, cudaStream_t s) {
-  auto kern = split_gemm_kernel<F32, KS>;
+  auto kern = split_gemm_kernel<F32, KS, kGlu>;
   static PerDeviceOnce once;
   if (const int dev = once.pending(); dev >= 0) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -363,7 +398,7 @@ cudaError_t launch_split_gemm(const SplitGemm& g, const SplitPlan& plan, cudaStr
   // three parts: whole tiles of zero-padded rows; else the caller's M rows (rows beyond them read as zeros)
   cudaError_t e = make_tmap_bf16_rows(&tx, g.x, g.xparts > 1 ? (long long)row_tiles * nt : (long long)g.M, g.K, nt);
   if (e != cudaSuccess) return e;
-  e = make_tmap_bf16_rows(&tw, g.w, (long long)g.wparts * g.groups * g.N, g.K, kSRows);
+  e = make_tmap_bf16_rows(&tw, g.w, (long long)g.wparts * g.groups * g.N, g.K, g.glu ? kSRows / 2 : kSRows);
   if (e != cudaSuccess) return e;
   SplitArgs p{};
   p.out = g.out;
@@ -391,6 +426,10 @@ cudaError_t launch_split_gemm(const SplitGemm& g, const SplitPlan& plan, cudaStr
   p.x_group = g.x_group;
   p.w_raw = g.w_raw;
   p.w_low = g.w_low;
+  p.glu_kind = g.glu_kind;
+  p.glu_limit = g.glu_limit;
+  p.glu_alpha = g.glu_alpha;
+  if (g.glu && (g.out_f32 || g.xparts != 1 || g.bias != nullptr || g.N % 32)) return cudaErrorInvalidValue;
   p.low_span = split_low_span(g.K);
   p.low_spans = ceil_div(nkb, p.low_span);
   if (g.wparts > 1 && g.w_low == nullptr) return cudaErrorInvalidValue;
@@ -400,9 +439,10 @@ cudaError_t launch_split_gemm(const SplitGemm& g, const SplitPlan& plan, cudaStr
   // leaves fewer than 544 columns, and columns come in multiples of 32
   const int smem = std::max(ring + 2 * kSMaxStages * 8 + 16, p.tmem_cols * 430 - 1024);
   if (plan.stages < 1 || plan.stages > kSMaxStages || ring < plan.mt * kSRows * 4 || smem > 227 * 1024) return cudaErrorInvalidValue;
-  const dim3 grid(row_tiles * plan.ks, (g.N + kSRows - 1) / kSRows);
-#define KB2_SPLIT(KSV)                                                                  \
-  (g.out_f32 ? launch_one_split<true, KSV>(tx, tw, p, grid, smem, s) : launch_one_split<false, KSV>(tx, tw, p, grid, smem, s))
+  const dim3 grid(row_tiles * plan.ks, ceil_div(g.glu ? g.N / 2 : g.N, g.glu ? kSRows / 2 : kSRows));
+#define KB2_SPLIT(KSV)                                                                                                                                \
+  (g.glu ? launch_one_split<false, KSV, true>(tx, tw, p, grid, smem, s) : g.out_f32 ? launch_one_split<true, KSV, false>(tx, tw, p, grid, smem, s) \
+                                                                                   : launch_one_split<false, KSV, false>(tx, tw, p, grid, smem, s))
   switch (plan.ks) {
     case 1: return KB2_SPLIT(1);
     case 2: return KB2_SPLIT(2);

@@ -41,6 +41,11 @@ struct SplitGemm {
   const float* x_raw = nullptr;
   long long x_ld = 0, x_group = 0;
   const void* w_raw = nullptr;              // fp32 when wparts is 3, else bf16; rows of K
+  // W is [gate ; up] of N / 2 rows each and the output [M][N / 2] their gated unit (glu_value, seq_act.cuh) in bf16; both are rounded to bf16 first, as
+  // a product and an activation pass would
+  bool glu = false;
+  int glu_kind = 0;
+  float glu_limit = 0.f, glu_alpha = 0.f;
   const uint8_t* w_low = nullptr;           // wparts 3: what launch_split_weights says about the low parts
 };
 
@@ -49,6 +54,8 @@ inline int split_low_span(int K) { return K / 64 > 128 ? (K / 64 + 31) / 32 : 4;
 
 // One accumulator over all of K, K block by K block: the sums of dense_gemm.cu, bit for bit.  false: not estimated to take less than `us`.
 bool split_gemm_plan_whole(int M, int N, int K, int num_sms, float us, SplitPlan* out);
+// Whether launch_dense_gemm runs a product on these tiles, and how.
+bool dense_gemm_is_split(int M, int N, int K, int num_sms, SplitPlan* out);
 // Sums in chunks, in an order that depends on N, K, the parts and the groups, not on M.  false: sizes not taken.
 bool split_gemm_plan(int M, int N, int K, int num_sms, int xparts, int wparts, int groups, SplitPlan* out);
 // binned rows (one weight matrix per row tile): a CTA per tile and 128 columns, K uncut

@@ -96,6 +96,22 @@ def lin(a: torch.Tensor, w: torch.Tensor, out_dtype=torch.float32, min_n: int = 
     return ops.gemm(a, w, out_dtype)
 
 
+def lin_glu(a: torch.Tensor, w: torch.Tensor, kind: int, limit: float, alpha: float):
+    """The gated unit of a [M, K] @ w [2 F, K]^T = [gate | up] in bfloat16 by the product itself (the bits of lin and ops.glu), or None where
+    the product runs on other kernels."""
+    M, K = a.shape
+    F = w.shape[0] // 2
+    if (kind == ops.ACT_RELU2 or M <= GEMV_ROWS or a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or K % 64 or F % 16 or 2 * F < 256
+            or w.shape[1] != K or not a.is_contiguous() or not w.is_contiguous() or a.data_ptr() % 16 or w.data_ptr() % 16):
+        return None
+    core, dev = _core_lib(), a.get_device()
+    if not core or not core.kb2_linear_glu_bf16_takes(M, F, K, dev):
+        return None
+    out = torch.empty((M, F), dtype=torch.bfloat16, device=a.device)
+    _core_check(core.kb2_linear_glu_bf16(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, F, K, kind, limit, alpha, dev, stream_on(dev)))
+    return out
+
+
 def _lin_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
     """out[:, g] = a[:, g] @ w[g]^T for fp32 a [M, G, K] and fp32 or bfloat16 w [G, N, K] on the tensor cores, the operands as exact bf16
     parts: the accuracy of fp32 sums (kb2_linear_f32).  False: sizes, strides or alignment it does not take (K below 128 too, where the
@@ -660,6 +676,9 @@ class GatedMLP:
         self.out_bias = f(weights["down_b"]) if "down_b" in weights else None
 
     def forward(self, h: torch.Tensor) -> torch.Tensor:
+        a = lin_glu(h, self.w_gu, self.kind, self.limit, self.alpha) if self.bias is None else None
+        if a is not None:
+            return lin(a, self.w_down, torch.float32)
         gu = lin(h, self.w_gu, self.dtype)
         if self.kind == ops.GLU_GELU_TANH and self.bias is None:
             a = ops.act_mul(gu, self.dtype)
@@ -1022,6 +1041,11 @@ class RoutedExperts:
             else:
                 capi.check(core.kb2_linear_bf16_binned(x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, w.shape[1], w.shape[2], f32, tile, *table))
             return out
+        if tile < 128 and in_w is None and self.gated:          # the unit by the product itself
+            act = torch.empty((rows, F), dtype=torch.bfloat16, device=dev)
+            capi.check(core.kb2_linear_glu_bf16_binned(xs.data_ptr(), self.w_gu.data_ptr(), act.data_ptr(), rows, F, W, self.act_kind, self.limit, self.alpha,
+                                                       tile, t["tile_expert"].data_ptr(), t["n_tiles"].data_ptr(), E, di, s))
+            return product(act, self.w_down, torch.empty((rows, W), dtype=torch.float32, device=dev), 1), t["pos"]
         gu = product(xs, self.w_gu, torch.empty((rows, self.w_gu.shape[1]), dtype=torch.bfloat16, device=dev), 0)
         act = ops.glu(gu, torch.bfloat16, self.act_kind, self.limit, self.alpha, n_tiles=t["n_tiles"], tile_rows=tile, row_w=in_w,
                       row_map=t["slot_row"])
