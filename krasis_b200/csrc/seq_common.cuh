@@ -69,6 +69,13 @@ __device__ __forceinline__ uint4 ld_stream16(const void* p) {
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
+// 16 bytes from global to shared memory, zeros with in false; stream: past L1, for what is read once
+__device__ __forceinline__ void cp_async16(uint32_t to, const void* from, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async16_stream(uint32_t to, const void* from, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from), "r"(in ? 16 : 0) : "memory");
+}
 using kb2act::gelu_tanh;
 using kb2act::glu_value;
 using kb2act::silu;

@@ -157,7 +157,6 @@ __global__ void __launch_bounds__(256) gemv_nt_vec_kernel(const TA* __restrict__
   const int lane = threadIdx.x & 31;
   const int group = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) / KS, kpart = (threadIdx.x >> 5) % KS;
   const int n0 = group * CPW;
-  if (KS == 1 && n0 >= N) return;            // with K split over warps every warp stays for the block barrier
   float acc[MR][CPW];
 #pragma unroll
   for (int m = 0; m < MR; ++m)
@@ -190,32 +189,22 @@ __global__ void __launch_bounds__(256) gemv_nt_vec_kernel(const TA* __restrict__
 #pragma unroll
     for (int c = 0; c < CPW; ++c) wv[c] = wn[c];
   }
-  if constexpr (KS > 1) {
-    __shared__ float red[8][MR * CPW];
-    const int warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int m = 0; m < MR; ++m)
-#pragma unroll
-      for (int c = 0; c < CPW; ++c) {
-        const float v = warp_sum(acc[m][c]);
-        if (lane == 0) red[warp][m * CPW + c] = v;
-      }
-    __syncthreads();
-    if (kpart == 0 && lane < MR * CPW) {
-      const int m = lane / CPW, c = lane % CPW;
-      float v = 0.f;
-      for (int p = 0; p < KS; ++p) v += red[warp + p][lane];
-      if (m < M && n0 + c < N) stf(C, (long long)m * ldc + n0 + c, v);
-    }
-    return;
-  }
+  __shared__ float red[8][MR * CPW];
+  const int warp = threadIdx.x >> 5;
 #pragma unroll
   for (int m = 0; m < MR; ++m)
 #pragma unroll
     for (int c = 0; c < CPW; ++c) {
       const float v = warp_sum(acc[m][c]);
-      if (lane == 0 && m < M && n0 + c < N) stf(C, (long long)m * ldc + n0 + c, v);
+      if (lane == 0) red[warp][m * CPW + c] = v;
     }
+  __syncthreads();
+  if (kpart == 0 && lane < MR * CPW) {
+    const int m = lane / CPW, c = lane % CPW;
+    float v = 0.f;
+    for (int p = 0; p < KS; ++p) v += red[warp + p][lane];
+    if (m < M && n0 + c < N) stf(C, (long long)m * ldc + n0 + c, v);
+  }
 }
 
 template <typename TA, typename TC>
@@ -223,34 +212,26 @@ static bool launch_gemv_vec(const void* A, long long lda, const void* B, long lo
                             int batch, long long sA, long long sB, long long sC, cudaStream_t s) {
   const bool a16 = sizeof(TA) == 2;
   if (K % 8 || ldb % 8 || sB % 8 || ((uintptr_t)B & 15) || ((uintptr_t)A & 15) || lda % (a16 ? 8 : 4) || sA % (a16 ? 8 : 4)) return false;
-  // columns per warp: 4 where that still leaves two blocks per SM; few columns: one per warp group, K split over 4 warps.
-  // Up to 4 rows run the 4-row instantiation (half the accumulators: more blocks per SM, more weight bytes in flight).
-  const long long warps = (long long)N * batch;
-#define KB2_GEMV(MRV, CPWV, KSV, GX)                                                                                        \
-  kb2::launch_pdl(gemv_nt_vec_kernel<TA, TC, MRV, CPWV, KSV>, dim3(GX, 1, batch), 256, 0, s, (const TA*)A, lda, (const bf16*)B, ldb, (TC*)C, ldc, M, N, K, \
-                                                                                sA, sB, sC)
-  if (warps >= 4 * 8 * 296) {
-    if (M <= 4) KB2_GEMV(4, 4, 1, (N + 31) / 32); else KB2_GEMV(8, 4, 1, (N + 31) / 32);
-  } else if (warps >= 2 * 8 * 296) {
-    if (M <= 4) KB2_GEMV(4, 2, 1, (N + 15) / 16); else KB2_GEMV(8, 2, 1, (N + 15) / 16);
-  } else if (K >= 2048) {
-    if (M <= 4) KB2_GEMV(4, 1, 4, (N + 1) / 2); else KB2_GEMV(8, 1, 4, (N + 1) / 2);
-  } else {
-    if (M <= 4) KB2_GEMV(4, 1, 1, (N + 7) / 8); else KB2_GEMV(8, 1, 1, (N + 7) / 8);
-  }
+  // one column a group of four warps: this form is left for few columns
+#define KB2_GEMV(MRV)                                                                                                                        \
+  kb2::launch_pdl(gemv_nt_vec_kernel<TA, TC, MRV, 1, 4>, dim3((N + 1) / 2, 1, batch), 256, 0, s, (const TA*)A, lda, (const bf16*)B, ldb, (TC*)C, ldc, M, \
+                  N, K, sA, sB, sC)
+  if (M <= 4) KB2_GEMV(4); else KB2_GEMV(8);
 #undef KB2_GEMV
   return true;
 }
 
-// ---- few bfloat16 rows against bfloat16 weights, on the warp-level tensor instructions
+// ---- few rows against bfloat16 weights, on the warp-level tensor instructions
 // Bound: the weights' way from HBM; the arithmetic has to stay out of the way (fp32 FMAs on unpacked values took 200 instructions per KB of
 // weights at 4 rows).  A warp owns 16 weight rows (the 16-row side of mma.m16n8k16) and up to 8 rows of A (its 8-column side).  A product
 // does not care about the order along K, so a lane takes 16 neighbouring bytes of its weight row and the same 16 of its row of A, and word
-// pairs of the two go into two instructions as they are: no shuffles, no shared memory, 64-byte runs per quad and load.  KS warps of a block
-// share the rows and take pieces of 128 numbers in turn; the loads of the next piece are in flight under the current one.  Each instruction
+// pairs of the two go into two instructions as they are: no shuffles, 64-byte runs per quad and load.  The copies of the steps ahead are on their way
+// into a ring of the warp in shared memory, from which every lane reads what it copied itself, so that bytes in flight cost no registers (with the next
+// piece in registers: fp32 rows, N 32768, K 2048 42 us instead of 28.5, eight warps on an SM; bf16 rows, N 2048, K 2048 4.0 instead of 3.4).  KS warps of
+// a block share the rows and take pieces of 128 numbers in turn.  Each instruction
 // pair starts from zero, its 32 products join a compensated running sum, and the warps' sums meet pairwise: the error is that of the FMA form
 // (8e-8) or less.  From HBM at 4 rows, us before (gemv_nt_vec) and now: N 16384, K 2048 32.3 -> 13.7 (floor 10.3);
-// N 2048, K 8192 19.8 -> 9.2 (5.1); N 32768, K 2048 44.4 -> 25.3 (20.5); N 2048, K 2048 7.3 -> 3.8.
+// N 2048, K 8192 19.8 -> 8.2 (5.1); N 32768, K 2048 44.4 -> 24.7 (20.5); N 2048, K 2048 7.3 -> 3.4.
 __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -264,75 +245,124 @@ __device__ __forceinline__ void mma16816_new(float (&d)[4], uint32_t a0, uint32_
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
-template <typename TC, int KS>
-__global__ void __launch_bounds__(KS > 8 ? 512 : 256) gemv_mma_kernel(const bf16* __restrict__ A, long long lda, const bf16* __restrict__ B, long long ldb,
+// fp32 rows are three bf16 parts, exactly (the leading 8 bits, of what is left the next 8, the rest): the products with the first part go into one
+// accumulator, those with the others into a second, and both join the running sum.  The parts are made by every warp for itself; so that they serve
+// more weights, its pieces are 32 rows of 64 numbers.  fp32 rows, us before (gemv_nt_vec) at 1 / 2 / 4 / 8 rows and now at any: N 32768, K 2048 27.6 /
+// 30.4 / 40.6 / 79.9, 28.5; N 16384, K 2048 17.4 / 20.2 / 29.9 / 48.7, 17.5; N 2048, K 2048 5.1 / 6.0 / 8.4 / 12.7, 4.4; N 512, K 1024 2.6 / 3.4 / 5.1 /
+// 9.3, 2.5; error 1.6e-7 before, 6e-8 to 8e-8 now.  A sum that is not finite is made again in plain fp32 (the parts of an infinity are not numbers).
+template <bool kFp32, int kTiles> struct GemvPiece {
+  static constexpr int kRows = 16 * kTiles;                                    // weight rows of a warp
+  static constexpr int kSteps = kFp32 ? 2 : 4, kLen = 32 * kSteps;             // of K, 32 a step
+  static constexpr int kLoads = 2 * kTiles + (kFp32 ? 2 : 1);                  // 16-byte copies of a lane and step, the weights' first
+  static constexpr int kStages = kLoads > 4 ? 4 : kFp32 ? 6 : 8, kRing = kStages * kLoads * 512;  // bytes of a warp's ring
+};
+
+// {the bf16 that leads a, the one that leads b}; what is left of a and b
+__device__ __forceinline__ uint32_t lead_pair(float& a, float& b) {
+  const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
+  a -= __uint_as_float(ua & 0xffff0000u);
+  b -= __uint_as_float(ub & 0xffff0000u);
+  return __byte_perm(ua, ub, 0x7632);
+}
+
+__device__ __noinline__ float row_product(const float* a, const bf16* b, int K) {
+  float v = 0.f;
+  for (int k = 0; k < K; ++k) v = fmaf(a[k], __bfloat162float(b[k]), v);
+  return v;
+}
+
+template <typename TA, typename TC, int KS, int kTiles>
+__global__ void __launch_bounds__(KS > 8 ? 512 : 256) gemv_mma_kernel(const TA* __restrict__ A, long long lda, const bf16* __restrict__ B, long long ldb,
                                                                       TC* __restrict__ C, long long ldc, int M, int N, int K, long long sA, long long sB,
                                                                       long long sC) {
   kb2::pdl_enter(A, B, C);
-  constexpr int kStep = 128, kWarps = KS > 8 ? 16 : 8, kGroups = kWarps / KS;
-  __shared__ float red[kWarps][8][17];                   // [warp][row of A][weight row], odd pitch
+  constexpr bool kFp32 = sizeof(TA) == 4;
+  using P = GemvPiece<kFp32, kTiles>;
+  constexpr int kRows = P::kRows, kWarps = KS > 8 ? 16 : 8, kGroups = kWarps / KS, kW = 2 * kTiles;
+  extern __shared__ __align__(16) uint8_t gemv_ring[];
+  __shared__ float red[kWarps][8][kRows + 1];            // [warp][row of A][weight row], odd pitch
   A += (long long)blockIdx.z * sA;
   B += (long long)blockIdx.z * sB;
   C += (long long)blockIdx.z * sC;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quad = lane >> 2, t8 = (lane & 3) * 8;
-  const int n0 = (blockIdx.x * kGroups + warp / KS) * 16;
+  const int n0 = (blockIdx.x * kGroups + warp / KS) * kRows;
   // rows beyond the last one are read as the last one and not written
-  const bf16* w0 = B + (long long)min(n0 + quad, N - 1) * ldb + t8;
-  const bf16* w1 = B + (long long)min(n0 + quad + 8, N - 1) * ldb + t8;
-  const bf16* x = A + (long long)min(quad, M - 1) * lda + t8;
+  const bf16* w[kW];
+#pragma unroll
+  for (int i = 0; i < kW; ++i) w[i] = B + (long long)min(n0 + quad + 8 * i, N - 1) * ldb + t8;
+  const TA* x = A + (long long)min(quad, M - 1) * lda + t8;
   const bool row = quad < M;
-  uint4 cur[2][4], nxt[2][4];
-  auto fetch = [&](uint4 (&to)[2][4], int k) {
+  uint8_t* ring = gemv_ring + warp * P::kRing + lane * 16;     // a lane reads what it copied itself: no barrier
+  const int part = warp % KS, pieces = (K + P::kLen - 1) / P::kLen, steps = n0 < N ? (pieces - part + KS - 1) / KS * P::kSteps : 0;
+  auto fetch = [&](int i) {
+    if (i < steps) {
+      const int k = ((i / P::kSteps) * KS + part) * P::kLen + i % P::kSteps * 32;
+      const uint32_t to = kb2::smem_u32(ring + i % P::kStages * (P::kLoads * 512));
+      const bool in = k + t8 < K;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int kj = k + j * 32;
-      const bool in = kj + t8 < K;
-      to[0][j] = in ? ld_stream16(w0 + kj) : make_uint4(0, 0, 0, 0);
-      to[1][j] = in ? ld_stream16(w1 + kj) : make_uint4(0, 0, 0, 0);
+      for (int r = 0; r < kW; ++r) cp_async16_stream(to + r * 512, in ? w[r] + k : w[r], in);
+#pragma unroll
+      for (int h = 0; h < P::kLoads - kW; ++h) cp_async16(to + (kW + h) * 512, in ? x + k + 4 * h : x, in && row);
     }
+    kb2::cp_async_commit();
   };
-  float sum[4] = {0.f, 0.f, 0.f, 0.f}, lost[4] = {0.f, 0.f, 0.f, 0.f};
-  auto piece = [&](const uint4 (&w)[2][4], int k) {
-    uint4 xv[4];
+  float sum[kTiles][4] = {}, lost[kTiles][4] = {};
+  auto join = [&](int t, int i, float add) {             // compensated: what the addition rounds off goes into the next one
+    const float s = sum[t][i] + add;
+    // an infinity stays one: inf - inf must not reach the next addition (a sum of parts is made again in any case)
+    lost[t][i] = kFp32 || isfinite(s) ? (s - sum[t][i]) - add : 0.f;
+    sum[t][i] = s;
+  };
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      xv[j] = row && k + j * 32 + t8 < K ? *reinterpret_cast<const uint4*>(x + k + j * 32) : make_uint4(0, 0, 0, 0);
+  for (int i = 0; i < P::kStages - 1; ++i) fetch(i);
+#pragma unroll 1
+  for (int i = 0; i < steps; ++i) {
+    kb2::cp_async_wait<P::kStages - 2>();
+    const uint4* at = reinterpret_cast<const uint4*>(ring + i % P::kStages * (P::kLoads * 512));
+    uint4 v[P::kLoads];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint4 a = w[0][j], c = w[1][j];
-      float d[4] = {0.f, 0.f, 0.f, 0.f};
-      mma16816(d, a.x, c.x, a.y, c.y, xv[j].x, xv[j].y);
-      mma16816(d, a.z, c.z, a.w, c.w, xv[j].z, xv[j].w);
+    for (int r = 0; r < P::kLoads; ++r) v[r] = at[r * 32];
+    if constexpr (kFp32) {
+      const uint4 x0 = v[kW], x1 = v[kW + 1];
+      float f[8] = {__uint_as_float(x0.x), __uint_as_float(x0.y), __uint_as_float(x0.z), __uint_as_float(x0.w),
+                    __uint_as_float(x1.x), __uint_as_float(x1.y), __uint_as_float(x1.z), __uint_as_float(x1.w)};
+      uint32_t part[3][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {                // compensated: what the addition rounds off goes into the next one
-        const float add = d[i] - lost[i], t = sum[i] + add;
-        lost[i] = isfinite(t) ? (t - sum[i]) - add : 0.f;      // an infinity stays one: inf - inf must not reach the next addition
-        sum[i] = t;
+      for (int q = 0; q < 3; ++q)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) part[q][i] = lead_pair(f[2 * i], f[2 * i + 1]);
+#pragma unroll
+      for (int t = 0; t < kTiles; ++t) {
+        const uint4 a = v[2 * t], c = v[2 * t + 1];
+        float d[4], e[4];
+        mma16816_new(e, a.x, c.x, a.y, c.y, part[2][0], part[2][1]);
+        mma16816(e, a.z, c.z, a.w, c.w, part[2][2], part[2][3]);
+        mma16816(e, a.x, c.x, a.y, c.y, part[1][0], part[1][1]);
+        mma16816(e, a.z, c.z, a.w, c.w, part[1][2], part[1][3]);
+        mma16816_new(d, a.x, c.x, a.y, c.y, part[0][0], part[0][1]);
+        mma16816(d, a.z, c.z, a.w, c.w, part[0][2], part[0][3]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) join(t, i, d[i] + (e[i] - lost[t][i]));
       }
+    } else {
+      const uint4 a = v[0], c = v[1];
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
+      mma16816(d, a.x, c.x, a.y, c.y, v[2].x, v[2].y);
+      mma16816(d, a.z, c.z, a.w, c.w, v[2].z, v[2].w);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) join(0, i, d[i] - lost[0][i]);
     }
-  };
-  // two pieces per round, so that no copy between the buffers waits for the loads in flight
-  int k = (warp % KS) * kStep;
-  const int step = KS * kStep;
-  if (n0 < N) {
-    fetch(cur, k);
-    while (k < K) {
-      if (k + step < K) fetch(nxt, k + step);
-      piece(cur, k);
-      k += step;
-      if (k >= K) break;
-      if (k + step < K) fetch(cur, k + step);
-      piece(nxt, k);
-      k += step;
-    }
+    fetch(i + P::kStages - 1);
   }
-  // sum[0], [1]: weight row quad, rows 2 (lane & 3) and + 1 of A; [2], [3]: weight row quad + 8
+  // of a tile sum[0], [1]: weight row quad, rows 2 (lane & 3) and + 1 of A; [2], [3]: weight row quad + 8
   const int m = (lane & 3) * 2;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) red[warp][m + (i & 1)][quad + (i >> 1) * 8] = sum[i];
+  for (int t = 0; t < kTiles; ++t)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) red[warp][m + (i & 1)][16 * t + quad + (i >> 1) * 8] = sum[t][i];
   __syncthreads();
-  for (int i = threadIdx.x; i < kGroups * 128; i += kWarps * 32) {
-    const int g = i >> 7, mm = (i >> 4) & 7, r = i & 15, n = (blockIdx.x * kGroups + g) * 16 + r;
+  for (int i = threadIdx.x; i < kGroups * 8 * kRows; i += kWarps * 32) {
+    const int g = i / (8 * kRows), mm = i / kRows % 8, r = i % kRows, n = (blockIdx.x * kGroups + g) * kRows + r;
     if (mm >= M || n >= N) continue;
     float v[KS];
 #pragma unroll
@@ -341,27 +371,48 @@ __global__ void __launch_bounds__(KS > 8 ? 512 : 256) gemv_mma_kernel(const bf16
     for (int o = KS / 2; o > 0; o >>= 1)
 #pragma unroll
       for (int p = 0; p < o; ++p) v[p] += v[p + o];
+    if constexpr (kFp32) {
+      if (!isfinite(v[0])) v[0] = row_product(A + (long long)mm * lda, B + (long long)n * ldb, K);
+    }
     stf(C, (long long)mm * ldc + n, v[0]);
   }
 }
 
-template <typename TC>
-static bool launch_gemv_mma(const void* A, long long lda, const void* B, long long ldb, void* C, long long ldc, int M, int N, int K,
+template <typename TA, typename TC, int kTiles>
+static void launch_gemv_tiles(const void* A, long long lda, const void* B, long long ldb, void* C, long long ldc, int M, int N, int K,
                             int batch, long long sA, long long sB, long long sC, cudaStream_t s) {
-  if (K % 8 || ldb % 8 || sB % 8 || ((uintptr_t)B & 15) || ((uintptr_t)A & 15) || lda % 8 || sA % 8) return false;
-  // at any number of rows, so that a row's sums do not depend on the rows beside it; gemv_nt_vec, us at 1 / 2 / 4 / 8 rows and here at any: N 512, K 1024
-  // 2.7 / 3.5 / 5.3 / 9.7, 2.1; N 4096, K 224 2.3 / 2.7 / 3.4 / 5.2, 2.2; N 256, K 2048 2.2 / 2.6 / 3.5 / 5.6, 2.7; N 128, K 8184 3.9 / 5.6 / 9.2 / 17, 6.2
-  const int groups = (N + 15) / 16;
+  using Piece = GemvPiece<sizeof(TA) == 4, kTiles>;
+  const int groups = (N + Piece::kRows - 1) / Piece::kRows;
   int ks = 1;                                  // about 2048 warps, in one wave of two blocks per SM, as long as each has a piece of K
-  while (ks < 16 && (long long)groups * batch * 2 * ks <= 2368 && K > 128 * ks) ks *= 2;
+  while (ks < 16 && (long long)groups * batch * 2 * ks <= 2368 && K > Piece::kLen * ks) ks *= 2;
   const int per = (ks > 8 ? 16 : 8) / ks;
   const dim3 grid((groups + per - 1) / per, 1, batch);
-#define KB2_GEMV(KSV)                                                                                                                        \
-  case KSV:                                                                                                                                  \
-    kb2::launch_pdl(gemv_mma_kernel<TC, KSV>, grid, KSV > 8 ? 512 : 256, 0, s, (const bf16*)A, lda, (const bf16*)B, ldb, (TC*)C, ldc, M, N, K, sA, sB, sC); \
+  const size_t smem = (size_t)(ks > 8 ? 16 : 8) * Piece::kRing;
+#define KB2_GEMV(KSV)                                                                                                                            \
+  case KSV:                                                                                                                                      \
+    cudaFuncSetAttribute(gemv_mma_kernel<TA, TC, KSV, kTiles>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                                  \
+    kb2::launch_pdl(gemv_mma_kernel<TA, TC, KSV, kTiles>, grid, KSV > 8 ? 512 : 256, smem, s, (const TA*)A, lda, (const bf16*)B, ldb, (TC*)C, ldc, M, N, K, \
+                    sA, sB, sC);                                                                                                                 \
     break;
   switch (ks) { KB2_GEMV(1) KB2_GEMV(2) KB2_GEMV(4) KB2_GEMV(8) KB2_GEMV(16) }
 #undef KB2_GEMV
+}
+
+template <typename TA, typename TC>
+static bool launch_gemv_mma(const void* A, long long lda, const void* B, long long ldb, void* C, long long ldc, int M, int N, int K,
+                            int batch, long long sA, long long sB, long long sC, cudaStream_t s) {
+  constexpr int kA16 = 16 / sizeof(TA);
+  if (K % 8 || ldb % 8 || sB % 8 || ((uintptr_t)B & 15) || ((uintptr_t)A & 15) || lda % kA16 || sA % kA16) return false;
+  // at any number of rows, so that a row's sums do not depend on the rows beside it; bf16 rows, gemv_nt_vec, us at 1 / 2 / 4 / 8 rows and here at any:
+  // N 512, K 1024 2.7 / 3.5 / 5.3 / 9.7, 2.1; N 4096, K 224 2.3 / 2.7 / 3.4 / 5.2, 2.2; N 256, K 2048 2.2 / 2.6 / 3.5 / 5.6, 2.7; N 128, K 8184
+  // 3.9 / 5.6 / 9.2 / 17, 6.2
+  if constexpr (sizeof(TA) == 4) {             // 32 weight rows a warp where that still gives every SM a block (N 2048, K 8192: 15.9 us, with 16 rows 11.2)
+    if ((long long)((N + 31) / 32) * batch >= 148) {
+      launch_gemv_tiles<TA, TC, 2>(A, lda, B, ldb, C, ldc, M, N, K, batch, sA, sB, sC, s);
+      return true;
+    }
+  }
+  launch_gemv_tiles<TA, TC, 1>(A, lda, B, ldb, C, ldc, M, N, K, batch, sA, sB, sC, s);
   return true;
 }
 
@@ -370,10 +421,12 @@ static void launch_gemm(const void* A, long long lda, const void* B, long long l
                         int batch, long long sA, long long sB, long long sC, cudaStream_t s) {
   if (M <= 8) {
     if constexpr (sizeof(TB) == 2) {
-      if constexpr (sizeof(TA) == 2) {
-        if (launch_gemv_mma<TC>(A, lda, B, ldb, C, ldc, M, N, K, batch, sA, sB, sC, s)) return;
+      // fp32 rows, few columns and a long K: sixteen rows a block would leave the weights to a handful of SMs, and with one row the FMAs are few (us at
+      // 1 / 2 / 4 / 8 rows, N 256, K 2048 2.2 / 2.6 / 3.5 / 5.5 here, 3.5 at any on the tensor cores; N 128, K 8184 5.6 / 7.2 / 10.9 / 18.7, 10.4)
+      if constexpr (sizeof(TA) == 4) {
+        if ((long long)N * batch <= 256 && K >= 2048 && launch_gemv_vec<TA, TC>(A, lda, B, ldb, C, ldc, M, N, K, batch, sA, sB, sC, s)) return;
       }
-      if (launch_gemv_vec<TA, TC>(A, lda, B, ldb, C, ldc, M, N, K, batch, sA, sB, sC, s)) return;
+      if (launch_gemv_mma<TA, TC>(A, lda, B, ldb, C, ldc, M, N, K, batch, sA, sB, sC, s)) return;
     }
     dim3 grid((N + 7) / 8, 1, batch);
     kb2::launch_pdl(gemv_nt_kernel<TA, TB, TC, 8>, grid, 256, 0, s, (const TA*)A, lda, (const TB*)B, ldb, (TC*)C, ldc, M, N, K, sA, sB, sC);

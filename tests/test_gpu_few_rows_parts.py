@@ -1,0 +1,33 @@
+"""Few fp32 rows against bfloat16 weights as three bfloat16 parts: errors of fp32 sums, rows that do not notice one another, and what is not finite."""
+import pytest
+import torch
+
+from krasis_b200 import seqops as ops
+
+pytestmark = pytest.mark.gpu
+
+
+# columns around 16 and 32 rows of weights and around the counts that change the split along K; K that ends inside a step, a piece and a warp's turn
+@pytest.mark.parametrize("N,K", [(1, 8), (17, 40), (257, 2056), (1000, 64), (4720, 136), (4736, 2048), (9504, 328), (40000, 72)])
+@pytest.mark.parametrize("out", [torch.float32, torch.bfloat16])
+def test_few_fp32_rows(N, K, out):
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    w = torch.randn(N, K, device="cuda", generator=g).bfloat16()
+    x = torch.randn(8, K, device="cuda", generator=g) * torch.logspace(-12, 12, 8, device="cuda")[:, None]
+    got = ops.gemm(x, w, out)
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    # sums of 32 products that lose up to 2^-23 of their magnitude an instruction, joined in fp32: 2^-20 of the magnitudes is four times that
+    assert ((got.double() - want).abs() <= size * 2.0 ** -20 + (want.abs() * 2.0 ** -8 if out is torch.bfloat16 else 0)).all()
+    for m in (1, 2, 5):
+        assert torch.equal(ops.gemm(x[:m], w, out), got[:m])
+
+
+def test_not_finite():
+    g = torch.Generator(device="cuda").manual_seed(0)
+    w, x = torch.randn(4800, 512, device="cuda", generator=g).bfloat16(), torch.randn(4, 512, device="cuda", generator=g)
+    x[0, 3], x[1, 500] = float("inf"), float("nan")
+    w[7, 9] = float("-inf")
+    got, want = ops.gemm(x, w, torch.float32), x.double() @ w.double().T
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    inf = torch.isinf(want)
+    assert torch.equal(got[inf].sign(), want[inf].sign().float())
