@@ -220,6 +220,9 @@ KB2_API int64_t kb2_launch_count(const kb2_engine* e);
  * on; FP32 output of fewer rows is summed as kb2_linear_bf16_chunked does. */
 KB2_API int kb2_linear_bf16(const void* x_dev, const void* w_dev, const float* bias_dev, void* out_dev, int32_t M,
                             int32_t N, int32_t K, int32_t out_f32, int32_t device, void* stream);
+/* The form kb2_linear_bf16 runs a bf16 result in, for tests and tuning: the columns of a tile of a pair of CTAs, 0 where one CTA has a tile of
+ * 128 x 256, -1 for the tiles of few rows; smem_bytes (may be null): the shared memory of each CTA of a pair.  The sums are the same in each. */
+KB2_API int32_t kb2_linear_bf16_form(int32_t M, int32_t N, int32_t K, int32_t device, int32_t* smem_bytes);
 
 /* Grouped form of kb2_linear_bf16 for rows binned per group in tiles of 128 (routed experts): w [groups][N][K], row tile i of x
  * (rows 128 i .. 128 i + 127) is multiplied by w[tile_group_dev[i]], and only the first num_row_tiles_dev[0] row tiles are computed

@@ -116,6 +116,7 @@ SIGNATURES = {
                        [C.c_int32] * 4 + [C.c_void_p, C.c_size_t, C.c_int32, C.c_void_p]),
     "kb2_linear_bf16_chunked": (C.c_int, [C.c_void_p] * 4 + [C.c_int32] * 5 + [C.c_void_p]),
     "kb2_linear_bf16_binned": (C.c_int, [C.c_void_p] * 3 + [C.c_int32] * 5 + [C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_void_p]),
+    "kb2_linear_bf16_form": (C.c_int32, [C.c_int32] * 4 + [C.POINTER(C.c_int32)]),
     "kb2_linear_glu_bf16_takes": (C.c_int32, [C.c_int32] * 4),
     "kb2_linear_glu_bf16": (C.c_int, [C.c_void_p] * 3 + [C.c_int32] * 4 + [C.c_float, C.c_float, C.c_int32, C.c_void_p]),
     "kb2_linear_glu_bf16_binned": (C.c_int, [C.c_void_p] * 3 + [C.c_int32] * 4 + [C.c_float, C.c_float, C.c_int32, C.c_void_p, C.c_void_p, C.c_int32,

@@ -162,6 +162,13 @@ KB2_API int kb2_linear_bf16_chunked(const void* x_dev, const void* w_dev, const 
   return KB2_OK;
 }
 
+KB2_API int32_t kb2_linear_bf16_form(int32_t M, int32_t N, int32_t K, int32_t device, int32_t* smem_bytes) {
+  int smem = 0;
+  const int form = M <= 0 || N <= 0 || N % 16 || K <= 0 || K % 64 ? -1 : dense_gemm_form(M, N, K, device_sms(device), &smem);
+  if (smem_bytes) *smem_bytes = smem;
+  return form;
+}
+
 // the plan of the product that kb2_linear_glu_bf16 ends in a gated unit; false: the product runs on wide tiles
 static bool glu_plan(int32_t M, int32_t F, int32_t K, int32_t device, SplitPlan* plan) {
   const int sms = device_sms(device);

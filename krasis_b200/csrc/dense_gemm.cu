@@ -204,7 +204,8 @@ __global__ void __launch_bounds__(kDThreads, 1)
 // both.  A K block is still one instruction after the other into one accumulator: the same sums, bit for bit.
 // Columns per tile: what wastes least of the last round of 74 pairs (dense_pair_plan).  us with one CTA per tile and now: M 8192, N 12288, K 2048 316
 // / 271 (1.52 PFLOP/s, 0.91 of the measured burst rate); M 3333 134 / 120; M 3333, N 2048, K 4096 62.6 / 47.7; M 4096, N 12352, fp32 out 188 / 167.
-constexpr int kPStages = 6, kPStage = 32 * 1024, kPOffBar = kPStages * kPStage, kPSmem = kPOffBar + 256;
+constexpr int kPStages = 6, kPStage = 32 * 1024, kPOffBar = kPStages * kPStage, kPSmem = tmem_smem(512);
+static_assert(kPOffBar + 256 <= kPSmem && kPSmem <= 227 * 1024, "the ring and its barriers lie in what a CTA of a cluster takes for 512 columns");
 
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDThreads, 1)
@@ -363,6 +364,13 @@ bool dense_gemm_is_split(int M, int N, int K, int num_sms, SplitPlan* out) {
   float us;
   dense_pair_plan(M, N, K, num_sms, &us);
   return split_gemm_plan_whole(M, N, K, num_sms, us, out);
+}
+int dense_gemm_form(int M, int N, int K, int num_sms, int* smem) {
+  SplitPlan plan;
+  float us;
+  const int nt = dense_gemm_is_split(M, N, K, num_sms, &plan) ? -1 : dense_pair_plan(M, N, K, num_sms, &us);
+  *smem = nt > 0 ? kPSmem : 0;
+  return nt;
 }
 
 template <int MODE>

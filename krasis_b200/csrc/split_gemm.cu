@@ -434,10 +434,7 @@ cudaError_t launch_split_gemm(const SplitGemm& g, const SplitPlan& plan, cudaStr
   p.low_spans = ceil_div(nkb, p.low_span);
   if (g.wparts > 1 && g.w_low == nullptr) return cudaErrorInvalidValue;
   const int ring = plan.stages * (g.wparts * kSWBytes + nt * 128);
-  // a CTA that waits for tensor memory may have cluster peers that others wait for in turn, so co-resident CTAs must never ask for more
-  // than the 512 columns together: each takes at least 430 bytes of shared memory per column (1 KB of it is the system's); of 228 KB that
-  // leaves fewer than 544 columns, and columns come in multiples of 32
-  const int smem = std::max(ring + 2 * kSMaxStages * 8 + 16, p.tmem_cols * 430 - 1024);
+  const int smem = std::max(ring + 2 * kSMaxStages * 8 + 16, tmem_smem(p.tmem_cols));
   if (plan.stages < 1 || plan.stages > kSMaxStages || ring < plan.mt * kSRows * 4 || smem > 227 * 1024) return cudaErrorInvalidValue;
   const dim3 grid(row_tiles * plan.ks, ceil_div(g.glu ? g.N / 2 : g.N, g.glu ? kSRows / 2 : kSRows));
 #define KB2_SPLIT(KSV)                                                                                                                                \

@@ -14,6 +14,11 @@ constexpr int kSplitChunk = 8, kSplitChunkShort = 4;
 // Products of fewer rows sum in chunks where an fp32 result is asked for (kb2_linear_bf16).
 constexpr int kWholeSumRows = 256;
 
+// Shared memory that a CTA of a cluster takes at least when it allocates `cols` columns of tensor memory.  A CTA that waits for tensor memory may have
+// cluster peers that others wait for in turn, so CTAs of clusters (of any kernel, on any stream) that share an SM must never ask for more than its 512
+// columns together: at 430 bytes per column (1 KB of it is the system's) the 228 KB of an SM hold fewer than 544, and columns come in multiples of 32.
+constexpr int tmem_smem(int cols) { return cols * 430 - 1024; }
+
 struct SplitPlan {
   int mt = 0;       // rows of X per tile (a multiple of 16)
   int ks = 1;       // CTAs of a cluster that share a tile along K
@@ -56,6 +61,9 @@ inline int split_low_span(int K) { return K / 64 > 128 ? (K / 64 + 31) / 32 : 4;
 bool split_gemm_plan_whole(int M, int N, int K, int num_sms, float us, SplitPlan* out);
 // Whether launch_dense_gemm runs a product on these tiles, and how.
 bool dense_gemm_is_split(int M, int N, int K, int num_sms, SplitPlan* out);
+// The form launch_dense_gemm runs a product in: -1 these tiles, 0 one CTA per 128 x 256 tile, else the columns of a pair of CTAs; smem: shared memory
+// of a CTA of such a pair (0 for the others).
+int dense_gemm_form(int M, int N, int K, int num_sms, int* smem);
 // Sums in chunks, in an order that depends on N, K, the parts and the groups, not on M.  false: sizes not taken.
 bool split_gemm_plan(int M, int N, int K, int num_sms, int xparts, int wparts, int groups, SplitPlan* out);
 // binned rows (one weight matrix per row tile): a CTA per tile and 128 columns, K uncut
