@@ -60,11 +60,11 @@ constexpr int kNumEpiThreads = 256;
 
 template <int FMT>
 struct Fmt;
-// kStagesW: packed-weight ring depth of the wide form
+// kStagesW: packed-weight ring depth of the wide form, in K blocks
 template <> struct Fmt<kFmtInt4G128> { static constexpr int kTileBytes = kInt4TileBytes, kStagesW = 4; };
 template <> struct Fmt<kFmtInt8G128> { static constexpr int kTileBytes = kInt8TileBytes, kStagesW = 2; };
 template <> struct Fmt<kFmtQ8_0> { static constexpr int kTileBytes = kQ8_0TileBytes, kStagesW = 2; };
-template <> struct Fmt<kFmtQ4_K> { static constexpr int kTileBytes = kQ4KTileBytes, kStagesW = 3; };
+template <> struct Fmt<kFmtQ4_K> { static constexpr int kTileBytes = kQ4KTileBytes, kStagesW = 4; };
 template <> struct Fmt<kFmtAffine8> { static constexpr int kTileBytes = kAffine8TileBytes, kStagesW = 2; };
 template <int FMT>
 constexpr bool kHasScaleTiles = (FMT == kFmtInt4G128 || FMT == kFmtInt8G128);
@@ -83,7 +83,9 @@ struct SmemLayout {
   static constexpr int kBStageBytes = NT * kBlockK * 2;
   // token (B operand) ring: 4 stages wherever they fit the 227 KB (everything but the 12 KB Affine8 tiles).  With tcgen05.mma issued
   // at full rate the K loop waited ~200 cycles per k-block on token rows with 3 stages (profiles/r02i_gemm_item_timeline_*).
-  static constexpr int kStagesB = kShort ? 6 : (FMT == kFmtAffine8) ? 3 : 4;
+  // Q4_K gives one up for four K blocks of weights in place of two (three of them are not an even number, see below): a whole pass over 64 experts of
+  // 1536 columns, 1000 x 6 rows 240 -> 227 us, 2000 301 -> 293, 8192 959 -> 973; 128 experts of 768, 2000 x 8 rows 258 -> 248, 8192 722 -> 720.
+  static constexpr int kStagesB = kShort ? 6 : (FMT == kFmtAffine8 || FMT == kFmtQ4_K) ? 3 : 4;
   // K blocks per stage of packed weights: two, whose tiles lie side by side and whose scales are the same, wherever two stages of two fit.  The
   // producer takes 480 cycles to issue four copies; one K block each, that was the pace of the short form whatever the format.
   static constexpr int kKbW = kShort || Fmt<FMT>::kStagesW >= 4 ? 2 : 1;
@@ -94,6 +96,9 @@ struct SmemLayout {
   static constexpr int kOffW = kOffStage + NT * kStageRowBytes;
   static constexpr int kFitW = (227 * 1024 - 1024 - kOffW) / kWStageBytes;      // 1 KB left for weights of slots and barriers
   static constexpr int kStagesW = !kShort ? Fmt<FMT>::kStagesW / kKbW : kFitW < 16 ? kFitW : 16;
+  // The dequantiser groups take K blocks in turn.  With one block per stage each must always meet the same stages: one that another group has used in
+  // between has gone through two phases, and a wait for its parity is over before the data is there (copies from HBM do not end in their order).
+  static_assert(kKbW == 2 || kStagesW % 2 == 0, "stages of single K blocks: an even number");
   static constexpr int kOffSlotW = kOffW + kStagesW * kWStageBytes;             // GEMM2: routing weight of the chunk's token slots (f32)
   static constexpr int kOffBar = kOffSlotW + NT * 4;
   static constexpr int kNumBars = 2 * kStagesW + 2 * kStagesA + 2 * kStagesB + 2 * kAccBufs;
