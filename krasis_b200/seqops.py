@@ -176,12 +176,25 @@ class StepTables:
         self.h2d_bytes = n * 4
 
 
+def _plain_rows(cache: torch.Tensor) -> bool:
+    """Whether kb2_seq_portion_rows takes a cache as it lies."""
+    return cache.dtype == torch.bfloat16 and cache.is_contiguous() and cache.data_ptr() % 16 == 0
+
+
 def portion_rows(tb: StepTables, s: int, first: int, ca: torch.Tensor, wa: int, cb: torch.Tensor, wb: int, page_size: int, proj: torch.Tensor,
                  row0: int, n: int, nq: int):
     """The operands of sequence s's attention on the tensor cores, made in one launch: rows `first` up to the portion's end of two bfloat16
     caches (wa and wb numbers per row), and the first nq columns of proj's rows row0 .. row0 + n - 1 (fp32), rounded to bfloat16."""
-    _, m, start, _ = tb.layout[s]
+    _, m, start, pages = tb.layout[s]
     keys, dev = start + m - first, proj.device
+    if (start + m - 1) // page_size >= len(pages):           # the kernel would read on in the table
+        raise IndexError(f"sequence {s}: {len(pages)} pages of {page_size} rows do not hold {start + m} positions")
+    if not (_plain_rows(ca) and _plain_rows(cb)):
+        import numpy as np
+        j = np.arange(first, start + m, dtype=np.int64)
+        rows = torch.from_numpy(np.asarray(pages, dtype=np.int64)[j // page_size] * page_size + j % page_size).to(dev, non_blocking=True)
+        return (ca.view(-1, wa).index_select(0, rows), cb.view(-1, wb).index_select(0, rows),
+                proj[row0:row0 + n, :nq].to(torch.bfloat16).contiguous())
     a = torch.empty((keys, wa), dtype=torch.bfloat16, device=dev)
     b = torch.empty((keys, wb), dtype=torch.bfloat16, device=dev)
     q = torch.empty((n, nq), dtype=torch.bfloat16, device=dev)
