@@ -36,7 +36,7 @@ def _stamp(sources=None, header="krasis_b200.h"):
         for f in sorted(files):
             if sources is None and f in SEQ_SOURCES:
                 continue                      # the core library does not depend on the sequence operators
-            if sources is not None and f not in sources and f not in ("ptx.cuh", "pdl.cuh") and not (f.endswith(".cuh") and f.startswith("seq_")):
+            if sources is not None and f not in sources and f not in ("ptx.cuh", "pdl.cuh", "device_once.cuh") and not (f.endswith(".cuh") and f.startswith("seq_")):
                 continue
             h.update(open(os.path.join(root, f), "rb").read())
     h.update(open(os.path.join(HERE, "..", "include", header), "rb").read())

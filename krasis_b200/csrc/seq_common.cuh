@@ -9,6 +9,7 @@
 #include <stdio.h>
 
 #include "../../include/krasis_b200_seq.h"
+#include "device_once.cuh"
 #include "pdl.cuh"
 #include "seq_act.cuh"
 

@@ -390,7 +390,7 @@ static void launch_gemv_tiles(const void* A, long long lda, const void* B, long 
   const size_t smem = (size_t)(ks > 8 ? 16 : 8) * Piece::kRing;
 #define KB2_GEMV(KSV)                                                                                                                            \
   case KSV:                                                                                                                                      \
-    cudaFuncSetAttribute(gemv_mma_kernel<TA, TC, KSV, kTiles>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                                  \
+    kb2::allow_smem<gemv_mma_kernel<TA, TC, KSV, kTiles>>((KSV > 8 ? 16 : 8) * Piece::kRing);                                                        \
     kb2::launch_pdl(gemv_mma_kernel<TA, TC, KSV, kTiles>, grid, KSV > 8 ? 512 : 256, smem, s, (const TA*)A, lda, (const bf16*)B, ldb, (TC*)C, ldc, M, N, K, \
                     sA, sB, sC);                                                                                                                 \
     break;
@@ -2506,9 +2506,11 @@ static int launch_delta_tiles(const DeltaScratch& z, DeltaPrep p, float* state, 
   p.vimage = scratch + z.tiles * (p.Hk * z.image + p.H * z.wimage);
   p.sc = p.vimage + z.tiles * p.H * kDT * p.dv;
   *o = p.sc + z.tiles * p.H * kDTScalars;
-  SEQ_CUDA(cudaFuncSetAttribute(delta_tile_prep_kernel<NI, VB>, cudaFuncAttributeMaxDynamicSharedMemorySize, D::prep_smem(VB, p.H / p.Hk)));
-  SEQ_CUDA(cudaFuncSetAttribute(delta_tile_kernel<NI>, cudaFuncAttributeMaxDynamicSharedMemorySize, D::kSmem));
-  kb2::launch_pdl(delta_tile_prep_kernel<NI, VB>, (unsigned)(z.tiles * p.Hk), 256, D::prep_smem(VB, p.H / p.Hk), st, p);
+  const int prep_smem = D::prep_smem(VB, p.H / p.Hk);
+  if (prep_smem > 227 * 1024) return failf(KB2SEQ_ERR_VALUE, "delta_tiles: %d heads per key head are too many", p.H / p.Hk);
+  SEQ_CUDA((kb2::allow_smem<delta_tile_prep_kernel<NI, VB>>(227 * 1024)));
+  SEQ_CUDA((kb2::allow_smem<delta_tile_kernel<NI>>(D::kSmem)));
+  kb2::launch_pdl(delta_tile_prep_kernel<NI, VB>, (unsigned)(z.tiles * p.Hk), 256, prep_smem, st, p);
   SEQ_LAUNCHED();
   kb2::launch_pdl(delta_tile_kernel<NI>, dim3(p.S, p.H, p.dv / 32), D::kThreads, D::kSmem, st, p.image, p.wimage, p.vimage, p.sc, p.H, p.Hk, p.dv, state,
                   p.cu, slots, *o);
