@@ -265,10 +265,17 @@ __device__ __forceinline__ uint32_t lead_pair(float& a, float& b) {
   return __byte_perm(ua, ub, 0x7632);
 }
 
-__device__ __noinline__ float row_product(const float* a, const bf16* b, int K) {
+// A product in plain fp32 by a warp; K a multiple of 8, both rows 16-byte aligned.
+__device__ __noinline__ float row_product(const float* a, const bf16* b, int K, int lane) {
   float v = 0.f;
-  for (int k = 0; k < K; ++k) v = fmaf(a[k], __bfloat162float(b[k]), v);
-  return v;
+  for (int k = lane * 8; k < K; k += 256) {
+    float x[8], w[8];
+    load8(a + k, x);
+    load8(b + k, w);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v = fmaf(x[i], w[i], v);
+  }
+  return warp_sum(v);
 }
 
 template <typename TA, typename TC, int KS, int kTiles>
@@ -363,7 +370,7 @@ __global__ void __launch_bounds__(KS > 8 ? 512 : 256) gemv_mma_kernel(const TA* 
   __syncthreads();
   for (int i = threadIdx.x; i < kGroups * 8 * kRows; i += kWarps * 32) {
     const int g = i / (8 * kRows), mm = i / kRows % 8, r = i % kRows, n = (blockIdx.x * kGroups + g) * kRows + r;
-    if (mm >= M || n >= N) continue;
+    const bool in = mm < M && n < N;
     float v[KS];
 #pragma unroll
     for (int p = 0; p < KS; ++p) v[p] = red[g * KS + p][mm][r];
@@ -372,9 +379,13 @@ __global__ void __launch_bounds__(KS > 8 ? 512 : 256) gemv_mma_kernel(const TA* 
 #pragma unroll
       for (int p = 0; p < o; ++p) v[p] += v[p + o];
     if constexpr (kFp32) {
-      if (!isfinite(v[0])) v[0] = row_product(A + (long long)mm * lda, B + (long long)n * ldb, K);
+      for (unsigned again = __ballot_sync(0xffffffffu, in && !isfinite(v[0])); again; again &= again - 1) {      // the whole warp for one output after the other
+        const int src = __ffs(again) - 1;
+        const float t = row_product(A + (long long)__shfl_sync(0xffffffffu, mm, src) * lda, B + (long long)__shfl_sync(0xffffffffu, n, src) * ldb, K, lane);
+        if (lane == src) v[0] = t;
+      }
     }
-    stf(C, (long long)mm * ldc + n, v[0]);
+    if (in) stf(C, (long long)mm * ldc + n, v[0]);
   }
 }
 

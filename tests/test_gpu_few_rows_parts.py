@@ -31,3 +31,25 @@ def test_not_finite():
     assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
     inf = torch.isinf(want)
     assert torch.equal(got[inf].sign(), want[inf].sign().float())
+
+
+def test_a_row_that_is_not_finite_costs_no_more_than_a_few_products():
+    """Its sums are made again one after the other, each by a warp: not by one thread along all of K."""
+    g = torch.Generator(device="cuda").manual_seed(2)
+    w, x = torch.randn(16384, 8192, device="cuda", generator=g).bfloat16(), torch.randn(4, 8192, device="cuda", generator=g)
+
+    def best(x):
+        times = []
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            ops.gemm(x, w, torch.float32)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+    plain = best(x)
+    x[2, 77] = float("nan")
+    got = ops.gemm(x, w, torch.float32)
+    assert torch.isnan(got[2]).all() and torch.isfinite(got[[0, 1, 3]]).all()
+    assert best(x) < 8 * plain          # a warp: the weights once more, in turn; a thread reads 2 bytes of them at a time, hundreds of times in turn
