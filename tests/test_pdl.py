@@ -19,22 +19,86 @@ def _closing(text, at):
     raise AssertionError("unbalanced")
 
 
-def test_launched_kernels_wait():
-    bodies, launched = {}, set()
-    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
-        text = re.sub(r"//[^\n]*", "", open(path).read())
+def _sources():
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))):
+        yield os.path.basename(path), re.sub(r"//[^\n]*", "", open(path).read())
+
+
+def _first_argument(text, at):
+    """The first argument of the call whose parenthesis opens at `at`."""
+    depth = 0
+    for i in range(at, len(text)):
+        c = text[i]
+        depth += c in "([{"
+        depth -= c in ")]}"
+        if (c == "," and depth == 1 and text.count("<", at, i) <= text.count(">", at, i)) or depth == 0:
+            return text[at + 1:i].strip()
+    raise AssertionError("unbalanced")
+
+
+def _launched():
+    """{kernel: where} of every programmatic launch, those through a variable among them."""
+    found = {}
+    for name, text in _sources():
+        for m in re.finditer(r"(?:launch_pdl|cudaLaunchKernelEx)(\()", text):
+            ahead = text[:m.start()]
+            what = _first_argument(text, m.start(1))
+            if what in ("void (*kernel)(P...)",) or name == "pdl.cuh":       # the helper itself
+                continue
+            if what == "&cfg":
+                what = re.match(r"&cfg,\s*(\w+)", text[m.end(1):]).group(1)
+            kernels = re.findall(r"\w+_kernel\b", what)
+            if not kernels:                                                 # a variable: what it was last set to
+                assert re.fullmatch(r"\w+", what), (name, what)
+                kernels = re.findall(r"\w+_kernel\b", re.findall(r"auto %s = ([^;]*);" % what, ahead)[-1])
+            assert kernels, (name, what)
+            found.update({k: name for k in kernels})
+    return found
+
+
+def _bodies():
+    out = {}
+    for _, text in _sources():
         for m in re.finditer(r"__global__", text):
             k = re.compile(r"(\w+_kernel)\s*\(").search(text, m.end())
-            start = text.index("{", _closing(text, k.end() - 1))
-            bodies[k.group(1)] = text[start:_closing(text, start)]
-        launched |= set(re.findall(r"launch_pdl\((\w+_kernel)", text))
-    launched |= {"split_gemm_kernel", "grouped_gemm_kernel"}               # launched through a variable
-    assert len(launched) > 60
+            end = _closing(text, k.end() - 1)
+            start = text.index("{", end)
+            out[k.group(1)] = (text[k.end():end], text[start:_closing(text, start)])
+    return out
+
+
+def _reads_ahead(params, ahead):
+    """What a kernel's statements ahead of its wait do that they must not: leave, or touch memory that its parameters lead to."""
+    bad = [w for w in ("return", "__ldg", "tma_load", "tma_gather", "bulk_g2s", "bulk_s2g", "atomic", "cp_async", "ld_stream", "->") if w in ahead]
+    for p in re.split(r",(?![^<]*>)", params):
+        name = re.search(r"(\w+)\s*$", p.strip())
+        if name is None:
+            continue
+        n = name.group(1)
+        if "*" in p:
+            bad += [n] if re.search(r"\b%s\s*\[|\*\s*%s\b" % (n, n), ahead) else []
+        else:
+            bad += [n] if re.search(r"\b%s\.\w+\s*\[|[=(,;?:{&|!<>+-]\s*\*\s*%s\.\w+" % (n, n), ahead) else []
+    return bad
+
+
+def test_launched_kernels_wait():
+    bodies, launched = _bodies(), _launched()
+    assert len(launched) > 80
+    for k in ("split_gemm_kernel", "grouped_gemm_kernel", "split_weight_parts_kernel", "portion_rows_kernel", "dense_pair_kernel"):
+        assert k in launched, k
     for name in sorted(launched):
-        calls = re.findall(r"pdl_(?:enter|wait)\(", bodies[name])
-        assert len(calls) == 1, name
-        ahead = bodies[name][:re.search(r"pdl_(?:enter|wait)\(", bodies[name]).start()]
-        assert "return" not in ahead and "__ldg" not in ahead and "tma_load" not in ahead and "bulk_g2s" not in ahead, name
+        params, body = bodies[name]
+        assert len(re.findall(r"pdl_(?:enter|wait)\(", body)) == 1, name
+        assert not _reads_ahead(params, body[:re.search(r"pdl_(?:enter|wait)\(", body).start()]), name
+
+
+@pytest.mark.parametrize("name", ["split_weight_parts_kernel", "portion_rows_kernel", "split_gemm_kernel", "conv_run_vec_kernel"])
+def test_a_kernel_without_its_wait_is_found(name):
+    """The check above on kernels whose wait comes after their first access."""
+    params, body = _bodies()[name]
+    moved = re.sub(r"(?:kb2::)?pdl_(?:enter|wait)\([^;]*;", "", body) + "pdl_wait("
+    assert _reads_ahead(params, moved[:moved.index("pdl_wait(")])
 
 
 @pytest.mark.gpu
