@@ -9,7 +9,9 @@ pytestmark = pytest.mark.gpu
 
 # widths around the 1024 columns of a block and one that the scalar form takes, up to eight choices, more, and more than the table of choices holds
 @pytest.mark.parametrize("T,top,W,pos,gate", [(1, 1, 4, True, False), (5, 6, 1020, True, True), (3, 8, 1028, False, False), (7, 9, 2048, True, True),
-                                              (2, 64, 512, True, False), (2, 65, 512, True, False), (4, 6, 1022, True, True)])
+                                              (2, 64, 512, True, False), (2, 65, 512, True, False), (4, 6, 1022, True, True),
+                                              # long steps of few choices: a block per token
+                                              (512, 1, 1028, True, True), (1024, 4, 36, False, False), (1024, 2, 4, True, True)])
 def test_combine(T, top, W, pos, gate):
     E, ident = 16, 3
     g = torch.Generator().manual_seed(W + top)
