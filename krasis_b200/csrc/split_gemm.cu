@@ -430,7 +430,7 @@ cudaError_t launch_split_gemm(const SplitGemm& g, const SplitPlan& plan, cudaStr
   p.glu_limit = g.glu_limit;
   p.glu_alpha = g.glu_alpha;
   if (g.glu && (g.out_f32 || g.xparts != 1 || g.bias != nullptr || g.N % 32)) return cudaErrorInvalidValue;
-  p.low_span = split_low_span(g.K);
+  p.low_span = split_low_span(g.N, g.K, g.groups);
   p.low_spans = ceil_div(nkb, p.low_span);
   if (g.wparts > 1 && g.w_low == nullptr) return cudaErrorInvalidValue;
   const int ring = plan.stages * (g.wparts * kSWBytes + nt * 128);
@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(512) split_weight_parts_kernel(const float* __
 
 cudaError_t launch_split_weights(const float* w, int N, int K, int groups, void* parts, uint8_t* low, cudaStream_t s) {
   KernelSpan span(K_DENSE_BF16, s);
-  const int tiles = ceil_div(N, kSRows), cols = split_low_span(K) * kBlockK, spans = ceil_div(K, cols);
+  const int tiles = ceil_div(N, kSRows), cols = split_low_span(N, K, groups) * kBlockK, spans = ceil_div(K, cols);
   const unsigned blocks = (unsigned)groups * tiles * spans;
   auto kern = (uintptr_t)w & 15 ? split_weight_parts_kernel<false> : split_weight_parts_kernel<true>;
   return launch_pdl(kern, blocks, 512, 0, s, w, N, K, (long long)groups * N, tiles, cols, spans, (__nv_bfloat16*)parts, low);
