@@ -343,15 +343,19 @@ static cudaError_t dense_configure() {
 }
 
 // Columns per tile of dense_pair_kernel, or 0 where the 128 x 256 tiles of one CTA are estimated to be faster; *us: the estimate.  Constants fitted
-// to 120 timings (M 1000..8192, N 2048..16384, K 2048..8192, tiles of 96..256 columns); the choice is within 4 % of the best one at all of them, 1 %
-// on average.  On both sides of the line: M 2048, N 9216, K 2048 56.0 against 63.4 us with one CTA, M 2048, N 2048, K 4096 33.1 against 32.3.
+// to timings of calls that follow one another in a stream at 323 shapes (M 256..8192, N 512..16384, K 512..8192), together with the line to split_gemm.cu;
+// the weights' way from HBM bounds a pair's time from below.  Against the estimates before, which were of launches that wait for one another, these
+// shapes take 0.987 of the time (geometric mean): M 700, N 2048, K 512 7.8 -> 6.2 us, M 1700, N 1536, K 2048 15.3 -> 13.2, M 1000, N 10240, K 8192 158 ->
+// 134, M 300, N 12288, K 2048 31.7 -> 28.5; the worst M 2600, N 2048, K 512 11.5 -> 13.0, M 1300, N 6144, K 5120 64.7 -> 70.5.
 static int dense_pair_plan(int M, int N, int K, int num_sms, float* us) {
   const int nkb = K / kBlockK, pairs = num_sms / 2;
   const auto rounds = [](long long tiles, int at_once) { return (float)((tiles + at_once - 1) / at_once); };
   int best = 0;
-  *us = 5.f + 0.46f * nkb * rounds((long long)((M + 127) / 128) * ((N + 255) / 256), num_sms);
+  const float hbm = (float)N * K * 2.f / 5.76e6f;
+  *us = 3.6f + 0.345f * nkb * rounds((long long)((M + 127) / 128) * ((N + 255) / 256), num_sms);
   for (int nt = 256; nt >= 96; nt -= 16) {
-    const float time = 4.f + (1.f + nkb * (0.1f + 0.0011f * nt)) * rounds((long long)((M + 255) / 256) * ((N + nt - 1) / nt), pairs);
+    const float work = (1.1f + nkb * (0.0867f + 0.0007f * nt)) * rounds((long long)((M + 255) / 256) * ((N + nt - 1) / nt), pairs);
+    const float time = 5.3f + (work > hbm ? work : hbm);
     if (time < *us) {
       *us = time;
       best = nt;

@@ -356,11 +356,12 @@ static bool cheapest(int M, int N, int K, bool whole, int num_sms, int xparts, i
   return found;
 }
 
-// Taken only where the wide tiles of dense_gemm.cu are estimated to take longer (us).  Measured on both sides of the line (this / wide): M 1000, N 2048,
-// K 2048 14.0 / 14.4 us; M 2000 at the same shape 25.2 / 18.2; M 515, N 12288 26.6 / 32.1; M 700 32.2 / 32.0; M 256, N 9216 15.6 / 15.3.
+// Taken only where the wide tiles of dense_gemm.cu are estimated to take longer (us).  Launches that wait for one another, on both sides of the line (this /
+// wide): M 1000, N 2048, K 2048 14.0 / 14.4 us; M 2000 at the same shape 25.2 / 18.2; M 515, N 12288 26.6 / 32.1; M 700 32.2 / 32.0.
 bool split_gemm_plan_whole(int M, int N, int K, int num_sms, float us, SplitPlan* out) {
   if (M <= 0 || M > 2048 || K % kBlockK || N % 16) return false;
-  float best = us;
+  // the estimates of `cheapest` are of launches that wait for one another, `us` is of launches in a stream: both fitted at 323 shapes
+  float best = (us + 2.1f) / 0.948f;
   return cheapest(M, N, K, true, num_sms, 1, 1, 1, 1, &best, out);
 }
 
