@@ -1,4 +1,4 @@
-// Once per device and kernel: the opt-in to more shared memory than 48 KB.
+// What a launch asks a device once: the opt-in to more shared memory than 48 KB, the number of SMs.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -20,6 +20,17 @@ struct PerDeviceOnce {
   }
   void mark(int dev) { if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release); }
 };
+
+// SMs of the current device
+inline int current_sms() {
+  static std::atomic<int> known[64];
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  if ((sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return 148;
+  known[dev].store(sms, std::memory_order_relaxed);
+  return sms;
+}
 
 // The opt-in of kKernel to `bytes` of dynamic shared memory, the most that any of its launches takes: a size that followed from a call's arguments
 // could be lowered by another thread between a call's opt-in and its launch.

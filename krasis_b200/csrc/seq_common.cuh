@@ -13,6 +13,8 @@
 #include "pdl.cuh"
 #include "seq_act.cuh"
 
+#include <algorithm>
+
 namespace kb2seq {
 
 typedef __nv_bfloat16 bf16;

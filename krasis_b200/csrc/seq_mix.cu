@@ -1037,7 +1037,7 @@ KB2SEQ_API int kb2_seq_portion_rows(const void* cache_a, int wa, const void* cac
       keys <= 0 || n <= 0 || (((uintptr_t)cache_a | (uintptr_t)cache_b | (uintptr_t)a | (uintptr_t)b | (uintptr_t)qb) & 15))
     return failf(KB2SEQ_ERR_VALUE, "portion_rows: bad argument");
   const long long total = (long long)keys * (wa + wb) / 8 + (long long)n * nq / 8;
-  const unsigned blocks = (unsigned)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
+  const unsigned blocks = (unsigned)std::min((total + 255) / 256, kb2::current_sms() * 16ll);
   const bool vec = ldq % 4 == 0 && !((uintptr_t)q & 15);
   auto kern = vec ? portion_rows_kernel<true> : portion_rows_kernel<false>;
   kb2::launch_pdl(kern, blocks, 256, 0, (cudaStream_t)stream, (const uint4*)cache_a, wa / 8, (const uint4*)cache_b, wb / 8, pages, page_size, first, keys,
@@ -1127,14 +1127,14 @@ KB2SEQ_API int kb2_seq_glu(const void* in, int dt_in, long long ld_in, void* out
     return failf(KB2SEQ_ERR_VALUE, "glu: bad argument");
   if (dt_in == 1 && dt_out == 1 && F % 8 == 0 && ld_in % 8 == 0 && !((uintptr_t)in & 15) && !((uintptr_t)out & 15) && !((uintptr_t)bias & 15)) {
     const long long n8 = rows * (F / 8);
-    const unsigned blocks8 = (unsigned)((n8 + 255) / 256 > 148 * 16 ? 148 * 16 : (n8 + 255) / 256);
+    const unsigned blocks8 = (unsigned)std::min((n8 + 255) / 256, kb2::current_sms() * 16ll);
     kb2::launch_pdl(glu_bf16x8_kernel, blocks8, 256, 0, (cudaStream_t)stream, (const bf16*)in, ld_in, (bf16*)out, rows, F, kind, limit, alpha, n_tiles, tile_rows, bias, row_w,
                                                               row_map);
     SEQ_LAUNCHED();
     return KB2SEQ_OK;
   }
   const long long n = rows * F;
-  const unsigned blocks = (unsigned)((n + 255) / 256 > 148 * 16 ? 148 * 16 : (n + 255) / 256);
+  const unsigned blocks = (unsigned)std::min((n + 255) / 256, kb2::current_sms() * 16ll);
   kb2::launch_pdl(glu_kernel, blocks, 256, 0, (cudaStream_t)stream, in, dt_in, ld_in, out, dt_out, rows, F, kind, limit, alpha, n_tiles, tile_rows, bias, row_w,
                                                               row_map);
   SEQ_LAUNCHED();

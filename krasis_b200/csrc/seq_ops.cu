@@ -418,7 +418,7 @@ static bool launch_gemv_mma(const void* A, long long lda, const void* B, long lo
   // N 512, K 1024 2.7 / 3.5 / 5.3 / 9.7, 2.1; N 4096, K 224 2.3 / 2.7 / 3.4 / 5.2, 2.2; N 256, K 2048 2.2 / 2.6 / 3.5 / 5.6, 2.7; N 128, K 8184
   // 3.9 / 5.6 / 9.2 / 17, 6.2
   if constexpr (sizeof(TA) == 4) {             // 32 weight rows a warp where that still gives every SM a block (N 2048, K 8192: 15.9 us, with 16 rows 11.2)
-    if ((long long)((N + 31) / 32) * batch >= 148) {
+    if ((long long)((N + 31) / 32) * batch >= kb2::current_sms()) {
       launch_gemv_tiles<TA, TC, 2>(A, lda, B, ldb, C, ldc, M, N, K, batch, sA, sB, sC, s);
       return true;
     }
@@ -2427,7 +2427,7 @@ static int delta_out_launch(const float* o, const float* gproj, long long ldg, i
                             void* out, int dt_out, cudaStream_t st) {
   const unsigned blocks = (unsigned)(((long long)T * H + 7) / 8);
   const bool vec = dv % 4 == 0 && ldg % 4 == 0 && !(((uintptr_t)o | (uintptr_t)gproj | (uintptr_t)norm_w | (uintptr_t)out) & 15);
-  if (vec && dv == 128 && blocks >= 148 * 16)         // from two full rounds of resident blocks on
+  if (vec && dv == 128 && blocks >= kb2::current_sms() * 16u)         // from two full rounds of resident blocks on
     kb2::launch_pdl(delta_out_rows_kernel, (blocks + 3) / 4, 256, 0, st, o, gproj, ldg, gate_act, H, norm_w, eps, (long long)T * H, out, dt_out);
   else if (vec)
     kb2::launch_pdl(delta_out_kernel<4>, blocks, 256, 0, st, o, gproj, ldg, gate_act, H, dv, norm_w, eps, T, out, dt_out);
