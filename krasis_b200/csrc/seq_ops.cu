@@ -1594,7 +1594,8 @@ struct DeltaPrep {
   const float *bproj, *aproj, *A_log, *dt_bias;
   int H, Hk, dv, S;
   const int* cu;
-  long long tiles;
+  long long f0, f1;                // the slice of the step's tiles that is worked on: images lie from tile f0 on
+  bool whole;                      // the slice is all of them
   bf16 *image, *wimage;
   float *vimage, *sc;
 };
@@ -1609,8 +1610,8 @@ __device__ __forceinline__ void delta_fetch(const DeltaPrep& p, int t0, int nt, 
   }
 }
 
-// A block of eight warps per (tile, key head).  Bound by traffic: 16 bytes of k, q and v in and 26 out per token and column (4096 tokens, 32 / 16
-// heads x 128).  All loops are rolled as far as registers allow: with everything unrolled and a warp for each part the block took 35 KB of
+// A block of eight warps per (tile, key head).  Mostly traffic: at 4096 tokens, 32 / 16 heads x 128, 134 MB of k, q and v come
+// in and 304 MB go out in 107 us, 0.62 of the copy rate; the rest is the chain of a tile's products.  All loops are rolled as far as registers allow: with everything unrolled and a warp for each part the block took 35 KB of
 // instructions once, and waiting for them was most of its time.
 // image [tiles][Hk] | W [tiles][H] | V' [tiles][H][dv / 16][lane][8], in the order in which a lane of delta_tile_kernel takes them | scalars [tiles][H]
 template <int NI, int VB>
@@ -1622,7 +1623,7 @@ __global__ void __launch_bounds__(256, 3) delta_tile_prep_kernel(const DeltaPrep
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = tid & 31;
   const long long flat = blockIdx.x / p.Hk;
   const int hk = (int)(blockIdx.x - flat * p.Hk), H = p.H, rep = H / p.Hk;
-  long long tile = flat;
+  long long tile = p.f0 + flat;
   int sq = 0, t0 = 0, n = 0;                          // the tile's sequence: tiles are counted sequence by sequence
   for (; sq < p.S; ++sq) {
     t0 = p.cu[sq];
@@ -1896,7 +1897,7 @@ template <int NI>
 __global__ void __launch_bounds__(DeltaTile<NI>::kThreads, 1)
     delta_tile_kernel(const bf16* __restrict__ image, const bf16* __restrict__ wimage, const float* __restrict__ vimage, const float* __restrict__ sc,
                       int H, int Hk, int dv, float* __restrict__ state, const int* __restrict__ cu, const int* __restrict__ slots,
-                      float* __restrict__ o_out) {
+                      float* __restrict__ o_out, long long f0, long long f1, bool whole) {
   kb2::pdl_enter(image, wimage, vimage, sc, state, cu, slots, o_out);
   using D = DeltaTile<NI>;
   extern __shared__ __align__(128) uint8_t tsm[];
@@ -1909,7 +1910,18 @@ __global__ void __launch_bounds__(DeltaTile<NI>::kThreads, 1)
   uint64_t* o_free = o_there + 4;                  // the read-out has taken them
   const int s = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * 32, hk = h / (H / Hk);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int t0 = cu[s], n = cu[s + 1] - cu[s], tiles = (n + kDT - 1) / kDT;
+  const int n_all = cu[s + 1] - cu[s];
+  long long first = 0;                             // the sequence's tiles come after those of the sequences before it
+  if (!whole || warp == 2 * NI + 2)
+    for (int i = 0; i < s; ++i) first += (cu[i + 1] - cu[i] + kDT - 1) / kDT;
+  int skip = 0, tiles = (n_all + kDT - 1) / kDT;   // tiles of the sequence ahead of the slice, and in it
+  if (!whole) {
+    const long long all = first + tiles;
+    skip = (int)(min(max(f0, first), all) - first);
+    tiles = (int)(min(max(f1, first), all) - first) - skip;
+    if (tiles == 0) return;
+  }
+  const int t0 = cu[s] + skip * kDT, n = n_all - skip * kDT;      // tokens from the slice on
   if (threadIdx.x == 0) {
     for (int i = 0; i < kDTStages; ++i) {
       kb2::mbar_init(&full[i], 1);
@@ -1925,15 +1937,13 @@ __global__ void __launch_bounds__(DeltaTile<NI>::kThreads, 1)
   __syncthreads();
   const int quad = lane >> 2, pair = (lane & 3) * 2;      // fragment: columns quad, quad + 8; rows or tokens pair, pair + 1
   if (warp == 2 * NI + 2) {                        // ---- the tiles' way into shared memory
-    long long first = 0;                           // the sequence's tiles come after those of the sequences before it
-    for (int i = 0; i < s; ++i) first += (cu[i + 1] - cu[i] + kDT - 1) / kDT;
     for (int i = 0; i < tiles; ++i) {
       const int st = i % kDTStages;
       uint8_t* b = tsm + st * D::kStageBytes;
       kb2::mbar_wait(&empty[st], (uint32_t)(i / kDTStages & 1) ^ 1u);
       if (lane == 0) kb2::mbar_arrive_expect_tx(&full[st], (uint32_t)D::kStageBytes);
       __syncwarp();
-      const long long flat = first + i;
+      const long long flat = first + skip + i - f0;
       if (lane == 0) kb2::bulk_g2s(b, image + (flat * Hk + hk) * D::kImage, D::kImageBytes, &full[st]);
       else if (lane == 1) kb2::bulk_g2s(b + D::kImageBytes, wimage + (flat * H + h) * D::kWImage, D::kWBytes, &full[st]);
       else if (lane == 2) kb2::bulk_g2s(b + D::kImageBytes + D::kWBytes, vimage + (flat * H + h) * kDT * dv + j0 * kDT, D::kVBytes, &full[st]);
@@ -2492,14 +2502,20 @@ static int delta_rule_launch(const float* conv, int C, const float* bproj, long 
   return KB2SEQ_OK;
 }
 
-// scratch: images of k and q [tiles][Hk] | of W [tiles][H] | V' [tiles][H][16 dv] | scalars [tiles][H] | o [T, H, dv]; at most T / 16 + S tiles, a
-// partial one per sequence
+// scratch: images of k and q [slice][Hk] | of W [slice][H] | V' [slice][H][16 dv] | scalars [slice][H] | o [T, H, dv].  At most T / 16 + S tiles, a
+// partial one per sequence.  What belongs to tiles (74 KB per token with 32 / 16 heads x 128, twice that of tiles of eight, which had no W and no V') is
+// made and used a slice of tiles at a time, so that it stays below kDeltaSliceBytes: 8192 tokens take 435 MB in all instead of 704, in 2 % more time.
+// Slices of 96 MB cost 5 to 7 % (4096 tokens 488 -> 524 us) and 20 % with several sequences, whose chains no longer run side by side.
+constexpr long long kDeltaSliceBytes = 320ll << 20;
 struct DeltaScratch {
-  long long tiles, image, wimage, floats;             // floats of an image, of W, of everything
+  long long tiles, slice, image, wimage, floats;      // floats of an image, of W, of everything
   DeltaScratch(int T, int S, int H, int Hk, int dk, int dv) : tiles((long long)T / kDT + S) {
     image = dk == 32 ? DeltaTile<1>::kImage / 2 : dk == 64 ? DeltaTile<2>::kImage / 2 : DeltaTile<4>::kImage / 2;
     wimage = image / 2;
-    floats = tiles * (Hk * image + H * (wimage + (long long)kDT * dv + kDTScalars)) + (long long)T * H * dv;
+    const long long per = Hk * image + H * (wimage + (long long)kDT * dv + kDTScalars), most = std::max(1ll, kDeltaSliceBytes / 4 / per);
+    const long long slices = (tiles + most - 1) / most;
+    slice = (tiles + slices - 1) / slices;
+    floats = slice * per + (long long)T * H * dv;
   }
 };
 KB2SEQ_API long long kb2_seq_delta_tiles_scratch(int T, int S, int H, int Hk, int dk, int dv) {
@@ -2511,21 +2527,24 @@ extern "C++" {
 template <int NI, int VB>
 static int launch_delta_tiles(const DeltaScratch& z, DeltaPrep p, float* state, const int* slots, float* scratch, float** o, cudaStream_t st) {
   using D = DeltaTile<NI>;
-  p.tiles = z.tiles;
   p.image = (bf16*)scratch;
-  p.wimage = (bf16*)(scratch + z.tiles * p.Hk * z.image);
-  p.vimage = scratch + z.tiles * (p.Hk * z.image + p.H * z.wimage);
-  p.sc = p.vimage + z.tiles * p.H * kDT * p.dv;
-  *o = p.sc + z.tiles * p.H * kDTScalars;
+  p.wimage = (bf16*)(scratch + z.slice * p.Hk * z.image);
+  p.vimage = scratch + z.slice * (p.Hk * z.image + p.H * z.wimage);
+  p.sc = p.vimage + z.slice * p.H * kDT * p.dv;
+  *o = p.sc + z.slice * p.H * kDTScalars;
+  p.whole = z.slice == z.tiles;
   const int prep_smem = D::prep_smem(VB, p.H / p.Hk);
   if (prep_smem > 227 * 1024) return failf(KB2SEQ_ERR_VALUE, "delta_tiles: %d heads per key head are too many", p.H / p.Hk);
   SEQ_CUDA((kb2::allow_smem<delta_tile_prep_kernel<NI, VB>>(227 * 1024)));
   SEQ_CUDA((kb2::allow_smem<delta_tile_kernel<NI>>(D::kSmem)));
-  kb2::launch_pdl(delta_tile_prep_kernel<NI, VB>, (unsigned)(z.tiles * p.Hk), 256, prep_smem, st, p);
-  SEQ_LAUNCHED();
-  kb2::launch_pdl(delta_tile_kernel<NI>, dim3(p.S, p.H, p.dv / 32), D::kThreads, D::kSmem, st, p.image, p.wimage, p.vimage, p.sc, p.H, p.Hk, p.dv, state,
-                  p.cu, slots, *o);
-  SEQ_LAUNCHED();
+  for (p.f0 = 0; p.f0 < z.tiles; p.f0 += z.slice) {
+    p.f1 = std::min(p.f0 + z.slice, z.tiles);
+    kb2::launch_pdl(delta_tile_prep_kernel<NI, VB>, (unsigned)((p.f1 - p.f0) * p.Hk), 256, prep_smem, st, p);
+    SEQ_LAUNCHED();
+    kb2::launch_pdl(delta_tile_kernel<NI>, dim3(p.S, p.H, p.dv / 32), D::kThreads, D::kSmem, st, p.image, p.wimage, p.vimage, p.sc, p.H, p.Hk, p.dv, state,
+                    p.cu, slots, *o, p.f0, p.f1, p.whole);
+    SEQ_LAUNCHED();
+  }
   return KB2SEQ_OK;
 }
 }  // extern "C++"

@@ -1,4 +1,4 @@
-"""The delta rule eight tokens at a time, the short convolution's vector form and the gated read-out at their edges, against fp64."""
+"""The delta rule sixteen tokens at a time, the short convolution's vector form and the gated read-out at their edges, against fp64."""
 import pytest
 import torch
 
@@ -48,9 +48,9 @@ def _exact(m, h, tb, tail, state, lens, slots):
     return torch.cat(outs), states
 
 
-# portions that end anywhere in a tile of eight, one-token portions beside long ones, an odd number of slices and heads per key head
+# portions that end anywhere in a tile of sixteen, one-token portions beside long ones, an odd number of slices and heads per key head
 @pytest.mark.parametrize("H,Hk,dk,dv", [(2, 1, 32, 32), (4, 4, 64, 96), (6, 2, 128, 64), (9, 1, 32, 32)])
-@pytest.mark.parametrize("lens", [[16], [17, 1, 18], [1, 31, 2, 3], [64, 67], [71, 70, 69, 68]])
+@pytest.mark.parametrize("lens", [[16], [17, 1, 18], [1, 31, 2, 3], [64, 67], [71, 70, 69, 68], [15, 33], [79, 80, 81], [96, 1, 95]])
 @pytest.mark.parametrize("decay", [-3.0, 3.0])                 # slow, and so fast that a tile forgets all it knew
 def test_tiles_against_exact_and_token_form(H, Hk, dk, dv, lens, decay):
     m = _mixer(H, Hk, dk, dv, decay=decay)
@@ -118,6 +118,27 @@ def _rule(conv, proj, H, Hk, dk, dv, lens, state, tiles=True):
     s = torch.cuda.current_stream().cuda_stream
     ops.check(lib.kb2_seq_delta_tiles(*a, int(n), out.data_ptr(), 0, s) if tiles else lib.kb2_seq_delta_rule(*a, out.data_ptr(), 0, s))
     return out.view(T, H, dv), state
+
+
+@pytest.mark.parametrize("lens", [[3000, 1, 4001, 190], [16, 6500], [1, 1, 6200, 17, 1000]])
+def test_tiles_that_go_in_slices(lens):
+    """A step whose tiles do not fit the workspace at once, beside sequences that end in one slice or another: each as by itself, bit for bit."""
+    H, Hk, dk, dv, T = 32, 16, 128, 128, sum(lens)
+    size = lambda n: ops.load().kb2_seq_delta_tiles_scratch(n, 1, H, Hk, dk, dv) - n * H * dv  # noqa: E731
+    assert size(T) < 1.1 * size(T // 2)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    conv, proj = torch.randn(T, 2 * Hk * dk + H * dv, device="cuda", generator=g), torch.randn(T, H * dv + 2 * H, device="cuda", generator=g)
+    state = torch.randn(len(lens), H, dk, dv, device="cuda", generator=g)
+    got, after = _rule(conv, proj, H, Hk, dk, dv, lens, state)
+    at = 0
+    for s, n in enumerate(lens):
+        here = state[s:s + 1]
+        for a in range(0, n, 3200):                              # portions of whole tiles that one slice holds
+            m = min(3200, n - a)
+            alone, here = _rule(conv[at + a:at + a + m], proj[at + a:at + a + m], H, Hk, dk, dv, [m], here)
+            assert torch.equal(got[at + a:at + a + m], alone)
+        assert torch.equal(after[s], here[0])
+        at += n
 
 
 @pytest.mark.parametrize("what", ["value", "key", "query", "decay", "strength"])
