@@ -2562,9 +2562,12 @@ KB2SEQ_API int kb2_seq_delta_tiles(const float* conv, int C, const float* proj, 
   p.conv = conv; p.C = C; p.ldp = ldp; p.bproj = proj + b_off; p.aproj = proj + a_off; p.A_log = A_log; p.dt_bias = dt_bias;
   p.H = H; p.Hk = Hk; p.dv = dv; p.S = S; p.cu = cu;
   float* ob = nullptr;
-#define KB2_DT(NIV) (dv % 128 == 0 ? launch_delta_tiles<NIV, 4>(z, p, state, slots, scratch, &ob, st) : launch_delta_tiles<NIV, 1>(z, p, state, slots, scratch, &ob, st))
-  const int rc = dk == 32 ? KB2_DT(1) : dk == 64 ? KB2_DT(2) : KB2_DT(4);      // values in passes of 128 columns, or of 32
+  // values in passes of 128 columns, 64 or 32 (32 portions of 64 tokens, 8 heads of 64: 32 columns a pass made the step slower than its eight-token form)
+#define KB2_DT1(NIV, VBV) launch_delta_tiles<NIV, VBV>(z, p, state, slots, scratch, &ob, st)
+#define KB2_DT(NIV) (dv % 128 == 0 ? KB2_DT1(NIV, 4) : dv % 64 == 0 ? KB2_DT1(NIV, 2) : KB2_DT1(NIV, 1))
+  const int rc = dk == 32 ? KB2_DT(1) : dk == 64 ? KB2_DT(2) : KB2_DT(4);
 #undef KB2_DT
+#undef KB2_DT1
   if (rc != KB2SEQ_OK) return rc;
   return delta_out_launch(ob, proj + g_off, ldp, 0, H, dv, norm_w, eps, T, out, dt_out, st);
 }
