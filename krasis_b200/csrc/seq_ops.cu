@@ -124,7 +124,24 @@ __global__ void __launch_bounds__(256) gemv_nt_kernel(const TA* __restrict__ A, 
 #pragma unroll
   for (int m = 0; m < MR; ++m) acc[m] = 0.f;
   const TB* b = B + (long long)n * ldb;
-  for (int k = lane; k < K; k += 32) {
+  // eight loads of a row ahead of their sums, which stay in their order (left to the compiler they go out one by one: N 16384, K 2048 in fp32 at one row
+  // 64 us instead of 25)
+  int k = lane;
+  for (; k + 7 * 32 < K; k += 8 * 32) {
+    float w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[i] = ldf(b, k + 32 * i);
+#pragma unroll
+    for (int m = 0; m < MR; ++m) {
+      if (m >= M) break;
+      float a[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a[i] = ldf(A, (long long)m * lda + k + 32 * i);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[m] = fmaf(a[i], w[i], acc[m]);
+    }
+  }
+  for (; k < K; k += 32) {
     const float w = ldf(b, k);
 #pragma unroll
     for (int m = 0; m < MR; ++m)
