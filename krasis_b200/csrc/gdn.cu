@@ -44,7 +44,7 @@ __device__ __forceinline__ int qkvz_col(const GdnDims& d, int c) {
 }
 
 // one CTA per token
-__global__ void __launch_bounds__(256) gdn_prep_kernel(GdnDims d, const __nv_bfloat16* __restrict__ qkvz,
+__global__ void __launch_bounds__(256, 8) gdn_prep_kernel(GdnDims d, const __nv_bfloat16* __restrict__ qkvz,
                                                        const __nv_bfloat16* __restrict__ ba,
                                                        const __nv_bfloat16* __restrict__ conv_w,      // [C][K]
                                                        const __nv_bfloat16* __restrict__ conv_state,  // [C][K]

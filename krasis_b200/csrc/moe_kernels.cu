@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(kCombineThreads) combine_kernel(const __nv_bfl
                                                       float rsf, int apply_rsf,
                                                       const __nv_bfloat16* __restrict__ shared,
                                                       __nv_bfloat16* __restrict__ out, CombineScatter sc) {
-  pdl_enter(c3, slot_of, shared, out);
+  pdl_enter_global(c3, slot_of, shared, out);
   const int vec_per_row = H >> 3;
   const int m = blockIdx.x, v = blockIdx.y * kCombineThreads + threadIdx.x;
   if (v >= vec_per_row) return;

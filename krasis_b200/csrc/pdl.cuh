@@ -32,6 +32,15 @@ __device__ __forceinline__ void pdl_enter(P&... p) {
   const long long zero = pdl_wait();
   ((p = (P)((const char*)p + zero)), ...);
 }
+// The same for kernels that the compiler would otherwise address through generic pointers; in exchange it no longer knows that they are __restrict__.
+// Whichever is faster (us with plain pointers, with pdl_enter, with this: moe_gemv 26.6 / 30.3 / 26.5, attn_finish 40.6 / 47.2 / 39.6, gla_reg 102 / 104 /
+// 100, delta_out_rows 23.4 / 24.1 / 21.7; but rmsnorm_warp 10.5 / 10.4 / 15.3, scatter 19.4 / 19.3 / 23.3).  Either takes registers for pointers that plain
+// ones read from the constant bank: gqa_prep went from 32 to 48 of them, five blocks on an SM instead of eight, 27.5 -> 34 us until its launch bounds said so.
+template <typename... P>
+__device__ __forceinline__ void pdl_enter_global(P&... p) {
+  const size_t zero = (size_t)pdl_wait();
+  ((p = (P)__cvta_global_to_generic(__cvta_generic_to_global((const void*)p) + zero)), ...);
+}
 
 template <typename... P, typename... A>
 inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {

@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(256) head_kv_prep_kernel(float* __restrict__ p
                                                            int page_size, void* __restrict__ kc, void* __restrict__ vc, int dt_cache,
                                                            int norm_whole, int rot_half, const double* __restrict__ vfreq, float amp,
                                                            int v_is_k) {
-  kb2::pdl_enter(proj, bias, qw, kw, freq, positions, seq_of, pages, kc, vc, vfreq);
+  kb2::pdl_enter_global(proj, bias, qw, kw, freq, positions, seq_of, pages, kc, vc, vfreq);
   extern __shared__ float rot_tab[];          // [rot_dims / 2][2]: cos, sin of the token's position, shared by all its vectors
   __shared__ float red[32];
   const long long t = blockIdx.x;
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kPAThreads) paged_attn_kernel(
     float* __restrict__ part_acc, float* __restrict__ part_ml, const int* __restrict__ cu, int skip_from, float softcap,
     const float* __restrict__ sinks, int pool, int rows_per_page, const void* __restrict__ kp, const void* __restrict__ vp, int pool_only,
     const float* __restrict__ slopes) {
-  kb2::pdl_enter(proj, kc, vc, positions, seq_of, pages, out, part_acc, part_ml, cu, sinks, kp, vp, slopes);
+  kb2::pdl_enter_global(proj, kc, vc, positions, seq_of, pages, out, part_acc, part_ml, cu, sinks, kp, vp, slopes);
   extern __shared__ __align__(16) float sm[];
   constexpr int KT = kPAKT;
   const long long t = blockIdx.x;
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(256) attn_finish_kernel(const float* __restric
                                                           int dt_out, const int* __restrict__ seq_of, const int* __restrict__ cu,
                                                           int skip_from, int gate_wide, const int* __restrict__ positions,
                                                           const double* __restrict__ vfreq, int rot_half) {
-  kb2::pdl_enter(a, part_acc, part_ml, coef, gate, out, seq_of, cu, positions, vfreq);
+  kb2::pdl_enter_global(a, part_acc, part_ml, coef, gate, out, seq_of, cu, positions, vfreq);
   __shared__ float turn_buf[8][32 * NA];
   const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -861,7 +861,7 @@ template <typename TA, typename TB, typename TC>
 __global__ void __launch_bounds__(256) moe_gemv_kernel(const TA* __restrict__ A, long long lda, int div, const int* __restrict__ ids, int E,
                                                        const TB* __restrict__ B, long long ldb, long long sB, TC* __restrict__ C,
                                                        long long ldc, int N, int K) {
-  kb2::pdl_enter(A, ids, B, C);
+  kb2::pdl_enter_global(A, ids, B, C);
   const int slot = blockIdx.y;
   const int e = ids[slot];
   if (e < 0 || e >= E) return;

@@ -2178,7 +2178,7 @@ __global__ void __launch_bounds__(DeltaTile<NI>::kThreads, 1)
 // heads: 52 -> 44 us; a row per warp leaves too few bytes under way).
 __global__ void __launch_bounds__(256) delta_out_rows_kernel(const float* __restrict__ o, const float* __restrict__ gproj, long long ldg, int gate_act, int H,
                                                              const float* __restrict__ norm_w, float eps, long long rows, void* __restrict__ out, int dt_out) {
-  kb2::pdl_enter(o, gproj, norm_w, out);
+  kb2::pdl_enter_global(o, gproj, norm_w, out);
   const long long w = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * 4;
   const int j = (threadIdx.x & 31) * 4;
   float4 f[4], g[4];

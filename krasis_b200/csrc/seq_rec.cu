@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(32 * kGlaWarps) gla_reg_kernel(const float* __
                                                                  const float* __restrict__ alpha, float q_scale, int H, int dv,
                                                                  float* __restrict__ state, const int* __restrict__ cu,
                                                                  const int* __restrict__ slots, float* __restrict__ out) {
-  kb2::pdl_enter(qkv, alpha, state, cu, slots, out);
+  kb2::pdl_enter_global(qkv, alpha, state, cu, slots, out);
   constexpr int P = kGlaWarps, NT = 32 * P, Q = DK / P;
   extern __shared__ __align__(16) float sm[];
   float* as = sm;                                   // [2][kGlaTile][DK]
@@ -784,7 +784,7 @@ __global__ void __launch_bounds__(256) head_norm_gate_vec_kernel(const float* __
                                                                  const float* __restrict__ gate, long long ldg, int gate_act, int H, int dv,
                                                                  long long T, void* __restrict__ out, int dt_out, const float* __restrict__ den,
                                                                  int w_heads) {
-  kb2::pdl_enter(o, w, gate, out, den);
+  kb2::pdl_enter_global(o, w, gate, out, den);
   const long long wi = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (wi >= T * H) return;
@@ -877,7 +877,7 @@ __global__ void __launch_bounds__(256) branch_merge_kernel(const float* __restri
 __global__ void __launch_bounds__(256) depth_mix_kernel(float* __restrict__ stack, long long stride, int n, const float* __restrict__ coef,
                                                         float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ w,
                                                         void* __restrict__ h, int dt_h, int W, float eps) {
-  kb2::pdl_enter(stack, coef, x, y, w, h);
+  kb2::pdl_enter_global(stack, coef, x, y, w, h);
   __shared__ float red[32];
   const long long t = blockIdx.x;
   float* xr = x + t * W;

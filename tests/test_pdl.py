@@ -40,7 +40,7 @@ def _launched():
     """{kernel: where} of every programmatic launch, those through a variable among them."""
     found = {}
     for name, text in _sources():
-        for m in re.finditer(r"(?:launch_pdl|cudaLaunchKernelEx)(\()", text):
+        for m in re.finditer(r"(?:launch_pdl|launch_pdl_clusters|cudaLaunchKernelEx)(\()", text):
             ahead = text[:m.start()]
             what = _first_argument(text, m.start(1))
             if what in ("void (*kernel)(P...)",) or name == "pdl.cuh":       # the helper itself
@@ -89,15 +89,15 @@ def test_launched_kernels_wait():
         assert k in launched, k
     for name in sorted(launched):
         params, body = bodies[name]
-        assert len(re.findall(r"pdl_(?:enter|wait)\(", body)) == 1, name
-        assert not _reads_ahead(params, body[:re.search(r"pdl_(?:enter|wait)\(", body).start()]), name
+        assert len(re.findall(r"pdl_(?:enter|enter_global|wait)\(", body)) == 1, name
+        assert not _reads_ahead(params, body[:re.search(r"pdl_(?:enter|enter_global|wait)\(", body).start()]), name
 
 
 @pytest.mark.parametrize("name", ["split_weight_parts_kernel", "portion_rows_kernel", "split_gemm_kernel", "conv_run_vec_kernel"])
 def test_a_kernel_without_its_wait_is_found(name):
     """The check above on kernels whose wait comes after their first access."""
     params, body = _bodies()[name]
-    moved = re.sub(r"(?:kb2::)?pdl_(?:enter|wait)\([^;]*;", "", body) + "pdl_wait("
+    moved = re.sub(r"(?:kb2::)?pdl_(?:enter|enter_global|wait)\([^;]*;", "", body) + "pdl_wait("
     assert _reads_ahead(params, moved[:moved.index("pdl_wait(")])
 
 
