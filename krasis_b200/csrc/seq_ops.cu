@@ -263,23 +263,55 @@ __device__ __forceinline__ void mma16816_new(float (&d)[4], uint32_t a0, uint32_
 }
 
 // fp32 rows are three bf16 parts, exactly (the leading 8 bits, of what is left the next 8, the rest): the products with the first part go into one
-// accumulator, those with the others into a second, and both join the running sum.  The parts are made by every warp for itself; so that they serve
-// more weights, its pieces are 32 rows of 64 numbers.  fp32 rows, us before (gemv_nt_vec) at 1 / 2 / 4 / 8 rows and now at any: N 32768, K 2048 27.6 /
-// 30.4 / 40.6 / 79.9, 28.5; N 16384, K 2048 17.4 / 20.2 / 29.9 / 48.7, 17.5; N 2048, K 2048 5.1 / 6.0 / 8.4 / 12.7, 4.4; N 512, K 1024 2.6 / 3.4 / 5.1 /
-// 9.3, 2.5; error 1.6e-7 before, 6e-8 to 8e-8 now.  A sum that is not finite is made again in plain fp32 (the parts of an infinity are not numbers).
+// accumulator, those with the others into a second, and both join the running sum.  The later parts are taken 2^16 times as large: bf16 ends at 2^-133,
+// and parts of the smallest numbers lie below; above 2^119 they overflow, and the sum is made again like others that are not finite.  The parts are made
+// by every warp for itself, numbers in pairs; so that they serve more weights, its pieces are 32 rows of 64 numbers.  fp32 rows, us before
+// (gemv_nt_vec) at 1 / 2 / 4 / 8 rows and now at one and eight: N 65536, K 2048 47.4 / 52.3 / 76.8 / 149, 56.8 / 58; N 32768 27.4 / 30.2 / 40.4 / 79.9,
+// 29.4 / 29.6; N 16384 17.7 / 19.5 / 29.6 / 48.6, 17.0 / 17.2; N 2048 5.2 / 6.0 / 8.3 / 12.7, 4.6 / 5.3; N 512, K 512 2.6 /
+// 2.8 / 3.5 / 5.8, 1.9; error 1.6e-7 before, 6e-8 to 8e-8 now.  A sum that is not finite is made again in plain fp32 (the parts of an infinity are not
+// numbers).
 template <bool kFp32, int kTiles> struct GemvPiece {
   static constexpr int kRows = 16 * kTiles;                                    // weight rows of a warp
   static constexpr int kSteps = kFp32 ? 2 : 4, kLen = 32 * kSteps;             // of K, 32 a step
+  // warps of a block: few of them share a group's sums, so that the SMs get the same number of warps (N 65536: 14 at most instead of 16)
+  static constexpr int warps(int ks) { return kFp32 ? (ks < 2 ? 2 : ks) : ks > 8 ? 16 : 8; }
   static constexpr int kLoads = 2 * kTiles + (kFp32 ? 2 : 1);                  // 16-byte copies of a lane and step, the weights' first
   static constexpr int kStages = kLoads > 4 ? 4 : kFp32 ? 6 : 8, kRing = kStages * kLoads * 512;  // bytes of a warp's ring
 };
 
-// {the bf16 that leads a, the one that leads b}; what is left of a and b
-__device__ __forceinline__ uint32_t lead_pair(float& a, float& b) {
-  const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
-  a -= __uint_as_float(ua & 0xffff0000u);
-  b -= __uint_as_float(ub & 0xffff0000u);
-  return __byte_perm(ua, ub, 0x7632);
+// Two fp32 numbers that go through the arithmetic together.
+struct Pair {
+  uint64_t v;
+  __device__ __forceinline__ static Pair of(uint32_t a, uint32_t b) {
+    Pair p;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p.v) : "r"(a), "r"(b));
+    return p;
+  }
+  __device__ __forceinline__ static Pair of(float a, float b) { return of(__float_as_uint(a), __float_as_uint(b)); }
+  __device__ __forceinline__ void get(uint32_t& a, uint32_t& b) const { asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(v)); }
+};
+__device__ __forceinline__ Pair add2(Pair a, Pair b) {
+  Pair p;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(p.v) : "l"(a.v), "l"(b.v));
+  return p;
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
+  Pair p;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p.v) : "l"(a.v), "l"(b.v));
+  return p;
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
+  Pair p;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return p;
+}
+
+// {the bf16 that leads the first, the one that leads the second}; what is left of them
+__device__ __forceinline__ uint32_t lead_pair(Pair& f) {
+  uint32_t a, b;
+  f.get(a, b);
+  f = fma2(Pair::of(a & 0xffff0000u, b & 0xffff0000u), Pair::of(-1.f, -1.f), f);
+  return __byte_perm(a, b, 0x7632);
 }
 
 // A product in plain fp32 by a warp; K a multiple of 8, both rows 16-byte aligned.
@@ -296,13 +328,13 @@ __device__ __noinline__ float row_product(const float* a, const bf16* b, int K, 
 }
 
 template <typename TA, typename TC, int KS, int kTiles>
-__global__ void __launch_bounds__(KS > 8 ? 512 : 256) gemv_mma_kernel(const TA* __restrict__ A, long long lda, const bf16* __restrict__ B, long long ldb,
-                                                                      TC* __restrict__ C, long long ldc, int M, int N, int K, long long sA, long long sB,
-                                                                      long long sC) {
+__global__ void __launch_bounds__(32 * GemvPiece<sizeof(TA) == 4, kTiles>::warps(KS))
+    gemv_mma_kernel(const TA* __restrict__ A, long long lda, const bf16* __restrict__ B, long long ldb, TC* __restrict__ C, long long ldc, int M, int N, int K,
+                    long long sA, long long sB, long long sC) {
   kb2::pdl_enter(A, B, C);
   constexpr bool kFp32 = sizeof(TA) == 4;
   using P = GemvPiece<kFp32, kTiles>;
-  constexpr int kRows = P::kRows, kWarps = KS > 8 ? 16 : 8, kGroups = kWarps / KS, kW = 2 * kTiles;
+  constexpr int kRows = P::kRows, kWarps = P::warps(KS), kGroups = kWarps / KS, kW = 2 * kTiles;
   extern __shared__ __align__(16) uint8_t gemv_ring[];
   __shared__ float red[kWarps][8][kRows + 1];            // [warp][row of A][weight row], odd pitch
   A += (long long)blockIdx.z * sA;
@@ -323,18 +355,22 @@ __global__ void __launch_bounds__(KS > 8 ? 512 : 256) gemv_mma_kernel(const TA* 
       const int k = ((i / P::kSteps) * KS + part) * P::kLen + i % P::kSteps * 32;
       const uint32_t to = kb2::smem_u32(ring + i % P::kStages * (P::kLoads * 512));
       const bool in = k + t8 < K;
+      const int at = in ? k : 0;                           // the step's address from one base (fp32) or from two: each the faster for its rows, by 4 %
 #pragma unroll
-      for (int r = 0; r < kW; ++r) cp_async16_stream(to + r * 512, in ? w[r] + k : w[r], in);
+      for (int r = 0; r < kW; ++r) cp_async16_stream(to + r * 512, kFp32 ? w[r] + at : in ? w[r] + k : w[r], in);
 #pragma unroll
-      for (int h = 0; h < P::kLoads - kW; ++h) cp_async16(to + (kW + h) * 512, in ? x + k + 4 * h : x, in && row);
+      for (int h = 0; h < P::kLoads - kW; ++h) cp_async16(to + (kW + h) * 512, kFp32 ? x + at + 4 * h : in ? x + k : x, in && row);
     }
     kb2::cp_async_commit();
   };
   float sum[kTiles][4] = {}, lost[kTiles][4] = {};
+  Pair total[kTiles][2], kept[kTiles][2];                // fp32 rows: sums, and what their last additions rounded off
+#pragma unroll
+  for (int t = 0; t < kTiles; ++t) total[t][0] = total[t][1] = kept[t][0] = kept[t][1] = Pair::of(0.f, 0.f);
   auto join = [&](int t, int i, float add) {             // compensated: what the addition rounds off goes into the next one
     const float s = sum[t][i] + add;
-    // an infinity stays one: inf - inf must not reach the next addition (a sum of parts is made again in any case)
-    lost[t][i] = kFp32 || isfinite(s) ? (s - sum[t][i]) - add : 0.f;
+    // an infinity stays one: inf - inf must not reach the next addition
+    lost[t][i] = isfinite(s) ? (s - sum[t][i]) - add : 0.f;
     sum[t][i] = s;
   };
 #pragma unroll
@@ -348,13 +384,16 @@ __global__ void __launch_bounds__(KS > 8 ? 512 : 256) gemv_mma_kernel(const TA* 
     for (int r = 0; r < P::kLoads; ++r) v[r] = at[r * 32];
     if constexpr (kFp32) {
       const uint4 x0 = v[kW], x1 = v[kW + 1];
-      float f[8] = {__uint_as_float(x0.x), __uint_as_float(x0.y), __uint_as_float(x0.z), __uint_as_float(x0.w),
-                    __uint_as_float(x1.x), __uint_as_float(x1.y), __uint_as_float(x1.z), __uint_as_float(x1.w)};
+      Pair f[4] = {Pair::of(x0.x, x0.y), Pair::of(x0.z, x0.w), Pair::of(x1.x, x1.y), Pair::of(x1.z, x1.w)};
       uint32_t part[3][4];
 #pragma unroll
-      for (int q = 0; q < 3; ++q)
+      for (int q = 0; q < 3; ++q) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) part[q][i] = lead_pair(f[2 * i], f[2 * i + 1]);
+        for (int i = 0; i < 4; ++i) {
+          part[q][i] = lead_pair(f[i]);
+          if (q == 0) f[i] = mul2(f[i], Pair::of(65536.f, 65536.f));
+        }
+      }
 #pragma unroll
       for (int t = 0; t < kTiles; ++t) {
         const uint4 a = v[2 * t], c = v[2 * t + 1];
@@ -366,7 +405,12 @@ __global__ void __launch_bounds__(KS > 8 ? 512 : 256) gemv_mma_kernel(const TA* 
         mma16816_new(d, a.x, c.x, a.y, c.y, part[0][0], part[0][1]);
         mma16816(d, a.z, c.z, a.w, c.w, part[0][2], part[0][3]);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) join(t, i, d[i] + (e[i] - lost[t][i]));
+        for (int i = 0; i < 2; ++i) {
+          const Pair add = add2(Pair::of(d[2 * i], d[2 * i + 1]), fma2(Pair::of(e[2 * i], e[2 * i + 1]), Pair::of(1.f / 65536.f, 1.f / 65536.f), kept[t][i]));
+          const Pair s = add2(total[t][i], add);
+          kept[t][i] = add2(fma2(s, Pair::of(-1.f, -1.f), total[t][i]), add);
+          total[t][i] = s;
+        }
       }
     } else {
       const uint4 a = v[0], c = v[1];
@@ -378,6 +422,16 @@ __global__ void __launch_bounds__(KS > 8 ? 512 : 256) gemv_mma_kernel(const TA* 
     }
     fetch(i + P::kStages - 1);
   }
+  if constexpr (kFp32)
+#pragma unroll
+    for (int t = 0; t < kTiles; ++t)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        uint32_t a, b;
+        total[t][i].get(a, b);
+        sum[t][2 * i] = __uint_as_float(a);
+        sum[t][2 * i + 1] = __uint_as_float(b);
+      }
   // of a tile sum[0], [1]: weight row quad, rows 2 (lane & 3) and + 1 of A; [2], [3]: weight row quad + 8
   const int m = (lane & 3) * 2;
 #pragma unroll
@@ -413,13 +467,13 @@ static void launch_gemv_tiles(const void* A, long long lda, const void* B, long 
   const int groups = (N + Piece::kRows - 1) / Piece::kRows;
   int ks = 1;                                  // about 2048 warps, in one wave of two blocks per SM, as long as each has a piece of K
   while (ks < 16 && (long long)groups * batch * 2 * ks <= 2368 && K > Piece::kLen * ks) ks *= 2;
-  const int per = (ks > 8 ? 16 : 8) / ks;
+  const int warps = Piece::warps(ks), per = warps / ks;
   const dim3 grid((groups + per - 1) / per, 1, batch);
-  const size_t smem = (size_t)(ks > 8 ? 16 : 8) * Piece::kRing;
+  const size_t smem = (size_t)warps * Piece::kRing;
 #define KB2_GEMV(KSV)                                                                                                                            \
   case KSV:                                                                                                                                      \
-    kb2::allow_smem<gemv_mma_kernel<TA, TC, KSV, kTiles>>((KSV > 8 ? 16 : 8) * Piece::kRing);                                                        \
-    kb2::launch_pdl(gemv_mma_kernel<TA, TC, KSV, kTiles>, grid, KSV > 8 ? 512 : 256, smem, s, (const TA*)A, lda, (const bf16*)B, ldb, (TC*)C, ldc, M, N, K, \
+    kb2::allow_smem<gemv_mma_kernel<TA, TC, KSV, kTiles>>(Piece::warps(KSV) * Piece::kRing);                                                     \
+    kb2::launch_pdl(gemv_mma_kernel<TA, TC, KSV, kTiles>, grid, 32 * warps, smem, s, (const TA*)A, lda, (const bf16*)B, ldb, (TC*)C, ldc, M, N, K, \
                     sA, sB, sC);                                                                                                                 \
     break;
   switch (ks) { KB2_GEMV(1) KB2_GEMV(2) KB2_GEMV(4) KB2_GEMV(8) KB2_GEMV(16) }

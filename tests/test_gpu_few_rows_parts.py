@@ -53,3 +53,19 @@ def test_a_row_that_is_not_finite_costs_no_more_than_a_few_products():
     got = ops.gemm(x, w, torch.float32)
     assert torch.isnan(got[2]).all() and torch.isfinite(got[[0, 1, 3]]).all()
     assert best(x) < 8 * plain          # a warp: the weights once more, in turn; a thread reads 2 bytes of them at a time, hundreds of times in turn
+
+
+# the second and third part of numbers below 1e-33 lie below the smallest bf16 number; the largest numbers have parts that overflow where those are kept
+@pytest.mark.parametrize("N,K", [(40, 256), (4800, 64)])
+def test_smallest_and_largest_numbers(N, K):
+    g = torch.Generator(device="cuda").manual_seed(N)
+    w = torch.randn(N, K, device="cuda", generator=g).bfloat16()
+    scale = torch.tensor([1e-30, 1e-34, 1e-36, 1e-37, 3e-38, 1e-39, 1e35, 1e-45], device="cuda", dtype=torch.float64)
+    x = (torch.randn(8, K, device="cuda", generator=g).double() * scale[:, None]).float()
+    x[6] = x[6].clamp(-3.4e38 / K, 3.4e38 / K)
+    x[6, 3] = 3.4e38                                    # of which the parts overflow, against a weight that leaves the sum finite
+    w[:, 3] = 0.25
+    got, want = ops.gemm(x, w, torch.float32), x.double() @ w.double().T
+    size = x.double().abs() @ w.double().abs().T
+    # as for other numbers, and K sums and products that end at the smallest fp32 number, 2^-149, each rounded to a multiple of it
+    assert ((got.double() - want).abs() <= size * 2.0 ** -20 + K * 2.0 ** -149).all()
