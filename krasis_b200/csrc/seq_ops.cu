@@ -327,7 +327,8 @@ __device__ __noinline__ float row_product(const float* a, const bf16* b, int K, 
   return warp_sum(v);
 }
 
-template <typename TA, typename TC, int KS, int kTiles>
+// kShare: the blocks of a cluster along y share the pieces
+template <typename TA, typename TC, int KS, int kTiles, bool kShare>
 __global__ void __launch_bounds__(32 * GemvPiece<sizeof(TA) == 4, kTiles>::warps(KS))
     gemv_mma_kernel(const TA* __restrict__ A, long long lda, const bf16* __restrict__ B, long long ldb, TC* __restrict__ C, long long ldc, int M, int N, int K,
                     long long sA, long long sB, long long sC) {
@@ -349,10 +350,11 @@ __global__ void __launch_bounds__(32 * GemvPiece<sizeof(TA) == 4, kTiles>::warps
   const TA* x = A + (long long)min(quad, M - 1) * lda + t8;
   const bool row = quad < M;
   uint8_t* ring = gemv_ring + warp * P::kRing + lane * 16;     // a lane reads what it copied itself: no barrier
-  const int part = warp % KS, pieces = (K + P::kLen - 1) / P::kLen, steps = n0 < N ? (pieces - part + KS - 1) / KS * P::kSteps : 0;
+  const int parts = kShare ? KS * gridDim.y : KS, part = kShare ? warp % KS + KS * blockIdx.y : warp % KS;
+  const int pieces = (K + P::kLen - 1) / P::kLen, steps = n0 < N ? (pieces - part + parts - 1) / parts * P::kSteps : 0;
   auto fetch = [&](int i) {
     if (i < steps) {
-      const int k = ((i / P::kSteps) * KS + part) * P::kLen + i % P::kSteps * 32;
+      const int k = ((i / P::kSteps) * parts + part) * P::kLen + i % P::kSteps * 32;
       const uint32_t to = kb2::smem_u32(ring + i % P::kStages * (P::kLoads * 512));
       const bool in = k + t8 < K;
       const int at = in ? k : 0;                           // the step's address from one base (fp32) or from two: each the faster for its rows, by 4 %
@@ -439,9 +441,9 @@ __global__ void __launch_bounds__(32 * GemvPiece<sizeof(TA) == 4, kTiles>::warps
 #pragma unroll
     for (int i = 0; i < 4; ++i) red[warp][m + (i & 1)][16 * t + quad + (i >> 1) * 8] = sum[t][i];
   __syncthreads();
-  for (int i = threadIdx.x; i < kGroups * 8 * kRows; i += kWarps * 32) {
-    const int g = i / (8 * kRows), mm = i / kRows % 8, r = i % kRows, n = (blockIdx.x * kGroups + g) * kRows + r;
-    const bool in = mm < M && n < N;
+  constexpr int kOut = kGroups * 8 * kRows;
+  auto total_of = [&](int i) {
+    const int g = i / (8 * kRows), mm = i / kRows % 8, r = i % kRows;
     float v[KS];
 #pragma unroll
     for (int p = 0; p < KS; ++p) v[p] = red[g * KS + p][mm][r];
@@ -449,14 +451,38 @@ __global__ void __launch_bounds__(32 * GemvPiece<sizeof(TA) == 4, kTiles>::warps
     for (int o = KS / 2; o > 0; o >>= 1)
 #pragma unroll
       for (int p = 0; p < o; ++p) v[p] += v[p + o];
+    return v[0];
+  };
+  auto finish = [&](int i, float v) {
+    const int g = i / (8 * kRows), mm = i / kRows % 8, r = i % kRows, n = (blockIdx.x * kGroups + g) * kRows + r;
+    const bool in = mm < M && n < N;
     if constexpr (kFp32) {
-      for (unsigned again = __ballot_sync(0xffffffffu, in && !isfinite(v[0])); again; again &= again - 1) {      // the whole warp for one output after the other
+      for (unsigned again = __ballot_sync(0xffffffffu, in && !isfinite(v)); again; again &= again - 1) {      // the whole warp for one output after the other
         const int src = __ffs(again) - 1;
         const float t = row_product(A + (long long)__shfl_sync(0xffffffffu, mm, src) * lda, B + (long long)__shfl_sync(0xffffffffu, n, src) * ldb, K, lane);
-        if (lane == src) v[0] = t;
+        if (lane == src) v = t;
       }
     }
-    if (in) stf(C, (long long)mm * ldc + n, v[0]);
+    if (in) stf(C, (long long)mm * ldc + n, v);
+  };
+  if constexpr (kShare) {
+    static_assert(kOut <= kWarps * 32, "an output per thread");
+    __shared__ float whole[kOut];
+    const int i = threadIdx.x;
+    if (i < kOut) whole[i] = total_of(i);
+    kb2::cluster_sync_all();
+    if (blockIdx.y == 0 && i < kOut) {                     // whole warps
+      float v = whole[i];
+      for (unsigned b = 1; b < gridDim.y; ++b) {
+        float of;
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(of) : "r"(kb2::cluster_addr(whole + i, b)) : "memory");
+        v += of;
+      }
+      finish(i, v);
+    }
+    kb2::cluster_sync_all();                               // nobody leaves while its sums are read
+  } else {
+    for (int i = threadIdx.x; i < kOut; i += kWarps * 32) finish(i, total_of(i));
   }
 }
 
@@ -468,15 +494,26 @@ static void launch_gemv_tiles(const void* A, long long lda, const void* B, long 
   int ks = 1;                                  // about 2048 warps, in one wave of two blocks per SM, as long as each has a piece of K
   while (ks < 16 && (long long)groups * batch * 2 * ks <= 2368 && K > Piece::kLen * ks) ks *= 2;
   const int warps = Piece::warps(ks), per = warps / ks;
-  const dim3 grid((groups + per - 1) / per, 1, batch);
+  // few columns and a long K: up to four blocks along K where SMs stand idle, as long as a warp has more than four steps of fp32 rows to share out, eight
+  // of bf16 (us without and with them, four rows: fp32, K 8192, N 288 10.2 / 5.9, N 512 10.3 / 6.3, N 1024 10.5 / 8.4, N 300, K 16384 18.2 / 8.1; bf16
+  // 7.2 / 5.0, 7.2 / 5.4, 7.5 / 7.0, 12.7 / 6.4; below the line, fp32, N 1024, K 2048 3.8 / 4.5, bf16, N 512, K 4096 4.5 / 4.9)
+  unsigned blocks = 1;
+  if (ks == 16 && K > 32 * ks * (sizeof(TA) == 4 ? 4 : 8))
+    while (blocks < 4 && (long long)groups * batch * 2 * blocks <= kb2::current_sms() && K > 128 * ks * (int)blocks) blocks *= 2;
+  const dim3 grid((groups + per - 1) / per, blocks, batch);
   const size_t smem = (size_t)warps * Piece::kRing;
-#define KB2_GEMV(KSV)                                                                                                                            \
-  case KSV:                                                                                                                                      \
-    kb2::allow_smem<gemv_mma_kernel<TA, TC, KSV, kTiles>>(Piece::warps(KSV) * Piece::kRing);                                                     \
-    kb2::launch_pdl(gemv_mma_kernel<TA, TC, KSV, kTiles>, grid, 32 * warps, smem, s, (const TA*)A, lda, (const bf16*)B, ldb, (TC*)C, ldc, M, N, K, \
-                    sA, sB, sC);                                                                                                                 \
-    break;
-  switch (ks) { KB2_GEMV(1) KB2_GEMV(2) KB2_GEMV(4) KB2_GEMV(8) KB2_GEMV(16) }
+#define KB2_GEMV(KSV, SHARE)                                                                                                                     \
+  do {                                                                                                                                           \
+    kb2::allow_smem<gemv_mma_kernel<TA, TC, KSV, kTiles, SHARE>>(Piece::warps(KSV) * Piece::kRing);                                              \
+    kb2::launch_pdl_clusters(gemv_mma_kernel<TA, TC, KSV, kTiles, SHARE>, grid, 32 * warps, smem, s, blocks, (const TA*)A, lda, (const bf16*)B,  \
+                             ldb, (TC*)C, ldc, M, N, K, sA, sB, sC);                                                                             \
+  } while (0)
+  if (blocks > 1) KB2_GEMV(16, true);
+  else if (ks == 16) KB2_GEMV(16, false);
+  else if (ks == 8) KB2_GEMV(8, false);
+  else if (ks == 4) KB2_GEMV(4, false);
+  else if (ks == 2) KB2_GEMV(2, false);
+  else KB2_GEMV(1, false);
 #undef KB2_GEMV
 }
 

@@ -8,7 +8,8 @@ pytestmark = pytest.mark.gpu
 
 
 # columns around 16 and 32 rows of weights and around the counts that change the split along K; K that ends inside a step, a piece and a warp's turn
-@pytest.mark.parametrize("N,K", [(1, 8), (17, 40), (257, 2056), (1000, 64), (4720, 136), (4736, 2048), (9504, 328), (40000, 72)])
+@pytest.mark.parametrize("N,K", [(1, 8), (17, 40), (257, 2056), (1000, 64), (4720, 136), (4736, 2048), (9504, 328), (40000, 72),
+                                 (257, 4104), (1041, 8200), (300, 16392)])        # two and four blocks along K
 @pytest.mark.parametrize("out", [torch.float32, torch.bfloat16])
 def test_few_fp32_rows(N, K, out):
     g = torch.Generator(device="cuda").manual_seed(N + K)
@@ -22,9 +23,10 @@ def test_few_fp32_rows(N, K, out):
         assert torch.equal(ops.gemm(x[:m], w, out), got[:m])
 
 
-def test_not_finite():
+@pytest.mark.parametrize("N,K", [(4800, 512), (300, 16392)])
+def test_not_finite(N, K):
     g = torch.Generator(device="cuda").manual_seed(0)
-    w, x = torch.randn(4800, 512, device="cuda", generator=g).bfloat16(), torch.randn(4, 512, device="cuda", generator=g)
+    w, x = torch.randn(N, K, device="cuda", generator=g).bfloat16(), torch.randn(4, K, device="cuda", generator=g)
     x[0, 3], x[1, 500] = float("inf"), float("nan")
     w[7, 9] = float("-inf")
     got, want = ops.gemm(x, w, torch.float32), x.double() @ w.double().T
