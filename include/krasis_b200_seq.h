@@ -139,15 +139,16 @@ KB2SEQ_API int kb2_seq_head_kv_prep(float* proj, long long ldp, int T, int H, in
                                     const int* seq_of, const int* pages, int max_pages, int page_size, void* kc, void* vc, int dt_cache,
                                     int norm_whole, int rot_half, const double* vfreq, float amp, int v_is_k, void* stream);
 
+/* The bf16 operands of a portion's attention in one pass: cache rows `first` .. first + keys - 1 of a sequence (its page list `pages`, which holds
+ * them all) of two bf16 caches with rows of wa and wb numbers (multiples of 8), side by side in a [keys][wa] and b [keys][wb]; and rows of nq fp32
+ * numbers (a multiple of 8, ldq apart) rounded to bf16 in qb [n][nq].  Caches and outputs 16-byte aligned. */
+KB2SEQ_API int kb2_seq_portion_rows(const void* cache_a, int wa, const void* cache_b, int wb, const int* pages, int page_size, int first, int keys,
+                                    void* a, void* b, const float* q, long long ldq, int n, int nq, void* qb, void* stream);
+
 /* Pooled blocks: every `pool` consecutive positions of a sequence, b pool .. b pool + pool - 1, are summarised by the mean of their
  * cached key rows (width kw) and the mean of their cached value rows (width vw), taken in fp32 from the cache as it holds them.  The
  * pooled pools kp / vp have ceil(page_size / pool) rows per page and share the page numbering of kc / vc; block b lies in the page of
  * its last position.  Call after kb2_seq_head_kv_prep of the same step: the tokens of the step that complete a block write its summary. */
-/* The bf16 operands of a portion's attention in one pass: cache rows `first` .. first + keys - 1 of a sequence (its page list `pages`) of two
- * bf16 caches with rows of wa and wb numbers (multiples of 8), side by side in a [keys][wa] and b [keys][wb]; and rows of nq fp32 numbers (a
- * multiple of 8, ldq apart) rounded to bf16 in qb [n][nq].  Caches and outputs 16-byte aligned. */
-KB2SEQ_API int kb2_seq_portion_rows(const void* cache_a, int wa, const void* cache_b, int wb, const int* pages, int page_size, int first, int keys,
-                                    void* a, void* b, const float* q, long long ldq, int n, int nq, void* qb, void* stream);
 KB2SEQ_API int kb2_seq_kv_pool(const void* kc, const void* vc, void* kp, void* vp, int dt_cache, int kw, int vw, int pool, int T,
                                const int* positions, const int* seq_of, const int* pages, int max_pages, int page_size, void* stream);
 

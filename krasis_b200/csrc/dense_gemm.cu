@@ -346,7 +346,8 @@ static cudaError_t dense_configure() {
 // to timings of calls that follow one another in a stream at 323 shapes (M 256..8192, N 512..16384, K 512..8192), together with the line to split_gemm.cu;
 // the weights' way from HBM bounds a pair's time from below.  Against the estimates before, which were of launches that wait for one another, these
 // shapes take 0.987 of the time (geometric mean): M 700, N 2048, K 512 7.8 -> 6.2 us, M 1700, N 1536, K 2048 15.3 -> 13.2, M 1000, N 10240, K 8192 158 ->
-// 134, M 300, N 12288, K 2048 31.7 -> 28.5; the worst M 2600, N 2048, K 512 11.5 -> 13.0, M 1300, N 6144, K 5120 64.7 -> 70.5.
+// 134, M 300, N 12288, K 2048 31.7 -> 28.5; the worst M 2600, N 2048, K 512 11.5 -> 13.0, M 1300, N 6144, K 5120 64.7 -> 70.5.  On both
+// sides of the line, pairs / one CTA: M 2048, N 4096, K 2048 29.0 / 31.4, M 2300, N 2048, K 2048 18.2 / 17.1.
 static int dense_pair_plan(int M, int N, int K, int num_sms, float* us) {
   const int nkb = K / kBlockK, pairs = num_sms / 2;
   const auto rounds = [](long long tiles, int at_once) { return (float)((tiles + at_once - 1) / at_once); };

@@ -858,7 +858,7 @@ cudaError_t launch_gdn_prepare_tc(const void* qn, const void* kn, const void* vc
                                   void* kcd_img, void* intra_img, float* vcorr, float* gcum, int M, int n_chunks, int nk, int nv,
                                   int num_sms, cudaStream_t s);
 // Which chunk-prepare feeds the tcgen05 scan (dk == dv == 128).  QCN layer, 8192 tokens: the mma.sync prepare takes 332 us,
-// the tcgen05 prepare (gdn_tc.cu) 148 us after this round's work (460 us in its first version: profiles/r02c ... r02u).  The
+// the tcgen05 prepare (gdn_tc.cu) 148 us.  The
 // mma.sync kernel stays for other head sizes and as the A/B reference of tests/test_gpu_scale_parity.py:
 // KB2_GDN_PREPARE_MMA_SYNC=1 picks it, =0 the tcgen05 kernel; unset -> kDefaultPrepareTc.
 constexpr bool kDefaultPrepareTc = true;

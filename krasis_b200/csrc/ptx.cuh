@@ -37,18 +37,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Has the phase completed?  Never waits.
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
 // Bounded wait: a barrier that does not complete within ~2 s of SM clocks raises a sticky flag of its translation unit and returns, so that a
 // mis-counted pipeline runs to its end (with wrong data) and releases its tensor memory instead of spinning for ever.  While the flag is up later
 // waits give up early too: the host reads and clears the flags of a library through wait_flags() where it synchronises anyway.

@@ -161,80 +161,59 @@ template <> __device__ __forceinline__ void load8<float>(const float* p, float* 
 }
 template <> __device__ __forceinline__ void load8<bf16>(const bf16* p, float* f) { unpack8(*reinterpret_cast<const uint4*>(p), f); }
 
-// A warp owns CPW neighbouring output columns: the rows of A it loads (L1 hits after the first warp) serve CPW weight rows, and CPW
-// 16-byte weight loads per lane are in flight at once.
-template <typename TA, typename TC, int MR, int CPW, int KS>
-__global__ void __launch_bounds__(256) gemv_nt_vec_kernel(const TA* __restrict__ A, long long lda, const bf16* __restrict__ B, long long ldb,
-                                                          TC* __restrict__ C, long long ldc, int M, int N, int K, long long sA,
-                                                          long long sB, long long sC) {
+// fp32 rows and few columns: KS warps of a block share a column.
+template <typename TC, int MR, int KS>
+__global__ void __launch_bounds__(256) gemv_nt_vec_kernel(const float* __restrict__ A, long long lda, const bf16* __restrict__ B, long long ldb,
+                                                          TC* __restrict__ C, long long ldc, int M, int N, int K, long long sA, long long sB,
+                                                          long long sC) {
   kb2::pdl_enter(A, B, C);
   A += (long long)blockIdx.z * sA;
   B += (long long)blockIdx.z * sB;
   C += (long long)blockIdx.z * sC;
-  const int lane = threadIdx.x & 31;
-  const int group = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) / KS, kpart = (threadIdx.x >> 5) % KS;
-  const int n0 = group * CPW;
-  float acc[MR][CPW];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kpart = warp % KS;
+  const int n = (blockIdx.x * (blockDim.x >> 5) + warp) / KS;
+  float acc[MR];
 #pragma unroll
-  for (int m = 0; m < MR; ++m)
-#pragma unroll
-    for (int c = 0; c < CPW; ++c) acc[m][c] = 0.f;
-  // KS warps share a column group and take interleaved 256-element pieces of K; the weights of the next piece are requested before
-  // the current ones are used
+  for (int m = 0; m < MR; ++m) acc[m] = 0.f;
+  // the warps take interleaved pieces of 256; the weights of the next piece are requested before the current ones are used
   const int kstep = 256 * KS;
-  uint4 wv[CPW], wn[CPW];
   int k = (kpart * 32 + lane) * 8;
-#pragma unroll
-  for (int c = 0; c < CPW; ++c) wv[c] = (k < K && n0 + c < N) ? ld_stream16(B + (long long)(n0 + c) * ldb + k) : make_uint4(0, 0, 0, 0);
+  const auto weights = [&](int k) { return k < K && n < N ? ld_stream16(B + (long long)n * ldb + k) : make_uint4(0, 0, 0, 0); };
+  uint4 wv = weights(k);
   for (; k < K; k += kstep) {
-    const int kn = k + kstep;
-#pragma unroll
-    for (int c = 0; c < CPW; ++c) wn[c] = (kn < K && n0 + c < N) ? ld_stream16(B + (long long)(n0 + c) * ldb + kn) : make_uint4(0, 0, 0, 0);
+    const uint4 wn = weights(k + kstep);
 #pragma unroll
     for (int m = 0; m < MR; ++m)
       if (m < M) {
-        float a[8];
-        load8<TA>(A + (long long)m * lda + k, a);
+        float a[8], w[8];
+        load8<float>(A + (long long)m * lda + k, a);
+        unpack8(wv, w);
 #pragma unroll
-        for (int c = 0; c < CPW; ++c) {
-          float w[8];
-          unpack8(wv[c], w);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) acc[m][c] = fmaf(a[i], w[i], acc[m][c]);
-        }
+        for (int i = 0; i < 8; ++i) acc[m] = fmaf(a[i], w[i], acc[m]);
       }
-#pragma unroll
-    for (int c = 0; c < CPW; ++c) wv[c] = wn[c];
+    wv = wn;
   }
-  __shared__ float red[8][MR * CPW];
-  const int warp = threadIdx.x >> 5;
+  __shared__ float red[8][MR];
 #pragma unroll
-  for (int m = 0; m < MR; ++m)
-#pragma unroll
-    for (int c = 0; c < CPW; ++c) {
-      const float v = warp_sum(acc[m][c]);
-      if (lane == 0) red[warp][m * CPW + c] = v;
-    }
+  for (int m = 0; m < MR; ++m) {
+    const float v = warp_sum(acc[m]);
+    if (lane == 0) red[warp][m] = v;
+  }
   __syncthreads();
-  if (kpart == 0 && lane < MR * CPW) {
-    const int m = lane / CPW, c = lane % CPW;
+  if (kpart == 0 && lane < MR) {
     float v = 0.f;
     for (int p = 0; p < KS; ++p) v += red[warp + p][lane];
-    if (m < M && n0 + c < N) stf(C, (long long)m * ldc + n0 + c, v);
+    if (lane < M && n < N) stf(C, (long long)lane * ldc + n, v);
   }
 }
 
-template <typename TA, typename TC>
-static bool launch_gemv_vec(const void* A, long long lda, const void* B, long long ldb, void* C, long long ldc, int M, int N, int K,
-                            int batch, long long sA, long long sB, long long sC, cudaStream_t s) {
-  const bool a16 = sizeof(TA) == 2;
-  if (K % 8 || ldb % 8 || sB % 8 || ((uintptr_t)B & 15) || ((uintptr_t)A & 15) || lda % (a16 ? 8 : 4) || sA % (a16 ? 8 : 4)) return false;
-  // one column a group of four warps: this form is left for few columns
-#define KB2_GEMV(MRV)                                                                                                                        \
-  kb2::launch_pdl(gemv_nt_vec_kernel<TA, TC, MRV, 1, 4>, dim3((N + 1) / 2, 1, batch), 256, 0, s, (const TA*)A, lda, (const bf16*)B, ldb, (TC*)C, ldc, M, \
-                  N, K, sA, sB, sC)
-  if (M <= 4) KB2_GEMV(4); else KB2_GEMV(8);
-#undef KB2_GEMV
+template <typename TC>
+static bool launch_gemv_vec(const float* A, long long lda, const bf16* B, long long ldb, TC* C, long long ldc, int M, int N, int K, int batch, long long sA,
+                            long long sB, long long sC, cudaStream_t s) {
+  if (K % 8 || ldb % 8 || sB % 8 || ((uintptr_t)B & 15) || ((uintptr_t)A & 15) || lda % 4 || sA % 4) return false;
+  const dim3 grid((N + 1) / 2, 1, batch);
+  auto kern = M <= 4 ? gemv_nt_vec_kernel<TC, 4, 4> : gemv_nt_vec_kernel<TC, 8, 4>;
+  kb2::launch_pdl(kern, grid, 256, 0, s, A, lda, B, ldb, C, ldc, M, N, K, sA, sB, sC);
   return true;
 }
 
@@ -543,7 +522,7 @@ static void launch_gemm(const void* A, long long lda, const void* B, long long l
       // fp32 rows, few columns and a long K: sixteen rows a block would leave the weights to a handful of SMs, and with one row the FMAs are few (us at
       // 1 / 2 / 4 / 8 rows, N 256, K 2048 2.2 / 2.6 / 3.5 / 5.5 here, 3.5 at any on the tensor cores; N 128, K 8184 5.6 / 7.2 / 10.9 / 18.7, 10.4)
       if constexpr (sizeof(TA) == 4) {
-        if ((long long)N * batch <= 256 && K >= 2048 && launch_gemv_vec<TA, TC>(A, lda, B, ldb, C, ldc, M, N, K, batch, sA, sB, sC, s)) return;
+        if ((long long)N * batch <= 256 && K >= 2048 && launch_gemv_vec((const float*)A, lda, (const bf16*)B, ldb, (TC*)C, ldc, M, N, K, batch, sA, sB, sC, s)) return;
       }
       if (launch_gemv_mma<TA, TC>(A, lda, B, ldb, C, ldc, M, N, K, batch, sA, sB, sC, s)) return;
     }
