@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kDThreads, 1)
   uint64_t* acc_empty = acc_full + 2;        // [2]
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(acc_empty + 2);
   // warp index through a shuffle so that the role branches are provably warp-uniform: tcgen05.mma issued from a divergent single-thread branch
-  // cost about 50 cycles more each (profiles/r02h_mma_uniform_ubench.txt)
+  // cost about 50 cycles more each
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 32) {

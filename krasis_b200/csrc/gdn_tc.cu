@@ -120,7 +120,7 @@ struct GdnTcParams {
 
 // --------------------------------------------------------------------------------------------------------------------
 // The scan kernel.  320 threads: warps 0-7 CUDA cores, warp 8 TMA producer, warp 9 MMA issuer (whole warp runs the role loop, one
-// elected lane issues: see ptx.cuh / ENGINEERING_NOTES.md on warp-uniform issue).  Core thread = (TMEM lane L, column half): warps w
+// elected lane issues: see ptx.cuh on warp-uniform issue).  Core thread = (TMEM lane L, column half): warps w
 // and w + 4 share lane quadrant w & 3 and take 16 of the slice's 32 columns each, so every scheduler has two core warps.
 //   TMEM columns   D1 [0,64)  = [q ; kcd_hi] [S_hi | S_lo]   (lanes 0-63 = IT parts, 64-127 = VP parts; the two 32-column halves are
 //                  D1b [64,96) = [* ; kcd_lo] S_hi             added by the cores: hi/lo halves of a B operand are STACKED ALONG N, one
@@ -130,7 +130,6 @@ struct GdnTcParams {
 //                  barrier -> every thread (column n = lane, token octet = warp) converts 8 tokens of one column pairwise
 //                  (cvt.rn.bf16x2: the packed word is the K-contiguous memory order) and writes v_hi / v_lo / vdec_hi / vdec_lo with
 //                  one 16-byte store each -> G2, G3 -> S = e^{g_last} S + dS in registers, new S_hi / S_lo tiles -> epilogue (local).
-// History of the layout with the measurements that drove each step: profiles/README.md (r02a ... r02l), ENGINEERING_NOTES.md.
 // --------------------------------------------------------------------------------------------------------------------
 constexpr int kT3Threads = 320;
 
@@ -497,7 +496,7 @@ struct GdnPrepParams {
 
 // --------------------------------------------------------------------------------------------------------------------
 // The kernel: EIGHT CUDA-core warps on one unit (thread = TMEM lane x column half, two warps per scheduler: the first version had
-// four and every phase ran at IPC ~0.2, profiles/r02f_*), and MMA-B/C stacked so that no partial sums have to be exchanged:  D_B = [T'_hi ; T''_hi] v + [T'_lo ; T''_lo] v  (lanes 0-63 = T' v = vcorr),  D_C = the same A operands against k
+// four and every phase ran at IPC ~0.2), and MMA-B/C stacked so that no partial sums have to be exchanged:  D_B = [T'_hi ; T''_hi] v + [T'_lo ; T''_lo] v  (lanes 0-63 = T' v = vcorr),  D_C = the same A operands against k
 // (lanes 64-127 = T'' k = kcd).  Twice the MMAs (16 of N = 128 per unit, still a few hundred cycles), no shared-memory round trip.
 // Warp 8 = TMA producer, warp 9 = MMA issuer.
 // --------------------------------------------------------------------------------------------------------------------
@@ -733,7 +732,7 @@ __global__ void __launch_bounds__(kT3Threads, 1)
       named_bar_sync(2, 256);
       if (tid == 0) stamp(it, 12);
       // levels 1 and 2 are small dense products: 16x8 output tiles on mma.sync m16n8k8 with 3xTF32 operands (fp32-grade; the CUDA-core
-      // dot products they replace took 770 + 2700 of the unit's 10.7 K cycles, profiles/r02t_gdn_prepare_inverse_phases.txt)
+      // dot products they replace took 770 + 2700 of the unit's 10.7 K cycles)
       const int fg = lane >> 2, ft = lane & 3;                              // accumulator fragment: rows fg, fg + 8; columns 2 ft, 2 ft + 1
       {                                       // level 1, stage 1: P_p = A[2p+1][2p] D_2p ; stage 2: T[2p+1][2p] = D_2p+1 P_p   (16x16x16)
         const int pp = warp >> 1, ct = warp & 1;                            // warps 0-3: pair pp, 8-column tile ct
@@ -900,7 +899,7 @@ cudaError_t launch_gdn_scan_tc(const void* qn, const void* kn, const void* kcd_i
     if (e != cudaSuccess) return e;
     once.mark(dev);
   }
-  // tuning only: KB2_GDN_SCAN_TRACE=<device pointer> receives clock64 stamps of CTA (0,0) (scripts/gdn_scan_tune.py)
+  // tuning only: KB2_GDN_SCAN_TRACE=<device pointer> receives clock64 stamps of CTA (0,0)
   const char* tv = getenv("KB2_GDN_SCAN_TRACE");
   long long* trace = tv ? reinterpret_cast<long long*>(strtoull(tv, nullptr, 0)) : nullptr;
   alignas(64) CUtensorMap tq, tk;

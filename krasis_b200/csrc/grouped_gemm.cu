@@ -16,7 +16,7 @@
 //   epilogue warps: tcgen05.ld -> SiLU(gate)*up | x routing weight -> BF16 -> smem staging -> 16 B coalesced stores
 // Keeping the dequantised A operand out of shared memory matters: a BF16 SS-MMA at M=128 reads
 // (128+N)*32 B of smem per N/2 cycles (~115 B/clk at N=160), which together with the dequant stores
-// exceeded the 128 B/clk smem port in the first version of this kernel (profiles/r01a_*).
+// exceeded the 128 B/clk smem port in the first version of this kernel.
 //   GEMM1: the pair is (gate tile t, up tile t) -> SiLU(gate)*up fused in the epilogue, BF16 act out
 //   GEMM2: the pair is two consecutive down-proj tiles -> x routing weight, BF16 c3 out
 // Warp roles (896 threads):
@@ -82,7 +82,7 @@ struct SmemLayout {
   static_assert(kATmemCol + kStagesA * 2 * kATileCols <= kTmemCols, "TMEM columns");
   static constexpr int kBStageBytes = NT * kBlockK * 2;
   // token (B operand) ring: 4 stages wherever they fit the 227 KB (everything but the 12 KB Affine8 tiles).  With tcgen05.mma issued
-  // at full rate the K loop waited ~200 cycles per k-block on token rows with 3 stages (profiles/r02i_gemm_item_timeline_*).
+  // at full rate the K loop waited ~200 cycles per k-block on token rows with 3 stages.
   // Q4_K gives one up for four K blocks of weights in place of two (three of them are not an even number, see below): a whole pass over 64 experts of
   // 1536 columns, 1000 x 6 rows 240 -> 227 us, 2000 301 -> 293, 8192 959 -> 973; 128 experts of 768, 2000 x 8 rows 258 -> 248, 8192 722 -> 720.
   static constexpr int kStagesB = kShort ? 6 : (FMT == kFmtAffine8 || FMT == kFmtQ4_K) ? 3 : 4;
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
 
   // warp index through a shuffle: the role branches below are then provably warp-uniform.  Issued from a divergent `lane == 0` branch every
   // tcgen05.mma took about 50 cycles of issue, which made the K loop issue-bound (135
-  // cycles per N=160 MMA in situ against 80 of execution: profiles/r02h_gemm_item_timeline.txt, r02h_mma_uniform_ubench.txt).
+  // cycles per N=160 MMA in situ against 80 of execution).
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
 
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
   const int n_chunks = *p.n_chunks;
   const int n_items = n_chunks * p.items_per_chunk;
   const int nkb = p.n_kblocks;
-  // tuning aid: per work item of CTA 0, slot = clock64 stamp or accumulated wait cycles (see scripts/gemm_trace.py)
+  // tuning aid: per work item of CTA 0, slot = clock64 stamp or accumulated wait cycles
   const bool tracing = TRACE && blockIdx.x == 0;
   auto stamp = [&](int it, int slot, long long v) {
     if (tracing && it < 16 && (lane == 0 || threadIdx.x == 256)) p.trace[it * 16 + slot] = v;
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
       const int n_pad = (cd.n_tok + 15) & ~15;
       if constexpr (!kGemm1) {
         // routing weights of this chunk -> shared memory while the MMAs run (a global load per accumulator column inside the
-        // drain loop made phase 1 of the down projection 3x longer than the gate/up one: profiles/r02h_gemm_item_timeline.txt)
+        // drain loop made phase 1 of the down projection 3x longer than the gate/up one)
         float* sw = reinterpret_cast<float*>(smem + L::kOffSlotW);
         for (int i = et; i < n_pad; i += kNumEpiThreads) sw[i] = (i < cd.n_tok) ? p.slot_weight[cd.slot_begin + i] : 0.f;
       }

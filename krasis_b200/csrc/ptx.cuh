@@ -201,8 +201,7 @@ __device__ __forceinline__ float exp_fast_nobranch(float x) {
 }
 
 // bf16 RNE of one float, result in the LOW 16 bits (high bits zero), by the packed conversion: with __float2bfloat16_rn on single values that are
-// reused as integers, conversions bounded the CUDA-core phases of the tcgen05 Gated-DeltaNet kernels (gdn_prep 155 -> 129 us, prepare 347 -> 325 us,
-// profiles/r02g_*).
+// reused as integers, conversions bounded the CUDA-core phases of the tcgen05 Gated-DeltaNet kernels (gdn_prep 155 -> 129 us, prepare 347 -> 325 us).
 __device__ __forceinline__ uint32_t bf16_bits_rn(float x) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(0.f), "f"(x));

@@ -546,7 +546,7 @@ class KrasisModel:
             self.layers.append(lay)
         self._ones = self._zero_ids = None
         self._side_stream = None
-        # chunk-pipelined attention collectives under token sharding: OFF by default.  Measured on 2 GPUs (profiles/r02p_*): 70.0 ms per
+        # chunk-pipelined attention collectives under token sharding: OFF by default.  Measured on 2 GPUs: 70.0 ms per
         # step against 65.1 ms with one all-gather + one reduce-scatter per layer — the NCCL kernels that now run next to the attention
         # hold SMs that the persistent one-CTA-per-SM GEMM / scan kernels are sized for (Gated DeltaNet 24.8 -> 32.0 ms), which costs
         # more than the 2 x 1 ms of hidden communication.  KB2_PIPELINE_ATTENTION=1 enables it.
@@ -555,7 +555,7 @@ class KrasisModel:
         self.fused_ep = os.environ.get("KB2_FUSED_EP", "1") != "0"
         self._ep_recv, self._ep_recv_rows = None, 0
         self._graphs = {}
-        # attention out_proj GEMM -> reduce-scatter fused the same way: OFF by default.  Measured on 2 GPUs (profiles/r02s_*): the
+        # attention out_proj GEMM -> reduce-scatter fused the same way: OFF by default.  Measured on 2 GPUs: the
         # reduce-scatter itself drops from 3.1 to 2.2 ms per step, but the GEMM epilogue holds its TMEM accumulator while half of its
         # rows cross NVLink (Gated DeltaNet 24.6 -> 28.0 ms, GQA 7.0 -> 8.2 ms): 67.0 ms per step against 63.7.  The combine kernel
         # of the experts is HBM-bound elementwise work and hides the remote stores; a tensor-core epilogue does not.
