@@ -176,11 +176,6 @@ class StepTables:
         self.h2d_bytes = n * 4
 
 
-def _plain_rows(cache: torch.Tensor) -> bool:
-    """Whether kb2_seq_portion_rows takes a cache as it lies."""
-    return cache.dtype == torch.bfloat16 and cache.is_contiguous() and cache.data_ptr() % 16 == 0
-
-
 def portion_rows(tb: StepTables, s: int, first: int, ca: torch.Tensor, wa: int, cb: torch.Tensor, wb: int, page_size: int, proj: torch.Tensor,
                  row0: int, n: int, nq: int):
     """The operands of sequence s's attention on the tensor cores, made in one launch: rows `first` up to the portion's end of two bfloat16
@@ -189,16 +184,15 @@ def portion_rows(tb: StepTables, s: int, first: int, ca: torch.Tensor, wa: int, 
     keys, dev = start + m - first, proj.device
     if (start + m - 1) // page_size >= len(pages):           # the kernel would read on in the table
         raise IndexError(f"sequence {s}: {len(pages)} pages of {page_size} rows do not hold {start + m} positions")
-    if not (_plain_rows(ca) and _plain_rows(cb)):
+    pa, pb, bf = ca.data_ptr(), cb.data_ptr(), torch.bfloat16
+    if (pa | pb) & 15 or ca.dtype is not bf or cb.dtype is not bf or not (ca.is_contiguous() and cb.is_contiguous()):      # what the kernel does not take
         import numpy as np
         j = np.arange(first, start + m, dtype=np.int64)
         rows = torch.from_numpy(np.asarray(pages, dtype=np.int64)[j // page_size] * page_size + j % page_size).to(dev, non_blocking=True)
         return (ca.view(-1, wa).index_select(0, rows), cb.view(-1, wb).index_select(0, rows),
                 proj[row0:row0 + n, :nq].to(torch.bfloat16).contiguous())
-    a = torch.empty((keys, wa), dtype=torch.bfloat16, device=dev)
-    b = torch.empty((keys, wb), dtype=torch.bfloat16, device=dev)
-    q = torch.empty((n, nq), dtype=torch.bfloat16, device=dev)
-    check(load().kb2_seq_portion_rows(ca.data_ptr(), wa, cb.data_ptr(), wb, tb.pages.data_ptr() + 4 * s * tb.max_pages, page_size, first, keys,
+    a, b, q = torch.empty((keys, wa), dtype=bf, device=dev), torch.empty((keys, wb), dtype=bf, device=dev), torch.empty((n, nq), dtype=bf, device=dev)
+    check(load().kb2_seq_portion_rows(pa, wa, pb, wb, tb.pages.data_ptr() + 4 * s * tb.max_pages, page_size, first, keys,
                                       a.data_ptr(), b.data_ptr(), proj.data_ptr() + row0 * proj.stride(0) * 4, proj.stride(0), n, nq, q.data_ptr(), _s(proj)))
     return a, b, q
 

@@ -8,7 +8,8 @@ _raw = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: to
 
 def stream_of(t: torch.Tensor) -> int:
     """Handle of the current stream of the CUDA tensor t's device."""
-    return stream_on(t.get_device()) if t.is_cuda else _refuse(t.device)
+    index = t.get_device()            # negative: not on a GPU
+    return _raw(index) if index >= 0 else _refuse(t.device)
 
 
 def stream_on(device) -> int:
