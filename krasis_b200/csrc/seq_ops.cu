@@ -502,8 +502,8 @@ static bool launch_gemv_mma(const void* A, long long lda, const void* B, long lo
   constexpr int kA16 = 16 / sizeof(TA);
   if (K % 8 || ldb % 8 || sB % 8 || ((uintptr_t)B & 15) || ((uintptr_t)A & 15) || lda % kA16 || sA % kA16) return false;
   // at any number of rows, so that a row's sums do not depend on the rows beside it; bf16 rows, gemv_nt_vec, us at 1 / 2 / 4 / 8 rows and here at any:
-  // N 512, K 1024 2.7 / 3.5 / 5.3 / 9.7, 2.1; N 4096, K 224 2.3 / 2.7 / 3.4 / 5.2, 2.2; N 256, K 2048 2.2 / 2.6 / 3.5 / 5.6, 2.7; N 128, K 8184
-  // 3.9 / 5.6 / 9.2 / 17, 6.2
+  // N 512, K 1024 2.7 / 3.5 / 5.3 / 9.7, 2.1; N 4096, K 224 2.3 / 2.7 / 3.4 / 5.2, 2.2; N 256, K 2048 2.2 / 2.6 / 3.5 / 5.6, 2.7; N 128, K 8192
+  // 3.9 / 5.6 / 9.2 / 17, 4.8
   if constexpr (sizeof(TA) == 4) {             // 32 weight rows a warp where that still gives every SM a block (N 2048, K 8192: 15.9 us, with 16 rows 11.2)
     if ((long long)((N + 31) / 32) * batch >= kb2::current_sms()) {
       launch_gemv_tiles<TA, TC, 2>(A, lda, B, ldb, C, ldc, M, N, K, batch, sA, sB, sC, s);
@@ -520,7 +520,8 @@ static void launch_gemm(const void* A, long long lda, const void* B, long long l
   if (M <= 8) {
     if constexpr (sizeof(TB) == 2) {
       // fp32 rows, few columns and a long K: sixteen rows a block would leave the weights to a handful of SMs, and with one row the FMAs are few (us at
-      // 1 / 2 / 4 / 8 rows, N 256, K 2048 2.2 / 2.6 / 3.5 / 5.5 here, 3.5 at any on the tensor cores; N 128, K 8184 5.6 / 7.2 / 10.9 / 18.7, 10.4)
+      // 1 / 2 / 4 / 8 rows, N 256, K 2048 2.2 / 2.6 / 3.5 / 5.5 here, 3.5 at any on the tensor cores; N 128, K 8192 5.5 / 6.6 / 9.9 / 17.6, 10.4 there with
+      // all of K in one block.  With K shared by four blocks N 288 takes 5.8 / 5.8 / 5.9 / 6.6 there: from two rows on this line lies too high for long K)
       if constexpr (sizeof(TA) == 4) {
         if ((long long)N * batch <= 256 && K >= 2048 && launch_gemv_vec((const float*)A, lda, (const bf16*)B, ldb, (TC*)C, ldc, M, N, K, batch, sA, sB, sC, s)) return;
       }
