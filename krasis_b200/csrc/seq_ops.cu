@@ -869,6 +869,15 @@ __global__ void act_mul_kernel(const void* __restrict__ in, int dt_in, void* __r
   const float a = ld_dt(in, dt_in, t * 2 * F + f), b = ld_dt(in, dt_in, t * 2 * F + F + f);
   st_dt(out, dt_out, t * F + f, gelu_tanh(a) * b);
 }
+// fp32 in and out, F a multiple of 4: 16-byte accesses (512 rows of 8192: 16.9 -> 7.9 us, 50 MB)
+__global__ void __launch_bounds__(256) act_mul_f32x4_kernel(const float* __restrict__ in, float* __restrict__ out, int F) {
+  kb2::pdl_enter(in, out);
+  const long long t = blockIdx.y;
+  const int f = (blockIdx.x * 256 + threadIdx.x) * 4;
+  if (f >= F) return;
+  const float4 a = *reinterpret_cast<const float4*>(in + t * 2 * F + f), b = *reinterpret_cast<const float4*>(in + t * 2 * F + F + f);
+  *reinterpret_cast<float4*>(out + t * F + f) = make_float4(gelu_tanh(a.x) * b.x, gelu_tanh(a.y) * b.y, gelu_tanh(a.z) * b.z, gelu_tanh(a.w) * b.w);
+}
 // bf16 in and out, F a multiple of 8: 16-byte accesses
 __global__ void act_mul_bf16x8_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, int F) {
   kb2::pdl_enter(in, out);
@@ -2387,6 +2396,8 @@ KB2SEQ_API int kb2_seq_act_mul(const void* in, int dt_in, void* out, int dt_out,
   if (T > 65535) return failf(KB2SEQ_ERR_VALUE, "act_mul: more than 65535 rows in one step");
   if (dt_in == 1 && dt_out == 1 && F % 8 == 0 && !((uintptr_t)in & 15) && !((uintptr_t)out & 15))
     kb2::launch_pdl(act_mul_bf16x8_kernel, dim3((F / 8 + 127) / 128, T), 128, 0, (cudaStream_t)stream, (const bf16*)in, (bf16*)out, F);
+  else if (dt_in == 0 && dt_out == 0 && F % 4 == 0 && !((uintptr_t)in & 15) && !((uintptr_t)out & 15))
+    kb2::launch_pdl(act_mul_f32x4_kernel, dim3((F / 4 + 255) / 256, T), 256, 0, (cudaStream_t)stream, (const float*)in, (float*)out, F);
   else
     kb2::launch_pdl(act_mul_kernel, dim3((F + 255) / 256, T), 256, 0, (cudaStream_t)stream, in, dt_in, out, dt_out, T, F);
   SEQ_LAUNCHED();

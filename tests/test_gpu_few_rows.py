@@ -111,3 +111,14 @@ def test_embed(W, dtype):
     assert torch.equal(ops.embed(table, tokens, 1.5), table[tokens.long()].float() * 1.5)
     off = torch.randn(50 * W + 1, device="cuda").to(dtype)[1:].view(50, W)          # rows off a 16-byte boundary
     assert torch.equal(ops.embed(off, tokens, 0.5), off[tokens.long()].float() * 0.5)
+
+
+@pytest.mark.parametrize("T,F,at", [(1, 4, 0), (3, 1028, 0), (5, 8192, 0), (3, 1028, 1), (2, 1027, 0)])
+def test_act_mul_of_fp32_rows(T, F, at):
+    """Widths in groups of four and not, rows that do not start on 16 bytes: the same numbers from either form."""
+    base = torch.randn(T * 2 * F + at, device="cuda", generator=torch.Generator(device="cuda").manual_seed(F))
+    gu = base[at:].view(T, 2 * F)
+    want = torch.nn.functional.gelu(gu[:, :F].double(), approximate="tanh") * gu[:, F:].double()
+    got = ops.act_mul(gu, torch.float32)
+    # tanhf and seven products and sums in fp32, of numbers that are 1 + tanh at most twice as large as the result
+    assert ((got.double() - want).abs() <= 16 * 2.0 ** -23 * (gu[:, :F].double().abs() * gu[:, F:].double().abs()) + 1e-12).all()
