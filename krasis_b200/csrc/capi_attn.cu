@@ -257,7 +257,7 @@ KB2_API size_t kb2_linear_f32_workspace(int32_t M, int32_t N, int32_t K, int32_t
   if (M <= 0 || N <= 0 || K <= 0 || groups <= 0) return 0;
   const int32_t cols = linear_f32_columns(N, K, w_f32, groups);
   if (N % 16 || !linear_f32_plan(M, cols, K, w_f32, groups, device, &plan)) return 0;
-  return x_parts_bytes(plan, M, K, groups) + (w_f32 ? (size_t)groups * (cols * (size_t)K * 6 + (cols + 127) / 128 * 32) : 0);
+  return x_parts_bytes(plan, M, K, groups) + (plan.pair ? parts_partial_bytes(M, cols, groups, plan.ks) : 0) + (w_f32 ? (size_t)groups * (cols * (size_t)K * 6 + (cols + 127) / 128 * 32) : 0);
 }
 
 KB2_API int kb2_linear_f32(const float* x_dev, int64_t x_ld, int64_t x_group, const void* w_dev, int32_t w_f32, void* out_dev, int32_t out_f32,
@@ -274,7 +274,8 @@ KB2_API int kb2_linear_f32(const float* x_dev, int64_t x_ld, int64_t x_group, co
   const int32_t cols = linear_f32_columns(N, K, w_f32, groups);
   SplitPlan plan;                       // one plan for all slices: the row tiles of the parts follow it
   linear_f32_plan(M, cols, K, w_f32, groups, device, &plan);
-  char* wparts = (char*)workspace_dev + x_parts_bytes(plan, M, K, groups);
+  char* partial = (char*)workspace_dev + x_parts_bytes(plan, M, K, groups);
+  char* wparts = partial + (plan.pair ? parts_partial_bytes(M, cols, groups, plan.ks) : 0);
   CUDA_TRY(launch_split_parts(x_dev, x_ld, x_group, M, K, plan.mt, groups, workspace_dev, device_sms(device), s));
   for (int32_t n0 = 0; n0 < N; n0 += cols) {
     SplitGemm g;
@@ -282,6 +283,7 @@ KB2_API int kb2_linear_f32(const float* x_dev, int64_t x_ld, int64_t x_group, co
     uint8_t* low = (uint8_t*)wparts + (size_t)groups * cols * K * 6;
     if (w_f32) CUDA_TRY(launch_split_weights((const float*)w_dev + (size_t)n0 * K, g.N, K, groups, wparts, low, s));
     g.w_low = low;
+    g.partial = (float*)partial;
     g.x = workspace_dev; g.w = w_f32 ? wparts : w_dev;
     g.out = (char*)out_dev + (size_t)n0 * (out_f32 ? 4 : 2);
     g.M = M; g.K = K; g.ldo = out_ld; g.out_f32 = out_f32 != 0;

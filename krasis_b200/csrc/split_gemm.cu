@@ -20,9 +20,9 @@
 // Intelligence Datatype For Higher-Precision Computations", ARITH 2019).  The parts of a tile's rows lie side by side on the N side, so one
 // weight tile serves all of them: w x1 goes to the main accumulators, w x2 and w x3 to two small ones.  With fp32 weights in three parts
 // too, w1 [x1 x2 x3], w2 [x1 x2] and w3 [x1] are added in: six of the nine products, the other three are below 2^-26 of the result.  512 rows,
-// N 16384, K 2048: 231 us, 2-norm error 4.7e-7; fp32-FMA tiles 1494 us, 8.1e-7.  Where w2 and w3 are zeros (the fp32 form of a bf16 checkpoint),
+// N 16384, K 2048: 222 us (on pairs of CTAs, below; 263 without), 2-norm error 4.7e-7; fp32-FMA tiles 1494 us, 8.1e-7.  Where w2 and w3 are zeros (the fp32 form of a bf16 checkpoint),
 // the pass that makes the parts says so per 128 rows x 256 columns; they are then neither written nor loaded nor multiplied: the same sums to
-// the last bit, 180 us (weights of 134 MB among them: 4 bytes of each read, 2 written).
+// the last bit, 138 us (175 without pairs; weights of 134 MB among them: 4 bytes of each read, 2 written).
 #include <cuda.h>
 
 #include <algorithm>
@@ -197,19 +197,27 @@ __global__ void __launch_bounds__(kSThreads)
   float* part = reinterpret_cast<float*>(smem);    // [mt][128]
   const int lanes = warp % 4 * 32;                 // of the tensor memory that this warp can read
   const uint32_t taddr = tmem_base + ((uint32_t)lanes << 16);
-  const int n_sets = (kb1 - kb0 + p.chunk - 1) / p.chunk + (p.xparts > 1 ? 2 : 0);      // the small ones come first
+  const int n_small = p.xparts > 1 ? 2 : 0, n_sets = (kb1 - kb0 + p.chunk - 1) / p.chunk + n_small;      // the small ones come first
   for (int c0 = warp / 4 * 16; c0 < p.mt; c0 += kSWarps * 4) {
     float v[16];
     uint32_t r[16];
-    tmem_ld16(taddr + c0, r);
+    tmem_ld16(taddr + n_small * p.mt + c0, r);
     tmem_ld_wait();
 #pragma unroll
     for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
-    for (int a = 1; a < n_sets; ++a) {
+    for (int a = n_small + 1; a < n_sets; ++a) {
       tmem_ld16(taddr + a * p.mt + c0, r);
       tmem_ld_wait();
 #pragma unroll
       for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(r[j]);
+    }
+    if (n_small) {                                 // their sum goes in last, as pairs of CTAs add it (parts_pair_kernel)
+      uint32_t t[16];
+      tmem_ld16(taddr + c0, r);
+      tmem_ld16(taddr + p.mt + c0, t);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(r[j]) + __uint_as_float(t[j]);
     }
 #pragma unroll
     for (int j = 0; j < 16; ++j) part[(c0 + j) * kSRows + lanes + lane] = v[j];
@@ -276,6 +284,293 @@ __global__ void __launch_bounds__(kSThreads)
   }
   if constexpr (KS > 1) cluster_sync_all(); else __syncthreads();      // nobody's image goes while a peer still reads it
   if (warp == 0) tmem_dealloc(tmem_base, p.tmem_cols);
+}
+
+// ---- fp32 operands in parts on pairs of CTAs, for steps that fill the chip
+// A tile of split_gemm_kernel holds 80 rows at most (three parts of them are one operand, every chunk has an accumulator), its CTA can neither load
+// nor multiply while it reads its accumulators out, and 512 rows x 8192 columns were 448 such tiles on 148 SMs: four rounds for three.  Here a pair of
+// CTAs has 256 weight rows and up to 128 rows of X, each CTA half of either, and goes through its tiles one after the other: eight warps take every
+// chunk's accumulator (two in turn) into registers while the next chunk runs, so a tile needs four accumulators whatever K is.  The largest products,
+// those with x2 and those with x3 go to accumulators of their own, as there; where CTAs of a cluster share K there, tiles are cut into the same segments here, and
+// parts_reduce_kernel adds these in the same order: the same sums, bit for bit.
+// 512 rows, N 8192, K 2048 in three products: 61 -> 43 us (1.2 PFLOP/s; 128 tiles of 128 rows on 74 pairs are two rounds for 1.73, and under this load the clock
+// is that of a cuBLAS product at 1.64 PFLOP/s); N 2048, K 8192 69 -> 42 us and 5 for the segments' sums.
+// Per K block of 64 a CTA takes in 16 KB of weights and 24 KB of x for 768 cycles of MMAs (128 rows): [w1 | its half of x1 | x2 (the first CTA) or
+// x3], so that one MMA of twice the columns multiplies x2 and x3 (an MMA of a pair takes 89 cycles at least: a K block 711 cycles with 32 or 64 rows, 868
+// with 128).  Where w2 and w3 hold anything, a second stage [w2 | w3 | halves of x1 | of x2] follows.
+constexpr int kPTThreads = 384, kPTWarps = 8, kPTMaxStages = 8, kPTRing = 216 * 1024, kPTSmem = kPTRing + (2 * kPTMaxStages + 6) * 8 + 8;
+static_assert(kPTSmem >= tmem_smem(512) && kPTSmem <= 227 * 1024, "what a CTA of a cluster takes for 512 columns");
+
+struct PartsArgs {
+  void* out;
+  long long ldo, out_group, w_part_rows;
+  int M, N, n_kblocks, nt, wparts, chunk, segments, row_tiles, tiles_per_group, w_tiles;
+  const uint8_t* w_low;      // [group][tile of 128 rows][low_spans]
+  int low_span, low_spans;
+  const float* x_raw;
+  long long x_ld, x_group;
+  const void* w_raw;
+  float* partial;            // [segment][group * M + row][N] where there are several, else null
+  long long partial_rows;
+};
+
+template <bool kOutF32>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPTThreads, 1)
+    parts_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const PartsArgs p) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kPTRing);        // of the first CTA: both CTAs' loads
+  uint64_t* empty = full + kPTMaxStages;
+  uint64_t* acc_full = empty + kPTMaxStages;       // [2] a chunk, [2] the two small ones
+  uint64_t* acc_empty = acc_full + 3;              // of the first CTA: both CTAs' read-outs
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(acc_empty + 3);
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  if (threadIdx.x == 32) {
+    if (smem_u32(smem) & 1023u) __trap();
+    for (int i = 0; i < kPTMaxStages; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < 3; ++i) {
+      mbar_init(&acc_full[i], 1);
+      mbar_init(&acc_empty[i], 2 * kPTWarps);
+    }
+    fence_mbar_init();
+  }
+  if (threadIdx.x == 64) {
+    prefetch_tmap(&tmap_x);
+    prefetch_tmap(&tmap_w);
+  }
+  if (warp == 0) tmem_alloc_pair(tmem_ptr_smem, 512);
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();                              // the other CTA's barriers are there
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_wait();
+  // a unit is a segment of K of a tile: row tiles first, so that neighbours share the weights
+  const int tiles = p.w_tiles * p.row_tiles, total = tiles * p.segments, first = blockIdx.x >> 1, step = gridDim.x >> 1;
+  const int nt = p.nt, half = nt / 2, tiles128 = (p.N + kSRows - 1) / kSRows;
+  // what launch_split_weights says about a span of the K blocks of the 128 rows that CTA r has of tile t
+  const auto said = [&](int unit, int r, int span) {
+    const int t = unit % tiles, wt = t / p.row_tiles * 2 + r;
+    return wt < tiles128 && p.w_low[(long long)(t % p.row_tiles / p.tiles_per_group * tiles128 + wt) * p.low_spans + span] != 0;
+  };
+  bool any_low = false;                            // of all tiles of the pair: stages then have room for three parts of the weights
+  if (p.wparts > 1) {
+    for (int i = threadIdx.x; i < (total - first + step - 1) / step * 2 * p.low_spans; i += kPTThreads)
+      any_low |= said(first + i / (2 * p.low_spans) * step, i / p.low_spans & 1, i % p.low_spans);
+    // broadcasts: what addresses and branches of the MMA loop follow from has to be uniform for the compiler, too
+    any_low = __shfl_sync(0xffffffffu, (int)__syncthreads_or(any_low), 0);
+  }
+  const auto low_of = [&](int t, int r) {
+    return any_low ? __shfl_sync(0xffffffffu, __ballot_sync(0xffffffffu, lane < p.low_spans && said(t, r, lane)), 0) : 0u;
+  };
+  const int bytes1 = kSWBytes + 3 * half * 128, bytes2 = 2 * kSWBytes + 2 * half * 128;
+  const int stage_bytes = any_low ? max(bytes1, bytes2) : bytes1, stages = min(kPTMaxStages, kPTRing / stage_bytes);
+  const auto seg_begin = [&](int s) { return (int)((long long)p.n_kblocks * s / p.segments); };
+
+  if (warp == 0) {
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int unit = first; unit < total; unit += step) {
+      const int t = unit % tiles, rt = t % p.row_tiles, group = rt / p.tiles_per_group;
+      const int w0 = t / p.row_tiles * 2 * kSRows + (int)rank * kSRows + group * p.N, x0 = rt * 3 * nt;
+      const uint32_t own = low_of(unit, rank), both = own | low_of(unit, rank ^ 1);
+      for (int kb = seg_begin(unit / tiles), kb1 = seg_begin(unit / tiles + 1); kb < kb1; ++kb) {
+        const int span = kb / p.low_span;
+        for (int low = 0; low <= (int)(both >> span & 1); ++low) {
+          mbar_wait(&empty[stage], phase ^ 1);
+          uint8_t* a = smem + stage * stage_bytes;
+          if (elect_one()) {
+            const uint32_t bar = cluster_addr(&full[stage], 0);
+            if (rank == 0) mbar_arrive_expect_tx(&full[stage], 2 * (low ? bytes2 : bytes1));
+            if (low == 0) {
+              tma_load_2d_pair(a, &tmap_w, kb * kBlockK, w0, bar);
+              a += kSWBytes;
+              tma_load_2d_pair(a, &tmap_x, kb * kBlockK, x0 + (int)rank * half, bar);
+              for (int i = 0; i < 2; ++i) tma_load_2d_pair(a + (1 + i) * half * 128, &tmap_x, kb * kBlockK, x0 + (1 + (int)rank) * nt + i * half, bar);
+            } else {
+              // parts that are zeros were not written: rows behind the last one read as zeros
+              for (int q = 1; q < 3; ++q, a += kSWBytes)
+                tma_load_2d_pair(a, &tmap_w, kb * kBlockK, own >> span & 1 ? w0 + (int)(q * p.w_part_rows) : (int)(3 * p.w_part_rows), bar);
+              for (int q = 0; q < 2; ++q, a += half * 128) tma_load_2d_pair(a, &tmap_x, kb * kBlockK, x0 + q * nt + (int)rank * half, bar);
+            }
+          }
+          __syncwarp();
+          if (++stage == stages) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+    for (int i = 0; i < stages; ++i) {             // the last reports of freed stages have arrived, too
+      mbar_wait(&empty[stage], phase ^ 1);
+      if (++stage == stages) { stage = 0; phase ^= 1; }
+    }
+  } else if (warp == 1 && rank == 0) {
+    int stage = 0, b = 0;
+    uint32_t phase = 0, taken = 0;                 // a bit per accumulator: the parity of its turn
+    const uint32_t idesc = umma_idesc_bf16_m128(nt) + ((128u >> 4) << 24), idesc2 = umma_idesc_bf16_m128(2 * nt) + ((128u >> 4) << 24);      // M = 256
+    const uint32_t small = tmem_base + 2 * nt;
+    for (int unit = first; unit < total; unit += step) {
+      const uint32_t low = low_of(unit, 0) | low_of(unit, 1);
+      const int kb0 = seg_begin(unit / tiles), kb1 = seg_begin(unit / tiles + 1);
+      for (int kb = kb0, in_chunk = 0; kb < kb1; ++kb) {
+        if (in_chunk == 0) {
+          mbar_wait(&acc_empty[b], (taken >> b & 1) ^ 1);
+          taken ^= 1u << b;
+        }
+        mbar_wait(&full[stage], phase);
+        tc_fence_after_sync();
+        const uint32_t a_addr = smem_u32(smem + stage * stage_bytes);
+        const uint64_t w1 = umma_desc_k_sw128(a_addr), x1 = umma_desc_k_sw128(a_addr + kSWBytes), x23 = umma_desc_k_sw128(a_addr + kSWBytes + half * 128);
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_bf16_pair(tmem_base + b * nt, w1 + 2 * k, x1 + 2 * k, idesc, (in_chunk > 0 || k > 0) ? 1u : 0u);
+        }
+        __syncwarp();
+        if (kb == kb0) {
+          mbar_wait(&acc_empty[2], (taken >> 2 & 1) ^ 1);
+          taken ^= 4u;
+          tc_fence_after_sync();
+        }
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_bf16_pair(small, w1 + 2 * k, x23 + 2 * k, idesc2, (kb > kb0 || k > 0) ? 1u : 0u);
+          umma_commit_pair(&empty[stage]);
+        }
+        __syncwarp();
+        if (++stage == stages) { stage = 0; phase ^= 1; }
+        if (low >> (kb / p.low_span) & 1) {
+          mbar_wait(&full[stage], phase);
+          tc_fence_after_sync();
+          const uint32_t l_addr = smem_u32(smem + stage * stage_bytes);
+          const uint64_t w2 = umma_desc_k_sw128(l_addr), w3 = umma_desc_k_sw128(l_addr + kSWBytes), y1 = umma_desc_k_sw128(l_addr + 2 * kSWBytes),
+                         y2 = umma_desc_k_sw128(l_addr + 2 * kSWBytes + half * 128);
+          if (elect_one()) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) umma_bf16_pair(small, w2 + 2 * k, y1 + 2 * k, idesc, 1u);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) umma_bf16_pair(small + nt, w2 + 2 * k, y2 + 2 * k, idesc, 1u);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) umma_bf16_pair(small + nt, w3 + 2 * k, y1 + 2 * k, idesc, 1u);
+            umma_commit_pair(&empty[stage]);
+          }
+          __syncwarp();
+          if (++stage == stages) { stage = 0; phase ^= 1; }
+        }
+        if (elect_one()) {
+          if (kb + 1 == kb1) umma_commit_pair(&acc_full[2]);
+          if (in_chunk + 1 == p.chunk || kb + 1 == kb1) umma_commit_pair(&acc_full[b]);
+        }
+        __syncwarp();
+        if (++in_chunk == p.chunk || kb + 1 == kb1) {
+          in_chunk = 0;
+          b ^= 1;
+        }
+      }
+    }
+  } else if (warp >= 4) {
+    // lane = weight row; the two warps of a quarter of the rows have half the columns (rows of X) each
+    constexpr int kCols = 64;
+    const int q = warp & 3, c0 = (warp - 4) / 4 * half;
+    const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + c0;
+    uint32_t turns = 0;
+    int b = 0;
+    const auto take = [&](uint32_t at, int c, uint32_t (&r)[16]) {
+      tmem_ld16(at + c, r);
+      tmem_ld_wait();
+    };
+    const auto leave = [&](int which) {            // the accumulator may be written again
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(cluster_addr(&acc_empty[which], 0));
+    };
+    for (int unit = first; unit < total; unit += step) {
+      const int seg = unit / tiles, t = unit % tiles, blocks = seg_begin(seg + 1) - seg_begin(seg);
+      float acc[kCols];
+      for (int k = 0; k < blocks; k += p.chunk) {
+        mbar_wait(&acc_full[b], turns >> b & 1);
+        turns ^= 1u << b;
+        tc_fence_after_sync();
+#pragma unroll
+        for (int c = 0; c < kCols; c += 16)
+          if (c < half) {
+            uint32_t r[16];
+            take(taddr + b * nt, c, r);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) acc[c + j] = k == 0 ? __uint_as_float(r[j]) : acc[c + j] + __uint_as_float(r[j]);
+          }
+        leave(b);
+        b ^= 1;
+      }
+      mbar_wait(&acc_full[2], turns >> 2 & 1);
+      turns ^= 4u;
+      tc_fence_after_sync();
+#pragma unroll
+      for (int c = 0; c < kCols; c += 16)
+        if (c < half) {
+          uint32_t r[16], u[16];
+          tmem_ld16(taddr + 2 * nt + c, r);
+          take(taddr + 3 * nt, c, u);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) acc[c + j] += __uint_as_float(r[j]) + __uint_as_float(u[j]);
+        }
+      leave(2);
+      const int rt = t % p.row_tiles, group = rt / p.tiles_per_group, m0 = rt % p.tiles_per_group * nt + c0;
+      const int n = t / p.row_tiles * 2 * kSRows + (int)rank * kSRows + q * 32 + lane;
+      const int rows = n < p.N ? min(half, p.M - m0) : 0;
+      if (p.partial != nullptr) {
+        float* to = p.partial + (seg * p.partial_rows + (long long)group * p.M + m0) * p.N + n;
+#pragma unroll
+        for (int c = 0; c < kCols; ++c) {
+          if (c >= rows) break;
+          to[(long long)c * p.N] = acc[c];
+        }
+      } else {
+        const long long at = group * p.out_group + (long long)m0 * p.ldo + n;
+#pragma unroll
+        for (int c = 0; c < kCols; ++c) {
+          if (c >= rows) break;
+          if (isnan(acc[c]))
+            acc[c] = product_again(p.x_raw + group * p.x_group + (long long)(m0 + c) * p.x_ld, p.w_raw, ((long long)group * p.N + n) * p.n_kblocks * kBlockK,
+                                   p.wparts > 1, p.n_kblocks * kBlockK);
+          if constexpr (kOutF32) reinterpret_cast<float*>(p.out)[at + c * p.ldo] = acc[c];
+          else reinterpret_cast<__nv_bfloat16*>(p.out)[at + c * p.ldo] = __float2bfloat16_rn(acc[c]);
+        }
+      }
+    }
+  }
+  __syncwarp();
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();                              // nobody leaves while the other may still report to its barriers
+  tc_fence_after_sync();
+  if (warp == 0) tmem_dealloc_pair(tmem_base, 512);
+}
+
+// The segments' sums, added in order; four neighbouring columns per thread (N % 16 == 0).  Bound by traffic, from L2.
+template <bool kOutF32>
+__global__ void __launch_bounds__(256) parts_reduce_kernel(const PartsArgs p) {
+  pdl_wait();
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x, step = p.partial_rows * p.N;
+  const int n4 = p.N / 4, n = (int)(i % n4) * 4;
+  const long long r = i / n4;
+  if (r >= p.partial_rows) return;
+  const float* from = p.partial + r * p.N + n;
+  float4 v = *reinterpret_cast<const float4*>(from);
+  for (int s = 1; s < p.segments; ++s) {
+    const float4 f = *reinterpret_cast<const float4*>(from + s * step);
+    v.x += f.x; v.y += f.y; v.z += f.z; v.w += f.w;
+  }
+  const int group = (int)(r / p.M), K = p.n_kblocks * kBlockK;
+  const long long m = r - (long long)group * p.M, at = group * p.out_group + m * p.ldo + n, w0 = ((long long)group * p.N + n) * K;
+  const float* x = p.x_raw + group * p.x_group + m * p.x_ld;
+  if (isnan(v.x)) v.x = product_again(x, p.w_raw, w0, p.wparts > 1, K);
+  if (isnan(v.y)) v.y = product_again(x, p.w_raw, w0 + K, p.wparts > 1, K);
+  if (isnan(v.z)) v.z = product_again(x, p.w_raw, w0 + 2 * K, p.wparts > 1, K);
+  if (isnan(v.w)) v.w = product_again(x, p.w_raw, w0 + 3 * K, p.wparts > 1, K);
+  if constexpr (kOutF32) *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + at) = v;
+  else *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + at) = make_uint2(bf16x2_bits_rn(v.y, v.x), bf16x2_bits_rn(v.w, v.z));
 }
 
 cudaError_t make_tmap_bf16_rows(void* out_tmap, const void* base, long long rows, long long cols, int box_rows);
@@ -365,6 +660,31 @@ bool split_gemm_plan_whole(int M, int N, int K, int num_sms, float us, SplitPlan
   return cheapest(M, N, K, true, num_sms, 1, 1, 1, 1, &best, out);
 }
 
+// Products of fp32 rows on pairs, cut along K as `out` says, where that is estimated to take less than the plan that is there.  Both estimates (us) are fitted to
+// 270 timings of M 33..2048 x 7 weight shapes, bf16 and fp32 weights, from HBM: the chosen form is within 0.8 % of the better one on average.  On both sides of
+// the line (tiles of 80 rows / pairs, bf16 weights): N 16384, K 2048: 160 rows 39.9 / 44.5, 200 rows 63.4 / 46.6, 512 rows 109 / 82, 2048 rows 399 / 282; N 2048,
+// K 8192: 300 rows 44.0 / 55.8, 400 rows 83.5 / 59.8, 2048 rows 335 / 190; N 4096, K 512: 512 rows 18.4 / 16.9.  Fewer rows than 128 never gained.
+static void parts_pair_plan(int M, int N, int K, int num_sms, int wparts, int groups, SplitPlan* out) {
+  const int nkb = K / kBlockK, kb = ceil_div(nkb, out->ks);
+  const int chunk = nkb <= kSplitChunk ? kSplitChunkShort : std::max(kSplitChunk, ceil_div(kb, 30));
+  const size_t partial = parts_partial_bytes(M, N, groups, out->ks);
+  if (M < 128 || chunk != out->chunk || partial > kPartialMost) return;
+  const int per_sm = ceil_div((long long)ceil_div(M, out->mt) * groups * ceil_div(N, kSRows) * out->ks, num_sms);
+  const bool share = per_sm > 1 && 4 * (wparts * kSWBytes + 3 * out->mt * 128) <= 112 * 1024;
+  float us = 0.97f * (4.f + per_sm * (share ? 0.75f : 1.f) * (3.5f + 0.41f * kb * (out->mt > 64 ? 1.2f : 1.f)));
+  const float hbm = (float)N * K * 2.f * groups / 5.76e6f;
+  for (int nt = 128; nt >= 32; nt -= 32) {
+    const long long units = (long long)ceil_div(N, 2 * kSRows) * ceil_div(M, nt) * groups * out->ks;
+    const float rounds = (float)((units + num_sms / 2 - 1) / (num_sms / 2));
+    const float block = 4.f * (std::max(89.f, nt * 0.5f) + std::max(89.f, (float)nt)) / 1550.f;      // an MMA takes 89 cycles at least
+    const float time = 11.5f + std::max(hbm, rounds * (1.5f + kb * block)) + (partial ? 3.f + 2.f * partial / 8e6f : 0.f);
+    if (time >= us) continue;
+    us = time;
+    out->pair = true;
+    out->mt = nt;
+  }
+}
+
 // K is cut as for a step of 64 rows (128 with operands in parts), whatever M is, so that a row's sums do not depend on the rows beside it.  By the
 // estimate above that costs nothing at 9..255 rows of 14 weight shapes (at most 4 % but for two of 112 cases), and 3 % on average with parts
 // at 9..2048 rows (50 % in the worst case, N 1024, K 2048 at 2048 rows).
@@ -374,7 +694,9 @@ bool split_gemm_plan(int M, int N, int K, int num_sms, int xparts, int wparts, i
   if (!cheapest(xparts > 1 ? 128 : 64, N, K, false, num_sms, xparts, wparts, groups, 0, &best, out)) return false;
   const int ks = out->ks;
   best = 1e30f;
-  return cheapest(M, N, K, false, num_sms, xparts, wparts, groups, ks, &best, out);
+  if (!cheapest(M, N, K, false, num_sms, xparts, wparts, groups, ks, &best, out)) return false;
+  if (xparts > 1) parts_pair_plan(M, N, K, num_sms, wparts, groups, out);
+  return true;
 }
 
 // Tiles of 16 rows sum in chunks, as the products of 9 to 255 rows do; larger ones in one accumulator, as the tiles of 128 rows do: which tile
@@ -388,10 +710,58 @@ SplitPlan split_gemm_binned_plan(int K, int tile_rows) {
   return p;
 }
 
+static cudaError_t launch_parts_pair(const SplitGemm& g, const SplitPlan& plan, cudaStream_t s) {
+  const int tiles = ceil_div(g.M, plan.mt), row_tiles = tiles * g.groups;
+  if (g.xparts != 3 || !g.batched || g.tile_group || g.bias || g.glu || !g.x_raw || !g.w_raw || plan.mt % 32 || plan.mt > 128 || plan.chunk < 1 || plan.ks < 1 ||
+      (plan.ks > 1 && !g.partial) || (g.wparts != 1 && (g.wparts != 3 || !g.w_low)))
+    return cudaErrorInvalidValue;
+  alignas(64) CUtensorMap tx, tw;
+  cudaError_t e = make_tmap_bf16_rows(&tx, g.x, (long long)row_tiles * 3 * plan.mt, g.K, plan.mt / 2);
+  if (e != cudaSuccess) return e;
+  e = make_tmap_bf16_rows(&tw, g.w, (long long)g.wparts * g.groups * g.N, g.K, kSRows);
+  if (e != cudaSuccess) return e;
+  PartsArgs p{};
+  p.out = g.out;
+  p.ldo = g.ldo;
+  p.out_group = g.out_group;
+  p.w_part_rows = (long long)g.groups * g.N;
+  p.M = g.M;
+  p.N = g.N;
+  p.n_kblocks = g.K / kBlockK;
+  p.nt = plan.mt;
+  p.wparts = g.wparts;
+  p.chunk = plan.chunk;
+  p.segments = plan.ks;
+  p.row_tiles = row_tiles;
+  p.tiles_per_group = tiles;
+  p.w_tiles = ceil_div(g.N, 2 * kSRows);
+  p.w_low = g.w_low;
+  p.low_span = split_low_span(g.N, g.K, g.groups);
+  p.low_spans = ceil_div(p.n_kblocks, p.low_span);
+  p.x_raw = g.x_raw;
+  p.x_ld = g.x_ld;
+  p.x_group = g.x_group;
+  p.w_raw = g.w_raw;
+  p.partial = plan.ks > 1 ? g.partial : nullptr;
+  p.partial_rows = (long long)g.groups * g.M;
+  const int pairs = (int)std::min<long long>((long long)p.w_tiles * row_tiles * plan.ks, current_sms() / 2);
+  const unsigned blocks = (unsigned)((p.partial_rows * (g.N / 4) + 255) / 256);
+  const auto run = [&](auto f32) {
+    constexpr bool kF32 = decltype(f32)::value;
+    cudaError_t r = allow_smem<parts_pair_kernel<kF32>>(kPTSmem);
+    if (r == cudaSuccess) r = launch_pdl(parts_pair_kernel<kF32>, dim3(2 * pairs), dim3(kPTThreads), kPTSmem, s, tx, tw, p);
+    if (r == cudaSuccess && plan.ks > 1) r = launch_pdl(parts_reduce_kernel<kF32>, blocks, 256, 0, s, p);
+    return r;
+  };
+  return g.out_f32 ? run(std::true_type{}) : run(std::false_type{});
+}
+
 cudaError_t launch_split_gemm(const SplitGemm& g, const SplitPlan& plan, cudaStream_t s) {
   KernelSpan span(K_DENSE_BF16, s);
   const int nkb = g.K / kBlockK, nt = g.xparts * plan.mt;
-  if (g.K % kBlockK || g.N % 16 || g.M <= 0 || g.groups <= 0 || plan.mt < 16 || nt > 256 || plan.mt % 16 || plan.ks < 1 || nkb < plan.ks ||
+  if (g.K % kBlockK || g.N % 16 || g.M <= 0 || g.groups <= 0) return cudaErrorInvalidValue;
+  if (plan.pair) return launch_parts_pair(g, plan, s);
+  if (plan.mt < 16 || nt > 256 || plan.mt % 16 || plan.ks < 1 || nkb < plan.ks ||
       plan.chunk < 1 || (g.xparts != 1 && g.xparts != 3) || (g.wparts != 1 && g.wparts != g.xparts))
     return cudaErrorInvalidValue;
   const int tiles = ceil_div(g.M, plan.mt), row_tiles = g.batched ? tiles * g.groups : tiles;

@@ -24,6 +24,7 @@ struct SplitPlan {
   int ks = 1;       // CTAs of a cluster that share a tile along K
   int stages = 0;   // depth of the TMA ring
   int chunk = 0;    // K blocks per accumulator (all of a CTA's: one sum)
+  bool pair = false; // three parts of x on pairs of CTAs: tiles of mt rows (a multiple of 32), K in ks segments whose sums meet in a workspace
 };
 
 // x [M][K] and w [groups][N][K] as bf16 arrays, or as three bf16 parts of fp32 arrays laid out by launch_split_parts.
@@ -51,6 +52,7 @@ struct SplitGemm {
   bool glu = false;
   int glu_kind = 0;
   float glu_limit = 0.f, glu_alpha = 0.f;
+  float* partial = nullptr;                 // pairs with several segments: parts_partial_bytes of workspace
   const uint8_t* w_low = nullptr;           // wparts 3: what launch_split_weights says about the low parts
 };
 
@@ -62,6 +64,10 @@ inline int split_low_span(int N, int K, int groups) {
   while (span > 1 && (long long)groups * ((N + 127) / 128) * ((nkb + span - 1) / span) < 512) span /= 2;
   return span > least ? span : least;
 }
+
+// The segments' sums of a product on pairs; calls that would take more of them than kPartialMost stay with split_gemm_kernel.
+constexpr size_t kPartialMost = 256u << 20;
+inline size_t parts_partial_bytes(int M, int N, int groups, int ks) { return ks > 1 ? (size_t)ks * groups * M * N * 4 : 0; }
 
 // One accumulator over all of K, K block by K block: the sums of dense_gemm.cu, bit for bit.  false: not estimated to take less than `us`.
 bool split_gemm_plan_whole(int M, int N, int K, int num_sms, float us, SplitPlan* out);
