@@ -9,12 +9,12 @@
 //                     cache (:596-642), then attn * sigmoid(gate) (:665-666)
 // The q/k/v/o projections are dense_gemm_kernel.
 //
-// FMHA layout: one CTA = 128 query rows of one head; KV tiles of 64 keys.  12 warps:
-//   warps 0-3  KV loaders: FP8 pages -> BF16 -> 128B-swizzled smem (K as K-major B operand, V as MN-major B operand)
-//   warp  4    tcgen05.mma issuer: S = Q K^T (SS), O += P V (P from TMEM)
-//   warp  5    Q loader (2-D TMA)
-//   warps 8-11 softmax: S (TMEM) -> exp2 -> P (BF16, TMEM); running max with lazy rescale of O in TMEM; epilogue
-// TMEM: S [0,64) | P [64,96) | O [128,128+D).
+// FMHA layout: one CTA = 128 query rows of one head; KV tiles of FK = 128 keys (64 with values of 256).  12 warps:
+//   warps 0, 3 loaders of K and of V (2-D TMA): a loader of both would ask for K(it + 2) behind V(it + 1), which waits for PV(it - 1)
+//   warp  1    tcgen05.mma issuer: S = Q K^T (SS), O += P V (P from TMEM)
+//   warp  2    Q loader (2-D TMA)
+//   warps 4-11 softmax, two threads per row: S (TMEM) -> exp2 -> P (BF16, TMEM); running max with lazy rescale of O in TMEM; epilogue
+// TMEM: S, two buffers [0,2 FK) | P, two buffers [2 FK,3 FK) | O [3 FK,3 FK + DV).
 #include <cuda.h>
 #include <cuda_fp8.h>
 
@@ -122,23 +122,24 @@ __global__ void __launch_bounds__(256, 8) gqa_prep_kernel(GqaDims g, const __nv_
 // FMHA
 // ------------------------------------------------------------------------------------------------
 constexpr int kFQ = 128;        // query rows per CTA
-constexpr int kFK = 64;         // keys per KV tile
-constexpr int kFThreads = 512;   // 16 warps: 0 KV TMA, 4 MMA, 5 Q TMA + TMEM, 8-15 softmax (two threads per query row)
-constexpr int kFStages = 2;
+constexpr int kFThreads = 384;
+template <int DV> constexpr int kFK = DV > 128 ? 64 : 128;      // keys per KV tile: what tensor memory has room for
 
 template <int DQ, int DV>
 struct FmhaSmem {
   static constexpr int kQBytes = kFQ * DQ * 2;
-  static constexpr int kKBytes = kFK * DQ * 2;
-  static constexpr int kVBytes = kFK * DV * 2;
+  static constexpr int kKBytes = kFK<DV> * DQ * 2;
+  static constexpr int kVBytes = kFK<DV> * DV * 2;
+  static constexpr int kStages = 2;
   static constexpr int kOffQ = 0;
   static constexpr int kOffK = kOffQ + kQBytes;
-  static constexpr int kOffV = kOffK + kFStages * kKBytes;
-  static constexpr int kOffBar = kOffV + kFStages * kVBytes;
-  static constexpr int kOffXchg = kOffBar + 128;          // float [2 tile parities][2 halves][128 rows]
+  static constexpr int kOffV = kOffK + kStages * kKBytes;
+  static constexpr int kOffBar = kOffV + kStages * kVBytes;
+  static constexpr int kOffXchg = kOffBar + 256;          // float [maximum, sum][group][128 rows]
   static constexpr int kTotal = kOffXchg + 2 * 2 * kFQ * 4;
   static_assert(kTotal <= 227 * 1024, "smem");
   static_assert(kQBytes % 1024 == 0 && kKBytes % 1024 == 0 && kVBytes % 1024 == 0, "swizzle atoms");
+  static_assert(3 * kFK<DV> + DV <= 512, "tensor memory");
 };
 
 __device__ __forceinline__ uint32_t umma_idesc_bf16_m128_bmn(uint32_t n) {   // B operand MN-major
@@ -161,6 +162,32 @@ __device__ __forceinline__ float ex2_approx(float x) {       // 2^x, MUFU.EX2 (2
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float m;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+  return m;
+}
+// two fp32 numbers that go through the arithmetic together
+__device__ __forceinline__ uint64_t pair_of(float a, float b) {
+  uint64_t p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(a), "f"(b));
+  return p;
+}
+__device__ __forceinline__ float2 pair_get(uint64_t p) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(p));
+  return f;
+}
+__device__ __forceinline__ uint64_t pair_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t p;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p) : "l"(a), "l"(b), "l"(c));
+  return p;
+}
+__device__ __forceinline__ uint64_t pair_add(uint64_t a, uint64_t b) {
+  uint64_t p;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(p) : "l"(a), "l"(b));
+  return p;
+}
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
@@ -175,6 +202,13 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 //   tmap_k   [kv_len][*]: this head's keys at column k_col0 + kvh * (PE ? DQ - 64 : DQ)
 //   tmap_kpe [kv_len][64] (PE only, MLA): the rope part of the key, shared by all heads, is the last 64-wide chunk
 //   tmap_v   [kv_len][*]: this head's values at column v_col0 + kvh * DV
+// A tile is a chain: S = Q K^T, the row maxima, exponentials, O += P V.  S and P have two buffers each, so the tensor pipe makes the S of the next two tiles
+// while the softmax warps work, and these hardly wait for it; K and V have a loader each.  An MMA reads its 128 x 16 piece of Q from shared memory again, 32
+// cycles for 32 of work with 64 keys: tiles of 128 where tensor memory has room.  What is left: with 128 value columns the exponentials (64 x 128 of them take
+// 1030 cycles of the special function units, a tile 2400), with 256 the MMAs (1280 cycles of 1570 a tile; the whole runs at the power limit).  us with
+// single buffers, one loader and tiles of 64 keys, and now: 2048 x 16 heads of 256 after 2500 keys 140 -> 134; latent attention of 1000 tokens, 16 heads 20.2 ->
+// 16.7, 100 tokens after 2000 32.6 -> 25.8; 2048 tokens, 16 heads of 128 36.6 -> 29.7; 17 tokens after 300 9.2 -> 9.8 (latent), 20.7 -> 20.4 (256).  Tried: the
+// tiles to two groups of warps in turn, a thread per row (latent 18.0: its warps are one per scheduler); pairs of CTAs with heads of 256 (164).
 template <int DQ, int DV, bool PE>
 __global__ void __launch_bounds__(kFThreads, 1)
     gqa_fmha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -195,21 +229,16 @@ __global__ void __launch_bounds__(kFThreads, 1)
                     const float* __restrict__ head_gate, long long ldg) {   // if given, [M][ldg]: head h's output rows are
                                                                  // multiplied by sigmoid(head_gate[row][h])
   using L = FmhaSmem<DQ, DV>;
-  constexpr int D = DQ;
+  constexpr int D = DQ, FK = kFK<DV>, KS = L::kStages;
   constexpr int NC = DQ / 64;                      // 64-wide d chunks of q/k
   constexpr int NKC = PE ? NC - 1 : NC;            // of which from tmap_k
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kOffBar);
   uint64_t* q_full = bars;
-  uint64_t* k_full = bars + 1;       // [2]  K and V stages are filled and released separately: K(it) is free as soon as
-  uint64_t* k_empty = bars + 3;      // [2]  QK^T(it) has run, one PV earlier than V(it), so the next K tile's TMA starts
-  uint64_t* v_full = bars + 10;      // [2]  a whole tile period earlier (the 64 KB tile loads were the latency chain)
-  uint64_t* v_empty = bars + 12;     // [2]
-  uint64_t* s_full = bars + 5;
-  uint64_t* s_cons = bars + 6;
-  uint64_t* p_full = bars + 7;
-  uint64_t* pv_done = bars + 8;      // [2]: PV(it) commits to pv_done[it & 1] (P is double-buffered)
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 14);
+  // K and V stages are filled and released separately: K(it) is free as soon as QK^T(it) has run, ahead of V(it)
+  uint64_t *k_full = bars + 1, *k_empty = k_full + KS, *v_full = k_empty + KS, *v_empty = v_full + KS;
+  uint64_t *s_full = v_empty + KS, *s_cons = s_full + 2, *p_full = s_cons + 2, *pv_done = p_full + 2;      // [2], by tile parity
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(pv_done + 2);
   // shuffle-broadcast warp index: role branches provably warp-uniform (issued from a divergent `lane == 0` branch each tcgen05.mma costs about
   // 50 cycles, more than an N=64 MMA runs)
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -224,189 +253,164 @@ __global__ void __launch_bounds__(kFThreads, 1)
   const int n_keys = min(kv_len, q_start + last_q + 1);
   // sliding window: the tile's first query needs no key before q_start + q0 - window + 1, so whole KV tiles below are skipped;
   // every role counts tiles from tile0 (TMA coordinates and key positions add it back)
-  const int tile0 = max(0, q_start + q0 - window + 1) / kFK;
-  const int n_tiles = (n_keys + kFK - 1) / kFK - tile0;
+  const int tile0 = max(0, q_start + q0 - window + 1) / FK;
+  const int n_tiles = (n_keys + FK - 1) / FK - tile0;
 
-  if (threadIdx.x == 128) {
+  if (threadIdx.x == 96) {
     if (smem_u32(smem) & 1023u) __trap();
     mbar_init(q_full, 1);
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < KS; ++i) {
       mbar_init(&k_full[i], 1);
       mbar_init(&k_empty[i], 1);
       mbar_init(&v_full[i], 1);
       mbar_init(&v_empty[i], 1);
     }
-    mbar_init(s_full, 1);
-    mbar_init(s_cons, 256);
-    mbar_init(p_full, 256);
-    mbar_init(&pv_done[0], 1);
-    mbar_init(&pv_done[1], 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&s_full[i], 1);
+      mbar_init(&s_cons[i], 8);
+      mbar_init(&p_full[i], 8);
+      mbar_init(&pv_done[i], 1);
+    }
     fence_mbar_init();
   }
-  if (warp == 5) tmem_alloc(tmem_ptr_smem, 512);
+  if (warp == 2) tmem_alloc(tmem_ptr_smem, 512);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
   pdl_enter(q_raw, out, sinks, out_f32, lse_out, slopes, head_gate);
-  constexpr uint32_t kColS = 0, kColP = 64, kColO = 128;      // P: two buffers of 32 columns at 64 and 96
+  constexpr uint32_t kColS = 0, kColP = 2 * FK, kColO = 3 * FK;
 
-  if (warp < 4) {
-    // ------------------------------------------------------------ KV producer: one thread issues the TMA boxes of a tile
-    if (warp == 0) {
-      const int kx = k_col0 + kkh * (PE ? DQ - 64 : DQ), vx = v_col0 + kvh * DV;
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int it = 0; it < n_tiles; ++it) {
-        uint8_t* ks = smem + L::kOffK + stage * L::kKBytes;
-        uint8_t* vs = smem + L::kOffV + stage * L::kVBytes;
-        mbar_wait(&k_empty[stage], phase ^ 1);
-        if (elect_one()) {
-          mbar_arrive_expect_tx(&k_full[stage], L::kKBytes);
+  if (warp == 0) {
+    // ------------------------------------------------------------ K: one thread issues the TMA boxes of a tile
+    const int kx = k_col0 + kkh * (PE ? DQ - 64 : DQ);
+    for (int it = 0; it < n_tiles; ++it) {
+      const int b = it % KS;
+      uint8_t* ks = smem + L::kOffK + b * L::kKBytes;
+      mbar_wait(&k_empty[b], (it / KS & 1) ^ 1);
+      if (elect_one()) {
+        mbar_arrive_expect_tx(&k_full[b], L::kKBytes);
 #pragma unroll
-          for (int c = 0; c < NKC; ++c) tma_load_2d(ks + c * (kFK * 128), &tmap_k, kx + c * 64, (it + tile0) * kFK, &k_full[stage]);
-          if constexpr (PE) tma_load_2d(ks + NKC * (kFK * 128), &tmap_kpe, 0, (it + tile0) * kFK, &k_full[stage]);
-        }
-        __syncwarp();
-        mbar_wait(&v_empty[stage], phase ^ 1);
-        if (elect_one()) {
-          mbar_arrive_expect_tx(&v_full[stage], L::kVBytes);
-#pragma unroll
-          for (int c = 0; c < DV / 64; ++c) tma_load_2d(vs + c * (kFK * 128), &tmap_v, vx + c * 64, (it + tile0) * kFK, &v_full[stage]);
-        }
-        __syncwarp();
-        if (++stage == kFStages) { stage = 0; phase ^= 1; }
+        for (int c = 0; c < NKC; ++c) tma_load_2d(ks + c * (FK * 128), &tmap_k, kx + c * 64, (it + tile0) * FK, &k_full[b]);
+        if constexpr (PE) tma_load_2d(ks + NKC * (FK * 128), &tmap_kpe, 0, (it + tile0) * FK, &k_full[b]);
       }
+      __syncwarp();
     }
-    __syncwarp();
-  } else if (warp == 4) {
+  } else if (warp == 3) {
+    // ------------------------------------------------------------ V
+    const int vx = v_col0 + kvh * DV;
+    for (int it = 0; it < n_tiles; ++it) {
+      const int b = it % KS;
+      uint8_t* vs = smem + L::kOffV + b * L::kVBytes;
+      mbar_wait(&v_empty[b], (it / KS & 1) ^ 1);
+      if (elect_one()) {
+        mbar_arrive_expect_tx(&v_full[b], L::kVBytes);
+#pragma unroll
+        for (int c = 0; c < DV / 64; ++c) tma_load_2d(vs + c * (FK * 128), &tmap_v, vx + c * 64, (it + tile0) * FK, &v_full[b]);
+      }
+      __syncwarp();
+    }
+  } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     if (n_tiles > 0) {
-      const uint32_t id_s = umma_idesc_bf16_m128(kFK);
+      const uint32_t id_s = umma_idesc_bf16_m128(FK);
       const uint32_t id_o = umma_idesc_bf16_m128_bmn(DV);
       mbar_wait(q_full, 0);
-      int stage = 0;
-      uint32_t phase = 0, sc_phase = 0, pf_phase = 0;
       const uint32_t q_addr = smem_u32(smem + L::kOffQ);
-      auto issue_pv = [&](int st, bool first, int pbuf) {
-        const uint32_t v_addr = smem_u32(smem + L::kOffV + st * L::kVBytes);
-#pragma unroll
-        for (int k = 0; k < kFK / 16; ++k) {
-          const uint64_t bd = umma_desc_mn_sw128(v_addr + k * 2048, kFK * 128, 1024);
-          umma_bf16_ts(tmem_base + kColO, tmem_base + kColP + pbuf * 32 + 8 * k, bd, id_o, (first && k == 0) ? 0u : 1u);
-        }
-      };
-      int prev_stage = 0;
-      uint32_t prev_phase = 0;
-      for (int it = 0; it < n_tiles; ++it) {
-        mbar_wait(&k_full[stage], phase);
-        if (it > 0) {
-          mbar_wait(s_cons, sc_phase);
-          sc_phase ^= 1;
-        }
+      auto issue_s = [&](int it) {                   // S(it) = Q K(it)^T
+        const int b = it & 1, st = it % KS;
+        mbar_wait(&k_full[st], it / KS & 1);
+        if (it >= 2) mbar_wait(&s_cons[b], (it >> 1 & 1) ^ 1);
         tc_fence_after_sync();
-        const uint32_t k_addr = smem_u32(smem + L::kOffK + stage * L::kKBytes);
+        const uint32_t k_addr = smem_u32(smem + L::kOffK + st * L::kKBytes);
         if (elect_one()) {
 #pragma unroll
           for (int c = 0; c < NC; ++c) {
             const uint64_t ad = umma_desc_k_sw128(q_addr + c * (kFQ * 128));
-            const uint64_t bd = umma_desc_k_sw128(k_addr + c * (kFK * 128));
+            const uint64_t bd = umma_desc_k_sw128(k_addr + c * (FK * 128));
 #pragma unroll
-            for (int k = 0; k < 4; ++k) umma_bf16(tmem_base + kColS, ad + 2 * k, bd + 2 * k, id_s, (c > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < 4; ++k) umma_bf16(tmem_base + kColS + b * FK, ad + 2 * k, bd + 2 * k, id_s, (c > 0 || k > 0) ? 1u : 0u);
           }
-          umma_commit(s_full);
-          umma_commit(&k_empty[stage]);              // K(it) is free once QK^T(it) has run
+          umma_commit(&s_full[b]);
+          umma_commit(&k_empty[st]);
         }
         __syncwarp();
-        if (it > 0) {
-          mbar_wait(&v_full[prev_stage], prev_phase);
-          mbar_wait(p_full, pf_phase);
-          pf_phase ^= 1;
-          tc_fence_after_sync();
-          if (elect_one()) {
-            issue_pv(prev_stage, it == 1, (it - 1) & 1);
-            umma_commit(&pv_done[(it - 1) & 1]);
-            umma_commit(&v_empty[prev_stage]);
+      };
+      issue_s(0);
+      if (n_tiles > 1) issue_s(1);
+      for (int it = 0; it < n_tiles; ++it) {
+        if (it + 2 < n_tiles) issue_s(it + 2);
+        const int b = it & 1, st = it % KS;
+        mbar_wait(&v_full[st], it / KS & 1);
+        mbar_wait(&p_full[b], it >> 1 & 1);
+        tc_fence_after_sync();
+        const uint32_t v_addr = smem_u32(smem + L::kOffV + st * L::kVBytes);
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < FK / 16; ++k) {
+            const uint64_t bd = umma_desc_mn_sw128(v_addr + k * 2048, FK * 128, 1024);
+            umma_bf16_ts(tmem_base + kColO, tmem_base + kColP + b * (FK / 2) + 8 * k, bd, id_o, (it == 0 && k == 0) ? 0u : 1u);
           }
-          __syncwarp();
+          umma_commit(&pv_done[b]);
+          umma_commit(&v_empty[st]);
         }
-        prev_stage = stage;
-        prev_phase = phase;
-        if (++stage == kFStages) { stage = 0; phase ^= 1; }
+        __syncwarp();
       }
-      mbar_wait(&v_full[prev_stage], prev_phase);
-      mbar_wait(p_full, pf_phase);
-      tc_fence_after_sync();
-      if (elect_one()) {
-        issue_pv(prev_stage, n_tiles == 1, (n_tiles - 1) & 1);
-        umma_commit(&pv_done[(n_tiles - 1) & 1]);
-        umma_commit(&v_empty[prev_stage]);
-      }
-      __syncwarp();
     }
-    __syncwarp();
-  } else if (warp == 5) {
+  } else if (warp == 2) {
     if (n_tiles > 0 && elect_one()) {
       mbar_arrive_expect_tx(q_full, L::kQBytes);
 #pragma unroll
       for (int c = 0; c < NC; ++c)
         tma_load_2d(smem + L::kOffQ + c * (kFQ * 128), &tmap_q, head * D + c * 64, q0, q_full);
     }
-    __syncwarp();
-  } else if (warp >= 8) {
+  } else if (warp >= 4) {
     // ------------------------------------------------------------ softmax + epilogue: two threads per query row.
-    // Warp w serves TMEM lane quarter q = w & 3; warps 8-11 take key columns [0,32) of each tile and the first half of
-    // the O columns, warps 12-15 the second halves.  The two threads of a row exchange their tile maxima through smem
-    // (one 64-thread named barrier per tile), make identical running-max decisions, and keep partial row sums that
-    // are added once at the end.
-    const int q = warp & 3, hf = (warp - 8) >> 2;
+    // Warp w serves TMEM lane quarter q = w & 3; warps 4-7 take the first half of a tile's key columns and of the O columns, warps 8-11 the second.
+    // The two threads of a row exchange their tile maxima through smem (one 64-thread named barrier per tile), make identical running-max decisions,
+    // and keep partial row sums that are added once at the end.
+    const int q = warp & 3, hf = (warp - 4) >> 2;
     const int row = q * 32 + lane;
     const int qi = q0 + row;                       // query index within this call
     const int q_pos = q_start + qi;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     float* xchg = reinterpret_cast<float*>(smem + L::kOffXchg);
-    constexpr int KH = kFK / 2, OH = DV / 2;
+    constexpr int KH = FK / 2, OH = DV / 2;
     float m_ref = -INFINITY, l_sum = 0.f;
     // the penalty in units of the raw scores, so that the scale folded into the exponent applies to both
     const float slope = slopes != nullptr ? slopes[head] * 1.4426950408889634f / sm_scale_log2 : 0.f;
-    uint32_t sf_phase = 0;
-    // PV completions observed so far on each of the two pv_done barriers.  P is double-buffered, so a tile only has to
-    // wait for PV(it-2) (its P buffer is free again) — and for PV(it-1) in the rare case it rescales O.  A thread never
-    // lags two completions behind on one barrier: the next PV on it cannot be issued before this thread's p_full arrive.
-    uint32_t pv_seen[2] = {0u, 0u};
-    auto pv_wait = [&](int b, uint32_t need) {
-      while (pv_seen[b] < need) {
-        mbar_wait(&pv_done[b], pv_seen[b] & 1);
-        ++pv_seen[b];
-      }
+    auto tell = [&](uint64_t* bar) {
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    // PV(it) has run.  The caller has seen PV(it - 2), so the barrier's turn is this one or the next
+    auto pv_wait = [&](int it) {
+      mbar_wait(&pv_done[it & 1], it >> 1 & 1);
       tc_fence_after_sync();
     };
     for (int it = 0; it < n_tiles; ++it) {
-      mbar_wait(s_full, sf_phase);
-      sf_phase ^= 1;
+      const int b = it & 1;
+      mbar_wait(&s_full[b], it >> 1 & 1);
       tc_fence_after_sync();
       float s[KH];                                   // raw scores (the softmax scale is folded into the exponent FMA)
       {
-        uint32_t r0[16], r1[16];
-        tmem_ld16(lane_addr + kColS + hf * KH, r0);
-        tmem_ld16(lane_addr + kColS + hf * KH + 16, r1);
+        uint32_t r[KH / 16][16];
+#pragma unroll
+        for (int c = 0; c < KH / 16; ++c) tmem_ld16(lane_addr + kColS + b * FK + hf * KH + 16 * c, r[c]);
         tmem_ld_wait();
 #pragma unroll
-        for (int jj = 0; jj < 16; ++jj) {
-          s[jj] = __uint_as_float(r0[jj]);
-          s[16 + jj] = __uint_as_float(r1[jj]);
-        }
+        for (int jj = 0; jj < KH; ++jj) s[jj] = __uint_as_float(r[jj / 16][jj % 16]);
       }
-      tc_fence_before_sync();
-      mbar_arrive(s_cons);                         // S may be overwritten by the next QK^T
-      if (cap_in != 0.f) {                         // tanh(x) = 1 - 2 / (2^(2 x log2 e) + 1): exact limits at +-inf, two MUFU ops per score
+      tell(&s_cons[b]);                              // S may be overwritten by QK^T(it + 2)
+      if (cap_in != 0.f) {                           // tanh(x) = 1 - 2 / (2^(2 x log2 e) + 1): exact limits at +-inf, two MUFU ops per score
         const float c2 = cap_in * 2.8853900817779268f;
 #pragma unroll
         for (int jj = 0; jj < KH; ++jj) s[jj] = cap_out * (1.f - __fdividef(2.f, ex2_approx(s[jj] * c2) + 1.f));
       }
-      const int key0 = (it + tile0) * kFK + hf * KH;
+      const int key0 = (it + tile0) * FK + hf * KH;
       if (slope != 0.f) {
-        const float back = (float)(key0 - q_pos);          // minus the distance; invisible keys are masked below whatever this gives
+        const float back = (float)(key0 - q_pos);            // minus the distance; invisible keys are masked below whatever this gives
 #pragma unroll
         for (int jj = 0; jj < KH; ++jj) s[jj] = fmaf(slope, back + (float)jj, s[jj]);
       }
@@ -416,11 +420,13 @@ __global__ void __launch_bounds__(kFThreads, 1)
         for (int jj = 0; jj < KH; ++jj)
           if (key0 + jj > q_pos || key0 + jj >= kv_len || key0 + jj + window <= q_pos) s[jj] = -INFINITY;
       }
-      float m_tile = -INFINITY;
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int jj = 0; jj < KH; ++jj) m_tile = fmaxf(m_tile, s[jj]);
-      float* xb = xchg + (it & 1) * (2 * kFQ);
+      for (int jj = 0; jj < KH; jj += 2) mx[jj >> 1 & 3] = max3(mx[jj >> 1 & 3], s[jj], s[jj + 1]);
+      float m_tile = max3(fmaxf(mx[0], mx[1]), mx[2], mx[3]);
+      float* xb = xchg + b * (2 * kFQ);
       xb[hf * kFQ + row] = m_tile;
+      __syncwarp();
       named_bar_sync(1 + q, 64);
       m_tile = fmaxf(m_tile, xb[(hf ^ 1) * kFQ + row]) * sm_scale_log2;      // sm_scale > 0: max commutes with the scale
       // lazy rescale: keep the reference max until the true max exceeds it by 8 (p stays <= 2^8)
@@ -435,21 +441,24 @@ __global__ void __launch_bounds__(kFThreads, 1)
         }
       }
       const float neg_m = (m_ref == -INFINITY) ? 0.f : -m_ref;   // row fully masked so far: every s is -inf -> p = 0
-      float psum = 0.f;
-      uint32_t pk[KH / 2];
+      const uint64_t scale2 = pair_of(sm_scale_log2, sm_scale_log2), neg2 = pair_of(neg_m, neg_m);
+      uint64_t psum[2] = {0, 0};                     // two numbers each
+      uint32_t pk[KH / 32][16];
 #pragma unroll
       for (int jj = 0; jj < KH; jj += 2) {
-        const float p0 = ex2_approx(fmaf(s[jj], sm_scale_log2, neg_m));
-        const float p1 = ex2_approx(fmaf(s[jj + 1], sm_scale_log2, neg_m));
-        __nv_bfloat162 pb = __floats2bfloat162_rn(p0, p1);
-        psum += __low2float(pb) + __high2float(pb);     // normalise with the values the MMA actually uses
-        pk[jj / 2] = *reinterpret_cast<uint32_t*>(&pb);
+        const float2 e = pair_get(pair_fma(pair_of(s[jj], s[jj + 1]), scale2, neg2));
+        const uint32_t pb = bf16x2_bits_rn(ex2_approx(e.y), ex2_approx(e.x));
+        // normalise with the values the MMA actually uses
+        psum[jj >> 1 & 1] = pair_add(psum[jj >> 1 & 1], pair_of(__uint_as_float(pb << 16), __uint_as_float(pb & 0xFFFF0000u)));
+        pk[jj / 32][jj / 2 % 16] = pb;
       }
-      l_sum = l_sum * scale_o + psum;
+      const float2 sum2 = pair_get(pair_add(psum[0], psum[1]));
+      l_sum = l_sum * scale_o + (sum2.x + sum2.y);
+      if (it >= 2) pv_wait(it - 2);                  // PV(it-2) has read this P buffer
       // tcgen05.ld/st are warp-collective (.sync.aligned): the decision must be warp-uniform; rows that keep their
       // reference max multiply by 1
       if (__any_sync(0xffffffffu, rescale)) {
-        pv_wait((it - 1) & 1, (uint32_t)((it - 1) / 2 + 1));     // O must hold every PV up to tile it-1 (rescale => it >= 1)
+        pv_wait(it - 1);                             // O must hold every PV up to tile it-1 (rescale => it >= 1)
         const float sc = rescale ? scale_o : 1.f;
 #pragma unroll 2
         for (int c0 = hf * OH; c0 < (hf + 1) * OH; c0 += 16) {
@@ -461,22 +470,22 @@ __global__ void __launch_bounds__(kFThreads, 1)
           tmem_st16(lane_addr + kColO + c0, r);
         }
       }
-      if (it >= 2) pv_wait(it & 1, (uint32_t)(it / 2));          // PV(it-2) has read this P buffer
-      tmem_st16(lane_addr + kColP + (it & 1) * 32 + hf * (KH / 2), pk);
+#pragma unroll
+      for (int c = 0; c < KH / 32; ++c) tmem_st16(lane_addr + kColP + b * (FK / 2) + hf * (KH / 2) + c * 16, pk[c]);
       tmem_st_wait();
-      tc_fence_before_sync();
-      mbar_arrive(p_full);
+      tell(&p_full[b]);
     }
     if (n_tiles > 0) {
       float* xb = xchg + (n_tiles & 1) * (2 * kFQ);   // the buffer the last tile did not use
       if (sinks != nullptr && hf == 0 && m_ref != -INFINITY) l_sum += ex2_approx(fmaf(sinks[head], 1.4426950408889634f, -m_ref));
       xb[hf * kFQ + row] = l_sum;
+      __syncwarp();
       named_bar_sync(1 + q, 64);
       l_sum += xb[(hf ^ 1) * kFQ + row];
       if (lse_out != nullptr && hf == 0 && qi < M)
         lse_out[(long long)qi * g.nh + head] = l_sum > 0.f ? (m_ref + log2f(l_sum)) * 0.6931471805599453f : -INFINITY;
-      if (n_tiles >= 2) pv_wait((n_tiles - 2) & 1, (uint32_t)((n_tiles - 2) / 2 + 1));
-      pv_wait((n_tiles - 1) & 1, (uint32_t)((n_tiles - 1) / 2 + 1));
+      if (n_tiles >= 2) pv_wait(n_tiles - 2);
+      pv_wait(n_tiles - 1);
       const bool live = qi < M;
       float inv_l = l_sum > 0.f ? 1.0f / l_sum : 0.f;
       if (head_gate != nullptr && live) inv_l *= 1.0f / (1.0f + expf(-head_gate[(long long)qi * ldg + head]));
@@ -519,9 +528,10 @@ __global__ void __launch_bounds__(kFThreads, 1)
       }
     }
   }
+  __syncwarp();
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 5) tmem_dealloc(tmem_base, 512);
+  if (warp == 2) tmem_dealloc(tmem_base, 512);
 }
 
 __device__ __forceinline__ void fp8x16_to_bf16(const uint4& q, uint4& lo, uint4& hi) {
@@ -590,9 +600,9 @@ cudaError_t launch_gqa_core(const GqaDims& g, const void* q_raw, const void* k_r
   alignas(64) CUtensorMap tq, tk, tv;
   cudaError_t e = make_tmap_bf16_rows(&tq, q_rot, M, (long long)g.nh * g.d, kFQ);
   if (e != cudaSuccess) return e;
-  e = make_tmap_bf16_rows(&tk, k_bf, kv_len, row, kFK);
+  e = make_tmap_bf16_rows(&tk, k_bf, kv_len, row, g.d == 256 ? kFK<256> : kFK<128>);
   if (e != cudaSuccess) return e;
-  e = make_tmap_bf16_rows(&tv, v_bf, kv_len, row, kFK);
+  e = make_tmap_bf16_rows(&tv, v_bf, kv_len, row, g.d == 256 ? kFK<256> : kFK<128>);
   if (e != cudaSuccess) return e;
   const float sl2 = (1.0f / sqrtf((float)g.d)) * 1.4426950408889634f;
   dim3 grid((M + kFQ - 1) / kFQ, g.nh);
@@ -740,9 +750,9 @@ cudaError_t launch_mla_core(const MlaDims& m, void* q_full, const void* kv_a, co
   alignas(64) CUtensorMap tq, tk, tpe;
   e = make_tmap_bf16_rows(&tq, q_full, M, m.q_ld, kFQ);
   if (e != cudaSuccess) return e;
-  e = make_tmap_bf16_rows(&tk, kv_up, kv_len, up, kFK);
+  e = make_tmap_bf16_rows(&tk, kv_up, kv_len, up, kFK<128>);
   if (e != cudaSuccess) return e;
-  e = make_tmap_bf16_rows(&tpe, kpe_bf16, kv_len, m.rope, kFK);
+  e = make_tmap_bf16_rows(&tpe, kpe_bf16, kv_len, m.rope, kFK<128>);
   if (e != cudaSuccess) return e;
   GqaDims g{m.H, m.nh, m.nh, m.nope + m.rope, 0, 0, 0.f, m.eps};
   const float sl2 = sm_scale * 1.4426950408889634f;
@@ -772,9 +782,9 @@ cudaError_t launch_fmha_latent(const void* q, const void* kv_up, const void* kpe
   alignas(64) CUtensorMap tq, tk, tpe;
   cudaError_t e = make_tmap_bf16_rows(&tq, q, M, (long long)nh * 192, kFQ);
   if (e != cudaSuccess) return e;
-  e = make_tmap_bf16_rows(&tk, kv_up, kv_len, up, kFK);
+  e = make_tmap_bf16_rows(&tk, kv_up, kv_len, up, kFK<128>);
   if (e != cudaSuccess) return e;
-  e = make_tmap_bf16_rows(&tpe, kpe, kv_len, 64, kFK);
+  e = make_tmap_bf16_rows(&tpe, kpe, kv_len, 64, kFK<128>);
   if (e != cudaSuccess) return e;
   GqaDims g{0, nh, nh, 192, 0, 0, 0.f, 0.f};
   dim3 grid((M + kFQ - 1) / kFQ, nh);
@@ -811,9 +821,9 @@ cudaError_t launch_fmha_maps(const void* q, const void* k, const void* v, float*
   alignas(64) CUtensorMap tq, tk, tv;
   cudaError_t e = make_tmap_bf16_rows(&tq, q, M, (long long)nq * 128, kFQ);
   if (e != cudaSuccess) return e;
-  e = make_tmap_bf16_rows(&tk, k, kv_len, (long long)nkv * maps * 128, kFK);
+  e = make_tmap_bf16_rows(&tk, k, kv_len, (long long)nkv * maps * 128, dv == 256 ? kFK<256> : kFK<128>);
   if (e != cudaSuccess) return e;
-  e = make_tmap_bf16_rows(&tv, v, kv_len, (long long)nkv * dv, kFK);
+  e = make_tmap_bf16_rows(&tv, v, kv_len, (long long)nkv * dv, dv == 256 ? kFK<256> : kFK<128>);
   if (e != cudaSuccess) return e;
   GqaDims g{0, nq, nkv, 128, 0, 0, 0.f, 0.f};
   dim3 grid((M + kFQ - 1) / kFQ, nq);
