@@ -98,6 +98,9 @@ KB2SEQ_API int kb2_seq_residual_post_rms(float* x, const float* y1, float c1, co
  * scratch (fp32, 2 T Hk dk + 2 T H + T H dv + 4 elements, 16-byte aligned) selects the register-state kernels when dk is 32, 64 or
  * 128 and dv a multiple of 32; with scratch == NULL, or other sizes, one block per (sequence, head) keeps the state in shared memory
  * (a state too large for that is cut into slices of value columns, one block each; this needs scratch). */
+KB2SEQ_API int kb2_seq_delta_step(const float* proj, long long ldp, int g_off, int a_off, int b_off, int T, int H, int Hk, int dk, int dv, int K,
+                                  const float* taps, float* tail, const float* A_log, const float* dt_bias, const float* norm_w, float eps, float* state,
+                                  const int* slots, void* out, int dt_out, void* stream);
 KB2SEQ_API int kb2_seq_delta_rule(const float* conv, int C, const float* proj, long long ldp, int g_off, int a_off, int b_off, int T,
                                   int S, int H, int Hk, int dk, int dv, const float* A_log, const float* dt_bias, const float* norm_w,
                                   float eps, float* state, const int* cu, const int* slots, float* scratch, void* out, int dt_out,

@@ -42,28 +42,28 @@ __device__ __forceinline__ void pdl_enter_global(P&... p) {
   ((p = (P)__cvta_global_to_generic(__cvta_generic_to_global((const void*)p) + zero)), ...);
 }
 
-// The kernel in clusters of `cluster` blocks along y.
+// The kernel in clusters of `cluster` blocks.
 template <typename... P, typename... A>
-inline cudaError_t launch_pdl_clusters(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, unsigned cluster, A&&... args) {
+inline cudaError_t launch_pdl_clusters(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, dim3 cluster, A&&... args) {
   cudaLaunchAttribute at[2] = {};
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = 1;
-  at[1].val.clusterDim.y = cluster;
-  at[1].val.clusterDim.z = 1;
+  at[1].val.clusterDim.x = cluster.x;
+  at[1].val.clusterDim.y = cluster.y;
+  at[1].val.clusterDim.z = cluster.z;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = at;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  cfg.numAttrs = cluster.x * cluster.y * cluster.z > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 template <typename... P, typename... A>
 inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
-  return launch_pdl_clusters(kernel, grid, block, smem, s, 1u, std::forward<A>(args)...);
+  return launch_pdl_clusters(kernel, grid, block, smem, s, dim3(1, 1, 1), std::forward<A>(args)...);
 }
 
 }  // namespace kb2

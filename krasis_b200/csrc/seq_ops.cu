@@ -311,10 +311,10 @@ template <typename TA, typename TC, int KS, int kTiles, bool kShare>
 __global__ void __launch_bounds__(32 * GemvPiece<sizeof(TA) == 4, kTiles>::warps(KS))
     gemv_mma_kernel(const TA* __restrict__ A, long long lda, const bf16* __restrict__ B, long long ldb, TC* __restrict__ C, long long ldc, int M, int N, int K,
                     long long sA, long long sB, long long sC) {
-  kb2::pdl_enter(A, B, C);
   constexpr bool kFp32 = sizeof(TA) == 4;
   using P = GemvPiece<kFp32, kTiles>;
   constexpr int kRows = P::kRows, kWarps = P::warps(KS), kGroups = kWarps / KS, kW = 2 * kTiles;
+  kb2::pdl_enter(A, B, C);
   extern __shared__ __align__(16) uint8_t gemv_ring[];
   __shared__ float red[kWarps][8][kRows + 1];            // [warp][row of A][weight row], odd pitch
   A += (long long)blockIdx.z * sA;
@@ -484,7 +484,7 @@ static void launch_gemv_tiles(const void* A, long long lda, const void* B, long 
 #define KB2_GEMV(KSV, SHARE)                                                                                                                     \
   do {                                                                                                                                           \
     kb2::allow_smem<gemv_mma_kernel<TA, TC, KSV, kTiles, SHARE>>(Piece::warps(KSV) * Piece::kRing);                                              \
-    kb2::launch_pdl_clusters(gemv_mma_kernel<TA, TC, KSV, kTiles, SHARE>, grid, 32 * warps, smem, s, blocks, (const TA*)A, lda, (const bf16*)B,  \
+    kb2::launch_pdl_clusters(gemv_mma_kernel<TA, TC, KSV, kTiles, SHARE>, grid, 32 * warps, smem, s, dim3(1, blocks, 1), (const TA*)A, lda, (const bf16*)B,  \
                              ldb, (TC*)C, ldc, M, N, K, sA, sB, sC);                                                                             \
   } while (0)
   if (blocks > 1) KB2_GEMV(16, true);
@@ -2326,6 +2326,155 @@ __global__ void __launch_bounds__(256) delta_out_kernel(const float* __restrict_
   }
 }
 
+// ---- a step in which every sequence has one token, 128 key and 128 value channels: convolution, its tail, unit rows, gates, the recurrence and the read-out in
+// one launch.  Bound: latency (a block per (token, head) takes its state of 64 KB in and out, and six short phases follow one another); as five launches
+// (conv_silu, conv_tail, delta_prep, delta_rule_reg, delta_out) most of the time was theirs: 4 tokens x 32 / 16 heads 18.2 -> 6.9 us.  All sums in the order of
+// those, so that a token's numbers do not depend on what else is in its step.  A warp has a piece of 16 rows of the state, a lane four neighbouring columns.  The
+// heads of a key head are a cluster: each convolves q and k for itself, and the first one moves their tail on when all have read it.
+struct DeltaStep {
+  const float* proj;               // [T][ldp]: q | k | v ahead of the convolution, gates from g_off, decay and strength inputs from a_off and b_off
+  long long ldp;
+  int g_off, a_off, b_off, H, Hk;
+  const float *taps, *A_log, *dt_bias, *norm_w;
+  float eps;
+  float *tail, *state;             // [slots][channels][K - 1], [slots][H][128][128]
+  const int* slots;                // of token t's sequence
+  void* out;
+  int dt_out;
+};
+template <int K>
+__global__ void __launch_bounds__(256, 2) delta_step_kernel(const DeltaStep p) {
+  kb2::pdl_wait();
+  constexpr int D = 128, Q = D / kRegPieces;
+  __shared__ __align__(16) float qk[2 * D], vs[D], part[kRegPieces][D], os[kRegPieces][D];
+  __shared__ float gates[2];       // decay, strength
+  const long long t = blockIdx.y;
+  const int h = blockIdx.x, rep = p.H / p.Hk, hk = h / rep;
+  const int tid = threadIdx.x, lane = tid & 31, piece = tid >> 5;
+  const float* row = p.proj + t * p.ldp;
+  const long long slot = p.slots[t], C = 2ll * p.Hk * D + (long long)p.H * D;
+  // a channel of q or k per thread, and one of v for the first half
+  const long long c_qk = tid < D ? hk * D + tid : p.Hk * D + hk * D + (tid - D), c_v = 2ll * p.Hk * D + (long long)h * D + (tid & (D - 1));
+  float x[2][K], w[2][K];
+  const auto fetch = [&](long long c, float (&x)[K], float (&w)[K]) {
+    const float* tl = p.tail + (slot * C + c) * (K - 1);
+#pragma unroll
+    for (int j = 0; j < K - 1; ++j) x[j] = tl[j];
+    x[K - 1] = row[c] + 0.f;
+#pragma unroll
+    for (int j = 0; j < K; ++j) w[j] = p.taps[c * K + j];
+  };
+  fetch(c_qk, x[0], w[0]);
+  if (tid < D) fetch(c_v, x[1], w[1]);
+  float4* Sg = reinterpret_cast<float4*>(p.state + ((slot * p.H + h) * D + piece * Q) * D) + lane;
+  float4 S[Q], gz, nw;
+#pragma unroll
+  for (int i = 0; i < Q; ++i) S[i] = Sg[i * (D / 4)];
+  if (piece == 0) {
+    gz = *reinterpret_cast<const float4*>(row + p.g_off + (long long)h * D + lane * 4);
+    nw = *reinterpret_cast<const float4*>(p.norm_w + lane * 4);
+  }
+  const auto filtered = [&](const float (&x)[K], const float (&w)[K]) {
+    float acc = 0.f;
+#pragma unroll
+    for (int j = 0; j < K; ++j) acc = fmaf(w[j], x[j], acc);
+    return silu(acc);
+  };
+  const auto move_on = [&](long long c, const float (&x)[K]) {
+    float* tl = p.tail + (slot * C + c) * (K - 1);
+#pragma unroll
+    for (int j = 0; j < K - 1; ++j) tl[j] = x[j + 1];
+  };
+  qk[tid] = filtered(x[0], w[0]);
+  if (tid < D) {
+    vs[tid] = filtered(x[1], w[1]);
+    move_on(c_v, x[1]);
+  }
+  if (piece == kRegPieces - 1 && lane < 2)
+    gates[lane] = lane ? 1.f / (1.f + expf(-row[p.b_off + h])) : decay_of(p.A_log[h], row[p.a_off + h], p.dt_bias[h]);
+  if (rep > 1) kb2::cluster_sync_all();      // every head has read the tails of q and k
+  else __syncthreads();
+  if (h == hk * rep) move_on(c_qk, x[0]);
+  if (piece < 2) {                 // unit rows
+    float *r = qk + piece * D, a = 0.f;
+#pragma unroll
+    for (int i = 0; i < D / 32; ++i) a += r[lane + 32 * i] * r[lane + 32 * i];
+    a = warp_sum(a);
+    const float f = piece ? 1.f / sqrtf(a + 1e-6f) : (1.f / sqrtf((float)D)) / sqrtf(a + 1e-6f);
+#pragma unroll
+    for (int i = 0; i < D / 32; ++i) r[lane + 32 * i] *= f;
+  }
+  __syncthreads();
+  const float g = gates[0], b = gates[1];
+  const float4 *q4 = reinterpret_cast<const float4*>(qk + piece * Q), *k4 = reinterpret_cast<const float4*>(qk + D + piece * Q);
+  // the sums over a piece's rows i = 0, 4, 8, ..; 1, 5, ..; 2, ..; 3, .. of S times a row's number, for the lane's four columns
+  const auto dot = [](const float4 (&S)[Q], const float4* f4) {
+    float4 a[4] = {};
+#pragma unroll
+    for (int i = 0; i < Q / 4; ++i) {
+      const float4 f = f4[i];
+      const float fv[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        a[e].x = fmaf(S[4 * i + e].x, fv[e], a[e].x);
+        a[e].y = fmaf(S[4 * i + e].y, fv[e], a[e].y);
+        a[e].z = fmaf(S[4 * i + e].z, fv[e], a[e].z);
+        a[e].w = fmaf(S[4 * i + e].w, fv[e], a[e].w);
+      }
+    }
+    return make_float4((a[0].x + a[1].x) + (a[2].x + a[3].x), (a[0].y + a[1].y) + (a[2].y + a[3].y), (a[0].z + a[1].z) + (a[2].z + a[3].z),
+                       (a[0].w + a[1].w) + (a[2].w + a[3].w));
+  };
+  *reinterpret_cast<float4*>(&part[piece][lane * 4]) = dot(S, k4);
+  __syncthreads();
+  float4 u;
+  {
+    float4 pp[kRegPieces];
+#pragma unroll
+    for (int i = 0; i < kRegPieces; ++i) pp[i] = *reinterpret_cast<const float4*>(&part[i][lane * 4]);
+    const float4 v = *reinterpret_cast<const float4*>(&vs[lane * 4]);
+    const auto strength = [&](float p0, float p1, float p2, float p3, float p4, float p5, float p6, float p7, float vv) {
+      const float sk = ((p0 + p1) + (p2 + p3)) + ((p4 + p5) + (p6 + p7));
+      return b * (vv - g * sk);
+    };
+    u = make_float4(strength(pp[0].x, pp[1].x, pp[2].x, pp[3].x, pp[4].x, pp[5].x, pp[6].x, pp[7].x, v.x),
+                    strength(pp[0].y, pp[1].y, pp[2].y, pp[3].y, pp[4].y, pp[5].y, pp[6].y, pp[7].y, v.y),
+                    strength(pp[0].z, pp[1].z, pp[2].z, pp[3].z, pp[4].z, pp[5].z, pp[6].z, pp[7].z, v.z),
+                    strength(pp[0].w, pp[1].w, pp[2].w, pp[3].w, pp[4].w, pp[5].w, pp[6].w, pp[7].w, v.w));
+  }
+#pragma unroll
+  for (int i = 0; i < Q / 4; ++i) {
+    const float4 f = k4[i];
+    const float fv[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float4& s = S[4 * i + e];
+      s = make_float4(fmaf(fv[e], u.x, g * s.x), fmaf(fv[e], u.y, g * s.y), fmaf(fv[e], u.z, g * s.z), fmaf(fv[e], u.w, g * s.w));
+      Sg[(4 * i + e) * (D / 4)] = s;
+    }
+  }
+  *reinterpret_cast<float4*>(&os[piece][lane * 4]) = dot(S, q4);
+  __syncthreads();
+  if (piece == 0) {
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < kRegPieces; ++i) {
+      const float4 f = *reinterpret_cast<const float4*>(&os[i][lane * 4]);
+      o.x += f.x; o.y += f.y; o.z += f.z; o.w += f.w;
+    }
+    const float rstd = 1.f / sqrtf(warp_sum((o.x * o.x + o.y * o.y) + (o.z * o.z + o.w * o.w)) / (float)D + p.eps);
+    const auto finish = [&](float v, float z, float n) { return v * rstd * n * silu(z); };
+    const float4 r = make_float4(finish(o.x, gz.x, nw.x), finish(o.y, gz.y, nw.y), finish(o.z, gz.z, nw.z), finish(o.w, gz.w, nw.w));
+    const long long at = (t * p.H + h) * D + lane * 4;
+    if (p.dt_out == 0) {
+      *reinterpret_cast<float4*>((float*)p.out + at) = r;
+    } else {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(r.x, r.y), hi = __floats2bfloat162_rn(r.z, r.w);
+      *reinterpret_cast<uint2*>((bf16*)p.out + at) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+  }
+}
+
 }  // namespace kb2seq
 
 using namespace kb2seq;
@@ -2687,6 +2836,22 @@ KB2SEQ_API int kb2_seq_delta_rule_ch(const float* conv, int C, const float* beta
   if (gate_act < 0 || gate_act > 1) return failf(KB2SEQ_ERR_VALUE, "delta_rule_ch: bad argument");
   return delta_rule_launch(conv, C, beta_in, ldb, decay_in, lda, 1, gate_in, ldg, gate_act, T, S, H, Hk, dk, dv, A_log, dt_bias, norm_w, eps,
                            state, cu, slots, scratch, out, dt_out, stream);
+}
+
+// The convolution of proj's first channels, its tail and the delta rule with its gated read-out for a step of T sequences of one token each (row t: the
+// sequence with state slot slots[t]); see kb2_seq_conv_silu and kb2_seq_delta_rule.  dk and dv 128, H / Hk <= 8, 2 to 4 taps, 16-byte aligned rows.
+KB2SEQ_API int kb2_seq_delta_step(const float* proj, long long ldp, int g_off, int a_off, int b_off, int T, int H, int Hk, int dk, int dv, int K,
+                                  const float* taps, float* tail, const float* A_log, const float* dt_bias, const float* norm_w, float eps, float* state,
+                                  const int* slots, void* out, int dt_out, void* stream) {
+  if (!proj || !taps || !tail || !A_log || !dt_bias || !norm_w || !state || !slots || !out || T <= 0 || H <= 0 || Hk <= 0 || H % Hk || bad_dt(dt_out))
+    return failf(KB2SEQ_ERR_VALUE, "delta_step: bad argument");
+  if (dk != 128 || dv != 128 || K < 2 || K > 4 || H / Hk > 8 || T > 65535 || ldp % 4 || g_off % 4 || (((uintptr_t)proj | (uintptr_t)norm_w | (uintptr_t)state | (uintptr_t)out) & 15))
+    return failf(KB2SEQ_ERR_VALUE, "delta_step: 128 key and value channels, at most 8 heads per key head, 2 to 4 taps and 16-byte aligned rows");
+  const DeltaStep p{proj, ldp, g_off, a_off, b_off, H, Hk, taps, A_log, dt_bias, norm_w, eps, tail, state, slots, out, dt_out};
+  auto kern = K == 2 ? delta_step_kernel<2> : K == 3 ? delta_step_kernel<3> : delta_step_kernel<4>;
+  kb2::launch_pdl_clusters(kern, dim3(H, T), 256, 0, (cudaStream_t)stream, dim3(H / Hk, 1, 1), p);
+  SEQ_LAUNCHED();
+  return KB2SEQ_OK;
 }
 
 }  // extern "C"

@@ -323,6 +323,7 @@ class GatedDeltaMixer:
         # key sizes 32 / 64 / 128 with value sizes that are multiples of 32 keep the state in registers; others in shared memory
         self.register_state_kernel = dim in (32, 64, 128) and vdim % 32 == 0
         self.tile_min_portion = TILE_PORTION
+        self.one_launch = dim == 128 and vdim == 128 and 2 <= self.K <= 4 and heads // kv_heads <= 8 and self.g_off % 4 == 0 and self.norm.data_ptr() % 16 == 0
 
     def register_state(self, pool):
         """(conv tail [slots, C, taps - 1], recurrent state [slots, H, dk, dv]) in a RecurrentStatePool."""
@@ -332,6 +333,12 @@ class GatedDeltaMixer:
         lib, T = ops.load(), h.shape[0]
         proj = lin(h, self.w_in, torch.float32)
         s = stream_of(h)
+        if self.one_launch and T == tb.S and proj.stride(0) % 4 == 0 and all(n == 1 for _, n, _, _ in tb.layout):      # every sequence decodes
+            o = torch.empty((T, self.H * self.dv), dtype=self.dtype, device=h.device)
+            ops.check(lib.kb2_seq_delta_step(proj.data_ptr(), proj.stride(0), self.g_off, self.a_off, self.b_off, T, self.H, self.Hk, self.dk, self.dv, self.K,
+                                             self.taps.data_ptr(), tail.data_ptr(), self.A_log.data_ptr(), self.dt_bias.data_ptr(), self.norm.data_ptr(),
+                                             self.eps, state.data_ptr(), tb.slots.data_ptr(), o.data_ptr(), ops.dt_code(self.dtype), s))
+            return lin(o, self.w_o, torch.float32)
         conv = torch.empty((T, self.C), dtype=torch.float32, device=h.device)
         ops.check(lib.kb2_seq_conv_silu(proj.data_ptr(), proj.stride(0), T, tb.S, self.C, self.K, self.taps.data_ptr(), tail.data_ptr(),
                                         tb.seq_of.data_ptr(), tb.cu.data_ptr(), tb.slots.data_ptr(), conv.data_ptr(), s))

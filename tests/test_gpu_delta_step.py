@@ -1,0 +1,38 @@
+"""Steps in which every sequence has one token: the one-launch form of the delta mixer gives what the five launches of other steps give, bit for bit."""
+import pytest
+import torch
+
+from krasis_b200 import seqops
+from krasis_b200.mixers import GatedDeltaMixer
+
+pytestmark = pytest.mark.gpu
+
+
+# one, two and three heads per key head (the last pair is half empty), two to four taps
+@pytest.mark.parametrize("H,Hk,K", [(4, 4, 4), (8, 4, 4), (6, 2, 3), (2, 2, 2), (32, 16, 4)])
+@pytest.mark.parametrize("T", [1, 5])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_same_as_separate_launches(H, Hk, K, T, dtype):
+    g = torch.Generator().manual_seed(H + K + T)
+    W, n, slots = 256, 128, 8
+    r = lambda *s, sd=1.0: torch.randn(*s, generator=g) * sd  # noqa: E731
+    w = {"g": r(H * n, W, sd=W ** -0.5), "a": r(H, W, sd=W ** -0.5), "b": r(H, W, sd=W ** -0.5), "A_log": r(H), "dt_bias": r(H) - 3.0,
+         "norm": 1.0 + 0.1 * r(n), "o": r(W, H * n, sd=(H * n) ** -0.5)}
+    for nm, rows in (("q", Hk * n), ("k", Hk * n), ("v", H * n)):
+        w[nm], w[nm + "_conv"] = r(rows, W, sd=W ** -0.5), r(rows, K, sd=0.5)
+    m = GatedDeltaMixer(w, H, Hk, n, n, K, 1e-5, dtype, "cuda")
+    order = [5, 0, 7, 2, 3][:T]
+    x = r(3, T, W).cuda().to(dtype)
+    ends = []
+    for one in (True, False):
+        assert m.one_launch
+        m.one_launch = one
+        tail, state = r(slots, m.C, K - 1).cuda() * 0 + 0.3, torch.full((slots, H, n, n), 0.01, device="cuda")
+        outs = [m.forward(x[i], seqops.StepTables([([0], i, s, [0]) for s in order], "cuda"), tail, state) for i in range(3)]
+        ends.append(outs + [tail, state])
+        m.one_launch = True
+    for a, b in zip(*ends):
+        assert torch.equal(a, b)
+    assert torch.isfinite(ends[0][0]).all()
+    untouched = [s for s in range(slots) if s not in order]
+    assert (ends[0][-1][untouched] == 0.01).all() and (ends[0][-2][untouched] == 0.3).all()
