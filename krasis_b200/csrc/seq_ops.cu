@@ -908,7 +908,7 @@ __global__ void side_gate_kernel(const float* __restrict__ g, const void* __rest
 // ------------------------------------------------------------------------------------------------ latent attention
 // proj [T, ldp] fp32 = [q (H x (dn + dr)) | latent (r) | shared rotated key (dr)].  Per token: RMS-normed latent and rotated key part
 // go to the page the token's position maps to; the query's rotated parts are rotated in place.
-__global__ void __launch_bounds__(128) latent_prep_kernel(float* __restrict__ proj, long long ldp, int H, int dn, int dr, int r,
+__global__ void __launch_bounds__(512) latent_prep_kernel(float* __restrict__ proj, long long ldp, int H, int dn, int dr, int r,
                                                           const float* __restrict__ cw, float eps, const double* __restrict__ freq,
                                                           int rot_dims, float amp, const int* __restrict__ positions,
                                                           const int* __restrict__ seq_of, const int* __restrict__ pages, int max_pages,
@@ -922,7 +922,8 @@ __global__ void __launch_bounds__(128) latent_prep_kernel(float* __restrict__ pr
   const long long slot = (long long)pages[(long long)seq_of[t] * max_pages + pos / page_size] * page_size + pos % page_size;
   const float* lat = lat_rows != nullptr ? lat_rows + t * ldl : p + (long long)H * (dn + dr);
   float ss = 0.f;
-  for (int d = threadIdx.x; d < r; d += blockDim.x) ss += lat[d] * lat[d];
+  if (threadIdx.x < 128)                     // the first four warps' sum, whatever else the block has
+    for (int d = threadIdx.x; d < r; d += 128) ss += lat[d] * lat[d];
   ss = block_sum(ss, red);
   const float rstd = 1.f / sqrtf(ss / (float)r + eps);
   for (int d = threadIdx.x; d < r; d += blockDim.x) st_dt(ckv, dt_cache, slot * r + d, lat[d] * rstd * cw[d]);
@@ -955,8 +956,11 @@ __global__ void __launch_bounds__(128) latent_prep_kernel(float* __restrict__ pr
 //   scores    every warp takes an eighth of the dimensions for all HG heads: one 16-byte read of a key row serves HG dot products, whose
 //             pieces meet in shared memory
 //   values    a thread owns NC columns for all HG heads: one read of a latent element serves HG sums
+// Bound where few tokens decode: latency, a chain of position, page, key rows and four phases on them.  Loads of a phase go out together, and the key range is
+// cut into pieces of 8 keys and more, so that short contexts reach all SMs, too (4 tokens x 16 heads, 116 keys, from HBM: pieces of 32 18.6 us, now 11.4).
 // gate [T, ldg] (may be null): head h's output is multiplied by sigmoid(gate[t, h]); it commutes with the value up-projection.
 constexpr int kAttnThreads = 256, kAttnAcc = 16, kAttnKT = 32, kAttnWarps = kAttnThreads / 32;
+constexpr int kAttnPiece = 8;              // keys of a piece are a multiple of this
 __device__ __forceinline__ float head_gate(const float* __restrict__ gate, long long ldg, long long t, int h) {
   return gate != nullptr ? 1.f / (1.f + expf(-gate[t * ldg + h])) : 1.f;
 }
@@ -971,7 +975,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) latent_window_attn_kernel(
     const void* __restrict__ ckv, const void* __restrict__ kr, int dt_cache, const int* __restrict__ positions,
     const int* __restrict__ seq_of, const int* __restrict__ pages, int max_pages, int page_size, const float* __restrict__ sinks,
     float scale, int window, float* __restrict__ out, const int* __restrict__ cu, int skip_from, int nsplit,
-    float* __restrict__ part_acc, float* __restrict__ part_ml, const float* __restrict__ gate, long long ldg) {
+    float* __restrict__ part_acc, float* __restrict__ part_ml, const float* __restrict__ gate, long long ldg, bool vec_q) {
   kb2::pdl_enter(q_abs, proj, ckv, kr, positions, seq_of, pages, sinks, out, cu, part_acc, part_ml, gate);
   static_assert(HG <= kAttnWarps, "a warp per head runs the softmax");
   constexpr int KT = kAttnKT;
@@ -994,19 +998,45 @@ __global__ void __launch_bounds__(kAttnThreads, 2) latent_window_attn_kernel(
   const int nh = min(HG, H - h0);
   const int pos = positions[t], seq = seq_of[t];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = tid; i < HG * QP; i += kAttnThreads) {
-    const int hh = i / QP, d = i - hh * QP;
-    float v = 0.f;
-    if (hh < nh && d < D) v = d < r ? q_abs[(t * H + h0 + hh) * r + d] : proj[t * ldp + (long long)(h0 + hh) * (dn + dr) + dn + (d - r)];
-    qs[i] = v;
+  // nsplit > 1: block z takes the z-th piece of the token's key range and leaves an unnormalised partial result (running max, sum,
+  // weighted latents) for latent_attn_combine_kernel; the sink belongs to piece 0
+  const int z = blockIdx.z;
+  const int j_lo = max(0, pos - window + 1);
+  int j_begin = j_lo, j_end = pos;
+  if (nsplit > 1) {
+    const int piece = (((pos - j_lo + 1) + nsplit - 1) / nsplit + kAttnPiece - 1) / kAttnPiece * kAttnPiece;
+    j_begin = j_lo + z * piece;
+    j_end = min(pos, j_begin + piece - 1);
+  }
+  const auto row_of = [&](int j) { return (long long)pages[(long long)seq * max_pages + j / page_size] * page_size + j % page_size; };
+  if (tid < KT && j_begin + tid <= j_end) krow[tid] = row_of(j_begin + tid);      // of the first tile, under way together with the query
+  if (vec_q) {                            // sizes, strides and pointers in units of four numbers: five loads of a thread in flight
+    constexpr int kAhead = 5;
+    for (int base = tid; base < HG * n4; base += kAhead * kAttnThreads) {
+      float4 v[kAhead];
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        const int u = base + i * kAttnThreads, hh = u / n4, d = (u - hh * n4) * 4;
+        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (hh < nh)
+          v[i] = *reinterpret_cast<const float4*>(d < r ? q_abs + (t * H + h0 + hh) * r + d : proj + t * ldp + (long long)(h0 + hh) * (dn + dr) + dn + (d - r));
+      }
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i)
+        if (base + i * kAttnThreads < HG * n4) reinterpret_cast<float4*>(qs)[base + i * kAttnThreads] = v[i];
+    }
+  } else {
+    for (int i = tid; i < HG * QP; i += kAttnThreads) {
+      const int hh = i / QP, d = i - hh * QP;
+      float v = 0.f;
+      if (hh < nh && d < D) v = d < r ? q_abs[(t * H + h0 + hh) * r + d] : proj[t * ldp + (long long)(h0 + hh) * (dn + dr) + dn + (d - r)];
+      qs[i] = v;
+    }
   }
   for (int i = tid; i < KT * (DP - D); i += kAttnThreads) {      // the rows' padding stays zero: tiles write D numbers per row only
     const int k = i / (DP - D);
     kt[k * DP + D + i - k * (DP - D)] = 0.f;
   }
-  // nsplit > 1: block z takes the z-th piece of the token's key range and leaves an unnormalised partial result (running max, sum,
-  // weighted latents) for latent_attn_combine_kernel; the sink belongs to piece 0
-  const int z = blockIdx.z;
   if (tid < HG) {
     const bool sk = z == 0 && sinks != nullptr && tid < nh;       // no sinks: an ordinary softmax over the keys
     m_run[tid] = sk ? sinks[h0 + tid] : -INFINITY;
@@ -1017,31 +1047,35 @@ __global__ void __launch_bounds__(kAttnThreads, 2) latent_window_attn_kernel(
   for (int c = 0; c < NC; ++c)
 #pragma unroll
     for (int hh = 0; hh < HG; ++hh) acc[c][hh] = 0.f;
-  const int j_lo = max(0, pos - window + 1);
-  int j_begin = j_lo, j_end = pos;
-  if (nsplit > 1) {
-    const int piece = (((pos - j_lo + 1) + nsplit - 1) / nsplit + KT - 1) / KT * KT;
-    j_begin = j_lo + z * piece;
-    j_end = min(pos, j_begin + piece - 1);
-  }
   const int seg = (n4 + kAttnWarps - 1) / kAttnWarps, u_lo = min(n4, warp * seg), u_hi = min(n4, u_lo + seg);
   for (int j0 = j_begin; j0 <= j_end; j0 += KT) {
     const int nk = min(KT, j_end - j0 + 1);
     __syncthreads();
-    if (tid < nk) {
-      const int j = j0 + tid;
-      krow[tid] = (long long)pages[(long long)seq * max_pages + j / page_size] * page_size + j % page_size;
+    if (j0 > j_begin) {
+      if (tid < nk) krow[tid] = row_of(j0 + tid);
+      __syncthreads();
     }
-    __syncthreads();
     if (dt_cache == 1 && (r & 7) == 0 && (dr & 7) == 0) {
       const int D8 = D >> 3;
-      for (int i = tid; i < nk * D8; i += kAttnThreads) {
-        const int k = i / D8, d = (i - k * D8) << 3;
-        const bf16* src = d < r ? (const bf16*)ckv + krow[k] * r + d : (const bf16*)kr + krow[k] * dr + (d - r);
-        float f[8];
-        unpack8(*reinterpret_cast<const uint4*>(src), f);
-        *reinterpret_cast<float4*>(kt + k * DP + d) = make_float4(f[0], f[1], f[2], f[3]);
-        *reinterpret_cast<float4*>(kt + k * DP + d + 4) = make_float4(f[4], f[5], f[6], f[7]);
+      for (int base = tid; base < nk * D8; base += 4 * kAttnThreads) {      // four loads of a thread in flight
+        uint4 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int i = base + j * kAttnThreads;
+          if (i >= nk * D8) continue;
+          const int k = i / D8, d = (i - k * D8) << 3;
+          v[j] = *reinterpret_cast<const uint4*>(d < r ? (const bf16*)ckv + krow[k] * r + d : (const bf16*)kr + krow[k] * dr + (d - r));
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int i = base + j * kAttnThreads;
+          if (i >= nk * D8) continue;
+          const int k = i / D8, d = (i - k * D8) << 3;
+          float f[8];
+          unpack8(v[j], f);
+          *reinterpret_cast<float4*>(kt + k * DP + d) = make_float4(f[0], f[1], f[2], f[3]);
+          *reinterpret_cast<float4*>(kt + k * DP + d + 4) = make_float4(f[4], f[5], f[6], f[7]);
+        }
       }
     } else {
       for (int i = tid; i < nk * D; i += kAttnThreads) {
@@ -1050,15 +1084,16 @@ __global__ void __launch_bounds__(kAttnThreads, 2) latent_window_attn_kernel(
       }
     }
     __syncthreads();
-    // scores: a lane per key, a piece of the dimensions per warp, all heads of the group
+    // scores: a lane per key, a piece of the dimensions per warp, all heads of the group; of up to 8 or 16 keys four or two lanes share one
     {
+      const int keys = nk <= 8 ? 8 : nk <= 16 ? 16 : 32, key = lane & (keys - 1), step = 32 / keys;
       float s[HG];
 #pragma unroll
       for (int hh = 0; hh < HG; ++hh) s[hh] = 0.f;
-      if (lane < nk) {
-        const float4* kk = reinterpret_cast<const float4*>(kt + lane * DP);
+      if (key < nk) {
+        const float4* kk = reinterpret_cast<const float4*>(kt + key * DP);
         const float4* qq = reinterpret_cast<const float4*>(qs);
-        for (int u = u_lo; u < u_hi; ++u) {
+        for (int u = u_lo + lane / keys; u < u_hi; u += step) {
           const float4 kv = kk[u];
 #pragma unroll
           for (int hh = 0; hh < HG; ++hh) {
@@ -1070,6 +1105,9 @@ __global__ void __launch_bounds__(kAttnThreads, 2) latent_window_attn_kernel(
           }
         }
       }
+      for (int o = keys; o < 32; o <<= 1)
+#pragma unroll
+        for (int hh = 0; hh < HG; ++hh) s[hh] += __shfl_xor_sync(0xffffffffu, s[hh], o);
 #pragma unroll
       for (int hh = 0; hh < HG; ++hh) sp[(warp * HG + hh) * KT + lane] = s[hh];
     }
@@ -2571,7 +2609,7 @@ KB2SEQ_API int kb2_seq_latent_prep(float* proj, long long ldp, int T, int H, int
   if (!proj || !cw || !freq || !positions || !seq_of || !pages || !ckv || !kr || T <= 0 || H <= 0 || dn < 0 || dr < 0 || r <= 0 ||
       rot_dims < 0 || rot_dims > dr || (rot_dims & 1) || page_size <= 0 || max_pages <= 0 || bad_dt(dt_cache))
     return failf(KB2SEQ_ERR_VALUE, "latent_prep: bad argument");
-  kb2::launch_pdl(latent_prep_kernel, T, 128, 0, (cudaStream_t)stream, proj, ldp, H, dn, dr, r, cw, eps, freq, rot_dims, amp, positions, seq_of, pages,
+  kb2::launch_pdl(latent_prep_kernel, T, 512, 0, (cudaStream_t)stream, proj, ldp, H, dn, dr, r, cw, eps, freq, rot_dims, amp, positions, seq_of, pages,
                                                           max_pages, page_size, ckv, kr, dt_cache, lat, ldl);
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
@@ -2595,13 +2633,14 @@ KB2SEQ_API int kb2_seq_latent_window_attn(const float* q_abs, const float* proj,
   const size_t smem = attn_smem_floats(HG, D) * 4;
   if (smem > 200 * 1024) return failf(KB2SEQ_ERR_VALUE, "latent_window_attn: latent + rotated size %d too large", D);
   const dim3 grid(T, (H + HG - 1) / HG, nsplit);
+  const bool vec_q = r % 4 == 0 && dr % 4 == 0 && dn % 4 == 0 && ldp % 4 == 0 && !(((uintptr_t)q_abs | (uintptr_t)proj) & 15);
 #define KB2_LA(HGV, NCV)                                                                                                                      \
   case HGV * 32 + NCV: {                                                                                                                      \
     if (smem > 48 * 1024)                                                                                                                     \
       SEQ_CUDA(cudaFuncSetAttribute(latent_window_attn_kernel<HGV, NCV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));            \
     kb2::launch_pdl(latent_window_attn_kernel<HGV, NCV>, grid, kAttnThreads, smem, (cudaStream_t)stream,                                                    \
         q_abs, proj, ldp, H, dn, dr, r, ckv, kr, dt_cache, positions, seq_of, pages, max_pages, page_size, sinks, scale, window, out, cu,     \
-        skip_from, nsplit, part_acc, part_ml, gate, ldg);                                                                                     \
+        skip_from, nsplit, part_acc, part_ml, gate, ldg, vec_q);                                                                              \
     break;                                                                                                                                    \
   }
   switch (HG * 32 + NC) {

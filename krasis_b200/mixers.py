@@ -276,7 +276,7 @@ class WindowLatentAttention:
                 # few tokens (decoding): each token's keys are cut into pieces so that the whole GPU works on them
                 blocks = n * ((H + 7) // 8)
                 max_keys = max(min(self.window, tb.layout[i][2] + tb.layout[i][1]) for i in seqs)
-                nsplit = max(1, min(296 // max(blocks, 1), (max_keys + 31) // 32, 64))
+                nsplit = max(1, min(296 // max(blocks, 1), (max_keys + 7) // 8, 64))
                 part_acc = torch.empty((n, nsplit, H, self.r), dtype=torch.float32, device=h.device) if nsplit > 1 else None
                 part_ml = torch.empty((n, nsplit, H, 2), dtype=torch.float32, device=h.device) if nsplit > 1 else None
                 ops.check(lib.kb2_seq_latent_window_attn(q_abs.data_ptr(), _row(proj, r0), ldp, n, H, self.dn, self.dr, self.r,
