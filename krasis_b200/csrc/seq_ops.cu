@@ -625,6 +625,7 @@ __global__ void __launch_bounds__(256) residual_norm_vec_kernel(float* __restric
                                                                 const float* __restrict__ bb, void* __restrict__ h, int dt_h, int W, float eps,
                                                                 const float* __restrict__ y2) {
   kb2::pdl_enter(x, y, wa, ba, x0, wb, bb, h, y2);
+  kb2::pdl_trigger();
   __shared__ float red[4][8];
   const long long base = (long long)blockIdx.x * W;
   const int tid = threadIdx.x;
@@ -881,6 +882,7 @@ __global__ void __launch_bounds__(256) act_mul_f32x4_kernel(const float* __restr
 // bf16 in and out, F a multiple of 8: 16-byte accesses
 __global__ void act_mul_bf16x8_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, int F) {
   kb2::pdl_enter(in, out);
+  kb2::pdl_trigger();
   const long long t = blockIdx.y;
   const int f = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (f >= F) return;
@@ -897,6 +899,7 @@ __global__ void act_mul_bf16x8_kernel(const bf16* __restrict__ in, bf16* __restr
 __global__ void side_gate_kernel(const float* __restrict__ g, const void* __restrict__ table, int dt_table, long long table_ld,
                                  const int* __restrict__ tokens, int col0, int dim, long long T, void* __restrict__ out, int dt_out) {
   kb2::pdl_enter(g, table, tokens, out);
+  kb2::pdl_trigger();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= T * dim) return;
   const long long t = i / dim;
@@ -1007,6 +1010,13 @@ __global__ void __launch_bounds__(kAttnThreads, 2) latent_window_attn_kernel(
     const int piece = (((pos - j_lo + 1) + nsplit - 1) / nsplit + kAttnPiece - 1) / kAttnPiece * kAttnPiece;
     j_begin = j_lo + z * piece;
     j_end = min(pos, j_begin + piece - 1);
+  }
+  if (j_begin > j_end) {                  // no keys: the join takes the pieces ahead of the first empty one (a whole range always has its own position)
+    if (tid < nh) {
+      part_ml[((t * nsplit + z) * H + h0 + tid) * 2] = -INFINITY;
+      part_ml[((t * nsplit + z) * H + h0 + tid) * 2 + 1] = 0.f;
+    }
+    return;
   }
   const auto row_of = [&](int j) { return (long long)pages[(long long)seq * max_pages + j / page_size] * page_size + j % page_size; };
   if (tid < KT && j_begin + tid <= j_end) krow[tid] = row_of(j_begin + tid);      // of the first tile, under way together with the query
@@ -1191,13 +1201,13 @@ __global__ void __launch_bounds__(kAttnThreads, 2) latent_window_attn_kernel(
   }
 }
 
-// out[t, h, :] = sum_z w_z acc_z / sum_z w_z l_z with w_z = exp(m_z - max_z m_z); pieces without keys have l_z = 0, hold zeros and get the
-// weight 0, so that no load waits for a branch
+// out[t, h, :] = sum_z w_z acc_z / sum_z w_z l_z with w_z = exp(m_z - max_z m_z); pieces without keys come last and have l_z = 0
 __global__ void __launch_bounds__(512) latent_attn_combine_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
                                                                   int H, int r, int nsplit, float* __restrict__ out,
                                                                   const int* __restrict__ seq_of, const int* __restrict__ cu, int skip_from,
                                                                   const float* __restrict__ gate, long long ldg) {
   kb2::pdl_enter(part_acc, part_ml, out, seq_of, cu, gate);
+  kb2::pdl_trigger();
   extern __shared__ float wz[];           // [nsplit]
   __shared__ float red[32];
   const long long t = blockIdx.x;
@@ -1208,9 +1218,12 @@ __global__ void __launch_bounds__(512) latent_attn_combine_kernel(const float* _
   }
   auto ml = [&](int z) { return *reinterpret_cast<const float2*>(part_ml + ((t * nsplit + z) * H + h) * 2); };
   float M = -INFINITY;
-  for (int z = threadIdx.x; z < nsplit; z += blockDim.x) {
-    const float2 v = ml(z);
+  int there = 0;
+  for (int z0 = 0; z0 < nsplit; z0 += blockDim.x) {
+    const int z = z0 + threadIdx.x;
+    const float2 v = z < nsplit ? ml(z) : make_float2(0.f, 0.f);
     if (v.y > 0.f) M = fmaxf(M, v.x);
+    there += __syncthreads_count(v.y > 0.f);
   }
   M = warp_max(M);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = M;
@@ -1230,7 +1243,7 @@ __global__ void __launch_bounds__(512) latent_attn_combine_kernel(const float* _
   for (int d = threadIdx.x; d < r; d += blockDim.x) {
     float v = 0.f;
 #pragma unroll 8
-    for (int z = 0; z < nsplit; ++z) v = fmaf(wz[z], pa[z * step + d], v);
+    for (int z = 0; z < there; ++z) v = fmaf(wz[z], pa[z * step + d], v);
     out[(t * H + h) * r + d] = v * f;
   }
 }
@@ -2383,6 +2396,7 @@ struct DeltaStep {
 template <int K>
 __global__ void __launch_bounds__(256, 2) delta_step_kernel(const DeltaStep p) {
   kb2::pdl_wait();
+  kb2::pdl_trigger();
   constexpr int D = 128, Q = D / kRegPieces;
   __shared__ __align__(16) float qk[2 * D], vs[D], part[kRegPieces][D], os[kRegPieces][D];
   __shared__ float gates[2];       // decay, strength

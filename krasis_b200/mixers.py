@@ -275,7 +275,8 @@ class WindowLatentAttention:
                 o_lat = torch.empty((n, H, self.r), dtype=torch.float32, device=h.device)
                 # few tokens (decoding): each token's keys are cut into pieces so that the whole GPU works on them
                 blocks = n * ((H + 7) // 8)
-                max_keys = max(min(self.window, tb.layout[i][2] + tb.layout[i][1]) for i in seqs)
+                # by the room of the page lists, in eights as captured steps have them: steps that are replayed cut as others do
+                max_keys = min(self.window, (tb.max_pages + 7) // 8 * 8 * page_size)
                 nsplit = max(1, min(296 // max(blocks, 1), (max_keys + 7) // 8, 64))
                 part_acc = torch.empty((n, nsplit, H, self.r), dtype=torch.float32, device=h.device) if nsplit > 1 else None
                 part_ml = torch.empty((n, nsplit, H, 2), dtype=torch.float32, device=h.device) if nsplit > 1 else None
