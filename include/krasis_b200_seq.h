@@ -142,6 +142,15 @@ KB2SEQ_API int kb2_seq_head_kv_prep(float* proj, long long ldp, int T, int H, in
                                     const int* seq_of, const int* pages, int max_pages, int page_size, void* kc, void* vc, int dt_cache,
                                     int norm_whole, int rot_half, const double* vfreq, float amp, int v_is_k, void* stream);
 
+/* Everything between the two products of an attention layer whose heads have one map and keys and values of their own, without gates, chunks or pooled blocks:
+ * head_kv_prep, then per run of sequences portion_rows and `fmha` (the core library's kb2_fmha_maps_bf16; its error e comes back as 100 + e) for portions of
+ * min_long tokens and more (0: none), paged_attn and attn_finish for the others.  layout (host): [S][4] first row, tokens, first position, pages. */
+KB2SEQ_API size_t kb2_seq_attention_step_workspace(const int* layout, int S, int H, int G, int d, int dv, int window, int min_long);
+KB2SEQ_API int kb2_seq_attention_step(float* proj, long long ldp, const int* layout, int S, int T, int H, int G, int d, int dv, const float* bias,
+                                      const float* qw, const float* kw, float eps, const double* freq, int rot_dims, const int* positions, const int* seq_of,
+                                      const int* pages, int max_pages, int page_size, void* kc, void* vc, int dt_cache, int norm_whole, int rot_half, float amp,
+                                      int v_is_k, float scale, int window, float softcap, const float* sinks, const float* slopes, int min_long,
+                                      void* fmha, void* work, size_t work_bytes, void* out, int dt_out, int device, void* stream);
 /* The bf16 operands of a portion's attention in one pass: cache rows `first` .. first + keys - 1 of a sequence (its page list `pages`, which holds
  * them all) of two bf16 caches with rows of wa and wb numbers (multiples of 8), side by side in a [keys][wa] and b [keys][wb]; and rows of nq fp32
  * numbers (a multiple of 8, ldq apart) rounded to bf16 in qb [n][nq].  Caches and outputs 16-byte aligned. */

@@ -1013,6 +1013,41 @@ __global__ void __launch_bounds__(256) moe_combine_vec_kernel(const float* __res
 
 using namespace kb2seq;
 
+namespace {
+using FmhaMaps = int (*)(const void*, const void*, const void*, void*, int, int, int, int, int, int, int, float, float, int, const float*, float*, const float*,
+                         int, void*);
+struct AttnSeq {
+  int row, n, start, pages;        // first row, tokens, first position, pages in its list
+};
+// Neighbouring sequences of one kind, long portions (at least min_long tokens; 0: none is long) or others.
+template <typename F> int attn_runs(const AttnSeq* seq, int S, int min_long, F each) {
+  for (int i = 0, j; i < S; i = j) {
+    const bool fast = min_long > 0 && seq[i].n >= min_long;
+    for (j = i + 1; j < S && (min_long > 0 && seq[j].n >= min_long) == fast; ++j) {}
+    const int rows = seq[j - 1].row + seq[j - 1].n - seq[i].row;
+    if (rows > 0)
+      if (const int rc = each(fast, i, j, seq[i].row, rows)) return rc;
+  }
+  return KB2SEQ_OK;
+}
+size_t up16(size_t n) { return (n + 15) / 16 * 16; }
+// few tokens (decoding): each token's keys are cut into pieces so that the whole GPU works on them
+int attn_pieces(const AttnSeq* seq, int i, int j, int rows, int G, int window) {
+  int most = 1;
+  for (int q = i; q < j; ++q) most = std::max(most, std::min(window, seq[q].start + seq[q].n));
+  return std::max(1, std::min({296 / std::max(rows * G, 1), (most + 31) / 32, 64}));
+}
+struct AttnWork {                  // of a long portion: its keys, values and queries in bf16
+  size_t k, v, q;
+  AttnWork(const AttnSeq& s, int H, int G, int d, int dv, int window) {
+    const size_t keys = (size_t)(s.start + s.n - std::max(0, s.start - window + 1));
+    k = up16(keys * G * d * 2);
+    v = up16(keys * G * dv * 2);
+    q = up16((size_t)s.n * H * d * 2);
+  }
+};
+}  // namespace
+
 extern "C" {
 
 KB2SEQ_API int kb2_seq_head_kv_prep(float* proj, long long ldp, int T, int H, int G, int M, int d, int dv, const float* bias,
@@ -1079,7 +1114,7 @@ KB2SEQ_API int kb2_seq_paged_attn(const float* proj, long long ldp, int T, int H
   while (RB > 1 && (RB * dv > kPAThreads * kPAAcc || smem_of(RB) > 200 * 1024)) RB = (RB + 1) / 2;
   const size_t smem = smem_of(RB);
   if (smem > 200 * 1024) return failf(KB2SEQ_ERR_VALUE, "paged_attn: head sizes %d / %d too large", M * d, dv);
-  if (smem > 48 * 1024) SEQ_CUDA(cudaFuncSetAttribute(paged_attn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024) SEQ_CUDA(kb2::allow_smem<paged_attn_kernel>(200 * 1024));
   const int nrb = (R + RB - 1) / RB;
   if ((long long)G * nrb > 65535) return failf(KB2SEQ_ERR_VALUE, "paged_attn: too many heads");
   kb2::launch_pdl(paged_attn_kernel, dim3(T, G * nrb, nsplit), kPAThreads, smem, (cudaStream_t)stream, 
@@ -1118,6 +1153,73 @@ KB2SEQ_API int kb2_seq_attn_finish(const float* a, const float* part_acc, const 
 #undef KB2_FIN
   SEQ_LAUNCHED();
   return KB2SEQ_OK;
+}
+
+
+// ---- everything between an attention layer's two products, in one call: a mixed step is seven launches, and what a host needs for each of them from Python
+// took longer than the kernels (512 tokens beside three decoded ones: 93 us for 66).
+KB2SEQ_API size_t kb2_seq_attention_step_workspace(const int* layout, int S, int H, int G, int d, int dv, int window, int min_long) {
+  const AttnSeq* seq = reinterpret_cast<const AttnSeq*>(layout);
+  size_t most = 16;
+  attn_runs(seq, S, min_long, [&](bool fast, int i, int j, int, int rows) {
+    if (fast) {
+      for (int q = i; q < j; ++q) {
+        const AttnWork w(seq[q], H, G, d, dv, window);
+        most = std::max(most, w.k + w.v + w.q);
+      }
+    } else {
+      const int pieces = attn_pieces(seq, i, j, rows, G, window);
+      most = std::max(most, (size_t)rows * H * (pieces > 1 ? (size_t)pieces * (dv + 2) : dv) * 4);
+    }
+    return KB2SEQ_OK;
+  });
+  return most;
+}
+
+// Heads of one map, of the layer's own keys and values, without gates, chunks or pooled blocks.  proj [T][ldp] fp32 = q | k | v; layout (host): [S][4] first row,
+// tokens, first position, pages.  Portions of min_long tokens and more run on `fmha` (kb2_fmha_maps_bf16 of the core library), whose error code e comes back as 100 + e.
+KB2SEQ_API int kb2_seq_attention_step(float* proj, long long ldp, const int* layout, int S, int T, int H, int G, int d, int dv, const float* bias,
+                                      const float* qw, const float* kw, float eps, const double* freq, int rot_dims, const int* positions, const int* seq_of,
+                                      const int* pages, int max_pages, int page_size, void* kc, void* vc, int dt_cache, int norm_whole, int rot_half, float amp,
+                                      int v_is_k, float scale, int window, float softcap, const float* sinks, const float* slopes, int min_long,
+                                      void* fmha, void* work, size_t work_bytes, void* out, int dt_out, int device, void* stream) {
+  if (!layout || S <= 0 || !work || !out || G <= 0 || window <= 0 || (min_long > 0 && (!fmha || dt_cache != 1 || dt_out != 1)))
+    return failf(KB2SEQ_ERR_VALUE, "attention_step: bad argument");
+  if (work_bytes < kb2_seq_attention_step_workspace(layout, S, H, G, d, dv, window, min_long) || ((uintptr_t)work & 15))
+    return failf(KB2SEQ_ERR_VALUE, "attention_step: workspace too small, or not on 16 bytes");
+  const AttnSeq* seq = reinterpret_cast<const AttnSeq*>(layout);
+  for (int q = 0; q < S; ++q)
+    if (min_long > 0 && seq[q].n >= min_long && (seq[q].start + seq[q].n - 1) / page_size >= seq[q].pages)
+      return failf(KB2SEQ_ERR_VALUE, "attention_step: sequence %d: %d pages of %d rows do not hold %d positions", q, seq[q].pages, page_size, seq[q].start + seq[q].n);
+  int rc = kb2_seq_head_kv_prep(proj, ldp, T, H, G, 1, d, dv, bias, qw, kw, eps, freq, rot_dims, positions, seq_of, pages, max_pages, page_size, kc, vc, dt_cache,
+                                norm_whole, rot_half, nullptr, amp, v_is_k, stream);
+  if (rc) return rc;
+  const size_t es = dt_out ? 2 : 4;
+  return attn_runs(seq, S, min_long, [&](bool fast, int i, int j, int r0, int rows) {
+    if (fast) {
+      for (int q = i; q < j; ++q) {
+        const AttnSeq& s = seq[q];
+        const int first = std::max(0, s.start - window + 1), keys = s.start + s.n - first;
+        const AttnWork w(s, H, G, d, dv, window);
+        char *k = (char*)work, *v = k + w.k, *qb = v + w.v;
+        if (int e = kb2_seq_portion_rows(kc, G * d, vc, G * dv, pages + (long long)q * max_pages, page_size, first, keys, k, v, proj + s.row * ldp, ldp, s.n,
+                                         H * d, qb, stream))
+          return e;
+        if (int e = reinterpret_cast<FmhaMaps>(fmha)(qb, k, v, (char*)out + (size_t)s.row * H * dv * es, s.n, s.start - first, keys, H, G, 1, dv, scale, softcap,
+                                                     window, sinks, nullptr, slopes, device, stream))
+          return 100 + e;
+      }
+      return KB2SEQ_OK;
+    }
+    const int pieces = attn_pieces(seq, i, j, rows, G, window);
+    float* acc = (float*)work;
+    float* ml = pieces > 1 ? acc + (size_t)rows * H * pieces * dv : nullptr;
+    if (int e = kb2_seq_paged_attn(proj + r0 * ldp, ldp, rows, H, G, 1, d, dv, kc, vc, dt_cache, positions + r0, seq_of + r0, pages, max_pages, page_size, scale, 0,
+                                   window, acc, pieces, pieces > 1 ? acc : nullptr, ml, nullptr, 0, softcap, sinks, 0, nullptr, nullptr, 0, slopes, stream))
+      return e;
+    return kb2_seq_attn_finish(acc, pieces > 1 ? acc : nullptr, ml, pieces, rows, H, 1, dv, nullptr, 0, eps, 1.f, nullptr, 0,
+                               (char*)out + (size_t)r0 * H * dv * es, dt_out, nullptr, nullptr, 0, 0, positions + r0, nullptr, rot_half, stream);
+  });
 }
 
 KB2SEQ_API int kb2_seq_glu(const void* in, int dt_in, long long ld_in, void* out, int dt_out, long long rows, int F, int kind, float limit,

@@ -74,6 +74,12 @@ def _core_lib():
     return _core
 
 
+def _fmha_maps(core) -> int:
+    """Address of the core library's attention for heads of one or more maps, for calls from the sequence library."""
+    import ctypes
+    return ctypes.cast(core.kb2_fmha_maps_bf16, ctypes.c_void_p).value
+
+
 def lin(a: torch.Tensor, w: torch.Tensor, out_dtype=torch.float32, min_n: int = 256) -> torch.Tensor:
     """a [M, K] (row stride free) @ w [N, K]^T with fp32 accumulation.  bfloat16 products run as a GEMV (at most 8 rows, the weights are
     streamed), on the tensor cores with chunked sums (fewer than 256 rows, or fewer than min_n columns: the accuracy of fp32 sums) or with one
@@ -870,6 +876,10 @@ class MultiMapAttention:
         ldp = proj.stride(0)
         s = stream_of(h)
         dtc = ops.dt_code(kc.dtype)
+        if self._one_call() and kc.dtype is vc.dtype and kc.is_contiguous() and vc.is_contiguous() and not (kc.data_ptr() | vc.data_ptr()) & 15:
+            core = _core_lib() if self.tc_shape and kc.dtype is torch.bfloat16 else False
+            if core or not self.tc_shape:
+                return lin(self._step(lib, core, proj, tb, kc, vc, dtc, page_size, s), self.w_o, torch.float32)
         ops.check(lib.kb2_seq_head_kv_prep(proj.data_ptr(), ldp, T, H, G if self.own_kv else 0, M, self.d, self.dv, ops._ptr(bias),
                                            ops._ptr(self.q_norm), ops._ptr(self.k_norm), self.eps, ops._ptr(self.freq), self.rot_dims,
                                            tb.positions.data_ptr(), tb.seq_of.data_ptr(), tb.pages.data_ptr(), tb.max_pages, page_size,
@@ -887,6 +897,31 @@ class MultiMapAttention:
         for fast, seqs, r0, rows in runs:
             self._attend(core if fast else None, proj, o, gate, tb, seqs, r0, rows, kc, vc, kp, vp, page_size, s)
         return lin(o, self.w_o, torch.float32)
+
+    def _one_call(self) -> bool:
+        """Whether kb2_seq_attention_step does all there is between the two products."""
+        return (self.M == 1 and self.own_kv and not (self.K or self.chunk or self.pool or self.unit_norm) and self.gate_off < 0 and self.map_coef is None
+                and self.vfreq is None)
+
+    def _step(self, lib, core, proj, tb, kc, vc, dtc, page_size, s):
+        """The finished heads of the whole step."""
+        T, H, G, d, dv, window, ptr = proj.shape[0], self.H, self.G, self.d, self.dv, min(self.window, 1 << 30), ops._ptr
+        long, dev = (self.tc_min_portion or 0) if core else 0, proj.get_device()
+        if long:
+            for i, (_, n, start, pages) in enumerate(tb.layout):
+                if n >= long and (start + n - 1) // page_size >= len(pages):         # the kernel would read on in the table
+                    raise IndexError(f"sequence {i}: {len(pages)} pages of {page_size} rows do not hold {start + n} positions")
+        size = lib.kb2_seq_attention_step_workspace(tb.layout_ptr, tb.S, H, G, d, dv, window, long)
+        o, work = torch.empty((T, H * dv), dtype=self.dtype, device=proj.device), torch.empty(size, dtype=torch.uint8, device=proj.device)
+        rc = lib.kb2_seq_attention_step(proj.data_ptr(), proj.stride(0), tb.layout_ptr, tb.S, T, H, G, d, dv, ptr(self.bias), ptr(self.q_norm), ptr(self.k_norm),
+                                        self.eps, ptr(self.freq), self.rot_dims, tb.positions.data_ptr(), tb.seq_of.data_ptr(), tb.pages.data_ptr(),
+                                        tb.max_pages, page_size, kc.data_ptr(), vc.data_ptr(), dtc, self.norm_whole, self.rot_half, self.rot_amp, self.kv_one,
+                                        self.scale, window, self.softcap, ptr(self.sink), ptr(self.slopes), long, _fmha_maps(core) if long else None,
+                                        work.data_ptr(), size, o.data_ptr(), ops.dt_code(self.dtype), dev, s)
+        if rc >= 100:
+            _core_check(rc - 100)
+        ops.check(rc)
+        return o
 
     def _attend(self, core, proj, o, gate, tb, seqs, r0, T, kc, vc, kp, vp, page_size, s):
         """Rows r0 .. r0 + T - 1 of the step (the sequences `seqs`): attention, the finished heads into o.  core: the library whose

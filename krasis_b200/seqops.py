@@ -36,6 +36,9 @@ SIGNATURES = {
     "kb2_seq_delta_rule_ch": (_I, [_P, _I, _P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _F, _P, _P, _P, _P, _P, _I, _P]),
     "kb2_seq_residual_add_norm": (_I, [_P, _P, _P, _P, _P, _P, _I, _I, _I, _F, _P]),
     "kb2_seq_head_kv_prep": (_I, [_P, _L, _I, _I, _I, _I, _I, _I, _P, _P, _P, _F, _P, _I, _P, _P, _P, _I, _I, _P, _P, _I, _I, _I, _P, _F, _I, _P]),
+    "kb2_seq_attention_step_workspace": (C.c_size_t, [_P, _I, _I, _I, _I, _I, _I, _I]),
+    "kb2_seq_attention_step": (_I, [_P, _L, _P, _I, _I, _I, _I, _I, _I, _P, _P, _P, _F, _P, _I, _P, _P, _P, _I, _I, _P, _P, _I, _I, _I, _F, _I, _F, _I, _F, _P, _P,
+                                    _I, _P, _P, C.c_size_t, _P, _I, _I, _P]),
     "kb2_seq_portion_rows": (_I, [_P, _I, _P, _I, _P, _I, _I, _I, _P, _P, _P, _L, _I, _I, _P, _P]),
     "kb2_seq_kv_pool": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _I, _P]),
     "kb2_seq_paged_attn": (_I, [_P, _L, _I, _I, _I, _I, _I, _I, _P, _P, _I, _P, _P, _P, _I, _I, _F, _I, _I, _P, _I, _P, _P, _P, _I, _F, _P, _I,
@@ -163,6 +166,9 @@ class StepTables:
             self.layout.append((row, len(toks), int(start), list(pages)))
             row += len(toks)
         self.max_portion = max(len(e[0]) for e in entries)
+        # the same for the C interfaces: [S][4] int32, pages by their number
+        self.layout_host = np.array([(r, n, start, len(pages)) for r, n, start, pages in self.layout], dtype=np.int32)
+        self.layout_ptr = self.layout_host.ctypes.data
         if device_buf is not None:
             if device_buf.numel() != n:
                 raise ValueError("device_buf does not fit this step's tables")
