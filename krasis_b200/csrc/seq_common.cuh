@@ -82,6 +82,8 @@ __device__ __forceinline__ void cp_async16_stream(uint32_t to, const void* from,
 using kb2act::gelu_tanh;
 using kb2act::glu_value;
 using kb2act::silu;
+using kb2act::gate_value;
+using kb2act::over;
 // Per-token decay exp(-exp(A_log) * softplus(a + dt_bias)).  A recurrent state multiplies by it at every token, so a rounding bias of
 // the fp32 exp / log1p chain (a fraction of an ulp, but of one sign) would grow linearly with the distance to a far token; evaluated in
 // fp64 and rounded once, the fp32 decay carries only its own unbiased half ulp.

@@ -772,7 +772,7 @@ __global__ void __launch_bounds__(256) head_norm_gate_kernel(const float* __rest
     if (w != nullptr) v *= w[j];
     if (gate != nullptr) {
       const float gz = gate[t * ldg + h * dv + j];
-      v *= gate_act ? 1.f / (1.f + expf(-gz)) : silu(gz);
+      v *= gate_value(gz, gate_act);
     }
     st_dt(out, dt_out, wi * dv + j, v);
   }
@@ -814,7 +814,7 @@ __global__ void __launch_bounds__(256) head_norm_gate_vec_kernel(const float* __
     rstd = dinv / sqrtf(warp_sum(ss) / (float)dv + eps);
     if (w_heads) w += (long long)h * dv;
   }
-  auto act = [&](float z) { return gate_act ? 1.f / (1.f + expf(-z)) : silu(z); };
+  auto act = [&](float z) { return gate_value(z, gate_act); };
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int j = (lane + 32 * i) * 4;
