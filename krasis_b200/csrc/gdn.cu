@@ -193,23 +193,71 @@ __global__ void __launch_bounds__(256) gdn_prep_tiled_kernel(GdnDims d, const __
 }
 
 
-// Vectorised variant (dk == dv == 128, conv width 4): one warp per (token tile, head); every lane owns FOUR CONSECUTIVE
-// channels of the head, so a token row is one 8-byte load / store per lane (the kernel above issues four 2-byte ones) and
-// the conv window lives in registers.  SiLU uses ex2-based __expf / __fdividef: the f32 result differs from expf by <= 2 ulp,
+// Vectorised variant (dk == dv == 128, conv width 4): one warp per (tile of 16 tokens, head); every lane owns FOUR CONSECUTIVE
+// channels of the head and asks for all its rows before the first is used (8 bytes a row, read back by the lane that copied them), and
+// the conv window lives in registers.  Products and sums run on pairs of numbers, roundings on the packed converter, the same bits as one by one.
+// SiLU uses ex2 and an approximate reciprocal: the f32 result differs from expf by <= 2 ulp,
 // which moves a BF16 rounding only when the value sits within 2^-22 of a rounding boundary (p ~ 6e-5 per element).
 // Rounding points are those of gdn_prep_kernel; the l2norm partial sums are grouped per lane differently (f32 addition order).
-constexpr int kGdnGateRows = 8;
-template <int TT>
-__global__ void __launch_bounds__(256) gdn_prep_vec_kernel(GdnDims d, const __nv_bfloat16* __restrict__ qkvz,
-                                                           const __nv_bfloat16* __restrict__ ba,
-                                                           const __nv_bfloat16* __restrict__ conv_w,
-                                                           const __nv_bfloat16* __restrict__ conv_state,
-                                                           const float* __restrict__ A_log, const float* __restrict__ dt_bias,
-                                                           __nv_bfloat16* __restrict__ qn, __nv_bfloat16* __restrict__ kn,
-                                                           __nv_bfloat16* __restrict__ vc, float* __restrict__ beta,
-                                                           float* __restrict__ g, int M, int n_tiles) {
+// Bound by its instructions and, in short steps, by the way of its rows.  64 heads of 128, 100 / 500 / 1000 / 2000 / 3333 tokens: one number at a time with four rows
+// ahead, tiles of 16 rows up to 2048 tokens and of 32 beyond, 8.9 / 11.7 / 20.1 / 33.0 / 51.4 us; this way 8.0 / 9.5 / 14.1 / 24.0 / 35.8.
+constexpr int kGdnGateRows = 8, kGdnTile = 16, kGdnPrepSmem = 8 * (kGdnTile + 3) * 256;
+struct F2 {                          // two numbers for the paired instructions
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 f2_get(F2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_of_bf16(uint32_t x) { return f2(__uint_as_float(x << 16), __uint_as_float(x & 0xFFFF0000u)); }
+__device__ __forceinline__ uint32_t bf16_of_f2(F2 a) {
+  const float2 f = f2_get(a);
+  return bf16x2_bits_rn(f.y, f.x);
+}
+__device__ __forceinline__ F2 bf16r2(F2 a) { return f2_of_bf16(bf16_of_f2(a)); }
+// y / (1 + e^-y)
+__device__ __forceinline__ F2 silu2(F2 y) {
+  const float2 z = f2_get(f2_mul(y, f2(-1.4426950408889634f, -1.4426950408889634f)));
+  float2 e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(z.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(z.y));
+  const float2 d = f2_get(f2_add(f2(e.x, e.y), f2(1.f, 1.f)));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(d.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(d.y));
+  return f2_mul(y, f2(r.x, r.y));
+}
+__global__ void __launch_bounds__(256, 4) gdn_prep_vec_kernel(GdnDims d, const __nv_bfloat16* __restrict__ qkvz,
+                                                              const __nv_bfloat16* __restrict__ ba,
+                                                              const __nv_bfloat16* __restrict__ conv_w,
+                                                              const __nv_bfloat16* __restrict__ conv_state,
+                                                              const float* __restrict__ A_log, const float* __restrict__ dt_bias,
+                                                              __nv_bfloat16* __restrict__ qn, __nv_bfloat16* __restrict__ kn,
+                                                              __nv_bfloat16* __restrict__ vc, float* __restrict__ beta,
+                                                              float* __restrict__ g, int M, int n_tiles) {
   pdl_enter(qkvz, ba, conv_w, conv_state, A_log, dt_bias, qn, kn, vc, beta, g);
-  constexpr int KW = 4;
+  constexpr int KW = 4, TT = kGdnTile;
+  extern __shared__ __align__(16) uint2 prep_rows[];          // [warp][3 rows ahead of the tile, the tile][lane]
   const int lane = threadIdx.x & 31;
   const long long wg = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int n_units = 2 * d.nk + d.nv + TT / kGdnGateRows;
@@ -217,8 +265,7 @@ __global__ void __launch_bounds__(256) gdn_prep_vec_kernel(GdnDims d, const __nv
   if (tile >= n_tiles) return;
   const int t_begin = tile * TT, t_end = min(M, t_begin + TT);
   const int kd = d.nk * d.dk, vd = d.nv * d.dv, ld = 2 * kd + 2 * vd, r = d.nv / d.nk;
-  if (u >= 2 * d.nk + d.nv) {             // gates of kGdnGateRows tokens, loaded together (one warp for a tile's 64, row by row, outlived the rest:
-                                          // 3333 tokens 65 us, 49 with this and the shorter tiles)
+  if (u >= 2 * d.nk + d.nv) {             // gates of kGdnGateRows tokens, loaded together (a warp that took a tile's 64 row by row outlived the rest)
     const int t0 = t_begin + (u - 2 * d.nk - d.nv) * kGdnGateRows;
     for (int h = lane; h < d.nv; h += 32) {
       const int col = h / r * 2 * r + h % r;
@@ -244,76 +291,92 @@ __global__ void __launch_bounds__(256) gdn_prep_vec_kernel(GdnDims d, const __nv
   const bool is_q = u < d.nk, is_k = !is_q && u < 2 * d.nk;
   const int c0 = (is_q ? u * d.dk : (is_k ? kd + (u - d.nk) * d.dk : 2 * kd + (u - 2 * d.nk) * d.dv)) + lane * 4;   // conv channel
   const int col0 = qkvz_col(d, c0);                                 // the 4 channels are consecutive columns of qkvz
-  float w[4][KW], hist[4][KW - 1];
+  uint2* mine = prep_rows + (threadIdx.x >> 5) * (TT + KW - 1) * 32 + lane;
+  const __nv_bfloat16* src = qkvz + (long long)t_begin * ld + col0;
+#pragma unroll
+  for (int i = 1 - KW; i < TT; ++i) {
+    if (i >= 0 ? t_begin + i < t_end : t_begin > 0)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(mine + (i + KW - 1) * 32)), "l"(src + (long long)i * ld) : "memory");
+    if (i >= 0 && i % 4 == 3) cp_async_commit();
+  }
+  F2 w[2][KW], hist[2][KW - 1];                                     // channels 0 and 1, 2 and 3
   {
     const uint4 w01 = *reinterpret_cast<const uint4*>(conv_w + (long long)c0 * KW);          // 16 bf16 = 4 channels x 4 taps
     const uint4 w23 = *reinterpret_cast<const uint4*>(conv_w + (long long)c0 * KW + 8);
     const uint32_t ww[8] = {w01.x, w01.y, w01.z, w01.w, w23.x, w23.y, w23.z, w23.w};
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      w[e][0] = __uint_as_float(ww[2 * e] << 16); w[e][1] = __uint_as_float(ww[2 * e] & 0xFFFF0000u);
-      w[e][2] = __uint_as_float(ww[2 * e + 1] << 16); w[e][3] = __uint_as_float(ww[2 * e + 1] & 0xFFFF0000u);
-    }
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+      for (int j = 0; j < KW; ++j) {
+        const uint32_t a = ww[4 * p + j / 2], b = ww[4 * p + 2 + j / 2];
+        w[p][j] = j & 1 ? f2(__uint_as_float(a & 0xFFFF0000u), __uint_as_float(b & 0xFFFF0000u)) : f2(__uint_as_float(a << 16), __uint_as_float(b << 16));
+      }
   }
+  if (t_begin == 0) {
 #pragma unroll
-  for (int j = 0; j < KW - 1; ++j) {
-    const int tt = t_begin - (KW - 1) + j;
-    if (tt >= 0) {
-      const uint2 x = *reinterpret_cast<const uint2*>(qkvz + (long long)tt * ld + col0);
-      hist[0][j] = __uint_as_float(x.x << 16); hist[1][j] = __uint_as_float(x.x & 0xFFFF0000u);
-      hist[2][j] = __uint_as_float(x.y << 16); hist[3][j] = __uint_as_float(x.y & 0xFFFF0000u);
-    } else {
+    for (int j = 0; j < KW - 1; ++j) {
+      float o[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) hist[e][j] = __bfloat162float(conv_state[(long long)(c0 + e) * KW + (KW + tt)]);
+      for (int e = 0; e < 4; ++e) o[e] = __bfloat162float(conv_state[(long long)(c0 + e) * KW + j + 1]);
+      hist[0][j] = f2(o[0], o[1]);
+      hist[1][j] = f2(o[2], o[3]);
     }
   }
   __nv_bfloat16* dst = is_q ? qn + (long long)u * d.dk : (is_k ? kn + (long long)(u - d.nk) * d.dk : vc + (long long)(u - 2 * d.nk) * d.dv);
   const int dst_ld = (is_q || is_k) ? kd : vd;
-  // rows are consumed strictly in order (the convolution history lives in registers), so the only memory-level parallelism a warp
-  // has is how far ahead it loads: four rows (1 KB per warp) in flight instead of one took this kernel off the latency bound
-  constexpr int kAhead = 4;
-  uint2 ring[kAhead];
+  dst += (long long)t_begin * dst_ld + lane * 4;
+  const int n = t_end - t_begin;
+  auto four = [&](int i0) {                                         // four rows of the tile, without a branch between them
 #pragma unroll
-  for (int j = 0; j < kAhead; ++j)
-    ring[j] = t_begin + j < t_end ? *reinterpret_cast<const uint2*>(qkvz + (long long)(t_begin + j) * ld + col0) : make_uint2(0u, 0u);
-  for (int t0 = t_begin; t0 < t_end; t0 += kAhead) {
+    for (int i = i0; i < i0 + 4; ++i) {
+      const uint2 cur = mine[(i + KW - 1) * 32];
+      const F2 x[2] = {f2_of_bf16(cur.x), f2_of_bf16(cur.y)};
+      uint32_t bits[2];
+      F2 sv[2];
 #pragma unroll
-   for (int jr = 0; jr < kAhead; ++jr) {
-    const int t = t0 + jr;
-    if (t >= t_end) break;                                   // warp-uniform
-    const uint2 cur = ring[jr];
-    if (t + kAhead < t_end) ring[jr] = *reinterpret_cast<const uint2*>(qkvz + (long long)(t + kAhead) * ld + col0);
-    const float x[4] = {__uint_as_float(cur.x << 16), __uint_as_float(cur.x & 0xFFFF0000u), __uint_as_float(cur.y << 16),
-                        __uint_as_float(cur.y & 0xFFFF0000u)};
-    float sv[4];
+      for (int p = 0; p < 2; ++p) {
+        F2 acc = f2_fma(w[p][0], hist[p][0], f2(0.f, 0.f));
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float acc = 0.f;
+        for (int j = 1; j < KW - 1; ++j) acc = f2_fma(w[p][j], hist[p][j], acc);
+        acc = f2_fma(w[p][KW - 1], x[p], acc);
 #pragma unroll
-      for (int j = 0; j < KW - 1; ++j) acc = fmaf(w[e][j], hist[e][j], acc);
-      acc = fmaf(w[e][KW - 1], x[e], acc);
-#pragma unroll
-      for (int j = 0; j < KW - 2; ++j) hist[e][j] = hist[e][j + 1];
-      hist[e][KW - 2] = x[e];
-      const float y = bf16r(acc);
-      sv[e] = bf16r(__fdividef(y, 1.0f + __expf(-y)));
-    }
-    if (is_q || is_k) {
-      float ss = (bf16r(sv[0] * sv[0]) + bf16r(sv[1] * sv[1])) + (bf16r(sv[2] * sv[2]) + bf16r(sv[3] * sv[3]));
-#pragma unroll
-      for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      const float inv = bf16r(rsqrtf(bf16r(bf16r(ss) + 1e-6f)));
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        sv[e] = bf16r(sv[e] * inv);
-        if (is_q) sv[e] = bf16r(sv[e] * d.scale);
+        for (int j = 0; j < KW - 2; ++j) hist[p][j] = hist[p][j + 1];
+        hist[p][KW - 2] = x[p];
+        bits[p] = bf16_of_f2(silu2(bf16r2(acc)));
+        sv[p] = f2_of_bf16(bits[p]);
       }
+      if (is_q || is_k) {
+        const float2 a = f2_get(bf16r2(f2_mul(sv[0], sv[0]))), b = f2_get(bf16r2(f2_mul(sv[1], sv[1])));
+        float ss = (a.x + a.y) + (b.x + b.y);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        const float inv = bf16r(rsqrtf(bf16r(bf16r(ss) + 1e-6f)));
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          bits[p] = bf16_of_f2(f2_mul(sv[p], f2(inv, inv)));
+          if (is_q) bits[p] = bf16_of_f2(f2_mul(f2_of_bf16(bits[p]), f2(d.scale, d.scale)));
+        }
+      }
+      if (i < n) *reinterpret_cast<uint2*>(dst + (long long)i * dst_ld) = make_uint2(bits[0], bits[1]);
     }
-    __nv_bfloat162 lo = __floats2bfloat162_rn(sv[0], sv[1]), hi = __floats2bfloat162_rn(sv[2], sv[3]);
-    *reinterpret_cast<uint2*>(dst + (long long)t * dst_ld + lane * 4) =
-        make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
-   }
+  };
+  cp_async_wait<3>();
+  if (t_begin > 0) {
+#pragma unroll
+    for (int j = 0; j < KW - 1; ++j) {
+      const uint2 x = mine[j * 32];
+      hist[0][j] = f2_of_bf16(x.x);
+      hist[1][j] = f2_of_bf16(x.y);
+    }
   }
+  static_assert(TT == 16 && KW == 4, "a group of four rows per wait");
+  four(0);
+  cp_async_wait<2>();
+  four(4);
+  cp_async_wait<1>();
+  four(8);
+  cp_async_wait<0>();
+  four(12);
 }
 
 // new conv state = last K pre-conv inputs (older entries come from the previous state when M < K)
@@ -891,20 +954,12 @@ cudaError_t launch_gdn_core(const GdnDims& d, const void* qkvz, const void* ba, 
   }
   { KernelSpan ks(K_GDN_PREP, s);
   if (d.dk == 128 && d.dv == 128 && d.K == 4 && !gdn_legacy_env()) {
-    auto prep = [&](auto tt) {
-      constexpr int TT = decltype(tt)::value;
-      const int n_tiles = (M + TT - 1) / TT;
-      const long long warps = (long long)n_tiles * (2 * d.nk + d.nv + TT / kGdnGateRows);
-      launch_pdl(gdn_prep_vec_kernel<TT>, (unsigned)((warps + 7) / 8), 256, 0, s,
-          d, (const __nv_bfloat16*)qkvz, (const __nv_bfloat16*)ba, (const __nv_bfloat16*)conv_w,
-          (const __nv_bfloat16*)conv_state, A_log, dt_bias, (__nv_bfloat16*)qn, (__nv_bfloat16*)kn, (__nv_bfloat16*)vc, beta, g,
-          M, n_tiles);
-    };
-    // A warp walks its tile's rows in order, so tiles are as short as filling the chip asks for; each reads three rows of history again.
-    // Tiles of 16 / 32 / 64 rows (64 heads of 128): 100 tokens 8.7 / 14.7 / 26.2 us, 1000 20.0 / 19.6 / 31.8, 2000 32.5 / 38.4 / 35.8,
-    // 3333 48.8 / 49.2 / 54.0, 8192 114.5 / 113.0 / 121.1.
-    if (M <= 2048) prep(std::integral_constant<int, 16>{});
-    else prep(std::integral_constant<int, 32>{});
+    const int n_tiles = (M + kGdnTile - 1) / kGdnTile;
+    const long long warps = (long long)n_tiles * (2 * d.nk + d.nv + kGdnTile / kGdnGateRows);
+    launch_pdl(gdn_prep_vec_kernel, (unsigned)((warps + 7) / 8), 256, kGdnPrepSmem, s,
+        d, (const __nv_bfloat16*)qkvz, (const __nv_bfloat16*)ba, (const __nv_bfloat16*)conv_w,
+        (const __nv_bfloat16*)conv_state, A_log, dt_bias, (__nv_bfloat16*)qn, (__nv_bfloat16*)kn, (__nv_bfloat16*)vc, beta, g,
+        M, n_tiles);
   } else if (d.dk == 128 && d.dv == 128 && d.K == 4) {
     const int n_tiles = (M + 31) / 32;
     const long long warps = (long long)n_tiles * (2 * d.nk + d.nv + 1);
