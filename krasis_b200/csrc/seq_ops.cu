@@ -1741,8 +1741,10 @@ template <int NI> struct DeltaTile {
   static constexpr int kUFloats = 2 * 2 * 256;             // [buffer][column group][lane][8]
   static constexpr int kSmem = kDTStages * kStageBytes + (kRedFloats + kUFloats) * 4 + (2 * kDTStages + 12) * 8;
   static constexpr int kThreads = 64 * NI + 96;
-// image | k | q | v of two heads | k.k and q.k in two halves | per head of a pair L, T beta G, T beta | gates
-  static constexpr int prep_smem(int vb, int rep) { return kImageBytes + (2 * kDT * DK + 2 * kDT * 32 * vb + 10 * kDT * 20 + 2 * kDT * rep) * 4; }
+  // image, then v of a pair's second head | k | q, then v of the first head | k.k and q.k in two halves | per head of a pair L, T beta G, T beta | gates
+  static constexpr int prep_image(int vb) { return kImageBytes > kDT * 32 * vb * 4 ? kImageBytes : kDT * 32 * vb * 4; }
+  static constexpr int prep_rows(int vb) { return kDT * DK + kDT * (DK > 32 * vb ? DK : 32 * vb); }
+  static constexpr int prep_smem(int vb, int rep) { return prep_image(vb) + (prep_rows(vb) + 10 * kDT * 20 + 2 * kDT * rep) * 4; }
   static_assert(kImageBytes % 16 == 0 && kWBytes % 16 == 0 && kScalarBytes % 16 == 0 && kStageBytes % 16 == 0, "bulk copies");
   static_assert(kSmem <= 227 * 1024, "shared memory");
 };
@@ -1795,11 +1797,12 @@ __device__ __forceinline__ void delta_fetch(const DeltaPrep& p, int t0, int nt, 
 }
 
 // A block of eight warps per (tile, key head).  Mostly traffic: at 4096 tokens, 32 / 16 heads x 128, 134 MB of k, q and v come
-// in and 304 MB go out in 107 us, 0.62 of the copy rate; the rest is the chain of a tile's products.  All loops are rolled as far as registers allow: with everything unrolled and a warp for each part the block took 35 KB of
+// in and 304 MB go out in 98 us, 0.68 of the copy rate; the rest is the chain of a tile's products, half of whose phases keep two or four of the warps busy.
+// Four blocks share an SM since the values lie where q and the image were (three: 111 us).  All loops are rolled as far as registers allow: with everything unrolled and a warp for each part the block took 35 KB of
 // instructions once, and waiting for them was most of its time.
 // image [tiles][Hk] | W [tiles][H] | V' [tiles][H][dv / 16][lane][8], in the order in which a lane of delta_tile_kernel takes them | scalars [tiles][H]
 template <int NI, int VB>
-__global__ void __launch_bounds__(256, 3) delta_tile_prep_kernel(const DeltaPrep p) {
+__global__ void __launch_bounds__(256, 4) delta_tile_prep_kernel(const DeltaPrep p) {
   kb2::pdl_wait();
   using D = DeltaTile<NI>;
   constexpr int DK = D::DK, kCols = 32 * VB;          // value columns of a pass
@@ -1820,9 +1823,9 @@ __global__ void __launch_bounds__(256, 3) delta_tile_prep_kernel(const DeltaPrep
   t0 += (int)tile * kDT;
   const int nt = min(kDT, n - (int)tile * kDT);
   bf16* img = reinterpret_cast<bf16*>(tsm);
-  float* rows = reinterpret_cast<float*>(tsm + D::kImageBytes);        // k [16][DK] | q [16][DK] | v of two heads [2][16][kCols]
-  float* vrow = rows + 2 * kDT * DK;
-  float* pairs = vrow + 2 * kDT * kCols;              // [k.k, q.k][half of the sum][16][20]
+  float* rows = reinterpret_cast<float*>(tsm + D::prep_image(VB));     // k [16][DK] | q [16][DK]
+  float* const vrow[2] = {rows + kDT * DK, reinterpret_cast<float*>(tsm)};      // of a pair's heads [16][kCols], where q and the image were
+  float* pairs = rows + D::prep_rows(VB);             // [k.k, q.k][half of the sum][16][20]
   float* Lb = pairs + 4 * kDT * 20;                   // [head of the pair][16][20], as T beta G and T beta
   float* Tw = Lb + 2 * kDT * 20;
   float* Tv = Tw + 2 * kDT * 20;
@@ -1831,19 +1834,17 @@ __global__ void __launch_bounds__(256, 3) delta_tile_prep_kernel(const DeltaPrep
   delta_fetch<DK>(p, t0, nt, p.Hk * DK + hk * DK, rows);
   delta_fetch<DK>(p, t0, nt, hk * DK, rows + kDT * DK);
   kb2::cp_async_commit();
-  auto fetch_values = [&](int r0, int j0) {
-    for (int hh = 0; hh < 2 && r0 + hh < rep; ++hh)
-      delta_fetch<kCols>(p, t0, nt, 2 * p.Hk * DK + (hk * rep + r0 + hh) * p.dv + j0, vrow + hh * kDT * kCols);
+  auto fetch_values = [&](int hh, int r0, int j0) {
+    if (r0 + hh < rep) delta_fetch<kCols>(p, t0, nt, 2 * p.Hk * DK + (hk * rep + r0 + hh) * p.dv + j0, vrow[hh]);
     kb2::cp_async_commit();
   };
-  fetch_values(0, 0);
   // decays and write strengths of the block's heads, under the wait for the rows (fp64 exponentials: a few hundred dependent instructions)
   for (int i = tid; i < 2 * rep * kDT; i += 256) {
     const int which = i / (rep * kDT), h = hk * rep + i % (rep * kDT) / kDT, t = i % kDT;
     const long long row = (long long)(t0 + t) * p.ldp + h;
     gates[i] = t >= nt ? (which ? 0.f : 1.f) : which ? 1.f / (1.f + expf(-p.bproj[row])) : decay_of(p.A_log[h], p.aproj[row], p.dt_bias[h]);
   }
-  kb2::cp_async_wait<1>();
+  kb2::cp_async_wait<0>();
   __syncthreads();
 
   auto store = [&](bf16* to, int part, const float (&v)[NI]) {       // the three parts of a row, `part` numbers apart
@@ -1897,6 +1898,8 @@ __global__ void __launch_bounds__(256, 3) delta_tile_prep_kernel(const DeltaPrep
     kb2::bulk_s2g(p.image + (flat * p.Hk + hk) * D::kImage, img, D::kImageBytes);
     kb2::bulk_commit_group();
   }
+  fetch_values(0, 0, 0);
+  if (tid == 128) kb2::bulk_wait_group_read0();       // the image has left shared memory
   if (warp < 4) {                                     // k_i . k_j (warps 0, 1: halves of the sum) and q_i . k_j (2, 3)
     float s[2][4] = {};
     const bf16* row = img + ((lane >> 4) * 8 + (lane & 7)) * D::kPitch + ((lane >> 3) & 1) * 8;
@@ -1935,6 +1938,7 @@ __global__ void __launch_bounds__(256, 3) delta_tile_prep_kernel(const DeltaPrep
         *reinterpret_cast<float2*>(pairs + warp * kDT * 20 + ((lane >> 2) + e * 8) * 20 + b * 8 + (lane & 3) * 2) = make_float2(s[b][2 * e], s[b][2 * e + 1]);
   }
   __syncthreads();
+  fetch_values(1, 0, 0);
 #pragma unroll 1
   for (int r0 = 0; r0 < rep; r0 += 2) {
     if (warp < 2) {                                   // a lane per (head of the pair, token): what couples the tokens
@@ -2054,7 +2058,7 @@ __global__ void __launch_bounds__(256, 3) delta_tile_prep_kernel(const DeltaPrep
       } else if (there) {
         float a[4][VB], c[4][VB];
         const float* T = Tv + hh * kDT * 20;
-        const float* x = vrow + hh * kDT * kCols;
+        const float* x = vrow[hh];
         four(T, x, kCols, b0, a);
         four(T, x, kCols, b0 + 2, c);
         float* vi = p.vimage + (flat * H + hv) * kDT * p.dv;
@@ -2069,12 +2073,12 @@ __global__ void __launch_bounds__(256, 3) delta_tile_prep_kernel(const DeltaPrep
       }
       if (j0 + kCols < p.dv || r0 + 2 < rep) {
         __syncthreads();
-        if (j0 + kCols < p.dv) fetch_values(r0, j0 + kCols);
-        else fetch_values(r0 + 2, 0);
+        const bool more = j0 + kCols < p.dv;
+        for (int v = 0; v < 2; ++v) fetch_values(v, more ? r0 : r0 + 2, more ? j0 + kCols : 0);
       }
     }
   }
-  if (tid == 128) kb2::bulk_wait_group0();            // the image has left shared memory
+  if (tid == 128) kb2::bulk_wait_group0();
 }
 
 template <int NI>
