@@ -1724,9 +1724,10 @@ __global__ void __launch_bounds__(32 * kRegPieces) delta_rule_reg_kernel(const f
 // and transposed for k u^T; the partial sums of a group's warps meet in shared memory in fragment order, so nothing is moved between lanes.
 // The largest of the six products of an update and of a read-out goes eight tokens at a time, each to a sum of its own: the tensor cores cut off
 // what they add, and with sixteen at a time states were 1 % further off (6.6e-7 instead of 6.5e-7).
-// Bound: 1300 cycles of the tensor pipe and 1400 of shared memory per tile, of about 2400 (4096 tokens, 32 / 16 heads x 128: 342 us, the prep 110); left
-// is the chain split - W - exchange - u - update.  With eight tokens per tile, where each warp solved for u itself, a tile took 2400 cycles of dependent
-// short phases too, and the whole 642 + 56 us.
+// Bound: 1300 cycles of the tensor pipe and 1400 of shared memory per tile, of about 2200 (4096 tokens, 32 / 16 heads x 128: 310 us, the prep 98); left
+// is the chain split - W - exchange - u - update.  The next tile is waited for and its W fetched between the instructions of the update and the use of their sums,
+// and the read-out's buffer at its first store: with all three at the head of a tile 338 us (q fetched ahead of W's sums as well: 364).
+// With eight tokens per tile, where each warp solved for u itself, a tile took 2400 cycles of dependent short phases, and the whole 642 + 56 us.
 constexpr int kDT = 16, kDTStages = 4;
 // what couples the tokens of a (tile, head): G[16] | D_15,j [16] | G_15 and padding to 48 floats | D_ij q_i . k_j as three bf16 parts [i][24]
 constexpr int kDTG = 0, kDTEnd = 16, kDTAll = 32, kDTQK = 48, kDTQKPitch = 24, kDTQKPart = kDT * kDTQKPitch;
@@ -2107,8 +2108,8 @@ __global__ void __launch_bounds__(DeltaTile<NI>::kThreads, 1)
     const long long all = first + tiles;
     skip = (int)(min(max(f0, first), all) - first);
     tiles = (int)(min(max(f1, first), all) - first) - skip;
-    if (tiles == 0) return;
   }
+  if (tiles == 0) return;
   const int t0 = cu[s] + skip * kDT, n = n_all - skip * kDT;      // tokens from the slice on
   if (threadIdx.x == 0) {
     for (int i = 0; i < kDTStages; ++i) {
@@ -2231,12 +2232,24 @@ __global__ void __launch_bounds__(DeltaTile<NI>::kThreads, 1)
   // ldmatrix rows: tokens along the lanes' eights, plain and transposed
   const int plain = ((lane >> 4) * 8 + (lane & 7)) * D::kPitch + piece * 32 + ((lane >> 3) & 1) * 8;
   const int turned = (((lane >> 3) & 1) * 8 + (lane & 7)) * D::kPitch + piece * 32 + (lane >> 4) * 8;
+  // operand fragments of 16 tokens: [16 rows][part]
+  auto fetch = [&](const bf16* rows, int part, uint32_t (&x)[2][3][4]) {
+#pragma unroll
+    for (int kb = 0; kb < 2; ++kb)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) ldmatrix4<false>(x[kb][c], rows + c * part + plain + kb * 16);
+  };
+  uint32_t w[2][3][4];
+  auto enter = [&](int i) {                        // tile i is there, and W as operand: looked for under the update of the tile before it
+    kb2::mbar_wait(&full[i % kDTStages], (uint32_t)(i / kDTStages & 1));
+    fetch(reinterpret_cast<const bf16*>(tsm + i % kDTStages * D::kStageBytes + D::kImageBytes), D::kWPart, w);
+  };
+  enter(0);
   for (int i = 0; i < tiles; ++i) {
     const int st = i % kDTStages, buf = (i & 1) * 2 + cg;
     const uint32_t turn = (uint32_t)(i >> 1) & 1u;
     const uint8_t* b = tsm + st * D::kStageBytes;
     const bf16* img = reinterpret_cast<const bf16*>(b);
-    const bf16* wim = reinterpret_cast<const bf16*>(b + D::kImageBytes);
     const float* vs = reinterpret_cast<const float*>(b + D::kImageBytes + D::kWBytes) + cg * 256 + lane * 8;
     const float* ss = reinterpret_cast<const float*>(b + D::kImageBytes + D::kWBytes + D::kVBytes);
     float* mine = red + (buf * NI + piece) * 512 + lane * 4;
@@ -2251,20 +2264,14 @@ __global__ void __launch_bounds__(DeltaTile<NI>::kThreads, 1)
         for (int c = 0; c < 3; ++c) sp[kb][c][e] = p[c];
       }
     // S0^T [16 columns x 32 rows] times 16 tokens, in three sums of up to six instructions, each of which waits for the one before
-    auto product = [&](const bf16* rows, int part, float (&sum)[3][2][4]) {
+    auto product = [&](const uint32_t (&x)[2][3][4], float (&sum)[3][2][4]) {
 #pragma unroll
-      for (int kb = 0; kb < 2; ++kb) {
-        uint32_t x[3][4];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) ldmatrix4<false>(x[c], rows + c * part + plain + kb * 16);
+      for (int kb = 0; kb < 2; ++kb)
 #pragma unroll
         for (int m = 0; m < 6; ++m)
 #pragma unroll
-          for (int nb = 0; nb < 2; ++nb) one(sum[m ? 1 + (m & 1) : 0][nb], kb == 0 && m < 3, sp[kb], x, 2 * nb, m);
-      }
+          for (int nb = 0; nb < 2; ++nb) one(sum[m ? 1 + (m & 1) : 0][nb], kb == 0 && m < 3, sp[kb], x[kb], 2 * nb, m);
     };
-    kb2::mbar_wait(&full[st], (uint32_t)(i / kDTStages & 1));
-    kb2::mbar_wait(&o_free[buf], turn ^ 1u);
     auto keep = [&](float* to, const float (&sum)[3][2][4]) {
 #pragma unroll
       for (int nb = 0; nb < 2; ++nb) {
@@ -2274,15 +2281,18 @@ __global__ void __launch_bounds__(DeltaTile<NI>::kThreads, 1)
         *reinterpret_cast<float4*>(to + nb * 128) = make_float4(v[0], v[1], v[2], v[3]);
       }
     };
+    uint32_t q[2][3][4];
     {
       float ws[3][2][4];
-      product(wim, D::kWPart, ws);
+      product(w, ws);
+      kb2::mbar_wait(&o_free[buf], turn ^ 1u);
       keep(mine, ws);
     }
     __syncwarp();
     if (lane == 0) kb2::mbar_arrive(&w_there[buf]);
     float qs[3][2][4];                             // q, under the wait for the other pieces; put away when there is time
-    product(img + D::kWPart, D::kPart, qs);
+    fetch(img + D::kWPart, D::kPart, q);
+    product(q, qs);
     uint32_t kt[2][3][4];                          // k transposed: [16 rows][part]
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr)
@@ -2328,16 +2338,17 @@ __global__ void __launch_bounds__(DeltaTile<NI>::kThreads, 1)
     for (int m = 1; m < 6; ++m)
 #pragma unroll
       for (int r = 0; r < 4; ++r) one(small[r], m < 2, up, kt[r >> 1], (r & 1) * 2, m);
+    if (i + 1 < tiles) enter(i + 1);
     keep(mine + 256, qs);
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) S[r][e] = fmaf(S[r][e], total, (big[0][r][e] + big[1][r][e]) + small[r][e]);
     __syncwarp();
     if (lane == 0) {
       kb2::mbar_arrive(&o_there[buf]);
       kb2::mbar_arrive(&empty[st]);                // everything of the tile is in registers
     }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) S[r][e] = fmaf(S[r][e], total, (big[0][r][e] + big[1][r][e]) + small[r][e]);
   }
 #pragma unroll
   for (int r = 0; r < 4; ++r)
