@@ -681,16 +681,16 @@ cudaError_t launch_gqa_core(const GqaDims& g, const void* q_raw, const void* k_r
   }
   { KernelSpan ks(K_GQA_PREP, s);
   const int half = g.rotary_dim / 2;
-  auto prep = [&](auto kernel) {
-    const int tokens = M >= 512 ? kPrepTokens : 1;      // below that a block per token leaves more of them running
-    launch_pdl(kernel, (M + tokens - 1) / tokens, 256, 0, s, g, (const __nv_bfloat16*)q_raw, (const __nv_bfloat16*)k_raw, (const __nv_bfloat16*)v_raw, q_norm, k_norm,
+  auto by_rows = g.d == 256 && half == 32    ? gqa_prep_rows_kernel<256, 32>
+                 : g.d == 256 && half == 64  ? gqa_prep_rows_kernel<256, 64>
+                 : g.d == 256 && half == 128 ? gqa_prep_rows_kernel<256, 128>
+                 : g.d == 128 && half == 32  ? gqa_prep_rows_kernel<128, 32>
+                 : g.d == 128 && half == 64  ? gqa_prep_rows_kernel<128, 64>
+                                             : nullptr;
+  const int tokens = M >= 512 ? kPrepTokens : 1;      // below that a block per token leaves more of them running
+  if (by_rows)
+    launch_pdl(by_rows, (M + tokens - 1) / tokens, 256, 0, s, g, (const __nv_bfloat16*)q_raw, (const __nv_bfloat16*)k_raw, (const __nv_bfloat16*)v_raw, q_norm, k_norm,
                positions, kv_indices, (__nv_bfloat16*)q_rot, (uint8_t*)k_cache, (uint8_t*)v_cache, M, tokens);
-  };
-  if (g.d == 256 && half == 32) prep(gqa_prep_rows_kernel<256, 32>);
-  else if (g.d == 256 && half == 64) prep(gqa_prep_rows_kernel<256, 64>);
-  else if (g.d == 256 && half == 128) prep(gqa_prep_rows_kernel<256, 128>);
-  else if (g.d == 128 && half == 32) prep(gqa_prep_rows_kernel<128, 32>);
-  else if (g.d == 128 && half == 64) prep(gqa_prep_rows_kernel<128, 64>);
   else launch_pdl(gqa_prep_kernel, M, 256, (8 * g.d + g.rotary_dim) * sizeof(float), s, g, (const __nv_bfloat16*)q_raw, (const __nv_bfloat16*)k_raw,
                   (const __nv_bfloat16*)v_raw, q_norm, k_norm, positions, kv_indices, (__nv_bfloat16*)q_rot, (uint8_t*)k_cache, (uint8_t*)v_cache, M);
   }
