@@ -687,7 +687,9 @@ cudaError_t launch_gqa_core(const GqaDims& g, const void* q_raw, const void* k_r
                  : g.d == 128 && half == 32  ? gqa_prep_rows_kernel<128, 32>
                  : g.d == 128 && half == 64  ? gqa_prep_rows_kernel<128, 64>
                                              : nullptr;
-  const int tokens = M >= 512 ? kPrepTokens : 1;      // below that a block per token leaves more of them running
+  // below that a block per token leaves more of them running (one token a block / four, 300, 600, 800, 1000, 2000 tokens: 5.0 / 8.2, 8.6 / 9.4, 9.8 / 9.6, 10.0 / 9.8,
+  // 17.5 / 14.3 us; the row through shared memory 7.7, 10.0, 10.9, 12.2, 21.1)
+  const int tokens = M >= 768 ? kPrepTokens : 1;
   if (by_rows)
     launch_pdl(by_rows, (M + tokens - 1) / tokens, 256, 0, s, g, (const __nv_bfloat16*)q_raw, (const __nv_bfloat16*)k_raw, (const __nv_bfloat16*)v_raw, q_norm, k_norm,
                positions, kv_indices, (__nv_bfloat16*)q_rot, (uint8_t*)k_cache, (uint8_t*)v_cache, M, tokens);

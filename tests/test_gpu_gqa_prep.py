@@ -10,8 +10,8 @@ import test_gpu_attention as base  # noqa: E402
 pytestmark = pytest.mark.gpu
 
 
-# 515 tokens: blocks of four tokens with a remainder, then few tokens behind cached ones; the last two rotations have no form of their own
-@pytest.mark.parametrize("M1,M2", [(515, 3), (16, 512)])
+# 771 tokens: blocks of four tokens with a remainder, then few tokens behind cached ones; the last two rotations have no form of their own
+@pytest.mark.parametrize("M1,M2", [(771, 3), (16, 512)])
 @pytest.mark.parametrize("nh,nkv,d,rot,gated", [(3, 1, 256, 64, True), (2, 1, 256, 128, False), (2, 2, 256, 256, True), (4, 2, 128, 64, False), (5, 1, 128, 128, True),
                                                 (2, 1, 256, 96, False), (2, 2, 128, 32, True)])
 def test_preparation(nh, nkv, d, rot, gated, M1, M2):
