@@ -9,14 +9,15 @@ __device__ __forceinline__ float gelu_tanh(float z) {
   return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
 }
 // x / d for d >= 1, infinity with it, without a branch: an approximate quotient and one step along its residual (Markstein 1990, "Computation of elementary
-// functions on the IBM RISC System/6000 processor").  Where the residual is not a number (d or x infinite) the product is the answer.  x / d has a path of
-// its own for what is out of range, a branch per number, across which nothing is in flight.  Errors of silu against fp64 over 4 M numbers each of five scales are those
+// functions on the IBM RISC System/6000 processor").  Where the residual is not a number (d or x infinite) the product is the answer, and where it is zero the
+// product stays as it is: a step of zero would make -0 a +0.  In place of x / d: the convolution of 4096 tokens x 8192
+// channels 88 -> 80 us.  Errors of silu against fp64 over 4 M numbers each of five scales are those
 // of the quotient: at most 2.14e-7, 3.7e-8 to 4.5e-8 in the mean.
 __device__ __forceinline__ float over(float x, float d) {
   float r;
   asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
   const float q = x * r, left = fmaf(-q, d, x);
-  return left == left ? fmaf(left, r, q) : q;
+  return fabsf(left) > 0.f ? fmaf(left, r, q) : q;
 }
 __device__ __forceinline__ float silu(float z) { return over(z, 1.f + expf(-z)); }
 // what a gate's number multiplies by: silu, or its sigmoid

@@ -27,3 +27,16 @@ def test_silu(T):
     assert ((got - want).abs() <= 2.0 ** -21 * want.abs() + 3e-37)[~odd].all()
     i = ends.numel()
     assert got[0, i - 3] == float("inf") and got[0, i - 2:i].isnan().all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_sign_of_zero(dtype):
+    """silu(-0) u is -0 u, and so is a clamped swish of it."""
+    from krasis_b200 import seqops as ops
+    F = 64
+    g = torch.zeros(2, F, device="cuda")
+    g[:, ::2] = -0.0
+    gu = torch.cat([g, torch.ones(2, F, device="cuda")], 1).to(dtype)
+    for kind, kw in ((1, {}), (2, {"limit": 7.0, "alpha": 1.7})):
+        got = ops.glu(gu, dtype, kind, **kw)
+        assert torch.equal(got.float().signbit(), g.signbit()) and not got.any()
