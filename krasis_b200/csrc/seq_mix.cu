@@ -1074,6 +1074,14 @@ int attn_pieces(const AttnSeq* seq, int i, int j, int rows, int G, int window) {
   for (int q = i; q < j; ++q) most = std::max(most, std::min(window, seq[q].start + seq[q].n));
   return std::max(1, std::min({296 / std::max(rows * G, 1), (most + 31) / 32, 64}));
 }
+// Rows of a paged_attn block and its shared memory; 0: the sizes do not fit.
+int paged_attn_rows(int R, int M, int d, int dv, size_t* smem) {
+  auto bytes = [&](int rb) { return (size_t)(2 * kPAKT + rb * d + kPAKT * ((M * d) | 1) + kPAKT * dv + rb * kPAKT + 3 * rb) * 4; };
+  int rb = R;
+  while (rb > 1 && (rb * dv > kPAThreads * kPAAcc || bytes(rb) > 200 * 1024)) rb = (rb + 1) / 2;
+  *smem = bytes(rb);
+  return *smem > 200 * 1024 ? 0 : rb;
+}
 struct AttnWork {                  // of a long portion: its keys, values and queries in bf16
   size_t k, v, q;
   AttnWork(const AttnSeq& s, int H, int G, int d, int dv, int window) {
@@ -1144,13 +1152,9 @@ KB2SEQ_API int kb2_seq_paged_attn(const float* proj, long long ldp, int T, int H
   if (nsplit < 1 || nsplit > 1024 || (nsplit > 1 && (!part_acc || !part_ml))) return failf(KB2SEQ_ERR_VALUE, "paged_attn: bad key split");
   if (dv > kPAThreads * kPAAcc) return failf(KB2SEQ_ERR_VALUE, "paged_attn: value size %d > %d", dv, kPAThreads * kPAAcc);
   const int R = (H / G) * M;
-  int RB = R;
-  auto smem_of = [&](int rb) {
-    return (size_t)(2 * kPAKT + rb * d + kPAKT * ((M * d) | 1) + kPAKT * dv + rb * kPAKT + 3 * rb) * 4;
-  };
-  while (RB > 1 && (RB * dv > kPAThreads * kPAAcc || smem_of(RB) > 200 * 1024)) RB = (RB + 1) / 2;
-  const size_t smem = smem_of(RB);
-  if (smem > 200 * 1024) return failf(KB2SEQ_ERR_VALUE, "paged_attn: head sizes %d / %d too large", M * d, dv);
+  size_t smem;
+  const int RB = paged_attn_rows(R, M, d, dv, &smem);
+  if (!RB) return failf(KB2SEQ_ERR_VALUE, "paged_attn: head sizes %d / %d too large", M * d, dv);
   if (smem > 48 * 1024) SEQ_CUDA(kb2::allow_smem<paged_attn_kernel>(200 * 1024));
   const int nrb = (R + RB - 1) / RB;
   if ((long long)G * nrb > 65535) return failf(KB2SEQ_ERR_VALUE, "paged_attn: too many heads");
@@ -1203,6 +1207,7 @@ KB2SEQ_API int kb2_seq_attn_finish(const float* a, const float* part_acc, const 
 // ---- everything between an attention layer's two products, in one call: a mixed step is seven launches, and what a host needs for each of them from Python
 // took longer than the kernels (512 tokens beside three decoded ones: 93 us for 66).
 KB2SEQ_API size_t kb2_seq_attention_step_workspace(const int* layout, int S, int H, int G, int d, int dv, int window, int min_long) {
+  if (!layout || S <= 0) return 0;
   const AttnSeq* seq = reinterpret_cast<const AttnSeq*>(layout);
   size_t most = 16;
   attn_runs(seq, S, min_long, [&](bool fast, int i, int j, int, int rows) {
@@ -1227,14 +1232,27 @@ KB2SEQ_API int kb2_seq_attention_step(float* proj, long long ldp, const int* lay
                                       const int* pages, int max_pages, int page_size, void* kc, void* vc, int dt_cache, int norm_whole, int rot_half, float amp,
                                       int v_is_k, float scale, int window, float softcap, const float* sinks, const float* slopes, int min_long,
                                       void* fmha, void* work, size_t work_bytes, void* out, int dt_out, int device, void* stream) {
-  if (!layout || S <= 0 || !work || !out || G <= 0 || window <= 0 || (min_long > 0 && (!fmha || dt_cache != 1 || dt_out != 1)))
+  // all that a later launch would refuse or take for granted, ahead of the first one: that writes the caches
+  if (!proj || !layout || !positions || !seq_of || !pages || !kc || !vc || !work || !out || S <= 0 || T <= 0 || H <= 0 || G <= 0 || H % G || d <= 0 || dv <= 0 ||
+      window <= 0 || max_pages <= 0 || page_size <= 0 || bad_dt(dt_cache) || bad_dt(dt_out) || !(softcap >= 0.f) || (((uintptr_t)kc | (uintptr_t)vc) & 15))
     return failf(KB2SEQ_ERR_VALUE, "attention_step: bad argument");
-  if (work_bytes < kb2_seq_attention_step_workspace(layout, S, H, G, d, dv, window, min_long) || ((uintptr_t)work & 15))
-    return failf(KB2SEQ_ERR_VALUE, "attention_step: workspace too small, or not on 16 bytes");
+  size_t smem;
+  const int rb = dv > 32 * kFinAcc ? 0 : paged_attn_rows(H / G, 1, d, dv, &smem);
+  if (!rb || (long long)G * ((H / G + rb - 1) / rb) > 65535) return failf(KB2SEQ_ERR_VALUE, "attention_step: head sizes %d / %d too large", d, dv);
+  if (min_long > 0 && (!fmha || dt_cache != 1 || dt_out != 1 || d != 128 || (dv != 128 && dv != 256) || !(scale > 0.f) || ((uintptr_t)out & 15)))
+    return failf(KB2SEQ_ERR_VALUE, "attention_step: long portions need bf16 caches and outputs on 16 bytes, 128 query and key and 128 or 256 value columns, a scale above 0");
   const AttnSeq* seq = reinterpret_cast<const AttnSeq*>(layout);
+  long long rows_seen = 0;
+  for (int q = 0; q < S; rows_seen += seq[q++].n)
+    if (seq[q].row != rows_seen || seq[q].n < 0 || seq[q].start < 0 || seq[q].start > INT_MAX - seq[q].n || seq[q].pages < 0 || seq[q].pages > max_pages ||
+        rows_seen + seq[q].n > T)
+      return failf(KB2SEQ_ERR_VALUE, "attention_step: sequence %d: rows follow one another, page lists have at most %d entries", q, max_pages);
+  if (rows_seen != T) return failf(KB2SEQ_ERR_VALUE, "attention_step: sequences of %lld rows for a step of %d", rows_seen, T);
   for (int q = 0; q < S; ++q)
     if (min_long > 0 && seq[q].n >= min_long && (seq[q].start + seq[q].n - 1) / page_size >= seq[q].pages)
       return failf(KB2SEQ_ERR_VALUE, "attention_step: sequence %d: %d pages of %d rows do not hold %d positions", q, seq[q].pages, page_size, seq[q].start + seq[q].n);
+  if (work_bytes < kb2_seq_attention_step_workspace(layout, S, H, G, d, dv, window, min_long) || ((uintptr_t)work & 15))
+    return failf(KB2SEQ_ERR_VALUE, "attention_step: workspace too small, or not on 16 bytes");
   int rc = kb2_seq_head_kv_prep(proj, ldp, T, H, G, 1, d, dv, bias, qw, kw, eps, freq, rot_dims, positions, seq_of, pages, max_pages, page_size, kc, vc, dt_cache,
                                 norm_whole, rot_half, nullptr, amp, v_is_k, stream);
   if (rc) return rc;
