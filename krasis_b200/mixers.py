@@ -906,7 +906,7 @@ class MultiMapAttention:
     def _step(self, lib, core, proj, tb, kc, vc, dtc, page_size, s):
         """The finished heads of the whole step."""
         T, H, G, d, dv, window, ptr = proj.shape[0], self.H, self.G, self.d, self.dv, min(self.window, 1 << 30), ops._ptr
-        long, dev = (self.tc_min_portion or 0) if core else 0, proj.get_device()
+        long, dev = max(self.tc_min_portion, 1) if core and self.tc_min_portion is not None else 0, proj.get_device()      # 0: none is long
         if long:
             for i, (_, n, start, pages) in enumerate(tb.layout):
                 if n >= long and (start + n - 1) // page_size >= len(pages):         # the kernel would read on in the table

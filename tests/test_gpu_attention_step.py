@@ -60,3 +60,25 @@ def test_pages_that_do_not_hold_a_portion():
     with pytest.raises(IndexError):
         m.forward(torch.zeros(130, 256, dtype=torch.bfloat16, device="cuda"), tb, kc, kc.clone(), 64)
     assert not kc.any()
+
+
+@pytest.mark.parametrize("least", [0, 1, 5])
+def test_shortest_portion_of_the_tensor_cores(least, monkeypatch):
+    """tc_min_portion: 0 and 1 send every portion to the tensor cores, in one call as in single ones."""
+    from krasis_b200 import seqops as ops
+    from krasis_b200.mixers import MultiMapAttention
+    g = torch.Generator().manual_seed(3)
+    r = lambda *s: torch.randn(*s, generator=g) * 0.06  # noqa: E731
+    m = MultiMapAttention({"q": r(512, 256), "k": r(128, 256), "v": r(128, 256), "o": r(256, 512)}, 4, 1, 1, 128, 128, 128 ** -0.5, 1e-5, torch.bfloat16, "cuda")
+    m.tc_min_portion = least
+    tb = ops.StepTables([([0] * 3, 20, 0, [0]), ([0], 70, 1, [2, 1]), ([0] * 140, 0, 2, [3, 4, 5])], "cuda")
+    kc, vc = (torch.randn(6, 64, 128, generator=g).bfloat16().cuda() for _ in range(2))
+    h = torch.randn(tb.T, 256, generator=g).bfloat16().cuda()
+    portions = []
+    portion_rows = ops.portion_rows
+    monkeypatch.setattr(ops, "portion_rows", lambda tb, s, *a: portions.append(s) or portion_rows(tb, s, *a))
+    got = m.forward(h, tb, kc.clone(), vc.clone(), 64)
+    assert not portions and m._one_call()
+    monkeypatch.setattr(MultiMapAttention, "_one_call", lambda self: False)
+    want = m.forward(h, tb, kc, vc, 64)
+    assert torch.equal(got, want) and portions == {0: [0, 1, 2], 1: [0, 1, 2], 5: [2]}[least]
