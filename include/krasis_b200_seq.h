@@ -29,6 +29,7 @@ extern "C" {
 #define KB2SEQ_OK 0
 #define KB2SEQ_ERR_VALUE 2
 #define KB2SEQ_ERR_CUDA 3
+#define KB2SEQ_ERR_RANGE 4 /* positions that the page lists do not hold */
 
 KB2SEQ_API const char* kb2_seq_last_error(void);
 KB2SEQ_API long long kb2_seq_total_launches(void);
@@ -146,7 +147,7 @@ KB2SEQ_API int kb2_seq_head_kv_prep(float* proj, long long ldp, int T, int H, in
  * head_kv_prep, then per run of sequences portion_rows and `fmha` (the core library's kb2_fmha_maps_bf16; its error e comes back as 100 + e) for portions of
  * min_long tokens and more (0: none), paged_attn and attn_finish for the others.  layout (host): [S][4] first row, tokens, first position, pages; its rows follow one
  * another and are T in all.  Caches on 16 bytes; with min_long > 0 they and out are bf16, out on 16 bytes, d 128, dv 128 or 256, and a long portion's pages hold its
- * positions.  What does not fit comes back as KB2SEQ_ERR_VALUE ahead of the first launch. */
+ * positions.  What does not fit comes back as KB2SEQ_ERR_VALUE, or KB2SEQ_ERR_RANGE for the pages, ahead of the first launch. */
 KB2SEQ_API size_t kb2_seq_attention_step_workspace(const int* layout, int S, int H, int G, int d, int dv, int window, int min_long);
 KB2SEQ_API int kb2_seq_attention_step(float* proj, long long ldp, const int* layout, int S, int T, int H, int G, int d, int dv, const float* bias,
                                       const float* qw, const float* kw, float eps, const double* freq, int rot_dims, const int* positions, const int* seq_of,

@@ -1250,7 +1250,7 @@ KB2SEQ_API int kb2_seq_attention_step(float* proj, long long ldp, const int* lay
   if (rows_seen != T) return failf(KB2SEQ_ERR_VALUE, "attention_step: sequences of %lld rows for a step of %d", rows_seen, T);
   for (int q = 0; q < S; ++q)
     if (min_long > 0 && seq[q].n >= min_long && (seq[q].start + seq[q].n - 1) / page_size >= seq[q].pages)
-      return failf(KB2SEQ_ERR_VALUE, "attention_step: sequence %d: %d pages of %d rows do not hold %d positions", q, seq[q].pages, page_size, seq[q].start + seq[q].n);
+      return failf(KB2SEQ_ERR_RANGE, "attention_step: sequence %d: %d pages of %d rows do not hold %d positions", q, seq[q].pages, page_size, seq[q].start + seq[q].n);
   if (work_bytes < kb2_seq_attention_step_workspace(layout, S, H, G, d, dv, window, min_long) || ((uintptr_t)work & 15))
     return failf(KB2SEQ_ERR_VALUE, "attention_step: workspace too small, or not on 16 bytes");
   int rc = kb2_seq_head_kv_prep(proj, ldp, T, H, G, 1, d, dv, bias, qw, kw, eps, freq, rot_dims, positions, seq_of, pages, max_pages, page_size, kc, vc, dt_cache,

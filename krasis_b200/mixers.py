@@ -907,10 +907,6 @@ class MultiMapAttention:
         """The finished heads of the whole step."""
         T, H, G, d, dv, window, ptr = proj.shape[0], self.H, self.G, self.d, self.dv, min(self.window, 1 << 30), ops._ptr
         long, dev = max(self.tc_min_portion, 1) if core and self.tc_min_portion is not None else 0, proj.get_device()      # 0: none is long
-        if long:
-            for i, (_, n, start, pages) in enumerate(tb.layout):
-                if n >= long and (start + n - 1) // page_size >= len(pages):         # the kernel would read on in the table
-                    raise IndexError(f"sequence {i}: {len(pages)} pages of {page_size} rows do not hold {start + n} positions")
         size = lib.kb2_seq_attention_step_workspace(tb.layout_ptr, tb.S, H, G, d, dv, window, long)
         o, work = torch.empty((T, H * dv), dtype=self.dtype, device=proj.device), torch.empty(size, dtype=torch.uint8, device=proj.device)
         rc = lib.kb2_seq_attention_step(proj.data_ptr(), proj.stride(0), tb.layout_ptr, tb.S, T, H, G, d, dv, ptr(self.bias), ptr(self.q_norm), ptr(self.k_norm),

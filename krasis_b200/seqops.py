@@ -94,6 +94,8 @@ def check(rc: int):
     msg = load().kb2_seq_last_error().decode()
     if rc == 2:
         raise ValueError(msg)
+    if rc == 4:
+        raise IndexError(msg)
     raise SeqOpsError(msg)
 
 
@@ -161,14 +163,12 @@ class StepTables:
         a[o_cu + S] = cu
         self.T, self.S, self.max_pages = T, S, maxp
         # host copy of the step's layout: (first row, tokens, first position, page list) per sequence
-        self.layout, row = [], 0
+        layout, row = [], 0
         for toks, start, _, pages in entries:
-            self.layout.append((row, len(toks), int(start), list(pages)))
+            layout.append((row, len(toks), int(start), list(pages)))
             row += len(toks)
+        self.layout = layout
         self.max_portion = max(len(e[0]) for e in entries)
-        # the same for the C interfaces: [S][4] int32, pages by their number
-        self.layout_host = np.array([(r, n, start, len(pages)) for r, n, start, pages in self.layout], dtype=np.int32)
-        self.layout_ptr = self.layout_host.ctypes.data
         if device_buf is not None:
             if device_buf.numel() != n:
                 raise ValueError("device_buf does not fit this step's tables")
@@ -181,6 +181,17 @@ class StepTables:
         self.tokens, self.positions, self.seq_of = self.buf[:T], self.buf[o_pos:o_pos + T], self.buf[o_seq:o_seq + T]
         self.cu, self.slots, self.pages = self.buf[o_cu:o_cu + S + 1], self.buf[o_slot:o_slot + S], self.buf[o_pg:]
         self.h2d_bytes = n * 4
+
+    @property
+    def layout(self):
+        return self._layout
+
+    @layout.setter
+    def layout(self, layout):
+        import numpy as np
+        self._layout = tuple(layout)                             # no changes in place: the C interfaces have a copy, [S][4] int32, pages by their number
+        self._layout_host = np.array([(r, n, start, len(pages)) for r, n, start, pages in self._layout], dtype=np.int32)
+        self.layout_ptr = self._layout_host.ctypes.data
 
 
 def portion_rows(tb: StepTables, s: int, first: int, ca: torch.Tensor, wa: int, cb: torch.Tensor, wb: int, page_size: int, proj: torch.Tensor,

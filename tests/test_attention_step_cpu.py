@@ -26,12 +26,30 @@ def _call(layout=((0, 130, 62, 3), (130, 1, 5, 1)), **kw):
     {"proj": None}, {"positions": None}, {"seq_of": None}, {"pages": None}, {"kc": None}, {"work": None}, {"out": None},
     {"T": 130}, {"T": 132}, {"layout": ((0, 130, 62, 3), (129, 1, 5, 1))}, {"layout": ((1, 130, 62, 3), (131, 1, 5, 1))}, {"layout": ((0, 132, 60, 3), (132, -1, 5, 1))},
     {"layout": ((0, 130, -1, 3), (130, 1, 5, 1))}, {"layout": ((0, 130, 2 ** 31 - 100, 3), (130, 1, 5, 1))}, {"layout": ((0, 130, 62, 4), (130, 1, 5, 1))},
-    {"layout": ((0, 130, 63, 3), (130, 1, 5, 1))},                                                                                  # 193 positions in three pages of 64
 ])
 def test_refused_ahead_of_the_first_launch(kw):
     rc, text = _call(**kw)
     assert rc == 2 and text.startswith("attention_step"), (rc, text)
 
 
+def test_pages_that_do_not_hold_a_long_portion():
+    rc, text = _call(layout=((0, 130, 63, 3), (130, 1, 5, 1)))            # 193 positions in three pages of 64
+    assert rc == 4 and text.startswith("attention_step"), (rc, text)
+
+
 def test_workspace_of_nothing():
     assert ops.load().kb2_seq_attention_step_workspace(None, 2, 4, 2, 128, 128, 1 << 20, 128) == 0
+
+
+def test_one_layout():
+    """The C interfaces see what StepTables.layout was set to, and it cannot be changed in place."""
+    import ctypes
+    tb = ops.StepTables([([5, 6, 7], 60, 0, [2, 1]), ([8], 9, 1, [0])], "cpu")
+
+    def seen():
+        return [tuple((ctypes.c_int * 4).from_address(tb.layout_ptr + 16 * i)) for i in range(tb.S)]
+    assert seen() == [(0, 3, 60, 2), (3, 1, 9, 1)] and list(tb.layout) == [(0, 3, 60, [2, 1]), (3, 1, 9, [0])]
+    tb.layout = [(0, 3, 30, [2]), (3, 1, 10, [0])]
+    assert seen() == [(0, 3, 30, 1), (3, 1, 10, 1)]
+    with pytest.raises(TypeError):
+        tb.layout[0] = (0, 3, 0, [])
