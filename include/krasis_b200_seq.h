@@ -143,16 +143,19 @@ KB2SEQ_API int kb2_seq_head_kv_prep(float* proj, long long ldp, int T, int H, in
                                     const int* seq_of, const int* pages, int max_pages, int page_size, void* kc, void* vc, int dt_cache,
                                     int norm_whole, int rot_half, const double* vfreq, float amp, int v_is_k, void* stream);
 
+/* Into how many pieces the keys of a step's tokens are cut, so that few tokens (decoding) reach the whole GPU: `blocks` is the number of blocks that there would be
+ * with one piece, keys the most that one of the tokens sees, room the most that the page lists hold (in eights of pages), least the fewest keys of a piece. */
+KB2SEQ_API int kb2_seq_key_pieces(long long blocks, long long keys, long long room, int least);
 /* Everything between the two products of an attention layer whose heads have one map and keys and values of their own, without gates, chunks or pooled blocks:
  * head_kv_prep, then per run of sequences portion_rows and `fmha` (the core library's kb2_fmha_maps_bf16; its error e comes back as 100 + e) for portions of
  * min_long tokens and more (0: none), paged_attn and attn_finish for the others.  layout (host): [S][4] first row, tokens, first position, pages; its rows follow one
- * another and are T in all.  Caches on 16 bytes; with min_long > 0 they and out are bf16, out on 16 bytes, d 128, dv 128 or 256, and a long portion's pages hold its
+ * another and are T in all.  replayed: the launches are captured and run again with later positions in the same tables.  Caches on 16 bytes; with min_long > 0 they and out are bf16, out on 16 bytes, d 128, dv 128 or 256, and a long portion's pages hold its
  * positions.  What does not fit comes back as KB2SEQ_ERR_VALUE, or KB2SEQ_ERR_RANGE for the pages, ahead of the first launch. */
-KB2SEQ_API size_t kb2_seq_attention_step_workspace(const int* layout, int S, int H, int G, int d, int dv, int window, int min_long);
+KB2SEQ_API size_t kb2_seq_attention_step_workspace(const int* layout, int S, int H, int G, int d, int dv, int max_pages, int page_size, int window, int min_long, int replayed);
 KB2SEQ_API int kb2_seq_attention_step(float* proj, long long ldp, const int* layout, int S, int T, int H, int G, int d, int dv, const float* bias,
                                       const float* qw, const float* kw, float eps, const double* freq, int rot_dims, const int* positions, const int* seq_of,
                                       const int* pages, int max_pages, int page_size, void* kc, void* vc, int dt_cache, int norm_whole, int rot_half, float amp,
-                                      int v_is_k, float scale, int window, float softcap, const float* sinks, const float* slopes, int min_long,
+                                      int v_is_k, float scale, int window, float softcap, const float* sinks, const float* slopes, int min_long, int replayed,
                                       void* fmha, void* work, size_t work_bytes, void* out, int dt_out, int device, void* stream);
 /* The bf16 operands of a portion's attention in one pass: cache rows `first` .. first + keys - 1 of a sequence (its page list `pages`, which holds
  * them all) of two bf16 caches with rows of wa and wb numbers (multiples of 8), side by side in a [keys][wa] and b [keys][wb]; and rows of nq fp32

@@ -1067,13 +1067,14 @@ template <typename F> int attn_runs(const AttnSeq* seq, int S, int min_long, F e
   }
   return KB2SEQ_OK;
 }
-size_t up16(size_t n) { return (n + 15) / 16 * 16; }
-// few tokens (decoding): each token's keys are cut into pieces so that the whole GPU works on them
-int attn_pieces(const AttnSeq* seq, int i, int j, int rows, int G, int window) {
-  int most = 1;
-  for (int q = i; q < j; ++q) most = std::max(most, std::min(window, seq[q].start + seq[q].n));
-  return std::max(1, std::min({296 / std::max(rows * G, 1), (most + 31) / 32, 64}));
+// the pieces of a run's keys on paged_attn
+int attn_pieces(const AttnSeq* seq, int i, int j, int rows, int G, int window, int max_pages, int page_size, int replayed) {
+  const long long room = std::min<long long>(window, (max_pages + 7ll) / 8 * 8 * page_size);
+  long long keys = 1;
+  for (int q = i; q < j; ++q) keys = std::max<long long>(keys, std::min(window, seq[q].start + seq[q].n));
+  return kb2_seq_key_pieces((long long)rows * G, replayed ? room : std::min(keys, room), room, kPAKT);
 }
+size_t up16(size_t n) { return (n + 15) / 16 * 16; }
 // Rows of a paged_attn block and its shared memory; 0: the sizes do not fit.
 int paged_attn_rows(int R, int M, int d, int dv, size_t* smem) {
   auto bytes = [&](int rb) { return (size_t)(2 * kPAKT + rb * d + kPAKT * ((M * d) | 1) + kPAKT * dv + rb * kPAKT + 3 * rb) * 4; };
@@ -1094,6 +1095,14 @@ struct AttnWork {                  // of a long portion: its keys, values and qu
 }  // namespace
 
 extern "C" {
+
+// Two blocks an SM.  A step that runs once is cut by its own keys, one that is captured by the most that its page lists hold, and both alike: where the keys' number
+// sets that of the pieces they have `least` keys each, and further ones are empty.  One piece alone is not joined, which rounds differently, hence two at least.
+KB2SEQ_API int kb2_seq_key_pieces(long long blocks, long long keys, long long room, int least) {
+  if (blocks <= 0 || keys <= 0 || room <= 0 || least <= 0) return 1;
+  const auto pieces = [&](long long k) { return std::max(1ll, std::min({2ll * kb2::current_sms() / blocks, (k + least - 1) / least, 64ll})); };
+  return (int)std::min(pieces(room), std::max(2ll, pieces(keys)));
+}
 
 KB2SEQ_API int kb2_seq_head_kv_prep(float* proj, long long ldp, int T, int H, int G, int M, int d, int dv, const float* bias,
                                     const float* qw, const float* kw, float eps, const double* freq, int rot_dims, const int* positions,
@@ -1206,7 +1215,7 @@ KB2SEQ_API int kb2_seq_attn_finish(const float* a, const float* part_acc, const 
 
 // ---- everything between an attention layer's two products, in one call: a mixed step is seven launches, and what a host needs for each of them from Python
 // took longer than the kernels (512 tokens beside three decoded ones: 93 us for 66).
-KB2SEQ_API size_t kb2_seq_attention_step_workspace(const int* layout, int S, int H, int G, int d, int dv, int window, int min_long) {
+KB2SEQ_API size_t kb2_seq_attention_step_workspace(const int* layout, int S, int H, int G, int d, int dv, int max_pages, int page_size, int window, int min_long, int replayed) {
   if (!layout || S <= 0) return 0;
   const AttnSeq* seq = reinterpret_cast<const AttnSeq*>(layout);
   size_t most = 16;
@@ -1217,7 +1226,7 @@ KB2SEQ_API size_t kb2_seq_attention_step_workspace(const int* layout, int S, int
         most = std::max(most, w.k + w.v + w.q);
       }
     } else {
-      const int pieces = attn_pieces(seq, i, j, rows, G, window);
+      const int pieces = attn_pieces(seq, i, j, rows, G, window, max_pages, page_size, replayed);
       most = std::max(most, (size_t)rows * H * (pieces > 1 ? (size_t)pieces * (dv + 2) : dv) * 4);
     }
     return KB2SEQ_OK;
@@ -1230,7 +1239,7 @@ KB2SEQ_API size_t kb2_seq_attention_step_workspace(const int* layout, int S, int
 KB2SEQ_API int kb2_seq_attention_step(float* proj, long long ldp, const int* layout, int S, int T, int H, int G, int d, int dv, const float* bias,
                                       const float* qw, const float* kw, float eps, const double* freq, int rot_dims, const int* positions, const int* seq_of,
                                       const int* pages, int max_pages, int page_size, void* kc, void* vc, int dt_cache, int norm_whole, int rot_half, float amp,
-                                      int v_is_k, float scale, int window, float softcap, const float* sinks, const float* slopes, int min_long,
+                                      int v_is_k, float scale, int window, float softcap, const float* sinks, const float* slopes, int min_long, int replayed,
                                       void* fmha, void* work, size_t work_bytes, void* out, int dt_out, int device, void* stream) {
   // all that a later launch would refuse or take for granted, ahead of the first one: that writes the caches
   if (!proj || !layout || !positions || !seq_of || !pages || !kc || !vc || !work || !out || S <= 0 || T <= 0 || H <= 0 || G <= 0 || H % G || d <= 0 || dv <= 0 ||
@@ -1251,7 +1260,7 @@ KB2SEQ_API int kb2_seq_attention_step(float* proj, long long ldp, const int* lay
   for (int q = 0; q < S; ++q)
     if (min_long > 0 && seq[q].n >= min_long && (seq[q].start + seq[q].n - 1) / page_size >= seq[q].pages)
       return failf(KB2SEQ_ERR_RANGE, "attention_step: sequence %d: %d pages of %d rows do not hold %d positions", q, seq[q].pages, page_size, seq[q].start + seq[q].n);
-  if (work_bytes < kb2_seq_attention_step_workspace(layout, S, H, G, d, dv, window, min_long) || ((uintptr_t)work & 15))
+  if (work_bytes < kb2_seq_attention_step_workspace(layout, S, H, G, d, dv, max_pages, page_size, window, min_long, replayed) || ((uintptr_t)work & 15))
     return failf(KB2SEQ_ERR_VALUE, "attention_step: workspace too small, or not on 16 bytes");
   int rc = kb2_seq_head_kv_prep(proj, ldp, T, H, G, 1, d, dv, bias, qw, kw, eps, freq, rot_dims, positions, seq_of, pages, max_pages, page_size, kc, vc, dt_cache,
                                 norm_whole, rot_half, nullptr, amp, v_is_k, stream);
@@ -1273,7 +1282,7 @@ KB2SEQ_API int kb2_seq_attention_step(float* proj, long long ldp, const int* lay
       }
       return KB2SEQ_OK;
     }
-    const int pieces = attn_pieces(seq, i, j, rows, G, window);
+    const int pieces = attn_pieces(seq, i, j, rows, G, window, max_pages, page_size, replayed);
     float* acc = (float*)work;
     float* ml = pieces > 1 ? acc + (size_t)rows * H * pieces * dv : nullptr;
     if (int e = kb2_seq_paged_attn(proj + r0 * ldp, ldp, rows, H, G, 1, d, dv, kc, vc, dt_cache, positions + r0, seq_of + r0, pages, max_pages, page_size, scale, 0,

@@ -279,11 +279,8 @@ class WindowLatentAttention:
                 q_abs = torch.empty((n, H, self.r), dtype=torch.float32, device=h.device)
                 lin_heads(q[r0:r0 + n, :, :self.dn], self.uk_t, q_abs)
                 o_lat = torch.empty((n, H, self.r), dtype=torch.float32, device=h.device)
-                # few tokens (decoding): each token's keys are cut into pieces so that the whole GPU works on them
-                blocks = n * ((H + 7) // 8)
-                # by the room of the page lists, in eights as captured steps have them: steps that are replayed cut as others do
-                max_keys = min(self.window, (tb.max_pages + 7) // 8 * 8 * page_size)
-                nsplit = max(1, min(296 // max(blocks, 1), (max_keys + 7) // 8, 64))
+                room = min(self.window, tb.room(page_size))
+                nsplit = lib.kb2_seq_key_pieces(n * ((H + 7) // 8), room, room, 8)
                 part_acc = torch.empty((n, nsplit, H, self.r), dtype=torch.float32, device=h.device) if nsplit > 1 else None
                 part_ml = torch.empty((n, nsplit, H, 2), dtype=torch.float32, device=h.device) if nsplit > 1 else None
                 ops.check(lib.kb2_seq_latent_window_attn(q_abs.data_ptr(), _row(proj, r0), ldp, n, H, self.dn, self.dr, self.r,
@@ -907,12 +904,12 @@ class MultiMapAttention:
         """The finished heads of the whole step."""
         T, H, G, d, dv, window, ptr = proj.shape[0], self.H, self.G, self.d, self.dv, min(self.window, 1 << 30), ops._ptr
         long, dev = max(self.tc_min_portion, 1) if core and self.tc_min_portion is not None else 0, proj.get_device()      # 0: none is long
-        size = lib.kb2_seq_attention_step_workspace(tb.layout_ptr, tb.S, H, G, d, dv, window, long)
+        size = lib.kb2_seq_attention_step_workspace(tb.layout_ptr, tb.S, H, G, d, dv, tb.max_pages, page_size, window, long, tb.replayed)
         o, work = torch.empty((T, H * dv), dtype=self.dtype, device=proj.device), torch.empty(size, dtype=torch.uint8, device=proj.device)
         rc = lib.kb2_seq_attention_step(proj.data_ptr(), proj.stride(0), tb.layout_ptr, tb.S, T, H, G, d, dv, ptr(self.bias), ptr(self.q_norm), ptr(self.k_norm),
                                         self.eps, ptr(self.freq), self.rot_dims, tb.positions.data_ptr(), tb.seq_of.data_ptr(), tb.pages.data_ptr(),
                                         tb.max_pages, page_size, kc.data_ptr(), vc.data_ptr(), dtc, self.norm_whole, self.rot_half, self.rot_amp, self.kv_one,
-                                        self.scale, window, self.softcap, ptr(self.sink), ptr(self.slopes), long, _fmha_maps(core) if long else None,
+                                        self.scale, window, self.softcap, ptr(self.sink), ptr(self.slopes), long, tb.replayed, _fmha_maps(core) if long else None,
                                         work.data_ptr(), size, o.data_ptr(), ops.dt_code(self.dtype), dev, s)
         if rc >= 100:
             _core_check(rc - 100)
@@ -940,11 +937,10 @@ class MultiMapAttention:
                                              self.tc_min_portion, self.softcap, None if pool_only else ops._ptr(self.sink), self.pool, ops._ptr(kp),
                                              ops._ptr(vp), int(pool_only), None if pool_only else ops._ptr(self.slopes), s))
         if core is None:
-            # few tokens (decoding): each token's keys are cut into pieces so that the whole GPU works on them
-            reach = min(self.window, self.chunk) if self.chunk else self.window
-            ends = [start + n for _, n, start, _ in (tb.layout[q] for q in seqs)]
-            max_keys = max(min(reach, e) + (e // self.pool if self.pool else 0) for e in ends)
-            nsplit = max(1, min(296 // max(T * G, 1), (max_keys + 31) // 32, 64))
+            reach = min(window, self.chunk) if self.chunk else window
+            room, *keys = (min(reach, e) + (e // self.pool if self.pool else 0)
+                           for e in [tb.room(page_size)] + [start + n for _, n, start, _ in (tb.layout[q] for q in seqs)])
+            nsplit = lib.kb2_seq_key_pieces(T * G, room if tb.replayed else max(keys), room, 32)
             if nsplit > 1:
                 part_acc = torch.empty((T * H * M, nsplit, self.dv), dtype=torch.float32, device=dev)
                 part_ml = torch.empty((T * H * M, nsplit, 2), dtype=torch.float32, device=dev)

@@ -36,9 +36,10 @@ SIGNATURES = {
     "kb2_seq_delta_rule_ch": (_I, [_P, _I, _P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _F, _P, _P, _P, _P, _P, _I, _P]),
     "kb2_seq_residual_add_norm": (_I, [_P, _P, _P, _P, _P, _P, _I, _I, _I, _F, _P]),
     "kb2_seq_head_kv_prep": (_I, [_P, _L, _I, _I, _I, _I, _I, _I, _P, _P, _P, _F, _P, _I, _P, _P, _P, _I, _I, _P, _P, _I, _I, _I, _P, _F, _I, _P]),
-    "kb2_seq_attention_step_workspace": (C.c_size_t, [_P, _I, _I, _I, _I, _I, _I, _I]),
+    "kb2_seq_key_pieces": (_I, [_L, _L, _L, _I]),
+    "kb2_seq_attention_step_workspace": (C.c_size_t, [_P] + [_I] * 10),
     "kb2_seq_attention_step": (_I, [_P, _L, _P, _I, _I, _I, _I, _I, _I, _P, _P, _P, _F, _P, _I, _P, _P, _P, _I, _I, _P, _P, _I, _I, _I, _F, _I, _F, _I, _F, _P, _P,
-                                    _I, _P, _P, C.c_size_t, _P, _I, _I, _P]),
+                                    _I, _I, _P, _P, C.c_size_t, _P, _I, _I, _P]),
     "kb2_seq_portion_rows": (_I, [_P, _I, _P, _I, _P, _I, _I, _I, _P, _P, _P, _L, _I, _I, _P, _P]),
     "kb2_seq_kv_pool": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _I, _P]),
     "kb2_seq_paged_attn": (_I, [_P, _L, _I, _I, _I, _I, _I, _I, _P, _P, _I, _P, _P, _P, _I, _I, _F, _I, _I, _P, _I, _P, _P, _P, _I, _F, _P, _I,
@@ -162,6 +163,7 @@ class StepTables:
             cu += k
         a[o_cu + S] = cu
         self.T, self.S, self.max_pages = T, S, maxp
+        self.replayed = device_buf is not None                   # launches that read the tables may run again with others in their place
         # host copy of the step's layout: (first row, tokens, first position, page list) per sequence
         layout, row = [], 0
         for toks, start, _, pages in entries:
@@ -181,6 +183,10 @@ class StepTables:
         self.tokens, self.positions, self.seq_of = self.buf[:T], self.buf[o_pos:o_pos + T], self.buf[o_seq:o_seq + T]
         self.cu, self.slots, self.pages = self.buf[o_cu:o_cu + S + 1], self.buf[o_slot:o_slot + S], self.buf[o_pg:]
         self.h2d_bytes = n * 4
+
+    def room(self, page_size: int) -> int:
+        """Positions that page lists of this width hold, the width in eights as it is in the tables of captured steps."""
+        return (self.max_pages + 7) // 8 * 8 * page_size
 
     @property
     def layout(self):

@@ -14,7 +14,7 @@ def _call(layout=((0, 130, 62, 3), (130, 1, 5, 1)), **kw):
     table = np.array(layout, dtype=np.int32)
     rc = ops.load().kb2_seq_attention_step(a["proj"], 1024, table.ctypes.data, a["S"], a["T"], a["H"], a["G"], a["d"], a["dv"], None, None, None, 1e-6, None, 0,
                                            a["positions"], a["seq_of"], a["pages"], a["max_pages"], a["page_size"], a["kc"], a["vc"], a["dt_cache"], 0, 0, 1.0, 0,
-                                           a["scale"], a["window"], a["softcap"], None, None, a["min_long"], a["fmha"], a["work"], a["work_bytes"], a["out"],
+                                           a["scale"], a["window"], a["softcap"], None, None, a["min_long"], 0, a["fmha"], a["work"], a["work_bytes"], a["out"],
                                            a["dt_out"], 0, None)
     return rc, ops.load().kb2_seq_last_error().decode()
 
@@ -37,8 +37,25 @@ def test_pages_that_do_not_hold_a_long_portion():
     assert rc == 4 and text.startswith("attention_step"), (rc, text)
 
 
+@pytest.mark.parametrize("blocks", [1, 2, 3, 7, 20, 147, 148, 149, 296, 297, 5000])
+@pytest.mark.parametrize("least", [8, 32])
+def test_pieces_of_a_step_and_of_its_replay(blocks, least):
+    """Cut by its own keys or by the room: the pieces that have keys are the same, and a row is joined in both or in neither."""
+    pieces = ops.load().kb2_seq_key_pieces
+
+    def cut(keys, n):
+        size = -(-(-(-keys // n)) // least) * least
+        return [(a, min(keys, a + size)) for a in range(0, keys, size)]
+    for room in (1, 8, 40, 512, 4096, 1 << 20):
+        for keys in sorted({1, 7, 31, 32, 33, 64, 65, 500, 2047, 2048, 2049, 4000, room} | {room - 1 if room > 1 else 1}):
+            if keys <= room:
+                one, many = pieces(blocks, keys, room, least), pieces(blocks, room, room, least)
+                assert 1 <= one <= many <= 64 and (one == 1) == (many == 1) and cut(keys, one) == cut(keys, many)
+                assert many == 1 or blocks * many <= 2 * 148
+
+
 def test_workspace_of_nothing():
-    assert ops.load().kb2_seq_attention_step_workspace(None, 2, 4, 2, 128, 128, 1 << 20, 128) == 0
+    assert ops.load().kb2_seq_attention_step_workspace(None, 2, 4, 2, 128, 128, 3, 64, 1 << 20, 128, 0) == 0
 
 
 def test_one_layout():
