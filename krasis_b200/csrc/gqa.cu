@@ -296,11 +296,13 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 //   tmap_v   [kv_len][*]: this head's values at column v_col0 + kvh * DV
 // A tile is a chain: S = Q K^T, the row maxima, exponentials, O += P V.  S and P have two buffers each, so the tensor pipe makes the S of the next two tiles
 // while the softmax warps work, and these hardly wait for it; K and V have a loader each.  An MMA reads its 128 x 16 piece of Q from shared memory again, 32
-// cycles for 32 of work with 64 keys: tiles of 128 where tensor memory has room.  What is left: with 128 value columns the exponentials (64 x 128 of them take
-// 1030 cycles of the special function units, a tile 2400), with 256 the MMAs (1280 cycles of 1570 a tile; the whole runs at the power limit).  us with
-// single buffers, one loader and tiles of 64 keys, and now: 2048 x 16 heads of 256 after 2500 keys 140 -> 134; latent attention of 1000 tokens, 16 heads 20.2 ->
-// 16.7, 100 tokens after 2000 32.6 -> 25.8; 2048 tokens, 16 heads of 128 36.6 -> 29.7; 17 tokens after 300 9.2 -> 9.8 (latent), 20.7 -> 20.4 (256).  Tried: the
-// tiles to two groups of warps in turn, a thread per row (latent 18.0: its warps are one per scheduler); pairs of CTAs with heads of 256 (164).
+// cycles for 32 of work with 64 keys: tiles of 128 where tensor memory has room.  Where the last tile has keys in its first 64 alone, the softmax warps and the
+// second product take that half: the same bits, as the others have weight 0.  What is left: with 128 value columns the softmax (17 tokens after 1000 and 3000 keys
+// 14.6 and 32.1 us: 1.12 us a tile, 0.53 of it the exponentials, 16 of them a cycle), with 256 the MMAs (17.2 and 40.5 us: 0.75 us a tile of 64).  us with single
+// buffers, one loader and tiles of 64 keys, and now: 2048 x 16 heads of 256 after 2500 keys 140 -> 134; latent attention of 16 heads: 2000 tokens 36.9 -> 32.0, 1000
+// 19.4 -> 16.4, 512 after 700 21.8 -> 18.5, 17 after 300 9.2 -> 8.3, 128 alone 7.5 -> 8.2 (one tile where two overlapped), 64 alone 5.9 -> 6.2 (7.2 without the half);
+// 16 heads of 128, 2000 tokens 36.3 -> 29.5.  Tried: the tiles to two groups of warps in turn, a thread per row (latent 18.0: its warps are one per scheduler); pairs
+// of CTAs with heads of 256 (164); boxes of 64 rows and a first product of half a tile (1000 tokens 17.1); the half chosen within the loop (17 after 3000: 33.1).
 template <int DQ, int DV, bool PE>
 __global__ void __launch_bounds__(kFThreads, 1)
     gqa_fmha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -347,6 +349,8 @@ __global__ void __launch_bounds__(kFThreads, 1)
   // every role counts tiles from tile0 (TMA coordinates and key positions add it back)
   const int tile0 = max(0, q_start + q0 - window + 1) / FK;
   const int n_tiles = (n_keys + FK - 1) / FK - tile0;
+  // the last tile may have keys in its first 64 alone: then nobody looks at the others
+  const int whole = n_tiles - (FK > 64 && n_tiles > 0 && n_keys - (n_tiles - 1 + tile0) * FK <= 64);
 
   if (threadIdx.x == 96) {
     if (smem_u32(smem) & 1023u) __trap();
@@ -428,10 +432,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
         }
         __syncwarp();
       };
-      issue_s(0);
-      if (n_tiles > 1) issue_s(1);
-      for (int it = 0; it < n_tiles; ++it) {
-        if (it + 2 < n_tiles) issue_s(it + 2);
+      const auto issue_o = [&](auto steps, int it) {      // O += P(it) V(it), over 16 keys a step
         const int b = it & 1, st = it % KS;
         mbar_wait(&v_full[st], it / KS & 1);
         mbar_wait(&p_full[b], it >> 1 & 1);
@@ -439,7 +440,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
         const uint32_t v_addr = smem_u32(smem + L::kOffV + st * L::kVBytes);
         if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < FK / 16; ++k) {
+          for (int k = 0; k < decltype(steps)::value; ++k) {
             const uint64_t bd = umma_desc_mn_sw128(v_addr + k * 2048, FK * 128, 1024);
             umma_bf16_ts(tmem_base + kColO, tmem_base + kColP + b * (FK / 2) + 8 * k, bd, id_o, (it == 0 && k == 0) ? 0u : 1u);
           }
@@ -447,7 +448,14 @@ __global__ void __launch_bounds__(kFThreads, 1)
           umma_commit(&v_empty[st]);
         }
         __syncwarp();
+      };
+      issue_s(0);
+      if (n_tiles > 1) issue_s(1);
+      for (int it = 0; it < whole; ++it) {
+        if (it + 2 < n_tiles) issue_s(it + 2);
+        issue_o(std::integral_constant<int, FK / 16>{}, it);
       }
+      if (whole < n_tiles) issue_o(std::integral_constant<int, 4>{}, whole);
     }
   } else if (warp == 2) {
     if (n_tiles > 0 && elect_one()) {
@@ -458,7 +466,8 @@ __global__ void __launch_bounds__(kFThreads, 1)
     }
   } else if (warp >= 4) {
     // ------------------------------------------------------------ softmax + epilogue: two threads per query row.
-    // Warp w serves TMEM lane quarter q = w & 3; warps 4-7 take the first half of a tile's key columns and of the O columns, warps 8-11 the second.
+    // Warp w serves TMEM lane quarter q = w & 3; warps 4-7 take the first 32 of every 64 keys of a tile and the first half of the O columns, warps 8-11 the
+    // others: a row's sums are the same whether its last tile is taken whole or by half.
     // The two threads of a row exchange their tile maxima through smem (one 64-thread named barrier per tile), make identical running-max decisions,
     // and keep partial row sums that are added once at the end.
     const int q = warp & 3, hf = (warp - 4) >> 2;
@@ -467,7 +476,7 @@ __global__ void __launch_bounds__(kFThreads, 1)
     const int q_pos = q_start + qi;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     float* xchg = reinterpret_cast<float*>(smem + L::kOffXchg);
-    constexpr int KH = FK / 2, OH = DV / 2;
+    constexpr int OH = DV / 2;
     float m_ref = -INFINITY, l_sum = 0.f;
     // the penalty in units of the raw scores, so that the scale folded into the exponent applies to both
     const float slope = slopes != nullptr ? slopes[head] * 1.4426950408889634f / sm_scale_log2 : 0.f;
@@ -481,40 +490,57 @@ __global__ void __launch_bounds__(kFThreads, 1)
       mbar_wait(&pv_done[it & 1], it >> 1 & 1);
       tc_fence_after_sync();
     };
-    for (int it = 0; it < n_tiles; ++it) {
+    const auto tile = [&](auto runs, int it) {       // runs of 32 keys that a thread takes: all of a tile's, or of half a tile the one
+      constexpr int NB = decltype(runs)::value;
       const int b = it & 1;
       mbar_wait(&s_full[b], it >> 1 & 1);
       tc_fence_after_sync();
-      float s[KH];                                   // raw scores (the softmax scale is folded into the exponent FMA)
+      float s[NB][32];                               // raw scores (the softmax scale is folded into the exponent FMA)
       {
-        uint32_t r[KH / 16][16];
+        uint32_t r[NB][2][16];
 #pragma unroll
-        for (int c = 0; c < KH / 16; ++c) tmem_ld16(lane_addr + kColS + b * FK + hf * KH + 16 * c, r[c]);
+        for (int n = 0; n < NB; ++n) {
+          tmem_ld16(lane_addr + kColS + b * FK + n * 64 + hf * 32, r[n][0]);
+          tmem_ld16(lane_addr + kColS + b * FK + n * 64 + hf * 32 + 16, r[n][1]);
+        }
         tmem_ld_wait();
 #pragma unroll
-        for (int jj = 0; jj < KH; ++jj) s[jj] = __uint_as_float(r[jj / 16][jj % 16]);
+        for (int n = 0; n < NB; ++n)
+#pragma unroll
+          for (int jj = 0; jj < 32; ++jj) s[n][jj] = __uint_as_float(r[n][jj / 16][jj % 16]);
       }
       tell(&s_cons[b]);                              // S may be overwritten by QK^T(it + 2)
       if (cap_in != 0.f) {                           // tanh(x) = 1 - 2 / (2^(2 x log2 e) + 1): exact limits at +-inf, two MUFU ops per score
         const float c2 = cap_in * 2.8853900817779268f;
 #pragma unroll
-        for (int jj = 0; jj < KH; ++jj) s[jj] = cap_out * (1.f - __fdividef(2.f, ex2_approx(s[jj] * c2) + 1.f));
+        for (int n = 0; n < NB; ++n)
+#pragma unroll
+          for (int jj = 0; jj < 32; ++jj) s[n][jj] = cap_out * (1.f - __fdividef(2.f, ex2_approx(s[n][jj] * c2) + 1.f));
       }
-      const int key0 = (it + tile0) * FK + hf * KH;
+      const int key0 = (it + tile0) * FK + hf * 32;
       if (slope != 0.f) {
         const float back = (float)(key0 - q_pos);            // minus the distance; invisible keys are masked below whatever this gives
 #pragma unroll
-        for (int jj = 0; jj < KH; ++jj) s[jj] = fmaf(slope, back + (float)jj, s[jj]);
-      }
-      // causal / length / window mask only where a key of this half-tile can be invisible to a row of this warp (warp-uniform)
-      if (key0 + KH - 1 > q_start + q0 + q * 32 || key0 + KH > kv_len || key0 + window <= q_start + q0 + q * 32 + 31) {
+        for (int n = 0; n < NB; ++n)
 #pragma unroll
-        for (int jj = 0; jj < KH; ++jj)
-          if (key0 + jj > q_pos || key0 + jj >= kv_len || key0 + jj + window <= q_pos) s[jj] = -INFINITY;
+          for (int jj = 0; jj < 32; ++jj) s[n][jj] = fmaf(slope, back + (float)(n * 64 + jj), s[n][jj]);
+      }
+      // causal / length / window mask only where one of the thread's keys can be invisible to a row of this warp (warp-uniform)
+      constexpr int kLast = (NB - 1) * 64 + 31;
+      if (key0 + kLast > q_start + q0 + q * 32 || key0 + kLast >= kv_len || key0 + window <= q_start + q0 + q * 32 + 31) {
+#pragma unroll
+        for (int n = 0; n < NB; ++n)
+#pragma unroll
+          for (int jj = 0; jj < 32; ++jj) {
+            const int key = key0 + n * 64 + jj;
+            if (key > q_pos || key >= kv_len || key + window <= q_pos) s[n][jj] = -INFINITY;
+          }
       }
       float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int jj = 0; jj < KH; jj += 2) mx[jj >> 1 & 3] = max3(mx[jj >> 1 & 3], s[jj], s[jj + 1]);
+      for (int n = 0; n < NB; ++n)
+#pragma unroll
+        for (int jj = 0; jj < 32; jj += 2) mx[jj >> 1 & 3] = max3(mx[jj >> 1 & 3], s[n][jj], s[n][jj + 1]);
       float m_tile = max3(fmaxf(mx[0], mx[1]), mx[2], mx[3]);
       float* xb = xchg + b * (2 * kFQ);
       xb[hf * kFQ + row] = m_tile;
@@ -535,14 +561,17 @@ __global__ void __launch_bounds__(kFThreads, 1)
       const float neg_m = (m_ref == -INFINITY) ? 0.f : -m_ref;   // row fully masked so far: every s is -inf -> p = 0
       const uint64_t scale2 = pair_of(sm_scale_log2, sm_scale_log2), neg2 = pair_of(neg_m, neg_m);
       uint64_t psum[2] = {0, 0};                     // two numbers each
-      uint32_t pk[KH / 32][16];
+      uint32_t pk[NB][16];
 #pragma unroll
-      for (int jj = 0; jj < KH; jj += 2) {
-        const float2 e = pair_get(pair_fma(pair_of(s[jj], s[jj + 1]), scale2, neg2));
-        const uint32_t pb = bf16x2_bits_rn(ex2_approx(e.y), ex2_approx(e.x));
-        // normalise with the values the MMA actually uses
-        psum[jj >> 1 & 1] = pair_add(psum[jj >> 1 & 1], pair_of(__uint_as_float(pb << 16), __uint_as_float(pb & 0xFFFF0000u)));
-        pk[jj / 32][jj / 2 % 16] = pb;
+      for (int n = 0; n < NB; ++n) {
+#pragma unroll
+        for (int jj = 0; jj < 32; jj += 2) {
+          const float2 e = pair_get(pair_fma(pair_of(s[n][jj], s[n][jj + 1]), scale2, neg2));
+          const uint32_t pb = bf16x2_bits_rn(ex2_approx(e.y), ex2_approx(e.x));
+          // normalise with the values the MMA actually uses
+          psum[jj >> 1 & 1] = pair_add(psum[jj >> 1 & 1], pair_of(__uint_as_float(pb << 16), __uint_as_float(pb & 0xFFFF0000u)));
+          pk[n][jj / 2] = pb;
+        }
       }
       const float2 sum2 = pair_get(pair_add(psum[0], psum[1]));
       l_sum = l_sum * scale_o + (sum2.x + sum2.y);
@@ -563,10 +592,13 @@ __global__ void __launch_bounds__(kFThreads, 1)
         }
       }
 #pragma unroll
-      for (int c = 0; c < KH / 32; ++c) tmem_st16(lane_addr + kColP + b * (FK / 2) + hf * (KH / 2) + c * 16, pk[c]);
+      for (int n = 0; n < NB; ++n)
+        tmem_st16(lane_addr + kColP + b * (FK / 2) + n * 32 + hf * 16, pk[n]);
       tmem_st_wait();
       tell(&p_full[b]);
-    }
+    };
+    for (int it = 0; it < whole; ++it) tile(std::integral_constant<int, FK / 64>{}, it);
+    if (whole < n_tiles) tile(std::integral_constant<int, 1>{}, whole);
     if (n_tiles > 0) {
       float* xb = xchg + (n_tiles & 1) * (2 * kFQ);   // the buffer the last tile did not use
       if (sinks != nullptr && hf == 0 && m_ref != -INFINITY) l_sum += ex2_approx(fmaf(sinks[head], 1.4426950408889634f, -m_ref));

@@ -57,3 +57,29 @@ def test_latent(past, M):
         capi.check(core.kb2_fmha_latent_gated(q.data_ptr(), up.data_ptr(), kr.data_ptr(), out.data_ptr(), M, past, L, H, 192 ** -0.5, window, None, None, 0, dev,
                                               stream_on(dev)))
         _check(out, q, torch.cat([kn, kr[:, None].expand(L, H, 64)], -1), v, past, 192 ** -0.5, window)
+
+
+@pytest.mark.parametrize("past,M,more", [(0, 1, 90), (0, 64, 1), (0, 63, 200), (60, 4, 1), (64, 64, 64), (100, 28, 9), (130, 62, 1), (1000, 24, 100)])
+def test_rows_of_half_tiles(past, M, more):
+    """A last tile with keys in its first half alone: the rows that the same queries have where later ones fill it, bit for bit."""
+    core, H, G, L = capi.load(), 3, 1, past + M + more
+    g = torch.Generator(device="cuda").manual_seed(past + M)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()  # noqa: E731
+    dev = torch.cuda.current_device()
+    q, up, kr = r(M + more, H, 192), r(L, H * 256), r(L, 64)
+    q2, k2 = r(M + more, H, 128), r(L, G, 128)
+    for window in (1 << 30, 70):
+        got = []
+        for m in (M, M + more):
+            out = torch.empty(m, H, 128, device="cuda", dtype=torch.bfloat16)
+            capi.check(core.kb2_fmha_latent_gated(q.data_ptr(), up.data_ptr(), kr.data_ptr(), out.data_ptr(), m, past, past + m, H, 192 ** -0.5, window, None, None, 0, dev,
+                                                  stream_on(dev)))
+            parts = [out[:M]]
+            for dv in (128, 256):
+                v = up[:, :dv].contiguous()
+                out, lse = torch.empty(m, H, dv, device="cuda"), torch.empty(m, H, device="cuda")
+                capi.check(core.kb2_fmha_maps_slopes(q2.data_ptr(), k2.data_ptr(), v.data_ptr(), out.data_ptr(), m, past, past + m, H, G, 1, dv, 128 ** -0.5, 0.0, window,
+                                                     None, lse.data_ptr(), None, dev, stream_on(dev)))
+                parts += [out[:M], lse[:M]]
+            got.append(parts)
+        assert all(torch.equal(a, b) and bool(torch.isfinite(a).all()) for a, b in zip(*got))
