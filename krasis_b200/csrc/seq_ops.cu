@@ -961,6 +961,8 @@ __global__ void __launch_bounds__(512) latent_prep_kernel(float* __restrict__ pr
 //   values    a thread owns NC columns for all HG heads: one read of a latent element serves HG sums
 // Bound where few tokens decode: latency, a chain of position, page, key rows and four phases on them.  Loads of a phase go out together, and the key range is
 // cut into pieces of 8 keys and more, so that short contexts reach all SMs, too (4 tokens x 16 heads, 116 keys, from HBM: pieces of 32 18.6 us, now 11.4).
+// Where many do: instructions.  A thread finds its next unit of a row by addition, and the lanes' step through the scores is a constant in two forms of the loop or
+// three: a layer of 16 heads, 127 tokens after 1000 keys, with a division per unit and a variable step 434 us (bf16) and 1443 (fp32, 4 bytes a load), now 362 and 458.
 // gate [T, ldg] (may be null): head h's output is multiplied by sigmoid(gate[t, h]); it commutes with the value up-projection.
 constexpr int kAttnThreads = 256, kAttnAcc = 16, kAttnKT = 32, kAttnWarps = kAttnThreads / 32;
 constexpr int kAttnPiece = 8;              // keys of a piece are a multiple of this
@@ -978,7 +980,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) latent_window_attn_kernel(
     const void* __restrict__ ckv, const void* __restrict__ kr, int dt_cache, const int* __restrict__ positions,
     const int* __restrict__ seq_of, const int* __restrict__ pages, int max_pages, int page_size, const float* __restrict__ sinks,
     float scale, int window, float* __restrict__ out, const int* __restrict__ cu, int skip_from, int nsplit,
-    float* __restrict__ part_acc, float* __restrict__ part_ml, const float* __restrict__ gate, long long ldg, bool vec_q) {
+    float* __restrict__ part_acc, float* __restrict__ part_ml, const float* __restrict__ gate, long long ldg, bool vec_q, bool vec_k) {
   kb2::pdl_enter(q_abs, proj, ckv, kr, positions, seq_of, pages, sinks, out, cu, part_acc, part_ml, gate);
   static_assert(HG <= kAttnWarps, "a warp per head runs the softmax");
   constexpr int KT = kAttnKT;
@@ -1057,6 +1059,9 @@ __global__ void __launch_bounds__(kAttnThreads, 2) latent_window_attn_kernel(
   for (int c = 0; c < NC; ++c)
 #pragma unroll
     for (int hh = 0; hh < HG; ++hh) acc[c][hh] = 0.f;
+  // numbers of 16 bytes of a cache row, and such units a row (0: rows that are not made of them)
+  const int unit = dt_cache ? 8 : 4, units = vec_k ? D / unit : 0;
+  const int first_k = units ? tid / units : 0, first_d = tid - first_k * units, ahead_k = units ? kAttnThreads / units : 0, ahead_d = kAttnThreads - ahead_k * units;
   const int seg = (n4 + kAttnWarps - 1) / kAttnWarps, u_lo = min(n4, warp * seg), u_hi = min(n4, u_lo + seg);
   for (int j0 = j_begin; j0 <= j_end; j0 += KT) {
     const int nk = min(KT, j_end - j0 + 1);
@@ -1065,26 +1070,38 @@ __global__ void __launch_bounds__(kAttnThreads, 2) latent_window_attn_kernel(
       if (tid < nk) krow[tid] = row_of(j0 + tid);
       __syncthreads();
     }
-    if (dt_cache == 1 && (r & 7) == 0 && (dr & 7) == 0) {
-      const int D8 = D >> 3;
-      for (int base = tid; base < nk * D8; base += 4 * kAttnThreads) {      // four loads of a thread in flight
-        uint4 v[4];
+    if (units) {
+      // 16 bytes at a time, three loads of a thread in flight; a thread's next unit is ahead_k rows and ahead_d units on
+      for (int k = first_k, d = first_d; k < nk;) {
+        constexpr int kAhead = 3;
+        uint4 v[kAhead];
+        int at[kAhead];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int i = base + j * kAttnThreads;
-          if (i >= nk * D8) continue;
-          const int k = i / D8, d = (i - k * D8) << 3;
-          v[j] = *reinterpret_cast<const uint4*>(d < r ? (const bf16*)ckv + krow[k] * r + d : (const bf16*)kr + krow[k] * dr + (d - r));
+        for (int j = 0; j < kAhead; ++j) {
+          const int c = d * unit;
+          at[j] = k < nk ? k * DP + c : -1;
+          if (k < nk) {
+            const long long row = krow[k];
+            v[j] = *reinterpret_cast<const uint4*>((const char*)(c < r ? ckv : kr) + ((c < r ? row * r + c : row * dr + (c - r)) << (dt_cache ? 1 : 2)));
+          }
+          k += ahead_k;
+          d += ahead_d;
+          if (d >= units) {
+            d -= units;
+            ++k;
+          }
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int i = base + j * kAttnThreads;
-          if (i >= nk * D8) continue;
-          const int k = i / D8, d = (i - k * D8) << 3;
-          float f[8];
-          unpack8(v[j], f);
-          *reinterpret_cast<float4*>(kt + k * DP + d) = make_float4(f[0], f[1], f[2], f[3]);
-          *reinterpret_cast<float4*>(kt + k * DP + d + 4) = make_float4(f[4], f[5], f[6], f[7]);
+        for (int j = 0; j < kAhead; ++j) {
+          if (at[j] < 0) continue;
+          if (dt_cache) {
+            float f[8];
+            unpack8(v[j], f);
+            *reinterpret_cast<float4*>(kt + at[j]) = make_float4(f[0], f[1], f[2], f[3]);
+            *reinterpret_cast<float4*>(kt + at[j] + 4) = make_float4(f[4], f[5], f[6], f[7]);
+          } else {
+            *reinterpret_cast<uint4*>(kt + at[j]) = v[j];
+          }
         }
       }
     } else {
@@ -1095,15 +1112,17 @@ __global__ void __launch_bounds__(kAttnThreads, 2) latent_window_attn_kernel(
     }
     __syncthreads();
     // scores: a lane per key, a piece of the dimensions per warp, all heads of the group; of up to 8 or 16 keys four or two lanes share one
-    {
-      const int keys = nk <= 8 ? 8 : nk <= 16 ? 16 : 32, key = lane & (keys - 1), step = 32 / keys;
+    const auto scores = [&](auto lanes) {
+      constexpr int kKeys = decltype(lanes)::value, kStep = 32 / kKeys;
+      const int key = lane & (kKeys - 1);
       float s[HG];
 #pragma unroll
       for (int hh = 0; hh < HG; ++hh) s[hh] = 0.f;
       if (key < nk) {
         const float4* kk = reinterpret_cast<const float4*>(kt + key * DP);
         const float4* qq = reinterpret_cast<const float4*>(qs);
-        for (int u = u_lo + lane / keys; u < u_hi; u += step) {
+#pragma unroll(kKeys == 32 ? 2 : 1)
+        for (int u = u_lo + lane / kKeys; u < u_hi; u += kStep) {
           const float4 kv = kk[u];
 #pragma unroll
           for (int hh = 0; hh < HG; ++hh) {
@@ -1115,12 +1134,16 @@ __global__ void __launch_bounds__(kAttnThreads, 2) latent_window_attn_kernel(
           }
         }
       }
-      for (int o = keys; o < 32; o <<= 1)
+#pragma unroll
+      for (int o = kKeys; o < 32; o <<= 1)
 #pragma unroll
         for (int hh = 0; hh < HG; ++hh) s[hh] += __shfl_xor_sync(0xffffffffu, s[hh], o);
 #pragma unroll
       for (int hh = 0; hh < HG; ++hh) sp[(warp * HG + hh) * KT + lane] = s[hh];
-    }
+    };
+    if (nk > 16) scores(std::integral_constant<int, 32>{});
+    else if (nk > 8) scores(std::integral_constant<int, 16>{});
+    else scores(std::integral_constant<int, 8>{});
     __syncthreads();
     // running softmax: warp hh serves head hh
     if (warp < HG) {
@@ -2698,6 +2721,8 @@ KB2SEQ_API int kb2_seq_latent_window_attn(const float* q_abs, const float* proj,
   const size_t smem = attn_smem_floats(HG, D) * 4;
   if (smem > 200 * 1024) return failf(KB2SEQ_ERR_VALUE, "latent_window_attn: latent + rotated size %d too large", D);
   const dim3 grid(T, (H + HG - 1) / HG, nsplit);
+  const int unit = dt_cache ? 8 : 4;
+  const bool vec_k = r % unit == 0 && dr % unit == 0 && !(((uintptr_t)ckv | (uintptr_t)kr) & 15);
   const bool vec_q = r % 4 == 0 && dr % 4 == 0 && dn % 4 == 0 && ldp % 4 == 0 && !(((uintptr_t)q_abs | (uintptr_t)proj) & 15);
 #define KB2_LA(HGV, NCV)                                                                                                                      \
   case HGV * 32 + NCV: {                                                                                                                      \
@@ -2705,7 +2730,7 @@ KB2SEQ_API int kb2_seq_latent_window_attn(const float* q_abs, const float* proj,
       SEQ_CUDA(cudaFuncSetAttribute(latent_window_attn_kernel<HGV, NCV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));            \
     kb2::launch_pdl(latent_window_attn_kernel<HGV, NCV>, grid, kAttnThreads, smem, (cudaStream_t)stream,                                                    \
         q_abs, proj, ldp, H, dn, dr, r, ckv, kr, dt_cache, positions, seq_of, pages, max_pages, page_size, sinks, scale, window, out, cu,     \
-        skip_from, nsplit, part_acc, part_ml, gate, ldg, vec_q);                                                                              \
+        skip_from, nsplit, part_acc, part_ml, gate, ldg, vec_q, vec_k);                                                                              \
     break;                                                                                                                                    \
   }
   switch (HG * 32 + NC) {
