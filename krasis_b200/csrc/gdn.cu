@@ -196,11 +196,13 @@ __global__ void __launch_bounds__(256) gdn_prep_tiled_kernel(GdnDims d, const __
 // Vectorised variant (dk == dv == 128, conv width 4): one warp per (tile of 16 tokens, head); every lane owns FOUR CONSECUTIVE
 // channels of the head and asks for all its rows before the first is used (8 bytes a row, read back by the lane that copied them), and
 // the conv window lives in registers.  Products and sums run on pairs of numbers, roundings on the packed converter, the same bits as one by one.
-// SiLU uses ex2 and an approximate reciprocal: the f32 result differs from expf by <= 2 ulp,
-// which moves a BF16 rounding only when the value sits within 2^-22 of a rounding boundary (p ~ 6e-5 per element).
+// SiLU uses ex2 and an approximate reciprocal.  Its argument is a bf16 number y, and y log2(e) is rounded once ahead of ex2, so the f32 result is off by up to
+// (1.1 max(-y, 0) + 5) 2^-24 of its size; for none of the bf16 numbers from -87 to 88 does that move its bf16 rounding (all of them compared with fp64).
 // Rounding points are those of gdn_prep_kernel; the l2norm partial sums are grouped per lane differently (f32 addition order).
 // Bound by its instructions and, in short steps, by the way of its rows.  64 heads of 128, 100 / 500 / 1000 / 2000 / 3333 tokens: one number at a time with four rows
 // ahead, tiles of 16 rows up to 2048 tokens and of 32 beyond, 8.9 / 11.7 / 20.1 / 33.0 / 51.4 us; this way 8.0 / 9.5 / 14.1 / 24.0 / 35.8.
+// A call's last rows that do not make four go one by one: a layer's step of 1 / 4 / 8 tokens 55.5 / 59.3 / 61.3 us with the loop that left at the last row, 59.3 /
+// 62.0 / 62.5 with all sixteen rows always worked out, 55.5 / 58.8 / 60.5 now; 16 tokens 64.2 / 62.6 / 62.4.
 constexpr int kGdnGateRows = 8, kGdnTile = 16, kGdnPrepSmem = 8 * (kGdnTile + 3) * 256;
 struct F2 {                          // two numbers for the paired instructions
   unsigned long long v;
@@ -326,39 +328,36 @@ __global__ void __launch_bounds__(256, 4) gdn_prep_vec_kernel(GdnDims d, const _
   const int dst_ld = (is_q || is_k) ? kd : vd;
   dst += (long long)t_begin * dst_ld + lane * 4;
   const int n = t_end - t_begin;
-  auto four = [&](int i0) {                                         // four rows of the tile, without a branch between them
+  auto row = [&](int i) {
+    const uint2 cur = mine[(i + KW - 1) * 32];
+    const F2 x[2] = {f2_of_bf16(cur.x), f2_of_bf16(cur.y)};
+    uint32_t bits[2];
+    F2 sv[2];
 #pragma unroll
-    for (int i = i0; i < i0 + 4; ++i) {
-      const uint2 cur = mine[(i + KW - 1) * 32];
-      const F2 x[2] = {f2_of_bf16(cur.x), f2_of_bf16(cur.y)};
-      uint32_t bits[2];
-      F2 sv[2];
+    for (int p = 0; p < 2; ++p) {
+      F2 acc = f2_fma(w[p][0], hist[p][0], f2(0.f, 0.f));
+#pragma unroll
+      for (int j = 1; j < KW - 1; ++j) acc = f2_fma(w[p][j], hist[p][j], acc);
+      acc = f2_fma(w[p][KW - 1], x[p], acc);
+#pragma unroll
+      for (int j = 0; j < KW - 2; ++j) hist[p][j] = hist[p][j + 1];
+      hist[p][KW - 2] = x[p];
+      bits[p] = bf16_of_f2(silu2(bf16r2(acc)));
+      sv[p] = f2_of_bf16(bits[p]);
+    }
+    if (is_q || is_k) {
+      const float2 a = f2_get(bf16r2(f2_mul(sv[0], sv[0]))), b = f2_get(bf16r2(f2_mul(sv[1], sv[1])));
+      float ss = (a.x + a.y) + (b.x + b.y);
+#pragma unroll
+      for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const float inv = bf16r(rsqrtf(bf16r(bf16r(ss) + 1e-6f)));
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
-        F2 acc = f2_fma(w[p][0], hist[p][0], f2(0.f, 0.f));
-#pragma unroll
-        for (int j = 1; j < KW - 1; ++j) acc = f2_fma(w[p][j], hist[p][j], acc);
-        acc = f2_fma(w[p][KW - 1], x[p], acc);
-#pragma unroll
-        for (int j = 0; j < KW - 2; ++j) hist[p][j] = hist[p][j + 1];
-        hist[p][KW - 2] = x[p];
-        bits[p] = bf16_of_f2(silu2(bf16r2(acc)));
-        sv[p] = f2_of_bf16(bits[p]);
+        bits[p] = bf16_of_f2(f2_mul(sv[p], f2(inv, inv)));
+        if (is_q) bits[p] = bf16_of_f2(f2_mul(f2_of_bf16(bits[p]), f2(d.scale, d.scale)));
       }
-      if (is_q || is_k) {
-        const float2 a = f2_get(bf16r2(f2_mul(sv[0], sv[0]))), b = f2_get(bf16r2(f2_mul(sv[1], sv[1])));
-        float ss = (a.x + a.y) + (b.x + b.y);
-#pragma unroll
-        for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        const float inv = bf16r(rsqrtf(bf16r(bf16r(ss) + 1e-6f)));
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-          bits[p] = bf16_of_f2(f2_mul(sv[p], f2(inv, inv)));
-          if (is_q) bits[p] = bf16_of_f2(f2_mul(f2_of_bf16(bits[p]), f2(d.scale, d.scale)));
-        }
-      }
-      if (i < n) *reinterpret_cast<uint2*>(dst + (long long)i * dst_ld) = make_uint2(bits[0], bits[1]);
     }
+    *reinterpret_cast<uint2*>(dst + (long long)i * dst_ld) = make_uint2(bits[0], bits[1]);
   };
   cp_async_wait<3>();
   if (t_begin > 0) {
@@ -370,6 +369,11 @@ __global__ void __launch_bounds__(256, 4) gdn_prep_vec_kernel(GdnDims d, const _
     }
   }
   static_assert(TT == 16 && KW == 4, "a group of four rows per wait");
+  auto four = [&](int i0) {                                         // without a branch between them
+    if (n < i0 + 4) return;
+#pragma unroll
+    for (int i = i0; i < i0 + 4; ++i) row(i);
+  };
   four(0);
   cp_async_wait<2>();
   four(4);
@@ -377,6 +381,8 @@ __global__ void __launch_bounds__(256, 4) gdn_prep_vec_kernel(GdnDims d, const _
   four(8);
   cp_async_wait<0>();
   four(12);
+#pragma unroll 1
+  for (int i = n & ~3; i < n; ++i) row(i);                          // what is left of a call's last tile
 }
 
 // new conv state = last K pre-conv inputs (older entries come from the previous state when M < K)

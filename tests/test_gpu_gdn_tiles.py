@@ -1,5 +1,5 @@
-"""Token tiles of the DeltaNet preparation: a prompt in one call (32-row tiles past 2048 tokens) against the same prompt in parts (16-row tiles,
-history from the convolution state)."""
+"""Token tiles of the DeltaNet preparation, sixteen rows in groups of four and a remainder: a prompt in one call against the same prompt in parts (history from
+the convolution state)."""
 import types
 
 import pytest
@@ -33,3 +33,9 @@ def test_one_call_and_parts_agree(M, cuts):
     assert abs(conv - conv2).max() <= 2 ** -7 * abs(conv).max()
     assert abs(rec - rec2).max() <= 5e-3 * max(1.0, abs(rec).max())
     assert (whole - parts).abs().max() <= 3 * 2 ** -7 * whole.abs().max()
+
+
+@pytest.mark.parametrize("M,cuts", [(20, (1, 3, 6, 10, 15)), (31, (16, 23)), (45, (13, 14, 27, 36))])
+def test_remainders_of_a_tile(M, cuts):
+    """Calls of 1 to 16 tokens, and 17 and more: every number of rows in the last group of four."""
+    test_one_call_and_parts_agree(M, cuts)
