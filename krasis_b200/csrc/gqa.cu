@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(256, 4) gqa_prep_rows_kernel(GqaDims g, const 
                                                                uint8_t* __restrict__ k_cache, uint8_t* __restrict__ v_cache, int M, int tokens) {
   pdl_enter(q_raw, k_raw, v_raw, q_norm, k_norm, positions, kv_indices, q_out, k_cache, v_cache);
   constexpr int NP = D / 64;                 // a lane's pairs of a row: numbers 64 k + 2 lane and the one behind it
-  __shared__ float2 s_turn[kPrepTokens][HALF];      // cos, sin
+  __shared__ __align__(16) float2 s_turn[kPrepTokens][HALF];      // cos, sin, read two at a time
   __shared__ long long s_slot[kPrepTokens];
   const int t0 = blockIdx.x * tokens, nt = min(tokens, M - t0), warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int heads = g.nh + 2 * g.nkv, units = nt * heads;

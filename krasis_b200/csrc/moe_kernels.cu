@@ -25,8 +25,8 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const __nv_bfloat16*
                                                             const float* __restrict__ gate_bias,
                                                             float* __restrict__ logits, int M, int E, int H) {
   pdl_enter(h, gate, gate_bias, logits);
-  __shared__ float hs[RK][RT + 4];
-  __shared__ float gs[RK][RT + 4];
+  __shared__ __align__(16) float hs[RK][RT + 4];
+  __shared__ __align__(16) float gs[RK][RT + 4];
   const int m0 = blockIdx.y * RT, e0 = blockIdx.x * RT;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   float acc[4][4] = {};
