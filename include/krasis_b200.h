@@ -260,6 +260,8 @@ KB2_API int kb2_linear_glu_bf16_binned(const void* x_dev, const void* w_dev, voi
  * parts in workspace_dev, exact but for what lies below 2^-134 (numbers below 1e-33 keep fewer than 24 bits)
  * (kb2_linear_f32_workspace bytes, 16-byte aligned; 0: sizes not taken). */
 KB2_API size_t kb2_linear_f32_workspace(int32_t M, int32_t N, int32_t K, int32_t w_f32, int32_t groups, int32_t device);
+/* Rows of x per tile where such a product runs on pairs of CTAs, 0 where on single ones. */
+KB2_API int32_t kb2_linear_f32_pair_rows(int32_t M, int32_t N, int32_t K, int32_t w_f32, int32_t groups, int32_t device);
 KB2_API int kb2_linear_f32(const float* x_dev, int64_t x_ld, int64_t x_group, const void* w_dev, int32_t w_f32, void* out_dev, int32_t out_f32,
                            int64_t out_ld, int64_t out_group, int32_t M, int32_t N, int32_t K, int32_t groups, void* workspace_dev,
                            size_t workspace_bytes, int32_t device, void* stream);

@@ -112,6 +112,7 @@ SIGNATURES = {
     "kb2_fmha_latent_gated": (C.c_int, [C.c_void_p] * 4 + [C.c_int32] * 4 + [C.c_float, C.c_int32, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32,
                                                                               C.c_void_p]),
     "kb2_linear_f32_workspace": (C.c_size_t, [C.c_int32] * 6),
+    "kb2_linear_f32_pair_rows": (C.c_int32, [C.c_int32] * 6),
     "kb2_linear_f32": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_int32, C.c_void_p, C.c_int32, C.c_int64, C.c_int64] +
                        [C.c_int32] * 4 + [C.c_void_p, C.c_size_t, C.c_int32, C.c_void_p]),
     "kb2_linear_bf16_chunked": (C.c_int, [C.c_void_p] * 4 + [C.c_int32] * 5 + [C.c_void_p]),

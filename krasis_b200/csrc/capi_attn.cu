@@ -260,6 +260,12 @@ KB2_API size_t kb2_linear_f32_workspace(int32_t M, int32_t N, int32_t K, int32_t
   return x_parts_bytes(plan, M, K, groups) + (plan.pair ? parts_partial_bytes(M, cols, groups, plan.ks) : 0) + (w_f32 ? (size_t)groups * (cols * (size_t)K * 6 + (cols + 127) / 128 * 32) : 0);
 }
 
+KB2_API int32_t kb2_linear_f32_pair_rows(int32_t M, int32_t N, int32_t K, int32_t w_f32, int32_t groups, int32_t device) {
+  SplitPlan plan;
+  if (M <= 0 || N <= 0 || K <= 0 || groups <= 0 || !linear_f32_plan(M, linear_f32_columns(N, K, w_f32, groups), K, w_f32, groups, device, &plan)) return 0;
+  return plan.pair ? plan.mt : 0;
+}
+
 KB2_API int kb2_linear_f32(const float* x_dev, int64_t x_ld, int64_t x_group, const void* w_dev, int32_t w_f32, void* out_dev, int32_t out_f32,
                            int64_t out_ld, int64_t out_group, int32_t M, int32_t N, int32_t K, int32_t groups, void* workspace_dev,
                            size_t workspace_bytes, int32_t device, void* stream) {

@@ -57,3 +57,31 @@ def test_what_is_not_finite(M, N, K, G):
         assert torch.equal(test(got), test(want))
     rows = [i for i in range(M) if i not in (3, 200, M - 1)]
     _close(got[rows], x[rows], w)
+
+
+# rows of the tiles that the shapes above take, with bf16 and with fp32 weights; a shape for each that takes tiles of 64
+TILES = [s + r for s, r in zip(SHAPES, [(96, 96), (128, 128), (96, 96), (128, 128), (96, 96)])] + [(145, 12304, 4096, 1, 64, 0), (193, 4112, 512, 1, 0, 64)]
+
+
+@pytest.mark.parametrize("M,N,K,G,narrow,wide", TILES)
+def test_forms_that_are_compared(M, N, K, G, narrow, wide):
+    """The tests of this file compare pairs of CTAs with single ones: steps of M rows run on the former, of nine on the latter."""
+    from krasis_b200 import capi
+    dev = torch.cuda.current_device()
+    if torch.cuda.get_device_properties(dev).multi_processor_count != 148:
+        pytest.skip("the tiles are those of 148 SMs")
+    rows = capi.load().kb2_linear_f32_pair_rows
+    assert (rows(M, N, K, 0, G, dev), rows(M, N, K, 1, G, dev)) == (narrow, wide)
+    assert rows(9, N, K, 0, G, dev) == rows(9, N, K, 1, G, dev) == 0
+
+
+@pytest.mark.parametrize("M,N,K,G,narrow,wide", TILES[len(SHAPES):])
+def test_tiles_of_64_rows(M, N, K, G, narrow, wide):
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn(M, G, K, device="cuda", generator=g)
+    w = torch.randn(G, N, K, device="cuda", generator=g) * K ** -0.5
+    for m in [w.bfloat16()] if narrow else [w, w.bfloat16().float()]:
+        got = _product(x, m)
+        _close(got, x, m)
+        assert torch.equal(_product(x[:9].contiguous(), m), got[:9])
+        assert torch.equal(_product(x[M - 9:].contiguous(), m), got[M - 9:])
