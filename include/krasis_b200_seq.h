@@ -95,13 +95,17 @@ KB2SEQ_API int kb2_seq_residual_scale_rms(float* x, const float* y, float y_mult
 KB2SEQ_API int kb2_seq_residual_post_rms(float* x, const float* y1, float c1, const float* y2, float c2, const float* bias, float mult,
                                          const float* w, const float* wh, void* h, int dt_h, int T, int W, float eps, void* stream);
 
+/* A step in which every sequence decodes: the short convolution of proj's first columns (kb2_seq_conv_silu) with its tail, then the gated delta rule below, in one
+ * launch and with the bits of those.  Row t is the one token of the sequence with state slot slots[t], all of them different.  dk and dv 128, at most 8 heads per key
+ * head, K = 2 to 4 taps; ldp and g_off multiples of 4; proj, norm_w, state and out 16-byte aligned. */
+KB2SEQ_API int kb2_seq_delta_step(const float* proj, long long ldp, int g_off, int a_off, int b_off, int T, int H, int Hk, int dk, int dv, int K,
+                                  const float* taps, float* tail, const float* A_log, const float* dt_bias, const float* norm_w, float eps, float* state,
+                                  const int* slots, void* out, int dt_out, void* stream);
+
 /* gated delta rule over each sequence's portion; state [slots][H][dk][dv] fp32 is read and written back.
  * scratch (fp32, 2 T Hk dk + 2 T H + T H dv + 4 elements, 16-byte aligned) selects the register-state kernels when dk is 32, 64 or
  * 128 and dv a multiple of 32; with scratch == NULL, or other sizes, one block per (sequence, head) keeps the state in shared memory
  * (a state too large for that is cut into slices of value columns, one block each; this needs scratch). */
-KB2SEQ_API int kb2_seq_delta_step(const float* proj, long long ldp, int g_off, int a_off, int b_off, int T, int H, int Hk, int dk, int dv, int K,
-                                  const float* taps, float* tail, const float* A_log, const float* dt_bias, const float* norm_w, float eps, float* state,
-                                  const int* slots, void* out, int dt_out, void* stream);
 KB2SEQ_API int kb2_seq_delta_rule(const float* conv, int C, const float* proj, long long ldp, int g_off, int a_off, int b_off, int T,
                                   int S, int H, int Hk, int dk, int dv, const float* A_log, const float* dt_bias, const float* norm_w,
                                   float eps, float* state, const int* cu, const int* slots, float* scratch, void* out, int dt_out,

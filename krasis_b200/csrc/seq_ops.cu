@@ -2969,8 +2969,6 @@ KB2SEQ_API int kb2_seq_delta_rule_ch(const float* conv, int C, const float* beta
                            state, cu, slots, scratch, out, dt_out, stream);
 }
 
-// The convolution of proj's first channels, its tail and the delta rule with its gated read-out for a step of T sequences of one token each (row t: the
-// sequence with state slot slots[t]); see kb2_seq_conv_silu and kb2_seq_delta_rule.  dk and dv 128, H / Hk <= 8, 2 to 4 taps, 16-byte aligned rows.
 KB2SEQ_API int kb2_seq_delta_step(const float* proj, long long ldp, int g_off, int a_off, int b_off, int T, int H, int Hk, int dk, int dv, int K,
                                   const float* taps, float* tail, const float* A_log, const float* dt_bias, const float* norm_w, float eps, float* state,
                                   const int* slots, void* out, int dt_out, void* stream) {

@@ -36,3 +36,19 @@ def test_same_as_separate_launches(H, Hk, K, T, dtype):
     assert torch.isfinite(ends[0][0]).all()
     untouched = [s for s in range(slots) if s not in order]
     assert (ends[0][-1][untouched] == 0.01).all() and (ends[0][-2][untouched] == 0.3).all()
+
+
+@pytest.mark.parametrize("H,Hk,K", [(10, 2, 4), (8, 1, 2), (14, 2, 3), (16, 2, 4)])
+def test_clusters_of_more_heads(H, Hk, K):
+    """Five, seven and eight heads per key head: a cluster of as many blocks."""
+    test_same_as_separate_launches(H, Hk, K, 5, torch.bfloat16)
+
+
+@pytest.mark.parametrize("kw", [{"dk": 64}, {"dv": 64}, {"K": 5}, {"K": 1}, {"H": 18, "Hk": 2}, {"H": 5, "Hk": 2}, {"ldp": 4098}, {"g_off": 2}, {"T": 0}, {"state": 8}])
+def test_what_is_refused(kw):
+    a = dict(ldp=4096, g_off=1024, T=1, H=4, Hk=2, dk=128, dv=128, K=4, state=0)
+    a.update(kw)
+    buf = torch.zeros(4, dtype=torch.int32, device="cuda")
+    p = buf.data_ptr()
+    rc = seqops.load().kb2_seq_delta_step(p, a["ldp"], a["g_off"], 0, 0, a["T"], a["H"], a["Hk"], a["dk"], a["dv"], a["K"], p, p, p, p, p, 1e-5, p + a["state"], p, p, 1, None)
+    assert rc == 2
