@@ -337,7 +337,8 @@ class GatedDeltaMixer:
         lib, T = ops.load(), h.shape[0]
         proj = lin(h, self.w_in, torch.float32)
         s = stream_of(h)
-        if self.one_launch and T == tb.S and proj.stride(0) % 4 == 0 and all(n == 1 for _, n, _, _ in tb.layout):      # every sequence decodes
+        if (self.one_launch and T == tb.S and proj.stride(0) % 4 == 0 and not state.data_ptr() & 15
+                and all(n == 1 for _, n, _, _ in tb.layout)):                   # every sequence decodes
             o = torch.empty((T, self.H * self.dv), dtype=self.dtype, device=h.device)
             ops.check(lib.kb2_seq_delta_step(proj.data_ptr(), proj.stride(0), self.g_off, self.a_off, self.b_off, T, self.H, self.Hk, self.dk, self.dv, self.K,
                                              self.taps.data_ptr(), tail.data_ptr(), self.A_log.data_ptr(), self.dt_bias.data_ptr(), self.norm.data_ptr(),

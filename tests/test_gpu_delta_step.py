@@ -52,3 +52,22 @@ def test_what_is_refused(kw):
     p = buf.data_ptr()
     rc = seqops.load().kb2_seq_delta_step(p, a["ldp"], a["g_off"], 0, 0, a["T"], a["H"], a["Hk"], a["dk"], a["dv"], a["K"], p, p, p, p, p, 1e-5, p + a["state"], p, p, 1, None)
     assert rc == 2
+
+
+def test_state_off_16_bytes():
+    """States that begin off 16 bytes are taken, and give the same bits."""
+    g = torch.Generator().manual_seed(2)
+    W, n, H, slots = 256, 128, 2, 3
+    r = lambda *s, sd=0.06: torch.randn(*s, generator=g) * sd  # noqa: E731
+    w = {"g": r(H * n, W), "a": r(H, W), "b": r(H, W), "A_log": r(H), "dt_bias": r(H) - 3.0, "norm": 1.0 + r(n), "o": r(W, H * n)}
+    for nm in ("q", "k", "v"):
+        w[nm], w[nm + "_conv"] = r(H * n, W), r(H * n, 4, sd=0.5)
+    m = GatedDeltaMixer(w, H, H, n, n, 4, 1e-5, torch.bfloat16, "cuda")
+    x, tb = r(2, W, sd=1.0).cuda().bfloat16(), seqops.StepTables([([0], 4, 2, [0]), ([0], 9, 0, [0])], "cuda")
+    ends = []
+    for off in (0, 1):
+        state = torch.empty(slots * H * n * n + off, device="cuda")[off:].view(slots, H, n, n).fill_(0.01)
+        tail = torch.full((slots, m.C, 3), 0.3, device="cuda")
+        ends.append([m.forward(x, tb, tail, state), tail, state])
+    for a, b in zip(*ends):
+        assert torch.equal(a, b)
