@@ -3,8 +3,9 @@
 // written.  Between plain launches the chip stands idle for 1 to 2 us; small steps are chains of dozens of them.  us per call, plain launches
 // and these: 3 tokens through 8 of 256 experts (6 launches) 55.8 / 43, a latent-attention layer of 1000 tokens (6) 79.3 / 68.7, 128 tokens
 // through routed bf16 experts (11) 211 / 188, a captured decode step of 4 requests (46) 254 / 244.
-// Kernels of few registers and no shared memory to speak of let the next one come up when their own wait is over (pdl_trigger: residual norms, gates, the delta
-// rule's decode step, the join of latent attention's pieces): a serving run of 4 requests 4880 -> 4765 us.  The others do not: with that at the start of
+// Some kernels let the next one come up when their own wait is over (pdl_trigger): those of few registers and next to no shared memory that many short steps run
+// (residual norms, gates, the join of latent attention's pieces), and the delta rule's decode step (256 threads of 128 registers, 10 KB, a block per token and head:
+// what it leaves of an SM is room for the next): a serving run of 4 requests 4880 -> 4765 us.  The others do not: with that at the start of
 // every kernel waiting blocks took slots for whole kernels, and 8192 tokens through routed experts took 734 us instead of 720, 389 tokens 144 instead of
 // 137, the decode step 262.  Bringing the waiting products' weights into L2 meanwhile gained nothing (4720; all of a product's weights at once 4880).
 // Rules that keep this safe:
@@ -26,8 +27,7 @@ __device__ __forceinline__ long long pdl_wait() {
   asm volatile("griddepcontrol.wait;\n\tmov.u64 %0, 0;" : "=l"(zero)::"memory");
   return zero;
 }
-// Lets the next kernel in the stream come up now, as soon as every block of this one has said so or left.  For kernels of few registers and little shared
-// memory, behind their own wait.
+// Lets the next kernel in the stream come up now, as soon as every block of this one has said so or left.  Behind the kernel's own wait.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // pdl_wait for a kernel with the pointers p: loads through a __restrict__ pointer may otherwise move ahead of the wait, so each of them gets the
 // wait's zero added.

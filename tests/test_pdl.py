@@ -101,6 +101,28 @@ def test_a_kernel_without_its_wait_is_found(name):
     assert _reads_ahead(params, moved[:moved.index("pdl_wait(")])
 
 
+def _early(body):
+    """Whether a kernel lets the next one come up ahead of its own wait, or of a place where some of its blocks may leave without saying so."""
+    wait, at = re.search(r"pdl_(?:enter|enter_global|wait)\([^;]*;", body), re.search(r"pdl_trigger\(", body)
+    return at.start() < wait.end() or bool(re.sub(r"[\s]|kb2::", "", body[wait.end():at.start()]))
+
+
+def test_triggers_stand_behind_the_wait():
+    """Right behind it: what is launched early waits for the whole of this kernel, which has then waited for all ahead of it."""
+    launched, found = _launched(), []
+    for name, (_, body) in _bodies().items():
+        if "pdl_trigger(" in body:
+            assert name in launched and len(re.findall(r"pdl_trigger\(", body)) == 1 and not _early(body), name
+            found.append(name)
+    assert sorted(found) == ["act_mul_bf16x8_kernel", "delta_step_kernel", "latent_attn_combine_kernel", "residual_norm_vec_kernel", "side_gate_kernel"]
+
+
+def test_an_early_trigger_is_found():
+    body = _bodies()["side_gate_kernel"][1]
+    moved = re.sub(r"(?:kb2::)?pdl_trigger\(\);", "", body)
+    assert _early("{ kb2::pdl_trigger();" + moved[1:])
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("rows", [1, 8, 77, 300])
 def test_chain_equals_single_launches(rows):
