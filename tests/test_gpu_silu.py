@@ -40,3 +40,43 @@ def test_sign_of_zero(dtype):
     for kind, kw in ((1, {}), (2, {"limit": 7.0, "alpha": 1.7})):
         got = ops.glu(gu, dtype, kind, **kw)
         assert torch.equal(got.float().signbit(), g.signbit()) and not got.any()
+
+
+def _arguments(n):
+    """Numbers of either sign and all sizes, a fine row around zero, and both ends of exp."""
+    size = torch.logspace(-44, 38, n // 4, device="cuda")
+    return torch.cat([size, -size, torch.linspace(-4.0, 4.0, n // 4, device="cuda"), torch.linspace(-104.0, 104.0, n - 3 * (n // 4), device="cuda")])
+
+
+@pytest.mark.parametrize("act", ["silu", "sigmoid"])
+@pytest.mark.parametrize("dv", [64, 63])                     # four columns a lane, and one
+def test_gates(act, dv):
+    from krasis_b200 import seqops as ops
+    T, H = 128, 2
+    z = _arguments(T * H * dv).view(T, H * dv)
+    got = ops.head_norm_gate(torch.ones_like(z), H, dv, torch.float32, gate=z, gate_act=act).double()
+    x = z.double()
+    want = (x if act == "silu" else 1.0) / (1.0 + torch.exp(-x))
+    # expf 2 ulp (2^-22), a sum (2^-24), a quotient (2^-23); where e^-x passes fp32's largest number the answer is 0 for x e^-88.7 or e^-88.7, and what lies below fp32's
+    # smallest normal number is rounded to multiples of 2^-149
+    assert ((got - want).abs() <= 1.75 * 2.0 ** -22 * want.abs() + (3e-37 if act == "silu" else 4e-39)).all()
+    ends = torch.tensor([[float("inf"), -float("inf"), float("nan"), 0.0]], device="cuda").repeat(1, dv)[:, :dv].contiguous()
+    got = ops.head_norm_gate(torch.ones_like(ends), 1, dv, torch.float32, gate=ends, gate_act=act)[0, :4].tolist()
+    assert got[0] == (float("inf") if act == "silu" else 1.0) and got[2] != got[2] and got[3] == (0.0 if act == "silu" else 0.5)
+    assert got[1] != got[1] if act == "silu" else got[1] == 0.0
+
+
+@pytest.mark.parametrize("F", [4096, 4095])
+def test_clamped_swish(F):
+    """g' sigmoid(alpha g') (u' + 1) with g' = min(g, limit), u' = clamp(u, -limit, limit)."""
+    from krasis_b200 import seqops as ops
+    limit, alpha = 7.0, 1.702
+    g = torch.stack([_arguments(F), torch.linspace(-60.0, 9.0, F, device="cuda")])
+    u = torch.linspace(-9.0, 9.0, F, device="cuda").repeat(2, 1)
+    got = ops.glu(torch.cat([g, u], 1).contiguous(), torch.float32, ops.GLU_CLAMPED_SWISH, limit=limit, alpha=alpha).double()
+    a = torch.tensor(alpha, device="cuda").double()           # as fp32 has it
+    x, y = g.double().clamp(max=limit), u.double().clamp(-limit, limit)
+    want = x / (1.0 + torch.exp(-a * x)) * (y + 1.0)
+    # as above, the argument of expf rounded once (|alpha x| 2^-24 of e^-alpha x) up to where the answer is 0, u + 1 and the product once each
+    room = (1.75 * 2.0 ** -22 + 2.0 ** -23 + (a * x).abs().clamp(max=104.0) * 2.0 ** -24) * want.abs() + 2.0 ** -24 * x.abs() / (1.0 + torch.exp(-a * x))
+    assert ((got - want).abs() <= room + 2e-36).all()
