@@ -298,7 +298,7 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 // while the softmax warps work, and these hardly wait for it; K and V have a loader each.  An MMA reads its 128 x 16 piece of Q from shared memory again, 32
 // cycles for 32 of work with 64 keys: tiles of 128 where tensor memory has room.  Where the last tile has keys in its first 64 alone, the softmax warps and the
 // second product take that half: the same bits, as the others have weight 0.  What is left: with 128 value columns the softmax (17 tokens after 1000 and 3000 keys
-// 14.6 and 32.1 us: 1.12 us a tile, 0.53 of it the exponentials, 16 of them a cycle), with 256 the MMAs (17.2 and 40.5 us: 0.75 us a tile of 64).  us with single
+// 14.6 and 32.1 us: 1.12 us a tile, 0.53 of it the exponentials, 16 of them a cycle), with 256 0.75 us a tile of 64 (17.2 and 40.5 us; an MMA with 64 keys takes as long as one with 128).  us with single
 // buffers, one loader and tiles of 64 keys, and now: 2048 x 16 heads of 256 after 2500 keys 140 -> 134; latent attention of 16 heads: 2000 tokens 36.9 -> 32.0, 1000
 // 19.4 -> 16.4, 512 after 700 21.8 -> 18.5, 17 after 300 9.2 -> 8.3, 128 alone 7.5 -> 8.2 (one tile where two overlapped), 64 alone 5.9 -> 6.2 (7.2 without the half);
 // 16 heads of 128, 2000 tokens 36.3 -> 29.5.  Tried: the tiles to two groups of warps in turn, a thread per row (latent 18.0: its warps are one per scheduler); pairs

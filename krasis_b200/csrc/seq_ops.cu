@@ -1747,10 +1747,10 @@ __global__ void __launch_bounds__(32 * kRegPieces) delta_rule_reg_kernel(const f
 // and transposed for k u^T; the partial sums of a group's warps meet in shared memory in fragment order, so nothing is moved between lanes.
 // The largest of the six products of an update and of a read-out goes eight tokens at a time, each to a sum of its own: the tensor cores cut off
 // what they add, and with sixteen at a time states were 1 % further off (6.6e-7 instead of 6.5e-7).
-// Bound: 1300 cycles of the tensor pipe and 1400 of shared memory per tile, of about 2200 (4096 tokens, 32 / 16 heads x 128: 310 us, the prep 98); left
+// Bound: 1270 cycles of the tensor pipe and 1370 of shared memory per tile, of 2210 (counters at 2048 tokens; 4096 tokens, 32 / 16 heads x 128: 310 us, the prep 98); left
 // is the chain split - W - exchange - u - update.  The next tile is waited for and its W fetched between the instructions of the update and the use of their sums,
 // and the read-out's buffer at its first store: with all three at the head of a tile 338 us (q fetched ahead of W's sums as well: 364).
-// With eight tokens per tile, where each warp solved for u itself, a tile took 2400 cycles of dependent short phases, and the whole 642 + 56 us.
+// With eight tokens per tile, where each warp solved for u itself, the phases were shorter and as dependent, and the whole took 642 + 56 us.
 constexpr int kDT = 16, kDTStages = 4;
 // what couples the tokens of a (tile, head): G[16] | D_15,j [16] | G_15 and padding to 48 floats | D_ij q_i . k_j as three bf16 parts [i][24]
 constexpr int kDTG = 0, kDTEnd = 16, kDTAll = 32, kDTQK = 48, kDTQKPitch = 24, kDTQKPart = kDT * kDTQKPitch;

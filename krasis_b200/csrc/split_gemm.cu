@@ -296,8 +296,7 @@ __global__ void __launch_bounds__(kSThreads)
 // 512 rows, N 8192, K 2048 in three products: 61 -> 43 us (1.2 PFLOP/s; 128 tiles of 128 rows on 74 pairs are two rounds for 1.73, and under this load the clock
 // is that of a cuBLAS product at 1.64 PFLOP/s); N 2048, K 8192 69 -> 42 us and 5 for the segments' sums.
 // Per K block of 64 a CTA takes in 16 KB of weights and 24 KB of x for 768 cycles of MMAs (128 rows): [w1 | its half of x1 | x2 (the first CTA) or
-// x3], so that one MMA of twice the columns multiplies x2 and x3 (an MMA of a pair takes 89 cycles at least: a K block 711 cycles with 64 rows or fewer, 868
-// with 128).  Where w2 and w3 hold anything, a second stage [w2 | w3 | halves of x1 | of x2] follows.
+// x3], so that one MMA of twice the columns multiplies x2 and x3 (512 rows, N 8192, K 2048: the tensor pipe is active in 0.63 of the cycles, 768 a K block).  Where w2 and w3 hold anything, a second stage [w2 | w3 | halves of x1 | of x2] follows.
 constexpr int kPTThreads = 384, kPTWarps = 8, kPTMaxStages = 8, kPTRing = 216 * 1024, kPTSmem = kPTRing + (2 * kPTMaxStages + 6) * 8 + 8;
 static_assert(kPTSmem >= tmem_smem(512) && kPTSmem <= 227 * 1024, "what a CTA of a cluster takes for 512 columns");
 
@@ -676,7 +675,7 @@ static void parts_pair_plan(int M, int N, int K, int num_sms, int wparts, int gr
   for (int nt = 128; nt >= 64; nt -= 32) {                     // fewer rows take as long as 64
     const long long units = (long long)ceil_div(N, 2 * kSRows) * ceil_div(M, nt) * groups * out->ks;
     const float rounds = (float)((units + num_sms / 2 - 1) / (num_sms / 2));
-    const float block = 4.f * (std::max(89.f, nt * 0.5f) + std::max(89.f, (float)nt)) / 1550.f;      // an MMA takes 89 cycles at least
+    const float block = 4.f * (std::max(89.f, nt * 0.5f) + std::max(89.f, (float)nt)) / 1550.f;      // the two MMAs of a step; what fits the timings
     const float time = 11.5f + std::max(hbm, rounds * (1.5f + kb * block)) + (partial ? 3.f + 2.f * partial / 8e6f : 0.f);
     if (time >= us) continue;
     us = time;
